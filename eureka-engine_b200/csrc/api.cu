@@ -104,13 +104,13 @@ int llb_b200_sync(void) {
 }
 llb_b200_dptr llb_b200_stream(void) { return (llb_b200_dptr)(uintptr_t)g_llb.stream; }
 
-size_t llb_b200_weight_bytes(int fmt, int rows, int cols) { return (size_t)rows * dev_row_bytes(fmt, cols); }
+size_t llb_b200_weight_bytes(int fmt, int rows, int cols) { return dev_bytes(fmt, rows, cols); }
 
 int llb_b200_weight_upload(int fmt, int rows, int cols, const void *src, int src_on_device, llb_b200_dptr dst) {
   NEED_INIT(-1)
   const size_t pb = (size_t)rows * pack_row_bytes(fmt, cols);
   if (!pack_row_bytes(fmt, cols)) return llb_fail("weight_upload: format %d / cols %d", fmt, cols);
-  if (fmt != LLB_FM_Q6_K) {
+  if (fmt == LLB_FM_F32) {
     CU_OK(cudaMemcpyAsync((void *)(uintptr_t)dst, src, pb, src_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                           g_llb.stream));
     if (!src_on_device) CU_OK(cudaStreamSynchronize(g_llb.stream));
@@ -124,7 +124,7 @@ int llb_b200_weight_upload(int fmt, int rows, int cols, const void *src, int src
     if (ce != cudaSuccess) { cudaFree(tmp); return llb_fail("weight_upload: copy of %zu bytes: %s", pb, cudaGetErrorString(ce)); }
     s = (const uint8_t *)tmp;
   }
-  int rc = ops_repack_q6k(g_llb.stream, s, (uint8_t *)(uintptr_t)dst, (size_t)rows * (cols / 256));
+  int rc = ops_to_tiles(g_llb.stream, fmt, s, rows, cols, (uint8_t *)(uintptr_t)dst);
   if (tmp) {
     cudaStreamSynchronize(g_llb.stream);
     cudaFree(tmp);
@@ -308,7 +308,7 @@ int llb_b200_gemm_noalloc(int fmt, llb_b200_dptr w, int rows, int K, llb_b200_dp
   if (K < 256 || K % 256 || K > NOALLOC_MAX_K) return llb_fail("gemm_noalloc: K = %d; this entry point takes multiples of 256 up to %d", K, NOALLOC_MAX_K);
   if (T < 1 || T > NOALLOC_MAX_T) return llb_fail("gemm_noalloc: T = %d; this entry point takes 1..%d rows", T, NOALLOC_MAX_T);
   if (rows < 1) return llb_fail("gemm_noalloc: rows = %d", rows);
-  if (!dev_row_bytes(fmt, K) || fmt == LLB_FM_F32) return llb_fail("gemm_noalloc: format %d has no kernel", fmt);
+  if (!tile_bytes(fmt)) return llb_fail("gemm_noalloc: format %d has no kernel", fmt);
   const int NC = 8;
   const int ks = gemm_pick_ksplit(fmt, NC, (rows + 15) / 16, K / 256, g_llb.sms);
   if ((size_t)ks * T * rows > NOALLOC_PART_FLOATS)

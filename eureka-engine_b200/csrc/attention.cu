@@ -14,9 +14,8 @@
 // The scalar-FMA kernel this replaces spent 2400 warp instructions per 32 positions and warp; this one about 350.
 #include "host.cuh"
 #include "model.cuh"
+#include "rowops.cuh"
 
-#define ATT_PT 32
-#define ATT_PS 40   // halves per row of the probability tiles: 80-byte rows keep ldmatrix conflict-free
 
 __device__ __forceinline__ float aw_max(float v) {
 #pragma unroll
@@ -28,16 +27,6 @@ __device__ __forceinline__ float aw_sum(float v) {
   for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
   return v;
 }
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-}
-
 // bytes of shared memory for NQG groups of 8 queries
 template <int HD> static size_t att_smem(int nqg) {
   const size_t rsk = (size_t)(HD + 8) * 2, nqp = (size_t)nqg * 8;

@@ -1,12 +1,14 @@
 // common.cuh -- shared device helpers of the B200 speculative-decoding library.
 //
-// Weight formats are the reference's (host/llb_formats.h:4-15).  Device layouts:
-//   Q8_0  as stored in a pack: row = [cols x int8][cols/32 x f16]          (tools/q8_pack.py:7-10)
-//   Q4_K  as stored: 144-byte super-blocks                                  (tools/qwen35_engine.c:258-272)
-//   Q5_K  as stored: 176-byte super-blocks                                  (tools/qwen35_engine.c:273-289)
-//   Q6_K  re-sliced at load: each 210-byte super-block is padded to 224 bytes
-//         [ql 128 | qh 64 | scales 16 | d 2 | zero 14] so that every super-block starts on a
-//         16-byte boundary (the stored 210-byte stride does not); values are unchanged.
+// Weight formats are the reference's (host/llb_formats.h:4-15).  In device memory a quantised matrix is made of
+// TILES of 16 rows x 256 columns (one super-block of 16 rows), [row tile][super-block], each tile contiguous, so that
+// one bulk copy brings a warp's next piece of work.  Inside a tile a row's block stays together:
+//   Q4_K  row r at 144 r, as stored: f16 d, f16 dmin, 12 B scales / mins, 128 B nibbles   (tools/qwen35_engine.c:258-272)
+//   Q5_K  row r at 176 r, as stored: Q4_K plus 32 B of fifth bits before the nibbles       (tools/qwen35_engine.c:273-289)
+//   Q6_K  row r at 208 r: ql 128 | qh 64 | scales 16; the sixteen f16 d follow at 3328 + 2 r (210 bytes a row, as stored)
+//   Q8_0  row r at 272 r: 256 codes as q + 128 | 8 f16 scales                              (tools/q8_pack.py:7-10)
+// Rows past the matrix (up to the next multiple of 16) and columns past it (Q8_0, up to the next multiple of 256) are zero
+// weights.  F32 matrices are row-major.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -18,20 +20,28 @@
 #define LLB_FM_Q6_K 4
 #define LLB_FM_Q5_K 9
 
-// bytes of one row in the DEVICE layout
-__host__ __device__ inline size_t dev_row_bytes(int fmt, int cols) {
+// bytes of one 16 x 256 tile, and of one row inside it
+__host__ __device__ constexpr int tile_bytes(int fmt) {
+  return fmt == LLB_FM_Q4_K ? 2304 : fmt == LLB_FM_Q5_K ? 2816 : fmt == LLB_FM_Q6_K ? 3360 : fmt == LLB_FM_Q8_0 ? 4352 : 0;
+}
+__host__ __device__ constexpr int tile_row(int fmt) {
+  return fmt == LLB_FM_Q4_K ? 144 : fmt == LLB_FM_Q5_K ? 176 : fmt == LLB_FM_Q6_K ? 208 : 272;
+}
+// bytes of a matrix in the DEVICE layout (0: no such format)
+__host__ __device__ inline size_t dev_bytes(int fmt, int rows, int cols) {
+  if (fmt == LLB_FM_F32) return (size_t)rows * cols * 4;
+  return (size_t)((rows + 15) >> 4) * ((cols + 255) >> 8) * tile_bytes(fmt);
+}
+// bytes of one row as stored in a pack (host/llb_formats.h:17)
+__host__ __device__ inline size_t pack_row_bytes(int fmt, int cols) {
   switch (fmt) {
     case LLB_FM_F32: return (size_t)cols * 4;
     case LLB_FM_Q8_0: return (size_t)cols / 32 * 34;
     case LLB_FM_Q4_K: return (size_t)cols / 256 * 144;
     case LLB_FM_Q5_K: return (size_t)cols / 256 * 176;
-    case LLB_FM_Q6_K: return (size_t)cols / 256 * 224;
+    case LLB_FM_Q6_K: return (size_t)cols / 256 * 210;
   }
   return 0;
-}
-// bytes of one row as stored in a pack (host/llb_formats.h:17)
-__host__ __device__ inline size_t pack_row_bytes(int fmt, int cols) {
-  return fmt == LLB_FM_Q6_K ? (size_t)cols / 256 * 210 : dev_row_bytes(fmt, cols);
 }
 
 // ---- activation planes -------------------------------------------------------------------------
@@ -216,15 +226,15 @@ __device__ __forceinline__ void q4k_scale_min(const uint8_t *s, int j, int &sc, 
   if (j < 4) { sc = s[j] & 63; mn = s[j + 4] & 63; }
   else { sc = (s[j + 4] & 15) | ((s[j - 4] >> 6) << 4); mn = (s[j + 4] >> 4) | ((s[j] >> 6) << 4); }
 }
-__device__ __forceinline__ float deq_elem(int fmt, const uint8_t *row, int cols, int c) {
-  if (fmt == LLB_FM_F32) return ((const float *)row)[c];
+__device__ __forceinline__ float deq_elem(int fmt, const uint8_t *W, int cols, int row, int c) {
+  if (fmt == LLB_FM_F32) return ((const float *)W)[(size_t)row * cols + c];
+  const int r = row & 15, i = c & 255;
+  const uint8_t *tile = W + ((size_t)(row >> 4) * ((cols + 255) >> 8) + (c >> 8)) * tile_bytes(fmt), *blk = tile + r * tile_row(fmt);
   if (fmt == LLB_FM_Q8_0) {
-    float d = h2f_bits(((const unsigned short *)(row + cols))[c >> 5]);
-    return __fmul_rn((float)((const int8_t *)row)[c], d);
+    float d = h2f_bits(((const unsigned short *)(blk + 256))[i >> 5]);
+    return __fmul_rn((float)((int)blk[i] - 128), d);
   }
-  int b = c >> 8, i = c & 255;
   if (fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K) {
-    const uint8_t *blk = row + (size_t)b * (fmt == LLB_FM_Q4_K ? 144 : 176);
     float d = h2f_bits(blk[0] | (blk[1] << 8)), dm = h2f_bits(blk[2] | (blk[3] << 8));
     int g = i >> 6, hi = (i >> 5) & 1, l = i & 31, sc, mn;
     q4k_scale_min(blk + 4, 2 * g + hi, sc, mn);
@@ -234,12 +244,11 @@ __device__ __forceinline__ float deq_elem(int fmt, const uint8_t *row, int cols,
     return __fsub_rn(__fmul_rn(__fmul_rn(d, (float)sc), (float)q), __fmul_rn(dm, (float)mn));
   }
   if (fmt == LLB_FM_Q6_K) {
-    const uint8_t *blk = row + (size_t)b * 224;
     int hf = i >> 7, qd = (i >> 5) & 3, l = i & 31;
     uint8_t lq = blk[64 * hf + 32 * (qd & 1) + l];
     int nib = qd < 2 ? (lq & 15) : (lq >> 4);
     int code = (nib | (((blk[128 + 32 * hf + l] >> (2 * qd)) & 3) << 4)) - 32;
-    float d = h2f_bits(blk[208] | (blk[209] << 8));
+    float d = h2f_bits(((const unsigned short *)(tile + 3328))[r]);
     float sc = (float)((const int8_t *)(blk + 192))[8 * hf + 2 * qd + (l >> 4)];
     return __fmul_rn(__fmul_rn(d, sc), (float)code);
   }

@@ -321,7 +321,7 @@ static int load_tensor(llb_spec *m, const TensorRec &t, const uint8_t *pack, siz
   if (!in_range(t.off, t.bytes, src_bytes)) return llb_fail("index: tensor at %llu (%llu bytes) reaches past the end of its source (%zu bytes)",
                                                              (unsigned long long)t.off, (unsigned long long)t.bytes, src_bytes);
   bool fresh;
-  void *dst = walloc(m, (size_t)t.rows * dev_row_bytes(t.fmt, t.cols), &fresh);
+  void *dst = walloc(m, dev_bytes(t.fmt, t.rows, t.cols), &fresh);
   if (!dst) return -1;
   if (!fresh) { dedupe[t.off] = dst; *out = dst; return 0; }
   if (t.blocked) {
@@ -337,7 +337,7 @@ static int load_tensor(llb_spec *m, const TensorRec &t, const uint8_t *pack, siz
         uint8_t *q = tmp.data() + (size_t)r * rb, *sc = q + t.cols;
         for (size_t b = 0; b < nb; b++) { memcpy(sc + 2 * b, src + 34 * b, 2); memcpy(q + 32 * b, src + 34 * b + 2, 32); }
       }
-      CK(llb_b200_weight_upload(t.fmt, nr, t.cols, tmp.data(), 0, (llb_b200_dptr)(uintptr_t)((uint8_t *)dst + (size_t)r0 * dev_row_bytes(t.fmt, t.cols))));
+      CK(llb_b200_weight_upload(t.fmt, nr, t.cols, tmp.data(), 0, (llb_b200_dptr)(uintptr_t)((uint8_t *)dst + dev_bytes(t.fmt, r0, t.cols))));
     }
     dedupe[t.off] = dst;
     *out = dst;
@@ -363,9 +363,8 @@ static int load_sliced(llb_spec *m, const TensorRec &t, const uint8_t *pack, siz
   if (!rows) rows = &allr;
   if (!cols) cols = &allc;
   const int lr = rows->total(), lc = cols->total();
-  const size_t frb = dev_row_bytes(t.fmt, t.cols), lrb = dev_row_bytes(t.fmt, lc);
   int rc = 0;
-  uint8_t *dst = (uint8_t *)dalloc(m, (size_t)lr * lrb);
+  uint8_t *dst = (uint8_t *)dalloc(m, dev_bytes(t.fmt, lr, lc));
   if (!dst) rc = -1;
   const int unit = t.fmt == LLB_FM_F32 ? 1 : t.fmt == LLB_FM_Q8_0 ? 32 : 256;
   int drow = 0;
@@ -374,17 +373,13 @@ static int load_sliced(llb_spec *m, const TensorRec &t, const uint8_t *pack, siz
     for (int j = 0; j < cols->n && !rc; j++) {
       const int c0 = cols->start[j], cn = cols->count[j];
       if (c0 % unit || cn % unit) { rc = llb_fail("tensor slice: columns %d + %d are not whole blocks", c0, cn); break; }
-      const uint8_t *src = (const uint8_t *)full + (size_t)rows->start[i] * frb;
-      cudaError_t e;
-      if (t.fmt == LLB_FM_Q8_0) {   // [cols x int8][cols / 32 x f16]: the codes and the scales are two column ranges
-        e = cudaMemcpy2DAsync(dst + (size_t)drow * lrb + dcol, lrb, src + c0, frb, cn, rows->count[i], cudaMemcpyDeviceToDevice, g_llb.stream);
-        if (e == cudaSuccess)
-          e = cudaMemcpy2DAsync(dst + (size_t)drow * lrb + lc + dcol / 16, lrb, src + t.cols + c0 / 16, frb, cn / 16, rows->count[i], cudaMemcpyDeviceToDevice, g_llb.stream);
+      if (t.fmt == LLB_FM_F32) {
+        const cudaError_t e = cudaMemcpy2DAsync(dst + ((size_t)drow * lc + dcol) * 4, (size_t)lc * 4, (const uint8_t *)full + ((size_t)rows->start[i] * t.cols + c0) * 4,
+                                                (size_t)t.cols * 4, (size_t)cn * 4, rows->count[i], cudaMemcpyDeviceToDevice, g_llb.stream);
+        if (e != cudaSuccess) rc = llb_fail("tensor slice: %s", cudaGetErrorString(e));
       } else {
-        e = cudaMemcpy2DAsync(dst + (size_t)drow * lrb + dev_row_bytes(t.fmt, dcol), lrb, src + dev_row_bytes(t.fmt, c0), frb, dev_row_bytes(t.fmt, cn),
-                              rows->count[i], cudaMemcpyDeviceToDevice, g_llb.stream);
+        rc = ops_tile_slice(g_llb.stream, t.fmt, (const uint8_t *)full, t.cols, dst, lc, rows->start[i], drow, rows->count[i], c0, dcol, cn);
       }
-      if (e != cudaSuccess) rc = llb_fail("tensor slice: %s", cudaGetErrorString(e));
       dcol += cn;
     }
     drow += rows->count[i];
@@ -437,9 +432,8 @@ static int load_moe(llb_spec *m, FfnW &w, const std::string &p, const std::unord
   bool fresh;
   w.router = (float *)walloc(m, (size_t)(ne + 1) * d * 4, &fresh);
   if (!w.router) return -1;
-  const size_t rb_gu0 = dev_row_bytes(eg.fmt, d), rb_dn0 = dev_row_bytes(ed.fmt, ef);
   if (!fresh) {
-    w.es_gu = (long long)(2 * ef * rb_gu0); w.es_dn = (long long)(d * rb_dn0);
+    w.es_gu = (long long)dev_bytes(eg.fmt, 2 * ef, d); w.es_dn = (long long)dev_bytes(ed.fmt, d, ef);
     w.gu = (uint8_t *)walloc(m, (size_t)(ne + 1) * w.es_gu, &fresh);
     w.dn = (uint8_t *)walloc(m, (size_t)(ne + 1) * w.es_dn, &fresh);
     return w.gu && w.dn ? 0 : -1;
@@ -447,9 +441,8 @@ static int load_moe(llb_spec *m, FfnW &w, const std::string &p, const std::unord
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   CU_OK(cudaMemcpyAsync(w.router, pack + r_in.off, (size_t)ne * d * 4, kind, g_llb.stream));
   CU_OK(cudaMemcpyAsync(w.router + (size_t)ne * d, pack + r_sh.off, (size_t)d * 4, kind, g_llb.stream));
-  const size_t rb_gu = dev_row_bytes(eg.fmt, d), rb_dn = dev_row_bytes(ed.fmt, ef);
   const size_t pb_gu = pack_row_bytes(eg.fmt, d), pb_dn = pack_row_bytes(ed.fmt, ef);
-  w.es_gu = (long long)(2 * ef * rb_gu); w.es_dn = (long long)(d * rb_dn);
+  w.es_gu = (long long)dev_bytes(eg.fmt, 2 * ef, d); w.es_dn = (long long)dev_bytes(ed.fmt, d, ef);
   w.gu = (uint8_t *)walloc(m, (size_t)(ne + 1) * w.es_gu, &fresh);
   w.dn = (uint8_t *)walloc(m, (size_t)(ne + 1) * w.es_dn, &fresh);
   if (!w.gu || !w.dn) return -1;
@@ -458,7 +451,7 @@ static int load_moe(llb_spec *m, FfnW &w, const std::string &p, const std::unord
     const uint8_t *u = e < ne ? pack + eu.off + (size_t)e * gu_stride * pb_gu : pack + su.off;
     const uint8_t *dn = e < ne ? pack + ed.off + (size_t)e * d * pb_dn : pack + sd.off;
     CK(llb_b200_weight_upload(eg.fmt, ef, d, g, on_device, (llb_b200_dptr)(uintptr_t)(w.gu + (size_t)e * w.es_gu)));
-    CK(llb_b200_weight_upload(eg.fmt, ef, d, u, on_device, (llb_b200_dptr)(uintptr_t)(w.gu + (size_t)e * w.es_gu + (size_t)ef * rb_gu)));
+    CK(llb_b200_weight_upload(eg.fmt, ef, d, u, on_device, (llb_b200_dptr)(uintptr_t)(w.gu + (size_t)e * w.es_gu + dev_bytes(eg.fmt, ef, d))));
     CK(llb_b200_weight_upload(ed.fmt, d, ef, dn, on_device, (llb_b200_dptr)(uintptr_t)(w.dn + (size_t)e * w.es_dn)));
   }
   return 0;
@@ -588,8 +581,7 @@ static int enq_moe_core(llb_spec *m, const FfnW &w, const RowSet *rs) {
   PK("moe gate|up", gemm_launch_moe(s, w.fmt_gu, false, m->xp_d, a, &one, nullptr));
   const bool silu_in_down = m->NC == 8;
   if (!silu_in_down) PK("moe silu", op_silu_scaled_xp(s, PartIn{m->moe_g, 1, 0}, PartIn{m->moe_u, 1, 0}, fe, m->xp_e, rs, m->Tmax, m->moe_wt, m->ef));
-  const bool sel = m->NC >= 32;
-  int ks = gemm_fix_ksplit(w.fmt_dn, m->NC, fe / 256, gemm_pick_ksplit(w.fmt_dn, m->NC, m->Tmax * (m->d / 16), fe / 256, g_llb.sms, sel), sel);
+  int ks = gemm_fix_ksplit(w.fmt_dn, m->NC, fe / 256, gemm_pick_ksplit(w.fmt_dn, m->NC, m->Tmax * (m->d / 16), fe / 256, g_llb.sms));
   CK(out_prepare(m, m->b_dn, m->d, ks));
   a.W = w.dn; a.es = w.es_dn; a.out = m->b_dn.p; a.split_stride = m->b_dn.stride;
   PK("moe down", gemm_launch_moe(s, w.fmt_dn, true, m->xp_e, a, &ks, silu_in_down ? m->moe_wt : nullptr));

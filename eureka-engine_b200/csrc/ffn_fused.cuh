@@ -48,18 +48,14 @@ template <int FMT> __device__ __forceinline__ void ffn_store4(uint8_t *xh_s, uin
   }
   {
     const __half2 a = __halves2half2(hi[0], hi[2]), b = __halves2half2(hi[1], hi[3]);
-    *(uint2 *)(xh_s + (size_t)t * CS + (size_t)c * 2) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
+    const int o = g2_xpos<FMT, 1>(c >> 3) + (c & 4) * 2;
+    *(uint2 *)(xh_s + (size_t)t * CS + o) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
     const __half2 e = __halves2half2(lo[0], lo[2]), f = __halves2half2(lo[1], lo[3]);
-    *(uint2 *)(xh_s + (size_t)(NH + t) * CS + (size_t)c * 2) = make_uint2(*(const uint32_t *)&e, *(const uint32_t *)&f);
+    *(uint2 *)(xh_s + (size_t)(NH + t) * CS + o) = make_uint2(*(const uint32_t *)&e, *(const uint32_t *)&f);
   }
-  hs += __shfl_xor_sync(0xffffffffu, hs, 1); ls += __shfl_xor_sync(0xffffffffu, ls, 1);
-  hs += __shfl_xor_sync(0xffffffffu, hs, 2); ls += __shfl_xor_sync(0xffffffffu, ls, 2);   // 16 columns
-  if constexpr (FMT == LLB_FM_Q6_K) {
-    if ((lane & 3) == 0) {   // f32 sums of 16 columns: [16-column group][NC]
-      float *x16 = (float *)xsf_s + (size_t)(c >> 4) * NC;
-      x16[t] = hs; x16[NH + t] = ls;
-    }
-  } else {
+  if constexpr (g2_aux(FMT) != 0) {
+    hs += __shfl_xor_sync(0xffffffffu, hs, 1); ls += __shfl_xor_sync(0xffffffffu, ls, 1);
+    hs += __shfl_xor_sync(0xffffffffu, hs, 2); ls += __shfl_xor_sync(0xffffffffu, ls, 2);
     const float h32 = hs + __shfl_xor_sync(0xffffffffu, hs, 4), l32 = ls + __shfl_xor_sync(0xffffffffu, ls, 4);
     if ((lane & 7) == 0) {   // 32-column means as fp16 hi / rest, in the order the min-term MMA's B fragment reads them
       const int sb = c >> 8, b = (c >> 5) & 7;
@@ -111,11 +107,14 @@ template <int FMT> struct FfnStageSilu {
 };
 
 template <int FMT2>
-__global__ void __launch_bounds__(512, 1) k_ffn(const GemmArgs a1, const GemmArgs a2, const int cps1, const int cps2, unsigned int *sync,
-                                                unsigned int *err) {
+__global__ void __launch_bounds__(G2_MAXWARPS * 32, 1) k_ffn(const GemmArgs a1, const GemmArgs a2, const int cps1, const int cps2, unsigned int *sync,
+                                                       unsigned int *err) {
   extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int RB1 = g2_ring_bytes(LLB_FM_Q4_K, 8), RB2 = g2_ring_bytes(FMT2, 8), RB = RB1 > RB2 ? RB1 : RB2;
   pdl_trigger();
-  g2_phase<LLB_FM_Q4_K, 1>(a1, cps1, (int)blockIdx.x, smem, G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K>{a1});
-  __syncthreads();   // the CTA is done with the first launch's shared memory
-  g2_phase<FMT2, 1>(a2, cps2, (int)blockIdx.x, smem, FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err}, G2MatsPlain<FMT2>{a2});
+  G2Ring rg = g2_ring_init(smem, RB / G2_MAXWARPS);
+  g2_phase<LLB_FM_Q4_K, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K, 1>{a1});
+  __syncthreads();   // the CTA is done with the first launch's planes
+  g2_phase<FMT2, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err},
+                    G2MatsPlain<FMT2, 1>{a2});
 }

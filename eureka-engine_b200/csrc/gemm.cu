@@ -5,29 +5,20 @@
 #include "moe.cuh"
 #include "host.cuh"
 
-static int g2_max_sb(int fmt, int NC, bool sel = false) {
-  return fmt == LLB_FM_Q4_K ? g2_max_slice_sb<LLB_FM_Q4_K>(NC, sel) : fmt == LLB_FM_Q5_K ? g2_max_slice_sb<LLB_FM_Q5_K>(NC, sel)
-       : fmt == LLB_FM_Q8_0 ? g2_max_slice_sb<LLB_FM_Q8_0>(NC, sel) : g2_max_slice_sb<LLB_FM_Q6_K>(NC, sel);
-}
 // the tcgen05 kernel takes Q4_K with T <= 4 (8 plane columns)
 static bool is_g3(int fmt, int NC) { return g_llb.gemm3 && fmt == LLB_FM_Q4_K && NC == 8; }
 static unsigned int *g_ffn_sync = nullptr;   // the fused FFN's grid barrier: two counters
-static unsigned int *g_g3_err = nullptr;   // device word: set when a bounded wait of k_gemm3 ran out
-static int g2_warps_of(int fmt, int NC, bool sel = false) {
-  return fmt == LLB_FM_Q6_K ? g2_warps<LLB_FM_Q6_K>(NC, sel) : fmt == LLB_FM_Q8_0 ? g2_warps<LLB_FM_Q8_0>(NC, sel)
-       : fmt == LLB_FM_Q5_K ? g2_warps<LLB_FM_Q5_K>(NC, sel) : g2_warps<LLB_FM_Q4_K>(NC, sel);
-}
-
+static unsigned int *g_g3_err = nullptr;   // device word: set when a bounded wait of a kernel ran out
+unsigned int *gemm_err_word(void) { return g_g3_err; }
 template <int FMT, int NT> static int launch_two(cudaStream_t s, const GemmArgs &a) {
   const int NC = 8 * NT, nsl = (a.nsb + a.ksplit - 1) / a.ksplit;
-  int cps = g_llb.sms * G2_CPSM / a.ksplit;
+  int cps = g_llb.sms / a.ksplit;
   if (cps < 1) cps = 1;
   // every SM takes part as long as there is a tile for it: the tiles are dealt out one per CTA in turn
-  constexpr int G2_WARPS = g2_warps<FMT>(8 * NT);
   if (cps > a.tile0[a.nmat]) cps = a.tile0[a.nmat];
-  const size_t smem = (size_t)g2_xp_bytes<FMT>(nsl, NC) + g2_ring_bytes<FMT>(NC);
+  const size_t smem = g2_smem(FMT, nsl, NC);
   if (smem > G2_SMEM_MAX) return llb_fail("k_gemm2: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
-  cudaError_t e = llb_launch(k_gemm2<FMT, NT>, dim3(cps * a.ksplit), dim3(G2_WARPS * 32), smem, s, a, cps);
+  cudaError_t e = llb_launch(k_gemm2<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
   if (e != cudaSuccess) return llb_fail("k_gemm2 launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -124,15 +115,14 @@ int gemm_setup(void) {
   return 0;
 }
 
-// sel: a routed-expert launch (its own warp count and ring depth at 32 plane columns)
-int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool sel) {
+int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks) {
   if (ks < 1) ks = 1;
-  if (!sel && is_g3(fmt, NC)) {
+  if (is_g3(fmt, NC)) {
     const int mx = g3_max_slice_sb();
     const int lo = (nsb + mx - 1) / mx;
     if (ks < lo) ks = lo;
   } else {
-    const int mx = g2_max_sb(fmt, NC, sel);
+    const int mx = g2_max_slice_sb(fmt, NC);
     const int lo = (nsb + mx - 1) / mx;       // the activation slice of a CTA has to fit in shared memory
     if (ks < lo) ks = lo;
   }
@@ -141,31 +131,32 @@ int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool sel) {
   return ks;
 }
 
-// K-slices per row tile: the longest chain of work of any warp (tiles per warp x super-blocks per
-// slice), with a small charge per slice for the partial sums the consumer has to add.
-int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool sel) {
+// K-slices per row tile.  In cycles of one SM: the work of its tiles (about 45 + 6.3 cycles a plane column and tile, measured
+// with the copies left out on the 27B shape's gate|up launch at 4, 8 and 16 rows), or, where a warp's own chain is longer
+// (a tile takes a warp by itself about 900 cycles), that; then the staging of the slice at 32 bytes a cycle; and
+// a charge per slice for the partial sums that the consumer has to add.
+double gemm_split_cost(int NC, int warps, int ntiles, int nsb, int ks, int sms) {
+  const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps, rounds = (tiles + warps - 1) / warps;
+  const double work = (double)tiles * slice * (45.0 + 6.3 * NC), chain = (double)rounds * slice * 900.0;
+  return ((work > chain ? work : chain) + 16.0 * NC * slice) * (1.0 + 0.025 * (ks - 1));
+}
+int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms) {
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
-    if (gemm_fix_ksplit(fmt, NC, nsb, ks, sel) != ks) continue;
-    long long rounds;
-    if (!sel && is_g3(fmt, NC)) {
+    if (gemm_fix_ksplit(fmt, NC, nsb, ks) != ks) continue;
+    const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks;
+    double cost;
+    if (is_g3(fmt, NC)) {
       // 128-row tiles, one CTA per (tile, slice) at a time; 1.5 super-blocks of pipeline fill per tile
-      const int cps = sms / ks > 0 ? sms / ks : 1, nt128 = (ntiles + 7) / 8;
-      rounds = (nt128 + cps - 1) / cps;
-      const int slice = (nsb + ks - 1) / ks;
-      const double cost = (double)rounds * (slice + 1.5) * (1.0 + 0.02 * (ks - 1));
-      if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
-      continue;
+      const int nt128 = (ntiles + 7) / 8;
+      cost = (double)((nt128 + cps - 1) / cps) * (slice + 1.5) * (1.0 + 0.02 * (ks - 1));
     } else {
-      const int cps = sms * G2_CPSM / ks > 0 ? sms * G2_CPSM / ks : 1;
-      rounds = (ntiles + (long long)cps * g2_warps_of(fmt, NC, sel) - 1) / ((long long)cps * g2_warps_of(fmt, NC, sel));
+      cost = gemm_split_cost(NC, g2_warps(fmt, NC), ntiles, nsb, ks, sms);
     }
-    const int slice = (nsb + ks - 1) / ks;
-    const double cost = (double)rounds * slice * (1.0 + 0.02 * (ks - 1));
     if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
   }
-  return gemm_fix_ksplit(fmt, NC, nsb, best, sel);
+  return gemm_fix_ksplit(fmt, NC, nsb, best);
 }
 
 // One K-split for a launch whose partial sums outlive the pass (attn_qkv into the conv ring): valid at both
@@ -188,6 +179,7 @@ static int gemm_prepare(int fmt, GemmArgs &a) {
   if (a.K % 256) return llb_fail("gemm: K %d is not a multiple of 256", a.K);
   if (a.xp.NC != 8 && a.xp.NC != 16 && a.xp.NC != 32) return llb_fail("gemm: NC %d", a.xp.NC);
   if (a.xp.K != a.K) return llb_fail("gemm: planes hold %d columns, K is %d", a.xp.K, a.K);
+  a.err = g_g3_err;
   a.nsb = a.K / 256;
   a.tile0[0] = 0;
   for (int i = 0; i < a.nmat; i++) a.tile0[i + 1] = a.tile0[i] + (a.m[i].rows + 15) / 16;
@@ -204,10 +196,9 @@ template <int FMT2> static int launch_ffn(cudaStream_t s, const GemmArgs &a1, co
   if (cps2 > a2.tile0[a2.nmat]) cps2 = a2.tile0[a2.nmat];
   const int grid = cps1 > cps2 * a2.ksplit ? cps1 : cps2 * a2.ksplit;
   if (grid > g_llb.sms) return llb_fail("k_ffn: %d CTAs do not fit %d SMs", grid, g_llb.sms);   // the barrier needs them all resident
-  const size_t s1 = (size_t)g2_xp_bytes<LLB_FM_Q4_K>(a1.nsb, 8) + 16 * G2_STAGES * 16 * G2Traits<LLB_FM_Q4_K>::RS;
   const int nsl2 = (a2.nsb + a2.ksplit - 1) / a2.ksplit;
-  const size_t s2 = (size_t)g2_xp_bytes<FMT2>(nsl2, 8) + 16 * G2_STAGES * 16 * G2Traits<FMT2>::RS;
-  const size_t smem = s1 > s2 ? s1 : s2;
+  const int rb1 = g2_ring_bytes(LLB_FM_Q4_K, 8), rb2 = g2_ring_bytes(FMT2, 8), rb = rb1 > rb2 ? rb1 : rb2;
+  const size_t s1 = g2_smem(LLB_FM_Q4_K, a1.nsb, 8) - rb1 + rb, s2 = g2_smem(FMT2, nsl2, 8) - rb2 + rb, smem = s1 > s2 ? s1 : s2;
   if (smem > G2_SMEM_MAX) return llb_fail("k_ffn: %zu bytes of shared memory", smem);
   cudaError_t e = llb_launch(k_ffn<FMT2>, dim3(grid), dim3(512), smem, s, a1, a2, cps1, cps2, g_ffn_sync, g_g3_err);
   if (e != cudaSuccess) return llb_fail("k_ffn launch: %s", cudaGetErrorString(e));
@@ -217,7 +208,7 @@ template <int FMT2> static int launch_ffn(cudaStream_t s, const GemmArgs &a1, co
 bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d) {
   return g_llb.ffn_fused && g_ffn_sync && NC == 8 && fmt_gu == LLB_FM_Q4_K &&
          (fmt_dn == LLB_FM_Q4_K || fmt_dn == LLB_FM_Q5_K || fmt_dn == LLB_FM_Q6_K) && d % 256 == 0 &&
-         d / 256 <= g2_max_slice_sb<LLB_FM_Q4_K>(8);
+         d / 256 <= g2_max_slice_sb(LLB_FM_Q6_K, 8)   /* the widest ring of the two launches */;
 }
 // a1: gate and up (two matrices, Q4_K, ksplit 1, outputs complete); a2: down in format fmt2 with its own K-split
 int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2) {
@@ -233,19 +224,18 @@ int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2) {
 // ---- the routed experts' GEMMs (moe.cuh) ---------------------------------------------------------
 template <int FMT, int NT> static int launch_moe(cudaStream_t s, bool down, const GemmArgs &a, const MoeArgs &m, int ntiles, const float *wt_silu) {
   const int NC = 8 * NT, nsl = (a.nsb + a.ksplit - 1) / a.ksplit;
-  int cps = g_llb.sms * G2_CPSM / a.ksplit;
+  int cps = g_llb.sms / a.ksplit;
   if (cps < 1) cps = 1;
   if (cps > ntiles) cps = ntiles;
-  constexpr bool sel = moe_ntc<NT>() != NT;
-  const size_t smem = (size_t)g2_xp_bytes<FMT>(nsl, NC) + g2_ring_bytes<FMT>(NC, sel);
+  const size_t smem = g2_smem(FMT, nsl, NC);
   if (smem > G2_SMEM_MAX) return llb_fail("moe gemm: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   cudaError_t e;
   if (down && wt_silu) {
-    if constexpr (NT == 1) e = llb_launch(k_moe_dn_silu<FMT>, dim3(cps * a.ksplit), dim3(G2Traits<FMT>::WARPS * 32), smem, s, a, m, wt_silu, cps);
+    if constexpr (NT == 1) e = llb_launch(k_moe_dn_silu<FMT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, wt_silu, cps);
     else return llb_fail("moe gemm: the down launch builds its own activations for T <= 4 only");
   } else {
-    e = down ? llb_launch(k_moe_dn<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps<FMT>(NC, sel) * 32), smem, s, a, m, cps)
-             : llb_launch(k_moe_gu<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps<FMT>(NC, sel) * 32), smem, s, a, m, cps);
+    e = down ? llb_launch(k_moe_dn<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps)
+             : llb_launch(k_moe_gu<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps);
   }
   if (e != cudaSuccess) return llb_fail("moe gemm launch: %s", cudaGetErrorString(e));
   return 0;
@@ -260,12 +250,11 @@ int gemm_launch_moe(cudaStream_t s, int fmt, bool down, const XPlanes &xp, MoeAr
   memset(&a, 0, sizeof a);
   a.K = down ? m.nslot * m.ef : m.d;
   if (xp.K != a.K || (xp.NC != 8 && xp.NC != 16 && xp.NC != 32)) return llb_fail("moe gemm: planes of %d x %d columns, K is %d", xp.K, xp.NC, a.K);
-  a.nsb = a.K / 256; a.xp = xp; a.planes = 2; a.T = m.T; a.nmat = 0;
+  a.err = g_g3_err; a.nsb = a.K / 256; a.xp = xp; a.planes = 2; a.T = m.T; a.nmat = 0;
   const int ntiles = down ? m.T * (m.d / 16) : m.T * m.nslot * (m.ef / 8);
   int ks = 1;
-  const bool sel = xp.NC >= 32;
-  if (down) ks = *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, xp.NC, ntiles, a.nsb, g_llb.sms, sel);
-  ks = gemm_fix_ksplit(fmt, xp.NC, a.nsb, ks, sel);
+  if (down) ks = *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, xp.NC, ntiles, a.nsb, g_llb.sms);
+  ks = gemm_fix_ksplit(fmt, xp.NC, a.nsb, ks);
   if (!down && ks != 1) return llb_fail("moe gemm: %d columns do not fit one K-slice", a.K);
   a.ksplit = ks;
   if (ksplit) *ksplit = ks;

@@ -23,7 +23,7 @@
 #define GEMM_MAXSPLIT 16
 
 struct GemmMat {
-  const uint8_t *W;   // device layout, row stride dev_row_bytes(fmt, K)
+  const uint8_t *W;   // device layout (common.cuh)
   float *out;         // [ksplit][T][ostride] partial sums (row index within this matrix)
   int rows;
   int ostride;        // floats between consecutive tokens of one partial
@@ -50,6 +50,7 @@ struct GemmArgs {
   XPlanes xp;
   int planes;                  // 2: hi/lo columns are folded into T = NC/2 tokens; 1: NC independent tokens
   int T;                       // tokens actually written
+  unsigned int *err;           // device word set when a bounded wait runs out
 };
 
 // a routed-expert launch (moe.cuh)
@@ -61,7 +62,8 @@ struct MoeArgs {
   int ne;               // block ne is the shared expert; ids are clamped to 0..ne
   int ef, d, T;
   const int *n_rows;    // rows of the pass in flight (<= T); tiles of later rows are not computed
-  float *g, *u;         // k_moe_gu: [T][nslot * ef]
+  float *g, *u;         // gate|up: [K-slice][T][nslot * ef]
+  long long gu_stride;  // floats between their K-slices (one slice: any)
   float *out;           // k_moe_dn: [ksplit][T][d]
   long long split_stride;
 };
@@ -95,10 +97,10 @@ __device__ __forceinline__ uint32_t g2_hfma2(uint32_t a, uint32_t b, uint32_t c)
 }
 
 // ---- epilogue of one (row tile, K-slice) unit ---------------------------------------------------
-// Folds the planes and writes the unit's partial sums; the consumer adds the K-slices in index order.
+// row: the lane's first row of the matrix (its second one is 8 further on).  Folds the planes and writes the unit's partial sums; the consumer adds the K-slices in index order.
 template <int NT>
-__device__ __forceinline__ void gemm_epilogue(const GemmArgs &a, const GemmMat &M, int ks, int tile, int row0, float (&acc)[NT][4], int lane) {
-  const int gid = lane >> 2, j = lane & 3;
+__device__ __forceinline__ void gemm_epilogue(const GemmArgs &a, const GemmMat &M, int ks, int row, float (&acc)[NT][4], int lane) {
+  const int j = lane & 3;
   float val[NT][4];
   size_t idx[NT][4];
   bool on[NT][4];
@@ -112,7 +114,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs &a, const GemmMat &
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const float lo = __shfl_xor_sync(0xffffffffu, acc[0][i], 2);
-        const int t = 2 * j + (i & 1), r = row0 + gid + ((i >> 1) << 3);
+        const int t = 2 * j + (i & 1), r = row + ((i >> 1) << 3);
         on[0][i] = j < 2 && t < a.T && r < M.rows;
         if (on[0][i]) { idx[0][i] = (size_t)gemm_out_block(M, t) * M.ostride + r; val[0][i] = acc[0][i] + lo * XP_LO_INV; }
       }
@@ -122,7 +124,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs &a, const GemmMat &
       for (int nt = 0; nt < NT / 2; nt++)
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          const int t = nt * 8 + 2 * j + (i & 1), r = row0 + gid + ((i >> 1) << 3);
+          const int t = nt * 8 + 2 * j + (i & 1), r = row + ((i >> 1) << 3);
           on[nt][i] = t < a.T && r < M.rows;
           if (on[nt][i]) { idx[nt][i] = (size_t)gemm_out_block(M, t) * M.ostride + r; val[nt][i] = acc[nt][i] + acc[nt + NT / 2][i] * XP_LO_INV; }
         }
@@ -132,7 +134,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs &a, const GemmMat &
     for (int nt = 0; nt < NT; nt++)
 #pragma unroll
       for (int i = 0; i < 4; i++) {
-        const int t = nt * 8 + 2 * j + (i & 1), r = row0 + gid + ((i >> 1) << 3);
+        const int t = nt * 8 + 2 * j + (i & 1), r = row + ((i >> 1) << 3);
         on[nt][i] = t < a.T && r < M.rows;
         if (on[nt][i]) { idx[nt][i] = (size_t)gemm_out_block(M, t) * M.ostride + r; val[nt][i] = acc[nt][i]; }
       }

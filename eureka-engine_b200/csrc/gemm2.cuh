@@ -1,70 +1,61 @@
-// gemm2.cuh -- second-generation skinny GEMM for the 4/5-bit K-quants (Q4_K, Q5_K), the formats that
-// carry most of a Q4_K_M model's bytes.  Same arithmetic as gemm.cuh (integer codes as fp16
-// subnormals into mma.m16n8k16, scales applied to fp32 partial sums); what changes is everything
-// around the MMAs, driven by the first kernel's profile (issue-bound at 670 instructions per
-// 16-row x 256-column tile-super-block, activation loads waiting on L1/L2):
+// gemm2.cuh -- the skinny GEMM: Y[t][r] = sum_c W[r][c] x[t][c], T <= 16 rows against Q4_K / Q5_K / Q6_K / Q8_0 weights.
+// Integer codes go to the tensor cores as fp16 numbers (mma.m16n8k16, fp32 sums); scales never round a weight.
 //
 //  * a CTA owns ONE K-slice and stages that slice of the activation planes in shared memory once;
-//    all B-fragment reads are then conflict-free LDS.128 (column stride = 64 mod 128 bytes);
-//  * 16 warps per SM, one-super-block stages, three-deep private cp.async rings
-//    (row stride 160 / 224 bytes = 32 / 96 mod 128: conflict-free 8-byte A-fragment reads);
-//  * the copy issue loop has no division and no per-piece address arithmetic beyond one add;
-//  * the Q4_K "min" term  dmin * sum_b m_b * sum(x in sub-block b)  is ONE extra MMA per
-//    tile-super-block: A = the eight 6-bit mins as fp16 numbers (m against the means' hi halves,
-//    m / 2048 against their lo halves), B = the sub-block activation means as fp16 hi/lo pairs
-//    prepared with the planes;
-//  * first MMAs of a sub-block take a zero C operand instead of zeroing registers.
+//  * a warp's piece of work is one tile of 16 rows x 256 columns (common.cuh), which one bulk copy brings into the warp's
+//    private ring of two or three stages (an mbarrier a stage, no copy instructions in the other lanes).  Per-lane
+//    16-byte copies took 30 of the loop's 397 instructions, most of them integer adds;
+//  * Q4_K / Q5_K, up to 8 rows: a code in the low bits of an fp16 lane is the subnormal code * 2^-24, so two MMAs sum
+//    code * x of a 32-column sub-block exactly; the six-bit scale multiplies that fp32 sum, d the super-block's;
+//  * Q4_K / Q5_K, 16 rows (four n-tiles): the scale is multiplied into the codes instead, since sc * q <= 63 * 31 = 1953 is an
+//    exact fp16 integer: one HMUL2 a fragment register, shared by the n-tiles, and the MMAs of a whole super-block accumulate
+//    into one fragment.  Lane j of a row's four lanes then holds the k indices of column group j (64 columns, two
+//    sub-blocks) and needs that group's scales only.  gate|up of the 27B shape: 59 us against 64; with one n-tile the
+//    HMUL2s (half rate) cost more than the scales save, 31 us against 26;
+//  * the "min" term  dmin * sum_b m_b * sum(x in sub-block b)  is ONE extra MMA per tile: A = the eight mins as fp16 numbers
+//    (m against the means' hi halves, m / 2048 against their lo halves), B = the sub-block activation means;
+//  * Q6_K / Q8_0: a scale times a code does not fit fp16 exactly, so the scale multiplies the fp32 partial sum of its 16 or
+//    32 columns; the code's offset is taken off in fp16 (0x6400 | c is 1024 + c; one HADD2, exact).
 #pragma once
 #include "gemm.cuh"
+#include "tc5.cuh"
 
-#ifndef G2_STAGES
-#define G2_STAGES 3
-#endif
-// CTAs per SM.  With 2, two half-size CTAs (8 warps, at most half the shared memory) share an SM, so
-// that the CTAs of the next GEMM (programmatic dependent launch) can take the place of draining ones
-// and fill their weight rings early.  Measured on the 27B shape: the gate|up GEMM 30.4 us against
-// 27.9 us with one CTA, the verify pass 8.08 ms against 7.94 ms -- so the default stays 1.
-#ifndef G2_CPSM
-#define G2_CPSM 1
-#endif
-#define G2_SMEM_MAX ((233472 - 1024 * G2_CPSM) / G2_CPSM / 128 * 128)   // 228 KB per SM, 1 KB reserved per CTA
+#define G2_SMEM_MAX 226304   // 227 KB less the 6 KB that a phase may use beside the ring and the activation slice
+#define G2_MAXWARPS 16
+#define G2_BAR_BYTES 512     // one mbarrier per warp and stage (at most four)
 
-// SB bytes per super-block, RS ring row stride, P 16-byte pieces per row-super-block, WARPS per CTA,
-// XPAD: padding of a plane column in shared memory (column stride = 64 mod 128 bytes for the 16-byte
-// B reads of Q4_K/Q5_K, 32 mod 128 for the 8-byte ones of Q6_K), AUX: bytes per (super-block, column)
-// of the side array (Q4_K/Q5_K: 16 fp16 sub-block means; Q6_K: 16 f32 sums of 16 columns)
-template <int FMT> struct G2Traits;
-template <> struct G2Traits<LLB_FM_Q4_K> { enum { SB = 144, RS = 160, P = 9, QOFF = 16, WARPS = 16 / G2_CPSM, XPAD = 64, AUX = 32 }; };
-template <> struct G2Traits<LLB_FM_Q5_K> { enum { SB = 176, RS = 224, P = 11, QOFF = 48, WARPS = 16 / G2_CPSM, XPAD = 64, AUX = 32 }; };
-template <> struct G2Traits<LLB_FM_Q6_K> { enum { SB = 224, RS = 240, P = 14, QOFF = 0, WARPS = 16 / G2_CPSM, XPAD = 32, AUX = 64 }; };
-// Q8_0 rows are [K x int8][K/32 x f16]: a "super-block" here is 256 codes plus their 8 scales, which sit K - 256 sb + 16 sb
-// bytes further on in the row; piece 16 of a row-super-block is that scale piece (copy plan below).  AUX: 8 f32 sums of 32 columns.
-template <> struct G2Traits<LLB_FM_Q8_0> { enum { SB = 256, RS = 304, P = 17, QOFF = 0, WARPS = 8 / G2_CPSM, XPAD = 32, AUX = 32 }; };
+// XPAD: padding of a plane column in shared memory (column stride = 64 mod 128 bytes for the 16-byte B reads of Q4_K / Q5_K /
+// Q8_0, 32 mod 128 for the 8-byte ones of Q6_K), AUX: bytes per (super-block, column) of the sub-block means
+template <int FMT> struct G2Traits { enum { TB = tile_bytes(FMT), TR = tile_row(FMT), XPAD = FMT == LLB_FM_Q6_K ? 32 : 64,
+                                            AUX = FMT == LLB_FM_Q4_K || FMT == LLB_FM_Q5_K ? 32 : 0 }; };
+// Ring depth: 90 to 160 KB an SM in flight (44 KB cover HBM's latency at full rate), less beside 32 plane columns, whose whole
+// d = 2048 slice must fit.
+// Super-blocks a copy brings.  A bulk copy costs about 85 cycles of the SM's copy engine on top of its bytes (copies alone, no
+// arithmetic, gate|up of the 27B shape: 19.6 us at 2304 bytes, 11.8 us at 4608), so Q4_K takes two at a time.
+__host__ __device__ constexpr int g2_chunk(int fmt) { return fmt == LLB_FM_Q4_K ? 2 : 1; }
+__host__ __device__ constexpr int g2_stages(int fmt, int NC) { return fmt == LLB_FM_Q4_K ? (NC >= 32 ? 1 : 2) : NC >= 32 || fmt == LLB_FM_Q8_0 ? 2 : 3; }
+// Warps of a CTA: sixteen (128 registers a thread), fewer where the rings of sixteen would leave the activation slice less than
+// the widths in use need: Q8_0's tiles are twice the size, and 32 plane columns take half of the memory.
+__host__ __device__ constexpr int g2_warps(int fmt, int NC) {
+  return fmt == LLB_FM_Q8_0 ? 12 : NC < 32 ? 16 : fmt == LLB_FM_Q6_K ? 12 : 14;
+}
+__host__ __device__ constexpr int g2_ring_bytes(int fmt, int NC) { return g2_warps(fmt, NC) * g2_stages(fmt, NC) * g2_chunk(fmt) * tile_bytes(fmt); }
+__host__ __device__ constexpr int g2_aux(int fmt) { return fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K ? 32 : 0; }
+__host__ __device__ constexpr int g2_xpad(int fmt) { return fmt == LLB_FM_Q6_K ? 32 : 64; }
+// bytes of shared memory of a launch whose K-slices have nsl super-blocks, for NC activation columns
+__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC) {
+  return (size_t)G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC);
+}
+inline int g2_max_slice_sb(int fmt, int NC) {
+  const int left = G2_SMEM_MAX - G2_BAR_BYTES - g2_ring_bytes(fmt, NC) - NC * g2_xpad(fmt);
+  return left / (NC * (512 + g2_aux(fmt)));
+}
 
-// Warps of a CTA: the format's count, but eight at 32 plane columns (16 rows, four n-tiles).  Sixteen warps cap a thread
-// at 128 registers, and four n-tiles of accumulators, scale sums and min-term products do not fit in them: the 16-row
-// kernel spilled (40 bytes of stores, 120 of loads per thread and super-block) and spent its time waiting on local
-// memory (long-scoreboard stalls 1.3 per issue, 830 instructions per tile-super-block against 397 at 4 rows, tensor pipe
-// 34 % busy).  Eight warps get 255 registers and a ring half the size, which also leaves the activation slice more room.
-// sel: the routed-expert launches at 32 plane columns, which multiply a weight tile with two of the four staged n-tiles
-// (g2_phase's NTC = 2) and so need the registers of the two-n-tile kernel only: more warps (the eight-warp launch left its
-// schedulers two warps each and half their issue slots empty), two-deep rings so that the 32 staged columns of a whole
-// d = 2048 K-slice (139 KB) still fit beside them.
-template <int FMT> __host__ __device__ constexpr int g2_warps(int NC, bool sel = false) {
-  if (sel && NC >= 32 && G2_CPSM == 1) return FMT == LLB_FM_Q4_K ? 16 : FMT == LLB_FM_Q5_K ? 12 : 8;
-  return NC >= 32 && G2Traits<FMT>::WARPS > 8 ? 8 : G2Traits<FMT>::WARPS;
-}
-template <int FMT> __host__ __device__ constexpr int g2_stages(int NC, bool sel = false) { return sel && NC >= 32 && G2_CPSM == 1 ? 2 : G2_STAGES; }
-template <int FMT> __host__ __device__ constexpr int g2_ring_bytes(int NC, bool sel = false) {
-  return g2_warps<FMT>(NC, sel) * g2_stages<FMT>(NC, sel) * 16 * G2Traits<FMT>::RS;
-}
-// bytes of shared memory a K-slice of nsl super-blocks needs for NC activation columns
-template <int FMT> __host__ __device__ inline int g2_xp_bytes(int nsl, int NC) {
-  return NC * (nsl * 512 + G2Traits<FMT>::XPAD) + nsl * NC * G2Traits<FMT>::AUX;
-}
-template <int FMT> inline int g2_max_slice_sb(int NC, bool sel = false) {
-  int left = G2_SMEM_MAX - g2_ring_bytes<FMT>(NC, sel) - NC * G2Traits<FMT>::XPAD;
-  return left / (NC * 512 + NC * G2Traits<FMT>::AUX);
+// Where the 16-byte piece of columns c .. c+7 of a slice sits in a plane column (bytes).  Q4_K / Q5_K: lane j reads column group
+// j, so the pieces of the four groups that are read together lie side by side; the others keep their order.
+template <int FMT, int NT> __device__ __forceinline__ int g2_xpos(int piece) {
+  if constexpr ((FMT == LLB_FM_Q4_K || FMT == LLB_FM_Q5_K) && NT > 2) return ((piece & ~31) | ((piece & 7) << 2) | ((piece >> 3) & 3)) * 16;
+  else return piece * 16;
 }
 
 // D = A*B with a zero C operand
@@ -73,265 +64,177 @@ __device__ __forceinline__ void mma16816_z(float d[4], uint32_t a0, uint32_t a1,
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
+__device__ __forceinline__ uint32_t g2_hmul2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t g2_hadd2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar_s, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_s), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst_s, const void *src, uint32_t bytes, uint32_t bar_s) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_s), "l"(src), "r"(bytes), "r"(bar_s)
+               : "memory");
+}
 
-// One GEMM launch's work of a CTA (bid of cps * ksplit): fill the ring, call stage(xh_s, xsf_s, CS, sb0, nsl) --
-// which waits for whatever produces the activations, puts the CTA's slice of the planes and its side array into
-// shared memory and ends with a block-wide barrier --, then stream the CTA's tiles.  Warps beyond the format's
-// count and CTAs beyond the launch's only take part in the staging step's barriers.
-// Where a launch's row tiles live.  A policy says how many 16-row tiles there are, where tile i's rows and
-// the super-blocks of the CTA's K-slice start, and what to do with a finished tile.  G2MatsPlain is the
-// launch of up to four matrices that GemmArgs describes; the routed-expert launches (moe.cuh) find their
-// matrices through the expert ids an earlier kernel chose.
-//   EARLY   the weight addresses depend on no earlier kernel: the ring's prologue is issued before the wait
-//   Cur     per-thread cursor of the tile being copied
-//   locate  tile -> first row, row count, cursor;  src: row 0 of super-block (sb0 + c) of the slice
-template <int FMT> struct G2MatsPlain {
-  static constexpr bool EARLY = true;
-  const GemmArgs &a;
-  struct Cur { const uint8_t *W, *W0; };   // first code of the slice in row 0 of the matrix; the matrix itself
-  __device__ __forceinline__ int ntiles() const { return a.tile0[a.nmat]; }
-  __device__ __forceinline__ size_t row_bytes() const { return dev_row_bytes(FMT, a.K); }
-  __device__ __forceinline__ void locate(int tile, int sb0, Cur &c, int &row0, int &rows) const {
-    int m = 0;
-    while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
-    row0 = (tile - a.tile0[m]) * 16; rows = a.m[m].rows;
-    c.W0 = a.m[m].W;
-    c.W = c.W0 + (size_t)sb0 * G2Traits<FMT>::SB;
-  }
-  __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const { return c.W + (size_t)pc * G2Traits<FMT>::SB; }
-  template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
-    int m = 0;
-    while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
-    gemm_epilogue<NT>(a, a.m[m], ks, tile, (tile - a.tile0[m]) * 16, acc, lane);
-  }
-};
+// Fragment row gid (and gid + 8) of a tile is tile row g2_row(gid) (+ 8).  Q8_0 reads eight bytes a lane: even rows and odd
+// rows fall on different banks, consecutive rows do not.
+template <int FMT, int NT> __device__ __forceinline__ int g2_row(int gid) {
+  if constexpr (FMT == LLB_FM_Q8_0 || (FMT != LLB_FM_Q6_K && NT <= 2)) return ((gid & 3) << 1) | (gid >> 2);
+  else return gid;
+}
 
-// NTC < NT (the routed-expert launches at 16 rows): a weight tile is multiplied with NTC = 2 of the NT staged n-tiles only,
-// the hi and lo tiles of the eight rows its own row is among (Mats::col0(tile) = first plane column of the hi tile; the
-// lo tile is NC / 2 columns on), since the epilogue keeps one row of the tile.
-template <int FMT, int NT, class Stage, class Mats, int NTC = NT>
-__device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, uint8_t *smem, Stage stage, const Mats mats) {
-  using TR = G2Traits<FMT>;
-  constexpr int NC = 8 * NT, RS = TR::RS, SB = TR::SB, P = TR::P, NIT = (16 * P + 31) / 32, G2_WARPS = g2_warps<FMT>(8 * NT, NTC != NT), ST = g2_stages<FMT>(8 * NT, NTC != NT);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, j = lane & 3;
-  const bool live = bid < cps * a.ksplit && warp < G2_WARPS;
-  const int ks = bid % a.ksplit, ci = bid / a.ksplit;
-  const int sb0 = (int)(((long long)ks * a.nsb) / a.ksplit), nsl = (int)(((long long)(ks + 1) * a.nsb) / a.ksplit) - sb0;
-  const int CS = nsl * 512 + TR::XPAD;
-  uint8_t *xh_s = smem, *xsf_s = smem + NC * CS, *ring = xsf_s + nsl * NC * TR::AUX + (size_t)warp * ST * 16 * RS;
-  const uint32_t ring_s = smem_u32(ring);
-  int ntiles = live && Mats::EARLY ? mats.ntiles() : 0;   // a warp that is not live sees no tiles
-  const int nws = cps * G2_WARPS;
-  const size_t rb = mats.row_bytes();
+// The two scales and mins of column group j of a Q4_K / Q5_K row from its header words (bytes 4..15), as byte pairs:
+// sc = [sc(2j), sc(2j+1)], mn likewise (tools/qwen35_engine.c:66-72)
+__device__ __forceinline__ void g2_group_scales(uint32_t u0, uint32_t u1, uint32_t u2, int j, uint32_t &sc, uint32_t &mn) {
+  const int s = 16 * (j & 1);
+  const uint32_t a = u0 >> s, b = u1 >> s, c = u2 >> s;
+  sc = j < 2 ? a & 0x3f3fu : (c & 0x0f0fu) | ((a >> 2) & 0x3030u);
+  mn = j < 2 ? b & 0x3f3fu : ((c >> 4) & 0x0f0fu) | ((b >> 2) & 0x3030u);
+}
 
-  // per-lane copy plan: piece i = lane + 32*it of the 16 x P sixteen-byte pieces of a stage
-  uint32_t dst_rel[NIT], row_of[NIT], pc_of[NIT];
-  bool is_sc[NIT];
+// One staged tile times the staged planes of super-block c_c of the slice: acc[nt] += the tile's contribution to n-tile nt.
+//   st     the tile (shared memory);  xh_s, xsf_s, CS  the staged planes, means and column stride;  cb  first plane column
+//   NTS    plane columns from one computed n-tile to the next
+template <int FMT, int NT, int NTC>
+__device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, const uint8_t *xsf_s, const int CS, const int c_c, const int cb, const int lane, float (&acc)[NTC][4]) {
+  constexpr int NC = 8 * NT, NTS = NTC == NT ? 8 : NC / 2;
+  const int gid = lane >> 2, j = lane & 3, r0 = g2_row<FMT, NT>(gid);
+  const uint8_t *b0 = st + r0 * tile_row(FMT), *b1 = b0 + 8 * tile_row(FMT);
+  const uint8_t *xb = xh_s + (gid + cb) * CS + (size_t)c_c * 512;
+  if constexpr (FMT == LLB_FM_Q8_0) {
+    // eight blocks of 32 codes, two MMAs each; lane j holds columns 8 j .. 8 j + 7 of a block
+    const uint4 sw0 = *(const uint4 *)(b0 + 256), sw1 = *(const uint4 *)(b1 + 256);
+    const uint32_t d0w[4] = {sw0.x, sw0.y, sw0.z, sw0.w}, d1w[4] = {sw1.x, sw1.y, sw1.z, sw1.w};
+    xb += 16 * j;
 #pragma unroll
-  for (int it = 0; it < NIT; it++) {
-    is_sc[it] = false;
-    const int i = lane + 32 * it, r = i / P, p = i - r * P;
-    row_of[it] = r; pc_of[it] = p * 16; dst_rel[it] = i < 16 * P ? r * RS + p * 16 : 0xffffffffu;
-    // Q8_0: the scale piece comes from the row's scale area (K bytes into the row) and advances 16 bytes per
-    // super-block, not 256; its source is taken from the row start, not from the slice's first code
-    if (FMT == LLB_FM_Q8_0 && p == P - 1) { pc_of[it] = (uint32_t)a.K + (uint32_t)sb0 * 16; is_sc[it] = true; }
-  }
-  // producer cursor
-  // tile of (CTA ci, warp w, round n) = (n * WARPS + w) * cps + ci: consecutive tiles go to different SMs, so the
-  // SMs' tile counts differ by one at most (the kernel is issue-bound per SM: time follows the fullest SM)
-  int p_tile = warp * cps + ci, p_c = 0;
-  typename Mats::Cur p_cur;
-  uint32_t p_off[NIT];
-  auto plan_tile = [&](int tile) {
-    if (tile >= ntiles) return;
-    int row0, rows;
-    mats.locate(tile, sb0, p_cur, row0, rows);
+    for (int blk = 0; blk < 8; blk++) {
+      const uint2 w0 = *(const uint2 *)(b0 + 32 * blk + 8 * j), w1 = *(const uint2 *)(b1 + 32 * blk + 8 * j);
+      uint32_t A[2][4];
 #pragma unroll
-    for (int it = 0; it < NIT; it++) p_off[it] = (uint32_t)min(row0 + (int)row_of[it], rows - 1) * (uint32_t)rb + pc_of[it];
-  };
-  auto issue = [&](int stage) {
-    if (p_tile < ntiles) {
-      const uint8_t *src = mats.src(p_cur, sb0, p_c);
-      const uint32_t dst = ring_s + stage * 16 * RS;
+      for (int u = 0; u < 2; u++) {
+        const uint32_t p0 = u ? w0.y : w0.x, p1 = u ? w1.y : w1.x;
+        A[u][0] = g2_hadd2(__byte_perm(p0, 0x64646464u, 0x4240), 0xe480e480u);   // (1024 + byte) - 1152
+        A[u][1] = g2_hadd2(__byte_perm(p1, 0x64646464u, 0x4240), 0xe480e480u);
+        A[u][2] = g2_hadd2(__byte_perm(p0, 0x64646464u, 0x4341), 0xe480e480u);
+        A[u][3] = g2_hadd2(__byte_perm(p1, 0x64646464u, 0x4341), 0xe480e480u);
+      }
+      const float2 f0 = __half22float2(*(const __half2 *)&d0w[blk >> 1]), f1 = __half22float2(*(const __half2 *)&d1w[blk >> 1]);
+      const float d0 = (blk & 1) ? f0.y : f0.x, d1 = (blk & 1) ? f1.y : f1.x;
 #pragma unroll
-      for (int it = 0; it < NIT; it++)
-        if (dst_rel[it] != 0xffffffffu) {
-          if constexpr (FMT == LLB_FM_Q8_0) {
-            if (is_sc[it]) { cp_async16(dst + dst_rel[it], p_cur.W0 + (size_t)p_c * 16 + p_off[it]); continue; }
-          }
-          cp_async16(dst + dst_rel[it], src + p_off[it]);
-        }
-      if (++p_c == nsl) { p_c = 0; p_tile += nws; plan_tile(p_tile); }
+      for (int nt = 0; nt < NTC; nt++) {
+        const uint4 bx = *(const uint4 *)(xb + (size_t)nt * NTS * CS + 64 * blk);
+        float p[4];
+        mma16816_z(p, A[0][0], A[0][1], A[0][2], A[0][3], bx.x, bx.y);
+        mma16816(p, A[1][0], A[1][1], A[1][2], A[1][3], bx.z, bx.w);
+        acc[nt][0] += d0 * p[0]; acc[nt][1] += d0 * p[1]; acc[nt][2] += d1 * p[2]; acc[nt][3] += d1 * p[3];
+      }
     }
-    cp_async_commit();
-  };
-  if constexpr (Mats::EARLY) {
-    plan_tile(p_tile);
-    // weights first: the ring's prologue is in flight while the producer of the activations still
-    // runs (weights depend on no kernel), and while the activation slice is staged
-#pragma unroll 1
-    for (int s = 0; s < ST - 1; s++) issue(s);
-    stage(xh_s, xsf_s, CS, sb0, nsl);
-  } else {
-    // the weight addresses come from an earlier kernel's choice: the wait (inside stage) comes first
-    stage(xh_s, xsf_s, CS, sb0, nsl);
-    ntiles = live ? mats.ntiles() : 0;
-    plan_tile(p_tile);
-#pragma unroll 1
-    for (int s = 0; s < ST - 1; s++) issue(s);
-  }
-  // the XP group sits between prologue groups and later ones; from here on group accounting is per
-  // warp again: ST-1 chunks are complete, none pending
-  int pstage = ST - 1, cstage = 0;
-  int c_tile = warp * cps + ci, c_c = 0;
-  static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
-  constexpr int NTS = NTC == NT ? 8 : NC / 2;            // plane columns from one computed n-tile to the next
-  int cb = 0;                                            // first plane column of the computed n-tiles
-  float acc[NTC][4];
-  const uint8_t *xb = xh_s + gid * CS + 16 * j;          // B fragments of column gid (n-tile 0)
-  const uint8_t *xfb = xsf_s + gid * 32 + 8 * j;
-  const uint32_t mn_sel = (j & 1) ? 0x4342u : 0x4140u;
-#pragma unroll 1
-  while (c_tile < ntiles) {
-    if (c_c == 0) {
+  } else if constexpr (FMT == LLB_FM_Q6_K) {
+    // 16 scale groups of 16 columns, one MMA each; codes of quarters 2, 3 stay shifted left by four (16 q <= 1008)
+    const float d0 = h2f_bits(*(const unsigned short *)(st + 3328 + 2 * r0)), d1 = h2f_bits(*(const unsigned short *)(st + 3328 + 2 * (r0 + 8)));
+    const uint4 sw0 = *(const uint4 *)(b0 + 192), sw1 = *(const uint4 *)(b1 + 192);
+    const uint32_t sc0w[4] = {sw0.x ^ 0x80808080u, sw0.y ^ 0x80808080u, sw0.z ^ 0x80808080u, sw0.w ^ 0x80808080u};
+    const uint32_t sc1w[4] = {sw1.x ^ 0x80808080u, sw1.y ^ 0x80808080u, sw1.z ^ 0x80808080u, sw1.w ^ 0x80808080u};
+    xb += 8 * j;
+    float sS[NTC][4];
 #pragma unroll
-      for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-      if constexpr (NTC != NT) cb = mats.col0(c_tile);
-    }
-    issue(pstage);                       // refill the stage consumed last iteration
-    pstage = pstage + 1 == ST ? 0 : pstage + 1;
-    cp_async_wait<ST - 1>();             // all but the newest ST-1 groups: the stage to consume is in
-    __syncwarp();
-    if constexpr (FMT == LLB_FM_Q8_0) {
-      // eight blocks of 32 codes per super-block, two MMAs each; code (q ^ 0x80) = q + 128 as an fp16 subnormal,
-      // the offset taken back through the 32-column sums: d * (2^24 P - 128 sum x)
-      const uint8_t *b0 = ring + cstage * 16 * RS + gid * RS, *b1 = b0 + 8 * RS;
-      const uint4 sw0 = *(const uint4 *)(b0 + 256), sw1 = *(const uint4 *)(b1 + 256);
-      const uint32_t d0w[4] = {sw0.x, sw0.y, sw0.z, sw0.w}, d1w[4] = {sw1.x, sw1.y, sw1.z, sw1.w};
-      const uint8_t *xb8 = xh_s + (gid + cb) * CS + 8 * j + (size_t)c_c * 512;
-      const float *xs8 = (const float *)xsf_s + (size_t)c_c * 8 * NC + 2 * j + cb;
+    for (int nt = 0; nt < NTC; nt++) sS[nt][0] = sS[nt][1] = sS[nt][2] = sS[nt][3] = 0.0f;
 #pragma unroll
-      for (int blk = 0; blk < 8; blk++) {
-        float p[NTC][4];
+    for (int hf = 0; hf < 2; hf++) {
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int m = 2 * blk + u;
-          const uint32_t w0 = *(const uint32_t *)(b0 + 16 * m + 4 * j) ^ 0x80808080u, w1 = *(const uint32_t *)(b1 + 16 * m + 4 * j) ^ 0x80808080u;
-          const uint32_t a0 = __byte_perm(w0, 0, 0x4240), a2 = __byte_perm(w0, 0, 0x4341);
-          const uint32_t a1 = __byte_perm(w1, 0, 0x4240), a3 = __byte_perm(w1, 0, 0x4341);
+      for (int u = 0; u < 2; u++) {
+        const int o = 16 * u + 4 * j;
+        const uint32_t la0 = *(const uint32_t *)(b0 + 64 * hf + o), lb0 = *(const uint32_t *)(b0 + 64 * hf + 32 + o);
+        const uint32_t la1 = *(const uint32_t *)(b1 + 64 * hf + o), lb1 = *(const uint32_t *)(b1 + 64 * hf + 32 + o);
+        const uint32_t hq0 = *(const uint32_t *)(b0 + 128 + 32 * hf + o), hq1 = *(const uint32_t *)(b1 + 128 + 32 * hf + o);
+        const uint32_t h0s4 = hq0 << 4, h0s2 = hq0 << 2, h1s4 = hq1 << 4, h1s2 = hq1 << 2;
+        const uint32_t h0o4 = (hq0 >> 8) << 4, h0o2 = (hq0 >> 8) << 2, h1o4 = (hq1 >> 8) << 4, h1o2 = (hq1 >> 8) << 2;
+#pragma unroll
+        for (int qd = 0; qd < 4; qd++) {
+          const uint32_t l0 = (qd & 1) ? lb0 : la0, l1 = (qd & 1) ? lb1 : la1;
+          const uint32_t nm = qd < 2 ? 0x000f000fu : 0x00f000f0u, hm = qd < 2 ? 0x00300030u : 0x03000300u;
+          const uint32_t off = qd < 2 ? 0xe420e420u : 0xe600e600u;   // -(1024 + 32), -(1024 + 512)
+          // the two high bits of quarter 0 / 2 sit four bits up, those of 1 / 3 two bits up; quarters 2, 3 in the byte's upper half
+          const uint32_t e0 = g2_hadd2((l0 & nm) | ((((qd & 1) ? h0s2 : h0s4) & hm) | 0x64006400u), off);
+          const uint32_t e1 = g2_hadd2((l1 & nm) | ((((qd & 1) ? h1s2 : h1s4) & hm) | 0x64006400u), off);
+          const uint32_t o0 = g2_hadd2(((l0 >> 8) & nm) | ((((qd & 1) ? h0o2 : h0o4) & hm) | 0x64006400u), off);
+          const uint32_t o1 = g2_hadd2(((l1 >> 8) & nm) | ((((qd & 1) ? h1o2 : h1o4) & hm) | 0x64006400u), off);
+          const int gi = 8 * hf + 2 * qd + u;
+          // signed scale: (sc ^ 0x80) is sc + 128 as an unsigned byte
+          float s0 = __uint_as_float(__byte_perm(sc0w[gi >> 2], 0x4B000000u, 0x7650u | (gi & 3))) - 8388736.0f;
+          float s1 = __uint_as_float(__byte_perm(sc1w[gi >> 2], 0x4B000000u, 0x7650u | (gi & 3))) - 8388736.0f;
+          if (qd >= 2) { s0 *= 0.0625f; s1 *= 0.0625f; }
+          const int kl = 128 * hf + 32 * qd + 16 * u;
 #pragma unroll
           for (int nt = 0; nt < NTC; nt++) {
-            const uint2 bx = *(const uint2 *)(xb8 + (size_t)nt * NTS * CS + 32 * m);
-            if (u == 0) mma16816_z(p[nt], a0, a1, a2, a3, bx.x, bx.y);
-            else mma16816(p[nt], a0, a1, a2, a3, bx.x, bx.y);
-          }
-        }
-        const float d0 = h2f_bits((d0w[blk >> 1] >> (16 * (blk & 1))) & 0xffffu), d1 = h2f_bits((d1w[blk >> 1] >> (16 * (blk & 1))) & 0xffffu);
-#pragma unroll
-        for (int nt = 0; nt < NTC; nt++) {
-          const float2 xs = *(const float2 *)(xs8 + (size_t)blk * NC + nt * NTS);
-          acc[nt][0] += d0 * (p[nt][0] * TWO24 - 128.0f * xs.x);
-          acc[nt][1] += d0 * (p[nt][1] * TWO24 - 128.0f * xs.y);
-          acc[nt][2] += d1 * (p[nt][2] * TWO24 - 128.0f * xs.x);
-          acc[nt][3] += d1 * (p[nt][3] * TWO24 - 128.0f * xs.y);
-        }
-      }
-    } else if constexpr (FMT == LLB_FM_Q6_K) {
-      // 16 scale groups of 16 columns per super-block, one MMA each; code 0..63 as fp16 subnormals
-      // (quarters 2, 3 carry the code shifted left by 4), offset -32 through the 16-column sums
-      const uint8_t *b0 = ring + cstage * 16 * RS + gid * RS, *b1 = b0 + 8 * RS;
-      const float d0 = h2f_bits(*(const unsigned short *)(b0 + 208)), d1 = h2f_bits(*(const unsigned short *)(b1 + 208));
-      const uint4 sw0 = *(const uint4 *)(b0 + 192), sw1 = *(const uint4 *)(b1 + 192);
-      const uint32_t sc0w[4] = {sw0.x ^ 0x80808080u, sw0.y ^ 0x80808080u, sw0.z ^ 0x80808080u, sw0.w ^ 0x80808080u};
-      const uint32_t sc1w[4] = {sw1.x ^ 0x80808080u, sw1.y ^ 0x80808080u, sw1.z ^ 0x80808080u, sw1.w ^ 0x80808080u};
-      const uint8_t *xb6 = xh_s + (gid + cb) * CS + 8 * j + (size_t)c_c * 512;
-      const float *xs6 = (const float *)xsf_s + (size_t)c_c * 16 * NC + 2 * j + cb;
-#pragma unroll
-      for (int hf = 0; hf < 2; hf++) {
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int o = 16 * u + 4 * j;
-          const uint32_t la0 = *(const uint32_t *)(b0 + 64 * hf + o), lb0 = *(const uint32_t *)(b0 + 64 * hf + 32 + o);
-          const uint32_t la1 = *(const uint32_t *)(b1 + 64 * hf + o), lb1 = *(const uint32_t *)(b1 + 64 * hf + 32 + o);
-          const uint32_t hq0 = *(const uint32_t *)(b0 + 128 + 32 * hf + o), hq1 = *(const uint32_t *)(b1 + 128 + 32 * hf + o);
-          const uint32_t h0s4 = hq0 << 4, h0s2 = hq0 << 2, h1s4 = hq1 << 4, h1s2 = hq1 << 2;
-          const uint32_t h0o4 = (hq0 >> 8) << 4, h0o2 = (hq0 >> 8) << 2, h1o4 = (hq1 >> 8) << 4, h1o2 = (hq1 >> 8) << 2;
-#pragma unroll
-          for (int qd = 0; qd < 4; qd++) {
-            const uint32_t l0 = (qd & 1) ? lb0 : la0, l1 = (qd & 1) ? lb1 : la1;
-            const uint32_t nm = qd < 2 ? 0x000f000fu : 0x00f000f0u, hm = qd < 2 ? 0x00300030u : 0x03000300u;
-            const uint32_t e0 = (l0 & nm) | (((qd & 1) ? h0s2 : h0s4) & hm), e1 = (l1 & nm) | (((qd & 1) ? h1s2 : h1s4) & hm);
-            const uint32_t o0 = ((l0 >> 8) & nm) | (((qd & 1) ? h0o2 : h0o4) & hm), o1 = ((l1 >> 8) & nm) | (((qd & 1) ? h1o2 : h1o4) & hm);
-            const float w = qd < 2 ? TWO24 : TWO24 * 0.0625f;
-            const int gi = 8 * hf + 2 * qd + u;
-            // signed scale: (sc ^ 0x80) is sc + 128 as an unsigned byte
-            const float s0 = d0 * (__uint_as_float(__byte_perm(sc0w[gi >> 2], 0x4B000000u, 0x7650u | (gi & 3))) - 8388736.0f);
-            const float s1 = d1 * (__uint_as_float(__byte_perm(sc1w[gi >> 2], 0x4B000000u, 0x7650u | (gi & 3))) - 8388736.0f);
-            const int kl = 128 * hf + 32 * qd + 16 * u;
-#pragma unroll
-            for (int nt = 0; nt < NTC; nt++) {
-              const uint2 bx = *(const uint2 *)(xb6 + (size_t)nt * NTS * CS + kl * 2);
-              float p[4];
-              mma16816_z(p, e0, e1, o0, o1, bx.x, bx.y);
-              const float2 xs = *(const float2 *)(xs6 + (size_t)(kl >> 4) * NC + nt * NTS);
-              acc[nt][0] += s0 * (p[0] * w - 32.0f * xs.x);
-              acc[nt][1] += s0 * (p[1] * w - 32.0f * xs.y);
-              acc[nt][2] += s1 * (p[2] * w - 32.0f * xs.x);
-              acc[nt][3] += s1 * (p[3] * w - 32.0f * xs.y);
-            }
+            const uint2 bx = *(const uint2 *)(xb + (size_t)nt * NTS * CS + kl * 2);
+            float p[4];
+            mma16816_z(p, e0, e1, o0, o1, bx.x, bx.y);
+            sS[nt][0] += s0 * p[0]; sS[nt][1] += s0 * p[1]; sS[nt][2] += s1 * p[2]; sS[nt][3] += s1 * p[3];
           }
         }
       }
-    } else {
-      const uint8_t *b0 = ring + cstage * 16 * RS + gid * RS, *b1 = b0 + 8 * RS;
-      const uint4 h0 = *(const uint4 *)b0, h1 = *(const uint4 *)b1;
+    }
+#pragma unroll
+    for (int nt = 0; nt < NTC; nt++) { acc[nt][0] += d0 * sS[nt][0]; acc[nt][1] += d0 * sS[nt][1]; acc[nt][2] += d1 * sS[nt][2]; acc[nt][3] += d1 * sS[nt][3]; }
+  } else {
+    constexpr int QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
+    const uint4 h0 = *(const uint4 *)b0, h1 = *(const uint4 *)b1;
+    if constexpr (NT <= 2) {
       uint32_t scA0, scB0, mnA0, mnB0, scA1, scB1, mnA1, mnB1;
       k4_scales(h0.y, h0.z, h0.w, scA0, scB0, mnA0, mnB0);
       k4_scales(h1.y, h1.z, h1.w, scA1, scB1, mnA1, mnB1);
-      // the two mins of this thread's k-pair as fp16 numbers: 0x6400 | m is 1024 + m exactly; one FMA each gives m for
-      // the means' hi halves and m / 2048 for their lo halves (which are stored times 2048), both exact
-      const uint32_t at0 = __byte_perm(j < 2 ? mnA0 : mnB0, 0, mn_sel) | 0x64006400u, at1 = __byte_perm(j < 2 ? mnA1 : mnB1, 0, mn_sel) | 0x64006400u;
+      const uint32_t ms = (j & 1) ? 0x4342u : 0x4140u;
+      const uint32_t at0 = __byte_perm(j < 2 ? mnA0 : mnB0, 0x64646464u, ms), at1 = __byte_perm(j < 2 ? mnA1 : mnB1, 0x64646464u, ms);
       const uint32_t am0 = g2_hfma2(at0, 0x3c003c00u, 0xe400e400u), am1 = g2_hfma2(at1, 0x3c003c00u, 0xe400e400u);       // * 1 - 1024
       const uint32_t al0 = g2_hfma2(at0, 0x10001000u, 0xb800b800u), al1 = g2_hfma2(at1, 0x10001000u, 0xb800b800u);       // * 2^-11 - 0.5
-      uint32_t qh0 = 0, qh0b = 0, qh1 = 0, qh1b = 0;
-      if constexpr (FMT == LLB_FM_Q5_K) {
-        const uint2 t0 = *(const uint2 *)(b0 + 16 + 8 * j), t1 = *(const uint2 *)(b1 + 16 + 8 * j);
-        qh0 = t0.x; qh0b = t0.y; qh1 = t1.x; qh1b = t1.y;
-      }
       float sS[NTC][4], pm[NTC][4];
 #pragma unroll
       for (int nt = 0; nt < NTC; nt++) {
-        const uint2 xf = *(const uint2 *)(xfb + (size_t)c_c * NC * 32 + (nt * NTS + cb) * 32);
+        const uint2 xf = *(const uint2 *)(xsf_s + ((size_t)c_c * NC + nt * NTS + cb + gid) * 32 + 8 * j);
         mma16816_z(pm[nt], am0, am1, al0, al1, xf.x, xf.y);
         sS[nt][0] = sS[nt][1] = sS[nt][2] = sS[nt][3] = 0.0f;
       }
+      xb += 16 * j;
 #pragma unroll
       for (int g = 0; g < 4; g++) {
-        const uint2 a0 = *(const uint2 *)(b0 + TR::QOFF + 32 * g + 8 * j), a1 = *(const uint2 *)(b1 + TR::QOFF + 32 * g + 8 * j);
-        uint32_t f0l = 0, f0h = 0, f1l = 0, f1h = 0, f0lb = 0, f0hb = 0, f1lb = 0, f1hb = 0;
-        if constexpr (FMT == LLB_FM_Q5_K) {
-          f0l = (qh0 >> (2 * g)) & 0x01010101u; f0h = (qh0 >> (2 * g + 1)) & 0x01010101u;
-          f1l = (qh1 >> (2 * g)) & 0x01010101u; f1h = (qh1 >> (2 * g + 1)) & 0x01010101u;
-          f0lb = (qh0b >> (2 * g)) & 0x01010101u; f0hb = (qh0b >> (2 * g + 1)) & 0x01010101u;
-          f1lb = (qh1b >> (2 * g)) & 0x01010101u; f1hb = (qh1b >> (2 * g + 1)) & 0x01010101u;
+        const uint2 a0 = *(const uint2 *)(b0 + QOFF + 32 * g + 8 * j), a1 = *(const uint2 *)(b1 + QOFF + 32 * g + 8 * j);
+        uint2 f0 = make_uint2(0u, 0u), f1 = f0;
+        if constexpr (FMT == LLB_FM_Q5_K) { f0 = *(const uint2 *)(b0 + 16 + 8 * j); f1 = *(const uint2 *)(b1 + 16 + 8 * j); }
+        uint32_t A[2][2][4];               // [word][low / high nibbles]
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+          const uint32_t x0 = w ? a0.y : a0.x, x1 = w ? a1.y : a1.x, y0 = x0 >> 8, y1 = x1 >> 8;
+          A[w][0][0] = x0 & 0x000f000fu; A[w][0][1] = x1 & 0x000f000fu; A[w][0][2] = y0 & 0x000f000fu; A[w][0][3] = y1 & 0x000f000fu;
+          A[w][1][0] = x0 & 0x00f000f0u; A[w][1][1] = x1 & 0x00f000f0u; A[w][1][2] = y0 & 0x00f000f0u; A[w][1][3] = y1 & 0x00f000f0u;
+          if constexpr (FMT == LLB_FM_Q5_K) {
+            const uint32_t z0 = w ? f0.y : f0.x, z1 = w ? f1.y : f1.x;
+            // fifth bits 2 g (low) and 2 g + 1 (high) of every byte to bits 4 and 8
+            const int sl = 4 - 2 * g, sh = 7 - 2 * g;
+            const uint32_t l0 = sl >= 0 ? z0 << sl : z0 >> -sl, l1 = sl >= 0 ? z1 << sl : z1 >> -sl;
+            const uint32_t u0 = z0 << sh, u1 = z1 << sh;
+            A[w][0][0] |= l0 & 0x00100010u; A[w][0][1] |= l1 & 0x00100010u; A[w][0][2] |= (l0 >> 8) & 0x00100010u; A[w][0][3] |= (l1 >> 8) & 0x00100010u;
+            A[w][1][0] |= u0 & 0x01000100u; A[w][1][1] |= u1 & 0x01000100u; A[w][1][2] |= (z0 >> (8 - sh)) & 0x01000100u; A[w][1][3] |= (z1 >> (8 - sh)) & 0x01000100u;
+          }
         }
         const uint32_t s0 = g < 2 ? scA0 : scB0, s1 = g < 2 ? scA1 : scB1;
         const float sc0l = byte_f(s0, (2 * g) & 3), sc0h = byte_f_scaled(s0, (2 * g + 1) & 3, 0.0625f);
         const float sc1l = byte_f(s1, (2 * g) & 3), sc1h = byte_f_scaled(s1, (2 * g + 1) & 3, 0.0625f);
-        const uint32_t a0x8 = a0.x >> 8, a0y8 = a0.y >> 8, a1x8 = a1.x >> 8, a1y8 = a1.y >> 8;
 #pragma unroll
         for (int nt = 0; nt < NTC; nt++) {
-          const uint8_t *xr = xb + (size_t)(nt * NTS + cb) * CS + ((size_t)c_c * 256 + 64 * g) * 2;
+          const uint8_t *xr = xb + (size_t)nt * NTS * CS + 128 * g;
           const uint4 bl = *(const uint4 *)xr, bh = *(const uint4 *)(xr + 64);
           float pl[4], ph[4];
-          mma16816_z(pl, (a0.x & 0x000f000fu) | ((f0l & 0x00010001u) << 4), (a1.x & 0x000f000fu) | ((f1l & 0x00010001u) << 4),
-                     (a0x8 & 0x000f000fu) | (((f0l >> 8) & 0x00010001u) << 4), (a1x8 & 0x000f000fu) | (((f1l >> 8) & 0x00010001u) << 4), bl.x, bl.y);
-          mma16816(pl, (a0.y & 0x000f000fu) | ((f0lb & 0x00010001u) << 4), (a1.y & 0x000f000fu) | ((f1lb & 0x00010001u) << 4),
-                   (a0y8 & 0x000f000fu) | (((f0lb >> 8) & 0x00010001u) << 4), (a1y8 & 0x000f000fu) | (((f1lb >> 8) & 0x00010001u) << 4), bl.z, bl.w);
-          mma16816_z(ph, (a0.x & 0x00f000f0u) | ((f0h & 0x00010001u) << 8), (a1.x & 0x00f000f0u) | ((f1h & 0x00010001u) << 8),
-                     (a0x8 & 0x00f000f0u) | (((f0h >> 8) & 0x00010001u) << 8), (a1x8 & 0x00f000f0u) | (((f1h >> 8) & 0x00010001u) << 8), bh.x, bh.y);
-          mma16816(ph, (a0.y & 0x00f000f0u) | ((f0hb & 0x00010001u) << 8), (a1.y & 0x00f000f0u) | ((f1hb & 0x00010001u) << 8),
-                   (a0y8 & 0x00f000f0u) | (((f0hb >> 8) & 0x00010001u) << 8), (a1y8 & 0x00f000f0u) | (((f1hb >> 8) & 0x00010001u) << 8), bh.z, bh.w);
+          mma16816_z(pl, A[0][0][0], A[0][0][1], A[0][0][2], A[0][0][3], bl.x, bl.y);
+          mma16816_z(ph, A[0][1][0], A[0][1][1], A[0][1][2], A[0][1][3], bh.x, bh.y);
+          mma16816(pl, A[1][0][0], A[1][0][1], A[1][0][2], A[1][0][3], bl.z, bl.w);
+          mma16816(ph, A[1][1][0], A[1][1][1], A[1][1][2], A[1][1][3], bh.z, bh.w);
           sS[nt][0] += sc0l * pl[0] + sc0h * ph[0];
           sS[nt][1] += sc0l * pl[1] + sc0h * ph[1];
           sS[nt][2] += sc1l * pl[2] + sc1h * ph[2];
@@ -347,35 +250,226 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
         acc[nt][2] += d1 * sS[nt][2] - dm1 * pm[nt][2];
         acc[nt][3] += d1 * sS[nt][3] - dm1 * pm[nt][3];
       }
+      return;
     }
-    __syncwarp();
-    cstage = cstage + 1 == ST ? 0 : cstage + 1;
-    if (++c_c == nsl) {
-      mats.template epilogue<NTC>(ks, c_tile, acc, lane);
-      c_c = 0;
-      c_tile += nws;
+    uint32_t sc0, mn0, sc1, mn1;
+    g2_group_scales(h0.y, h0.z, h0.w, j, sc0, mn0);
+    g2_group_scales(h1.y, h1.z, h1.w, j, sc1, mn1);
+    // the scales as fp16 (0x6400 | s is 1024 + s), times 2^10 for the low nibbles and 2^6 for the high ones, which stay four
+    // bits up: q 2^-24 * s 2^10 = 16 q 2^-24 * s 2^6 = s q 2^-14, exact
+    const uint32_t L0 = g2_hmul2(g2_hadd2(__byte_perm(sc0, 0x64646464u, 0x4040), 0xe400e400u), 0x64006400u);
+    const uint32_t L1 = g2_hmul2(g2_hadd2(__byte_perm(sc1, 0x64646464u, 0x4040), 0xe400e400u), 0x64006400u);
+    const uint32_t H0 = g2_hmul2(g2_hadd2(__byte_perm(sc0, 0x64646464u, 0x4141), 0xe400e400u), 0x54005400u);
+    const uint32_t H1 = g2_hmul2(g2_hadd2(__byte_perm(sc1, 0x64646464u, 0x4141), 0xe400e400u), 0x54005400u);
+    // this lane's two mins: 1024 + m exactly; one FMA each gives m for the means' hi halves and m / 2048 for their lo halves
+    const uint32_t at0 = __byte_perm(mn0, 0x64646464u, 0x4140), at1 = __byte_perm(mn1, 0x64646464u, 0x4140);
+    const uint32_t am0 = g2_hfma2(at0, 0x3c003c00u, 0xe400e400u), am1 = g2_hfma2(at1, 0x3c003c00u, 0xe400e400u);       // * 1 - 1024
+    const uint32_t al0 = g2_hfma2(at0, 0x10001000u, 0xb800b800u), al1 = g2_hfma2(at1, 0x10001000u, 0xb800b800u);       // * 2^-11 - 0.5
+    float pl[NTC][4], ph[NTC][4], pm[NTC][4];
+#pragma unroll
+    for (int nt = 0; nt < NTC; nt++) {
+      const uint2 xf = *(const uint2 *)(xsf_s + ((size_t)c_c * NC + nt * NTS + cb + gid) * 32 + 8 * j);
+      mma16816_z(pm[nt], am0, am1, al0, al1, xf.x, xf.y);
+    }
+    xb += 16 * j;
+    const int rl = FMT == LLB_FM_Q5_K ? (4 - 2 * j) & 31 : 0;     // rotates bit 2 j of a byte to bit 4
+#pragma unroll
+    for (int q = 0; q < 4; q++) {        // words 2 q and 2 q + 1 of the group's 32 bytes: columns 8 q .. 8 q + 7 of both sub-blocks
+      const uint2 a0 = *(const uint2 *)(b0 + QOFF + 32 * j + 8 * q), a1 = *(const uint2 *)(b1 + QOFF + 32 * j + 8 * q);
+      uint2 f0 = make_uint2(0u, 0u), f1 = f0;
+      if constexpr (FMT == LLB_FM_Q5_K) { f0 = *(const uint2 *)(b0 + 16 + 8 * q); f1 = *(const uint2 *)(b1 + 16 + 8 * q); }
+      uint32_t A[2][2][4];               // [word][low / high nibbles]
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        const uint32_t x0 = w ? a0.y : a0.x, x1 = w ? a1.y : a1.x, y0 = x0 >> 8, y1 = x1 >> 8;
+        if constexpr (FMT == LLB_FM_Q4_K) {
+          A[w][0][0] = g2_hmul2(x0 & 0x000f000fu, L0); A[w][0][1] = g2_hmul2(x1 & 0x000f000fu, L1);
+          A[w][0][2] = g2_hmul2(y0 & 0x000f000fu, L0); A[w][0][3] = g2_hmul2(y1 & 0x000f000fu, L1);
+          A[w][1][0] = g2_hmul2(x0 & 0x00f000f0u, H0); A[w][1][1] = g2_hmul2(x1 & 0x00f000f0u, H1);
+          A[w][1][2] = g2_hmul2(y0 & 0x00f000f0u, H0); A[w][1][3] = g2_hmul2(y1 & 0x00f000f0u, H1);
+        } else {
+          const uint32_t z0 = w ? f0.y : f0.x, z1 = w ? f1.y : f1.x;
+          const uint32_t u0 = __funnelshift_l(z0, z0, rl), u1 = __funnelshift_l(z1, z1, rl);         // fifth bits at 4 (low), 5 (high) of every byte
+          const uint32_t v0 = u0 << 3, v1 = u1 << 3, t0 = u0 >> 8, t1 = u1 >> 8, s0 = u0 >> 5, s1 = u1 >> 5;   // high ones at 8
+          A[w][0][0] = g2_hmul2((x0 & 0x000f000fu) | (u0 & 0x00100010u), L0); A[w][0][1] = g2_hmul2((x1 & 0x000f000fu) | (u1 & 0x00100010u), L1);
+          A[w][0][2] = g2_hmul2((y0 & 0x000f000fu) | (t0 & 0x00100010u), L0); A[w][0][3] = g2_hmul2((y1 & 0x000f000fu) | (t1 & 0x00100010u), L1);
+          A[w][1][0] = g2_hmul2((x0 & 0x00f000f0u) | (v0 & 0x01000100u), H0); A[w][1][1] = g2_hmul2((x1 & 0x00f000f0u) | (v1 & 0x01000100u), H1);
+          A[w][1][2] = g2_hmul2((y0 & 0x00f000f0u) | (s0 & 0x01000100u), H0); A[w][1][3] = g2_hmul2((y1 & 0x00f000f0u) | (s1 & 0x01000100u), H1);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < NTC; nt++) {
+        const uint8_t *xr = xb + (size_t)nt * NTS * CS + 64 * q;
+        const uint4 bl = *(const uint4 *)xr, bh = *(const uint4 *)(xr + 256);
+        if (q == 0) {
+          mma16816_z(pl[nt], A[0][0][0], A[0][0][1], A[0][0][2], A[0][0][3], bl.x, bl.y);
+          mma16816_z(ph[nt], A[0][1][0], A[0][1][1], A[0][1][2], A[0][1][3], bh.x, bh.y);
+        } else {
+          mma16816(pl[nt], A[0][0][0], A[0][0][1], A[0][0][2], A[0][0][3], bl.x, bl.y);
+          mma16816(ph[nt], A[0][1][0], A[0][1][1], A[0][1][2], A[0][1][3], bh.x, bh.y);
+        }
+        mma16816(pl[nt], A[1][0][0], A[1][0][1], A[1][0][2], A[1][0][3], bl.z, bl.w);
+        mma16816(ph[nt], A[1][1][0], A[1][1][1], A[1][1][2], A[1][1][3], bh.z, bh.w);
+      }
+    }
+    const float d0 = h2f_bits(h0.x & 0xffffu) * 16384.0f, dm0 = h2f_bits(h0.x >> 16) * 32.0f;
+    const float d1 = h2f_bits(h1.x & 0xffffu) * 16384.0f, dm1 = h2f_bits(h1.x >> 16) * 32.0f;
+#pragma unroll
+    for (int nt = 0; nt < NTC; nt++) {
+      acc[nt][0] += d0 * (pl[nt][0] + ph[nt][0]) - dm0 * pm[nt][0];
+      acc[nt][1] += d0 * (pl[nt][1] + ph[nt][1]) - dm0 * pm[nt][1];
+      acc[nt][2] += d1 * (pl[nt][2] + ph[nt][2]) - dm1 * pm[nt][2];
+      acc[nt][3] += d1 * (pl[nt][3] + ph[nt][3]) - dm1 * pm[nt][3];
     }
   }
-  cp_async_wait<0>();
+}
+
+// The warp's ring as it passes from one GEMM phase to the next: barriers (one a stage), stage memory, and the parity that
+// each stage's next wait looks for.
+struct G2Ring { uint32_t bar_s, ring_s; const uint8_t *ring; uint32_t par; };
+// smem: G2_BAR_BYTES of barriers and then the rings, `per_warp` bytes each.  Private to a warp: no block barrier needed.
+__device__ __forceinline__ G2Ring g2_ring_init(uint8_t *smem, int per_warp) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  G2Ring r;
+  r.bar_s = smem_u32(smem) + warp * 32;
+  r.ring = smem + G2_BAR_BYTES + warp * per_warp;
+  r.ring_s = smem_u32(r.ring);
+  r.par = 0;
+  if (warp < G2_MAXWARPS && lane == 0) {
+    for (int s = 0; s < 4; s++) mbar_init(r.bar_s + 8 * s, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  return r;
+}
+
+// Where a launch's row tiles live.  A policy says how many 16-row tiles there are, where tile i's 16 x 256 tiles in the
+// CTA's K-slice are, and what to do with a finished row tile.  G2MatsPlain is the launch of up to four matrices that
+// GemmArgs describes; the routed-expert launches (moe.cuh) find their matrices through the expert ids an earlier kernel chose.
+//   EARLY   the weight addresses depend on no earlier kernel: the ring's prologue is issued before the wait
+//   Cur     cursor of the row tile being copied;  locate  row tile -> cursor;  src  tile of super-block sb0 + c of the slice
+template <int FMT, int NTP> struct G2MatsPlain {
+  static constexpr bool EARLY = true, CONTIG = true;
+  const GemmArgs &a;
+  struct Cur { const uint8_t *W; };
+  __device__ __forceinline__ int ntiles() const { return a.tile0[a.nmat]; }
+  __device__ __forceinline__ void locate(int tile, int sb0, Cur &c) const {
+    int m = 0;
+    while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
+    c.W = a.m[m].W + ((size_t)(tile - a.tile0[m]) * a.nsb + sb0) * tile_bytes(FMT);
+  }
+  __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const { return c.W + (size_t)pc * tile_bytes(FMT); }
+  template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
+    int m = 0;
+    while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
+    gemm_epilogue<NT>(a, a.m[m], ks, (tile - a.tile0[m]) * 16 + g2_row<FMT, NTP>(lane >> 2), acc, lane);
+  }
+};
+
+// One GEMM's work of a CTA (bid of cps * ksplit).  g2_fill requests the first tiles of every warp's ring; g2_run (after the
+// activation slice has been staged) streams the CTA's tiles through it.
+// NTC < NT (the routed-expert launches at 16 rows): a weight tile is multiplied with NTC = 2 of the NT staged n-tiles only,
+// the hi and lo tiles of the eight rows its own row is among (Mats::col0(tile) = first plane column of the hi tile; the
+// lo tile is NC / 2 columns on), since the epilogue keeps one row of the tile.
+struct G2Slice { int ks, ci, sb0, nsl; bool live; };
+__device__ __forceinline__ G2Slice g2_slice(const GemmArgs &a, int cps, int bid) {
+  G2Slice s;
+  s.live = bid < cps * a.ksplit;
+  s.ks = bid % a.ksplit; s.ci = bid / a.ksplit;
+  s.sb0 = (int)(((long long)s.ks * a.nsb) / a.ksplit); s.nsl = (int)(((long long)(s.ks + 1) * a.nsb) / a.ksplit) - s.sb0;
+  return s;
+}
+// The warp's sequence of copies: (row tile, first super-block of the chunk), chunk after chunk, tile after tile.
+// tile of (CTA ci, warp w, round n) = (n * WARPS + w) * cps + ci: consecutive tiles go to different SMs, so the SMs' tile
+// counts differ by one at most
+template <int FMT, class Mats> struct G2Feed {
+  int tile, c;
+  typename Mats::Cur cur;
+  __device__ __forceinline__ void next(const G2Slice &sl, int nws, int n) { c += n; if (c == sl.nsl) { c = 0; tile += nws; } }
+  __device__ __forceinline__ void issue(const Mats &mats, const G2Slice &sl, const G2Ring &rg, int s, int ntiles, int nws, int lane) {
+    constexpr int TB = tile_bytes(FMT), CH = g2_chunk(FMT);
+    if (tile >= ntiles) return;
+    if (c == 0) mats.locate(tile, sl.sb0, cur);
+    const int n = min(CH, sl.nsl - c);
+    if (lane == 0) {
+      const uint32_t bar = rg.bar_s + 8 * s, dst = rg.ring_s + s * CH * TB;
+      mbar_expect(bar, n * TB);
+      if (Mats::CONTIG || CH == 1) bulk_load(dst, mats.src(cur, sl.sb0, c), n * TB, bar);
+      else for (int u = 0; u < n; u++) bulk_load(dst + u * TB, mats.src(cur, sl.sb0, c + u), TB, bar);
+    }
+    next(sl, nws, n);
+  }
+};
+template <int FMT, int NC, int WARPS, class Mats>
+__device__ __forceinline__ void g2_fill(const G2Slice &sl, int cps, const G2Ring &rg, const Mats &mats) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ntiles = sl.live && warp < WARPS ? mats.ntiles() : 0;
+  G2Feed<FMT, Mats> f;
+  f.tile = warp * cps + sl.ci; f.c = 0;
+#pragma unroll 1
+  for (int s = 0; s < g2_stages(FMT, NC); s++) f.issue(mats, sl, rg, s, ntiles, cps * WARPS, lane);
+}
+template <int FMT, int NT, int WARPS, class Mats, int NTC = NT>
+__device__ __forceinline__ void g2_run(const GemmArgs &a, const G2Slice &sl, int cps, G2Ring &rg, const uint8_t *xh_s, const uint8_t *xsf_s, int CS, const Mats &mats) {
+  constexpr int NC = 8 * NT, TB = tile_bytes(FMT), ST = g2_stages(FMT, NC), CH = g2_chunk(FMT);
+  static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nws = cps * WARPS, ntiles = sl.live && warp < WARPS ? mats.ntiles() : 0;
+  G2Feed<FMT, Mats> f;
+  f.tile = warp * cps + sl.ci; f.c = 0;
+  // behind what g2_fill has requested
+  for (int s = 0; s < ST && f.tile < ntiles; s++) f.next(sl, nws, min(CH, sl.nsl - f.c));
+  if (f.c > 0 && f.tile < ntiles) mats.locate(f.tile, sl.sb0, f.cur);
+  int s = 0;
+#pragma unroll 1
+  for (int tile = warp * cps + sl.ci; tile < ntiles; tile += nws) {
+    int cb = 0;                                            // first plane column of the computed n-tiles
+    if constexpr (NTC != NT) cb = mats.col0(tile);
+    float acc[NTC][4];
+#pragma unroll
+    for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < sl.nsl; c += CH) {
+      if (!mbar_wait(rg.bar_s + 8 * s, (rg.par >> s) & 1u) && a.err) atomicExch(a.err, 1u);
+      rg.par ^= 1u << s;
+#pragma unroll 1
+      for (int u = 0; u < CH && c + u < sl.nsl; u++) g2_tile<FMT, NT, NTC>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
+      __syncwarp();                                        // every lane has read the stage
+      f.issue(mats, sl, rg, s, ntiles, nws, lane);
+      s = s + 1 == ST ? 0 : s + 1;
+    }
+    mats.template epilogue<NTC>(sl.ks, tile, acc, lane);
+  }
+}
+// One launch: fill the ring, call stage(xh_s, xsf_s, CS, sb0, nsl) -- which waits for whatever produces the activations, puts the
+// CTA's slice of the planes and its side array into shared memory and ends with a block-wide barrier --, then stream.
+template <int FMT, int NT, class Stage, class Mats, int NTC = NT>
+__device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, G2Ring &rg, uint8_t *planes, Stage stage, const Mats mats) {
+  constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC);
+  const G2Slice sl = g2_slice(a, cps, bid);
+  const int CS = sl.nsl * 512 + g2_xpad(FMT);
+  // weights first where their addresses depend on no kernel: the ring is in flight while the producer of the activations
+  // still runs, and while the activation slice is staged
+  if constexpr (Mats::EARLY) g2_fill<FMT, NC, WARPS>(sl, cps, rg, mats);
+  stage(planes, planes + NC * CS, CS, sl.sb0, sl.nsl);
+  if constexpr (!Mats::EARLY) g2_fill<FMT, NC, WARPS>(sl, cps, rg, mats);
+  g2_run<FMT, NT, WARPS, Mats, NTC>(a, sl, cps, rg, planes, planes + NC * CS, CS, mats);
 }
 
 // the activation slice from the planes in global memory: cp.async, one wait, one barrier
 template <int FMT, int NT> struct G2StagePlanes {
   const GemmArgs &a;
   __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
-    using TR = G2Traits<FMT>;
     constexpr int NC = 8 * NT;
     pdl_wait();
-    const int per_col = nsl * 32;   // 16-byte pieces of one column's slice
-    for (int i = threadIdx.x; i < NC * per_col; i += blockDim.x) {
-      const int c = i / per_col, p = i - c * per_col;
-      cp_async16(smem_u32(xh_s + c * CS + p * 16), (const uint8_t *)(a.xp.xh + (size_t)c * a.K + (size_t)sb0 * 256) + p * 16);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int c = warp; c < NC; c += nw) {   // a warp takes a column: 32 sixteen-byte pieces a super-block
+      const uint8_t *src = (const uint8_t *)(a.xp.xh + (size_t)c * a.K + (size_t)sb0 * 256);
+      const uint32_t dst = smem_u32(xh_s + c * CS);
+      for (int p = lane; p < nsl * 32; p += 32) cp_async16(dst + g2_xpos<FMT, NT>(p), src + p * 16);
     }
-    // the side array of the slice: contiguous in global memory for all kinds
-    const uint8_t *xf = FMT == LLB_FM_Q6_K   ? (const uint8_t *)(a.xp.xs16 + (size_t)sb0 * 16 * NC)
-                        : FMT == LLB_FM_Q8_0 ? (const uint8_t *)(a.xp.xs32 + (size_t)sb0 * 8 * NC)
-                                             : (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
-    for (int i = threadIdx.x; i < nsl * NC * (TR::AUX / 16); i += blockDim.x) cp_async16(smem_u32(xsf_s + i * 16), xf + i * 16);
+    if constexpr (g2_aux(FMT) != 0) {       // the means of the slice: contiguous in global memory
+      const uint8_t *xf = (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
+      for (int i = threadIdx.x; i < nsl * NC * 2; i += blockDim.x) cp_async16(smem_u32(xsf_s + i * 16), xf + i * 16);
+    }
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
@@ -383,8 +477,9 @@ template <int FMT, int NT> struct G2StagePlanes {
 };
 
 template <int FMT, int NT>
-__global__ void __launch_bounds__(g2_warps<FMT>(8 * NT) * 32, G2_CPSM) k_gemm2(const GemmArgs a, const int cps) {
+__global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_gemm2(const GemmArgs a, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  g2_phase<FMT, NT>(a, cps, (int)blockIdx.x, smem, G2StagePlanes<FMT, NT>{a}, G2MatsPlain<FMT>{a});
+  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
+  g2_phase<FMT, NT>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT), G2StagePlanes<FMT, NT>{a}, G2MatsPlain<FMT, NT>{a});
 }

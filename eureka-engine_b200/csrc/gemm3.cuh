@@ -68,7 +68,6 @@ __global__ void __launch_bounds__(G3_BLOCK, 1) k_gemm3(const GemmArgs a, const i
   for (int m = 0; m < GEMM_MAXMAT; m++) t128[m + 1] = t128[m] + (m < a.nmat ? (a.m[m].rows + 127) / 128 : 0);
   const int ntiles = t128[GEMM_MAXMAT];
   const int my_tiles = ci < ntiles ? (ntiles - ci + cps - 1) / cps : 0, n_items = my_tiles * nsl;
-  const size_t rb = dev_row_bytes(LLB_FM_Q4_K, a.K);
 
   // The four warps of a lane quarter load the quarter's 32 rows x 144 bytes of a super-block together:
   // 288 sixteen-byte pieces, piece i = tq + 128 * it of thread tq = 32 c + lane, nine consecutive pieces per row.
@@ -82,16 +81,17 @@ __global__ void __launch_bounds__(G3_BLOCK, 1) k_gemm3(const GemmArgs a, const i
     if (tile >= ntiles) return;
     const int m = (tile >= t128[1]) + (tile >= t128[2]) + (tile >= t128[3]);   // t128[k] = ntiles beyond the last matrix
     const int row0 = (tile - (m == 0 ? 0 : m == 1 ? t128[1] : m == 2 ? t128[2] : t128[3])) * 128 + 32 * q, rows = a.m[m].rows;
-    p_W = a.m[m].W + (size_t)sb0 * 144;
+    p_W = a.m[m].W + (size_t)sb0 * tile_bytes(LLB_FM_Q4_K);
 #pragma unroll
     for (int it = 0; it < 3; it++) {
       const int i = tq + 128 * it, rr = i / 9, pp = i - rr * 9;
-      p_off[it] = (uint32_t)min(row0 + rr, rows - 1) * (uint32_t)rb + pp * 16;
+      const int r = min(row0 + rr, rows - 1);
+      p_off[it] = (uint32_t)(r >> 4) * (uint32_t)(a.nsb * tile_bytes(LLB_FM_Q4_K)) + (r & 15) * 144 + pp * 16;
     }
   };
   auto issue = [&]() {
     if (p_left > 0) {
-      const uint8_t *src = p_W + (size_t)p_c * 144;
+      const uint8_t *src = p_W + (size_t)p_c * tile_bytes(LLB_FM_Q4_K);
       const uint32_t dst = qring_s + p_stage * G3_STAGE_BYTES + tq * 16;
       cp_async16(dst, src + p_off[0]);
       cp_async16(dst + 2048, src + p_off[1]);

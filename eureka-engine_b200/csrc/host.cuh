@@ -46,8 +46,8 @@ inline cudaError_t llb_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
 }
 
 // gemm.cu
-int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool sel = false);   // sel: for a routed-expert launch
-int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool sel = false);   // clamps a requested K-split to what the format's kernel can take
+int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms);
+int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks);   // clamps a requested K-split to what the format's kernel can take
 int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int sms, int cap);
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a);   // fills tile0 / nsb, picks NT from xp.NC
 int gemm_setup(void);
@@ -64,4 +64,6 @@ int ops_xp_from_f32(cudaStream_t s, const float *x, int T, int planes, XPlanes x
 int ops_xp_from_bf16(cudaStream_t s, const void *x, int T, XPlanes xp);
 int ops_dequant_rows(cudaStream_t s, int fmt, const uint8_t *W, int rows, int cols, const int *row_ids, int nrows, float *out);
 int ops_repack_q6k(cudaStream_t s, const uint8_t *src210, uint8_t *dst224, size_t nblocks);
+int ops_to_tiles(cudaStream_t s, int fmt, const uint8_t *src, int rows, int cols, uint8_t *dst);
+int ops_tile_slice(cudaStream_t s, int fmt, const uint8_t *src, int scols, uint8_t *dst, int dcols, int srow, int drow, int n, int scol, int dcol, int nc);
 int ops_sum_parts(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int n, float *out);

@@ -45,19 +45,17 @@ template <int NTC> __device__ __forceinline__ void moe_col(const float (&acc)[NT
   v1 = acc[0][i + 2] + lo[i + 2] * XP_LO_INV;
 }
 
-template <int FMT> struct MoeGuMats {
-  static constexpr bool EARLY = false;
+template <int FMT, int NTP> struct MoeGuMats {
+  static constexpr bool EARLY = false, CONTIG = true;
   const MoeArgs &m;
   struct Cur { const uint8_t *W; };
   __device__ __forceinline__ int ntiles() const { return min(*m.n_rows, m.T) * m.nslot * (m.ef >> 3); }   // 2 ef / 16 tiles per slot
-  __device__ __forceinline__ size_t row_bytes() const { return dev_row_bytes(FMT, m.d); }
-  __device__ __forceinline__ void locate(int tile, int sb0, Cur &c, int &row0, int &rows) const {
+  __device__ __forceinline__ void locate(int tile, int sb0, Cur &c) const {
     const int tps = m.ef >> 3, slot = tile / tps;
     const int e = min(max(m.ids[slot], 0), m.ne);
-    row0 = (tile - slot * tps) * 16; rows = 2 * m.ef;
-    c.W = m.W + (size_t)e * m.es + (size_t)sb0 * G2Traits<FMT>::SB;
+    c.W = m.W + (size_t)e * m.es + ((size_t)(tile - slot * tps) * (m.d >> 8) + sb0) * tile_bytes(FMT);
   }
-  __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const { return c.W + (size_t)pc * G2Traits<FMT>::SB; }
+  __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const { return c.W + (size_t)pc * tile_bytes(FMT); }
   __device__ __forceinline__ int col0(int tile) const { return ((tile / (m.ef >> 3)) / m.nslot) & ~7; }
   template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
     const int tps = m.ef >> 3, slot = tile / tps, t = slot / m.nslot, jx = slot - t * m.nslot;
@@ -65,27 +63,26 @@ template <int FMT> struct MoeGuMats {
     bool mine;
     moe_col<NT>(acc, t, lane, v0, v1, mine);
     if (!mine) return;
-    const int r = (tile - slot * tps) * 16 + (lane >> 2);          // rows r and r + 8 of [gate | up]; a tile is all gate or all up
-    float *dst = (r < m.ef ? m.g : m.u) + (size_t)t * m.nslot * m.ef + (size_t)jx * m.ef + (r < m.ef ? r : r - m.ef);
+    const int r = (tile - slot * tps) * 16 + g2_row<FMT, NTP>(lane >> 2);          // rows r and r + 8 of [gate | up]; a tile is all gate or all up
+    float *dst = (r < m.ef ? m.g : m.u) + (size_t)ks * m.gu_stride + (size_t)t * m.nslot * m.ef + (size_t)jx * m.ef + (r < m.ef ? r : r - m.ef);
     dst[0] = v0; dst[8] = v1;
   }
 };
 
-template <int FMT> struct MoeDnMats {
-  static constexpr bool EARLY = false;
+template <int FMT, int NTP> struct MoeDnMats {
+  static constexpr bool EARLY = false, CONTIG = false;
   const MoeArgs &m;
-  struct Cur { const int *ids; };
+  struct Cur { const int *ids; int tile; };
   __device__ __forceinline__ int ntiles() const { return min(*m.n_rows, m.T) * (m.d >> 4); }
-  __device__ __forceinline__ size_t row_bytes() const { return dev_row_bytes(FMT, m.ef); }
-  __device__ __forceinline__ void locate(int tile, int sb0, Cur &c, int &row0, int &rows) const {
+  __device__ __forceinline__ void locate(int tile, int sb0, Cur &c) const {
     const int tpt = m.d >> 4, t = tile / tpt;
-    row0 = (tile - t * tpt) * 16; rows = m.d;
+    c.tile = tile - t * tpt;
     c.ids = m.ids + t * m.nslot;
   }
   __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const {
     const int eb = m.ef >> 8, sbi = sb0 + pc, g = sbi / eb;
     const int e = min(max(c.ids[g], 0), m.ne);
-    return m.W + (size_t)e * m.es + (size_t)(sbi - g * eb) * G2Traits<FMT>::SB;
+    return m.W + (size_t)e * m.es + ((size_t)c.tile * eb + sbi - g * eb) * tile_bytes(FMT);
   }
   __device__ __forceinline__ int col0(int tile) const { return (tile / (m.d >> 4)) & ~7; }
   template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
@@ -94,16 +91,18 @@ template <int FMT> struct MoeDnMats {
     bool mine;
     moe_col<NT>(acc, t, lane, v0, v1, mine);
     if (!mine) return;
-    float *dst = m.out + (size_t)ks * m.split_stride + (size_t)t * m.d + (tile - t * tpt) * 16 + (lane >> 2);
+    float *dst = m.out + (size_t)ks * m.split_stride + (size_t)t * m.d + (tile - t * tpt) * 16 + g2_row<FMT, NTP>(lane >> 2);
     dst[0] = v0; dst[8] = v1;
   }
 };
 
 template <int FMT, int NT>
-__global__ void __launch_bounds__(g2_warps<FMT>(8 * NT, moe_ntc<NT>() != NT) * 32, G2_CPSM) k_moe_gu(const GemmArgs a, const MoeArgs m, const int cps) {
+__global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_gu(const GemmArgs a, const MoeArgs m, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeGuMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, smem, G2StagePlanes<FMT, NT>{a}, MoeGuMats<FMT>{m});
+  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeGuMats<FMT, NT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                          G2StagePlanes<FMT, NT>{a}, MoeGuMats<FMT, NT>{m});
 }
 // The down launch's activation slice built in shared memory from the gate|up outputs (T <= 4 rows): wt * silu(g) * u
 // of the CTA's K-slice, planes and side array exactly as k_silu_xp + G2StagePlanes would have left them, without the
@@ -144,15 +143,18 @@ template <int FMT> struct MoeStageSilu {
 };
 
 template <int FMT>
-__global__ void __launch_bounds__(G2Traits<FMT>::WARPS * 32, G2_CPSM) k_moe_dn_silu(const GemmArgs a, const MoeArgs m, const float *wt, const int cps) {
+__global__ void __launch_bounds__(g2_warps(FMT, 8) * 32, 1) k_moe_dn_silu(const GemmArgs a, const MoeArgs m, const float *wt, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, smem, MoeStageSilu<FMT>{m, wt}, MoeDnMats<FMT>{m});
+  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8) / g2_warps(FMT, 8));
+  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStageSilu<FMT>{m, wt}, MoeDnMats<FMT, 1>{m});
 }
 
 template <int FMT, int NT>
-__global__ void __launch_bounds__(g2_warps<FMT>(8 * NT, moe_ntc<NT>() != NT) * 32, G2_CPSM) k_moe_dn(const GemmArgs a, const MoeArgs m, const int cps) {
+__global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_dn(const GemmArgs a, const MoeArgs m, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeDnMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, smem, G2StagePlanes<FMT, NT>{a}, MoeDnMats<FMT>{m});
+  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeDnMats<FMT, NT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                          G2StagePlanes<FMT, NT>{a}, MoeDnMats<FMT, NT>{m});
 }

@@ -43,9 +43,8 @@ __global__ void k_dequant_rows(int fmt, const uint8_t *__restrict__ W, int cols,
   pdl_wait();
   const int r = blockIdx.y;
   const int row = row_ids ? row_ids[r] : r;
-  const uint8_t *src = W + (size_t)row * dev_row_bytes(fmt, cols);
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x)
-    out[(size_t)r * cols + c] = deq_elem(fmt, src, cols, c);
+    out[(size_t)r * cols + c] = deq_elem(fmt, W, cols, row, c);
 }
 int ops_dequant_rows(cudaStream_t s, int fmt, const uint8_t *W, int rows, int cols, const int *row_ids, int nrows,
                      float *out) {
@@ -53,10 +52,10 @@ int ops_dequant_rows(cudaStream_t s, int fmt, const uint8_t *W, int rows, int co
   if (nrows < 1) return 0;
   int gx = (cols + 255) / 256;
   if (gx > 64) gx = 64;
-  // gridDim.y is limited to 65535 rows per launch
-  for (int r0 = 0; r0 < nrows; r0 += 65535) {
-    int n = nrows - r0 < 65535 ? nrows - r0 : 65535;
-    CU_OK(llb_launch(k_dequant_rows, dim3(gx, n), dim3(256), (size_t)(0), s, fmt, row_ids ? W : W + (size_t)r0 * dev_row_bytes(fmt, cols), cols,
+  // gridDim.y is limited to 65535 rows per launch; whole row tiles a launch, so that its first row starts one
+  for (int r0 = 0; r0 < nrows; r0 += 65520) {
+    int n = nrows - r0 < 65520 ? nrows - r0 : 65520;
+    CU_OK(llb_launch(k_dequant_rows, dim3(gx, n), dim3(256), (size_t)(0), s, fmt, row_ids ? W : W + dev_bytes(fmt, r0, cols), cols,
                                               row_ids ? row_ids + r0 : nullptr, out + (size_t)r0 * cols));
     CU_OK(cudaGetLastError());
   }
@@ -80,6 +79,66 @@ int ops_repack_q6k(cudaStream_t s, const uint8_t *src210, uint8_t *dst224, size_
   size_t n = nblocks * 224;
   int grid = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
   CU_OK(llb_launch(k_repack_q6k, dim3(grid), dim3(256), (size_t)(0), s, src210, dst224, nblocks));
+  CU_OK(cudaGetLastError());
+  return 0;
+}
+
+// ---- pack rows -> device tiles (common.cuh) ------------------------------------------------------
+// A block per tile; a thread moves two bytes at a time (a stored Q6_K block is only 2-byte aligned).  Runs once per
+// matrix, at load.
+__global__ void __launch_bounds__(256) k_to_tiles(int fmt, const uint8_t *__restrict__ src, int rows, int cols, unsigned short *__restrict__ dst) {
+  const int nsb = (cols + 255) >> 8, tb = tile_bytes(fmt), tr = tile_row(fmt);
+  const size_t prb = pack_row_bytes(fmt, cols);
+  for (size_t tile = blockIdx.x; tile < (size_t)((rows + 15) >> 4) * nsb; tile += gridDim.x) {
+    const int row0 = (int)(tile / nsb) * 16, sb = (int)(tile % nsb);
+    for (int i = threadIdx.x; i < tb / 2; i += blockDim.x) {
+      const int o = 2 * i;
+      int r = o / tr, b = o - r * tr;                      // row of the tile, byte of its block
+      if (fmt == LLB_FM_Q6_K && o >= 3328) { r = (o - 3328) >> 1; b = 208; }
+      unsigned short v = 0;
+      const uint8_t *p = src + (size_t)(row0 + r) * prb;
+      if (fmt == LLB_FM_Q8_0) {
+        if (b < 256) { if (row0 + r < rows && sb * 256 + b < cols) v = *(const unsigned short *)(p + sb * 256 + b); v ^= 0x8080; }
+        else if (row0 + r < rows && sb * 256 + 16 * (b - 256) < cols) v = *(const unsigned short *)(p + cols + sb * 16 + b - 256);
+      } else if (row0 + r < rows) {
+        v = *(const unsigned short *)(p + (size_t)sb * (prb / nsb) + b);
+      }
+      dst[tile * (tb / 2) + i] = v;
+    }
+  }
+}
+int ops_to_tiles(cudaStream_t s, int fmt, const uint8_t *src, int rows, int cols, uint8_t *dst) {
+  const size_t n = (size_t)((rows + 15) >> 4) * ((cols + 255) >> 8);
+  if (!n) return 0;
+  k_to_tiles<<<(unsigned)(n < 16384 ? n : 16384), 256, 0, s>>>(fmt, src, rows, cols, (unsigned short *)dst);
+  CU_OK(cudaGetLastError());
+  return 0;
+}
+// A range of rows and columns of one tiled matrix into another (a tensor-parallel rank's share): `n` rows from srow to
+// drow, `nc` columns from scol to dcol, in blocks of 256 columns (Q8_0: 32).  Called at load only.
+__global__ void __launch_bounds__(128) k_tile_slice(int fmt, const uint8_t *__restrict__ src, int scols, uint8_t *__restrict__ dst, int dcols, int srow, int drow,
+                                                    int scol, int dcol, int nc) {
+  const int tb = tile_bytes(fmt), tr = tile_row(fmt), unit = fmt == LLB_FM_Q8_0 ? 32 : 256;
+  const int rs = srow + blockIdx.x, rd = drow + blockIdx.x;
+  for (int u = 0; u < nc / unit; u++) {
+    const int cs = scol + u * unit, cd = dcol + u * unit;
+    const uint8_t *st = src + ((size_t)(rs >> 4) * ((scols + 255) >> 8) + (cs >> 8)) * tb;
+    uint8_t *dt = dst + ((size_t)(rd >> 4) * ((dcols + 255) >> 8) + (cd >> 8)) * tb;
+    const uint8_t *sr = st + (rs & 15) * tr;
+    uint8_t *dr = dt + (rd & 15) * tr;
+    if (fmt == LLB_FM_Q8_0) {
+      const int is = cs & 255, id = cd & 255;
+      if (threadIdx.x < 32) dr[id + threadIdx.x] = sr[is + threadIdx.x];
+      else if (threadIdx.x < 34) dr[256 + 2 * (id >> 5) + threadIdx.x - 32] = sr[256 + 2 * (is >> 5) + threadIdx.x - 32];
+    } else {
+      for (int i = threadIdx.x; i < tr; i += blockDim.x) dr[i] = sr[i];
+      if (fmt == LLB_FM_Q6_K && threadIdx.x < 2) dt[3328 + 2 * (rd & 15) + threadIdx.x] = st[3328 + 2 * (rs & 15) + threadIdx.x];
+    }
+  }
+}
+int ops_tile_slice(cudaStream_t s, int fmt, const uint8_t *src, int scols, uint8_t *dst, int dcols, int srow, int drow, int n, int scol, int dcol, int nc) {
+  if (n < 1 || nc < 1) return 0;
+  k_tile_slice<<<n, 128, 0, s>>>(fmt, src, scols, dst, dcols, srow, drow, scol, dcol, nc);
   CU_OK(cudaGetLastError());
   return 0;
 }

@@ -5,18 +5,9 @@
 #include <cooperative_groups.h>
 
 #include "model.cuh"
+#include "rowops.cuh"
 namespace cg = cooperative_groups;
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-  return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, m));
-  return v;
-}
 // sum over the block; every thread gets the result (red: >= 32 floats of shared memory)
 __device__ __forceinline__ float block_sum(float v, float *red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -41,8 +32,8 @@ __global__ void k_embed(int fmt, const uint8_t *__restrict__ W, int d, const Row
   const int t = blockIdx.y;
   rs = rs_begin_row(rs, sg, t, rs_n, rs_p0, tl);
   if (tl >= rs_n) return;
-  const uint8_t *row = W + (size_t)rs->tok[tl] * dev_row_bytes(fmt, d);
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d; c += gridDim.x * blockDim.x) x[(size_t)t * d + c] = deq_elem(fmt, row, d, c);
+  const int row = rs->tok[tl];
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d; c += gridDim.x * blockDim.x) x[(size_t)t * d + c] = deq_elem(fmt, W, d, row, c);
 }
 int op_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const RowSet *rs, int Tmax, float *x) {
   CU_OK(llb_launch(k_embed, dim3((d + 255) / 256, Tmax), dim3(256), (size_t)(0), s, fmt, W, d, rs, g_streams, x));
@@ -172,61 +163,8 @@ int op_silu_scaled_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, con
   return 0;
 }
 
-// ---- the router of a routed-expert layer (host/llb_host.c:622-724; llb_moe_topk of tools/payload-moeany.patch) ----
-// One warp per row of the pass: softmax over the ne logits, the k largest probabilities in descending order with
-// ties to the lower index, their weights divided by their sum clamped at 6.103515625e-5; slot k is the shared
-// expert (id ne) with weight sigmoid(its gate logit).
-template <int NQ> __device__ __forceinline__ void moe_route_row(const float *l, int ne, int nk, int *ids, float *wt, int lane) {
-  float p[NQ];   // experts lane, lane + 32, ...: ne <= 32 NQ
-  float mx = -INFINITY;
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int e = lane + 32 * q;
-    p[q] = e < ne ? __ldcg(l + e) : -INFINITY;
-    mx = fmaxf(mx, p[q]);
-  }
-  mx = warp_max(mx);
-  float sm = 0.0f;
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int e = lane + 32 * q;
-    if (e < ne) { p[q] = expf(p[q] - mx); sm += p[q]; }
-    else p[q] = -1.0f;
-  }
-  sm = warp_sum(sm);
-  const float inv = 1.0f / sm;
-#pragma unroll
-  for (int q = 0; q < NQ; q++)
-    if (p[q] >= 0.0f) p[q] *= inv;
-  float s = 0.0f, mine_w = 0.0f;   // lane j keeps the weight of rank j
-  int mine_id = 0;
-  for (int j = 0; j < nk; j++) {
-    float bv = -1.0f;
-    int bi = 0x7fffffff;
-#pragma unroll
-    for (int q = 0; q < NQ; q++)
-      if (p[q] > bv) { bv = p[q]; bi = lane + 32 * q; }   // ascending q: the lane's lowest index among equals
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, m);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, m);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if ((bi & 31) == lane) {
-#pragma unroll
-      for (int q = 0; q < NQ; q++)
-        if (q == (bi >> 5)) p[q] = -2.0f;
-    }
-    s += bv;
-    if (j == lane) { mine_w = bv; mine_id = bi; }
-  }
-  s = s < 6.103515625e-5f ? 6.103515625e-5f : s;
-  if (lane < nk) { ids[lane] = mine_id; wt[lane] = mine_w / s; }
-  if (lane == 0) {
-    ids[nk] = ne;
-    wt[nk] = 1.0f / (1.0f + expf(-__ldcg(l + ne)));
-  }
-}
+// ---- the router of a routed-expert layer (host/llb_host.c:622-724; llb_moe_topk of tools/payload-moeany.patch; the top k of a
+// row is moe_route_row, rowops.cuh) ----
 // Router logits lg[t][r] = W[r] . h[t] for the ne router rows and the shared expert's gate row (row ne): F32
 // weights, a block per row (every load of the row in flight at once), all rows of the pass.  The block that
 // finishes last (a counter, no waiting) then routes: its warp t takes row t of the pass.
@@ -304,11 +242,6 @@ int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne,
 // grid (H + 2 KV, Tmax), block hd.  q input rows are [H][q(hd) | gate(hd)].  The cache keeps a value as two
 // fp16 numbers in two planes kv_plane halves apart, hi = fp16(x) and lo = fp16((x - hi) * 2048): the bytes
 // of the f32, in the form the attention kernel's tensor-core operands take.
-__device__ __forceinline__ void kv_put(__half *c, long long plane, size_t i, float x) {
-  const __half h = __float2half_rn(x);
-  c[i] = h;
-  c[plane + i] = __float2half_rn((x - __half2float(h)) * XP_LO_SCALE);
-}
 __global__ void k_qkrope(PartIn q, PartIn k, PartIn v, const float *__restrict__ qn_w, const float *__restrict__ kn_w,
                          const double *__restrict__ invfreq, AttnShape sh, float *__restrict__ qout, __half *__restrict__ Kc,
                          __half *__restrict__ Vc, const RowSet *rs, Streams sg, int blk0) {
@@ -541,23 +474,6 @@ int op_delta_fused(cudaStream_t s, float *S, const SpecCtl *ctl, const float *y,
 
 // ---- top-2 over the logits (llb_t_amaxp / llb_t_amax, tools/payload-spec2.patch:450-483) ---------
 // Order: larger value first, lower id on equal values (tools/qwen35_engine.c:763-778).
-struct Top2 { float v1; int i1; float v2; int i2; };
-__device__ __forceinline__ bool t2_before(float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia < ib); }
-__device__ __forceinline__ void t2_push(Top2 &a, float v, int i) {
-  if (i < 0) return;
-  if (a.i1 < 0 || t2_before(v, i, a.v1, a.i1)) { a.v2 = a.v1; a.i2 = a.i1; a.v1 = v; a.i1 = i; }
-  else if (a.i2 < 0 || t2_before(v, i, a.v2, a.i2)) { a.v2 = v; a.i2 = i; }
-}
-__device__ __forceinline__ Top2 t2_warp(Top2 a) {
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1) {
-    float v1 = __shfl_xor_sync(0xffffffffu, a.v1, m), v2 = __shfl_xor_sync(0xffffffffu, a.v2, m);
-    int i1 = __shfl_xor_sync(0xffffffffu, a.i1, m), i2 = __shfl_xor_sync(0xffffffffu, a.i2, m);
-    t2_push(a, v1, i1);
-    t2_push(a, v2, i2);
-  }
-  return a;
-}
 __global__ void __launch_bounds__(256) k_top2_part(PartIn logits, int V, long long row_stride,
                                                    float *__restrict__ part, const RowSet *rs, Streams sg) {
   int rs_n, rs_p0, tl;

@@ -97,8 +97,8 @@ __global__ void k_pf_embed(int fmt, const uint8_t *__restrict__ W, int d, const 
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.y;
-  const uint8_t *row = W + (size_t)ids[t] * dev_row_bytes(fmt, d);
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d; c += gridDim.x * blockDim.x) x[(size_t)t * d + c] = deq_elem(fmt, row, d, c);
+  const int row = ids[t];
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d; c += gridDim.x * blockDim.x) x[(size_t)t * d + c] = deq_elem(fmt, W, d, row, c);
 }
 int op_pf_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const int *ids, int R, float *x) {
   CU_OK(llb_launch(k_pf_embed, dim3((d + 255) / 256, R), dim3(256), (size_t)0, s, fmt, W, d, ids, x));
@@ -353,7 +353,7 @@ extern "C" __attribute__((visibility("default")))
 int llb_b200_pf_gemm(int fmt, unsigned long long w, int rows, int K, unsigned long long x_f32, int R, unsigned long long out_f32, int ksplit) {
   if (!g_llb.stream) return llb_fail("llb_b200_init has not been called");
   if (K < 256 || K % 256 || rows < 1 || R < 1 || R > PF_RMAX) return llb_fail("pf_gemm: rows %d, K %d, R %d (K a multiple of 256, R up to %d)", rows, K, R, PF_RMAX);
-  if (!dev_row_bytes(fmt, K) || fmt == LLB_FM_F32) return llb_fail("pf_gemm: format %d has no kernel", fmt);
+  if (!tile_bytes(fmt)) return llb_fail("pf_gemm: format %d has no kernel", fmt);
   if (pf_setup()) return -1;
   const int nsb = K / 256;
   if (ksplit <= 0) ksplit = pf_pick_ksplit((rows + 127) / 128, nsb, g_llb.sms);

@@ -4,7 +4,7 @@
 
 #define PF_MAXMAT 4
 struct PfMat {
-  const uint8_t *W;     // device layout, row stride dev_row_bytes(fmt, K)
+  const uint8_t *W;     // device layout (common.cuh)
   float *out;           // [ksplit][PF rows][ostride]
   int rows, ostride;
   long long split_stride;

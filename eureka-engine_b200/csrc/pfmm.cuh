@@ -59,23 +59,24 @@ __device__ __forceinline__ void pf_bulk_copy(uint32_t dst_s, const void *src, ui
 // values with pf_deq, then pf_split8 turns every eight of them into a 16-byte row of each plane (k-groups c0/8 .. + 3).
 struct PfRaw { uint32_t w[8], x[8], h[4]; };
 
-template <int FMT> __device__ __forceinline__ void pf_load(const uint8_t *row, int K, int c0, PfRaw &r) {
+// row: the row's block in the first super-block of its row tile;  doff: from there to the row's d (Q6_K)
+template <int FMT> __device__ __forceinline__ void pf_load(const uint8_t *row, int doff, int c0, PfRaw &r) {
+  const uint8_t *blk = row + (size_t)(c0 >> 8) * tile_bytes(FMT);
   if constexpr (FMT == LLB_FM_Q8_0) {
-    const uint4 a = ldg128(row + c0), b = ldg128(row + c0 + 16);
+    const int i = c0 & 255;
+    const uint4 a = ldg128(blk + i), b = ldg128(blk + i + 16);
     r.w[0] = a.x; r.w[1] = a.y; r.w[2] = a.z; r.w[3] = a.w; r.w[4] = b.x; r.w[5] = b.y; r.w[6] = b.z; r.w[7] = b.w;
-    r.h[0] = *(const unsigned short *)(row + K + 2 * (c0 >> 5));
+    r.h[0] = *(const unsigned short *)(blk + 256 + 2 * (i >> 5));
   } else if constexpr (FMT == LLB_FM_Q6_K) {
-    const uint8_t *blk = row + (size_t)(c0 >> 8) * 224;
     const int j8 = (c0 >> 5) & 7, hf = j8 >> 2, qd = j8 & 3;
     const uint4 a = ldg128(blk + 64 * hf + 32 * (qd & 1)), b = ldg128(blk + 64 * hf + 32 * (qd & 1) + 16);
     const uint4 c = ldg128(blk + 128 + 32 * hf), d = ldg128(blk + 128 + 32 * hf + 16);
     r.w[0] = a.x; r.w[1] = a.y; r.w[2] = a.z; r.w[3] = a.w; r.w[4] = b.x; r.w[5] = b.y; r.w[6] = b.z; r.w[7] = b.w;
     r.x[0] = c.x; r.x[1] = c.y; r.x[2] = c.z; r.x[3] = c.w; r.x[4] = d.x; r.x[5] = d.y; r.x[6] = d.z; r.x[7] = d.w;
     r.h[0] = *(const unsigned short *)(blk + 192 + 8 * hf + 2 * qd);   // the two int8 scales of this quarter
-    r.h[1] = *(const unsigned short *)(blk + 208);
+    r.h[1] = *(const unsigned short *)(blk + doff);
   } else {
-    constexpr int SB = FMT == LLB_FM_Q4_K ? 144 : 176, QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
-    const uint8_t *blk = row + (size_t)(c0 >> 8) * SB;
+    constexpr int QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
     const int g = (c0 >> 6) & 3;
     const uint4 hd = ldg128(blk), a = ldg128(blk + QOFF + 32 * g), b = ldg128(blk + QOFF + 32 * g + 16);
     r.h[0] = hd.x; r.h[1] = hd.y; r.h[2] = hd.z; r.h[3] = hd.w;
@@ -103,7 +104,7 @@ template <int FMT> __device__ __forceinline__ void pf_deq(const PfRaw &r, int c0
     const float d = h2f_bits(r.h[0]), c = -384.0f * d;     // byte = q + 128, float = 256 + byte
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const uint32_t x = r.w[i] ^ 0x80808080u;
+      const uint32_t x = r.w[i];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const uint32_t v = j == 0 ? x << 15 : j == 1 ? x << 7 : j == 2 ? x >> 1 : x >> 9;
@@ -183,7 +184,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
   uint8_t *ring = smem + 1024;
   const uint32_t ring_s = smem_u32(ring);
   const int ntiles = a.t128[a.nmat], nunits = ntiles * a.ksplit;
-  const size_t rb = dev_row_bytes(FMT, a.K);
   const int nun = a.R > PF_R ? 2 : 1;   // units of PF_R rows in this chunk
 
   pdl_trigger();
@@ -216,16 +216,19 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
     // the loads run two stages ahead of the conversion: cursor (lu, ls) is the stage to load next
     int lu = blockIdx.x, ls = 0, lkbase = 0, lnst = 0, lm = 0, lrow0 = 0;
     const uint8_t *lrow = nullptr;
+    int ldoff = 0;
     auto lplan = [&]() {
       if (lu < nunits) {
         pf_locate(a, lu % ntiles, lm, lrow0);
         pf_slice(a, lu, ntiles, lkbase, lnst);
-        lrow = a.m[lm].W + (size_t)min(lrow0 + r, a.m[lm].rows - 1) * rb;
+        const int row = min(lrow0 + r, a.m[lm].rows - 1);
+        lrow = a.m[lm].W + (size_t)(row >> 4) * (a.K >> 8) * tile_bytes(FMT) + (row & 15) * tile_row(FMT);
+        ldoff = 3328 + 2 * (row & 15) - (row & 15) * 208;
       }
     };
     auto lnext = [&](PfRaw &dst) {
       if (lu < nunits) {
-        pf_load<FMT>(lrow, a.K, lkbase + ls * PF_KS + 32 * h, dst);
+        pf_load<FMT>(lrow, ldoff, lkbase + ls * PF_KS + 32 * h, dst);
         if (++ls == lnst) { ls = 0; lu += gridDim.x; lplan(); }
       }
     };
