@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm,
   if (lane == 0) red[i >> 5] = M;
   __syncthreads();
   M = red[0];
+#pragma unroll 1
   for (int k = 1; k < (blockDim.x >> 5); k++) M = fmaxf(M, red[k]);
   const float wgt = (i < nact && m != -INFINITY) ? expf(m - M) : 0.0f;
   if (i < 128) wsm[i] = wgt;
@@ -256,11 +257,13 @@ __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm,
   if (lane == 0) red[i >> 5] = L;
   __syncthreads();   // (wsm is visible after it too)
   L = 0.0f;
+#pragma unroll 1
   for (int k = 0; k < (blockDim.x >> 5); k++) L += red[k];
   const int hd4 = hd >> 2, ng = blockDim.x / hd4, sg = i / hd4, i4 = i - sg * hd4;   // ng split groups of hd/4 threads
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   if (sg < ng) {
     // split s = sg + ng*j: four loads in flight per trip, added in split order within the group
+#pragma unroll 1
     for (int s0 = sg; s0 < nact; s0 += 4 * ng) {
       float4 v[4];
       float ws[4];
@@ -278,8 +281,10 @@ __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm,
   __syncthreads();
   if (i < hd4) {   // a multiple of 8 threads: eight lanes per 32 dims
     float4 a = *(const float4 *)&osm[4 * i];
+#pragma unroll 1
     for (int g = 1; g < ng; g++) { const float4 b = *(const float4 *)&osm[g * hd + 4 * i]; a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
-    const float4 gate = part_get4(qg, (size_t)t * 2 * sh.H * hd + (size_t)h * 2 * hd + hd + 4 * i);
+    float4 gate = make_float4(0.f, 0.f, 0.f, 0.f);
+    p_parts4(qg, (size_t)t * 2 * sh.H * hd + (size_t)h * 2 * hd + hd + 4 * i, gate);
     const float hv[4] = {(a.x / L) / (1.0f + expf(-gate.x)), (a.y / L) / (1.0f + expf(-gate.y)), (a.z / L) / (1.0f + expf(-gate.z)),
                          (a.w / L) / (1.0f + expf(-gate.w))};
     // the prompt path takes the rows as fp16 in the dense GEMM's k-group-major order instead of the T-row planes

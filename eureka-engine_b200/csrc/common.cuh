@@ -51,28 +51,22 @@ __host__ __device__ inline size_t pack_row_bytes(int fmt, int cols) {
 // rows (bf16/fp16 inputs that need no second plane).
 //   xh   [NC][K]    fp16, K-index permuted inside every aligned group of 8: stored order
 //                   0 2 1 3 4 6 5 7, which is the order the tensor-core B fragments consume
-//   xs16 [K/16][NC] f32 sums of the fp16 values over 16 consecutive columns
-//   xs32 [K/32][NC] f32 sums over 32 consecutive columns
 //   xsf  [K/256][NC][16] fp16: the eight 32-column MEANS of a super-block as hi/lo pairs (hi = fp16(m),
 //                   lo = fp16((m - hi) * 2048), like the planes), in the order the min-term MMA's B fragment
 //                   reads them: for j = 0..3: hi(2j) hi(2j+1) lo(2j) lo(2j+1)
 struct XPlanes {
   __half *xh;
-  float *xs16;
-  float *xs32;
   __half *xsf;
   int K;
   int NC;
 };
 __host__ __device__ inline size_t xp_bytes(int K, int NC) {
-  return (size_t)NC * K * 2 + (size_t)(K / 16) * NC * 4 + (size_t)(K / 32) * NC * 4 + (size_t)(K / 256) * NC * 32;
+  return (size_t)NC * K * 2 + (size_t)(K / 256) * NC * 32;
 }
 __host__ __device__ inline XPlanes xp_carve(void *base, int K, int NC) {
   char *b = (char *)base;
   XPlanes xp;
   xp.xh = (__half *)b; b += (size_t)NC * K * 2;
-  xp.xs16 = (float *)b; b += (size_t)(K / 16) * NC * 4;
-  xp.xs32 = (float *)b; b += (size_t)(K / 32) * NC * 4;
   xp.xsf = (__half *)b;
   xp.K = K; xp.NC = NC;
   return xp;
@@ -82,90 +76,33 @@ __host__ __device__ inline XPlanes xp_carve(void *base, int K, int NC) {
 
 __host__ __device__ inline int xp_perm(int c) { return (c & ~7) | ((c & 4) | ((c & 1) << 1) | ((c & 2) >> 1)); }
 
-// Warp-cooperative store of 32 consecutive columns (lane = column c0 + lane) of row t.
-__device__ __forceinline__ void xp_store32(const XPlanes &xp, int t, int planes, int c0, float v, int lane) {
-  int c = c0 + lane, NH = xp.NC >> 1;
-  __half hi = __float2half_rn(v);
-  float hif = __half2float(hi);
-  float lof = 0.0f;
-  xp.xh[(size_t)t * xp.K + xp_perm(c)] = hi;
-  if (planes == 2) {
-    __half lo = __float2half_rn((v - hif) * XP_LO_SCALE);
-    lof = __half2float(lo);
-    xp.xh[(size_t)(NH + t) * xp.K + xp_perm(c)] = lo;
-  }
-#pragma unroll
-  for (int m = 1; m < 16; m <<= 1) {
-    hif += __shfl_xor_sync(0xffffffffu, hif, m);
-    lof += __shfl_xor_sync(0xffffffffu, lof, m);
-  }
-  float hi32 = hif + __shfl_xor_sync(0xffffffffu, hif, 16);
-  float lo32 = lof + __shfl_xor_sync(0xffffffffu, lof, 16);
-  if ((lane & 15) == 0) {
-    xp.xs16[(size_t)(c >> 4) * xp.NC + t] = hif;
-    if (planes == 2) xp.xs16[(size_t)(c >> 4) * xp.NC + NH + t] = lof;
-  }
-  if (lane == 0) {
-    xp.xs32[(size_t)(c >> 5) * xp.NC + t] = hi32;
-    if (planes == 2) xp.xs32[(size_t)(c >> 5) * xp.NC + NH + t] = lo32;
-    const int b = (c >> 5) & 7;
-    __half *f = xp.xsf + ((size_t)(c >> 8) * xp.NC + t) * 16 + 4 * (b >> 1) + (b & 1);
-    float v = hi32 * 0.03125f;
-    __half h1 = __float2half_rn(v);
-    f[0] = h1; f[2] = __float2half_rn((v - __half2float(h1)) * XP_LO_SCALE);
-    if (planes == 2) {
-      f += (size_t)NH * 16;
-      v = lo32 * 0.03125f;
-      h1 = __float2half_rn(v);
-      f[0] = h1; f[2] = __float2half_rn((v - __half2float(h1)) * XP_LO_SCALE);
-    }
-  }
-}
-
-// The same for a thread that holds FOUR consecutive columns c .. c+3 (c a multiple of 4) of row t; the eight
-// lanes 8j .. 8j+7 of a warp must hold one aligned group of 32 columns.  `on` is false for a thread past
-// the row's end (it still takes part in the shuffles).  Stored order inside the four: 0 2 1 3.
+// Four consecutive columns c .. c+3 (c a multiple of 4) of row t into the planes and the sub-block means; the eight lanes
+// 8 j .. 8 j + 7 of a warp hold one aligned group of 32 columns.  `on` is false for a thread past the row's end (it still
+// takes part in the shuffles).  Stored order inside the four: 0 2 1 3.  (Kept short: the kernels that end with it run for a
+// microsecond or two, and instructions that the SM does not hold come from L2.)
 __device__ __forceinline__ void xp_store4(const XPlanes &xp, int t, int planes, int c, const float (&v)[4], int lane, bool on) {
-  const int NH = xp.NC >> 1;
-  __half hi[4];
-  float hs = 0.0f, ls = 0.0f, hif[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) { hi[i] = __float2half_rn(on ? v[i] : 0.0f); hif[i] = __half2float(hi[i]); hs += hif[i]; }
-  if (on) {
-    const __half2 a = __halves2half2(hi[0], hi[2]), b = __halves2half2(hi[1], hi[3]);
-    *(uint2 *)(xp.xh + (size_t)t * xp.K + c) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
-  }
+  const __half2 a = __floats2half2_rn(on ? v[0] : 0.0f, on ? v[2] : 0.0f), b = __floats2half2_rn(on ? v[1] : 0.0f, on ? v[3] : 0.0f);
+  const float2 af = __half22float2(a), bf = __half22float2(b);
+  float hs = ((af.x + bf.x) + af.y) + bf.y, ls = 0.0f;
+  __half *x = xp.xh + (size_t)t * xp.K + c;
+  if (on) *(uint2 *)x = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
   if (planes == 2) {
-    __half lo[4];
+    const __half2 e = __floats2half2_rn(on ? (v[0] - af.x) * XP_LO_SCALE : 0.0f, on ? (v[2] - af.y) * XP_LO_SCALE : 0.0f);
+    const __half2 f = __floats2half2_rn(on ? (v[1] - bf.x) * XP_LO_SCALE : 0.0f, on ? (v[3] - bf.y) * XP_LO_SCALE : 0.0f);
+    const float2 ef = __half22float2(e), ff = __half22float2(f);
+    ls = ((ef.x + ff.x) + ef.y) + ff.y;
+    if (on) *(uint2 *)(x + (size_t)(xp.NC >> 1) * xp.K) = make_uint2(*(const uint32_t *)&e, *(const uint32_t *)&f);
+  }
 #pragma unroll
-    for (int i = 0; i < 4; i++) { lo[i] = __float2half_rn(on ? (v[i] - hif[i]) * XP_LO_SCALE : 0.0f); ls += __half2float(lo[i]); }
-    if (on) {
-      const __half2 a = __halves2half2(lo[0], lo[2]), b = __halves2half2(lo[1], lo[3]);
-      *(uint2 *)(xp.xh + (size_t)(NH + t) * xp.K + c) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
-    }
-  }
-  hs += __shfl_xor_sync(0xffffffffu, hs, 1); ls += __shfl_xor_sync(0xffffffffu, ls, 1);
-  hs += __shfl_xor_sync(0xffffffffu, hs, 2); ls += __shfl_xor_sync(0xffffffffu, ls, 2);
-  const float h32 = hs + __shfl_xor_sync(0xffffffffu, hs, 4), l32 = ls + __shfl_xor_sync(0xffffffffu, ls, 4);
-  if (!on) return;
-  if ((lane & 3) == 0) {
-    xp.xs16[(size_t)(c >> 4) * xp.NC + t] = hs;
-    if (planes == 2) xp.xs16[(size_t)(c >> 4) * xp.NC + NH + t] = ls;
-  }
-  if ((lane & 7) == 0) {
-    xp.xs32[(size_t)(c >> 5) * xp.NC + t] = h32;
-    if (planes == 2) xp.xs32[(size_t)(c >> 5) * xp.NC + NH + t] = l32;
-    const int b = (c >> 5) & 7;
-    __half *f = xp.xsf + ((size_t)(c >> 8) * xp.NC + t) * 16 + 4 * (b >> 1) + (b & 1);
-    float m = h32 * 0.03125f;
-    __half h1 = __float2half_rn(m);
-    f[0] = h1; f[2] = __float2half_rn((m - __half2float(h1)) * XP_LO_SCALE);
-    if (planes == 2) {
-      f += (size_t)NH * 16;
-      m = l32 * 0.03125f;
-      h1 = __float2half_rn(m);
-      f[0] = h1; f[2] = __float2half_rn((m - __half2float(h1)) * XP_LO_SCALE);
-    }
+  for (int m = 1; m < 8; m <<= 1) { hs += __shfl_xor_sync(0xffffffffu, hs, m); ls += __shfl_xor_sync(0xffffffffu, ls, m); }
+  // lane 0 of the eight writes the hi plane's mean, lane 1 the lo plane's: each as an fp16 hi / rest pair
+  if (on && (lane & 7) < planes) {
+    const bool second = lane & 1;
+    const int b32 = (c >> 5) & 7;
+    const float m = (second ? ls : hs) * 0.03125f;
+    const __half h1 = __float2half_rn(m);
+    __half *p = xp.xsf + ((size_t)(c >> 8) * xp.NC + t + (second ? xp.NC >> 1 : 0)) * 16 + 4 * (b32 >> 1) + (b32 & 1);
+    p[0] = h1; p[2] = __float2half_rn((m - __half2float(h1)) * XP_LO_SCALE);
   }
 }
 

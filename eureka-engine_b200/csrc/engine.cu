@@ -72,7 +72,7 @@ struct llb_spec {
   float rope_base = 1e7f, eps = 1e-6f;
   int ne = 0, nk = 0, ef = 0, sf = 0;   // routed experts, experts per token, expert width, shared expert width (ne = 0: dense FFN)
   float *moe_lg = nullptr, *moe_wt = nullptr, *moe_g = nullptr, *moe_u = nullptr, *hn2 = nullptr;
-  int *moe_ids = nullptr;
+  int *moe_ids = nullptr, *moe_live = nullptr;   // moe_live: how many rows of the pass are in use, then which
   XPlanes xp_e;
   size_t pack_bytes = 0;   // size of the pack the index describes: every tensor range is checked against it
   int k = 0, Tmax = 1, R = 2, max_ctx = 0, NC = 8;   // Tmax / NC: rows and plane columns of the pass being enqueued
@@ -81,7 +81,6 @@ struct llb_spec {
   // rings and host mirrors are arrays of B.  B = 1: per = the pass's width, as before.
   int B = 1, per = 1;
   long long kv_group = 0, s_group = 0, ring_group_unit = 0;   // halves between the streams' K (V) caches; floats between their state rings
-  int *const_rows = nullptr;   // device word holding B x per (the routed-expert launches' row count in a multi-stream pass)
   // A speculative pass has k + 1 rows; a prompt chunk has Tpf rows (8 where the attention kernel's query budget allows:
   // the weights stream once per pass whatever its rows, so a wider chunk halves the prompt's time).  The two widths
   // share every buffer; the planes have one view per column count.
@@ -128,11 +127,14 @@ struct llb_spec {
   // activations
   float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *beta = nullptr, *decay = nullptr,
         *logits = nullptr, *t2part = nullptr, *pm = nullptr, *pl = nullptr, *po = nullptr;
+  // the trunk's normed rows that the drafter pairs with: hn after a speculative pass (stream b's from row b * Tspec), hn_pf after a
+  // prompt pass (from row b * Tpf); one buffer where there is one stream
+  float *hn_pf = nullptr;
   float *mt_x = nullptr, *mt_hn = nullptr, *chain_h = nullptr, *mt_logits = nullptr;
   XPlanes xp_d, xp_f, xp_qa, xp_v, xp_2d;
   OutBuf b_q, b_k, b_v, b_z, b_bp, b_ap, b_a, b_g, b_u, b_dn, b_eh, b_lg, b_mlg, b_ring;
   int att_split = 1;
-  int att_min = 96;                   // fewest positions per attention block (three 32-position tiles)
+  int att_min = 32;                   // fewest positions per attention block: one 32-position tile (three of them took 6 us longer a layer at a context of 100)
   // tensor parallel (tp.cu): the dimensions above are this rank's share once the model is open; the full ones are kept
   // for slicing.  r_a / r_dn: the out-projections' [T, d] tiles summed over K-slices and ranks.
   TpPlan tp = {0, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -162,7 +164,7 @@ static inline int *hist_of(const llb_spec *m, int b) { return m->hist ? m->hist 
 struct StreamScope {
   Streams was;
   explicit StreamScope(const llb_spec *m, bool single = false) : was(ops_streams()) {
-    if (m->B > 1 && !single) ops_set_streams(m->Tspec, (int)sizeof(SpecCtl)); else ops_set_streams(0, 0);
+    if (m->B > 1 && !single) ops_set_streams(m->per, (int)sizeof(SpecCtl)); else ops_set_streams(0, 0);
   }
   ~StreamScope() { ops_set_streams(was.per, was.stride); }
 };
@@ -211,7 +213,7 @@ static void *walloc(llb_spec *m, size_t bytes, bool *fresh) {
 }
 // plane columns of a pass of T rows (hi and lo halves): 8, 16 or 32
 static int nc_of(int T) { return T <= 4 ? 8 : T <= 8 ? 16 : 32; }
-static int rows_cap(const llb_spec *m) { const int a = m->B * m->Tspec, b = m->Tpf; return a > b ? a : b; }
+static int rows_cap(const llb_spec *m) { const int a = m->Tspec, b = m->Tpf; return m->B * (a > b ? a : b); }
 static int xp_alloc(llb_spec *m, int which, int K) {
   const int ncmax = nc_of(rows_cap(m));
   void *b = dalloc(m, xp_bytes(K, ncmax));
@@ -224,7 +226,7 @@ static int xp_alloc(llb_spec *m, int which, int K) {
 // the width of the passes enqueued from here on: T rows in all, `per` of them to a stream
 static void set_width(llb_spec *m, int T) {
   m->Tmax = T; m->NC = nc_of(T);
-  m->per = m->B > 1 ? m->Tspec : T;
+  m->per = T / m->B;
   const XPlanes *v = m->xpv[m->NC == 8 ? 0 : m->NC == 16 ? 1 : 2];
   m->xp_d = v[0]; m->xp_f = v[1]; m->xp_qa = v[2]; m->xp_v = v[3]; m->xp_2d = v[4]; m->xp_e = v[5];
 }
@@ -571,11 +573,10 @@ static int enq_moe_ffn(llb_spec *m, const FfnW &w, const float *xin, float *x1, 
 static int enq_moe_core(llb_spec *m, const FfnW &w, const RowSet *rs) {
   cudaStream_t s = g_llb.stream;
   const int ns = m->nk + 1, fe = ns * m->ef;
-  const int *n_rows = m->B > 1 ? m->const_rows : &((const RowSet *)((uintptr_t)rs & ~(uintptr_t)1))->n;
-  PK("moe route", op_moe_route(s, w.router, m->hn2, m->d, m->ne, m->nk, m->moe_lg, m->moe_ids, m->moe_wt, rs, m->Tmax));
+  PK("moe route", op_moe_route(s, w.router, m->hn2, m->d, m->ne, m->nk, m->moe_lg, m->moe_ids, m->moe_wt, m->moe_live, rs, m->Tmax));
   MoeArgs a;
   memset(&a, 0, sizeof a);
-  a.ids = m->moe_ids; a.nslot = ns; a.ne = m->ne; a.ef = m->ef; a.d = m->d; a.T = m->Tmax; a.n_rows = n_rows;
+  a.ids = m->moe_ids; a.nslot = ns; a.ne = m->ne; a.ef = m->ef; a.d = m->d; a.T = m->Tmax; a.live = m->moe_live;
   a.W = w.gu; a.es = w.es_gu; a.g = m->moe_g; a.u = m->moe_u;
   int one = 1;
   PK("moe gate|up", gemm_launch_moe(s, w.fmt_gu, false, m->xp_d, a, &one, nullptr));
@@ -623,15 +624,14 @@ static int enq_delta(llb_spec *m, const DeltaW &w, float *ring, int ring_ks, flo
   PK("gemm qkv|z|b|a", site_gemm(m, {{&w.qkv, &m->b_ring, &m->ctl->verify.slot[0], ring, m->convd, (long long)CONV_RING * m->convd, ring_ks, ring_ks},
                    {&w.z, &m->b_z, nullptr, nullptr, 0}, {&w.beta, &m->b_bp, nullptr, nullptr, 0}, {&w.alpha, &m->b_ap, nullptr, nullptr, 0}},
                m->xp_d, 0));
-  PK("delta conv", op_delta_conv(s, as_in(m->b_ring), w.conv, as_in(m->b_bp), as_in(m->b_ap), w.dt, w.a, sh, m->y, m->beta, m->decay, rs, m->Tmax));
-  PK("delta scan+gnorm", op_delta_fused(s, S, m->ctl, m->y, m->beta, m->decay, as_in(m->b_z), w.norm, sh, m->xp_v, rs, m->B, m->s_group));
+  PK("delta", op_delta(s, S, m->ctl, as_in(m->b_ring), w.conv, as_in(m->b_bp), as_in(m->b_ap), w.dt, w.a, as_in(m->b_z), w.norm, sh, m->xp_v, rs, m->B, m->s_group));
   PK("gemm ssm_out", site_gemm(m, {{&w.out, &m->b_a, nullptr, nullptr, 0}}, m->xp_v, 0));
   PK("all-reduce", tp_reduce(m, m->b_a, m->r_a));
   return 0;
 }
 
 // the (k+1)-row verify pass (spec_rows, host/llb_host.c:1714-1769)
-static int enq_verify(llb_spec *m) {
+static int enq_verify(llb_spec *m, float *hn) {
   cudaStream_t s = g_llb.stream;
   // the verify rows were set before this pass began (k_accept of the previous cycle, or the host for a
   // prompt chunk): kernels may read them ahead of their wait
@@ -647,7 +647,7 @@ static int enq_verify(llb_spec *m) {
     else CK(enq_delta(m, l.dn, m->ring[il], m->ring_ks[il], m->S[il], rs));
     CK(enq_ffn(m, l.ffn, m->x, m->x1, rs));
   }
-  PK("norm out", op_norm_xp(s, m->x1, in_dn(m), m->out_norm, m->eps, m->d, m->x, m->xp_d, 0, m->hn, rs, m->Tmax, 0));
+  PK("norm out", op_norm_xp(s, m->x1, in_dn(m), m->out_norm, m->eps, m->d, m->x, m->xp_d, 0, hn, rs, m->Tmax, 0));
   PK("gemm head", site_gemm(m, {{&m->head, &m->b_lg, nullptr, nullptr, 0}}, m->xp_d, 0));
   PK("top2", op_top2_part(s, as_in(m->b_lg), m->V, m->V, m->t2part, rs, m->Tmax));
   return 0;
@@ -665,30 +665,40 @@ static int enq_mtp(llb_spec *m, const RowSet *rs, const float *h, bool with_head
   CK(site_gemm(m, {{&m->mt_eh, &m->b_eh, nullptr, nullptr, 0}}, m->xp_2d, 0));
   // x = eh_proj [e ; h]; normed by attn_norm into the planes; x itself kept in mt_x
   CK(op_norm_xp(s, nullptr, as_in(m->b_eh), m->mt_attn_norm, m->eps, m->d, m->mt_x, m->xp_d, 0, nullptr, rs, m->Tmax, 0));
+  if (!with_head) {   // rows whose head is not asked for leave nothing but their K and V rows
+    const AttnW &w = m->mt_at;
+    AttnShape sh{m->H, m->KV, m->hd, m->rope_dim, m->eps, m->att_min, (long long)m->max_ctx * m->KV * m->hd, m->B > 1 ? (int)sizeof(SpecCtl) : 0, m->B > 1 ? m->kv_group : 0};
+    CK(site_gemm(m, {{&w.k, &m->b_k, nullptr, nullptr, 0}, {&w.v, &m->b_v, nullptr, nullptr, 0}}, m->xp_d, 0));
+    return op_qkrope(s, none, as_in(m->b_k), as_in(m->b_v), w.qn, w.kn, m->invfreq, sh, m->qn, m->mt_Kc, m->mt_Vc, rs, m->Tmax, true);
+  }
   CK(enq_attn(m, m->mt_at, m->mt_Kc, m->mt_Vc, rs));
   CK(enq_ffn(m, m->mt_ffn, m->mt_x, m->x1, rs));
   CK(op_norm_xp(s, m->x1, in_dn(m), m->mt_shn, m->eps, m->d, nullptr, m->xp_d, 0, m->mt_hn, rs, m->Tmax, 0));
-  if (with_head) {
-    CK(site_gemm(m, {{&m->mt_head, &m->b_mlg, nullptr, nullptr, 0}}, m->xp_d, 0));
-    CK(op_top2_part(s, as_in(m->b_mlg), m->mt_nv, m->mt_nv, m->t2part + t2_mtp(m), rs, m->Tmax));
-  }
-  return 0;
+  CK(site_gemm(m, {{&m->mt_head, &m->b_mlg, nullptr, nullptr, 0}}, m->xp_d, 0));
+  return op_top2_part(s, as_in(m->b_mlg), m->mt_nv, m->mt_nv, m->t2part + t2_mtp(m), rs, m->Tmax);
 }
 
 static int enq_cycle(llb_spec *m, bool spec) {
   cudaStream_t s = g_llb.stream;
+  float *hn = spec ? m->hn : m->hn_pf;
   if (m->has_mtp) {
     // catch-up over the rows the previous cycle served; the hidden at position 0 is zero
     // (host/llb_host.c:1815-1817); in a speculative cycle its last row's head gives draft 1
-    CK(enq_mtp(m, &m->ctl->catchup, m->hn, spec && m->k > 0, 0));
+    CK(enq_mtp(m, &m->ctl->catchup, hn, spec && m->k > 0, 0));
     if (spec) {
       for (int j = 1; j <= m->k; j++) {
         CK(op_draft_pick(s, m->t2part + t2_mtp(m), m->mt_ids, m->ctl, j > 1, j, m->mt_hn, m->chain_h, m->d, m->B, m->B > 1 ? m->per : 0));
-        if (j < m->k) CK(enq_mtp(m, &m->ctl->chain, m->chain_h, true, 0));
+        if (j < m->k) {   // one stream's chained row is a pass of one row: one n-tile whatever k is, and two plane columns to stage
+          const int width = m->Tmax;
+          if (m->B == 1) set_width(m, 1);
+          const int rc = enq_mtp(m, &m->ctl->chain, m->chain_h, true, 0);
+          set_width(m, width);
+          if (rc) return rc;
+        }
       }
     }
   }
-  CK(enq_verify(m));
+  CK(enq_verify(m, hn));
   // sampling mode (speculative cycles only: a prompt chunk's rows are given): every row's emitted token from its logits
   const bool smp = spec && m->smp_on;
   if (smp) CK(op_smp_rows(s, m->smp, as_in(m->b_lg), m->V, m->smp_adj, m->ctl, m->Tmax, nullptr, nullptr, nullptr, nullptr, m->smp_tok, m->smp_val, nullptr,
@@ -706,7 +716,7 @@ static int capture(llb_spec *m, int which, cudaGraphExec_t *out, size_t *nodes) 
   CU_OK(cudaStreamSynchronize(s));
   StreamScope scope(m);
   CU_OK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  int rc = which == 2 ? enq_verify(m) : enq_cycle(m, which == 0);
+  int rc = which == 2 ? enq_verify(m, m->hn) : enq_cycle(m, which == 0);
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (rc) { if (g) cudaGraphDestroy(g); return -1; }
   if (e != cudaSuccess) return llb_fail("graph capture: %s", cudaGetErrorString(e));
@@ -804,7 +814,8 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
     if (e && atoi(e) >= 1 && atoi(e) <= SPEC_MAXT) pf = atoi(e);
     if (pf > 48 / (m->H / m->KV)) pf = 48 / (m->H / m->KV);
     m->Tpf = pf > m->Tspec ? pf : m->Tspec;
-    if (m->B > 1) m->Tpf = m->Tspec;     // several streams: a stream's prompt chunk is as wide as its speculative pass
+    // several streams: the sixteen rows of a pass shared out among them (eight streams of plain decoding feed two rows each)
+    if (m->B > 1) { const int share = 16 / m->B < pf ? 16 / m->B : pf; m->Tpf = share > m->Tspec ? share : m->Tspec; }
   }
   m->per = m->Tpf;
   m->Tmax = rows_cap(m);                 // buffers are sized for the widest pass
@@ -867,7 +878,7 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
         // the launch attn_qkv lands in: the matrices of its format among qkv | z | beta | alpha
         int ntiles = 0;
         for (const DevMat *w : {&l.dn.qkv, &l.dn.z, &l.dn.beta, &l.dn.alpha}) if (w->fmt == l.dn.qkv.fmt) ntiles += (w->rows + 15) / 16;
-        const int ks = gemm_ring_ksplit(l.dn.qkv.fmt, d / 256, ntiles, nc_of(B * m->Tspec), nc_of(B > 1 ? B * m->Tspec : m->Tpf), g_llb.sms, RING_MAXSPLIT);
+        const int ks = gemm_ring_ksplit(l.dn.qkv.fmt, d / 256, ntiles, nc_of(B * m->Tspec), nc_of(B * m->Tpf), g_llb.sms, RING_MAXSPLIT);
         if (ks < 1) return llb_fail("blk.%d.attn_qkv: %d columns need more than %d K-slices at a pass width in use", il, d, RING_MAXSPLIT);
         m->ring_ks[il] = ks;
       }
@@ -984,7 +995,7 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
   // activations
   int big = m->f > m->convd ? m->f : m->convd;
   const int Tc = T > SPEC_MAXT ? T : SPEC_MAXT;
-  m->x = falloc(m, (size_t)T * d); m->x1 = falloc(m, (size_t)T * d); m->hn = falloc(m, (size_t)Tc * d); m->e = falloc(m, (size_t)T * d);
+  m->x = falloc(m, (size_t)T * d); m->x1 = falloc(m, (size_t)T * d); m->hn = falloc(m, (size_t)Tc * d); m->hn_pf = B > 1 ? falloc(m, (size_t)Tc * d) : m->hn; m->e = falloc(m, (size_t)T * d);
   m->qn = falloc(m, (size_t)T * qa); m->y = falloc(m, (size_t)T * big); m->beta = falloc(m, (size_t)T * m->TR); m->decay = falloc(m, (size_t)T * m->TR);
   m->t2part = falloc(m, (size_t)2 * Tc * TOP2_NB * 4);
   m->mt_x = falloc(m, (size_t)T * d); m->mt_hn = falloc(m, (size_t)T * d); m->chain_h = falloc(m, (size_t)T * d);
@@ -998,15 +1009,13 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
   for (int v = 0; v < 3; v++) m->xpv[v][5] = m->xpv[v][0];   // placeholder where there are no routed experts
   if (m->ne > 0) {
     const int ns = m->nk + 1;
-    m->moe_lg = falloc(m, (size_t)T * (m->ne + 1)); m->moe_wt = falloc(m, (size_t)T * ns); m->moe_ids = (int *)dalloc(m, (size_t)T * ns * 4);
+    m->moe_lg = falloc(m, (size_t)T * (m->ne + 1)); m->moe_wt = falloc(m, (size_t)T * ns); m->moe_ids = (int *)dalloc(m, (size_t)T * ns * 4); m->moe_live = (int *)dalloc(m, 4 * 64);
     m->moe_g = falloc(m, (size_t)T * ns * m->ef); m->moe_u = falloc(m, (size_t)T * ns * m->ef); m->hn2 = falloc(m, (size_t)T * d);
     CK(xp_alloc(m, 5, ns * m->ef));
-    if (!m->moe_lg || !m->moe_wt || !m->moe_ids || !m->moe_g || !m->moe_u || !m->hn2) return -1;
+    if (!m->moe_lg || !m->moe_wt || !m->moe_ids || !m->moe_live || !m->moe_g || !m->moe_u || !m->hn2) return -1;
   }
   m->ctl = (SpecCtl *)dalloc(m, sizeof(SpecCtl) * B);
-  m->const_rows = (int *)dalloc(m, 4);
-  if (!m->x || !m->po || !m->ctl || !m->const_rows) return -1;
-  { const int rows = B * m->Tspec; CU_OK(cudaMemcpyAsync(m->const_rows, &rows, 4, cudaMemcpyHostToDevice, g_llb.stream)); CU_OK(cudaStreamSynchronize(g_llb.stream)); }
+  if (!m->x || !m->po || !m->ctl || !m->hn_pf) return -1;
   CU_OK(cudaHostAlloc((void **)&m->res_host, sizeof(SpecResult) * m->res_n * B, cudaHostAllocMapped));
   memset(m->res_host, 0, sizeof(SpecResult) * m->res_n * B);
   CU_OK(cudaHostGetDevicePointer((void **)&m->res_dev, m->res_host, 0));
@@ -1182,7 +1191,7 @@ static int pf_prefill(llb_spec *m, int b, const int *ids, int n_rows, int keep, 
   }
   if (p > 0) {
     // the stream's first row of the trunk's normed hidden rows: what the pending catch-up row pairs with
-    CU_OK(cudaMemcpyAsync(m->hn + (size_t)(m->B > 1 ? b * m->per : 0) * m->d, f.hn, (size_t)m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
+    CU_OK(cudaMemcpyAsync(m->hn_pf + (size_t)(m->B > 1 ? b * m->Tpf : 0) * m->d, f.hn, (size_t)m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
     struct { int n, pos0, tok[SPEC_MAXT], slot[SPEC_MAXT]; } c;
     memset(&c, 0, sizeof c);
     c.n = m->has_mtp ? 1 : 0; c.pos0 = p; c.tok[0] = ids[p];
@@ -1294,13 +1303,16 @@ static llb_spec *open_finish(llb_spec *m) {
   // between cycles lives in device memory.
   // (an eager pass at either width first: a K-split, and so a buffer's size, may differ between them)
   bool bad = false;
-  const int w_spec = m->B * m->Tspec, w_pf = m->B > 1 ? w_spec : m->Tpf;
+  const int w_spec = m->B * m->Tspec, w_pf = m->B * m->Tpf;
   if (m->tp.size > 1 && tp_host_barrier()) { llb_spec_close(m); return nullptr; }   // the ranks finished loading at different times
   {
-    StreamScope scope(m);
     set_width(m, w_pf);
+    StreamScope scope(m);
     bad = bad || llb_spec_reset(m) || enq_cycle(m, false);
+  }
+  {
     set_width(m, w_spec);
+    StreamScope scope(m);
     bad = bad || llb_spec_reset(m) || enq_cycle(m, true) || llb_spec_reset(m);
   }
   bad = bad || capture(m, 0, &m->g_spec, &m->n_spec_nodes);
@@ -1370,6 +1382,7 @@ static int reset_stream(llb_spec *m, int b) {
   // the trunk's normed hidden rows the drafter pairs with (the stream's rows of the widest pass)
   const int rows = m->B > 1 ? m->Tspec : (m->Tpf > SPEC_MAXT ? m->Tpf : SPEC_MAXT);
   CU_OK(cudaMemsetAsync(m->hn + (size_t)b * rows * m->d, 0, (size_t)rows * m->d * 4, g_llb.stream));
+  if (m->B > 1) CU_OK(cudaMemsetAsync(m->hn_pf + (size_t)b * m->Tpf * m->d, 0, (size_t)m->Tpf * m->d * 4, g_llb.stream));
   CK(ctl_write(m, b, ctl_fresh(m, b)));
   SeqHost &q = m->sq[b];
   q.pos = 0; q.primed = false; q.have_last = false;
@@ -1394,7 +1407,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
     if (in_set[b]) return llb_fail("prefill: stream %d given twice", b);
     in_set[b] = 1;
     if (n < 1) return llb_fail("prefill: empty prompt");
-    if (n + m->Tpf + 1 > m->max_ctx) return llb_fail("prefill: %d tokens do not fit a context of %d", n, m->max_ctx);
+    if (n + (m->B > 1 ? m->Tspec : m->Tpf) + 1 > m->max_ctx) return llb_fail("prefill: %d tokens do not fit a context of %d", n, m->max_ctx);
     for (int j = 0; j < n; j++) if (ids[i][j] < 0 || ids[i][j] >= m->V) return llb_fail("prefill: token %d out of range", ids[i][j]);
   }
   for (int i = 0; i < nb; i++) CK(reset_stream(m, bs[i]));
@@ -1418,7 +1431,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
     CU_OK(cudaMemcpyAsync(hist_of(m, b), ids[i], (size_t)ns[i] * 4, cudaMemcpyHostToDevice, g_llb.stream));
     // the drafter's row for position 0 pairs token 0 with a zero hidden (host/llb_host.c:1815-1817)
     c.catchup.n = 1; c.catchup.pos0 = 0; c.catchup.tok[0] = ids[i][0];
-    c.verify.n = m->lookup ? 1 : m->per;   // nothing to look up at position 0
+    c.verify.n = m->lookup ? 1 : m->per;   // nothing to look up at position 0 (a one-token prompt's first cycle)
     c.verify.pos0 = 0; c.verify.tok[0] = ids[i][0];
     for (int r = 0; r < SPEC_MAXT; r++) c.verify.slot[r] = r & (CONV_RING - 1);
     CK(ctl_write(m, b, c));
@@ -1462,6 +1475,9 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
       if (p[i] >= ns[i] - 1 && live > 1) CK(park(bs[i]));   // through, while others still have rows to feed
     }
   }
+  if (m->B > 1 && m->has_mtp)   // the rows that the first speculative cycle's drafter catches up over, where that cycle looks for them
+    for (int i = 0; i < nb; i++)
+      CU_OK(cudaMemcpyAsync(m->hn + (size_t)bs[i] * m->Tspec * m->d, m->hn_pf + (size_t)bs[i] * m->Tpf * m->d, (size_t)m->Tspec * m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
   for (int o = 0; o < m->B; o++) if (kept[o]) CK(ctl_write(m, o, keep[o]));
   for (int i = 0; i < nb; i++) {
     SeqHost &q = m->sq[bs[i]];
@@ -1696,7 +1712,7 @@ LLB_API int llb_spec_profile_verify(llb_spec *m, char *buf, int cap) {
     g_prof_on = true;
     prof_mark("start");
     StreamScope scope(m);
-    int rc = enq_verify(m);
+    int rc = enq_verify(m, m->hn);
     g_prof_on = false;
     if (rc) return -1;
     CU_OK(cudaStreamSynchronize(g_llb.stream));

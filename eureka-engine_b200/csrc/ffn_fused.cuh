@@ -117,4 +117,5 @@ __global__ void __launch_bounds__(G2_MAXWARPS * 32, 1) k_ffn(const GemmArgs a1, 
   __syncthreads();   // the CTA is done with the first launch's planes
   g2_phase<FMT2, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err},
                     G2MatsPlain<FMT2, 1>{a2});
+  g2_drain(rg);
 }

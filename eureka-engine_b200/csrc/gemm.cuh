@@ -57,11 +57,11 @@ struct GemmArgs {
 struct MoeArgs {
   const uint8_t *W;     // GU or D stack
   long long es;         // bytes per expert block
-  const int *ids;       // [T][nslot]
+  const int *ids;       // [live rows][nslot]
   int nslot;            // k + 1
   int ne;               // block ne is the shared expert; ids are clamped to 0..ne
   int ef, d, T;
-  const int *n_rows;    // rows of the pass in flight (<= T); tiles of later rows are not computed
+  const int *live;      // rows of the pass in use: how many, then which, ascending (rows without a token cost nothing)
   float *g, *u;         // gate|up: [K-slice][T][nslot * ef]
   long long gu_stride;  // floats between their K-slices (one slice: any)
   float *out;           // k_moe_dn: [ksplit][T][d]

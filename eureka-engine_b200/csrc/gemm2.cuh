@@ -22,6 +22,7 @@
 
 #define G2_SMEM_MAX 226304   // 227 KB less the 6 KB that a phase may use beside the ring and the activation slice
 #define G2_MAXWARPS 16
+#define G2_WAIT_LIMIT (1u << 19)   // tries of a bounded wait (up to a microsecond each)
 #define G2_BAR_BYTES 512     // one mbarrier per warp and stage (at most four)
 
 // XPAD: padding of a plane column in shared memory (column stride = 64 mod 128 bytes for the 16-byte B reads of Q4_K / Q5_K /
@@ -326,7 +327,7 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
 
 // The warp's ring as it passes from one GEMM phase to the next: barriers (one a stage), stage memory, and the parity that
 // each stage's next wait looks for.
-struct G2Ring { uint32_t bar_s, ring_s; const uint8_t *ring; uint32_t par; };
+struct G2Ring { uint32_t bar_s, ring_s; const uint8_t *ring; uint32_t par; bool dead; };   // dead: a wait ran out, nothing more is requested
 // smem: G2_BAR_BYTES of barriers and then the rings, `per_warp` bytes each.  Private to a warp: no block barrier needed.
 __device__ __forceinline__ G2Ring g2_ring_init(uint8_t *smem, int per_warp) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -334,13 +335,18 @@ __device__ __forceinline__ G2Ring g2_ring_init(uint8_t *smem, int per_warp) {
   r.bar_s = smem_u32(smem) + warp * 32;
   r.ring = smem + G2_BAR_BYTES + warp * per_warp;
   r.ring_s = smem_u32(r.ring);
-  r.par = 0;
+  r.par = 0; r.dead = false;
   if (warp < G2_MAXWARPS && lane == 0) {
     for (int s = 0; s < 4; s++) mbar_init(r.bar_s + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
   return r;
+}
+
+// After a wait ran out: give what is still in flight its time before the block leaves.
+__device__ __forceinline__ void g2_drain(const G2Ring &r) {
+  if (r.dead) for (int s = 0; s < 3; s++) mbar_wait(r.bar_s + 8 * s, (r.par >> s) & 1u, G2_WAIT_LIMIT);
 }
 
 // Where a launch's row tiles live.  A policy says how many 16-row tiles there are, where tile i's 16 x 256 tiles in the
@@ -428,7 +434,7 @@ __device__ __forceinline__ void g2_run(const GemmArgs &a, const G2Slice &sl, int
     for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
 #pragma unroll 1
     for (int c = 0; c < sl.nsl; c += CH) {
-      if (!mbar_wait(rg.bar_s + 8 * s, (rg.par >> s) & 1u) && a.err) atomicExch(a.err, 1u);
+      if (!rg.dead && !mbar_wait(rg.bar_s + 8 * s, (rg.par >> s) & 1u, G2_WAIT_LIMIT)) { rg.dead = true; if (a.err) atomicExch(a.err, 1u); }
       rg.par ^= 1u << s;
 #pragma unroll 1
       for (int u = 0; u < CH && c + u < sl.nsl; u++) g2_tile<FMT, NT, NTC>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
@@ -454,22 +460,23 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
   g2_run<FMT, NT, WARPS, Mats, NTC>(a, sl, cps, rg, planes, planes + NC * CS, CS, mats);
 }
 
-// the activation slice from the planes in global memory: cp.async, one wait, one barrier
+// The activation slice from the planes in global memory: the columns of the launch's rows only (a one-row pass uses two of
+// eight; an MMA's columns do not see one another, so what the others hold does not matter).  Sixteen-byte cp.async by all
+// warps; one bulk copy a column took 0.5 us longer a launch.
 template <int FMT, int NT> struct G2StagePlanes {
   const GemmArgs &a;
   __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
     constexpr int NC = 8 * NT;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, ntask = a.planes * a.T * nsl;
+    const uint8_t *xh = (const uint8_t *)(a.xp.xh + (size_t)sb0 * 256), *xf = (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
     pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int c = warp; c < NC; c += nw) {   // a warp takes a column: 32 sixteen-byte pieces a super-block
-      const uint8_t *src = (const uint8_t *)(a.xp.xh + (size_t)c * a.K + (size_t)sb0 * 256);
-      const uint32_t dst = smem_u32(xh_s + c * CS);
-      for (int p = lane; p < nsl * 32; p += 32) cp_async16(dst + g2_xpos<FMT, NT>(p), src + p * 16);
+#pragma unroll 2
+    for (int task = warp; task < ntask; task += nw) {   // (live column, super-block): 32 pieces, a lane each
+      const int i = task / nsl, sb = task - i * nsl, c = i < a.T ? i : NC / 2 + i - a.T, p = sb * 32 + lane;
+      cp_async16(smem_u32(xh_s + c * CS) + g2_xpos<FMT, NT>(p), xh + (size_t)c * a.K * 2 + p * 16);
     }
-    if constexpr (g2_aux(FMT) != 0) {       // the means of the slice: contiguous in global memory
-      const uint8_t *xf = (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
+    if constexpr (g2_aux(FMT) != 0)         // the means of the slice: contiguous in global memory
       for (int i = threadIdx.x; i < nsl * NC * 2; i += blockDim.x) cp_async16(smem_u32(xsf_s + i * 16), xf + i * 16);
-    }
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
@@ -482,4 +489,5 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_gemm2(const G
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
   g2_phase<FMT, NT>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT), G2StagePlanes<FMT, NT>{a}, G2MatsPlain<FMT, NT>{a});
+  g2_drain(rg);
 }

@@ -69,6 +69,18 @@ __device__ __forceinline__ float4 part_get4(const PartIn &a, size_t i) {
   }
   return v;
 }
+// (p_parts4: four slices of four consecutive values in flight a trip, in a rolled loop -- the small kernels' form)
+__device__ __forceinline__ void p_parts4(const PartIn &a, size_t i, float4 &v) {
+  const float *p = a.p + i;
+#pragma unroll 1
+  for (int k = 0; k < a.ns; k += 4, p += 4 * a.stride) {
+    float4 l[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) l[q] = k + q < a.ns ? __ldcg((const float4 *)(p + q * a.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 4; q++) { v.x += l[q].x; v.y += l[q].y; v.z += l[q].z; v.w += l[q].w; }
+  }
+}
 __device__ __forceinline__ float part_get(const PartIn &a, size_t i) {
   float v = __ldcg(a.p + i);
   for (int k = 1; k < a.ns; k += 4) {
@@ -102,8 +114,9 @@ int op_norm_xp(cudaStream_t s, const float *xin, PartIn add, const float *w, flo
                int xp_col0, float *hn_out, const RowSet *rs, int Tmax, int zero_if_pos0);
 int op_silu_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, int Tmax);
 int op_silu_scaled_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, int Tmax, const float *scale, int seg);
-// router logits (ne rows + the shared gate row of Wr, F32) on the normed rows h[T][d], then ids / wt [T][nk + 1]
-int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne, int nk, float *lg, int *ids, float *wt, const RowSet *rs, int Tmax);
+// router logits (ne rows + the shared gate row of Wr, F32) on the normed rows h[T][d], then wt [T][nk + 1] by row of the pass,
+// live = how many rows are in use and which (16 at most), ids [live][nk + 1]
+int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne, int nk, float *lg, int *ids, float *wt, int *live, const RowSet *rs, int Tmax);
 // kv_only: only the K and V rows (the drafter's cache fill of the prompt path: no query rows)
 int op_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, const float *kn_w, const double *invfreq,
               AttnShape sh, float *qout, float *Kc, float *Vc, const RowSet *rs, int Tmax, bool kv_only = false);
@@ -112,11 +125,10 @@ int op_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, c
 // by one group per grid z)
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,
                  float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg = nullptr, int kg_row0 = 0, int nz = 1);
-int op_delta_conv(cudaStream_t s, PartIn ring, const float *cw, PartIn bp, PartIn ap, const float *dt, const float *sa,
-                  DeltaShape sh, float *y, float *beta, float *decay, const RowSet *rs, int Tmax);
-// S: the streams' state rings one after the other (s_group floats apart); nz streams
-int op_delta_fused(cudaStream_t s, float *S, const SpecCtl *ctl, const float *y, const float *beta, const float *decay, PartIn z,
-                   const float *nw, DeltaShape sh, XPlanes xp, const RowSet *rs, int nz = 1, long long s_group = 0);
+// conv1d + gates + recurrent scan + gated norm -> planes.  S: the streams' state rings one after the other (s_group floats
+// apart); nz streams
+int op_delta(cudaStream_t s, float *S, const SpecCtl *ctl, PartIn ring, const float *cw, PartIn bp, PartIn ap, const float *dt, const float *sa,
+             PartIn z, const float *nw, DeltaShape sh, XPlanes xp, const RowSet *rs, int nz = 1, long long s_group = 0);
 // A row set that no kernel of the pass in flight writes (the verify rows: k_accept sets them at the end
 // of the previous cycle) may be read before the wait on the preceding kernel, which takes one trip to L2
 // off every small kernel's critical path.  The host says so by setting bit 0 of the pointer it passes.

@@ -49,16 +49,16 @@ template <int FMT, int NTP> struct MoeGuMats {
   static constexpr bool EARLY = false, CONTIG = true;
   const MoeArgs &m;
   struct Cur { const uint8_t *W; };
-  __device__ __forceinline__ int ntiles() const { return min(*m.n_rows, m.T) * m.nslot * (m.ef >> 3); }   // 2 ef / 16 tiles per slot
+  __device__ __forceinline__ int ntiles() const { return min(*m.live, m.T) * m.nslot * (m.ef >> 3); }   // 2 ef / 16 tiles per slot
   __device__ __forceinline__ void locate(int tile, int sb0, Cur &c) const {
     const int tps = m.ef >> 3, slot = tile / tps;
     const int e = min(max(m.ids[slot], 0), m.ne);
     c.W = m.W + (size_t)e * m.es + ((size_t)(tile - slot * tps) * (m.d >> 8) + sb0) * tile_bytes(FMT);
   }
   __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const { return c.W + (size_t)pc * tile_bytes(FMT); }
-  __device__ __forceinline__ int col0(int tile) const { return ((tile / (m.ef >> 3)) / m.nslot) & ~7; }
+  __device__ __forceinline__ int col0(int tile) const { return m.live[1 + (tile / (m.ef >> 3)) / m.nslot] & ~7; }
   template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
-    const int tps = m.ef >> 3, slot = tile / tps, t = slot / m.nslot, jx = slot - t * m.nslot;
+    const int tps = m.ef >> 3, slot = tile / tps, ri = slot / m.nslot, t = m.live[1 + ri], jx = slot - ri * m.nslot;
     float v0, v1;
     bool mine;
     moe_col<NT>(acc, t, lane, v0, v1, mine);
@@ -73,7 +73,7 @@ template <int FMT, int NTP> struct MoeDnMats {
   static constexpr bool EARLY = false, CONTIG = false;
   const MoeArgs &m;
   struct Cur { const int *ids; int tile; };
-  __device__ __forceinline__ int ntiles() const { return min(*m.n_rows, m.T) * (m.d >> 4); }
+  __device__ __forceinline__ int ntiles() const { return min(*m.live, m.T) * (m.d >> 4); }
   __device__ __forceinline__ void locate(int tile, int sb0, Cur &c) const {
     const int tpt = m.d >> 4, t = tile / tpt;
     c.tile = tile - t * tpt;
@@ -84,14 +84,14 @@ template <int FMT, int NTP> struct MoeDnMats {
     const int e = min(max(c.ids[g], 0), m.ne);
     return m.W + (size_t)e * m.es + ((size_t)c.tile * eb + sbi - g * eb) * tile_bytes(FMT);
   }
-  __device__ __forceinline__ int col0(int tile) const { return (tile / (m.d >> 4)) & ~7; }
+  __device__ __forceinline__ int col0(int tile) const { return m.live[1 + tile / (m.d >> 4)] & ~7; }
   template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
-    const int tpt = m.d >> 4, t = tile / tpt;
+    const int tpt = m.d >> 4, ri = tile / tpt, t = m.live[1 + ri];
     float v0, v1;
     bool mine;
     moe_col<NT>(acc, t, lane, v0, v1, mine);
     if (!mine) return;
-    float *dst = m.out + (size_t)ks * m.split_stride + (size_t)t * m.d + (tile - t * tpt) * 16 + g2_row<FMT, NTP>(lane >> 2);
+    float *dst = m.out + (size_t)ks * m.split_stride + (size_t)t * m.d + (tile - ri * tpt) * 16 + g2_row<FMT, NTP>(lane >> 2);
     dst[0] = v0; dst[8] = v1;
   }
 };
@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_gu(const 
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
   g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeGuMats<FMT, NT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
                                                                           G2StagePlanes<FMT, NT>{a}, MoeGuMats<FMT, NT>{m});
+  g2_drain(rg);
 }
 // The down launch's activation slice built in shared memory from the gate|up outputs (T <= 4 rows): wt * silu(g) * u
 // of the CTA's K-slice, planes and side array exactly as k_silu_xp + G2StagePlanes would have left them, without the
@@ -112,7 +113,7 @@ template <int FMT> struct MoeStageSilu {
   const float *wt;   // [T][nslot]
   __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
     pdl_wait();
-    const int lane = threadIdx.x & 31, T = min(*m.n_rows, m.T), f = m.nslot * m.ef;
+    const int lane = threadIdx.x & 31, nl = min(*m.live, m.T), T = nl > 0 ? m.live[nl] + 1 : 0, f = m.nslot * m.ef;
     const int ngrp = nsl * 64, ntask = 4 * ngrp;   // (row of the 4 plane pairs, group of four columns); rows >= T are zero planes
     for (int t0 = threadIdx.x; t0 < ntask; t0 += 4 * blockDim.x) {
       float4 gv[4], uv[4];
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8) * 32, 1) k_moe_dn_silu(const 
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8) / g2_warps(FMT, 8));
   g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStageSilu<FMT>{m, wt}, MoeDnMats<FMT, 1>{m});
+  g2_drain(rg);
 }
 
 template <int FMT, int NT>
@@ -157,4 +159,5 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_dn(const 
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
   g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeDnMats<FMT, NT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
                                                                           G2StagePlanes<FMT, NT>{a}, MoeDnMats<FMT, NT>{m});
+  g2_drain(rg);
 }

@@ -4,34 +4,44 @@
 #include "host.cuh"
 
 // ---- activations -> fp16 planes ----------------------------------------------------------------
-__global__ void k_xp_from_f32(const float *__restrict__ x, int K, int planes, XPlanes xp) {
+// a thread takes four consecutive columns; a warp may be partly past the row's end (K is a multiple of 32)
+__global__ void __launch_bounds__(256) k_xp_from_f32(const float *__restrict__ x, int K, int planes, XPlanes xp) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.y, lane = threadIdx.x & 31;
-  const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
-  if (c0 >= K) return;
-  xp_store32(xp, t, planes, c0, x[(size_t)t * K + c0 + lane], lane);
+  const int t = blockIdx.y, c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c < K) {
+    const float *r = x + (size_t)t * K + c;
+    if (!((uintptr_t)x & 15)) { const float4 f = __ldcg((const float4 *)r); v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; }
+    else for (int i = 0; i < 4; i++) v[i] = __ldcg(r + i);
+  }
+  xp_store4(xp, t, planes, c, v, threadIdx.x & 31, c < K);
 }
-__global__ void k_xp_from_bf16(const unsigned short *__restrict__ x, int K, XPlanes xp) {
+__global__ void __launch_bounds__(256) k_xp_from_bf16(const unsigned short *__restrict__ x, int K, XPlanes xp) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.y, lane = threadIdx.x & 31;
-  const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
-  if (c0 >= K) return;
-  float v = __uint_as_float((uint32_t)x[(size_t)t * K + c0 + lane] << 16);
-  xp_store32(xp, t, 1, c0, v, lane);
+  const int t = blockIdx.y, c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c < K) {
+    const unsigned short *r = x + (size_t)t * K + c;
+    uint2 w;
+    if (!((uintptr_t)x & 7)) w = __ldcg((const uint2 *)r);
+    else w = make_uint2(r[0] | ((uint32_t)r[1] << 16), r[2] | ((uint32_t)r[3] << 16));
+    v[0] = __uint_as_float(w.x << 16); v[1] = __uint_as_float(w.x & 0xffff0000u); v[2] = __uint_as_float(w.y << 16); v[3] = __uint_as_float(w.y & 0xffff0000u);
+  }
+  xp_store4(xp, t, 1, c, v, threadIdx.x & 31, c < K);
 }
 int ops_xp_from_f32(cudaStream_t s, const float *x, int T, int planes, XPlanes xp) {
   if (xp.K % 32) return llb_fail("xp: K %d", xp.K);
   if (T * planes > xp.NC) return llb_fail("xp: %d rows x %d planes do not fit %d columns", T, planes, xp.NC);
-  CU_OK(llb_launch(k_xp_from_f32, dim3((xp.K + 255) / 256, T), dim3(256), (size_t)(0), s, x, xp.K, planes, xp));
+  CU_OK(llb_launch(k_xp_from_f32, dim3((xp.K + 1023) / 1024, T), dim3(256), (size_t)(0), s, x, xp.K, planes, xp));
   CU_OK(cudaGetLastError());
   return 0;
 }
 int ops_xp_from_bf16(cudaStream_t s, const void *x, int T, XPlanes xp) {
   if (xp.K % 32) return llb_fail("xp: K %d", xp.K);
   if (T > xp.NC) return llb_fail("xp: %d rows do not fit %d columns", T, xp.NC);
-  CU_OK(llb_launch(k_xp_from_bf16, dim3((xp.K + 255) / 256, T), dim3(256), (size_t)(0), s, (const unsigned short *)x, xp.K, xp));
+  CU_OK(llb_launch(k_xp_from_bf16, dim3((xp.K + 1023) / 1024, T), dim3(256), (size_t)(0), s, (const unsigned short *)x, xp.K, xp));
   CU_OK(cudaGetLastError());
   return 0;
 }

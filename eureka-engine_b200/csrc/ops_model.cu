@@ -45,19 +45,19 @@ int op_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const RowSet *rs,
 // tools/payload-spec2.patch:35-112; rms_norm tools/qwen35_engine.c:510-515) ----------------------
 // v = xin + sum(partials); xout = v (optional); h = (v * s) * w, s = 1/sqrt(mean(v^2) + eps);
 // h goes to the planes at column offset xp_col0 and, optionally, to hn_out as f32.
-// One block per row; a thread holds NI groups of four consecutive columns (float4 loads and stores), so a
-// row of 5120 columns costs each of 640 threads a handful of instructions instead of one SM 13k.
+// One block per row; a thread holds NI groups of four consecutive columns (float4 loads and stores).
 #define NORM_MAXT 1024
 template <int NI>
 __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__ xin, PartIn add, const float *__restrict__ w, float eps, int d,
                                                        float *__restrict__ xout, XPlanes xp, int xp_col0, float *__restrict__ hn_out,
                                                        const RowSet *rs, Streams sg, int zero_if_pos0) {
   // the norm weights depend on no kernel: their trip to DRAM overlaps the wait on the producer
-  float4 wv[NI];
+  float4 wv[NI], v[NI];
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
-    wv[i] = c < d ? *(const float4 *)(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    wv[i] = c < d ? __ldg((const float4 *)(w + c)) : v[i];
   }
   int rs_n, rs_p0, tl;
   const int t = blockIdx.x;
@@ -66,27 +66,28 @@ __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__
   if (tl >= rs_n) return;
   const bool zero = zero_if_pos0 && (rs_p0 + tl == 0);
   const size_t row = (size_t)t * d;
-  // every load of a trip is issued before the first use: one round trip to L2 per four slices
-  float4 v[NI];
+  if (xin && !zero) {
 #pragma unroll
-  for (int i = 0; i < NI; i++) {
-    const int c = 4 * (threadIdx.x + i * blockDim.x);
-    v[i] = (c < d && xin && !zero) ? *(const float4 *)(xin + row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < NI; i++) {
+      const int c = 4 * (threadIdx.x + i * blockDim.x);
+      if (c < d) v[i] = __ldcg((const float4 *)(xin + row + c));
+    }
   }
   if (add.p && !zero) {
-    for (int k = 0; k < add.ns; k += 4) {
-      const float *pk = add.p + (size_t)k * add.stride + row;
-      const int nk = add.ns - k;
+    // four slices of every group in flight a trip, added in slice order
+    const float *pk = add.p + row;
+#pragma unroll 1
+    for (int k = 0; k < add.ns; k += 4, pk += 4 * add.stride) {
       float4 l[4][NI];
 #pragma unroll
       for (int q = 0; q < 4; q++)
 #pragma unroll
         for (int i = 0; i < NI; i++) {
           const int c = 4 * (threadIdx.x + i * blockDim.x);
-          l[q][i] = (c < d && q < nk) ? *(const float4 *)(pk + (size_t)q * add.stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+          l[q][i] = (c < d && k + q < add.ns) ? __ldcg((const float4 *)(pk + (size_t)q * add.stride + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-      for (int q = 0; q < 4; q++)   // added in slice order
+      for (int q = 0; q < 4; q++)
 #pragma unroll
         for (int i = 0; i < NI; i++) { v[i].x += l[q][i].x; v[i].y += l[q][i].y; v[i].z += l[q][i].z; v[i].w += l[q][i].w; }
     }
@@ -95,14 +96,15 @@ __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
-    if (c < d) {
-      if (xout) *(float4 *)(xout + row + c) = v[i];
-      ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
-    }
+    if (xout && c < d) *(float4 *)(xout + row + c) = v[i];
+    ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;   // (zeros past the row's end)
   }
-  ss = block_sum(ss, red);
+  const int lane = threadIdx.x & 31, nwp = blockDim.x >> 5;
+  ss = warp_sum(ss);
+  if (lane == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = warp_sum(lane < nwp ? red[lane] : 0.0f);
   const float sc = 1.0f / sqrtf(ss / (float)d + eps);
-  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);   // eight lanes hold 32 consecutive columns
@@ -141,12 +143,25 @@ __global__ void __launch_bounds__(256) k_silu_xp(PartIn g, PartIn u, int f, XPla
   float h[4] = {0.f, 0.f, 0.f, 0.f};
   if (on) {
     const size_t i = (size_t)t * f + c;
-    const float4 gv = part_get4(g, i), uv = part_get4(u, i);
-    h[0] = silu_f(gv.x) * uv.x; h[1] = silu_f(gv.y) * uv.y; h[2] = silu_f(gv.z) * uv.z; h[3] = silu_f(gv.w) * uv.w;
-    if (scale) {
-      const float w = scale[(size_t)t * (f / seg) + c / seg];
-      h[0] *= w; h[1] *= w; h[2] *= w; h[3] *= w;
+    float4 gv = make_float4(0.f, 0.f, 0.f, 0.f), uv = gv;
+    const float *pg = g.p + i, *pu = u.p + i;
+    const int ns = max(g.ns, u.ns);
+#pragma unroll 1
+    for (int k = 0; k < ns; k += 2, pg += 2 * g.stride, pu += 2 * u.stride) {   // both matrices' slices in flight together
+      float4 l[2], m[2];
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        l[q] = k + q < g.ns ? __ldcg((const float4 *)(pg + q * g.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        m[q] = k + q < u.ns ? __ldcg((const float4 *)(pu + q * u.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        gv.x += l[q].x; gv.y += l[q].y; gv.z += l[q].z; gv.w += l[q].w;
+        uv.x += m[q].x; uv.y += m[q].y; uv.z += m[q].z; uv.w += m[q].w;
+      }
     }
+    const float w = scale ? __ldcg(scale + (size_t)t * (f / seg) + c / seg) : 1.0f;
+    h[0] = silu_f(gv.x) * uv.x * w; h[1] = silu_f(gv.y) * uv.y * w; h[2] = silu_f(gv.z) * uv.z * w; h[3] = silu_f(gv.w) * uv.w * w;
   }
   xp_store4(xp, t, 2, c, h, lane, on);
 }
@@ -171,7 +186,7 @@ int op_silu_scaled_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, con
 #define MOE_MAXROWS 16   // rows of a pass the router takes (several streams of k + 1 rows)
 template <int NQ, int MR>   // MR: the most rows of a pass (8 or 16); two resident blocks a multiprocessor, so that the ne + 1 blocks are one wave
 __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__ W, const float *__restrict__ h, int d, int ne, int nk, float *__restrict__ lg,
-                                                    int *__restrict__ ids, float *__restrict__ wt, unsigned int *__restrict__ ctr, const RowSet *rs, int n_all) {
+                                                    int *__restrict__ ids, float *__restrict__ wt, unsigned int *__restrict__ ctr, int *__restrict__ live, const RowSet *rs, Streams sg, int n_all) {
   int rs_n, rs_p0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.x, nrows = ne + 1;
   __shared__ float red[8][MR];
@@ -218,10 +233,19 @@ __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__
   if (last != gridDim.x - 1) return;
   __threadfence();
   if (threadIdx.x == 0) *ctr = 0;   // ready for the next launch (launches of one stream do not overlap here)
-  for (int t = warp; t < rs_n; t += 8) moe_route_row<NQ>(lg + (size_t)t * nrows, ne, nk, ids + (size_t)t * (nk + 1), wt + (size_t)t * (nk + 1), lane);
+  // which rows are in use: all of them in a pass of one stream, else the first n of every stream's
+  bool on = lane < rs_n;
+  if (n_all > 0 && on) { const int z = lane / sg.per; on = lane - z * sg.per < ((const RowSet *)((const char *)rs + (size_t)z * sg.stride))->n; }
+  const unsigned int mask = __ballot_sync(0xffffffffu, on);
+  if (warp == 0) {
+    if (lane == 0) live[0] = __popc(mask);
+    if (on) live[1 + __popc(mask & ((1u << lane) - 1))] = lane;
+  }
+  for (int t = warp; t < rs_n; t += 8)
+    if ((mask >> t) & 1) moe_route_row<NQ>(lg + (size_t)t * nrows, ne, nk, ids + (size_t)__popc(mask & ((1u << t) - 1)) * (nk + 1), wt + (size_t)t * (nk + 1), lane);
 }
 static unsigned int *g_moe_ctr = nullptr;
-int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne, int nk, float *lg, int *ids, float *wt, const RowSet *rs, int Tmax) {
+int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne, int nk, float *lg, int *ids, float *wt, int *live, const RowSet *rs, int Tmax) {
   const int n_all = g_streams.stride ? Tmax : 0;
   if (Tmax > MOE_MAXROWS) return llb_fail("moe route: %d rows in a pass (at most %d)", Tmax, MOE_MAXROWS);
   if (ne < 1 || ne > 1024 || nk < 1 || nk > 32 || nk > ne || d % 4) return llb_fail("moe route: %d experts, top %d, d %d", ne, nk, d);
@@ -229,7 +253,7 @@ int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne,
     CU_OK(cudaMalloc(&g_moe_ctr, 4));
     CU_OK(cudaMemset(g_moe_ctr, 0, 4));
   }
-#define ROUTE_GO(NQ, MR) CU_OK(llb_launch(k_moe_router<NQ, MR>, dim3(ne + 1), dim3(256), (size_t)(0), s, Wr, h, d, ne, nk, lg, ids, wt, g_moe_ctr, rs, n_all))
+#define ROUTE_GO(NQ, MR) CU_OK(llb_launch(k_moe_router<NQ, MR>, dim3(ne + 1), dim3(256), (size_t)(0), s, Wr, h, d, ne, nk, lg, ids, wt, g_moe_ctr, live, rs, g_streams, n_all))
   if (ne <= 256) { if (Tmax <= 8) ROUTE_GO(8, 8); else ROUTE_GO(8, MOE_MAXROWS); }
   else { if (Tmax <= 8) ROUTE_GO(32, 8); else ROUTE_GO(32, MOE_MAXROWS); }
 #undef ROUTE_GO
@@ -300,175 +324,227 @@ int op_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, c
 }
 
 // ---- gated DeltaNet ------------------------------------------------------------------------------
-// conv1d + SiLU over the position-indexed ring, and the per-head gates
-// (llb_t_midconv, tools/payload-spec2.patch:319-350; tools/qwen35_engine.c:589-602).
-// grid (ceil(convd/256) + 1, Tmax): the last block computes beta = sigmoid(b), decay = exp(softplus(a + dt) * ssm_a).
-__global__ void k_delta_conv(PartIn ring, const float *__restrict__ cw, PartIn bp, PartIn ap,
-                             const float *__restrict__ dt, const float *__restrict__ sa, DeltaShape sh, float *__restrict__ y,
-                             float *__restrict__ beta, float *__restrict__ decay, const RowSet *rs, Streams sg) {
-  int rs_n, rs_p0, tl;
-  const int t = blockIdx.y;
-  rs = rs_begin_row(rs, sg, t, rs_n, rs_p0, tl);
-  if (tl >= rs_n) return;
-  if (blockIdx.x == gridDim.x - 1) {
-    for (int h = threadIdx.x; h < sh.TR; h += blockDim.x) {
-      const float b = part_get(bp, (size_t)t * sh.TR + h), a = part_get(ap, (size_t)t * sh.TR + h);
-      beta[t * sh.TR + h] = 1.0f / (1.0f + (float)exp((double)-b));
-      const float x = a + dt[h];
-      const float sp = x > 20.0f ? x : (float)log1p((double)(float)exp((double)(x < 88.0f ? x : 88.0f)));
-      decay[t * sh.TR + h] = (float)exp((double)(sp * sa[h]));
-    }
-    return;
-  }
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= sh.convd) return;
-  const int pos = rs_p0 + tl, slot0 = (t / sg.per) * ring.ns * CONV_RING;   // a stream's ring: [K-slice][CONV_RING slots], the streams' rings one after the other
-  float acc = 0.0f;
-  for (int k = 0; k < sh.KC; k++) {  // tap KC-1 is the current token (tools/qwen35_engine.c:599-600)
-    const int slot = slot0 + ((pos - (sh.KC - 1) + k) & (CONV_RING - 1));
-    acc = __fadd_rn(acc, __fmul_rn(part_get(ring, (size_t)slot * sh.convd + c), cw[c * sh.KC + k]));
-  }
-  y[(size_t)t * sh.convd + c] = silu_f(acc);
+// conv1d + SiLU over the position-indexed ring, gates, the recurrent scan over the T rows with per-row state checkpoints,
+// then the gated RMSNorm of each head's output into the planes of ssm_out's input: one kernel
+// (llb_t_midconv, llb_t_l2qk + llb_t_gdl, llb_t_grn, tools/payload-spec2.patch:319-447; tools/qwen35_engine.c:589-654).
+// grid (TR, 4) in clusters of four blocks = one value head, 256 threads: block (hh, jq) owns state rows j = 32 jq .. + 31 of
+// head hh, 16 registers of state per thread (thread = row jr, column eighth cq).  The state is read from ring slot sc and
+// the state after row r is written to slot (sc + r + 1) % R, so rejecting rows costs nothing: the next cycle simply starts
+// from the slot of the last served row.
+//
+// What bounds it is a chain of latencies, not bytes (a 27B layer moves 16 MB of state in 2.4 us; conv and scan as two kernels
+// took 3 + 13 us of a four-row pass).  What keeps the chain short: the conv is part of the kernel (every block redoes the 256
+// q and k channels of its group; with all rows x slices of the ring in flight as float4 loads that is one trip to L2 and one
+// launch less, where row by row and slice by slice the trips took 20 us); inputs are requested long before their use; the gates' double-precision functions run in the last warp while its loads and the other warps' conv do; and the
+// sums of squares of the gated norm are pushed into the peers' shared memory and cost one cluster barrier, behind which
+// the gate factors are made.
+#define DL_THREADS 256
+#define DL_MAXR (SPEC_MAXT + CONV_RING / 2 - 1)   // history rows of a pass: n + KC - 1
+__device__ __forceinline__ float4 dl_slice(const PartIn &a, size_t i, int k) {
+  return k < a.ns ? __ldcg((const float4 *)(a.p + i + k * a.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
-int op_delta_conv(cudaStream_t s, PartIn ring, const float *cw, PartIn bp, PartIn ap, const float *dt, const float *sa,
-                  DeltaShape sh, float *y, float *beta, float *decay, const RowSet *rs, int Tmax) {
-  if (sh.KC > CONV_RING / 2) return llb_fail("conv kernel %d", sh.KC);
-  CU_OK(llb_launch(k_delta_conv, dim3((sh.convd + 255) / 256 + 1, Tmax), dim3(256), (size_t)(0), s, ring, cw, bp, ap, dt, sa, sh, y, beta, decay, rs, g_streams));
-  CU_OK(cudaGetLastError());
-  return 0;
-}
-
-// ---- DeltaNet scan + gated RMSNorm as one kernel ------------------------------------------------
-// The recurrent scan over the T rows with per-row state checkpoints (llb_t_l2qk + llb_t_gdl,
-// tools/payload-spec2.patch:353-410; tools/qwen35_engine.c:610-646), then the gated RMSNorm of each head's
-// output into the planes of ssm_out's input (llb_t_grn, tools/payload-spec2.patch:413-447;
-// tools/qwen35_engine.c:648-654).  grid (TR, 4) in clusters of four blocks = one value head, 128 threads:
-// block (hh, jq) owns state rows j = 32 jq .. 32 jq + 31 of head hh, 32 registers of state per thread
-// (thread = row jr, column quarter cq); the RMSNorm's sum of squares over the head's 128 outputs is
-// exchanged through distributed shared memory.  The state is read from ring slot sc and the state after
-// row r is written to slot (sc + r + 1) % R, so rejecting rows costs nothing: the next cycle simply
-// starts from the slot of the last served row.
-// (Folding the conv in as well was measured and dropped: every block has to redo the conv of its whole
-// q/k group from the four partial-sum slices of the ring, 12x the loads, 65 us against 29 us for three kernels.)
-__global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(128)
-k_delta_fused(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ beta,
-              const float *__restrict__ decay, PartIn z, const float *__restrict__ nw, DeltaShape sh, XPlanes xp,
-              const RowSet *rs, Streams sg, long long s_group) {
-  __shared__ __align__(16) float qs[SPEC_MAXT][128], ks[SPEC_MAXT][128];
-  __shared__ float vs[SPEC_MAXT][32], db[SPEC_MAXT][2], os[SPEC_MAXT][32], ssq[SPEC_MAXT], tot[SPEC_MAXT];
-  __shared__ float red[2 * SPEC_MAXT][4];
+__device__ __forceinline__ void add4(float4 &v, const float4 l) { v.x += l.x; v.y += l.y; v.z += l.z; v.w += l.w; }
+__global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(DL_THREADS, 2)
+k_delta(float *__restrict__ S, const SpecCtl *__restrict__ ctl, PartIn ring, const float *__restrict__ cw, PartIn bp, PartIn ap,
+        const float *__restrict__ dt, const float *__restrict__ sa, PartIn z, const float *__restrict__ nw, DeltaShape sh, XPlanes xp,
+        const RowSet *rs, Streams sg, long long s_group) {
+  __shared__ __align__(16) float raw[DL_MAXR][288];          // channels: q 128 | k 128 | v 32 (this block's)
+  __shared__ __align__(16) float ys[SPEC_MAXT][288], os[SPEC_MAXT][32];
+  __shared__ float db[SPEC_MAXT][2], tot[SPEC_MAXT][4];
   cg::cluster_group cl = cg::this_cluster();
   const int hh = blockIdx.x, jq = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-  const int g = hh % sh.GK;
-  const int jr = tid >> 2, cq = tid & 3;
-  const size_t head_sz = 128 * 128, slot_sz = (size_t)sh.TR * head_sz;
-  const size_t off = (size_t)hh * head_sz + (size_t)(32 * jq + jr) * 128 + 4 * cq;
-  // The committed state (ring slot sc) was written by an earlier pass and sc by that pass's accept kernel: neither
-  // depends on the kernel in front, so the 16 KB a block reads from HBM are requested before the dependency wait.
+  const int g = hh % sh.GK, jr = tid >> 3, cq = tid & 7, KC = sh.KC;
+  const size_t slot_sz = (size_t)sh.TR * 128 * 128;
+  // The committed state (ring slot sc) was written by an earlier pass and sc by that pass's accept kernel, and the row set
+  // likewise (rs_stable): neither depends on the kernel in front, so the 16 KB of state that a block reads from HBM, and the
+  // conv's taps, are requested before the dependency wait.
   pdl_trigger();
-  {
-    // blockIdx.z: the stream -- its control block, its state ring, its rows of the pass
-    const size_t zz = blockIdx.z;
-    ctl = (const SpecCtl *)((const char *)ctl + zz * sg.stride);
-    rs = (const RowSet *)((uintptr_t)rs + zz * sg.stride);
-    S += zz * s_group;
-    const size_t r0 = sg.stride ? zz * sg.per : 0;
-    y += r0 * sh.convd; beta += r0 * sh.TR; decay += r0 * sh.TR; z.p += r0 * sh.vdc;
-  }
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before the first push: every peer runs
+  // blockIdx.z: the stream -- its control block, its state ring, its rows of the pass
+  ctl = (const SpecCtl *)((const char *)ctl + (size_t)blockIdx.z * sg.stride);
+  const bool early = (uintptr_t)rs & 1u;
+  rs = (const RowSet *)(((uintptr_t)rs & ~(uintptr_t)1) + (size_t)blockIdx.z * sg.stride);
   const int row0 = sg.stride ? blockIdx.z * sg.per : 0;
   const int R = *(const volatile int *)&ctl->R, sc = *(const volatile int *)&ctl->sc;
-  float st[32];
-  {
-    const float4 *src = (const float4 *)(S + (size_t)sc * slot_sz + off);
+  int n = 0, pos0 = 0;
+  if (early) { n = *(const volatile int *)&rs->n; pos0 = *(const volatile int *)&rs->pos0; }
+  float *St = S + blockIdx.z * s_group + (size_t)hh * 128 * 128 + (size_t)(32 * jq + jr) * 128 + 4 * cq;   // columns 4 cq + 32 i ..
+  float st[16];
 #pragma unroll
-    for (int i = 0; i < 8; i++) { float4 v = __ldcg(src + 4 * i); st[4 * i] = v.x; st[4 * i + 1] = v.y; st[4 * i + 2] = v.z; st[4 * i + 3] = v.w; }
+  for (int i = 0; i < 4; i++) { const float4 v = __ldcg((const float4 *)(St + (size_t)sc * slot_sz) + 8 * i); st[4 * i] = v.x; st[4 * i + 1] = v.y; st[4 * i + 2] = v.z; st[4 * i + 3] = v.w; }
+  // the conv's channels: tid and, in the first two warps, tid + 224, of the first seven warps; up to four taps kept in registers
+  float tap[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int c = tid + 224 * j, cc = c < 128 ? g * 128 + c : c < 256 ? sh.kdc + g * 128 + c - 128 : 2 * sh.kdc + hh * 128 + 32 * jq + c - 256;
+    const float *w = cw + (size_t)cc * KC + KC - 1;
+#pragma unroll
+    for (int k = 0; k < 4; k++) tap[j][k] = wp < (j ? 2 : 7) && k < KC ? __ldg(w - k) : 0.0f;
   }
-  const float nwv = nw[32 * jq + lane];
+  const float dtv = __ldg(dt + hh), sav = __ldg(sa + hh);
+  // rows this thread writes at the end: row zt, columns zc .. of the block's 32 (the first two warps)
+  const int zt = 4 * wp + (lane >> 3), zc = 4 * (lane & 7), col = hh * 128 + 32 * jq + zc;
+  const size_t zi = (size_t)(row0 + zt) * sh.vdc + col;
   pdl_wait();
-  rs = (const RowSet *)((uintptr_t)rs & ~(uintptr_t)1);
-  const int n = rs->n;
-  if (n < 1) return;   // every block of every cluster takes the same exit
-  float qv[SPEC_MAXT], kv[SPEC_MAXT];
+  if (!early) { n = rs->n; pos0 = rs->pos0; }
+  const int nr = n + KC - 1;
+  if (n < 1) { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); return; }   // every block of the cluster takes the same exit
+  // the gates' inputs, then the ring rows, then (behind them, for the end) z: four slices of each in flight
+  float gl[4], hl[4];
+  const size_t gi = (size_t)(row0 + lane) * sh.TR + hh;
+  const bool gon = wp == 7 && lane < n, zon = zt < n;
 #pragma unroll
-  for (int t = 0; t < SPEC_MAXT; t++) {
-    qv[t] = t < n ? y[(size_t)t * sh.convd + g * 128 + tid] : 0.0f;
-    kv[t] = t < n ? y[(size_t)t * sh.convd + sh.kdc + g * 128 + tid] : 0.0f;
+  for (int k = 0; k < 4; k++) {
+    gl[k] = gon && k < bp.ns ? __ldcg(bp.p + gi + k * bp.stride) : 0.0f;
+    hl[k] = gon && k < ap.ns ? __ldcg(ap.p + gi + k * ap.stride) : 0.0f;
   }
-  if (tid < 32) {
+  // history row r is position pos0 - (KC - 1) + r.  Item = (row, four channels); a stream's ring is [K-slice][CONV_RING slots]
+  const float *rp = ring.p + (size_t)blockIdx.z * ring.ns * CONV_RING * sh.convd;
+#pragma unroll 1
+  for (int i0 = tid; i0 < nr * 72; i0 += 2 * DL_THREADS) {
+    float4 v[2], l[4][2];
+    const float *p[2];
 #pragma unroll
-    for (int t = 0; t < SPEC_MAXT; t++) if (t < n) vs[t][tid] = y[(size_t)t * sh.convd + 2 * sh.kdc + hh * 128 + 32 * jq + tid];
-  }
-  if (tid < 2 * SPEC_MAXT && (tid >> 1) < n) db[tid >> 1][tid & 1] = (tid & 1) ? beta[(tid >> 1) * sh.TR + hh] : decay[(tid >> 1) * sh.TR + hh];
+    for (int q = 0; q < 2; q++) {
+      const int i = min(i0 + DL_THREADS * q, nr * 72 - 1), r = i / 72, c4 = i - r * 72;
+      const int c = c4 < 32 ? g * 128 + 4 * c4 : c4 < 64 ? sh.kdc + g * 128 + 4 * (c4 - 32) : 2 * sh.kdc + hh * 128 + 32 * jq + 4 * (c4 - 64);
+      p[q] = rp + (size_t)((pos0 - (KC - 1) + r) & (CONV_RING - 1)) * sh.convd + c;
+      v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
-  for (int t = 0; t < SPEC_MAXT; t++) {
-    const float a = warp_sum(qv[t] * qv[t]), b = warp_sum(kv[t] * kv[t]);
-    if (lane == 0) { red[2 * t][wp] = a; red[2 * t + 1][wp] = b; }
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int q = 0; q < 2; q++) l[u][q] = u < ring.ns ? __ldcg((const float4 *)(p[q] + u * ring.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (gon && i0 < DL_THREADS) {
+      // gates, while the rows are on their way: decay = exp(softplus(a + dt) ssm_a), beta = sigmoid(b)
+      float b = 0.0f, x = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) { b += gl[k]; x += hl[k]; }
+      for (int k = 4; k < bp.ns; k++) b += __ldcg(bp.p + gi + k * bp.stride);
+      for (int k = 4; k < ap.ns; k++) x += __ldcg(ap.p + gi + k * ap.stride);
+      x += dtv;
+      float sp = x;
+      if (x <= 20.0f) sp = (float)log1p((double)(float)exp((double)x));
+      db[lane][0] = (float)exp((double)(sp * sav));
+      db[lane][1] = 1.0f / (1.0f + (float)exp((double)-b));
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int q = 0; q < 2; q++) add4(v[q], l[u][q]);
+#pragma unroll 1
+    for (int k = 4; k < ring.ns; k++) { add4(v[0], __ldcg((const float4 *)(p[0] + k * ring.stride))); add4(v[1], __ldcg((const float4 *)(p[1] + k * ring.stride))); }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int i = i0 + DL_THREADS * q, r = i / 72;
+      if (i < nr * 72) *(float4 *)&raw[r][4 * (i - r * 72)] = v[q];
+    }
   }
+  float4 zl[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) zl[k] = zon ? dl_slice(z, zi, k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 nwv = __ldg((const float4 *)(nw + 32 * jq + zc));
   __syncthreads();
+  // conv: tap KC-1 is the current token (tools/qwen35_engine.c:599-600); thread = channel
+  if (KC <= 4) {
 #pragma unroll
-  for (int t = 0; t < SPEC_MAXT; t++) {
-    if (t < n) {
-      const float sq = red[2 * t][0] + red[2 * t][1] + red[2 * t][2] + red[2 * t][3];
-      const float sk = red[2 * t + 1][0] + red[2 * t + 1][1] + red[2 * t + 1][2] + red[2 * t + 1][3];
-      const float nq = sqrtf(sq), nk = sqrtf(sk);
-      const float iq = (1.0f / (nq > sh.eps ? nq : sh.eps)) / sqrtf(128.0f), ik = 1.0f / (nk > sh.eps ? nk : sh.eps);
-      qs[t][tid] = qv[t] * iq;
-      ks[t][tid] = kv[t] * ik;
+    for (int j = 0; j < 2; j++) {
+      if (wp >= (j ? 2 : 7)) break;
+      const int c = tid + 224 * j;
+      // the history slides through h; a tap that is not used adds exactly zero to the sum
+      float h1 = KC > 3 ? raw[KC - 4][c] : 0.0f, h2 = KC > 2 ? raw[KC - 3][c] : 0.0f, h3 = raw[KC - 2][c];
+#pragma unroll 2
+      for (int t = 0; t < n; t++) {
+        const float h = raw[t + KC - 1][c];
+        float a = __fadd_rn(0.0f, __fmul_rn(h1, tap[j][3]));
+        a = __fadd_rn(a, __fmul_rn(h2, tap[j][2]));
+        a = __fadd_rn(a, __fmul_rn(h3, tap[j][1]));
+        a = __fadd_rn(a, __fmul_rn(h, tap[j][0]));
+        ys[t][c] = silu_f(a);
+        h1 = h2; h2 = h3; h3 = h;
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int c = tid; c < 288; c += DL_THREADS) {
+      const int cc = c < 128 ? g * 128 + c : c < 256 ? sh.kdc + g * 128 + c - 128 : 2 * sh.kdc + hh * 128 + 32 * jq + c - 256;
+#pragma unroll 1
+      for (int t = 0; t < n; t++) {
+        float a = 0.0f;
+        for (int k = 0; k < KC; k++) a = __fadd_rn(a, __fmul_rn(raw[t + k][c], __ldg(cw + (size_t)cc * KC + k)));
+        ys[t][c] = silu_f(a);
+      }
     }
   }
   __syncthreads();
+  // L2 norms of q and k: a warp a row
+#pragma unroll 1
+  for (int i = wp; i < 2 * n; i += DL_THREADS / 32) {
+    float4 *p = (float4 *)&ys[i >> 1][128 * (i & 1)] + lane;
+    const float4 v = *p;
+    const float nq = sqrtf(warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w)));
+    float s = 1.0f / (nq > sh.eps ? nq : sh.eps);
+    if (!(i & 1)) s *= 0.08838834764831845f;   // 1 / sqrt(128)
+    *p = make_float4(v.x * s, v.y * s, v.z * s, v.w * s);
+  }
+  __syncthreads();
+  int slot = sc;
+#pragma unroll 1
   for (int t = 0; t < n; t++) {
     const float dec = db[t][0], bt = db[t][1];
-    float kq[32];
+    float kq[16], ka[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < 8; i++) { const float4 v = *(const float4 *)&ks[t][16 * i + 4 * cq]; kq[4 * i] = v.x; kq[4 * i + 1] = v.y; kq[4 * i + 2] = v.z; kq[4 * i + 3] = v.w; }
-    float ka[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int i = 0; i < 4; i++) { const float4 v = *(const float4 *)&ys[t][128 + 32 * i + 4 * cq]; kq[4 * i] = v.x; kq[4 * i + 1] = v.y; kq[4 * i + 2] = v.z; kq[4 * i + 3] = v.w; }
 #pragma unroll
-    for (int i = 0; i < 32; i++) { st[i] *= dec; ka[i & 3] += st[i] * kq[i]; }
+    for (int i = 0; i < 16; i++) { st[i] *= dec; ka[i & 3] += st[i] * kq[i]; }
     float kvacc = (ka[0] + ka[1]) + (ka[2] + ka[3]);
-    kvacc += __shfl_xor_sync(0xffffffffu, kvacc, 1);
-    kvacc += __shfl_xor_sync(0xffffffffu, kvacc, 2);
-    const float delta = (vs[t][jr] - kvacc) * bt;
 #pragma unroll
-    for (int i = 0; i < 32; i++) st[i] += kq[i] * delta;
-#pragma unroll
-    for (int i = 0; i < 8; i++) { const float4 v = *(const float4 *)&qs[t][16 * i + 4 * cq]; kq[4 * i] = v.x; kq[4 * i + 1] = v.y; kq[4 * i + 2] = v.z; kq[4 * i + 3] = v.w; }
+    for (int m = 1; m < 8; m <<= 1) kvacc += __shfl_xor_sync(0xffffffffu, kvacc, m);
+    const float delta = (ys[t][256 + jr] - kvacc) * bt;
     float oa[4] = {0.f, 0.f, 0.f, 0.f};
+    slot = slot + 1 == R ? 0 : slot + 1;
+    float4 *dst = (float4 *)(St + (size_t)slot * slot_sz);
 #pragma unroll
-    for (int i = 0; i < 32; i++) oa[i & 3] += st[i] * kq[i];
+    for (int i = 0; i < 4; i++) {
+      const float4 q = *(const float4 *)&ys[t][32 * i + 4 * cq];
+      st[4 * i] += kq[4 * i] * delta; st[4 * i + 1] += kq[4 * i + 1] * delta; st[4 * i + 2] += kq[4 * i + 2] * delta; st[4 * i + 3] += kq[4 * i + 3] * delta;
+      oa[0] += st[4 * i] * q.x; oa[1] += st[4 * i + 1] * q.y; oa[2] += st[4 * i + 2] * q.z; oa[3] += st[4 * i + 3] * q.w;
+      dst[8 * i] = make_float4(st[4 * i], st[4 * i + 1], st[4 * i + 2], st[4 * i + 3]);
+    }
     float oacc = (oa[0] + oa[1]) + (oa[2] + oa[3]);
-    oacc += __shfl_xor_sync(0xffffffffu, oacc, 1);
-    oacc += __shfl_xor_sync(0xffffffffu, oacc, 2);
-    if (cq == 0) os[t][jr] = oacc;
-    float4 *dst = (float4 *)(S + (size_t)((sc + t + 1) % R) * slot_sz + off);
 #pragma unroll
-    for (int i = 0; i < 8; i++) dst[4 * i] = make_float4(st[4 * i], st[4 * i + 1], st[4 * i + 2], st[4 * i + 3]);
+    for (int m = 1; m < 8; m <<= 1) oacc += __shfl_xor_sync(0xffffffffu, oacc, m);
+    if (cq == 0) os[t][jr] = oacc;
   }
   __syncthreads();
-  if (wp == 0) {
-    for (int t = 0; t < n; t++) {
-      const float v = os[t][lane], s2 = warp_sum(v * v);
-      if (lane == 0) ssq[t] = s2;
-    }
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (wp < n) {
+    const float v = os[wp][lane], s2 = warp_sum(v * v);
+    if (lane < 4) *cl.map_shared_rank(&tot[wp][jq], lane) = s2;
   }
-  cl.sync();                                   // every block's partial sums of squares are in place
-  if (tid < n) {
-    float s2 = 0.0f;
-    for (unsigned r = 0; r < 4; r++) s2 += *cl.map_shared_rank(&ssq[tid], r);   // rank order: the same sum in all four blocks
-    tot[tid] = s2;
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  float h[4] = {0.f, 0.f, 0.f, 0.f};
+  if (zon) {   // rows 4 wp .. 4 wp + 3, eight lanes a row
+    float4 zz = zl[0];
+    add4(zz, zl[1]); add4(zz, zl[2]); add4(zz, zl[3]);
+    for (int k = 4; k < z.ns; k++) add4(zz, dl_slice(z, zi, k));
+    const float4 o = *(const float4 *)&os[zt][zc];
+    h[0] = o.x * nwv.x * silu_f(zz.x); h[1] = o.y * nwv.y * silu_f(zz.y); h[2] = o.z * nwv.z * silu_f(zz.z); h[3] = o.w * nwv.w * silu_f(zz.w);
   }
-  cl.sync();                                   // nobody leaves while a peer still reads its shared memory
-  for (int t = wp; t < n; t += 4) {
-    const float r = 1.0f / sqrtf(tot[t] / 128.0f + sh.eps);
-    const int col = hh * 128 + 32 * jq;
-    const float zz = part_get(z, (size_t)t * sh.vdc + col + lane);
-    xp_store32(xp, row0 + t, 2, col, os[t][lane] * r * nwv * silu_f(zz), lane);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every block's sums of squares are here; nothing remote is touched after this
+  if (wp < 2) {
+    const float *tt = tot[zon ? zt : 0];
+    const float r = 1.0f / sqrtf((((tt[0] + tt[1]) + tt[2]) + tt[3]) / 128.0f + sh.eps);   // rank order
+#pragma unroll
+    for (int i = 0; i < 4; i++) h[i] *= r;
+    xp_store4(xp, row0 + zt, 2, col, h, lane, zon);
   }
 }
-int op_delta_fused(cudaStream_t s, float *S, const SpecCtl *ctl, const float *y, const float *beta, const float *decay, PartIn z,
-                   const float *nw, DeltaShape sh, XPlanes xp, const RowSet *rs, int nz, long long s_group) {
+int op_delta(cudaStream_t s, float *S, const SpecCtl *ctl, PartIn ring, const float *cw, PartIn bp, PartIn ap, const float *dt, const float *sa,
+             PartIn z, const float *nw, DeltaShape sh, XPlanes xp, const RowSet *rs, int nz, long long s_group) {
   if (sh.SZ != 128) return llb_fail("DeltaNet state size %d (only 128, as host/llb_host.c:1608)", sh.SZ);
-  CU_OK(llb_launch(k_delta_fused, dim3(sh.TR, 4, nz), dim3(128), (size_t)0, s, S, ctl, y, beta, decay, z, nw, sh, xp, rs, g_streams, s_group));
+  if (sh.KC > CONV_RING / 2) return llb_fail("conv kernel %d", sh.KC);
+  CU_OK(llb_launch(k_delta, dim3(sh.TR, 4, nz), dim3(DL_THREADS), (size_t)0, s, S, ctl, ring, cw, bp, ap, dt, sa, z, nw, sh, xp, rs, g_streams, s_group));
   return 0;
 }
 
@@ -484,6 +560,7 @@ __global__ void __launch_bounds__(256) k_top2_part(PartIn logits, int V, long lo
   const size_t z0 = (size_t)t * row_stride;
   const int per = (V + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * per, i1 = min(V, i0 + per);
   Top2 a = {0.f, -1, 0.f, -1};
+#pragma unroll 1
   for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) t2_push(a, part_get(logits, z0 + i), i);
   a = t2_warp(a);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
