@@ -173,7 +173,7 @@ int llb_b200_gemm(int fmt, int nmat, const llb_b200_dptr *w, const int *rows, co
   a.nmat = nmat; a.K = K; a.xp = xp->p; a.planes = xp->planes; a.T = xp->T;
   int ntiles = 0, total_rows = 0;
   for (int i = 0; i < nmat; i++) { ntiles += (rows[i] + 15) / 16; total_rows += rows[i]; }
-  a.ksplit = gemm_fix_ksplit(fmt, xp->p.NC, K / 256, ksplit > 0 ? ksplit : gemm_pick_ksplit(fmt, xp->p.NC, ntiles, K / 256, g_llb.sms));
+  a.ksplit = gemm_fix_ksplit(fmt, xp->p.NC, K / 256, ksplit > 0 ? ksplit : gemm_pick_ksplit(fmt, xp->p.NC, ntiles, K / 256, g_llb.sms, true));
   const size_t per_split = (size_t)xp->T * total_rows;
   if (a.ksplit > 1 && per_split * a.ksplit > g_parts_floats) {
     if (g_parts) {
@@ -311,7 +311,10 @@ int llb_b200_gemm_noalloc(int fmt, llb_b200_dptr w, int rows, int K, llb_b200_dp
   if (!tile_bytes(fmt)) return llb_fail("gemm_noalloc: format %d has no kernel", fmt);
   const int NC = 8;
   const int ks = gemm_pick_ksplit(fmt, NC, (rows + 15) / 16, K / 256, g_llb.sms);
-  if ((size_t)ks * T * rows > NOALLOC_PART_FLOATS)
+  // rows whose partial sums the array holds: all of them, or (where one K-slice would have fitted and the kernel needs more) a
+  // run of them at a time
+  const int run = (size_t)ks * T * rows <= NOALLOC_PART_FLOATS ? rows : (int)(NOALLOC_PART_FLOATS / ((size_t)ks * T)) & ~15;
+  if (run < rows && (size_t)T * rows > NOALLOC_PART_FLOATS)
     return llb_fail("gemm_noalloc: %d K-slices x %d rows x %d output rows need %zu floats of scratch, the built-in array holds %u",
                     ks, T, rows, (size_t)ks * T * rows, (unsigned)NOALLOC_PART_FLOATS);
   if (xp_bytes(K, NC) > NOALLOC_XP_BYTES) return llb_fail("gemm_noalloc: planes of %d columns do not fit", K);
@@ -336,15 +339,20 @@ int llb_b200_gemm_noalloc(int fmt, llb_b200_dptr w, int rows, int K, llb_b200_dp
   CU_OK(cudaMemsetAsync(scratch, 0, xp_bytes(K, NC), g_llb.stream));
   XPlanes xp = xp_carve(scratch, K, NC);
   if (ops_xp_from_f32(g_llb.stream, (const float *)(uintptr_t)x_f32, T, 2, xp)) return -1;
-  float *parts = (float *)(scratch + NOALLOC_XP_BYTES);
-  GemmArgs a;
-  memset(&a, 0, sizeof a);
-  a.nmat = 1; a.K = K; a.xp = xp; a.planes = 2; a.T = T; a.ksplit = ks;
-  a.m[0].W = (const uint8_t *)(uintptr_t)w; a.m[0].rows = rows; a.m[0].ostride = rows;
-  a.m[0].out = ks == 1 ? (float *)(uintptr_t)out_f32 : parts;
-  a.m[0].split_stride = ks == 1 ? 0 : (long long)T * rows;
-  if (gemm_launch(g_llb.stream, fmt, a)) return -1;
-  if (ks > 1 && ops_sum_parts(g_llb.stream, parts, ks, (long long)T * rows, T * rows, (float *)(uintptr_t)out_f32)) return -1;
+  float *parts = (float *)(scratch + NOALLOC_XP_BYTES), *out = (float *)(uintptr_t)out_f32;
+  for (int r0 = 0; r0 < rows; r0 += run) {
+    const int nr = rows - r0 < run ? rows - r0 : run;
+    GemmArgs a;
+    memset(&a, 0, sizeof a);
+    a.nmat = 1; a.K = K; a.xp = xp; a.planes = 2; a.T = T; a.ksplit = ks;
+    a.m[0].W = (const uint8_t *)(uintptr_t)w + dev_bytes(fmt, r0, K); a.m[0].rows = nr; a.m[0].ostride = ks == 1 ? rows : nr;
+    a.m[0].out = ks == 1 ? out + r0 : parts;
+    a.m[0].split_stride = ks == 1 ? 0 : (long long)T * nr;
+    if (gemm_launch(g_llb.stream, fmt, a)) return -1;
+    if (ks > 1 && nr == rows && ops_sum_parts(g_llb.stream, parts, ks, (long long)T * rows, T * rows, out)) return -1;
+    for (int t = 0; ks > 1 && nr < rows && t < T; t++)
+      if (ops_sum_parts(g_llb.stream, parts + (size_t)t * nr, ks, (long long)T * nr, nr, out + (size_t)t * rows + r0)) return -1;
+  }
   return 0;
 }
 

@@ -10,13 +10,32 @@ static bool is_g3(int fmt, int NC) { return g_llb.gemm3 && fmt == LLB_FM_Q4_K &&
 static unsigned int *g_ffn_sync = nullptr;   // the fused FFN's grid barrier: two counters
 static unsigned int *g_g3_err = nullptr;   // device word: set when a bounded wait of a kernel ran out
 unsigned int *gemm_err_word(void) { return g_g3_err; }
-template <int FMT, int NT> static int launch_two(cudaStream_t s, const GemmArgs &a) {
+// Cost model of a launch, in cycles of one SM.  The work of its tiles is about 45 + 6.3 cycles a plane column and
+// 16 x 256 tile, 65 + for Q5_K with its fifth bits (measured with the copies left out on the 27B shape's gate|up launch at 4, 8 and 16 rows); a warp's own
+// chain, where that is longer, about 1200 cycles a tile (two stages of copies in flight), with 350 for adding up the parts of
+// a row tile that warps share.  nc: plane columns that are multiplied
+static double gemm_stream_cost(int fmt, int warps, int nc, int tiles, int slice, int parts) {
+  const int rounds = (tiles * parts + warps - 1) / warps;
+  const double work = (double)tiles * slice * ((fmt == LLB_FM_Q5_K ? 65.0 : 45.0) + 6.3 * nc), chain = rounds * ((slice + parts - 1) / parts * 1200.0 + (parts > 1 ? 350.0 : 0.0));
+  return work > chain ? work : chain;
+}
+// Parts of a row tile's K-slice (g2_phase): the power of two with the lowest cost that divides the warps, leaves every part a
+// super-block and whose sums fit beside the activation slice.  tiles: row tiles of a CTA, nsb in ks slices
+static int gemm_pick_parts(int fmt, int NC, int ntc, int tiles, int nsb, int ks) {
+  const int warps = g2_warps(fmt, NC), slice = (nsb + ks - 1) / ks;
+  int best = 1;
+  for (int p = 2; p <= 16 && p <= nsb / ks && warps % p == 0; p *= 2)
+    if (g2_smem(fmt, slice, NC, p, ntc) <= G2_SMEM_MAX && gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, p) < gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, best)) best = p;
+  return best;
+}
+template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
   const int NC = 8 * NT, nsl = (a.nsb + a.ksplit - 1) / a.ksplit;
   int cps = g_llb.sms / a.ksplit;
   if (cps < 1) cps = 1;
   // every SM takes part as long as there is a tile for it: the tiles are dealt out one per CTA in turn
   if (cps > a.tile0[a.nmat]) cps = a.tile0[a.nmat];
-  const size_t smem = g2_smem(FMT, nsl, NC);
+  a.parts = gemm_pick_parts(FMT, NC, NT, (a.tile0[a.nmat] + cps - 1) / cps, a.nsb, a.ksplit);
+  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, NT);
   if (smem > G2_SMEM_MAX) return llb_fail("k_gemm2: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   cudaError_t e = llb_launch(k_gemm2<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
   if (e != cudaSuccess) return llb_fail("k_gemm2 launch: %s", cudaGetErrorString(e));
@@ -131,16 +150,14 @@ int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks) {
   return ks;
 }
 
-// K-slices per row tile.  In cycles of one SM: the work of its tiles (about 45 + 6.3 cycles a plane column and tile, measured
-// with the copies left out on the 27B shape's gate|up launch at 4, 8 and 16 rows), or, where a warp's own chain is longer
-// (a tile takes a warp by itself about 900 cycles), that; then the staging of the slice at 32 bytes a cycle; and
-// a charge per slice for the partial sums that the consumer has to add.
-double gemm_split_cost(int NC, int warps, int ntiles, int nsb, int ks, int sms) {
-  const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps, rounds = (tiles + warps - 1) / warps;
-  const double work = (double)tiles * slice * (45.0 + 6.3 * NC), chain = (double)rounds * slice * 900.0;
-  return ((work > chain ? work : chain) + 16.0 * NC * slice) * (1.0 + 0.025 * (ks - 1));
+// K-slices per row tile: streaming, the staging of the slice, and a charge per slice for the partial sums that the consumer
+// has to add (direct: a launch of its own adds them, 1.5 us).
+static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool direct, double stage) {
+  const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps;
+  const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, NC / 8, tiles, nsb, ks));
+  return (stream + stage * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
-int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms) {
+int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
@@ -152,7 +169,7 @@ int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms) {
       const int nt128 = (ntiles + 7) / 8;
       cost = (double)((nt128 + cps - 1) / cps) * (slice + 1.5) * (1.0 + 0.02 * (ks - 1));
     } else {
-      cost = gemm_split_cost(NC, g2_warps(fmt, NC), ntiles, nsb, ks, sms);
+      cost = gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
     }
     if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
   }
@@ -214,6 +231,7 @@ bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d) {
 int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2) {
   if (a1.nmat != 2 || a1.ksplit != 1 || a2.nmat != 1 || a1.xp.NC != 8 || a2.xp.NC != 8) return llb_fail("k_ffn: unsupported launch shape");
   if (gemm_prepare(LLB_FM_Q4_K, a1) || gemm_prepare(fmt2, a2)) return -1;
+  a1.parts = a2.parts = 1;
   if (a2.K != a1.m[0].rows || a1.m[1].rows != a1.m[0].rows) return llb_fail("k_ffn: down takes %d columns, gate/up have %d/%d rows", a2.K, a1.m[0].rows, a1.m[1].rows);
   if (fmt2 == LLB_FM_Q4_K) return launch_ffn<LLB_FM_Q4_K>(s, a1, a2);
   if (fmt2 == LLB_FM_Q5_K) return launch_ffn<LLB_FM_Q5_K>(s, a1, a2);
@@ -222,12 +240,14 @@ int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2) {
 }
 
 // ---- the routed experts' GEMMs (moe.cuh) ---------------------------------------------------------
-template <int FMT, int NT> static int launch_moe(cudaStream_t s, bool down, const GemmArgs &a, const MoeArgs &m, int ntiles, const float *wt_silu) {
+template <int FMT, int NT> static int launch_moe(cudaStream_t s, bool down, GemmArgs &a, const MoeArgs &m, int ntiles, const float *wt_silu) {
   const int NC = 8 * NT, nsl = (a.nsb + a.ksplit - 1) / a.ksplit;
   int cps = g_llb.sms / a.ksplit;
   if (cps < 1) cps = 1;
   if (cps > ntiles) cps = ntiles;
-  const size_t smem = g2_smem(FMT, nsl, NC);
+  // from the capacity of the launch, whatever rows are in use: a row's sums do not depend on its neighbours
+  a.parts = gemm_pick_parts(FMT, NC, moe_ntc<NT>(), (ntiles + cps - 1) / cps, a.nsb, a.ksplit);
+  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, moe_ntc<NT>());
   if (smem > G2_SMEM_MAX) return llb_fail("moe gemm: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   cudaError_t e;
   if (down && wt_silu) {

@@ -47,6 +47,7 @@ struct GemmArgs {
   int tile0[GEMM_MAXMAT + 1];  // prefix sums of 16-row tiles
   int K, nsb;                  // columns, super-blocks (256 columns) per row
   int ksplit;
+  int parts;                   // parts of a row tile's K-slice (a power of two), summed in order; see g2_phase
   XPlanes xp;
   int planes;                  // 2: hi/lo columns are folded into T = NC/2 tokens; 1: NC independent tokens
   int T;                       // tokens actually written

@@ -38,14 +38,15 @@ __host__ __device__ constexpr int g2_stages(int fmt, int NC) { return fmt == LLB
 // Warps of a CTA: sixteen (128 registers a thread), fewer where the rings of sixteen would leave the activation slice less than
 // the widths in use need: Q8_0's tiles are twice the size, and 32 plane columns take half of the memory.
 __host__ __device__ constexpr int g2_warps(int fmt, int NC) {
-  return fmt == LLB_FM_Q8_0 ? 12 : NC < 32 ? 16 : fmt == LLB_FM_Q6_K ? 12 : 14;
+  return fmt == LLB_FM_Q8_0 ? 12 : NC < 32 ? 16 : 12;
 }
 __host__ __device__ constexpr int g2_ring_bytes(int fmt, int NC) { return g2_warps(fmt, NC) * g2_stages(fmt, NC) * g2_chunk(fmt) * tile_bytes(fmt); }
 __host__ __device__ constexpr int g2_aux(int fmt) { return fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K ? 32 : 0; }
 __host__ __device__ constexpr int g2_xpad(int fmt) { return fmt == LLB_FM_Q6_K ? 32 : 64; }
-// bytes of shared memory of a launch whose K-slices have nsl super-blocks, for NC activation columns
-__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC) {
-  return (size_t)G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC);
+// bytes of shared memory of a launch whose K-slices have nsl super-blocks in `parts` parts, for NC activation columns (ntc
+// n-tiles of which are summed over the parts)
+__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC, int parts = 1, int ntc = 4) {
+  return (size_t)(parts > 1 ? g2_warps(fmt, NC) * ntc * 512 : 0) + G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC);
 }
 inline int g2_max_slice_sb(int fmt, int NC) {
   const int left = G2_SMEM_MAX - G2_BAR_BYTES - g2_ring_bytes(fmt, NC) - NC * g2_xpad(fmt);
@@ -372,92 +373,96 @@ template <int FMT, int NTP> struct G2MatsPlain {
   }
 };
 
-// One GEMM's work of a CTA (bid of cps * ksplit).  g2_fill requests the first tiles of every warp's ring; g2_run (after the
-// activation slice has been staged) streams the CTA's tiles through it.
+// One launch's work of a CTA (bid of cps * ksplit): fill the rings, call stage(xh_s, xsf_s, CS, sb0, nsl) -- which waits for
+// whatever produces the activations, puts the CTA's slice of the planes and its side array into shared memory and ends with
+// a block-wide barrier --, then stream the CTA's row tiles.  CTAs and warps beyond the launch's only take part in staging.
+//
+// a.parts = P warps share a row tile: its super-blocks of the slice are P parts, a warp each, and the first warp of the
+// group adds in order what the others leave in shared memory.  A small launch leaves most warps of an SM without a tile of
+// their own and the others with a chain of 1200 cycles a super-block (0.8B shape: four tiles an SM), which is what sharing a
+// tile shortens; it also needs fewer K-slices, whose partial sums the next kernel has to add.  P depends on the launch's
+// shape only, not on which of its rows are in use, so that a row's sums do not depend on its neighbours.
+//
+// Tile of (CTA ci, warp group w, round n) = (n * groups + w) * cps + ci: consecutive tiles go to different SMs, so the SMs'
+// tile counts differ by one at most.
 // NTC < NT (the routed-expert launches at 16 rows): a weight tile is multiplied with NTC = 2 of the NT staged n-tiles only,
 // the hi and lo tiles of the eight rows its own row is among (Mats::col0(tile) = first plane column of the hi tile; the
 // lo tile is NC / 2 columns on), since the epilogue keeps one row of the tile.
-struct G2Slice { int ks, ci, sb0, nsl; bool live; };
-__device__ __forceinline__ G2Slice g2_slice(const GemmArgs &a, int cps, int bid) {
-  G2Slice s;
-  s.live = bid < cps * a.ksplit;
-  s.ks = bid % a.ksplit; s.ci = bid / a.ksplit;
-  s.sb0 = (int)(((long long)s.ks * a.nsb) / a.ksplit); s.nsl = (int)(((long long)(s.ks + 1) * a.nsb) / a.ksplit) - s.sb0;
-  return s;
-}
-// The warp's sequence of copies: (row tile, first super-block of the chunk), chunk after chunk, tile after tile.
-// tile of (CTA ci, warp w, round n) = (n * WARPS + w) * cps + ci: consecutive tiles go to different SMs, so the SMs' tile
-// counts differ by one at most
-template <int FMT, class Mats> struct G2Feed {
-  int tile, c;
-  typename Mats::Cur cur;
-  __device__ __forceinline__ void next(const G2Slice &sl, int nws, int n) { c += n; if (c == sl.nsl) { c = 0; tile += nws; } }
-  __device__ __forceinline__ void issue(const Mats &mats, const G2Slice &sl, const G2Ring &rg, int s, int ntiles, int nws, int lane) {
-    constexpr int TB = tile_bytes(FMT), CH = g2_chunk(FMT);
-    if (tile >= ntiles) return;
-    if (c == 0) mats.locate(tile, sl.sb0, cur);
-    const int n = min(CH, sl.nsl - c);
+template <int FMT, int NT, class Stage, class Mats, int NTC = NT>
+__device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, G2Ring &rg, uint8_t *planes, Stage stage, const Mats mats) {
+  constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC), TB = tile_bytes(FMT), ST = g2_stages(FMT, NC), CH = g2_chunk(FMT);
+  static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool live = bid < cps * a.ksplit && warp < WARPS;
+  const int ks = bid % a.ksplit, ci = bid / a.ksplit;
+  const int sb0 = (int)(((long long)ks * a.nsb) / a.ksplit), nsl = (int)(((long long)(ks + 1) * a.nsb) / a.ksplit) - sb0;
+  const int CS = nsl * 512 + g2_xpad(FMT);
+  uint8_t *xh_s = planes, *xsf_s = planes + NC * CS;
+  const int P = a.parts, lp = 31 - __clz(P), grp = warp >> lp, mine = warp & (P - 1), nws = (WARPS >> lp) * cps;
+  const int tile0 = grp * cps + ci, c0 = (mine * nsl) >> lp, c1 = ((mine + 1) * nsl) >> lp;   // this warp's tiles; its part
+  if constexpr (!Mats::EARLY) stage(xh_s, xsf_s, CS, sb0, nsl);   // the weight addresses come from an earlier kernel's choice: the wait comes first
+  const int ntiles = live ? mats.ntiles() : 0;                    // a warp that is not live sees no tiles
+  int p_tile = tile0, p_c = c0;                                   // producer: (tile, super-block) of the next copy
+  typename Mats::Cur p_cur;
+  if (p_tile < ntiles) mats.locate(p_tile, sb0, p_cur);
+  auto issue = [&](int s) {
+    if (p_tile >= ntiles || rg.dead) return;
+    const int n = min(CH, c1 - p_c);
     if (lane == 0) {
       const uint32_t bar = rg.bar_s + 8 * s, dst = rg.ring_s + s * CH * TB;
       mbar_expect(bar, n * TB);
-      if (Mats::CONTIG || CH == 1) bulk_load(dst, mats.src(cur, sl.sb0, c), n * TB, bar);
-      else for (int u = 0; u < n; u++) bulk_load(dst + u * TB, mats.src(cur, sl.sb0, c + u), TB, bar);
+      if (Mats::CONTIG || CH == 1) bulk_load(dst, mats.src(p_cur, sb0, p_c), n * TB, bar);
+      else for (int u = 0; u < n; u++) bulk_load(dst + u * TB, mats.src(p_cur, sb0, p_c + u), TB, bar);
     }
-    next(sl, nws, n);
-  }
-};
-template <int FMT, int NC, int WARPS, class Mats>
-__device__ __forceinline__ void g2_fill(const G2Slice &sl, int cps, const G2Ring &rg, const Mats &mats) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ntiles = sl.live && warp < WARPS ? mats.ntiles() : 0;
-  G2Feed<FMT, Mats> f;
-  f.tile = warp * cps + sl.ci; f.c = 0;
+    p_c += n;
+    if (p_c == c1) {
+      p_c = c0; p_tile += nws;
+      if (p_tile < ntiles) mats.locate(p_tile, sb0, p_cur);
+    }
+  };
+  // weights first where their addresses depend on no kernel: the ring is in flight while the producer of the activations
+  // still runs, and while the activation slice is staged
 #pragma unroll 1
-  for (int s = 0; s < g2_stages(FMT, NC); s++) f.issue(mats, sl, rg, s, ntiles, cps * WARPS, lane);
-}
-template <int FMT, int NT, int WARPS, class Mats, int NTC = NT>
-__device__ __forceinline__ void g2_run(const GemmArgs &a, const G2Slice &sl, int cps, G2Ring &rg, const uint8_t *xh_s, const uint8_t *xsf_s, int CS, const Mats &mats) {
-  constexpr int NC = 8 * NT, TB = tile_bytes(FMT), ST = g2_stages(FMT, NC), CH = g2_chunk(FMT);
-  static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nws = cps * WARPS, ntiles = sl.live && warp < WARPS ? mats.ntiles() : 0;
-  G2Feed<FMT, Mats> f;
-  f.tile = warp * cps + sl.ci; f.c = 0;
-  // behind what g2_fill has requested
-  for (int s = 0; s < ST && f.tile < ntiles; s++) f.next(sl, nws, min(CH, sl.nsl - f.c));
-  if (f.c > 0 && f.tile < ntiles) mats.locate(f.tile, sl.sb0, f.cur);
+  for (int s = 0; s < ST; s++) issue(s);
+  if constexpr (Mats::EARLY) stage(xh_s, xsf_s, CS, sb0, nsl);
+  float4 *red = (float4 *)(planes + NC * (((a.nsb + a.ksplit - 1) / a.ksplit) * (512 + g2_aux(FMT)) + g2_xpad(FMT))) + warp * NTC * 32 + lane;
   int s = 0;
 #pragma unroll 1
-  for (int tile = warp * cps + sl.ci; tile < ntiles; tile += nws) {
+  for (int tile = tile0; tile < ntiles; tile += nws) {
     int cb = 0;                                            // first plane column of the computed n-tiles
     if constexpr (NTC != NT) cb = mats.col0(tile);
     float acc[NTC][4];
 #pragma unroll
     for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
 #pragma unroll 1
-    for (int c = 0; c < sl.nsl; c += CH) {
+    for (int c = c0; c < c1; c += CH) {
       if (!rg.dead && !mbar_wait(rg.bar_s + 8 * s, (rg.par >> s) & 1u, G2_WAIT_LIMIT)) { rg.dead = true; if (a.err) atomicExch(a.err, 1u); }
       rg.par ^= 1u << s;
 #pragma unroll 1
-      for (int u = 0; u < CH && c + u < sl.nsl; u++) g2_tile<FMT, NT, NTC>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
+      for (int u = 0; u < CH && c + u < c1; u++) g2_tile<FMT, NT, NTC>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
       __syncwarp();                                        // every lane has read the stage
-      f.issue(mats, sl, rg, s, ntiles, nws, lane);
+      issue(s);
       s = s + 1 == ST ? 0 : s + 1;
     }
-    mats.template epilogue<NTC>(sl.ks, tile, acc, lane);
+    if (P > 1) {
+      if (mine) {
+#pragma unroll
+        for (int nt = 0; nt < NTC; nt++) red[nt * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * P) : "memory");
+      if (!mine) {
+#pragma unroll 1
+        for (int q = 1; q < P; q++)
+#pragma unroll
+          for (int nt = 0; nt < NTC; nt++) {
+            const float4 v = red[(q * NTC + nt) * 32];
+            acc[nt][0] += v.x; acc[nt][1] += v.y; acc[nt][2] += v.z; acc[nt][3] += v.w;
+          }
+      }
+      if (tile + nws < ntiles) asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * P) : "memory");   // read before it is written again
+    }
+    if (!mine) mats.template epilogue<NTC>(ks, tile, acc, lane);
   }
-}
-// One launch: fill the ring, call stage(xh_s, xsf_s, CS, sb0, nsl) -- which waits for whatever produces the activations, puts the
-// CTA's slice of the planes and its side array into shared memory and ends with a block-wide barrier --, then stream.
-template <int FMT, int NT, class Stage, class Mats, int NTC = NT>
-__device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, G2Ring &rg, uint8_t *planes, Stage stage, const Mats mats) {
-  constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC);
-  const G2Slice sl = g2_slice(a, cps, bid);
-  const int CS = sl.nsl * 512 + g2_xpad(FMT);
-  // weights first where their addresses depend on no kernel: the ring is in flight while the producer of the activations
-  // still runs, and while the activation slice is staged
-  if constexpr (Mats::EARLY) g2_fill<FMT, NC, WARPS>(sl, cps, rg, mats);
-  stage(planes, planes + NC * CS, CS, sl.sb0, sl.nsl);
-  if constexpr (!Mats::EARLY) g2_fill<FMT, NC, WARPS>(sl, cps, rg, mats);
-  g2_run<FMT, NT, WARPS, Mats, NTC>(a, sl, cps, rg, planes, planes + NC * CS, CS, mats);
 }
 
 // The activation slice from the planes in global memory: the columns of the launch's rows only (a one-row pass uses two of
