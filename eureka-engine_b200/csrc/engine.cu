@@ -43,7 +43,7 @@ struct TensorRec { uint64_t off, bytes; int rows, cols, fmt; bool blocked = fals
 // dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows, and the row sets of the chunk.
 struct PfState {
   bool ready = false;
-  float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
+  float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *gram = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
   __half *kg_d = nullptr, *kg_f = nullptr, *kg_qa = nullptr, *kg_v = nullptr, *kg_2d = nullptr;
   OutBuf q, k, v, qkv, z, bp, ap, a, g, u, dn, eh;
   float *pm = nullptr, *pl = nullptr, *po = nullptr;   // split-K attention partials of every row group of a chunk
@@ -1033,7 +1033,7 @@ static int pf_alloc(llb_spec *m) {
   const int d = m->d, qa = m->H * m->hd;
   auto kg = [&](int K) { return (__half *)dalloc(m, (PF_RMAX / PF_R) * pf_kg_halves(K) * 2); };   // the chunk's units one after the other
   f.x = falloc(m, (size_t)PF_RMAX * d); f.x1 = falloc(m, (size_t)PF_RMAX * d); f.hn = falloc(m, (size_t)(PF_RMAX + 1) * d); f.e = falloc(m, (size_t)PF_RMAX * d);
-  f.qn = falloc(m, (size_t)PF_RMAX * qa); f.y = falloc(m, (size_t)PF_RMAX * m->convd); f.beta = falloc(m, (size_t)PF_RMAX * m->TR);
+  f.qn = falloc(m, (size_t)PF_RMAX * qa); f.y = falloc(m, (size_t)PF_RMAX * m->convd); f.beta = falloc(m, (size_t)PF_RMAX * m->TR); f.gram = falloc(m, (size_t)PF_RMAX / 8 * 64 * m->GK);
   f.decay = falloc(m, (size_t)PF_RMAX * m->TR); f.o = falloc(m, (size_t)PF_RMAX * m->vdc);
   f.kg_d = kg(d); f.kg_f = kg(m->f); f.kg_qa = kg(qa); f.kg_v = kg(m->vdc); f.kg_2d = kg(2 * d);
   {
@@ -1043,7 +1043,7 @@ static int pf_alloc(llb_spec *m) {
   }
   f.rs = (RowSet *)dalloc(m, sizeof(RowSet) * (1 + PF_GROUPS));
   f.ids = (int *)dalloc(m, (size_t)(PF_RMAX + 1) * 4);
-  if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
+  if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.gram || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
       !f.rs || !f.ids) return -1;
   f.ready = true;
   return 0;
@@ -1142,7 +1142,7 @@ static int pf_chunk(llb_spec *m, int b, const int *ids, int p0, int R) {
     } else {
       PFK("gemm qkv|z|b|a", pf_site(m, {{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));
       PFK("delta", op_pf_delta(s, as_in(f.qkv), as_in(f.z), as_in(f.bp), as_in(f.ap), ring_of(m, il, b), m->ring_ks[il], l.dn.conv, l.dn.dt, l.dn.a, l.dn.norm, dsh,
-                     state_of(m, il, b), ctl_of(m, b), f.y, f.beta, f.decay, f.o, f.kg_v, p0, R));
+                     state_of(m, il, b), ctl_of(m, b), f.y, f.gram, f.beta, f.decay, f.o, f.kg_v, p0, R));
       PFK("gemm ssm_out", pf_site(m, {{&l.dn.out, &f.a}}, f.kg_v, m->vdc, R));
     }
     PFK("norm", op_pf_norm(s, f.x, as_in(f.a), l.ffn.post, m->eps, d, f.x1, f.kg_d, d, 0, nullptr, R));

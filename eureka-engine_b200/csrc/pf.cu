@@ -16,8 +16,14 @@ template <int FMT> static int pf_attr() {
   CU_OK(cudaFuncSetAttribute(k_pfmm<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
   return 0;
 }
+#define PF_SCAN_NW 4                            // warps of a scan block, 8 state rows each
+#define PF_SCAN_BLOCKS (128 / (8 * PF_SCAN_NW)) // blocks of a head
+#define PF_SCAN_SMEM (220 * 1024)
+__global__ void k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
+                          const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R);
 int pf_setup(void) {
   if (pf_attr<LLB_FM_Q4_K>() || pf_attr<LLB_FM_Q5_K>() || pf_attr<LLB_FM_Q6_K>() || pf_attr<LLB_FM_Q8_0>()) return -1;
+  CU_OK(cudaFuncSetAttribute(k_pf_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SCAN_SMEM - 24 * 1024));
   if (!g_pf_err) {
     CU_OK(cudaMalloc(&g_pf_err, 4));
     CU_OK(cudaMemset(g_pf_err, 0, 4));
@@ -181,156 +187,345 @@ int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R) {
 }
 
 // ---- gated DeltaNet over a chunk (tools/qwen35_engine.c:581-662) -----------------------------------
-// beta = sigmoid(b), decay = exp(softplus(a + dt) * ssm_a) for every (row, head); transcendentals through double as the
-// T-row kernel k_delta_conv and the CPU engine do
-__global__ void k_pf_gates(PartIn bp, PartIn ap, const float *__restrict__ dt, const float *__restrict__ sa, int TR, float *__restrict__ beta,
-                           float *__restrict__ decay) {
-  pdl_trigger();
-  pdl_wait();
-  const int t = blockIdx.x;
-  for (int h = threadIdx.x; h < TR; h += blockDim.x) {
-    const float b = part_get(bp, (size_t)t * TR + h), a = part_get(ap, (size_t)t * TR + h);
-    beta[t * TR + h] = 1.0f / (1.0f + (float)exp((double)-b));
-    const float x = a + dt[h];
-    const float sp = x > 20.0f ? x : (float)log1p((double)(float)exp((double)(x < 88.0f ? x : 88.0f)));
-    decay[t * TR + h] = (float)exp((double)(sp * sa[h]));
+// What the scan needs, one launch: a warp takes one unit of eight rows.
+//   q or k group   conv1d + SiLU of its columns, then q / max(|q|, eps) / sqrt(128) or k / max(|k|, eps) (no eps inside the root,
+//                  :613-620).  A group's two warps share a block: k passes through shared memory, the k warp makes the rows'
+//                  products k_s . k_t (s < t), the q warp k_s . q_t (s <= t): 28 + 36 values, gram
+//   value head     conv1d + SiLU of its v columns
+//   32 gates       beta = sigmoid(b), decay = exp(softplus(a + dt) * ssm_a), head-major; transcendentals through double as
+//                  k_delta and the CPU engine do
+// conv1d: row t of the chunk (position p0 + t) reads its KC - 1 predecessors from the chunk's own raw rows or, before the
+// chunk's first row, from the position-indexed ring (tap KC - 1 is the current token, :599-600).  A lane has four channels of
+// the eight rows: a raw row is loaded 11 / 8 times instead of KC times, all rows of a K-slice in flight together.
+// MT: taps kept (the first MT - KC are zero and add exactly zero).
+#define PF_CH 8                 // rows of a scan step
+#define PF_GRAM 64
+__host__ __device__ __forceinline__ constexpr int pf_kk(int t, int s) { return t * (t - 1) / 2 + s; }          // k_s . k_t, s < t
+__host__ __device__ __forceinline__ constexpr int pf_kq(int t, int s) { return 28 + t * (t + 1) / 2 + s; }     // k_s . q_t, s <= t
+__device__ __forceinline__ float dot4(float4 a, float4 b) { return (a.x * b.x + a.y * b.y) + (a.z * b.z + a.w * b.w); }
+template <int MT>
+__device__ __forceinline__ void pf_conv_rows(const PartIn &qkv, const PartIn &ring, const float *__restrict__ cw, int convd, int KC, int p0, int R, int t0, int c, float4 (&out)[PF_CH]) {
+  constexpr int NR = PF_CH + MT - 1;
+  float4 x[NR];
+#pragma unroll
+  for (int r = 0; r < NR; r++) x[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int k = 0; k < qkv.ns; k++) {
+    const float *p = qkv.p + k * qkv.stride + c;
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+      const int t = t0 + r - (MT - 1);
+      if (t >= 0 && t < R) { const float4 l = __ldcg((const float4 *)(p + (size_t)t * convd)); x[r].x += l.x; x[r].y += l.y; x[r].z += l.z; x[r].w += l.w; }
+    }
+  }
+  if (t0 == 0) {
+#pragma unroll
+    for (int r = 0; r < MT - 1; r++)
+      if (r >= MT - KC) p_parts4(ring, (size_t)((p0 + r - (MT - 1)) & (CONV_RING - 1)) * convd + c, x[r]);
+  }
+  float w[4][MT];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int k = 0; k < MT; k++) w[i][k] = k >= MT - KC ? __ldg(cw + (size_t)(c + i) * KC + k - (MT - KC)) : 0.0f;
+#pragma unroll
+  for (int q = 0; q < PF_CH; q++) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < MT; k++) {
+      a[0] = __fadd_rn(a[0], __fmul_rn(x[q + k].x, w[0][k])); a[1] = __fadd_rn(a[1], __fmul_rn(x[q + k].y, w[1][k]));
+      a[2] = __fadd_rn(a[2], __fmul_rn(x[q + k].z, w[2][k])); a[3] = __fadd_rn(a[3], __fmul_rn(x[q + k].w, w[3][k]));
+    }
+    out[q] = make_float4(pf_silu(a[0]), pf_silu(a[1]), pf_silu(a[2]), pf_silu(a[3]));
   }
 }
-// conv1d + SiLU: row t of the chunk (position p0 + t) reads its KC - 1 predecessors from the chunk's own raw rows or,
-// before the chunk's first row, from the position-indexed ring (tap KC - 1 is the current token, :599-600)
-__global__ void k_pf_conv(PartIn qkv, PartIn ring, const float *__restrict__ cw, int convd, int KC, int p0, float *__restrict__ y) {
-  pdl_trigger();
-  pdl_wait();
-  const int t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= convd) return;
-  float acc = 0.0f;
-  for (int k = 0; k < KC; k++) {
-    const int tt = t - (KC - 1) + k;
-    const float x = tt >= 0 ? part_get(qkv, (size_t)tt * convd + c) : part_get(ring, (size_t)((p0 + tt) & (CONV_RING - 1)) * convd + c);
-    acc = __fadd_rn(acc, __fmul_rn(x, cw[c * KC + k]));
-  }
-  y[(size_t)t * convd + c] = pf_silu(acc);
-}
-// the chunk's last rows become the ring's history: whole values into slice 0, zeros into the other K-slices
-__global__ void k_pf_ring(PartIn qkv, float *__restrict__ ring, int ring_ks, long long ring_stride, int convd, int p0, int t0) {
-  pdl_trigger();
-  pdl_wait();
-  const int t = t0 + blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= convd) return;
-  const size_t dst = (size_t)((p0 + t) & (CONV_RING - 1)) * convd + c;
-  ring[dst] = part_get(qkv, (size_t)t * convd + c);
-  for (int k = 1; k < ring_ks; k++) ring[(size_t)k * ring_stride + dst] = 0.0f;
-}
-// per row and q/k group: q / max(|q|, eps) / sqrt(128), k / max(|k|, eps), in place (no eps inside the root, :613-620)
-__global__ void __launch_bounds__(128) k_pf_l2(float *__restrict__ y, int convd, int kdc, float eps) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ float red[32];
-  const int g = blockIdx.x, t = blockIdx.y, i = threadIdx.x;
-  float *q = y + (size_t)t * convd + g * 128 + i, *k = q + kdc;
-  const float qv = __ldcg(q), kv = __ldcg(k);
-  const float nq = sqrtf(pf_block_sum(qv * qv, red)), nk = sqrtf(pf_block_sum(kv * kv, red));
-  *q = qv * ((1.0f / (nq > eps ? nq : eps)) / sqrtf(128.0f));
-  *k = kv * (1.0f / (nk > eps ? nk : eps));
-}
-
-// The recurrence over the chunk's R rows.  grid (TR, 4), 128 threads, as k_delta_fused: block (hh, jq) keeps state rows
-// 32 jq .. 32 jq + 31 of value head hh in registers (thread = row jr, column quarter cq) from the first row of the chunk
-// to the last and writes the state back once.  Rows come in batches of eight through double-buffered shared memory:
-// the next batch's q, k, v, beta and decay are requested before the current batch is computed.  Per row and state
-// row j: S_j *= decay; delta = (v_j - S_j . k) * beta; S_j += k * delta; o_j = S_j . q   (:630-646)
-#define PF_SCAN_B 8
-__global__ void __launch_bounds__(128) k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y,
-                                                 const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R) {
-  __shared__ __align__(16) float qs[2][PF_SCAN_B][128], ks[2][PF_SCAN_B][128];
-  __shared__ float vs[2][PF_SCAN_B][32], db[2][PF_SCAN_B][2];
-  const int hh = blockIdx.x, jq = blockIdx.y, tid = threadIdx.x, g = hh % sh.GK, jr = tid >> 2, cq = tid & 3;
-  const size_t head_sz = 128 * 128, slot_sz = (size_t)sh.TR * head_sz;
-  const size_t off = (size_t)hh * head_sz + (size_t)(32 * jq + jr) * 128 + 4 * cq;
-  pdl_trigger();
-  float4 *Sp = (float4 *)(S + (size_t)(*(const volatile int *)&ctl->sc) * slot_sz + off);   // the committed slot: stable during the pass
-  float st[32];
+// Sums over the lanes of 32 values each: an exchange halves the values a lane holds, lane l ends with the sum of value l.
+__device__ __forceinline__ float pf_lane_sums(float (&v)[32], int lane) {
 #pragma unroll
-  for (int i = 0; i < 8; i++) { const float4 v = __ldcg(Sp + 4 * i); st[4 * i] = v.x; st[4 * i + 1] = v.y; st[4 * i + 2] = v.z; st[4 * i + 3] = v.w; }
-  pdl_wait();
-  float rq[PF_SCAN_B], rk[PF_SCAN_B], rv[PF_SCAN_B], rd = 0.0f;
-  auto fetch = [&](int b) {
+  for (int m = 16; m > 0; m >>= 1)
 #pragma unroll
-    for (int u = 0; u < PF_SCAN_B; u++) {
-      const int t = b * PF_SCAN_B + u;
-      const float *row = y + (size_t)min(t, R - 1) * sh.convd;
-      rq[u] = __ldcg(row + g * 128 + tid);
-      rk[u] = __ldcg(row + sh.kdc + g * 128 + tid);
-      rv[u] = tid < 32 ? __ldcg(row + 2 * sh.kdc + hh * 128 + 32 * jq + tid) : 0.0f;
+    for (int i = 0; i < m; i++) {
+      const float keep = lane & m ? v[i + m] : v[i], send = lane & m ? v[i] : v[i + m];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
     }
-    if (tid < 2 * PF_SCAN_B) { const int t = min(b * PF_SCAN_B + (tid >> 1), R - 1); rd = __ldcg((tid & 1) ? beta + t * sh.TR + hh : decay + t * sh.TR + hh); }
-  };
-  auto stash = [&](int buf) {
+  return v[0];
+}
+template <int MT>
+__global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const float *__restrict__ cw, PartIn bp, PartIn ap, const float *__restrict__ dt,
+                                                 const float *__restrict__ sa, DeltaShape sh, int p0, int R, float *__restrict__ y, float *__restrict__ gram,
+                                                 float *__restrict__ beta, float *__restrict__ decay) {
+  __shared__ __align__(16) float kx[2][PF_CH][128];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, t0 = blockIdx.y * PF_CH, nqk = (sh.GK + 1) / 2, nv = (sh.TR + 3) / 4;
+  int bx = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
+  if (bx < nqk) {
+    const int g = 2 * bx + (wp & 1), isk = wp >> 1;
+    const bool on = g < sh.GK;
+    float4 x[PF_CH];
+    const int c = min(g, sh.GK - 1) * 128 + 4 * lane + isk * sh.kdc;
+    pf_conv_rows<MT>(qkv, ring, cw, sh.convd, sh.KC, p0, R, t0, c, x);
 #pragma unroll
-    for (int u = 0; u < PF_SCAN_B; u++) { qs[buf][u][tid] = rq[u]; ks[buf][u][tid] = rk[u]; if (tid < 32) vs[buf][u][tid] = rv[u]; }
-    if (tid < 2 * PF_SCAN_B) db[buf][tid >> 1][tid & 1] = rd;
-  };
-  const int nb = (R + PF_SCAN_B - 1) / PF_SCAN_B;
-  fetch(0);
-  stash(0);
-  __syncthreads();
-  for (int b = 0; b < nb; b++) {
-    const int buf = b & 1;
-    if (b + 1 < nb) fetch(b + 1);
-    const int n = min(PF_SCAN_B, R - b * PF_SCAN_B);
-    for (int u = 0; u < n; u++) {
-      const float dec = db[buf][u][0], bt = db[buf][u][1];
-      float kq[32];
-#pragma unroll
-      for (int i = 0; i < 8; i++) { const float4 v = *(const float4 *)&ks[buf][u][16 * i + 4 * cq]; kq[4 * i] = v.x; kq[4 * i + 1] = v.y; kq[4 * i + 2] = v.z; kq[4 * i + 3] = v.w; }
-      float ka[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < 32; i++) { st[i] *= dec; ka[i & 3] += st[i] * kq[i]; }
-      float kvacc = (ka[0] + ka[1]) + (ka[2] + ka[3]);
-      kvacc += __shfl_xor_sync(0xffffffffu, kvacc, 1);
-      kvacc += __shfl_xor_sync(0xffffffffu, kvacc, 2);
-      const float delta = (vs[buf][u][jr] - kvacc) * bt;
-#pragma unroll
-      for (int i = 0; i < 32; i++) st[i] += kq[i] * delta;
-#pragma unroll
-      for (int i = 0; i < 8; i++) { const float4 v = *(const float4 *)&qs[buf][u][16 * i + 4 * cq]; kq[4 * i] = v.x; kq[4 * i + 1] = v.y; kq[4 * i + 2] = v.z; kq[4 * i + 3] = v.w; }
-      float oa[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < 32; i++) oa[i & 3] += st[i] * kq[i];
-      float oacc = (oa[0] + oa[1]) + (oa[2] + oa[3]);
-      oacc += __shfl_xor_sync(0xffffffffu, oacc, 1);
-      oacc += __shfl_xor_sync(0xffffffffu, oacc, 2);
-      if (cq == 0) o[(size_t)(b * PF_SCAN_B + u) * sh.vdc + hh * 128 + 32 * jq + jr] = oacc;
+    for (int t = 0; t < PF_CH; t++) {
+      const float nx = sqrtf(pf_warp_sum(dot4(x[t], x[t])));
+      const float ix = (isk ? 1.0f : 0.08838834764831845f) / (nx > sh.eps ? nx : sh.eps);   // 1 / sqrt(128)
+      x[t].x *= ix; x[t].y *= ix; x[t].z *= ix; x[t].w *= ix;
+      if (on && t0 + t < R) *(float4 *)(y + (size_t)(t0 + t) * sh.convd + c) = x[t];
+      if (isk) *(float4 *)&kx[wp & 1][t][4 * lane] = x[t];
     }
-    if (b + 1 < nb) stash(buf ^ 1);
     __syncthreads();
+    float *G = gram + ((size_t)g * (PF_RMAX / PF_CH) + blockIdx.y) * PF_GRAM;
+    float v[32];
+    if (isk) {
+#pragma unroll
+      for (int t = 0; t < PF_CH; t++)
+#pragma unroll
+        for (int s = 0; s < t; s++) v[pf_kk(t, s)] = dot4(x[s], x[t]);
+#pragma unroll
+      for (int i = 28; i < 32; i++) v[i] = 0.0f;
+      const float r = pf_lane_sums(v, lane);
+      if (on && lane < 28) G[lane] = r;
+    } else {
+      float last[4];
+#pragma unroll
+      for (int s = 0; s < PF_CH; s++) {
+        const float4 k = *(const float4 *)&kx[wp & 1][s][4 * lane];
+#pragma unroll
+        for (int t = s; t < PF_CH; t++) {
+          const float d = dot4(k, x[t]);
+          if (pf_kq(t, s) - 28 < 32) v[pf_kq(t, s) - 28] = d;
+          else last[pf_kq(t, s) - 60] = d;
+        }
+      }
+      const float r = pf_lane_sums(v, lane);
+#pragma unroll
+      for (int i = 0; i < 4; i++) last[i] = pf_warp_sum(last[i]);
+      if (on) {
+        G[28 + lane] = r;
+        if (lane == 0) *(float4 *)(G + 60) = make_float4(last[0], last[1], last[2], last[3]);
+      }
+    }
+    return;
+  }
+  bx -= nqk;
+  if (bx < nv) {
+    const int h = bx * 4 + wp, c = 2 * sh.kdc + h * 128 + 4 * lane;
+    if (h >= sh.TR) return;
+    float4 v[PF_CH];
+    pf_conv_rows<MT>(qkv, ring, cw, sh.convd, sh.KC, p0, R, t0, c, v);
+#pragma unroll
+    for (int t = 0; t < PF_CH; t++)
+      if (t0 + t < R) *(float4 *)(y + (size_t)(t0 + t) * sh.convd + c) = v[t];
+    return;
+  }
+  const int i = (bx - nv) * 128 + threadIdx.x, t = t0 + i / sh.TR, h = i % sh.TR;
+  if (i >= PF_CH * sh.TR || t >= R) return;
+  const float b = part_get(bp, (size_t)t * sh.TR + h), a = part_get(ap, (size_t)t * sh.TR + h);
+  beta[h * PF_RMAX + t] = 1.0f / (1.0f + (float)exp((double)-b));
+  const float x = a + dt[h];
+  const float sp = x > 20.0f ? x : (float)log1p((double)(float)exp((double)(x < 88.0f ? x : 88.0f)));
+  decay[h * PF_RMAX + t] = (float)exp((double)(sp * sa[h]));
+}
+// The recurrence over the chunk's R rows.  Block (hh, y) keeps 32 state rows of value head hh in registers from the first
+// row of the chunk to the last and writes them back once (a lane: four state rows, columns 4 cq .. and 64 + 4 cq ..).  Per row t and state row j: S_j *= decay; delta = (v_j - S_j . k) * beta; S_j += k * delta; o_j = S_j . q
+// (:630-646).
+//
+// Row by row that is a chain: a dot product, its shuffles, the update, 0.4 to 0.6 us a row.  Here a step takes eight rows.  With
+// S the state before them and d(s, t] the product of decays of rows s + 1 .. t,
+//     delta_t = beta_t (v_t - d[0, t] S . k_t - sum_{s < t} d(s, t] (k_s . k_t) delta_s)
+//     o_t     = d[0, t] S . q_t + sum_{s <= t} d(s, t] (k_s . q_t) delta_s
+//     S      <- d[0, 7] S + sum_s d(s, 7] delta_s k_s
+// so the sixteen dot products of a state row with S run side by side, their sums over the sixteen lanes are one exchange
+// tree (64 values, 60 shuffles) that leaves row t's sums of two state rows in a lane, and the chain is the substitution: eight
+// steps of a shuffle (which hands every lane delta_s for the update) and a multiply-add.  The decays' products never
+// divide, so a decay of nearly zero does no harm.  Multiply-adds: three a state element and row instead of four, two an
+// instruction.  Sixteen lanes a state row, not eight: the loads of q and k, which every state row repeats, were the longer
+// part of a step with eight (shared memory: 66 us a chunk of the 48-head shape against 48).  What bounds it now is one warp's
+// chain: 580 instructions a step in 2500 cycles.  The ops between a DeltaNet layer's GEMMs, before and now: 84.5 -> 55 ms of a
+// 3011-token prompt (48 layers, 48 heads), 47 -> 28 ms of 4096 tokens (24 layers, 32 heads), 23 -> 9.7 ms of 2000 tokens (18
+// layers, 8 heads).
+// Rows come through double-buffered shared memory, the next eight requested before the present ones are computed.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 x2_pack(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void x2_unpack(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 x2_fma(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 x2_mul(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
+                                                     const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R) {
+  constexpr int NT = 32 * PF_SCAN_NW, NJ = 8 * PF_SCAN_NW, VS = NJ + 4;   // a block's threads and state rows; v rows padded so that eight lanes' reads miss one another's banks
+  __shared__ __align__(16) float qs[2][PF_CH][128], ks[2][PF_CH][128], vs[2][PF_CH][VS], gs[2][PF_GRAM], bs[2][PF_CH], ds[2][PF_CH];
+  const int hh = blockIdx.x, jq = blockIdx.y, tid = threadIdx.x, g = hh % sh.GK, jg = tid >> 4, cq = tid & 15, tq = tid & 7, rh = (tid >> 3) & 1;
+  pdl_trigger();
+  const size_t head_sz = 128 * 128, slot_sz = (size_t)sh.TR * head_sz;
+  float4 *Sp = (float4 *)(S + (size_t)(*(const volatile int *)&ctl->sc) * slot_sz + (size_t)hh * head_sz + (size_t)(NJ * jq + 4 * jg) * 128 + 4 * cq);   // the committed slot: stable during the pass
+  f32x2 st[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int i = 0; i < 2; i++) { const float4 v = __ldcg(Sp + 32 * r + 16 * i); st[r][2 * i] = x2_pack(v.x, v.y); st[r][2 * i + 1] = x2_pack(v.z, v.w); }
+  pdl_wait();
+  const int nb = (R + PF_CH - 1) / PF_CH;
+  auto stage = [&](int b) {   // rows past the chunk repeat its last one; their beta counts as zero and their decay as one
+    const int buf = b & 1;
+#pragma unroll
+    for (int i = tid; i < PF_CH * 32; i += NT) {
+      const int r = i >> 5, c = 4 * (i & 31);
+      const float *row = y + (size_t)min(b * PF_CH + r, R - 1) * sh.convd + g * 128 + c;
+      cp_async16(smem_u32(&qs[buf][r][c]), row);
+      cp_async16(smem_u32(&ks[buf][r][c]), row + sh.kdc);
+    }
+    for (int i = tid; i < PF_CH * NJ / 4; i += NT) {
+      const int r = i / (NJ / 4), c = 4 * (i % (NJ / 4));
+      cp_async16(smem_u32(&vs[buf][r][c]), y + (size_t)min(b * PF_CH + r, R - 1) * sh.convd + 2 * sh.kdc + hh * 128 + NJ * jq + c);
+    }
+    if (tid < PF_GRAM / 4) cp_async16(smem_u32(&gs[buf][4 * tid]), gram + ((size_t)g * (PF_RMAX / PF_CH) + b) * PF_GRAM + 4 * tid);
+    else if (tid < PF_GRAM / 4 + 2) cp_async16(smem_u32(&bs[buf][4 * (tid & 1)]), beta + hh * PF_RMAX + b * PF_CH + 4 * (tid & 1));
+    else if (tid < PF_GRAM / 4 + 4) cp_async16(smem_u32(&ds[buf][4 * (tid & 1)]), decay + hh * PF_RMAX + b * PF_CH + 4 * (tid & 1));
+  };
+  stage(0);
+  cp_async_commit();
+  float *op = o + hh * 128 + NJ * jq + 4 * jg + 2 * rh;
+  for (int b = 0; b < nb; b++) {
+    const int buf = b & 1, n = min(PF_CH, R - b * PF_CH);
+    cp_async_wait<0>();
+    __syncthreads();   // the present rows are there, and nobody reads the buffer of the next ones any more
+    if (b + 1 < nb) stage(b + 1);
+    cp_async_commit();
+    f32x2 k[PF_CH][4];
+    float kv[4][PF_CH], qv[4][PF_CH];
+#pragma unroll
+    for (int t = 0; t < PF_CH; t++) {
+      f32x2 q[4];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const ulonglong2 a = *(const ulonglong2 *)&ks[buf][t][64 * i + 4 * cq], c = *(const ulonglong2 *)&qs[buf][t][64 * i + 4 * cq];
+        k[t][2 * i] = a.x; k[t][2 * i + 1] = a.y; q[2 * i] = c.x; q[2 * i + 1] = c.y;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        f32x2 a = x2_mul(st[r][0], k[t][0]), c = x2_mul(st[r][0], q[0]);
+#pragma unroll
+        for (int i = 1; i < 4; i++) { a = x2_fma(st[r][i], k[t][i], a); c = x2_fma(st[r][i], q[i], c); }
+        float lo, hi;
+        x2_unpack(a, lo, hi); kv[r][t] = lo + hi;
+        x2_unpack(c, lo, hi); qv[r][t] = lo + hi;
+      }
+    }
+    // the exchange over lane bit 3 keeps two of the four state rows, those over bits 2 .. 0 row t of the eight
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int t = 0; t < PF_CH; t++) {
+        const float kk = rh ? kv[r + 2][t] : kv[r][t], sk = rh ? kv[r][t] : kv[r + 2][t];
+        const float kq = rh ? qv[r + 2][t] : qv[r][t], sq = rh ? qv[r][t] : qv[r + 2][t];
+        kv[r][t] = kk + __shfl_xor_sync(0xffffffffu, sk, 8);
+        qv[r][t] = kq + __shfl_xor_sync(0xffffffffu, sq, 8);
+      }
+#pragma unroll
+    for (int m = 4; m > 0; m >>= 1)
+#pragma unroll
+      for (int i = 0; i < m; i++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          const float kk = tq & m ? kv[r][i + m] : kv[r][i], sk = tq & m ? kv[r][i] : kv[r][i + m];
+          const float kq = tq & m ? qv[r][i + m] : qv[r][i], sq = tq & m ? qv[r][i] : qv[r][i + m];
+          kv[r][i] = kk + __shfl_xor_sync(0xffffffffu, sk, m);
+          qv[r][i] = kq + __shfl_xor_sync(0xffffffffu, sq, m);
+        }
+    // lane tq is row t = tq from here on
+    float dec[PF_CH], M[PF_CH], N[PF_CH], e[PF_CH];
+#pragma unroll
+    for (int s = 0; s < PF_CH; s++) dec[s] = s < n ? ds[buf][s] : 1.0f;
+    const float bt = tq < n ? bs[buf][tq] : 0.0f;
+    float w = 1.0f;
+#pragma unroll
+    for (int s = PF_CH - 1; s >= 0; s--) {
+      if (s + 1 < PF_CH) w = s < tq ? w * dec[s + 1] : 1.0f;
+      M[s] = s < tq ? bt * w * gs[buf][pf_kk(tq, 0) + s] : 0.0f;
+      N[s] = s <= tq ? w * gs[buf][pf_kq(tq, 0) + s] : 0.0f;
+    }
+    const float P = w * dec[0];
+    e[PF_CH - 1] = 1.0f;
+#pragma unroll
+    for (int s = PF_CH - 2; s >= 0; s--) e[s] = e[s + 1] * dec[s + 1];
+    const float P7 = e[0] * dec[0];
+    const float2 vv = *(const float2 *)&vs[buf][tq][4 * jg + 2 * rh];
+    float x[2] = {bt * (vv.x - P * kv[0][0]), bt * (vv.y - P * kv[1][0])}, ov[2] = {P * qv[0][0], P * qv[1][0]};
+    const f32x2 pp = x2_pack(P7, P7);
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) st[r][i] = x2_mul(st[r][i], pp);
+#pragma unroll
+    for (int s = 0; s < PF_CH; s++) {
+      float d[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) d[r] = __shfl_sync(0xffffffffu, x[r & 1], s + 8 * (r >> 1), 16);
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const float dr = rh ? d[r + 2] : d[r];
+        x[r] -= M[s] * dr;
+        ov[r] += N[s] * dr;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const f32x2 d2 = x2_pack(e[s] * d[r], e[s] * d[r]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) st[r][i] = x2_fma(k[s][i], d2, st[r][i]);
+      }
+    }
+    if (tq < n) *(float2 *)(op + (size_t)(b * PF_CH + tq) * sh.vdc) = make_float2(ov[0], ov[1]);
   }
 #pragma unroll
-  for (int i = 0; i < 8; i++) Sp[4 * i] = make_float4(st[4 * i], st[4 * i + 1], st[4 * i + 2], st[4 * i + 3]);
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      float4 v;
+      x2_unpack(st[r][2 * i], v.x, v.y); x2_unpack(st[r][2 * i + 1], v.z, v.w);
+      Sp[32 * r + 16 * i] = v;
+    }
 }
-// gated RMSNorm of each head's output -> activations of ssm_out (:648-654); a warp per (head, row)
-__global__ void __launch_bounds__(32) k_pf_gnorm(const float *__restrict__ o, PartIn z, const float *__restrict__ nw, int vdc, float eps, __half *__restrict__ kg) {
+// gated RMSNorm of each head's output -> activations of ssm_out (:648-654); a warp per (head, row), eight rows a block.  One more
+// block a head copies the chunk's last raw rows into the conv history: whole values into K-slice 0, zeros into the rest
+// (here, because the conv kernel's first rows still read the old history).
+__global__ void __launch_bounds__(256) k_pf_gnorm(const float *__restrict__ o, PartIn z, const float *__restrict__ nw, DeltaShape sh, __half *__restrict__ kg,
+                                                  PartIn qkv, float *__restrict__ ring, int ring_ks, int p0, int R) {
+  const int hh = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5), i = threadIdx.x & 31;
+  const float4 w = __ldg((const float4 *)(nw + 4 * i));
   pdl_trigger();
   pdl_wait();
-  const int hh = blockIdx.x, t = blockIdx.y, i = threadIdx.x;
-  const size_t idx = (size_t)t * vdc + hh * 128 + 4 * i;
-  const float4 v = __ldcg((const float4 *)(o + idx)), zz = part_get4(z, idx), w = *(const float4 *)(nw + 4 * i);
-  const float r = 1.0f / sqrtf(pf_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) / 128.0f + eps);
-  pf_kg_store4(kg, vdc, t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
+  if (blockIdx.y == gridDim.y - 1) {
+    const int nr = min(R, CONV_RING), nc = sh.convd / 4;
+    for (int j = hh * 256 + threadIdx.x; j < nr * nc; j += sh.TR * 256) {
+      const int tr = R - nr + j / nc, c = 4 * (j % nc);
+      const size_t dst = (size_t)((p0 + tr) & (CONV_RING - 1)) * sh.convd + c;
+      *(float4 *)(ring + dst) = part_get4(qkv, (size_t)tr * sh.convd + c);
+      for (int k = 1; k < ring_ks; k++) *(float4 *)(ring + (size_t)k * CONV_RING * sh.convd + dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    return;
+  }
+  if (t >= R) return;
+  const size_t idx = (size_t)t * sh.vdc + hh * 128 + 4 * i;
+  const float4 v = __ldcg((const float4 *)(o + idx)), zz = part_get4(z, idx);
+  const float r = 1.0f / sqrtf(pf_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) / 128.0f + sh.eps);
+  pf_kg_store4(kg, sh.vdc, t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
 }
 
 // One DeltaNet layer's ops between its input GEMM (qkv | z | beta | alpha) and its output GEMM, for R rows at p0 ...
 int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, float *ring, int ring_ks, const float *cw, const float *dt, const float *sa,
-                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *beta, float *decay, float *o, __half *kg, int p0, int R) {
+                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int p0, int R) {
   if (sh.SZ != 128 || sh.KC > CONV_RING / 2) return llb_fail("pf delta: state size %d, conv kernel %d", sh.SZ, sh.KC);
   const long long rstride = (long long)CONV_RING * sh.convd;
-  CU_OK(llb_launch(k_pf_gates, dim3(R), dim3(64), (size_t)0, s, bp, ap, dt, sa, sh.TR, beta, decay));
-  CU_OK(llb_launch(k_pf_conv, dim3((sh.convd + 255) / 256, R), dim3(256), (size_t)0, s, qkv, PartIn{ring, ring_ks, rstride}, cw, sh.convd, sh.KC, p0, y));
-  const int nr = R < CONV_RING ? R : CONV_RING;
-  CU_OK(llb_launch(k_pf_ring, dim3((sh.convd + 255) / 256, nr), dim3(256), (size_t)0, s, qkv, ring, ring_ks, rstride, sh.convd, p0, R - nr));
-  CU_OK(llb_launch(k_pf_l2, dim3(sh.GK, R), dim3(128), (size_t)0, s, y, sh.convd, sh.kdc, sh.eps));
-  CU_OK(llb_launch(k_pf_scan, dim3(sh.TR, 4), dim3(128), (size_t)0, s, S, ctl, (const float *)y, (const float *)beta, (const float *)decay, sh, o, R));
-  CU_OK(llb_launch(k_pf_gnorm, dim3(sh.TR, R), dim3(32), (size_t)0, s, (const float *)o, z, nw, sh.vdc, sh.eps, kg));
+  const dim3 cgrid((sh.GK + 1) / 2 + (sh.TR + 3) / 4 + (PF_CH * sh.TR + 127) / 128, (R + PF_CH - 1) / PF_CH);
+  const PartIn rin{ring, ring_ks, rstride};
+  if (sh.KC <= 4) CU_OK(llb_launch(k_pf_conv<4>, cgrid, dim3(128), (size_t)0, s, qkv, rin, cw, bp, ap, dt, sa, sh, p0, R, y, gram, beta, decay));
+  else CU_OK(llb_launch(k_pf_conv<CONV_RING / 2>, cgrid, dim3(128), (size_t)0, s, qkv, rin, cw, bp, ap, dt, sa, sh, p0, R, y, gram, beta, decay));
+  // A block's chain takes as long alone as with others on its SM, but the scheduler stacks blocks on few SMs while others idle
+  // (32-head shape: 38 ms of a 4096-token prompt so, 28 ms spread): a block asks for the shared memory of its even share of an SM.
+  const int blocks = sh.TR * PF_SCAN_BLOCKS, per = (blocks + g_llb.sms - 1) / g_llb.sms;
+  const size_t pad = per < 6 ? (size_t)(PF_SCAN_SMEM / per - 24 * 1024) : 0;
+  CU_OK(llb_launch(k_pf_scan, dim3(sh.TR, PF_SCAN_BLOCKS), dim3(32 * PF_SCAN_NW), pad, s, S, ctl, (const float *)y, (const float *)gram, (const float *)beta, (const float *)decay, sh, o, R));
+  CU_OK(llb_launch(k_pf_gnorm, dim3(sh.TR, (R + 7) / 8 + 1), dim3(256), (size_t)0, s, (const float *)o, z, nw, sh, kg, qkv, ring, ring_ks, p0, R));
   return 0;
 }
 

@@ -28,4 +28,4 @@ int op_pf_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const int *ids
 int op_pf_norm(cudaStream_t s, const float *xin, PartIn add, const float *w, float eps, int d, float *xout, __half *kg, int kg_K, int kg_col0, float *hn_out, int R);
 int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R);
 int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, float *ring, int ring_ks, const float *cw, const float *dt, const float *sa,
-                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *beta, float *decay, float *o, __half *kg, int p0, int R);
+                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int p0, int R);   // gram: GK x PF_RMAX / 8 x 64
