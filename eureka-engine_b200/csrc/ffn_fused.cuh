@@ -48,7 +48,7 @@ template <int FMT> __device__ __forceinline__ void ffn_store4(uint8_t *xh_s, uin
   }
   {
     const __half2 a = __halves2half2(hi[0], hi[2]), b = __halves2half2(hi[1], hi[3]);
-    const int o = g2_xpos<FMT, 1>(c >> 3) + (c & 4) * 2;
+    const int o = g2_xpos<FMT, false>(c >> 3) + (c & 4) * 2;
     *(uint2 *)(xh_s + (size_t)t * CS + o) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
     const __half2 e = __halves2half2(lo[0], lo[2]), f = __halves2half2(lo[1], lo[3]);
     *(uint2 *)(xh_s + (size_t)(NH + t) * CS + o) = make_uint2(*(const uint32_t *)&e, *(const uint32_t *)&f);
@@ -113,9 +113,9 @@ __global__ void __launch_bounds__(G2_MAXWARPS * 32, 1) k_ffn(const GemmArgs a1, 
   constexpr int RB1 = g2_ring_bytes(LLB_FM_Q4_K, 8), RB2 = g2_ring_bytes(FMT2, 8), RB = RB1 > RB2 ? RB1 : RB2;
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, RB / G2_MAXWARPS);
-  g2_phase<LLB_FM_Q4_K, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K, 1>{a1});
+  g2_phase<LLB_FM_Q4_K, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K>{a1});
   __syncthreads();   // the CTA is done with the first launch's planes
   g2_phase<FMT2, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err},
-                    G2MatsPlain<FMT2, 1>{a2});
+                    G2MatsPlain<FMT2>{a2});
   g2_drain(rg);
 }

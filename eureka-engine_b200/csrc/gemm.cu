@@ -37,7 +37,8 @@ template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
   a.parts = gemm_pick_parts(FMT, NC, NT, (a.tile0[a.nmat] + cps - 1) / cps, a.nsb, a.ksplit);
   const size_t smem = g2_smem(FMT, nsl, NC, a.parts, NT);
   if (smem > G2_SMEM_MAX) return llb_fail("k_gemm2: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
-  cudaError_t e = llb_launch(k_gemm2<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
+  const bool fold = (long long)a.tile0[a.nmat] * a.nsb >= G2_FOLD_TILES;
+  cudaError_t e = llb_launch(fold ? k_gemm2<FMT, NT, g2_folds(FMT, NT)> : k_gemm2<FMT, NT, false>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
   if (e != cudaSuccess) return llb_fail("k_gemm2 launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -99,9 +100,10 @@ int gemm_wait_selftest(cudaStream_t s, int which, int limit) {
 }
 
 template <int FMT> static int setup_fmt2() {
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
+  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
+  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
+  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
+  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 4, g2_folds(FMT, 4)>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
   return 0;
 }
 

@@ -5,13 +5,14 @@
 //  * a warp's piece of work is one tile of 16 rows x 256 columns (common.cuh), which one bulk copy brings into the warp's
 //    private ring of two or three stages (an mbarrier a stage, no copy instructions in the other lanes).  Per-lane
 //    16-byte copies took 30 of the loop's 397 instructions, most of them integer adds;
-//  * Q4_K / Q5_K, up to 8 rows: a code in the low bits of an fp16 lane is the subnormal code * 2^-24, so two MMAs sum
+//  * Q4_K / Q5_K: a code in the low bits of an fp16 lane is the subnormal code * 2^-24, so two MMAs sum
 //    code * x of a 32-column sub-block exactly; the six-bit scale multiplies that fp32 sum, d the super-block's;
-//  * Q4_K / Q5_K, 16 rows (four n-tiles): the scale is multiplied into the codes instead, since sc * q <= 63 * 31 = 1953 is an
-//    exact fp16 integer: one HMUL2 a fragment register, shared by the n-tiles, and the MMAs of a whole super-block accumulate
-//    into one fragment.  Lane j of a row's four lanes then holds the k indices of column group j (64 columns, two
-//    sub-blocks) and needs that group's scales only.  gate|up of the 27B shape: 59 us against 64; with one n-tile the
-//    HMUL2s (half rate) cost more than the scales save, 31 us against 26;
+//  * Q4_K, 16 rows (four n-tiles), large launches: the scale is multiplied into the codes instead (FOLD), since sc * q <=
+//    63 * 15 is an exact fp16 integer: one HMUL2 a fragment register, shared by the n-tiles, and the MMAs of a whole super-block
+//    accumulate into one fragment.  Lane j of a row's four lanes then holds the k indices of column group j (64 columns, two
+//    sub-blocks) and needs that group's scales only.  The chain of MMAs into one fragment is longer, so it takes enough
+//    tiles an SM to hide it: gate|up of the 27B shape (43520 tiles) 62 us against 69, 12288 x 2048 (6144 tiles) 22.5
+//    against 17.4; with one n-tile the HMUL2s (half rate) cost more than the scales save, 31 us against 26;
 //  * the "min" term  dmin * sum_b m_b * sum(x in sub-block b)  is ONE extra MMA per tile: A = the eight mins as fp16 numbers
 //    (m against the means' hi halves, m / 2048 against their lo halves), B = the sub-block activation means;
 //  * Q6_K / Q8_0: a scale times a code does not fit fp16 exactly, so the scale multiplies the fp32 partial sum of its 16 or
@@ -53,10 +54,16 @@ inline int g2_max_slice_sb(int fmt, int NC) {
   return left / (NC * (512 + g2_aux(fmt)));
 }
 
-// Where the 16-byte piece of columns c .. c+7 of a slice sits in a plane column (bytes).  Q4_K / Q5_K: lane j reads column group
+// whether a launch of `work` 16 x 256 tiles has the scales folded into the codes: measured at 16 rows, the line lies between
+// 10000 tiles (25.4 us folded, 21.2 not) and 12800 (29.8 folded, 31.2 not); Q5_K, whose codes take more to assemble, gains
+// nothing at 12800 (30.9 against 30.5) and 3 % at 43520
+__host__ __device__ constexpr bool g2_folds(int fmt, int NT) { return NT == 4 && fmt == LLB_FM_Q4_K; }
+#define G2_FOLD_TILES 12000
+
+// Where the 16-byte piece of columns c .. c+7 of a slice sits in a plane column (bytes).  Folded: lane j reads column group
 // j, so the pieces of the four groups that are read together lie side by side; the others keep their order.
-template <int FMT, int NT> __device__ __forceinline__ int g2_xpos(int piece) {
-  if constexpr ((FMT == LLB_FM_Q4_K || FMT == LLB_FM_Q5_K) && NT > 2) return ((piece & ~31) | ((piece & 7) << 2) | ((piece >> 3) & 3)) * 16;
+template <int FMT, bool FOLD> __device__ __forceinline__ int g2_xpos(int piece) {
+  if constexpr (FOLD) return ((piece & ~31) | ((piece & 7) << 2) | ((piece >> 3) & 3)) * 16;
   else return piece * 16;
 }
 
@@ -86,8 +93,8 @@ __device__ __forceinline__ void bulk_load(uint32_t dst_s, const void *src, uint3
 
 // Fragment row gid (and gid + 8) of a tile is tile row g2_row(gid) (+ 8).  Q8_0 reads eight bytes a lane: even rows and odd
 // rows fall on different banks, consecutive rows do not.
-template <int FMT, int NT> __device__ __forceinline__ int g2_row(int gid) {
-  if constexpr (FMT == LLB_FM_Q8_0 || (FMT != LLB_FM_Q6_K && NT <= 2)) return ((gid & 3) << 1) | (gid >> 2);
+template <int FMT, bool FOLD> __device__ __forceinline__ int g2_row(int gid) {
+  if constexpr (FMT != LLB_FM_Q6_K && !FOLD) return ((gid & 3) << 1) | (gid >> 2);
   else return gid;
 }
 
@@ -103,10 +110,10 @@ __device__ __forceinline__ void g2_group_scales(uint32_t u0, uint32_t u1, uint32
 // One staged tile times the staged planes of super-block c_c of the slice: acc[nt] += the tile's contribution to n-tile nt.
 //   st     the tile (shared memory);  xh_s, xsf_s, CS  the staged planes, means and column stride;  cb  first plane column
 //   NTS    plane columns from one computed n-tile to the next
-template <int FMT, int NT, int NTC>
+template <int FMT, int NT, int NTC, bool FOLD>
 __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, const uint8_t *xsf_s, const int CS, const int c_c, const int cb, const int lane, float (&acc)[NTC][4]) {
   constexpr int NC = 8 * NT, NTS = NTC == NT ? 8 : NC / 2;
-  const int gid = lane >> 2, j = lane & 3, r0 = g2_row<FMT, NT>(gid);
+  const int gid = lane >> 2, j = lane & 3, r0 = g2_row<FMT, FOLD>(gid);
   const uint8_t *b0 = st + r0 * tile_row(FMT), *b1 = b0 + 8 * tile_row(FMT);
   const uint8_t *xb = xh_s + (gid + cb) * CS + (size_t)c_c * 512;
   if constexpr (FMT == LLB_FM_Q8_0) {
@@ -188,7 +195,7 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
   } else {
     constexpr int QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
     const uint4 h0 = *(const uint4 *)b0, h1 = *(const uint4 *)b1;
-    if constexpr (NT <= 2) {
+    if constexpr (!FOLD) {
       uint32_t scA0, scB0, mnA0, mnB0, scA1, scB1, mnA1, mnB1;
       k4_scales(h0.y, h0.z, h0.w, scA0, scB0, mnA0, mnB0);
       k4_scales(h1.y, h1.z, h1.w, scA1, scB1, mnA1, mnB1);
@@ -274,30 +281,17 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
       mma16816_z(pm[nt], am0, am1, al0, al1, xf.x, xf.y);
     }
     xb += 16 * j;
-    const int rl = FMT == LLB_FM_Q5_K ? (4 - 2 * j) & 31 : 0;     // rotates bit 2 j of a byte to bit 4
 #pragma unroll
     for (int q = 0; q < 4; q++) {        // words 2 q and 2 q + 1 of the group's 32 bytes: columns 8 q .. 8 q + 7 of both sub-blocks
       const uint2 a0 = *(const uint2 *)(b0 + QOFF + 32 * j + 8 * q), a1 = *(const uint2 *)(b1 + QOFF + 32 * j + 8 * q);
-      uint2 f0 = make_uint2(0u, 0u), f1 = f0;
-      if constexpr (FMT == LLB_FM_Q5_K) { f0 = *(const uint2 *)(b0 + 16 + 8 * q); f1 = *(const uint2 *)(b1 + 16 + 8 * q); }
       uint32_t A[2][2][4];               // [word][low / high nibbles]
 #pragma unroll
       for (int w = 0; w < 2; w++) {
         const uint32_t x0 = w ? a0.y : a0.x, x1 = w ? a1.y : a1.x, y0 = x0 >> 8, y1 = x1 >> 8;
-        if constexpr (FMT == LLB_FM_Q4_K) {
-          A[w][0][0] = g2_hmul2(x0 & 0x000f000fu, L0); A[w][0][1] = g2_hmul2(x1 & 0x000f000fu, L1);
-          A[w][0][2] = g2_hmul2(y0 & 0x000f000fu, L0); A[w][0][3] = g2_hmul2(y1 & 0x000f000fu, L1);
-          A[w][1][0] = g2_hmul2(x0 & 0x00f000f0u, H0); A[w][1][1] = g2_hmul2(x1 & 0x00f000f0u, H1);
-          A[w][1][2] = g2_hmul2(y0 & 0x00f000f0u, H0); A[w][1][3] = g2_hmul2(y1 & 0x00f000f0u, H1);
-        } else {
-          const uint32_t z0 = w ? f0.y : f0.x, z1 = w ? f1.y : f1.x;
-          const uint32_t u0 = __funnelshift_l(z0, z0, rl), u1 = __funnelshift_l(z1, z1, rl);         // fifth bits at 4 (low), 5 (high) of every byte
-          const uint32_t v0 = u0 << 3, v1 = u1 << 3, t0 = u0 >> 8, t1 = u1 >> 8, s0 = u0 >> 5, s1 = u1 >> 5;   // high ones at 8
-          A[w][0][0] = g2_hmul2((x0 & 0x000f000fu) | (u0 & 0x00100010u), L0); A[w][0][1] = g2_hmul2((x1 & 0x000f000fu) | (u1 & 0x00100010u), L1);
-          A[w][0][2] = g2_hmul2((y0 & 0x000f000fu) | (t0 & 0x00100010u), L0); A[w][0][3] = g2_hmul2((y1 & 0x000f000fu) | (t1 & 0x00100010u), L1);
-          A[w][1][0] = g2_hmul2((x0 & 0x00f000f0u) | (v0 & 0x01000100u), H0); A[w][1][1] = g2_hmul2((x1 & 0x00f000f0u) | (v1 & 0x01000100u), H1);
-          A[w][1][2] = g2_hmul2((y0 & 0x00f000f0u) | (s0 & 0x01000100u), H0); A[w][1][3] = g2_hmul2((y1 & 0x00f000f0u) | (s1 & 0x01000100u), H1);
-        }
+        A[w][0][0] = g2_hmul2(x0 & 0x000f000fu, L0); A[w][0][1] = g2_hmul2(x1 & 0x000f000fu, L1);
+        A[w][0][2] = g2_hmul2(y0 & 0x000f000fu, L0); A[w][0][3] = g2_hmul2(y1 & 0x000f000fu, L1);
+        A[w][1][0] = g2_hmul2(x0 & 0x00f000f0u, H0); A[w][1][1] = g2_hmul2(x1 & 0x00f000f0u, H1);
+        A[w][1][2] = g2_hmul2(y0 & 0x00f000f0u, H0); A[w][1][3] = g2_hmul2(y1 & 0x00f000f0u, H1);
       }
 #pragma unroll
       for (int nt = 0; nt < NTC; nt++) {
@@ -355,7 +349,7 @@ __device__ __forceinline__ void g2_drain(const G2Ring &r) {
 // GemmArgs describes; the routed-expert launches (moe.cuh) find their matrices through the expert ids an earlier kernel chose.
 //   EARLY   the weight addresses depend on no earlier kernel: the ring's prologue is issued before the wait
 //   Cur     cursor of the row tile being copied;  locate  row tile -> cursor;  src  tile of super-block sb0 + c of the slice
-template <int FMT, int NTP> struct G2MatsPlain {
+template <int FMT, bool FOLD = false> struct G2MatsPlain {
   static constexpr bool EARLY = true, CONTIG = true;
   const GemmArgs &a;
   struct Cur { const uint8_t *W; };
@@ -369,7 +363,7 @@ template <int FMT, int NTP> struct G2MatsPlain {
   template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
     int m = 0;
     while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
-    gemm_epilogue<NT>(a, a.m[m], ks, (tile - a.tile0[m]) * 16 + g2_row<FMT, NTP>(lane >> 2), acc, lane);
+    gemm_epilogue<NT>(a, a.m[m], ks, (tile - a.tile0[m]) * 16 + g2_row<FMT, FOLD>(lane >> 2), acc, lane);
   }
 };
 
@@ -388,7 +382,7 @@ template <int FMT, int NTP> struct G2MatsPlain {
 // NTC < NT (the routed-expert launches at 16 rows): a weight tile is multiplied with NTC = 2 of the NT staged n-tiles only,
 // the hi and lo tiles of the eight rows its own row is among (Mats::col0(tile) = first plane column of the hi tile; the
 // lo tile is NC / 2 columns on), since the epilogue keeps one row of the tile.
-template <int FMT, int NT, class Stage, class Mats, int NTC = NT>
+template <int FMT, int NT, class Stage, class Mats, int NTC = NT, bool FOLD = false>
 __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, G2Ring &rg, uint8_t *planes, Stage stage, const Mats mats) {
   constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC), TB = tile_bytes(FMT), ST = g2_stages(FMT, NC), CH = g2_chunk(FMT);
   static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
@@ -439,7 +433,7 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
       if (!rg.dead && !mbar_wait(rg.bar_s + 8 * s, (rg.par >> s) & 1u, G2_WAIT_LIMIT)) { rg.dead = true; if (a.err) atomicExch(a.err, 1u); }
       rg.par ^= 1u << s;
 #pragma unroll 1
-      for (int u = 0; u < CH && c + u < c1; u++) g2_tile<FMT, NT, NTC>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
+      for (int u = 0; u < CH && c + u < c1; u++) g2_tile<FMT, NT, NTC, FOLD>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
       __syncwarp();                                        // every lane has read the stage
       issue(s);
       s = s + 1 == ST ? 0 : s + 1;
@@ -468,7 +462,7 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
 // The activation slice from the planes in global memory: the columns of the launch's rows only (a one-row pass uses two of
 // eight; an MMA's columns do not see one another, so what the others hold does not matter).  Sixteen-byte cp.async by all
 // warps; one bulk copy a column took 0.5 us longer a launch.
-template <int FMT, int NT> struct G2StagePlanes {
+template <int FMT, int NT, bool FOLD = false> struct G2StagePlanes {
   const GemmArgs &a;
   __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
     constexpr int NC = 8 * NT;
@@ -478,7 +472,7 @@ template <int FMT, int NT> struct G2StagePlanes {
 #pragma unroll 2
     for (int task = warp; task < ntask; task += nw) {   // (live column, super-block): 32 pieces, a lane each
       const int i = task / nsl, sb = task - i * nsl, c = i < a.T ? i : NC / 2 + i - a.T, p = sb * 32 + lane;
-      cp_async16(smem_u32(xh_s + c * CS) + g2_xpos<FMT, NT>(p), xh + (size_t)c * a.K * 2 + p * 16);
+      cp_async16(smem_u32(xh_s + c * CS) + g2_xpos<FMT, FOLD>(p), xh + (size_t)c * a.K * 2 + p * 16);
     }
     if constexpr (g2_aux(FMT) != 0)         // the means of the slice: contiguous in global memory
       for (int i = threadIdx.x; i < nsl * NC * 2; i += blockDim.x) cp_async16(smem_u32(xsf_s + i * 16), xf + i * 16);
@@ -488,11 +482,12 @@ template <int FMT, int NT> struct G2StagePlanes {
   }
 };
 
-template <int FMT, int NT>
+template <int FMT, int NT, bool FOLD>
 __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_gemm2(const GemmArgs a, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT), G2StagePlanes<FMT, NT>{a}, G2MatsPlain<FMT, NT>{a});
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT, FOLD>, G2MatsPlain<FMT, FOLD>, NT, FOLD>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                                   G2StagePlanes<FMT, NT, FOLD>{a}, G2MatsPlain<FMT, FOLD>{a});
   g2_drain(rg);
 }

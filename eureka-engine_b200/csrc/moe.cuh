@@ -45,7 +45,7 @@ template <int NTC> __device__ __forceinline__ void moe_col(const float (&acc)[NT
   v1 = acc[0][i + 2] + lo[i + 2] * XP_LO_INV;
 }
 
-template <int FMT, int NTP> struct MoeGuMats {
+template <int FMT> struct MoeGuMats {
   static constexpr bool EARLY = false, CONTIG = true;
   const MoeArgs &m;
   struct Cur { const uint8_t *W; };
@@ -63,13 +63,13 @@ template <int FMT, int NTP> struct MoeGuMats {
     bool mine;
     moe_col<NT>(acc, t, lane, v0, v1, mine);
     if (!mine) return;
-    const int r = (tile - slot * tps) * 16 + g2_row<FMT, NTP>(lane >> 2);          // rows r and r + 8 of [gate | up]; a tile is all gate or all up
+    const int r = (tile - slot * tps) * 16 + g2_row<FMT, false>(lane >> 2);          // rows r and r + 8 of [gate | up]; a tile is all gate or all up
     float *dst = (r < m.ef ? m.g : m.u) + (size_t)ks * m.gu_stride + (size_t)t * m.nslot * m.ef + (size_t)jx * m.ef + (r < m.ef ? r : r - m.ef);
     dst[0] = v0; dst[8] = v1;
   }
 };
 
-template <int FMT, int NTP> struct MoeDnMats {
+template <int FMT> struct MoeDnMats {
   static constexpr bool EARLY = false, CONTIG = false;
   const MoeArgs &m;
   struct Cur { const int *ids; int tile; };
@@ -91,7 +91,7 @@ template <int FMT, int NTP> struct MoeDnMats {
     bool mine;
     moe_col<NT>(acc, t, lane, v0, v1, mine);
     if (!mine) return;
-    float *dst = m.out + (size_t)ks * m.split_stride + (size_t)t * m.d + (tile - ri * tpt) * 16 + g2_row<FMT, NTP>(lane >> 2);
+    float *dst = m.out + (size_t)ks * m.split_stride + (size_t)t * m.d + (tile - ri * tpt) * 16 + g2_row<FMT, false>(lane >> 2);
     dst[0] = v0; dst[8] = v1;
   }
 };
@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_gu(const 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeGuMats<FMT, NT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                          G2StagePlanes<FMT, NT>{a}, MoeGuMats<FMT, NT>{m});
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeGuMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                          G2StagePlanes<FMT, NT>{a}, MoeGuMats<FMT>{m});
   g2_drain(rg);
 }
 // The down launch's activation slice built in shared memory from the gate|up outputs (T <= 4 rows): wt * silu(g) * u
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8) * 32, 1) k_moe_dn_silu(const 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8) / g2_warps(FMT, 8));
-  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStageSilu<FMT>{m, wt}, MoeDnMats<FMT, 1>{m});
+  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStageSilu<FMT>{m, wt}, MoeDnMats<FMT>{m});
   g2_drain(rg);
 }
 
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_dn(const 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeDnMats<FMT, NT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                          G2StagePlanes<FMT, NT>{a}, MoeDnMats<FMT, NT>{m});
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeDnMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                          G2StagePlanes<FMT, NT>{a}, MoeDnMats<FMT>{m});
   g2_drain(rg);
 }

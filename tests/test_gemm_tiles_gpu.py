@@ -25,7 +25,7 @@ def test_tiles_hold_every_weight(llb, packs, dev, ty, rows, cols):
 
 
 @pytest.mark.parametrize("ksplit", [0, 1, 3])
-@pytest.mark.parametrize("rows,K,T", [(1, 256, 1), (16, 1024, 1), (17, 3328, 3), (100, 2048, 8), (2500, 1280, 4), (40, 4096, 16)])
+@pytest.mark.parametrize("rows,K,T", [(1, 256, 1), (16, 1024, 1), (17, 3328, 3), (100, 2048, 8), (2500, 1280, 4), (40, 4096, 16), (19200, 2560, 9), (19216, 2560, 16)])
 @pytest.mark.parametrize("ty", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
 def test_row_tiles_shared_by_warps(llb, packs, dev, ty, rows, K, T, ksplit):
     rng = np.random.default_rng(rows + K)
