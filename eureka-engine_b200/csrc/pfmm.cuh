@@ -333,27 +333,35 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
     }
   } else if (warp >= 12) {
     // ---- results: lane quarter q of the accumulators, one weight row per thread ----
-    const int q = warp - 12;
+    // The tensor core waits for this (both accumulators fill tensor memory), so the loop holds nothing but loads, sums and
+    // stores: with the matrix's fields read and the row count tested at every store a tile took 20000 cycles here, a tenth to a
+    // fifth of its life; now 2000.
+    const int q = warp - 12, R = a.R;
     int i = 0;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x, i++) {
       int m, row0;
       pf_locate(a, u % ntiles, m, row0);
-      const PfMat &M = a.m[m];
       const int row = row0 + 32 * q + lane;
-      float *out = M.out + (size_t)(u / ntiles) * M.split_stride + row;
+      const bool on = row < a.m[m].rows;
+      const size_t os = a.m[m].ostride;
+      float *out = a.m[m].out + (size_t)(u / ntiles) * a.m[m].split_stride + row;
       wait(acc_full(0), (uint32_t)i & 1u);
       t5_fence_after();
       const uint32_t t0 = tmem_base + ((uint32_t)(32 * q) << 16);
-      for (int c = 0; c < a.R; c += 16) {     // chunk rows c .. c + 15: unit c / 128, its columns c % 128 ..
+#pragma unroll 1
+      for (int c = 0; c < R; c += 16) {       // chunk rows c .. c + 15 are columns c .. of both accumulators
         float v[16], v2[16];
-        const uint32_t col = (uint32_t)((c / PF_R) * 2 * PF_R + (c % PF_R));
-        t5_ld16(t0 + col, v);
-        t5_ld16(t0 + col + PF_R, v2);
+        t5_ld16(t0 + c, v);
+        t5_ld16(t0 + c + PF_R, v2);
         t5_wait_ld();
-        if (row < M.rows) {
 #pragma unroll
-          for (int j = 0; j < 16; j++)
-            if (c + j < a.R) out[(size_t)(c + j) * M.ostride] = v[j] + v2[j] * XP_LO_INV;
+        for (int j = 0; j < 16; j++) v[j] += v2[j] * XP_LO_INV;
+        if (on && c + 16 <= R) {
+#pragma unroll
+          for (int j = 0; j < 16; j++) { *out = v[j]; out += os; }
+        } else if (on) {
+#pragma unroll
+          for (int j = 0; j < 16; j++) { if (c + j < R) *out = v[j]; out += os; }
         }
       }
       t5_fence_before();
