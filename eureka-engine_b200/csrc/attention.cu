@@ -12,6 +12,9 @@
 //   output  O[d][q] += V_hi^T (P_hi + P_lo) + V_lo^T P_hi / 2048        warps split the head dimension
 // Per (query, slice) it leaves a running max, a sum and an unnormalised accumulator for k_attn_comb.
 // The scalar-FMA kernel this replaces spent 2400 warp instructions per 32 positions and warp; this one about 350.
+// A warp has 16 dims of the output: sixteen warps at head dimension 256, where shared memory leaves room for one block an SM
+// (with eight, a 256-row chunk's launch took 307 us at 1500 positions on the 27B shape, with sixteen 258).  A tile's phases
+// (scores, softmax, output) follow one another and their latencies are what bounds it: tensor pipe 30 %, shared memory 45 %.
 #include "host.cuh"
 #include "model.cuh"
 #include "rowops.cuh"
@@ -34,7 +37,7 @@ template <int HD> static size_t att_smem(int nqg) {
 }
 
 template <int HD, int NQG>
-__global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, const __half *__restrict__ Kc, const __half *__restrict__ Vc,
+__global__ void __launch_bounds__(2 * HD, HD > 128 ? 1 : 2) k_attn_mma(const float *__restrict__ q, const __half *__restrict__ Kc, const __half *__restrict__ Vc,
                                                   AttnShape sh, int Tmax, float *__restrict__ pm, float *__restrict__ pl,
                                                   float *__restrict__ po, const RowSet *rs) {
   // blockIdx.z: one of several row groups -- the groups of a prompt chunk, which share a cache, or the streams of a pass,
@@ -48,7 +51,8 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
   int rs_n, rs_p0;
   rs = rs_begin(rs, rs_n, rs_p0);
   extern __shared__ __align__(128) uint8_t sm[];
-  constexpr int RSK = HD + 8, NQP = 8 * NQG, MTW = HD / 128, KSTEPS = HD / 16;
+  constexpr int RSK = HD + 8, NQP = 8 * NQG, KSTEPS = HD / 16;
+  constexpr int NW = HD / 16, NTH = 32 * NW, QPW = (NQP + NW - 1) / NW;   // warps (16 dims of the output each), threads, queries a warp
   constexpr int TILE_B = ATT_PT * RSK * 2;   // bytes of one staged array (32 rows)
   __half *qh = (__half *)sm, *ql = qh + NQP * RSK;
   uint8_t *kv = (uint8_t *)(ql + NQP * RSK);                  // [stage][Kh, Kl, Vh, Vl][32][RSK]
@@ -68,7 +72,7 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
       const int p0 = s0 + it * ATT_PT;
       const uint32_t dst0 = kv_s + (uint32_t)(it & 1) * 4 * TILE_B;
       // 4 arrays x 32 rows x HD/8 sixteen-byte pieces
-      for (int i = tid; i < 4 * ATT_PT * (HD / 8); i += 256) {
+      for (int i = tid; i < 4 * ATT_PT * (HD / 8); i += NTH) {
         const int arr = i / (ATT_PT * (HD / 8)), rem = i - arr * (ATT_PT * (HD / 8)), row = rem / (HD / 8), pc = rem - row * (HD / 8);
         const int p = min(p0 + row, s1 - 1);   // rows past the slice repeat its last row; their scores are masked
         const __half *src = ((arr < 2) ? Kc : Vc) + (size_t)(arr & 1) * sh.kv_plane + (size_t)p * kvd + kvh * HD + pc * 8;
@@ -79,7 +83,7 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
   };
   load_tile(0);
   // the queries of this kv head as hi / lo planes: local query g * Tmax + r is head kvh * G + g, row r
-  for (int i = tid; i < NQP * (HD / 2); i += 256) {
+  for (int i = tid; i < NQP * (HD / 2); i += NTH) {
     const int qi = i / (HD / 2), dd = 2 * (i - qi * (HD / 2)), g = qi / Tmax, r = qi - g * Tmax;
     float2 v = make_float2(0.f, 0.f);
     if (qi < NQ && r < n) v = __ldcg((const float2 *)(q + ((size_t)r * sh.H + kvh * G + g) * HD + dd));
@@ -88,16 +92,14 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
     *(__half2 *)(qh + qi * RSK + dd) = h;
     *(__half2 *)(ql + qi * RSK + dd) = __floats2half2_rn((v.x - hf.x) * XP_LO_SCALE, (v.y - hf.y) * XP_LO_SCALE);
   }
-  float m_r[NQG], l_r[NQG];      // running max and sum of query warp + 8 i (the same in every lane)
-  float acc[MTW][NQG][4], acl[MTW][NQG][4];
+  float m_r[QPW], l_r[QPW];      // running max and sum of query warp + NW i (the same in every lane)
+  float acc[NQG][4], acl[NQG][4];
 #pragma unroll
-  for (int i = 0; i < NQG; i++) { m_r[i] = -INFINITY; l_r[i] = 0.0f; }
+  for (int i = 0; i < QPW; i++) { m_r[i] = -INFINITY; l_r[i] = 0.0f; }
 #pragma unroll
-  for (int a = 0; a < MTW; a++)
+  for (int b = 0; b < NQG; b++)
 #pragma unroll
-    for (int b = 0; b < NQG; b++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) { acc[a][b][c] = 0.0f; acl[a][b][c] = 0.0f; }
+    for (int c = 0; c < 4; c++) { acc[b][c] = 0.0f; acl[b][c] = 0.0f; }
   const float scale = 1.0f / sqrtf((float)HD);
   const uint32_t qh_s = smem_u32(qh), ql_s = smem_u32(ql), ph_s = smem_u32(Ph), pl_s = smem_u32(Pl);
 
@@ -108,21 +110,20 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
     const int p0 = s0 + it * ATT_PT;
     const uint32_t st_s = kv_s + (uint32_t)(it & 1) * 4 * TILE_B;
     // ---- scores: work item = (16 positions, 8 queries) ----
-    for (int item = warp; item < 2 * NQG; item += 8) {
+    for (int item = warp; item < 2 * NQG; item += NW) {
       const int mt = item & 1, qg = item >> 1;
       float hh[4] = {0.f, 0.f, 0.f, 0.f}, hl[4] = {0.f, 0.f, 0.f, 0.f}, lh[4] = {0.f, 0.f, 0.f, 0.f};
       const uint32_t a_off = (uint32_t)((16 * mt + lr + ((mi & 1) ? 8 : 0)) * RSK + ((mi & 2) ? 8 : 0)) * 2;
-      const uint32_t b_off = (uint32_t)((8 * qg + lr) * RSK + ((mi & 1) ? 8 : 0)) * 2;
+      const uint32_t b_s = ((mi & 2) ? ql_s : qh_s) + (uint32_t)((8 * qg + lr) * RSK + ((mi & 1) ? 8 : 0)) * 2;   // both planes in one load
 #pragma unroll 4
       for (int ks = 0; ks < KSTEPS; ks++) {
-        uint32_t ah[4], al[4], bh[2], bl[2];
+        uint32_t ah[4], al[4], b[4];
         ldsm_x4(ah, st_s + a_off + ks * 32);
         ldsm_x4(al, st_s + TILE_B + a_off + ks * 32);
-        ldsm_x2(bh, qh_s + b_off + ks * 32);
-        ldsm_x2(bl, ql_s + b_off + ks * 32);
-        mma16816(hh, ah[0], ah[1], ah[2], ah[3], bh[0], bh[1]);
-        mma16816(hl, ah[0], ah[1], ah[2], ah[3], bl[0], bl[1]);
-        mma16816(lh, al[0], al[1], al[2], al[3], bh[0], bh[1]);
+        ldsm_x4(b, b_s + ks * 32);
+        mma16816(hh, ah[0], ah[1], ah[2], ah[3], b[0], b[1]);
+        mma16816(hl, ah[0], ah[1], ah[2], ah[3], b[2], b[3]);
+        mma16816(lh, al[0], al[1], al[2], al[3], b[0], b[1]);
       }
 #pragma unroll
       for (int c = 0; c < 4; c++) {
@@ -132,10 +133,11 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
       }
     }
     __syncthreads();
-    // ---- online softmax: warp w owns queries w, w + 8, ..; lane = position ----
+    // ---- online softmax: warp w owns queries w, w + NW, ..; lane = position ----
 #pragma unroll
-    for (int i = 0; i < NQG; i++) {
-      const int qi = warp + 8 * i;
+    for (int i = 0; i < QPW; i++) {
+      const int qi = warp + NW * i;
+      if (NQP % NW && qi >= NQP) break;
       const float s = Ssm[qi * 33 + lane];
       const float mt = aw_max(s);
       float e = 0.0f, cf = 1.0f;
@@ -152,38 +154,26 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
       if (lane == 0) corr[qi] = cf;
     }
     __syncthreads();
-    // ---- output: warp w owns dims 16 MTW w .. + 16 MTW - 1 of every query ----
+    // ---- output: warp w owns dims 16 w .. + 15 of every query ----
 #pragma unroll
     for (int nt = 0; nt < NQG; nt++) {
       const float c0 = corr[8 * nt + 2 * j], c1 = corr[8 * nt + 2 * j + 1];
-#pragma unroll
-      for (int a = 0; a < MTW; a++) {
-        acc[a][nt][0] *= c0; acc[a][nt][1] *= c1; acc[a][nt][2] *= c0; acc[a][nt][3] *= c1;
-        acl[a][nt][0] *= c0; acl[a][nt][1] *= c1; acl[a][nt][2] *= c0; acl[a][nt][3] *= c1;
-      }
+      acc[nt][0] *= c0; acc[nt][1] *= c1; acc[nt][2] *= c0; acc[nt][3] *= c1;
+      acl[nt][0] *= c0; acl[nt][1] *= c1; acl[nt][2] *= c0; acl[nt][3] *= c1;
     }
 #pragma unroll
     for (int ks = 0; ks < ATT_PT / 16; ks++) {
-      uint32_t bph[NQG][2], bpl[NQG][2];
+      const uint32_t v_off = (uint32_t)((16 * ks + lr + ((mi & 2) ? 8 : 0)) * RSK + 16 * warp + ((mi & 1) ? 8 : 0)) * 2;
+      uint32_t vh[4], vl[4];
+      ldsm_x4_t(vh, st_s + 2 * TILE_B + v_off);
+      ldsm_x4_t(vl, st_s + 3 * TILE_B + v_off);
 #pragma unroll
       for (int nt = 0; nt < NQG; nt++) {
-        const uint32_t off = (uint32_t)((8 * nt + lr) * ATT_PS + 16 * ks + ((mi & 1) ? 8 : 0)) * 2;
-        ldsm_x2(bph[nt], ph_s + off);
-        ldsm_x2(bpl[nt], pl_s + off);
-      }
-#pragma unroll
-      for (int a = 0; a < MTW; a++) {
-        const int d0 = 16 * (MTW * warp + a);
-        const uint32_t v_off = (uint32_t)((16 * ks + lr + ((mi & 2) ? 8 : 0)) * RSK + d0 + ((mi & 1) ? 8 : 0)) * 2;
-        uint32_t vh[4], vl[4];
-        ldsm_x4_t(vh, st_s + 2 * TILE_B + v_off);
-        ldsm_x4_t(vl, st_s + 3 * TILE_B + v_off);
-#pragma unroll
-        for (int nt = 0; nt < NQG; nt++) {
-          mma16816(acc[a][nt], vh[0], vh[1], vh[2], vh[3], bph[nt][0], bph[nt][1]);
-          mma16816(acc[a][nt], vh[0], vh[1], vh[2], vh[3], bpl[nt][0], bpl[nt][1]);
-          mma16816(acl[a][nt], vl[0], vl[1], vl[2], vl[3], bph[nt][0], bph[nt][1]);
-        }
+        uint32_t b[4];
+        ldsm_x4(b, ((mi & 2) ? pl_s : ph_s) + (uint32_t)((8 * nt + lr) * ATT_PS + 16 * ks + ((mi & 1) ? 8 : 0)) * 2);
+        mma16816(acc[nt], vh[0], vh[1], vh[2], vh[3], b[0], b[1]);
+        mma16816(acc[nt], vh[0], vh[1], vh[2], vh[3], b[2], b[3]);
+        mma16816(acl[nt], vl[0], vl[1], vl[2], vl[3], b[0], b[1]);
       }
     }
     __syncthreads();   // the stage and the probability tiles are free again
@@ -191,9 +181,9 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
   cp_async_wait<0>();
   // ---- per (query, slice): running max, sum, unnormalised output ----
 #pragma unroll
-  for (int i = 0; i < NQG; i++) {
-    const int qi = warp + 8 * i, g = qi / Tmax, r = qi - g * Tmax;
-    if (lane == 0) {
+  for (int i = 0; i < QPW; i++) {
+    const int qi = warp + NW * i, g = qi / Tmax, r = qi - g * Tmax;
+    if (lane == 0 && (NQP % NW == 0 || qi < NQP)) {
       mfin[qi] = m_r[i];
       if (qi < NQ && r < n) {
         const size_t o = ((size_t)(kvh * G + g) * Tmax + r) * nsplit + split;
@@ -209,11 +199,7 @@ __global__ void __launch_bounds__(256) k_attn_mma(const float *__restrict__ q, c
       const int qi = 8 * nt + 2 * j + (c & 1), g = qi / Tmax, r = qi - g * Tmax;
       if (qi >= NQ || r >= n || mfin[qi] == -INFINITY) continue;   // an empty slice: the merge skips it on m alone
       const size_t o = ((size_t)(kvh * G + g) * Tmax + r) * nsplit + split;
-#pragma unroll
-      for (int a = 0; a < MTW; a++) {
-        const int d = 16 * (MTW * warp + a) + gid + ((c & 2) ? 8 : 0);
-        po[o * HD + d] = acc[a][nt][c] + acl[a][nt][c] * XP_LO_INV;
-      }
+      po[o * HD + 16 * warp + gid + ((c & 2) ? 8 : 0)] = acc[nt][c] + acl[nt][c] * XP_LO_INV;
     }
 }
 
@@ -295,7 +281,7 @@ __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm,
 
 template <int HD, int NQG> static int att_go(cudaStream_t s, dim3 grid, const float *q, const __half *Kc, const __half *Vc, AttnShape sh, int Tmax,
                                              float *pm, float *pl, float *po, const RowSet *rs) {
-  CU_OK(llb_launch(k_attn_mma<HD, NQG>, grid, dim3(256), att_smem<HD>(NQG), s, q, Kc, Vc, sh, Tmax, pm, pl, po, rs));
+  CU_OK(llb_launch(k_attn_mma<HD, NQG>, grid, dim3(2 * HD), att_smem<HD>(NQG), s, q, Kc, Vc, sh, Tmax, pm, pl, po, rs));
   return 0;
 }
 template <int HD> static int att_hd(cudaStream_t s, int nqg, dim3 grid, const float *q, const __half *Kc, const __half *Vc, AttnShape sh, int Tmax,
@@ -309,6 +295,20 @@ template <int HD> static int att_hd(cudaStream_t s, int nqg, dim3 grid, const fl
     case 6: return att_go<HD, 6>(s, grid, q, Kc, Vc, sh, Tmax, pm, pl, po, rs);
   }
   return llb_fail("attention: %d queries per kv head", nqg * 8);
+}
+
+// K-slices of a prompt chunk's nz row groups: the fewest rounds of blocks, each as long as its slice's tiles plus about two for
+// the queries going in and the partial results coming out.  (With a decode pass's split, one wave for ONE group, a block had
+// two tiles to do and left 48 KB to merge: 92 ms of a 3011-token prompt on the 27B shape, 58 with one to eight slices.)
+int att_prompt_split(int KV, int hd, int nz, int total, int sms, int cap) {
+  const int slots = sms * (hd > 128 ? 1 : 2), tiles = (total + ATT_PT - 1) / ATT_PT;   // blocks on the chip at a time
+  int best = 1;
+  double best_cost = 1e30;
+  for (int ns = 1; ns <= cap && ns <= tiles; ns++) {
+    const double cost = (double)((KV * nz * ns + slots - 1) / slots) * ((tiles + ns - 1) / ns + 2.0);
+    if (cost < best_cost) { best_cost = cost; best = ns; }
+  }
+  return best;
 }
 
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,

@@ -1118,7 +1118,7 @@ static int pf_chunk(llb_spec *m, int b, const int *ids, int p0, int R) {
   PfState &f = m->pf;
   cudaStream_t s = g_llb.stream;
   StreamScope scope(m, true);   // the chunk's kernels see one stream: stream b's state is handed to them directly
-  const int d = m->d, qa = m->H * m->hd, gsz = m->Tpf, ngrp = (R + gsz - 1) / gsz;
+  const int d = m->d, qa = m->H * m->hd, gsz = m->Tpf, ngrp = (R + gsz - 1) / gsz, nsp = att_prompt_split(m->KV, m->hd, ngrp, p0 + R, g_llb.sms, m->att_split);
   std::vector<RowSet> rs(1 + ngrp);
   memset(rs.data(), 0, rs.size() * sizeof(RowSet));
   rs[0].n = R; rs[0].pos0 = p0;
@@ -1137,7 +1137,7 @@ static int pf_chunk(llb_spec *m, int b, const int *ids, int p0, int R) {
       PFK("gemm qkv", pf_site(m, {{&l.at.q, &f.q}, {&l.at.k, &f.k}, {&l.at.v, &f.v}}, f.kg_d, d, R));
       PFK("qkrope", op_qkrope(s, as_in(f.q), as_in(f.k), as_in(f.v), l.at.qn, l.at.kn, m->invfreq, ash, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), &f.rs[0], R));
       // every group of gsz rows in one launch (grid z): each streams the K/V rows up to its own last position
-      PFK("attention", op_attention(s, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), as_in(f.q), ash, m->att_split, f.pm, f.pl, f.po, m->xp_qa, &f.rs[1], gsz, f.kg_qa, 0, ngrp));
+      PFK("attention", op_attention(s, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), as_in(f.q), ash, nsp, f.pm, f.pl, f.po, m->xp_qa, &f.rs[1], gsz, f.kg_qa, 0, ngrp));
       PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
     } else {
       PFK("gemm qkv|z|b|a", pf_site(m, {{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));
