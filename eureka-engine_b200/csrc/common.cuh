@@ -107,13 +107,13 @@ __device__ __forceinline__ void xp_store4(const XPlanes &xp, int t, int planes, 
 }
 
 // ---- activations of a prompt chunk ----------------------------------------------------------------
-#define PF_R 256              // rows of a prompt chunk (= N of the dense GEMM's MMA, pfmm.cuh)
-#define PF_RMAX 256           // ... of PF_RMAX / PF_R units multiplied against the same dequantised weight stage (one)
+#define PF_R 128              // rows of a unit of a prompt chunk: the half of the dense GEMM's N = 256 that one CTA of a pair holds (pfmm.cuh)
+#define PF_RMAX 256           // rows of a chunk, PF_RMAX / PF_R units
 // Activations of a chunk for the dense GEMM, "k-group major", as two fp16 planes like the T-row planes: hi = fp16(x),
 // lo = fp16((x - hi) * 2048), about 22 bits of x.  Element (row r, column k) of a [PF_R][K] matrix sits at half index
 // ((k >> 3) * PF_R + r) * 8 + (k & 7) of its plane; the lo plane follows the hi plane (K * PF_R halves further on).  Eight
 // consecutive columns of one row are one 16-byte core-matrix row, the PF_R rows of a k-group are contiguous (2 KB), and
-// a 64-column stage of one plane is one contiguous run (32 KB).  A chunk of more than PF_R rows is two such matrices one after the other.
+// a 64-column stage of one plane is one contiguous run (16 KB).  A chunk of more than PF_R rows is two such matrices one after the other.
 __host__ __device__ inline size_t pf_kg_halves(int K) { return (size_t)2 * K * PF_R; }
 // four consecutive columns k .. k+3 (k a multiple of 4) of row r into both planes
 __device__ __forceinline__ void pf_kg_store4(__half *x, int K, int r, int k, float v0, float v1, float v2, float v3) {

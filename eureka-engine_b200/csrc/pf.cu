@@ -40,13 +40,13 @@ int pf_wait_errors_clear(void) {
   return 0;
 }
 
-// K-slices of a dense launch: whole waves of (tile, slice) units over the SMs, each unit costing its slice's
+// K-slices of a dense launch: whole waves of (pair of tiles, slice) units over the pairs of SMs, each unit costing its slice's
 // super-blocks plus about two super-blocks' worth of pipeline fill and epilogue; slices are whole super-blocks.
 int pf_pick_ksplit(int ntiles, int nsb, int sms) {
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= 8 && ks <= nsb; ks++) {
-    const long long units = (long long)ntiles * ks, waves = (units + sms - 1) / sms;
+    const long long units = (long long)((ntiles + 1) / 2) * ks, waves = (units + sms / 2 - 1) / (sms / 2);
     const double cost = (double)waves * ((nsb + ks - 1) / ks + 2.0) * (1.0 + 0.03 * (ks - 1));   // the longest slice sets the pace
     if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
   }
@@ -61,9 +61,9 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a) {
   a.t128[0] = 0;
   for (int i = 0; i < PF_MAXMAT; i++) a.t128[i + 1] = a.t128[i] + (i < a.nmat ? (a.m[i].rows + 127) / 128 : 0);
   a.err = g_pf_err;
-  const int units = a.t128[a.nmat] * a.ksplit;
+  const int units = (a.t128[a.nmat] + 1) / 2 * a.ksplit;   // pairs of tiles
   if (units < 1) return 0;
-  const int grid = units < g_llb.sms ? units : g_llb.sms;
+  const int grid = 2 * (units < g_llb.sms / 2 ? units : g_llb.sms / 2);
   cudaError_t e;
   switch (fmt) {
     case LLB_FM_Q4_K: e = llb_launch(k_pfmm<LLB_FM_Q4_K>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); break;

@@ -1,30 +1,29 @@
 // pfmm.cuh -- the prompt path's dense GEMM on the fifth-generation tensor cores: Y[r][n] = sum_k W[n][k] X[r][k] for a
-// chunk of up to PF_R = 256 prompt rows against Q4_K / Q5_K / Q6_K / Q8_0 weights.  It replaces, for this library, the
+// chunk of up to 256 prompt rows against Q4_K / Q5_K / Q6_K / Q8_0 weights.  It replaces, for this library, the
 // reference's chunked tensor-core prefill GEMM (tools/pf27/pfmm.cuh:311-384: int8 mma.sync + cp.async on sm_86; its
 // caller host/llb_pf.h:551 pf_take) with a design for sm_100a:
 //
-//   * the multiply is tcgen05.mma (kind::f16, M = 128 weight rows, N = 256 prompt rows, K = 16 per instruction), both
-//     operands in shared memory, fp32 accumulators in TENSOR MEMORY;
+//   * the multiply is tcgen05.mma over a PAIR of CTAs (kind::f16, cta_group::2: M = 256 weight rows, 128 a CTA, N = 256 prompt
+//     rows, K = 16 per instruction), both operands in shared memory, fp32 accumulators in TENSOR MEMORY;
 //   * BOTH operands are two fp16 planes, hi = fp16(v) and lo = fp16((v - hi) * 2048) (about 22 bits of v, as the T-row
 //     path's activation planes): a 16-column step is three MMAs, hi.hi into one accumulator of 256 columns and the
 //     two cross terms hi.lo and lo.hi into another (together all 512 columns of tensor memory); the epilogue adds the
 //     cross terms divided by 2048 (lo.lo is below fp32 resolution).  With one fp16 plane per operand every GEMM output carried a relative error of 4e-4, which a
 //     random 8-layer model amplified past the path's 2e-2 bar;
-//   * N = 256 because the kernel is bound by turning codes into fp16 planes (14.5 thread instructions per weight; with
-//     N = 128 the tensor pipe was 40 % busy): a dequantised weight stage now serves twice the rows.  Measured on the
-//     27B shape's gate|up launch: N = 128, three stages, three accumulators 174 us per 128 rows; two units of N = 128
-//     per stage (four accumulators) 262 us per 256 rows; N = 256 238 us per 256 rows;
+//   * a pair because each CTA then stages half of the chunk's rows only: a step of 16 columns moves 40 KB through its shared
+//     memory (60 KB alone), and a third stage fits.  N = 256 because a dequantised weight (14.5 thread instructions)
+//     then serves all rows of a chunk.  What bounds it is the tensor pipe, 384 cycles a step of 433.  gate|up of the 27B shape,
+//     256 rows: 270 us with two units of N = 128 a stage, 232 us with one CTA and N = 256, 194 us now (single CTAs took
+//     528 cycles a step: the issuing threads' three barriers a stage and MMAs out of vector registers were their chain);
 //   * the activation planes arrive by TMA: the chunk's activations are kept in global memory in the order the operand
-//     wants (k-group major, common.cuh), so a 64-column stage of one plane is ONE contiguous 16 KB cp.async.bulk that
-//     completes on an mbarrier (plain bulk copies of this GPU's own memory, no multicast);
+//     wants (two units of 128 rows, k-group major, common.cuh), so a CTA's 64-column stage of one plane is ONE contiguous
+//     16 KB cp.async.bulk that completes on an mbarrier (plain bulk copies of this GPU's own memory, no multicast);
 //   * the weight planes are made on the fly: eight warps read the packed super-blocks (each thread one row's 32 weights
 //     of a stage), dequantise in fp32 (the formulas of tools/qwen35_engine.c:233-307, one FMA per weight), split
 //     each weight into its two planes and store 16-byte core-matrix rows; stores of a warp are conflict-free;
-//   * a two-stage ring of (32 KB weights, 64 KB activations) with full / empty mbarriers decouples the roles, so
-//     loads and dequantisation run ahead of the MMAs; four more warps read a finished tile out with tcgen05.ld.
-//     (Separate rings -- three weight stages and four half-stages of 32 activation columns, which fit the same shared
-//     memory -- were measured and dropped: the issuing threads then wait and commit twice as often, and a gate|up launch
-//     took 319 us against 262 us);
+//   * a three-stage ring of (32 KB weights, 32 KB activations) with full / empty mbarriers decouples the roles, so
+//     loads and dequantisation run ahead of the MMAs; four more warps read a finished tile out with tcgen05.ld.  One full
+//     barrier a stage, the leader's: the other CTA's warps arrive on it through the cluster;
 //   * every wait is bounded: a wait that runs out sets *err, and all roles then run through without waiting, so the
 //     kernel returns, frees its tensor memory and leaves the context usable (llb_b200_wait_errors() reports it).
 #pragma once
@@ -33,20 +32,19 @@
 #include "pf.cuh"
 
 #define PF_KS 64              // columns per ring stage
-#define PF_STAGES 2
-#define PF_A_BYTES (128 * PF_KS * 2)     // one plane of 128 weight rows
-#define PF_B_BYTES (PF_R * PF_KS * 2)    // one plane of one unit of the chunk's rows
-#define PF_NUN (PF_RMAX / PF_R)   // units of a chunk
-#define PF_STAGE_BYTES (2 * PF_A_BYTES + 2 * PF_NUN * PF_B_BYTES)   // [A hi | A lo | per unit: B hi | B lo]
+#define PF_STAGES 3
+#define PF_A_BYTES (128 * PF_KS * 2)     // one plane of a CTA's 128 weight rows
+#define PF_B_BYTES (PF_R * PF_KS * 2)    // one plane of a CTA's half of the chunk's rows
+#define PF_STAGE_BYTES (2 * PF_A_BYTES + 2 * PF_B_BYTES)   // [A hi | A lo | B hi | B lo]
 #define PF_SMEM (1024 + PF_STAGES * PF_STAGE_BYTES)
-#define PF_THREADS 512        // warps 0-7 dequantise, 8 loads activations, 9-11 issue MMAs, 12-15 write results
-#define PF_IDESC (0x08000010u | ((uint32_t)(PF_R >> 3) << 17))  // kind::f16: D f32, A / B f16 K-major, N = PF_R, M = 128
+#define PF_THREADS 512        // warps 0-7 dequantise, 8 loads activations, 9-10 issue MMAs, 11 forwards, 12-15 write results
+#define PF_IDESC (0x10000010u | ((uint32_t)(PF_RMAX >> 3) << 17))  // kind::f16: D f32, A / B f16 K-major, N = 256, M = 256 over the pair
 
 
 __device__ __forceinline__ void pf_mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void pf_bulk_copy(uint32_t dst_s, const void *src, uint32_t bytes, uint32_t bar_s) {
@@ -155,57 +153,64 @@ __device__ __forceinline__ void pf_split8(const float *w, uint4 &hi, uint4 &lo) 
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------------
-// Work unit = (128-row tile, K-slice); CTA b takes units b, b + grid, ...  Every role walks the same unit sequence.
+// Work unit = (pair of 128-row tiles, K-slice); CTA pair b takes units b, b + pairs, ..., its CTA r tile 2 i + r of pair i.  Every
+// role walks the same unit sequence.  The last pair's second tile may not exist: its CTA repeats the last one and stores nothing.
 __device__ __forceinline__ void pf_locate(const PfArgs &a, int tile, int &m, int &row0) {
   m = 0;
   while (m + 1 < a.nmat && tile >= a.t128[m + 1]) m++;
   row0 = (tile - a.t128[m]) * 128;
 }
 // K-slices are whole super-blocks, as equal as they come: first column and 64-column stages of unit u
-__device__ __forceinline__ void pf_slice(const PfArgs &a, int u, int ntiles, int &kbase, int &nst) {
-  const int ks = u / ntiles, nsb = a.K >> 8;
+__device__ __forceinline__ void pf_slice(const PfArgs &a, int u, int npairs, int &kbase, int &nst) {
+  const int ks = u / npairs, nsb = a.K >> 8;
   const int sb0 = (int)(((long long)ks * nsb) / a.ksplit), sb1 = (int)(((long long)(ks + 1) * nsb) / a.ksplit);
   kbase = sb0 << 8; nst = (sb1 - sb0) << 2;
 }
 
 template <int FMT>
-__global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // header: full_a[4] +0, full_b[4] +32, empty[4] +64, acc_full +128, acc_empty +136, tensor-memory address +144, dead +148
+  // header: full[4] +0, full_b[4] +32, empty[4] +64, acc_full +128, acc_empty +136, tensor-memory address +144, dead +148.
+  // The pair's first CTA (the leader) issues the MMAs: its full counts the dequantising warps of both CTAs, its own activations and
+  // the other CTA's (which land on that CTA's full_b and are passed on), its acc_empty the result warps of both; the MMAs'
+  // commits arrive in both CTAs.
   const uint32_t bar_s = smem_u32(smem);
-  auto full_a = [&](int s) { return bar_s + 8u * (uint32_t)s; };
+  auto full = [&](int s) { return bar_s + 8u * (uint32_t)s; };
   auto full_b = [&](int s) { return bar_s + 32u + 8u * (uint32_t)s; };
   auto empty = [&](int s) { return bar_s + 64u + 8u * (uint32_t)s; };
-  auto acc_full = [&](int b) { return bar_s + 128u + 8u * (uint32_t)b; };
-  auto acc_empty = [&](int b) { return bar_s + 136u + 8u * (uint32_t)b; };
+  const uint32_t acc_full = bar_s + 128u, acc_empty = bar_s + 136u;
   uint32_t *tmem_slot = (uint32_t *)(smem + 144);
   volatile uint32_t *dead = (volatile uint32_t *)(smem + 148);
   uint8_t *ring = smem + 1024;
   const uint32_t ring_s = smem_u32(ring);
-  const int ntiles = a.t128[a.nmat], nunits = ntiles * a.ksplit;
-  const int nun = a.R > PF_R ? 2 : 1;   // units of PF_R rows in this chunk
+  const int ntiles = a.t128[a.nmat], npairs = (ntiles + 1) >> 1, nunits = npairs * a.ksplit;
+  const int rank = blockIdx.x & 1, unit0 = blockIdx.x >> 1, ustep = gridDim.x >> 1;
+  auto tile_of = [&](int u) { return 2 * (u % npairs) + rank; };
 
   pdl_trigger();
   if (tid == 0) {
-    for (int s = 0; s < PF_STAGES; s++) { mbar_init(full_a(s), 8); mbar_init(full_b(s), 1); mbar_init(empty(s), 3); }
-    mbar_init(acc_full(0), 3); mbar_init(acc_empty(0), 4);
+    for (int s = 0; s < PF_STAGES; s++) { mbar_init(full(s), 18); mbar_init(full_b(s), 1); mbar_init(empty(s), 2); }
+    mbar_init(acc_full, 2); mbar_init(acc_empty, 8);
     *dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 10) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   pdl_wait();              // the activations come from the kernel in front
   t5_fence_before();
-  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // both CTAs' barriers exist
   t5_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // a bounded wait that gives up for the whole CTA
+  // (a phase that is complete costs one try: the issuing warps' waits are part of the chain that paces the MMAs)
   auto wait = [&](uint32_t bar, uint32_t parity) {
-    if (*dead) return;
-    if (!mbar_wait(bar, parity)) { *dead = 1; if (a.err) atomicExch(a.err, 1u); }
+    for (uint32_t n = 0; !mbar_wait(bar, parity, 4); n += 4) {
+      if (*dead) return;
+      if (n >= T5_WAIT_LIMIT) { *dead = 1; if (a.err) atomicExch(a.err, 1u); return; }
+    }
   };
 
   if (warp < 8) {
@@ -214,13 +219,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
     PfRaw raw0, raw1;                                  // two stages of raw words in flight (never indexed: they stay in registers)
     int it = 0;                                        // stages produced so far by this CTA
     // the loads run two stages ahead of the conversion: cursor (lu, ls) is the stage to load next
-    int lu = blockIdx.x, ls = 0, lkbase = 0, lnst = 0, lm = 0, lrow0 = 0;
+    int lu = unit0, ls = 0, lkbase = 0, lnst = 0, lm = 0, lrow0 = 0;
     const uint8_t *lrow = nullptr;
     int ldoff = 0;
     auto lplan = [&]() {
       if (lu < nunits) {
-        pf_locate(a, lu % ntiles, lm, lrow0);
-        pf_slice(a, lu, ntiles, lkbase, lnst);
+        pf_locate(a, min(tile_of(lu), ntiles - 1), lm, lrow0);
+        pf_slice(a, lu, npairs, lkbase, lnst);
         const int row = min(lrow0 + r, a.m[lm].rows - 1);
         lrow = a.m[lm].W + (size_t)(row >> 4) * (a.K >> 8) * tile_bytes(FMT) + (row & 15) * tile_row(FMT);
         ldoff = 3328 + 2 * (row & 15) - (row & 15) * 208;
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
     auto lnext = [&](PfRaw &dst) {
       if (lu < nunits) {
         pf_load<FMT>(lrow, ldoff, lkbase + ls * PF_KS + 32 * h, dst);
-        if (++ls == lnst) { ls = 0; lu += gridDim.x; lplan(); }
+        if (++ls == lnst) { ls = 0; lu += ustep; lplan(); }
       }
     };
     // converts the stage held in rw (columns c0 ..), refills rw with the stage two ahead, publishes the stage
@@ -249,87 +254,98 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads these bytes through the async proxy
       __syncwarp();
-      if (lane == 0) mbar_arrive(full_a(slot));
+      if (lane == 0) mbar_arrive_cluster(t5_map_rank(full(slot), 0));
       it++;
     };
     lplan();
     lnext(raw0);
     lnext(raw1);
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+    for (int u = unit0; u < nunits; u += ustep) {
       int kbase, nst;
-      pf_slice(a, u, ntiles, kbase, nst);
+      pf_slice(a, u, npairs, kbase, nst);
       for (int s = 0; s < nst; s += 2) {               // nst is a multiple of four: a K-slice is whole super-blocks
         one(raw0, kbase + 32 * h + s * PF_KS);
         one(raw1, kbase + 32 * h + (s + 1) * PF_KS);
       }
     }
   } else if (warp == 8) {
-    // ---- activations: one 16 KB bulk copy per unit, plane and stage ----
+    // ---- activations of this CTA's half of the chunk's rows: one 16 KB bulk copy per plane and stage ----
     if (lane == 0) {
       int it = 0;
-      for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+      const __half *x = a.x + (size_t)rank * pf_kg_halves(a.K);   // a unit's planes follow the previous unit's (common.cuh)
+      for (int u = unit0; u < nunits; u += ustep) {
         int kbase, nst;
-        pf_slice(a, u, ntiles, kbase, nst);
+        pf_slice(a, u, npairs, kbase, nst);
         for (int s = 0; s < nst; s++, it++) {
           const int slot = it % PF_STAGES;
           if (it >= PF_STAGES) wait(empty(slot), (uint32_t)((it / PF_STAGES) + 1) & 1u);
           if (*dead) continue;
-          const __half *src = a.x + (size_t)((kbase + s * PF_KS) >> 3) * PF_R * 8;
-          const uint32_t dst = ring_s + slot * PF_STAGE_BYTES + 2 * PF_A_BYTES;
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_b(slot)), "r"((uint32_t)(nun * 2 * PF_B_BYTES)) : "memory");
-          for (int un = 0; un < nun; un++) {   // a unit's planes follow the previous unit's in global memory (common.cuh)
-            const __half *su = src + (size_t)un * pf_kg_halves(a.K);
-            pf_bulk_copy(dst + un * 2 * PF_B_BYTES, su, PF_B_BYTES, full_b(slot));
-            pf_bulk_copy(dst + un * 2 * PF_B_BYTES + PF_B_BYTES, su + (size_t)a.K * PF_R, PF_B_BYTES, full_b(slot));
-          }
+          const __half *src = x + (size_t)((kbase + s * PF_KS) >> 3) * PF_R * 8;
+          const uint32_t dst = ring_s + slot * PF_STAGE_BYTES + 2 * PF_A_BYTES, bar = rank ? full_b(slot) : full(slot);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)(2 * PF_B_BYTES)) : "memory");
+          pf_bulk_copy(dst, src, PF_B_BYTES, bar);
+          pf_bulk_copy(dst + PF_B_BYTES, src + (size_t)a.K * PF_R, PF_B_BYTES, bar);
         }
       }
     }
-  } else if (warp >= 9 && warp < 12) {
-    // ---- the tensor core.  Issuing one tcgen05.mma costs a thread 100 to 200 cycles, more than a 128 x 128 x 16 MMA
-    // takes to execute, so the products of a step are spread over three threads; MMAs into one accumulator come from
-    // one thread (a thread's MMAs execute in its issue order, MMAs of different threads would not be ordered):
-    //   warp 9: hi.hi -> D1     warp 10: hi.lo and lo.hi -> D23     result = D1 + D23 / 2048
-    //   (tensor-memory columns: D1 at 0, D23 at PF_R.  The code is written for PF_RMAX / PF_R units of PF_R rows, unit un
-    //   with its pair of accumulators at 2 un PF_R and warp 10 + un issuing its cross terms; PF_R = 256 leaves one unit)
-    if (lane == 0) {
-      const int which = warp - 9;
-      int it = 0, i = 0;
-      for (int u = blockIdx.x; u < nunits; u += gridDim.x, i++) {
+  } else if (warp == 11) {
+    // ---- tells the leader that the other CTA's activations are there ----
+    if (lane == 0 && rank == 1) {
+      int it = 0;
+      for (int u = unit0; u < nunits; u += ustep) {
         int kbase, nst;
-        pf_slice(a, u, ntiles, kbase, nst);
-        if (i >= 1) wait(acc_empty(0), (uint32_t)(i - 1) & 1u);   // the previous tile has been read out of tensor memory
-        t5_fence_after();
+        pf_slice(a, u, npairs, kbase, nst);
         for (int s = 0; s < nst; s++, it++) {
           const int slot = it % PF_STAGES;
-          wait(full_a(slot), (uint32_t)(it / PF_STAGES) & 1u);
           wait(full_b(slot), (uint32_t)(it / PF_STAGES) & 1u);
+          mbar_arrive_cluster(t5_map_rank(full(slot), 0));
+        }
+      }
+    }
+  } else if (warp == 9 || warp == 10) {
+    // ---- the tensor cores of the pair, from the leader.  The products of a step are spread over two warps; MMAs into one
+    // accumulator come from one thread (a thread's MMAs execute in its issue order, MMAs of different threads would not be
+    // ordered):
+    //   warp 9: hi.hi -> D1     warp 10: hi.lo and lo.hi -> D23     result = D1 + D23 / 2048
+    //   (tensor-memory columns of each CTA: D1 at 0, D23 at 256)
+    // The whole warp walks the stages and one elected lane issues, so that descriptors stay in uniform registers: inside a
+    // single lane's branch an MMA cost 100 to 200 cycles to issue, more than it takes to execute.
+    if (rank == 0) {
+      const int which = __shfl_sync(0xffffffffu, warp - 9, 0);
+      const bool el = t5_elect();
+      int it = 0, i = 0, slot = 0;
+      uint32_t par = 0;
+      for (int u = unit0; u < nunits; u += ustep, i++) {
+        int kbase, nst;
+        pf_slice(a, u, npairs, kbase, nst);
+        if (i >= 1) wait(acc_empty, (uint32_t)(i - 1) & 1u);   // the previous tiles have been read out of tensor memory
+        t5_fence_after();
+        for (int s = 0; s < nst; s++, it++) {
+          wait(full(slot), par);
           t5_fence_after();
           const uint32_t st = ring_s + slot * PF_STAGE_BYTES, b0 = st + 2 * PF_A_BYTES;
           const uint64_t a_hi = g3_desc(st, 2048, 128), a_lo = g3_desc(st + PF_A_BYTES, 2048, 128);
-          if (!*dead) {
+          const uint64_t b_hi = g3_desc(b0, 2048, 128), b_lo = g3_desc(b0 + PF_B_BYTES, 2048, 128);
+          if (el) {
 #pragma unroll
             for (int k = 0; k < PF_KS / 16; k++) {   // a step is two k-groups further on: the address field counts 16-byte units
-              const uint64_t ka = (uint64_t)(k * 2 * 2048 / 16), kb = (uint64_t)(k * 2 * PF_R * 16 / 16);
+              const uint64_t kk = (uint64_t)(k * 2 * 2048 / 16);
               const uint32_t first = (s | k) != 0;
-              if (which == 0) {
-                for (int un = 0; un < nun; un++)
-                  pf_mma_ss(tmem_base + (uint32_t)(un * 2 * PF_R), a_hi + ka, g3_desc(b0 + un * 2 * PF_B_BYTES, PF_R * 16, 128) + kb, PF_IDESC, first);
-              } else if (which - 1 < nun) {
-                const int un = which - 1;
-                const uint32_t d = tmem_base + (uint32_t)(un * 2 * PF_R + PF_R);
-                const uint64_t b_hi = g3_desc(b0 + un * 2 * PF_B_BYTES, PF_R * 16, 128) + kb, b_lo = g3_desc(b0 + un * 2 * PF_B_BYTES + PF_B_BYTES, PF_R * 16, 128) + kb;
-                pf_mma_ss(d, a_hi + ka, b_lo, PF_IDESC, first);
-                pf_mma_ss(d, a_lo + ka, b_hi, PF_IDESC, 1u);
+              if (which == 0) pf_mma_ss(tmem_base, a_hi + kk, b_hi + kk, PF_IDESC, first);
+              else {
+                pf_mma_ss(tmem_base + PF_RMAX, a_hi + kk, b_lo + kk, PF_IDESC, first);
+                pf_mma_ss(tmem_base + PF_RMAX, a_lo + kk, b_hi + kk, PF_IDESC, 1u);
               }
             }
+            t5_commit_pair(empty(slot));   // arrives in both CTAs when this thread's MMAs have read the stage
+            if (s + 1 == nst) t5_commit_pair(acc_full);   // ... and when this thread's share of the tiles is in tensor memory
           }
-          t5_commit(empty(slot));        // arrives when this thread's MMAs have read the stage
+          __syncwarp();
+          if (++slot == PF_STAGES) { slot = 0; par ^= 1u; }
         }
-        t5_commit(acc_full(0));          // ... and when this thread's share of the tile is in tensor memory
       }
-      // nothing of this CTA may still run on the tensor core when its tensor memory is freed
-      if (i > 0) wait(acc_full(0), (uint32_t)(i - 1) & 1u);
+      // nothing of the pair may still run on the tensor cores when its tensor memory is freed
+      if (i > 0) mbar_wait(acc_full, (uint32_t)(i - 1) & 1u);   // (bounded; after a wait that gave up too: the commits above always arrive)
     }
   } else if (warp >= 12) {
     // ---- results: lane quarter q of the accumulators, one weight row per thread ----
@@ -338,21 +354,22 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
     // fifth of its life; now 2000.
     const int q = warp - 12, R = a.R;
     int i = 0;
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x, i++) {
+    for (int u = unit0; u < nunits; u += ustep, i++) {
       int m, row0;
-      pf_locate(a, u % ntiles, m, row0);
+      const int tile = tile_of(u);
+      pf_locate(a, min(tile, ntiles - 1), m, row0);
       const int row = row0 + 32 * q + lane;
-      const bool on = row < a.m[m].rows;
+      const bool on = tile < ntiles && row < a.m[m].rows;
       const size_t os = a.m[m].ostride;
-      float *out = a.m[m].out + (size_t)(u / ntiles) * a.m[m].split_stride + row;
-      wait(acc_full(0), (uint32_t)i & 1u);
+      float *out = a.m[m].out + (size_t)(u / npairs) * a.m[m].split_stride + row;
+      wait(acc_full, (uint32_t)i & 1u);
       t5_fence_after();
       const uint32_t t0 = tmem_base + ((uint32_t)(32 * q) << 16);
 #pragma unroll 1
       for (int c = 0; c < R; c += 16) {       // chunk rows c .. c + 15 are columns c .. of both accumulators
         float v[16], v2[16];
         t5_ld16(t0 + c, v);
-        t5_ld16(t0 + c + PF_R, v2);
+        t5_ld16(t0 + c + PF_RMAX, v2);
         t5_wait_ld();
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] += v2[j] * XP_LO_INV;
@@ -366,13 +383,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pfmm(const PfArgs a) {
       }
       t5_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty(0));
+      if (lane == 0) mbar_arrive_cluster(t5_map_rank(acc_empty, 0));
     }
   }
+  __syncwarp();
   t5_fence_before();
-  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // no CTA leaves while the other still arrives here or reads its memory
   if (warp == 10) {
     t5_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }

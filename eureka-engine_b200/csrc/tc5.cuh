@@ -50,6 +50,26 @@ __device__ __forceinline__ void mbar_init(uint32_t bar_s, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar_s) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_s) : "memory");
 }
+// ---- pairs of CTAs (cta_group::2) ----
+// address of the same shared-memory word in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t t5_map_rank(uint32_t addr_s, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr_s), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr_cl) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr_cl) : "memory");
+}
+// arrives on this barrier word of both CTAs when the thread's MMAs are done
+__device__ __forceinline__ void t5_commit_pair(uint32_t bar_s) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar_s), "h"((uint16_t)3) : "memory");
+}
+// one thread of the warp (the same one every time); the warp has to be converged
+__device__ __forceinline__ bool t5_elect(void) {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
 // bounded wait for the phase with the given parity; false when the limit ran out
 __device__ __forceinline__ bool mbar_wait(uint32_t bar_s, uint32_t parity, uint32_t limit = T5_WAIT_LIMIT) {
   for (uint32_t it = 0; it < limit; it++) {
