@@ -199,7 +199,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1) k_pfm
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  pdl_wait();              // the activations come from the kernel in front
   t5_fence_before();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // both CTAs' barriers exist
   t5_fence_after();
@@ -272,6 +271,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1) k_pfm
     // ---- activations of this CTA's half of the chunk's rows: one 16 KB bulk copy per plane and stage ----
     if (lane == 0) {
       int it = 0;
+      pdl_wait();   // the activations come from the kernel in front; the weights do not, and nothing is written before MMAs have read activations
       const __half *x = a.x + (size_t)rank * pf_kg_halves(a.K);   // a unit's planes follow the previous unit's (common.cuh)
       for (int u = unit0; u < nunits; u += ustep) {
         int kbase, nst;
