@@ -74,8 +74,8 @@ LLB_API int llb_b200_graph_bail(void);
 LLB_API void llb_b200_graph_stats(unsigned long long out[4]);
 
 /* ---- 2. operator entry points --------------------------------------------------------------- */
-/* Bytes of a [rows x cols] matrix in the device layout (Q6_K super-blocks are padded from 210 to
- * 224 bytes at upload; every other format is stored as in a pack). */
+/* Bytes of a [rows x cols] matrix in the device layout (contiguous tiles of 16 rows x 256 columns; the last
+ * rows and columns are filled up to whole tiles). */
 LLB_API size_t llb_b200_weight_bytes(int fmt, int rows, int cols);
 /* Pack bytes (host pointer, or device address when src_on_device) -> device layout at dst. */
 LLB_API int llb_b200_weight_upload(int fmt, int rows, int cols, const void *src, int src_on_device, llb_b200_dptr dst);
