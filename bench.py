@@ -604,7 +604,7 @@ def main():
                                           "stream, so no one-block drafter (whatever eh_proj) predicts the trunk; value is the cycle rate. "
                                           "plain_decode is k = 0 on the same engine, prompt and position",
                        "prompt": len(prompt), "prefill_s": round(t_pre, 3), "prefill_tok_s": round(len(prompt) / t_pre, 1),
-                       "prefill": "8-row verify passes" if args.exact_prefill else "dense tcgen05 path, chunks of 128 rows (all but the last k + 1 rows)", "build_s": round(t_build, 2)},
+                       "prefill": "8-row verify passes" if args.exact_prefill else "dense tcgen05 path, chunks of 256 rows (all but the last k + 1 rows)", "build_s": round(t_build, 2)},
             "cycle_ms": ms / steps, "tokens_per_cycle": toks / (steps * world), "plain_decode": plain, "with_acceptance": accept_leg,
             "wait_errors": llb.lib().llb_b200_wait_errors(),   # 1 if a bounded device-side wait ever ran out (results then invalid)
             "clocks": clocks,
