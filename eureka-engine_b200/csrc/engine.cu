@@ -141,7 +141,7 @@ struct llb_spec {
   int Hf = 0, KVf = 0, ff = 0, GKf = 0, TRf = 0, kdcf = 0, vdcf = 0, convdf = 0;
   OutBuf r_a, r_dn;
   PfState pf;
-  int prefill_mode = 0;   // 0: every prompt row through the T-row pass; 1: chunks of PF_R rows through the dense path (LLB_PREFILL=fast)
+  int prefill_mode = 0;   // 0: every prompt row through the T-row pass; 1: chunks of PF_RMAX rows through the dense path (LLB_PREFILL=fast)
   double pf_rows = 0;     // prompt rows the dense path has processed since the engine was opened
   // graphs
   cudaGraphExec_t g_spec = nullptr, g_prefill = nullptr, g_verify = nullptr;

@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const 
   decay[h * PF_RMAX + t] = (float)exp((double)(sp * sa[h]));
 }
 // The recurrence over the chunk's R rows.  Block (hh, y) keeps 32 state rows of value head hh in registers from the first
-// row of the chunk to the last and writes them back once (a lane: four state rows, columns 4 cq .. and 64 + 4 cq ..).  Per row t and state row j: S_j *= decay; delta = (v_j - S_j . k) * beta; S_j += k * delta; o_j = S_j . q
-// (:630-646).
+// row of the chunk to the last and writes them back once (a lane: four state rows, columns 4 cq .. and 64 + 4 cq ..).
+// Per row t and state row j: S_j *= decay; delta = (v_j - S_j . k) * beta; S_j += k * delta; o_j = S_j . q (:630-646).
 //
 // Row by row that is a chain: a dot product, its shuffles, the update, 0.4 to 0.6 us a row.  Here a step takes eight rows.  With
 // S the state before them and d(s, t] the product of decays of rows s + 1 .. t,

@@ -103,3 +103,11 @@ def test_c2_shape_truncated(pkg, packs, llb):
     pack = packs.build_pack(cfg, device="cuda:0")
     mtp = packs.aux1_bytes(packs.build_mtp(pack))
     _compare(pkg, pack, mtp, 3, packs.synth_prompt(3, 600, cfg.vocab_size))
+
+
+@pytest.mark.parametrize("rows", [32, 33, 39, 127, 129, 257, 263])   # fewer than 32 rows do not take the dense path
+def test_rows_at_the_edges_of_steps_and_units(pkg, packs, llb, rows):
+    """The recurrence takes eight rows a step and the dense GEMM units of 128: chunks that end inside either, or one row past."""
+    cfg = packs.cfg_tiny(n_layers=4, seed=21)
+    pack = packs.build_pack(cfg)
+    _compare(pkg, pack, None, 0, packs.synth_prompt(9, rows + 2, cfg.vocab_size))
