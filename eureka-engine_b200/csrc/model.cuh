@@ -142,7 +142,7 @@ __device__ __forceinline__ const RowSet *rs_begin(const RowSet *rs, int &n, int 
   rs = (const RowSet *)((uintptr_t)rs & ~(uintptr_t)1);
   if (early) { n = *(const volatile int *)&rs->n; pos0 = *(const volatile int *)&rs->pos0; }
   pdl_wait();
-  if (!early) { n = rs->n; pos0 = rs->pos0; }
+  if (!early) { n = __ldcg(&rs->n); pos0 = __ldcg(&rs->pos0); }
   return rs;
 }
 // The same for row t of a pass over several streams: the row set of the row's stream, and tl, the row's index in it.

@@ -45,6 +45,28 @@ template <int NTC> __device__ __forceinline__ void moe_col(const float (&acc)[NT
   v1 = acc[0][i + 2] + lo[i + 2] * XP_LO_INV;
 }
 
+// The router's choice as a launch uses it: the expert ids and the rows in use, copied to shared memory behind the wait.  They are
+// rewritten layer after layer, so they come from L2 (a line of an earlier layer may still be in this SM's L1), once a block:
+// every copy that a warp requests looks its expert up.
+#define MOE_MAXIDS (16 * 33)   // sixteen rows of 32 experts and the shared one
+struct MoeSel { int live[17], ids[MOE_MAXIDS]; };
+__device__ __forceinline__ void moe_sel(const MoeArgs &m, MoeSel &s) {
+  pdl_wait();
+  for (int i = threadIdx.x; i < 17; i += blockDim.x) s.live[i] = __ldcg(m.live + i);
+  for (int i = threadIdx.x; i < m.T * m.nslot; i += blockDim.x) s.ids[i] = __ldcg(m.ids + i);
+}
+// a launch's own stage behind that copy (its barrier covers both)
+template <class Base> struct MoeStage {
+  const MoeArgs &m;   // the choice in global memory
+  MoeSel &s;
+  const Base base;
+  __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
+    moe_sel(m, s);
+    base(xh_s, xsf_s, CS, sb0, nsl);
+  }
+};
+
+// (m: the launch's arguments with ids and live in shared memory)
 template <int FMT> struct MoeGuMats {
   static constexpr bool EARLY = false, CONTIG = true;
   const MoeArgs &m;
@@ -101,8 +123,11 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_gu(const 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeGuMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                          G2StagePlanes<FMT, NT>{a}, MoeGuMats<FMT>{m});
+  __shared__ MoeSel sel;
+  MoeArgs ms = m;
+  ms.ids = sel.ids; ms.live = sel.live;
+  g2_phase<FMT, NT, MoeStage<G2StagePlanes<FMT, NT>>, MoeGuMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                                    MoeStage<G2StagePlanes<FMT, NT>>{m, sel, {a}}, MoeGuMats<FMT>{ms});
   g2_drain(rg);
 }
 // The down launch's activation slice built in shared memory from the gate|up outputs (T <= 4 rows): wt * silu(g) * u
@@ -113,7 +138,7 @@ template <int FMT> struct MoeStageSilu {
   const float *wt;   // [T][nslot]
   __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
     pdl_wait();
-    const int lane = threadIdx.x & 31, nl = min(*m.live, m.T), T = nl > 0 ? m.live[nl] + 1 : 0, f = m.nslot * m.ef;
+    const int lane = threadIdx.x & 31, nl = min(__ldcg(m.live), m.T), T = nl > 0 ? __ldcg(m.live + nl) + 1 : 0, f = m.nslot * m.ef;
     const int ngrp = nsl * 64, ntask = 4 * ngrp;   // (row of the 4 plane pairs, group of four columns); rows >= T are zero planes
     for (int t0 = threadIdx.x; t0 < ntask; t0 += 4 * blockDim.x) {
       float4 gv[4], uv[4];
@@ -148,7 +173,10 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8) * 32, 1) k_moe_dn_silu(const 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8) / g2_warps(FMT, 8));
-  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStageSilu<FMT>{m, wt}, MoeDnMats<FMT>{m});
+  __shared__ MoeSel sel;
+  MoeArgs ms = m;
+  ms.ids = sel.ids; ms.live = sel.live;
+  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStage<MoeStageSilu<FMT>>{m, sel, {m, wt}}, MoeDnMats<FMT>{ms});
   g2_drain(rg);
 }
 
@@ -157,7 +185,10 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_dn(const 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT>, MoeDnMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                          G2StagePlanes<FMT, NT>{a}, MoeDnMats<FMT>{m});
+  __shared__ MoeSel sel;
+  MoeArgs ms = m;
+  ms.ids = sel.ids; ms.live = sel.live;
+  g2_phase<FMT, NT, MoeStage<G2StagePlanes<FMT, NT>>, MoeDnMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
+                                                                                    MoeStage<G2StagePlanes<FMT, NT>>{m, sel, {a}}, MoeDnMats<FMT>{ms});
   g2_drain(rg);
 }

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(256) k_xp_from_bf16(const unsigned short *__re
     const unsigned short *r = x + (size_t)t * K + c;
     uint2 w;
     if (!((uintptr_t)x & 7)) w = __ldcg((const uint2 *)r);
-    else w = make_uint2(r[0] | ((uint32_t)r[1] << 16), r[2] | ((uint32_t)r[3] << 16));
+    else w = make_uint2(__ldcg(r) | ((uint32_t)__ldcg(r + 1) << 16), __ldcg(r + 2) | ((uint32_t)__ldcg(r + 3) << 16));
     v[0] = __uint_as_float(w.x << 16); v[1] = __uint_as_float(w.x & 0xffff0000u); v[2] = __uint_as_float(w.y << 16); v[3] = __uint_as_float(w.y & 0xffff0000u);
   }
   xp_store4(xp, t, 1, c, v, threadIdx.x & 31, c < K);
@@ -159,8 +159,8 @@ __global__ void k_sum_parts(const float *__restrict__ parts, int nsplit, long lo
   pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float v = parts[i];
-  for (int k = 1; k < nsplit; k++) v += parts[(size_t)k * stride + i];
+  float v = __ldcg(parts + i);   // (to L2: the GEMM in front wrote them, and the buffer is used by one call after another)
+  for (int k = 1; k < nsplit; k++) v += __ldcg(parts + (size_t)k * stride + i);
   out[i] = v;
 }
 int ops_sum_parts(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int n, float *out) {

@@ -32,7 +32,7 @@ __global__ void k_embed(int fmt, const uint8_t *__restrict__ W, int d, const Row
   const int t = blockIdx.y;
   rs = rs_begin_row(rs, sg, t, rs_n, rs_p0, tl);
   if (tl >= rs_n) return;
-  const int row = rs->tok[tl];
+  const int row = __ldcg(&rs->tok[tl]);   // (a draft's token was written by the kernel two launches in front)
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d; c += gridDim.x * blockDim.x) x[(size_t)t * d + c] = deq_elem(fmt, W, d, row, c);
 }
 int op_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const RowSet *rs, int Tmax, float *x) {
@@ -204,10 +204,10 @@ __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__
     acc[t] = 0.0f;
     if (t < rs_n) {
       const float4 *x = (const float4 *)(h + (size_t)t * d);
-      if (c0 < nc) { const float4 v = x[c0]; acc[t] += (w0.x * v.x + w0.y * v.y) + (w0.z * v.z + w0.w * v.w); }
-      if (c1 < nc) { const float4 v = x[c1]; acc[t] += (w1.x * v.x + w1.y * v.y) + (w1.z * v.z + w1.w * v.w); }
+      if (c0 < nc) { const float4 v = __ldcg(x + c0); acc[t] += (w0.x * v.x + w0.y * v.y) + (w0.z * v.z + w0.w * v.w); }
+      if (c1 < nc) { const float4 v = __ldcg(x + c1); acc[t] += (w1.x * v.x + w1.y * v.y) + (w1.z * v.z + w1.w * v.w); }
       for (int c = threadIdx.x + 512; c < nc; c += 256) {
-        const float4 w = __ldg(wr + c), v = x[c];
+        const float4 w = __ldg(wr + c), v = __ldcg(x + c);
         acc[t] += (w.x * v.x + w.y * v.y) + (w.z * v.z + w.w * v.w);
       }
     }
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__
   if (threadIdx.x == 0) *ctr = 0;   // ready for the next launch (launches of one stream do not overlap here)
   // which rows are in use: all of them in a pass of one stream, else the first n of every stream's
   bool on = lane < rs_n;
-  if (n_all > 0 && on) { const int z = lane / sg.per; on = lane - z * sg.per < ((const RowSet *)((const char *)rs + (size_t)z * sg.stride))->n; }
+  if (n_all > 0 && on) { const int z = lane / sg.per; on = lane - z * sg.per < __ldcg(&((const RowSet *)((const char *)rs + (size_t)z * sg.stride))->n); }
   const unsigned int mask = __ballot_sync(0xffffffffu, on);
   if (warp == 0) {
     if (lane == 0) live[0] = __popc(mask);
@@ -386,7 +386,7 @@ k_delta(float *__restrict__ S, const SpecCtl *__restrict__ ctl, PartIn ring, con
   const int zt = 4 * wp + (lane >> 3), zc = 4 * (lane & 7), col = hh * 128 + 32 * jq + zc;
   const size_t zi = (size_t)(row0 + zt) * sh.vdc + col;
   pdl_wait();
-  if (!early) { n = rs->n; pos0 = rs->pos0; }
+  if (!early) { n = __ldcg(&rs->n); pos0 = __ldcg(&rs->pos0); }
   const int nr = n + KC - 1;
   if (n < 1) { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); return; }   // every block of the cluster takes the same exit
   // the gates' inputs, then the ring rows, then (behind them, for the end) z: four slices of each in flight
@@ -582,9 +582,9 @@ int op_top2_part(cudaStream_t s, PartIn logits, int V, long long row_stride, flo
 __device__ __forceinline__ Top2 t2_final(const float *part, int t, int lane) {
   Top2 a = {0.f, -1, 0.f, -1};
   for (int b = lane; b < TOP2_NB; b += 32) {
-    const float *p = part + ((size_t)t * TOP2_NB + b) * 4;
-    t2_push(a, p[0], __float_as_int(p[1]));
-    t2_push(a, p[2], __float_as_int(p[3]));
+    const float4 p = __ldcg((const float4 *)part + (size_t)t * TOP2_NB + b);   // (to L2: every drafter step writes the same partials)
+    t2_push(a, p.x, __float_as_int(p.y));
+    t2_push(a, p.z, __float_as_int(p.w));
   }
   return t2_warp(a);
 }
@@ -604,27 +604,34 @@ __global__ void k_accept(const float *__restrict__ part, SpecCtl *__restrict__ c
   // one block per stream: its control block, its result ring, its rows of the pass
   ctl += blockIdx.x; ring += (size_t)blockIdx.x * ring_n;
   const int row0 = blockIdx.x * per;
-  const int T = ctl->verify.n;
+  const int T = __ldcg(&ctl->verify.n);
   if (T < 1) return;   // an empty pass (the sizing run at open, a stream that is not running) decides nothing
   if (warp < T) {
     Top2 a = t2_final(part, row0 + warp, lane);
     // sampling mode: the row's emitted token is the sampler's (llb_smp_verify / llb_smp_sample), not the argmax; the
     // argmax's runner-up stays in the record's third and fourth words
-    if (smp_tok) { if (a.i1 != smp_tok[row0 + warp]) { a.i2 = a.i1; a.v2 = a.v1; } a.i1 = smp_tok[row0 + warp]; a.v1 = smp_val[row0 + warp]; }
+    if (smp_tok) { const int st = __ldcg(smp_tok + row0 + warp); if (a.i1 != st) { a.i2 = a.i1; a.v2 = a.v1; } a.i1 = st; a.v1 = __ldcg(smp_val + row0 + warp); }
     if (lane == 0) rows[warp] = a;
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
-  const int p0 = ctl->verify.pos0;
+  const int p0 = __ldcg(&ctl->verify.pos0);
+  int tin[SPEC_MAXT];   // the drafts were written by this cycle's earlier kernels
+#pragma unroll
+  for (int r = 0; r < SPEC_MAXT; r++) tin[r] = __ldcg(&ctl->verify.tok[r]);
   SpecResult *res = ring + (ctl->seq % (unsigned long long)ring_n);
   int served = 1;
   if (ctl->forced > 0) served = T;
-  else while (served < T && rows[served - 1].i1 == ctl->verify.tok[served]) served++;
+  else {
+#pragma unroll
+    for (int r = 1; r < SPEC_MAXT; r++) if (served == r && r < T && rows[r - 1].i1 == tin[r]) served++;
+  }
   res->p0 = p0; res->T = T; res->served = served;
-  res->pad = (ctl->chk_on && (ctl->chk_pos != p0 || ctl->chk_tok != ctl->verify.tok[0])) ? 1 : 0;
+  res->pad = (ctl->chk_on && (ctl->chk_pos != p0 || ctl->chk_tok != tin[0])) ? 1 : 0;
   ctl->chk_on = 0;
+#pragma unroll
   for (int r = 0; r < SPEC_MAXT; r++) {
-    res->tin[r] = r < T ? ctl->verify.tok[r] : -1;
+    res->tin[r] = r < T ? tin[r] : -1;
     res->ids[r] = r < T ? rows[r].i1 : -1;
     res->top2[r][0] = r < T ? (unsigned)rows[r].i1 : 0u;
     res->top2[r][1] = r < T ? __float_as_uint(rows[r].v1) : 0u;
@@ -671,18 +678,19 @@ __global__ void __launch_bounds__(256) k_lookup_draft(SpecCtl *__restrict__ ctl)
   __shared__ int best[3];
   ctl += blockIdx.x;   // one block per stream
   const int *hist = ctl->hist;
-  const int pos = ctl->verify.pos0;
-  if (!hist || ctl->verify.n < 1) return;
+  const int pos = __ldcg(&ctl->verify.pos0);   // (this block, the row count and the history's end: just written by k_accept)
+  const int rows = __ldcg(&ctl->verify.n);
+  if (!hist || rows < 1) return;
   if (threadIdx.x < 3) best[threadIdx.x] = -1;
   __syncthreads();
-  const int t0 = hist[pos], t1 = pos >= 1 ? hist[pos - 1] : -1, t2 = pos >= 2 ? hist[pos - 2] : -1;
+  const int t0 = __ldcg(hist + pos), t1 = pos >= 1 ? __ldcg(hist + pos - 1) : -1, t2 = pos >= 2 ? __ldcg(hist + pos - 2) : -1;
   int b1 = -1, b2 = -1, b3 = -1;
   for (int j = pos - 1 - (int)threadIdx.x; j >= 0; j -= blockDim.x) {
-    if (hist[j] != t0) continue;
+    if (__ldcg(hist + j) != t0) continue;
     if (b1 < 0) b1 = j;
-    if (j >= 1 && pos >= 2 && hist[j - 1] == t1) {
+    if (j >= 1 && pos >= 2 && __ldcg(hist + j - 1) == t1) {
       if (b2 < 0) b2 = j;
-      if (j >= 2 && pos >= 3 && hist[j - 2] == t2) { if (b3 < 0) b3 = j; }
+      if (j >= 2 && pos >= 3 && __ldcg(hist + j - 2) == t2) { if (b3 < 0) b3 = j; }
     }
     if (b3 >= 0) break;   // later iterations only see smaller j
   }
@@ -694,8 +702,8 @@ __global__ void __launch_bounds__(256) k_lookup_draft(SpecCtl *__restrict__ ctl)
   const int j = best[2] >= 0 ? best[2] : best[1] >= 0 ? best[1] : best[0];
   int n = 0;
   if (j >= 0) {
-    const int room = ctl->verify.n - 1;   // the accept kernel already clipped the rows to the context
-    while (n < ctl->k && n < room && j + 1 + n <= pos) { ctl->verify.tok[1 + n] = hist[j + 1 + n]; n++; }
+    const int room = rows - 1;   // the accept kernel already clipped the rows to the context
+    while (n < ctl->k && n < room && j + 1 + n <= pos) { ctl->verify.tok[1 + n] = __ldcg(hist + j + 1 + n); n++; }
   }
   ctl->verify.n = 1 + n;
 }
@@ -718,17 +726,17 @@ __global__ void k_draft_pick(const float *__restrict__ part, const int *__restri
   const size_t row0 = (size_t)blockIdx.x * per;
   part += row0 * TOP2_NB * 4; mt_hn += row0 * d; chain_h += row0 * d;
   const RowSet *rs = from_chain ? &ctl->chain : &ctl->catchup;
-  const int last = rs->n - 1;
+  const int last = __ldcg(&rs->n) - 1;
   if (last < 0) return;
   if (threadIdx.x < 32) {
     Top2 a = t2_final(part, last, threadIdx.x);
     if (threadIdx.x == 0) s_tok = a.i1 < 0 ? 0 : ids ? ids[a.i1] : a.i1;
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < d; c += blockDim.x) chain_h[c] = mt_hn[(size_t)last * d + c];
+  for (int c = threadIdx.x; c < d; c += blockDim.x) chain_h[c] = __ldcg(mt_hn + (size_t)last * d + c);
   if (threadIdx.x == 0) {
-    const int p = ctl->verify.pos0;
-    if (j < ctl->verify.n) ctl->verify.tok[j] = s_tok;
+    const int p = __ldcg(&ctl->verify.pos0);
+    if (j < __ldcg(&ctl->verify.n)) ctl->verify.tok[j] = s_tok;
     ctl->chain.n = 1;
     ctl->chain.pos0 = p + j;
     ctl->chain.tok[0] = s_tok;

@@ -152,15 +152,16 @@ __global__ void __launch_bounds__(SMP_THREADS) k_smp_rows(SmpDev P, PartIn lg, i
     const int z = t / sg.per, tl = t - z * sg.per;
     const SpecCtl *c = (const SpecCtl *)((const char *)ctl + (size_t)z * sg.stride);
     const RowSet &rs = c->verify;
-    if (tl >= rs.n) return;
-    const int prow = rs.pos0 + tl;
+    const int n = __ldcg(&rs.n), pos0 = __ldcg(&rs.pos0);   // (to L2: earlier kernels of this cycle wrote the drafts)
+    if (tl >= n) return;
+    const int prow = pos0 + tl;
     pos = (unsigned long long)prow + 1ull;
-    draft = tl + 1 < rs.n ? rs.tok[tl + 1] : -1;
+    draft = tl + 1 < n ? __ldcg(&rs.tok[tl + 1]) : -1;
     if (P.pen_on) {
       // the tokens at positions prow + 1 - N .. prow: history up to the pass's first row, then the pass's own inputs
       const int N = P.repeat_last_n, q0 = prow + 1 - N > 0 ? prow + 1 - N : 0;
       nwin = prow + 1 - q0;
-      for (int a = tid; a < nwin; a += SMP_THREADS) { const int q = q0 + a; sh.win[a] = q <= rs.pos0 ? (q == rs.pos0 ? rs.tok[0] : (c->hist ? c->hist[q] : -1)) : rs.tok[q - rs.pos0]; }
+      for (int a = tid; a < nwin; a += SMP_THREADS) { const int q = q0 + a; sh.win[a] = q >= pos0 ? __ldcg(&rs.tok[q - pos0]) : c->hist ? __ldcg(c->hist + q) : -1; }
     }
   } else {
     draft = t_draft[t]; pos = (unsigned long long)t_pos[t];
