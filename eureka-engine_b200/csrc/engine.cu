@@ -459,6 +459,24 @@ static int load_moe(llb_spec *m, FfnW &w, const std::string &p, const std::unord
   return 0;
 }
 
+// Does a pass of T rows fit the GEMMs' shared memory?  Every matrix of the index in the K-slices it may have: sixteen, those of
+// the conv ring's launch RING_MAXSPLIT, one for the experts' gate and up.
+static bool width_fits(const llb_spec *m, const std::unordered_map<std::string, TensorRec> &tab, int T) {
+  const int NC = nc_of(T);
+  auto fits = [&](int fmt, int nsb, int cap) {
+    const int ks = cap > 1 ? gemm_fix_ksplit(fmt, NC, nsb, 1) : 1;
+    return ks <= cap && (nsb + ks - 1) / ks <= gemm_longest_slice(fmt, NC);
+  };
+  for (const auto &kv : tab) {
+    const TensorRec &t = kv.second;
+    const std::string &n = kv.first;
+    if (t.fmt == LLB_FM_F32 || n.find("_shexp") != std::string::npos) continue;   // (the shared expert is a block of the stacks)
+    if (n.find("down_exps") != std::string::npos) { if (!fits(t.fmt, (m->nk + 1) * m->ef / 256, 16)) return false; }
+    else if (n.find("_exps") != std::string::npos) { if (!fits(t.fmt, m->d / 256, 1)) return false; }
+    else if (!fits(t.fmt, (t.cols + 255) / 256, n.find("attn_qkv") != std::string::npos ? RING_MAXSPLIT : 16)) return false;
+  }
+  return fits(LLB_FM_Q8_0, 2 * m->d / 256, 16);   // a drafter's input projection, whatever its format
+}
 static int check_k(const DevMat &w, int rows, int cols, const char *what) {
   if (w.rows != rows || w.cols != cols) return llb_fail("%s is [%d x %d], the configuration needs [%d x %d]", what, w.rows, w.cols, rows, cols);
   if (w.fmt == LLB_FM_F32) return llb_fail("%s: F32 matrices have no GEMM kernel", what);
@@ -815,7 +833,12 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
     if (pf > 48 / (m->H / m->KV)) pf = 48 / (m->H / m->KV);
     m->Tpf = pf > m->Tspec ? pf : m->Tspec;
     // several streams: the sixteen rows of a pass shared out among them (eight streams of plain decoding feed two rows each)
-    if (m->B > 1) { const int share = 16 / m->B < pf ? 16 / m->B : pf; m->Tpf = share > m->Tspec ? share : m->Tspec; }
+    // (fewer where sixteen rows' activations leave a wide model's K-slices no room that the speculative width leaves them)
+    if (m->B > 1) {
+      int share = 16 / m->B < pf ? 16 / m->B : pf;
+      while (share > m->Tspec && !width_fits(m, tab, m->B * share)) share--;
+      m->Tpf = share > m->Tspec ? share : m->Tspec;
+    }
   }
   m->per = m->Tpf;
   m->Tmax = rows_cap(m);                 // buffers are sized for the widest pass

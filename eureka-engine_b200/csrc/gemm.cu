@@ -22,10 +22,10 @@ static double gemm_stream_cost(int fmt, int warps, int nc, int tiles, int slice,
 // Parts of a row tile's K-slice (g2_phase): the power of two with the lowest cost that divides the warps, leaves every part a
 // super-block and whose sums fit beside the activation slice.  tiles: row tiles of a CTA, nsb in ks slices
 static int gemm_pick_parts(int fmt, int NC, int ntc, int tiles, int nsb, int ks) {
-  const int warps = g2_warps(fmt, NC), slice = (nsb + ks - 1) / ks;
+  const int warps = g2_warps(fmt, NC), slice = (nsb + ks - 1) / ks, ring = g2_ring_of(fmt, NC, slice);
   int best = 1;
   for (int p = 2; p <= 16 && p <= nsb / ks && warps % p == 0; p *= 2)
-    if (g2_smem(fmt, slice, NC, p, ntc) <= G2_SMEM_MAX && gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, p) < gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, best)) best = p;
+    if (g2_smem(fmt, slice, NC, p, ntc, ring) <= G2_SMEM_MAX && gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, p) < gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, best)) best = p;
   return best;
 }
 template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
@@ -35,10 +35,12 @@ template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
   // every SM takes part as long as there is a tile for it: the tiles are dealt out one per CTA in turn
   if (cps > a.tile0[a.nmat]) cps = a.tile0[a.nmat];
   a.parts = gemm_pick_parts(FMT, NC, NT, (a.tile0[a.nmat] + cps - 1) / cps, a.nsb, a.ksplit);
-  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, NT);
+  const int ring = g2_ring_of(FMT, NC, nsl);
+  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, NT, ring);
   if (smem > G2_SMEM_MAX) return llb_fail("k_gemm2: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   const bool fold = (long long)a.tile0[a.nmat] * a.nsb >= G2_FOLD_TILES;
-  cudaError_t e = llb_launch(fold ? k_gemm2<FMT, NT, g2_folds(FMT, NT)> : k_gemm2<FMT, NT, false>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
+  cudaError_t e = llb_launch(ring ? k_gemm2<FMT, NT, false, g2_has_short(FMT, 8 * NT)> : fold ? k_gemm2<FMT, NT, g2_folds(FMT, NT), 0> : k_gemm2<FMT, NT, false, 0>,
+                             dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
   if (e != cudaSuccess) return llb_fail("k_gemm2 launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -99,29 +101,26 @@ int gemm_wait_selftest(cudaStream_t s, int which, int limit) {
   return 0;
 }
 
-template <int FMT> static int setup_fmt2() {
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_gemm2<FMT, 4, g2_folds(FMT, 4)>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
+template <typename K> static int setup_smem(K k) {
+  CU_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
   return 0;
 }
-
-template <int FMT> static int setup_moe() {
-  CU_OK(cudaFuncSetAttribute(k_moe_gu<FMT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_moe_gu<FMT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_moe_dn<FMT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_moe_dn<FMT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_moe_gu<FMT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_moe_dn<FMT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  CU_OK(cudaFuncSetAttribute(k_moe_dn_silu<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
-  return 0;
+template <int FMT, int NT> static int setup_fmt2() {
+  return setup_smem(k_gemm2<FMT, NT, false, 0>) || setup_smem(k_gemm2<FMT, NT, g2_folds(FMT, NT), 0>) || setup_smem(k_gemm2<FMT, NT, false, g2_has_short(FMT, 8 * NT)>);
+}
+template <int FMT, int NT> static int setup_moe() {
+  constexpr int SH = g2_has_short(FMT, 8 * NT);
+  return setup_smem(k_moe_gu<FMT, NT, 0>) || setup_smem(k_moe_gu<FMT, NT, SH>) || setup_smem(k_moe_dn<FMT, NT, 0>) || setup_smem(k_moe_dn<FMT, NT, SH>);
+}
+template <int FMT> static int setup_fmt() { return setup_fmt2<FMT, 1>() || setup_fmt2<FMT, 2>() || setup_fmt2<FMT, 4>(); }
+template <int FMT> static int setup_experts() {
+  return setup_moe<FMT, 1>() || setup_moe<FMT, 2>() || setup_moe<FMT, 4>() || setup_smem(k_moe_dn_silu<FMT, 0>) || setup_smem(k_moe_dn_silu<FMT, g2_has_short(FMT, 8)>);
 }
 
 int gemm_setup(void) {
-  if (setup_fmt2<LLB_FM_Q4_K>() || setup_fmt2<LLB_FM_Q5_K>() || setup_fmt2<LLB_FM_Q6_K>() || setup_fmt2<LLB_FM_Q8_0>()) return -1;
+  if (setup_fmt<LLB_FM_Q4_K>() || setup_fmt<LLB_FM_Q5_K>() || setup_fmt<LLB_FM_Q6_K>() || setup_fmt<LLB_FM_Q8_0>()) return -1;
   CU_OK(cudaFuncSetAttribute(k_gemm3, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM_MAX));
-  if (setup_moe<LLB_FM_Q4_K>() || setup_moe<LLB_FM_Q5_K>() || setup_moe<LLB_FM_Q6_K>()) return -1;
+  if (setup_experts<LLB_FM_Q4_K>() || setup_experts<LLB_FM_Q5_K>() || setup_experts<LLB_FM_Q6_K>()) return -1;
   CU_OK(cudaFuncSetAttribute(k_ffn<LLB_FM_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
   CU_OK(cudaFuncSetAttribute(k_ffn<LLB_FM_Q5_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
   CU_OK(cudaFuncSetAttribute(k_ffn<LLB_FM_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
@@ -143,14 +142,17 @@ int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks) {
     const int lo = (nsb + mx - 1) / mx;
     if (ks < lo) ks = lo;
   } else {
-    const int mx = g2_max_slice_sb(fmt, NC);
-    const int lo = (nsb + mx - 1) / mx;       // the activation slice of a CTA has to fit in shared memory
-    if (ks < lo) ks = lo;
+    // the activation slice of a CTA has to fit in shared memory: beside the usual ring, or where that would take too many
+    // slices, beside the shorter one
+    const int mx = g2_max_slice_sb(fmt, NC), most = g2_longest_slice(fmt, NC), lo = (nsb + mx - 1) / mx, least = lo <= GEMM_MAXSPLIT ? lo : (nsb + most - 1) / most;
+    if (ks < least) ks = least;
   }
   if (ks > GEMM_MAXSPLIT) ks = GEMM_MAXSPLIT;
   if (ks > nsb) ks = nsb;
   return ks;
 }
+
+int gemm_longest_slice(int fmt, int NC) { return g2_longest_slice(fmt, NC); }
 
 // K-slices per row tile: streaming, the staging of the slice, and a charge per slice for the partial sums that the consumer
 // has to add (direct: a launch of its own adds them, 1.5 us).
@@ -249,15 +251,17 @@ template <int FMT, int NT> static int launch_moe(cudaStream_t s, bool down, Gemm
   if (cps > ntiles) cps = ntiles;
   // from the capacity of the launch, whatever rows are in use: a row's sums do not depend on its neighbours
   a.parts = gemm_pick_parts(FMT, NC, moe_ntc<NT>(), (ntiles + cps - 1) / cps, a.nsb, a.ksplit);
-  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, moe_ntc<NT>());
+  constexpr int SH = g2_has_short(FMT, 8 * NT);
+  const int ring = g2_ring_of(FMT, NC, nsl);
+  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, moe_ntc<NT>(), ring);
   if (smem > G2_SMEM_MAX) return llb_fail("moe gemm: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   cudaError_t e;
   if (down && wt_silu) {
-    if constexpr (NT == 1) e = llb_launch(k_moe_dn_silu<FMT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, wt_silu, cps);
+    if constexpr (NT == 1) e = llb_launch(ring ? k_moe_dn_silu<FMT, SH> : k_moe_dn_silu<FMT, 0>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, wt_silu, cps);
     else return llb_fail("moe gemm: the down launch builds its own activations for T <= 4 only");
   } else {
-    e = down ? llb_launch(k_moe_dn<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps)
-             : llb_launch(k_moe_gu<FMT, NT>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps);
+    e = down ? llb_launch(ring ? k_moe_dn<FMT, NT, SH> : k_moe_dn<FMT, NT, 0>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps)
+             : llb_launch(ring ? k_moe_gu<FMT, NT, SH> : k_moe_gu<FMT, NT, 0>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps);
   }
   if (e != cudaSuccess) return llb_fail("moe gemm launch: %s", cudaGetErrorString(e));
   return 0;
@@ -276,8 +280,8 @@ int gemm_launch_moe(cudaStream_t s, int fmt, bool down, const XPlanes &xp, MoeAr
   const int ntiles = down ? m.T * (m.d / 16) : m.T * m.nslot * (m.ef / 8);
   int ks = 1;
   if (down) ks = *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, xp.NC, ntiles, a.nsb, g_llb.sms);
-  ks = gemm_fix_ksplit(fmt, xp.NC, a.nsb, ks);
-  if (!down && ks != 1) return llb_fail("moe gemm: %d columns do not fit one K-slice", a.K);
+  if (down) ks = gemm_fix_ksplit(fmt, xp.NC, a.nsb, ks);
+  else if (a.nsb > g2_longest_slice(fmt, xp.NC)) return llb_fail("moe gemm: %d columns do not fit one K-slice", a.K);
   a.ksplit = ks;
   if (ksplit) *ksplit = ks;
   const int NT = xp.NC / 8;

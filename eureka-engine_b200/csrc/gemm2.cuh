@@ -28,31 +28,38 @@
 
 // XPAD: padding of a plane column in shared memory (column stride = 64 mod 128 bytes for the 16-byte B reads of Q4_K / Q5_K /
 // Q8_0, 32 mod 128 for the 8-byte ones of Q6_K), AUX: bytes per (super-block, column) of the sub-block means
-template <int FMT> struct G2Traits { enum { TB = tile_bytes(FMT), TR = tile_row(FMT), XPAD = FMT == LLB_FM_Q6_K ? 32 : 64,
-                                            AUX = FMT == LLB_FM_Q4_K || FMT == LLB_FM_Q5_K ? 32 : 0 }; };
 // Ring depth: 90 to 160 KB an SM in flight (44 KB cover HBM's latency at full rate), less beside 32 plane columns, whose whole
 // d = 2048 slice must fit.
 // Super-blocks a copy brings.  A bulk copy costs about 85 cycles of the SM's copy engine on top of its bytes (copies alone, no
 // arithmetic, gate|up of the 27B shape: 19.6 us at 2304 bytes, 11.8 us at 4608), so Q4_K takes two at a time.
-__host__ __device__ constexpr int g2_chunk(int fmt) { return fmt == LLB_FM_Q4_K ? 2 : 1; }
-__host__ __device__ constexpr int g2_stages(int fmt, int NC) { return fmt == LLB_FM_Q4_K ? (NC >= 32 ? 1 : 2) : NC >= 32 || fmt == LLB_FM_Q8_0 ? 2 : 3; }
+// ring 1: a shorter ring for K-slices that do not fit beside the usual one (ring 0): one K-slice of wide routed-expert models
+// (their epilogue needs whole sums), and matrices of more than GEMM_MAXSPLIT of the usual slices.
+__host__ __device__ constexpr int g2_chunk(int fmt, int ring = 0) { return fmt == LLB_FM_Q4_K && !ring ? 2 : 1; }
+__host__ __device__ constexpr int g2_stages(int fmt, int NC, int ring = 0) {
+  if (ring) return fmt == LLB_FM_Q4_K ? 3 : NC >= 32 ? 1 : 2;
+  return fmt == LLB_FM_Q4_K ? (NC >= 32 ? 1 : 2) : NC >= 32 || fmt == LLB_FM_Q8_0 ? 2 : 3;
+}
+__host__ __device__ constexpr bool g2_has_short(int fmt, int NC) { return NC < 32 ? fmt == LLB_FM_Q4_K : fmt == LLB_FM_Q6_K; }
 // Warps of a CTA: sixteen (128 registers a thread), fewer where the rings of sixteen would leave the activation slice less than
 // the widths in use need: Q8_0's tiles are twice the size, and 32 plane columns take half of the memory.
 __host__ __device__ constexpr int g2_warps(int fmt, int NC) {
   return fmt == LLB_FM_Q8_0 ? 12 : NC < 32 ? 16 : 12;
 }
-__host__ __device__ constexpr int g2_ring_bytes(int fmt, int NC) { return g2_warps(fmt, NC) * g2_stages(fmt, NC) * g2_chunk(fmt) * tile_bytes(fmt); }
+__host__ __device__ constexpr int g2_ring_bytes(int fmt, int NC, int ring = 0) { return g2_warps(fmt, NC) * g2_stages(fmt, NC, ring) * g2_chunk(fmt, ring) * tile_bytes(fmt); }
 __host__ __device__ constexpr int g2_aux(int fmt) { return fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K ? 32 : 0; }
 __host__ __device__ constexpr int g2_xpad(int fmt) { return fmt == LLB_FM_Q6_K ? 32 : 64; }
 // bytes of shared memory of a launch whose K-slices have nsl super-blocks in `parts` parts, for NC activation columns (ntc
 // n-tiles of which are summed over the parts)
-__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC, int parts = 1, int ntc = 4) {
-  return (size_t)(parts > 1 ? g2_warps(fmt, NC) * ntc * 512 : 0) + G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC);
+__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC, int parts = 1, int ntc = 4, int ring = 0) {
+  return (size_t)(parts > 1 ? g2_warps(fmt, NC) * ntc * 512 : 0) + G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC, ring);
 }
-inline int g2_max_slice_sb(int fmt, int NC) {
-  const int left = G2_SMEM_MAX - G2_BAR_BYTES - g2_ring_bytes(fmt, NC) - NC * g2_xpad(fmt);
+inline int g2_max_slice_sb(int fmt, int NC, int ring = 0) {
+  const int left = G2_SMEM_MAX - G2_BAR_BYTES - g2_ring_bytes(fmt, NC, ring) - NC * g2_xpad(fmt);
   return left / (NC * (512 + g2_aux(fmt)));
 }
+// the ring that a K-slice of nsl super-blocks is launched with, and the longest slice of either
+inline int g2_ring_of(int fmt, int NC, int nsl) { return g2_has_short(fmt, NC) && nsl > g2_max_slice_sb(fmt, NC); }
+inline int g2_longest_slice(int fmt, int NC) { return g2_max_slice_sb(fmt, NC, g2_has_short(fmt, NC)); }
 
 // whether a launch of `work` 16 x 256 tiles has the scales folded into the codes: measured at 16 rows, the line lies between
 // 10000 tiles (25.4 us folded, 21.2 not) and 12800 (29.8 folded, 31.2 not); Q5_K, whose codes take more to assemble, gains
@@ -382,9 +389,9 @@ template <int FMT, bool FOLD = false> struct G2MatsPlain {
 // NTC < NT (the routed-expert launches at 16 rows): a weight tile is multiplied with NTC = 2 of the NT staged n-tiles only,
 // the hi and lo tiles of the eight rows its own row is among (Mats::col0(tile) = first plane column of the hi tile; the
 // lo tile is NC / 2 columns on), since the epilogue keeps one row of the tile.
-template <int FMT, int NT, class Stage, class Mats, int NTC = NT, bool FOLD = false>
+template <int FMT, int NT, class Stage, class Mats, int NTC = NT, bool FOLD = false, int RING = 0>
 __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, G2Ring &rg, uint8_t *planes, Stage stage, const Mats mats) {
-  constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC), TB = tile_bytes(FMT), ST = g2_stages(FMT, NC), CH = g2_chunk(FMT);
+  constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC), TB = tile_bytes(FMT), ST = g2_stages(FMT, NC, RING), CH = g2_chunk(FMT, RING);
   static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool live = bid < cps * a.ksplit && warp < WARPS;
@@ -482,12 +489,13 @@ template <int FMT, int NT, bool FOLD = false> struct G2StagePlanes {
   }
 };
 
-template <int FMT, int NT, bool FOLD>
+template <int FMT, int NT, bool FOLD, int RING>
 __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_gemm2(const GemmArgs a, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT, FOLD>, G2MatsPlain<FMT, FOLD>, NT, FOLD>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                                   G2StagePlanes<FMT, NT, FOLD>{a}, G2MatsPlain<FMT, FOLD>{a});
+  constexpr int RB = g2_ring_bytes(FMT, 8 * NT, RING);
+  G2Ring rg = g2_ring_init(smem, RB / g2_warps(FMT, 8 * NT));
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT, FOLD>, G2MatsPlain<FMT, FOLD>, NT, FOLD, RING>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<FMT, NT, FOLD>{a},
+                                                                                         G2MatsPlain<FMT, FOLD>{a});
   g2_drain(rg);
 }

@@ -118,16 +118,17 @@ template <int FMT> struct MoeDnMats {
   }
 };
 
-template <int FMT, int NT>
+template <int FMT, int NT, int RING>
 __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_gu(const GemmArgs a, const MoeArgs m, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
+  constexpr int RB = g2_ring_bytes(FMT, 8 * NT, RING);
+  G2Ring rg = g2_ring_init(smem, RB / g2_warps(FMT, 8 * NT));
   __shared__ MoeSel sel;
   MoeArgs ms = m;
   ms.ids = sel.ids; ms.live = sel.live;
-  g2_phase<FMT, NT, MoeStage<G2StagePlanes<FMT, NT>>, MoeGuMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                                    MoeStage<G2StagePlanes<FMT, NT>>{m, sel, {a}}, MoeGuMats<FMT>{ms});
+  g2_phase<FMT, NT, MoeStage<G2StagePlanes<FMT, NT>>, MoeGuMats<FMT>, moe_ntc<NT>(), false, RING>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB,
+                                                                                                 MoeStage<G2StagePlanes<FMT, NT>>{m, sel, {a}}, MoeGuMats<FMT>{ms});
   g2_drain(rg);
 }
 // The down launch's activation slice built in shared memory from the gate|up outputs (T <= 4 rows): wt * silu(g) * u
@@ -168,27 +169,30 @@ template <int FMT> struct MoeStageSilu {
   }
 };
 
-template <int FMT>
+template <int FMT, int RING>
 __global__ void __launch_bounds__(g2_warps(FMT, 8) * 32, 1) k_moe_dn_silu(const GemmArgs a, const MoeArgs m, const float *wt, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8) / g2_warps(FMT, 8));
+  constexpr int RB = g2_ring_bytes(FMT, 8, RING);
+  G2Ring rg = g2_ring_init(smem, RB / g2_warps(FMT, 8));
   __shared__ MoeSel sel;
   MoeArgs ms = m;
   ms.ids = sel.ids; ms.live = sel.live;
-  g2_phase<FMT, 1>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8), MoeStage<MoeStageSilu<FMT>>{m, sel, {m, wt}}, MoeDnMats<FMT>{ms});
+  g2_phase<FMT, 1, MoeStage<MoeStageSilu<FMT>>, MoeDnMats<FMT>, 1, false, RING>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, MoeStage<MoeStageSilu<FMT>>{m, sel, {m, wt}},
+                                                                               MoeDnMats<FMT>{ms});
   g2_drain(rg);
 }
 
-template <int FMT, int NT>
+template <int FMT, int NT, int RING>
 __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_moe_dn(const GemmArgs a, const MoeArgs m, const int cps) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
-  G2Ring rg = g2_ring_init(smem, g2_ring_bytes(FMT, 8 * NT) / g2_warps(FMT, 8 * NT));
+  constexpr int RB = g2_ring_bytes(FMT, 8 * NT, RING);
+  G2Ring rg = g2_ring_init(smem, RB / g2_warps(FMT, 8 * NT));
   __shared__ MoeSel sel;
   MoeArgs ms = m;
   ms.ids = sel.ids; ms.live = sel.live;
-  g2_phase<FMT, NT, MoeStage<G2StagePlanes<FMT, NT>>, MoeDnMats<FMT>, moe_ntc<NT>()>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + g2_ring_bytes(FMT, 8 * NT),
-                                                                                    MoeStage<G2StagePlanes<FMT, NT>>{m, sel, {a}}, MoeDnMats<FMT>{ms});
+  g2_phase<FMT, NT, MoeStage<G2StagePlanes<FMT, NT>>, MoeDnMats<FMT>, moe_ntc<NT>(), false, RING>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB,
+                                                                                                 MoeStage<G2StagePlanes<FMT, NT>>{m, sel, {a}}, MoeDnMats<FMT>{ms});
   g2_drain(rg);
 }
