@@ -611,7 +611,8 @@ static int enq_ffn(llb_spec *m, const FfnW &w, const float *xin, float *x1, cons
   cudaStream_t s = g_llb.stream;
   if (w.moe) return enq_moe_ffn(m, w, xin, x1, rs);
   PK("norm post", op_norm_xp(s, xin, in_a(m), w.post, m->eps, m->d, x1, m->xp_d, 0, nullptr, rs, m->Tmax, 0));
-  if (w.gate.fmt == w.up.fmt && gemm_ffn_fusable(w.gate.fmt, w.down.fmt, m->NC, m->d) && m->tp.size <= 1) {
+  int ks2 = 1;
+  if (w.gate.fmt == w.up.fmt && m->tp.size <= 1 && gemm_ffn_fusable(w.gate.fmt, w.down.fmt, m->NC, m->d, m->f, &ks2)) {
     // one launch: gate|up in one K-slice, a grid barrier, silu(gate) * up built in shared memory, down
     GemmArgs a1, a2;
     memset(&a1, 0, sizeof a1); memset(&a2, 0, sizeof a2);
@@ -619,7 +620,6 @@ static int enq_ffn(llb_spec *m, const FfnW &w, const float *xin, float *x1, cons
     CK(out_prepare(m, m->b_g, w.gate.rows, 1)); CK(out_prepare(m, m->b_u, w.up.rows, 1));
     a1.m[0].W = w.gate.w; a1.m[0].rows = w.gate.rows; a1.m[0].out = m->b_g.p; a1.m[0].ostride = w.gate.rows; a1.m[0].split_stride = m->b_g.stride;
     a1.m[1].W = w.up.w; a1.m[1].rows = w.up.rows; a1.m[1].out = m->b_u.p; a1.m[1].ostride = w.up.rows; a1.m[1].split_stride = m->b_u.stride;
-    const int ks2 = gemm_fix_ksplit(w.down.fmt, m->NC, m->f / 256, gemm_pick_ksplit(w.down.fmt, m->NC, (w.down.rows + 15) / 16, m->f / 256, g_llb.sms));
     a2.K = m->f; a2.xp = m->xp_f; a2.planes = 2; a2.T = m->Tmax; a2.nmat = 1; a2.ksplit = ks2;
     CK(out_prepare(m, m->b_dn, w.down.rows, ks2));
     a2.m[0].W = w.down.w; a2.m[0].rows = w.down.rows; a2.m[0].out = m->b_dn.p; a2.m[0].ostride = w.down.rows; a2.m[0].split_stride = m->b_dn.stride;

@@ -15,6 +15,10 @@
 #include "gemm2.cuh"
 
 #define FFN_SYNC_LIMIT (1u << 22)
+// The short rings of both phases (g2_stages): gate|up has one K-slice, all d columns, and d = 5120 does not fit beside the usual
+// one.  The widest of them is the gate|up phase's.
+constexpr int FFN_RING = g2_ring_bytes(LLB_FM_Q4_K, 8, 1);
+static_assert(g2_ring_bytes(LLB_FM_Q5_K, 8, 1) <= FFN_RING && g2_ring_bytes(LLB_FM_Q6_K, 8, 1) <= FFN_RING, "one ring for both phases");
 
 __device__ __forceinline__ void ffn_grid_sync(unsigned int *sync, unsigned int nblocks, unsigned int *err, unsigned int limit = FFN_SYNC_LIMIT) {
   __threadfence();   // this thread's gate|up outputs, before the CTA says it is done
@@ -110,12 +114,12 @@ template <int FMT2>
 __global__ void __launch_bounds__(G2_MAXWARPS * 32, 1) k_ffn(const GemmArgs a1, const GemmArgs a2, const int cps1, const int cps2, unsigned int *sync,
                                                        unsigned int *err) {
   extern __shared__ __align__(128) uint8_t smem[];
-  constexpr int RB1 = g2_ring_bytes(LLB_FM_Q4_K, 8), RB2 = g2_ring_bytes(FMT2, 8), RB = RB1 > RB2 ? RB1 : RB2;
   pdl_trigger();
-  G2Ring rg = g2_ring_init(smem, RB / G2_MAXWARPS);
-  g2_phase<LLB_FM_Q4_K, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K>{a1});
+  G2Ring rg = g2_ring_init(smem, FFN_RING / G2_MAXWARPS);
+  g2_phase<LLB_FM_Q4_K, 1, G2StagePlanes<LLB_FM_Q4_K, 1>, G2MatsPlain<LLB_FM_Q4_K>, 1, false, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + FFN_RING,
+                                                                                                G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K>{a1});
   __syncthreads();   // the CTA is done with the first launch's planes
-  g2_phase<FMT2, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err},
-                    G2MatsPlain<FMT2>{a2});
+  g2_phase<FMT2, 1, FfnStageSilu<FMT2>, G2MatsPlain<FMT2>, 1, false, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + FFN_RING,
+                                                                       FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err}, G2MatsPlain<FMT2>{a2});
   g2_drain(rg);
 }

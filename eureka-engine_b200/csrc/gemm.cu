@@ -195,7 +195,7 @@ int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int s
 }
 
 // fills nsb and the tile table of a launch and checks its shape
-static int gemm_prepare(int fmt, GemmArgs &a) {
+static int gemm_prepare(int fmt, GemmArgs &a, bool fused = false) {
   if (a.nmat < 1 || a.nmat > GEMM_MAXMAT) return llb_fail("gemm: nmat %d", a.nmat);
   if (a.K % 256) return llb_fail("gemm: K %d is not a multiple of 256", a.K);
   if (a.xp.NC != 8 && a.xp.NC != 16 && a.xp.NC != 32) return llb_fail("gemm: NC %d", a.xp.NC);
@@ -205,11 +205,16 @@ static int gemm_prepare(int fmt, GemmArgs &a) {
   a.tile0[0] = 0;
   for (int i = 0; i < a.nmat; i++) a.tile0[i + 1] = a.tile0[i] + (a.m[i].rows + 15) / 16;
   for (int i = a.nmat; i < GEMM_MAXMAT; i++) a.tile0[i + 1] = a.tile0[a.nmat];
-  if (a.ksplit != gemm_fix_ksplit(fmt, a.xp.NC, a.nsb, a.ksplit)) return llb_fail("gemm: ksplit %d is not valid for this shape", a.ksplit);
+  if (!fused && a.ksplit != gemm_fix_ksplit(fmt, a.xp.NC, a.nsb, a.ksplit)) return llb_fail("gemm: ksplit %d is not valid for this shape", a.ksplit);
   return 0;
 }
 
 // ---- the fused FFN launch (ffn_fused.cuh) ------------------------------------------------------
+// shared memory of the launch: the ring, and the larger of gate|up's planes (nsb1 super-blocks) and a down slice's (nsl2)
+static size_t ffn_smem(int fmt2, int nsb1, int nsl2) {
+  const size_t s1 = g2_smem(LLB_FM_Q4_K, nsb1, 8, 1, 1, 1), s2 = g2_smem(fmt2, nsl2, 8, 1, 1, 1) - g2_ring_bytes(fmt2, 8, 1) + FFN_RING;
+  return s1 > s2 ? s1 : s2;
+}
 template <int FMT2> static int launch_ffn(cudaStream_t s, const GemmArgs &a1, const GemmArgs &a2) {
   int cps1 = g_llb.sms, cps2 = g_llb.sms / a2.ksplit;
   if (cps1 > a1.tile0[a1.nmat]) cps1 = a1.tile0[a1.nmat];
@@ -217,24 +222,23 @@ template <int FMT2> static int launch_ffn(cudaStream_t s, const GemmArgs &a1, co
   if (cps2 > a2.tile0[a2.nmat]) cps2 = a2.tile0[a2.nmat];
   const int grid = cps1 > cps2 * a2.ksplit ? cps1 : cps2 * a2.ksplit;
   if (grid > g_llb.sms) return llb_fail("k_ffn: %d CTAs do not fit %d SMs", grid, g_llb.sms);   // the barrier needs them all resident
-  const int nsl2 = (a2.nsb + a2.ksplit - 1) / a2.ksplit;
-  const int rb1 = g2_ring_bytes(LLB_FM_Q4_K, 8), rb2 = g2_ring_bytes(FMT2, 8), rb = rb1 > rb2 ? rb1 : rb2;
-  const size_t s1 = g2_smem(LLB_FM_Q4_K, a1.nsb, 8) - rb1 + rb, s2 = g2_smem(FMT2, nsl2, 8) - rb2 + rb, smem = s1 > s2 ? s1 : s2;
+  const size_t smem = ffn_smem(FMT2, a1.nsb, (a2.nsb + a2.ksplit - 1) / a2.ksplit);
   if (smem > G2_SMEM_MAX) return llb_fail("k_ffn: %zu bytes of shared memory", smem);
   cudaError_t e = llb_launch(k_ffn<FMT2>, dim3(grid), dim3(512), smem, s, a1, a2, cps1, cps2, g_ffn_sync, g_g3_err);
   if (e != cudaSuccess) return llb_fail("k_ffn launch: %s", cudaGetErrorString(e));
   return 0;
 }
-// can the FFN of these formats and widths run as one launch?  (gate|up in one K-slice, T <= 4)
-bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d) {
-  return g_llb.ffn_fused && g_ffn_sync && NC == 8 && fmt_gu == LLB_FM_Q4_K &&
-         (fmt_dn == LLB_FM_Q4_K || fmt_dn == LLB_FM_Q5_K || fmt_dn == LLB_FM_Q6_K) && d % 256 == 0 &&
-         d / 256 <= g2_max_slice_sb(LLB_FM_Q6_K, 8)   /* the widest ring of the two launches */;
+// Can the FFN of these formats and widths run as one launch?  (gate|up in one K-slice, T <= 4.)  ks2: the down phase's K-split
+bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d, int f, int *ks2) {
+  if (!g_llb.ffn_fused || !g_ffn_sync || NC != 8 || fmt_gu != LLB_FM_Q4_K || d % 256 || f % 256) return false;
+  if (fmt_dn != LLB_FM_Q4_K && fmt_dn != LLB_FM_Q5_K && fmt_dn != LLB_FM_Q6_K) return false;
+  *ks2 = gemm_fix_ksplit(fmt_dn, NC, f / 256, gemm_pick_ksplit(fmt_dn, NC, d / 16, f / 256, g_llb.sms));
+  return ffn_smem(fmt_dn, d / 256, (f / 256 + *ks2 - 1) / *ks2) <= G2_SMEM_MAX;
 }
 // a1: gate and up (two matrices, Q4_K, ksplit 1, outputs complete); a2: down in format fmt2 with its own K-split
 int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2) {
   if (a1.nmat != 2 || a1.ksplit != 1 || a2.nmat != 1 || a1.xp.NC != 8 || a2.xp.NC != 8) return llb_fail("k_ffn: unsupported launch shape");
-  if (gemm_prepare(LLB_FM_Q4_K, a1) || gemm_prepare(fmt2, a2)) return -1;
+  if (gemm_prepare(LLB_FM_Q4_K, a1, true) || gemm_prepare(fmt2, a2, true)) return -1;
   a1.parts = a2.parts = 1;
   if (a2.K != a1.m[0].rows || a1.m[1].rows != a1.m[0].rows) return llb_fail("k_ffn: down takes %d columns, gate/up have %d/%d rows", a2.K, a1.m[0].rows, a1.m[1].rows);
   if (fmt2 == LLB_FM_Q4_K) return launch_ffn<LLB_FM_Q4_K>(s, a1, a2);

@@ -55,7 +55,7 @@ int gemm_setup(void);
 int gemm_wait_errors(void);
 int gemm_wait_errors_clear(void);
 int gemm_wait_selftest(cudaStream_t s, int which, int limit);
-bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d);
+bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d, int f, int *ks2);
 int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2);   // gate|up (Q4_K, one K-slice), silu, down in one launch
 int gemm_launch_moe(cudaStream_t s, int fmt, bool down, const XPlanes &xp, MoeArgs &m, int *ksplit, const float *wt_silu);   // moe.cuh
 
