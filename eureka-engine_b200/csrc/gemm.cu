@@ -73,9 +73,21 @@ int gemm_wait_errors_clear(void) {
 // The two device-side waits of this file, each made to run out on purpose with a small limit: an mbarrier nobody
 // arrives on (the wait of k_gemm3 and k_pfmm, tc5.cuh) and the fused FFN's grid barrier told to expect one block more
 // than the launch has.  One block, one waiting thread; the wait gives up after `limit` tries, sets the error word
-// exactly as in the real kernels and the kernel returns.
+// exactly as in the real kernels and the kernel returns.  which = 2: the skinny GEMM's ring with a stage that was never
+// requested and two that were.  The wait for the first runs out; the drain must leave nothing in flight, or the word reads 2.
 __global__ void k_wait_selftest(int which, unsigned int limit, unsigned int *sync, unsigned int *err) {
   __shared__ __align__(8) uint64_t bar;
+  if (which == 2) {
+    __shared__ __align__(128) uint8_t mem[G2_BAR_BYTES + 3 * 4096];
+    G2Ring r = g2_ring_init(mem, 3 * 4096);
+    if (threadIdx.x == 0)
+      for (int s = 1; s < 3; s++) { mbar_expect(r.bar_s + 8 * s, 4096); bulk_load(r.ring_s + s * 4096, sync, 4096, r.bar_s + 8 * s); }
+    __syncwarp();
+    for (int s = 0; s < 3; s++) g2_wait(r, s, limit, err);
+    g2_drain(r);
+    if (!r.dead || !mbar_wait(r.bar_s + 8, 0, 1) || !mbar_wait(r.bar_s + 16, 0, 1)) atomicExch(err, 2u);
+    return;
+  }
   if (which == 0) {
     const uint32_t bar_s = smem_u32(&bar);
     if (threadIdx.x == 0) {
@@ -90,10 +102,10 @@ __global__ void k_wait_selftest(int which, unsigned int limit, unsigned int *syn
   }
 }
 int gemm_wait_selftest(cudaStream_t s, int which, int limit) {
-  if (which < 0 || which > 1 || limit < 1 || limit > 100000) return llb_fail("wait selftest: which 0..1, limit 1..100000");
+  if (which < 0 || which > 2 || limit < 1 || limit > 100000) return llb_fail("wait selftest: which 0..2, limit 1..100000");
   unsigned int *sync = nullptr;
-  CU_OK(cudaMalloc(&sync, 8));           // a private pair of counters: the barrier of real launches is not touched
-  CU_OK(cudaMemsetAsync(sync, 0, 8, s));
+  CU_OK(cudaMalloc(&sync, 4096));        // a private pair of counters: the barrier of real launches is not touched; 4 KB to copy from
+  CU_OK(cudaMemsetAsync(sync, 0, 4096, s));
   k_wait_selftest<<<1, 32, 0, s>>>(which, (unsigned int)limit, sync, g_g3_err);
   CU_OK(cudaGetLastError());
   CU_OK(cudaStreamSynchronize(s));

@@ -24,6 +24,7 @@
 #define G2_SMEM_MAX 226304   // 227 KB less the 6 KB that a phase may use beside the ring and the activation slice
 #define G2_MAXWARPS 16
 #define G2_WAIT_LIMIT (1u << 19)   // tries of a bounded wait (up to a microsecond each)
+#define G2_DRAIN_LIMIT (1u << 13)
 #define G2_BAR_BYTES 512     // one mbarrier per warp and stage (at most four)
 
 // XPAD: padding of a plane column in shared memory (column stride = 64 mod 128 bytes for the 16-byte B reads of Q4_K / Q5_K /
@@ -346,9 +347,16 @@ __device__ __forceinline__ G2Ring g2_ring_init(uint8_t *smem, int per_warp) {
   return r;
 }
 
-// After a wait ran out: give what is still in flight its time before the block leaves.
+// The next wait on stage s.  Where one runs out, nothing is requested or waited for after it, and bits 8 .. of par keep the
+// parities as they are then: those of the phases that requests in flight will complete.
+__device__ __forceinline__ void g2_wait(G2Ring &r, int s, uint32_t limit, unsigned int *err) {
+  if (!r.dead && !mbar_wait(r.bar_s + 8 * s, (r.par >> s) & 1u, limit)) { r.dead = true; r.par |= (r.par & 7u) << 8; if (err) atomicExch(err, 1u); }
+  r.par ^= 1u << s;
+}
+// After a wait ran out: what is still in flight lands before the block leaves.  (A stage with no request has nothing to wait for
+// and costs the limit, some milliseconds.)
 __device__ __forceinline__ void g2_drain(const G2Ring &r) {
-  if (r.dead) for (int s = 0; s < 3; s++) mbar_wait(r.bar_s + 8 * s, (r.par >> s) & 1u, G2_WAIT_LIMIT);
+  if (r.dead) for (int s = 0; s < 3; s++) mbar_wait(r.bar_s + 8 * s, (r.par >> (8 + s)) & 1u, G2_DRAIN_LIMIT);
 }
 
 // Where a launch's row tiles live.  A policy says how many 16-row tiles there are, where tile i's 16 x 256 tiles in the
@@ -437,8 +445,7 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
     for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
 #pragma unroll 1
     for (int c = c0; c < c1; c += CH) {
-      if (!rg.dead && !mbar_wait(rg.bar_s + 8 * s, (rg.par >> s) & 1u, G2_WAIT_LIMIT)) { rg.dead = true; if (a.err) atomicExch(a.err, 1u); }
-      rg.par ^= 1u << s;
+      g2_wait(rg, s, G2_WAIT_LIMIT, a.err);
 #pragma unroll 1
       for (int u = 0; u < CH && c + u < c1; u++) g2_tile<FMT, NT, NTC, FOLD>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
       __syncwarp();                                        // every lane has read the stage
