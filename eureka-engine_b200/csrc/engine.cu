@@ -1032,7 +1032,7 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
   for (int v = 0; v < 3; v++) m->xpv[v][5] = m->xpv[v][0];   // placeholder where there are no routed experts
   if (m->ne > 0) {
     const int ns = m->nk + 1;
-    m->moe_lg = falloc(m, (size_t)T * (m->ne + 1)); m->moe_wt = falloc(m, (size_t)T * ns); m->moe_ids = (int *)dalloc(m, (size_t)T * ns * 4); m->moe_live = (int *)dalloc(m, 4 * 64);
+    m->moe_lg = falloc(m, (size_t)T * (m->ne + 1)); m->moe_wt = falloc(m, (size_t)T * ns); m->moe_ids = (int *)dalloc(m, ((size_t)T * ns * 4 + 15) & ~(size_t)15); m->moe_live = (int *)dalloc(m, 4 * 64);
     m->moe_g = falloc(m, (size_t)T * ns * m->ef); m->moe_u = falloc(m, (size_t)T * ns * m->ef); m->hn2 = falloc(m, (size_t)T * d);
     CK(xp_alloc(m, 5, ns * m->ef));
     if (!m->moe_lg || !m->moe_wt || !m->moe_ids || !m->moe_live || !m->moe_g || !m->moe_u || !m->hn2) return -1;

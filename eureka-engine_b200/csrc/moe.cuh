@@ -47,15 +47,19 @@ template <int NTC> __device__ __forceinline__ void moe_col(const float (&acc)[NT
 
 // The router's choice as a launch uses it: the expert ids and the rows in use, copied to shared memory behind the wait.  They are
 // rewritten layer after layer, so they come from L2 (a line of an earlier layer may still be in this SM's L1), once a block:
-// every copy that a warp requests looks its expert up.
+// every copy that a warp requests looks its expert up.  Asynchronous, under the staging of the activations: loads in front of it
+// are one more trip to L2 a launch.
 #define MOE_MAXIDS (16 * 33)   // sixteen rows of 32 experts and the shared one
-struct MoeSel { int live[17], ids[MOE_MAXIDS]; };
+struct __align__(16) MoeSel { int live[20], ids[MOE_MAXIDS]; };
 __device__ __forceinline__ void moe_sel(const MoeArgs &m, MoeSel &s) {
   pdl_wait();
-  for (int i = threadIdx.x; i < 17; i += blockDim.x) s.live[i] = __ldcg(m.live + i);
-  for (int i = threadIdx.x; i < m.T * m.nslot; i += blockDim.x) s.ids[i] = __ldcg(m.ids + i);
+  const int n = (m.T * m.nslot + 3) >> 2;   // (both arrays are allocated in whole sixteen bytes)
+  for (int i = threadIdx.x; i < 5 + n; i += blockDim.x) {
+    if (i < 5) cp_async16(smem_u32(s.live + 4 * i), m.live + 4 * i);
+    else cp_async16(smem_u32(s.ids + 4 * (i - 5)), m.ids + 4 * (i - 5));
+  }
 }
-// a launch's own stage behind that copy (its barrier covers both)
+// a launch's own stage behind those requests: it waits for all of its thread's copies and ends with a barrier
 template <class Base> struct MoeStage {
   const MoeArgs &m;   // the choice in global memory
   MoeSel &s;
@@ -139,7 +143,9 @@ template <int FMT> struct MoeStageSilu {
   const float *wt;   // [T][nslot]
   __device__ __forceinline__ void operator()(uint8_t *xh_s, uint8_t *xsf_s, int CS, int sb0, int nsl) const {
     pdl_wait();
-    const int lane = threadIdx.x & 31, nl = min(__ldcg(m.live), m.T), T = nl > 0 ? __ldcg(m.live + nl) + 1 : 0, f = m.nslot * m.ef;
+    const int4 l0 = __ldcg((const int4 *)m.live);   // the row count and the last row in use, in one trip
+    const int l4 = __ldcg(m.live + 4), nl = min(l0.x, m.T);
+    const int lane = threadIdx.x & 31, T = nl < 1 ? 0 : 1 + (nl == 1 ? l0.y : nl == 2 ? l0.z : nl == 3 ? l0.w : l4), f = m.nslot * m.ef;
     const int ngrp = nsl * 64, ntask = 4 * ngrp;   // (row of the 4 plane pairs, group of four columns); rows >= T are zero planes
     for (int t0 = threadIdx.x; t0 < ntask; t0 += 4 * blockDim.x) {
       float4 gv[4], uv[4];
@@ -165,6 +171,8 @@ template <int FMT> struct MoeStageSilu {
         }
       }
     }
+    cp_async_commit();
+    cp_async_wait<0>();   // the router's choice (moe_sel)
     __syncthreads();
   }
 };

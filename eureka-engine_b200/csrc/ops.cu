@@ -154,17 +154,41 @@ int ops_tile_slice(cudaStream_t s, int fmt, const uint8_t *src, int scols, uint8
 }
 
 // ---- fixed-order sum of K-slice partials --------------------------------------------------------
-__global__ void k_sum_parts(const float *__restrict__ parts, int nsplit, long long stride, int n, float *__restrict__ out) {
+// All slices of a value in one trip to L2 (NS of them; 0: any number, four a trip).  Loads to L2: the GEMM in front wrote the
+// partial sums, and the buffer is used by one call after another.
+template <int NS> __device__ __forceinline__ void sum_parts(const float *parts, int nsplit, long long stride, int n, float *out) {
   pdl_trigger();
   pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float v = __ldcg(parts + i);   // (to L2: the GEMM in front wrote them, and the buffer is used by one call after another)
-  for (int k = 1; k < nsplit; k++) v += __ldcg(parts + (size_t)k * stride + i);
+  const float *p = parts + i;
+  float v;
+  if constexpr (NS > 0) {
+    float l[NS];
+#pragma unroll
+    for (int k = 0; k < NS; k++) l[k] = __ldcg(p + k * stride);
+    v = l[0];
+#pragma unroll
+    for (int k = 1; k < NS; k++) v += l[k];
+  } else {
+    v = __ldcg(p);
+#pragma unroll 4
+    for (int k = 1; k < nsplit; k++) v += __ldcg(p + k * stride);
+  }
   out[i] = v;
 }
+__global__ void k_sum_parts(const float *__restrict__ parts, int nsplit, long long stride, int n, float *__restrict__ out) { sum_parts<0>(parts, nsplit, stride, n, out); }
+template <int NS> __global__ void __launch_bounds__(256) k_sum_slices(const float *__restrict__ parts, long long stride, int n, float *__restrict__ out) {
+  sum_parts<NS>(parts, NS, stride, n, out);
+}
 int ops_sum_parts(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int n, float *out) {
-  CU_OK(llb_launch(k_sum_parts, dim3((n + 255) / 256), dim3(256), (size_t)(0), s, parts, nsplit, split_stride, n, out));
+  const dim3 grid((n + 255) / 256);
+  switch (nsplit) {
+#define SUM_GO(NS) case NS: CU_OK(llb_launch(k_sum_slices<NS>, grid, dim3(256), (size_t)(0), s, parts, split_stride, n, out)); break;
+    SUM_GO(2) SUM_GO(3) SUM_GO(4) SUM_GO(5) SUM_GO(6) SUM_GO(7) SUM_GO(8) SUM_GO(9) SUM_GO(10) SUM_GO(11) SUM_GO(12) SUM_GO(13) SUM_GO(14) SUM_GO(15) SUM_GO(16)
+#undef SUM_GO
+    default: CU_OK(llb_launch(k_sum_parts, grid, dim3(256), (size_t)(0), s, parts, nsplit, split_stride, n, out));
+  }
   CU_OK(cudaGetLastError());
   return 0;
 }
