@@ -118,16 +118,19 @@ int llb_b200_weight_upload(int fmt, int rows, int cols, const void *src, int src
   }
   const uint8_t *s = (const uint8_t *)src;
   void *tmp = nullptr;
-  if (!src_on_device) {
+  // a source on the device that overlaps the destination goes through a copy too (a matrix laid out in place)
+  const bool lap = src_on_device && (uintptr_t)src < (uintptr_t)dst + dev_bytes(fmt, rows, cols) && (uintptr_t)dst < (uintptr_t)src + pb;
+  if (!src_on_device || lap) {
     CU_OK(cudaMalloc(&tmp, pb));
-    const cudaError_t ce = cudaMemcpyAsync(tmp, src, pb, cudaMemcpyHostToDevice, g_llb.stream);
+    const cudaError_t ce = cudaMemcpyAsync(tmp, src, pb, lap ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, g_llb.stream);
     if (ce != cudaSuccess) { cudaFree(tmp); return llb_fail("weight_upload: copy of %zu bytes: %s", pb, cudaGetErrorString(ce)); }
     s = (const uint8_t *)tmp;
   }
   int rc = ops_to_tiles(g_llb.stream, fmt, s, rows, cols, (uint8_t *)(uintptr_t)dst);
   if (tmp) {
-    cudaStreamSynchronize(g_llb.stream);
+    const cudaError_t ce = cudaStreamSynchronize(g_llb.stream);
     cudaFree(tmp);
+    if (!rc && ce != cudaSuccess) rc = llb_fail("weight_upload: %s", cudaGetErrorString(ce));
   }
   return rc;
 }

@@ -168,7 +168,8 @@ __device__ __forceinline__ float deq_elem(int fmt, const uint8_t *W, int cols, i
   const int r = row & 15, i = c & 255;
   const uint8_t *tile = W + ((size_t)(row >> 4) * ((cols + 255) >> 8) + (c >> 8)) * tile_bytes(fmt), *blk = tile + r * tile_row(fmt);
   if (fmt == LLB_FM_Q8_0) {
-    float d = h2f_bits(((const unsigned short *)(blk + 256))[i >> 5]);
+    const uint8_t *s = blk + 256 + 2 * (i >> 5);
+    float d = h2f_bits(s[0] | (s[1] << 8));
     return __fmul_rn((float)((int)blk[i] - 128), d);
   }
   if (fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K) {
@@ -185,7 +186,7 @@ __device__ __forceinline__ float deq_elem(int fmt, const uint8_t *W, int cols, i
     uint8_t lq = blk[64 * hf + 32 * (qd & 1) + l];
     int nib = qd < 2 ? (lq & 15) : (lq >> 4);
     int code = (nib | (((blk[128 + 32 * hf + l] >> (2 * qd)) & 3) << 4)) - 32;
-    float d = h2f_bits(((const unsigned short *)(tile + 3328))[r]);
+    float d = h2f_bits(tile[3328 + 2 * r] | (tile[3329 + 2 * r] << 8));
     float sc = (float)((const int8_t *)(blk + 192))[8 * hf + 2 * qd + (l >> 4)];
     return __fmul_rn(__fmul_rn(d, sc), (float)code);
   }

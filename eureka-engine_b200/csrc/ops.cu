@@ -94,33 +94,38 @@ int ops_repack_q6k(cudaStream_t s, const uint8_t *src210, uint8_t *dst224, size_
 }
 
 // ---- pack rows -> device tiles (common.cuh) ------------------------------------------------------
-// A block per tile; a thread moves two bytes at a time (a stored Q6_K block is only 2-byte aligned).  Runs once per
-// matrix, at load.
-__global__ void __launch_bounds__(256) k_to_tiles(int fmt, const uint8_t *__restrict__ src, int rows, int cols, unsigned short *__restrict__ dst) {
-  const int nsb = (cols + 255) >> 8, tb = tile_bytes(fmt), tr = tile_row(fmt);
-  const size_t prb = pack_row_bytes(fmt, cols);
+// A block per tile; a thread moves two bytes at a time (a stored Q6_K block is only 2-byte aligned), or one where an address is
+// odd.  Bytes past the stored row (columns that are not whole blocks) read as zero.  Runs once per matrix, at load.
+template <typename U>
+__global__ void __launch_bounds__(256) k_to_tiles(int fmt, const uint8_t *__restrict__ src, int rows, int cols, uint8_t *__restrict__ dst) {
+  const int nsb = (cols + 255) >> 8, tb = tile_bytes(fmt), tr = tile_row(fmt), sz = sizeof(U);
+  const size_t prb = pack_row_bytes(fmt, cols), blk = pack_row_bytes(fmt, 256);
   for (size_t tile = blockIdx.x; tile < (size_t)((rows + 15) >> 4) * nsb; tile += gridDim.x) {
     const int row0 = (int)(tile / nsb) * 16, sb = (int)(tile % nsb);
-    for (int i = threadIdx.x; i < tb / 2; i += blockDim.x) {
-      const int o = 2 * i;
+    for (int o = threadIdx.x * sz; o < tb; o += blockDim.x * sz) {
       int r = o / tr, b = o - r * tr;                      // row of the tile, byte of its block
-      if (fmt == LLB_FM_Q6_K && o >= 3328) { r = (o - 3328) >> 1; b = 208; }
-      unsigned short v = 0;
-      const uint8_t *p = src + (size_t)(row0 + r) * prb;
+      if (fmt == LLB_FM_Q6_K && o >= 3328) { r = (o - 3328) >> 1; b = 208 + (o & 1); }
+      const bool codes = fmt == LLB_FM_Q8_0 && b < 256;
+      size_t at = sb * blk + b;                            // byte of the stored row
+      bool in = row0 + r < rows;
       if (fmt == LLB_FM_Q8_0) {
-        if (b < 256) { if (row0 + r < rows && sb * 256 + b < cols) v = *(const unsigned short *)(p + sb * 256 + b); v ^= 0x8080; }
-        else if (row0 + r < rows && sb * 256 + 16 * (b - 256) < cols) v = *(const unsigned short *)(p + cols + sb * 16 + b - 256);
-      } else if (row0 + r < rows) {
-        v = *(const unsigned short *)(p + (size_t)sb * (prb / nsb) + b);
+        at = codes ? (size_t)sb * 256 + b : (size_t)cols + sb * 16 + b - 256;
+        in = in && (codes ? sb * 256 + b : sb * 256 + 16 * ((b - 256) & ~1)) < cols;
       }
-      dst[tile * (tb / 2) + i] = v;
+      U v = 0;
+      if (in && at + sz <= prb) v = *(const U *)(src + (size_t)(row0 + r) * prb + at);
+      if (codes) v ^= (U)0x8080;
+      *(U *)(dst + tile * tb + o) = v;
     }
   }
 }
 int ops_to_tiles(cudaStream_t s, int fmt, const uint8_t *src, int rows, int cols, uint8_t *dst) {
   const size_t n = (size_t)((rows + 15) >> 4) * ((cols + 255) >> 8);
   if (!n) return 0;
-  k_to_tiles<<<(unsigned)(n < 16384 ? n : 16384), 256, 0, s>>>(fmt, src, rows, cols, (unsigned short *)dst);
+  const bool odd = (((uintptr_t)src | (uintptr_t)dst | pack_row_bytes(fmt, cols) | (fmt == LLB_FM_Q8_0 ? cols : 0)) & 1) != 0;
+  const unsigned grid = (unsigned)(n < 16384 ? n : 16384);
+  if (odd) k_to_tiles<uint8_t><<<grid, 256, 0, s>>>(fmt, src, rows, cols, dst);
+  else k_to_tiles<unsigned short><<<grid, 256, 0, s>>>(fmt, src, rows, cols, dst);
   CU_OK(cudaGetLastError());
   return 0;
 }
