@@ -45,7 +45,7 @@ int llb_b200_init(int device) {
   cudaStream_t st = nullptr;
   CU_OK(cudaStreamCreate(&st));
   g_llb.device = device; g_llb.stream = st;
-  if (gemm_setup()) { cudaStreamDestroy(st); g_llb.stream = nullptr; g_llb.device = -1; return -1; }
+  if (gemm_setup() || ops_setup()) { cudaStreamDestroy(st); g_llb.stream = nullptr; g_llb.device = -1; return -1; }
   return 0;
 }
 const char *llb_b200_last_error(void) { return g_llb.err; }

@@ -93,6 +93,24 @@ int ops_repack_q6k(cudaStream_t s, const uint8_t *src210, uint8_t *dst224, size_
   return 0;
 }
 
+// A GEMM's first weight copies do not wait for the kernel in front of it (programmatic launch), so weights that a kernel has
+// just written need something between the two that is no kernel: what comes behind it starts when it is done.
+static unsigned int *g_fence = nullptr;
+int ops_setup(void) {
+  if (!g_fence) CU_OK(cudaMalloc(&g_fence, 4));
+  return 0;
+}
+static bool g_fence_held = false;
+static int ops_fence(cudaStream_t s) {
+  if (!g_fence_held) CU_OK(cudaMemsetAsync(g_fence, 0, 4, s));
+  return 0;
+}
+// while a model is loaded: no launch reads weights before the last of them is uploaded, one fence behind all of them is enough
+int ops_fence_hold(bool on) {
+  g_fence_held = on;
+  return on ? 0 : ops_fence(g_llb.stream);
+}
+
 // ---- pack rows -> device tiles (common.cuh) ------------------------------------------------------
 // A block per tile; a thread moves two bytes at a time (a stored Q6_K block is only 2-byte aligned), or one where an address is
 // odd.  Bytes past the stored row (columns that are not whole blocks) read as zero.  Runs once per matrix, at load.
@@ -127,7 +145,7 @@ int ops_to_tiles(cudaStream_t s, int fmt, const uint8_t *src, int rows, int cols
   if (odd) k_to_tiles<uint8_t><<<grid, 256, 0, s>>>(fmt, src, rows, cols, dst);
   else k_to_tiles<unsigned short><<<grid, 256, 0, s>>>(fmt, src, rows, cols, dst);
   CU_OK(cudaGetLastError());
-  return 0;
+  return ops_fence(s);
 }
 // A range of rows and columns of one tiled matrix into another (a tensor-parallel rank's share): `n` rows from srow to
 // drow, `nc` columns from scol to dcol, in blocks of 256 columns (Q8_0: 32).  Called at load only.
@@ -155,7 +173,7 @@ int ops_tile_slice(cudaStream_t s, int fmt, const uint8_t *src, int scols, uint8
   if (n < 1 || nc < 1) return 0;
   k_tile_slice<<<n, 128, 0, s>>>(fmt, src, scols, dst, dcols, srow, drow, scol, dcol, nc);
   CU_OK(cudaGetLastError());
-  return 0;
+  return ops_fence(s);
 }
 
 // ---- fixed-order sum of K-slice partials --------------------------------------------------------

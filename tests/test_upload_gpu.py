@@ -54,3 +54,26 @@ def test_columns_past_the_last_whole_block(llb, packs, dev, ty, cols, whole, on_
     got = _deq(llb, packs, dev, ty, rows, cols, w.ptr)
     assert np.array_equal(got[:, :whole], packs.dequant(ty, raw, rows, whole).numpy().view(np.uint32))
     assert not np.any(got[:, whole:] & 0x7fffffff)
+
+
+@pytest.mark.parametrize("ty", FMTS)
+def test_a_gemm_behind_an_upload_sees_it(llb, packs, dev, ty):
+    """Uploads and GEMMs in turn with no synchronisation between them: a GEMM's first weight copies start before the kernels
+    in front of it are done, but not before the upload is."""
+    rows, cols, T, n, L, fmt = 4096, 2048, 4, 12, llb.lib(), packs.FMT[ty]
+    rng = np.random.default_rng(8)
+    base = _raw(packs, ty, rows, cols)
+    srcs = [base, torch.flip(base, [0]).contiguous()]        # the same rows the other way round
+    x = rng.standard_normal((T, cols), dtype=np.float32)
+    w, xd = dev(L.llb_b200_weight_bytes(fmt, rows, cols)), dev(x.nbytes).write(x)
+    dsrc, outs = [dev(s.numel()).write(s.numpy()) for s in srcs], [dev(T * rows * 4) for _ in range(n)]
+    xp = llb.handle(L.llb_b200_xp_new(cols, T, 2), "xp_new")
+    llb.check(L.llb_b200_xp_set_f32(xp, xd.ptr), "xp_set")
+    for i in range(n):
+        llb.check(L.llb_b200_weight_upload(fmt, rows, cols, dsrc[i & 1].ptr, 1, w.ptr), "weight_upload")
+        llb.gemm(fmt, [w.ptr], [rows], [outs[i].ptr], cols, xp)
+    got = [o.read((T, rows), np.float32) for o in outs]
+    L.llb_b200_xp_free(xp)
+    for i in range(n):
+        assert np.array_equal(got[i], got[i & 1])
+    assert np.array_equal(got[0], got[1][:, ::-1])
