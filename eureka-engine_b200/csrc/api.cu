@@ -19,6 +19,43 @@ struct llb_xp {
 static float *g_parts = nullptr;
 static size_t g_parts_floats = 0;
 
+// Host memory to tiles through a staging buffer on the device, whole row tiles at a time.  An engine that loads a model keeps one
+// buffer from its first tensor to its last (upload_hold): with an allocation a call, a model with routed experts, three thousand
+// uploads in four layers, took 0.80 s to open from host memory; 0.33 s so.
+#define UPLOAD_STAGE ((size_t)32 << 20)
+static uint8_t *g_stage = nullptr;
+static int g_stage_holds = 0;
+void upload_hold(bool from_host) {
+  if (g_stage_holds++) return;
+  ops_fence_hold(true);
+  if (from_host && cudaMalloc(&g_stage, UPLOAD_STAGE) != cudaSuccess) { g_stage = nullptr; cudaGetLastError(); }
+}
+int upload_release(void) {
+  if (--g_stage_holds) return 0;
+  if (g_stage) { cudaFree(g_stage); g_stage = nullptr; }
+  return ops_fence_hold(false);
+}
+static int upload_host(int fmt, int rows, int cols, const uint8_t *src, uint8_t *dst) {
+  const size_t prb = pack_row_bytes(fmt, cols), all = (size_t)rows * prb;
+  size_t cap = UPLOAD_STAGE;
+  if (cap < 16 * prb) cap = 16 * prb;
+  uint8_t *buf = cap == UPLOAD_STAGE ? g_stage : nullptr;
+  const bool own = !buf;
+  if (own) CU_OK(cudaMalloc(&buf, cap < all ? cap : all));
+  const int step = (int)(cap / prb < (size_t)rows ? cap / prb & ~(size_t)15 : rows);
+  int rc = 0;
+  for (int r0 = 0; r0 < rows && !rc; r0 += step) {   // (the copies and the kernels that read the buffer are in stream order)
+    const int n = rows - r0 < step ? rows - r0 : step;
+    const cudaError_t ce = cudaMemcpyAsync(buf, src + (size_t)r0 * prb, (size_t)n * prb, cudaMemcpyHostToDevice, g_llb.stream);
+    if (ce != cudaSuccess) rc = llb_fail("weight_upload: copy of %zu bytes: %s", (size_t)n * prb, cudaGetErrorString(ce));
+    else rc = ops_to_tiles(g_llb.stream, fmt, buf, n, cols, dst + dev_bytes(fmt, r0, cols));
+  }
+  const cudaError_t ce = cudaStreamSynchronize(g_llb.stream);
+  if (own) cudaFree(buf);
+  if (!rc && ce != cudaSuccess) rc = llb_fail("weight_upload: %s", cudaGetErrorString(ce));
+  return rc;
+}
+
 extern "C" {
 
 int llb_b200_init(int device) {
@@ -120,9 +157,10 @@ int llb_b200_weight_upload(int fmt, int rows, int cols, const void *src, int src
   void *tmp = nullptr;
   // a source on the device that overlaps the destination goes through a copy too (a matrix laid out in place)
   const bool lap = src_on_device && (uintptr_t)src < (uintptr_t)dst + dev_bytes(fmt, rows, cols) && (uintptr_t)dst < (uintptr_t)src + pb;
-  if (!src_on_device || lap) {
+  if (!src_on_device) return upload_host(fmt, rows, cols, s, (uint8_t *)(uintptr_t)dst);
+  if (lap) {
     CU_OK(cudaMalloc(&tmp, pb));
-    const cudaError_t ce = cudaMemcpyAsync(tmp, src, pb, lap ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, g_llb.stream);
+    const cudaError_t ce = cudaMemcpyAsync(tmp, src, pb, cudaMemcpyDeviceToDevice, g_llb.stream);
     if (ce != cudaSuccess) { cudaFree(tmp); return llb_fail("weight_upload: copy of %zu bytes: %s", pb, cudaGetErrorString(ce)); }
     s = (const uint8_t *)tmp;
   }

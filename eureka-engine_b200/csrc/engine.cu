@@ -1288,9 +1288,9 @@ static llb_spec *open_any(const char *index_text, const void *pack, size_t pack_
   if (!index_text || !pack) { llb_fail("llb_spec_open: no index or no pack"); return nullptr; }
   llb_spec *m = new llb_spec();
   m->pack_bytes = pack_bytes;
-  ops_fence_hold(true);
+  upload_hold(!pack_on_device || (mtp && !mtp_on_device));
   const int rc = open_impl(m, index_text, (const uint8_t *)pack, pack_on_device, (const uint8_t *)mtp, mtp_bytes, mtp_on_device, k, max_ctx, layers, tp_n, nstreams);
-  if (ops_fence_hold(false) || rc) {
+  if (upload_release() || rc) {
     llb_spec_close(m);
     return nullptr;
   }

@@ -59,6 +59,10 @@ bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d, int f, int *ks2);
 int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2);   // gate|up (Q4_K, one K-slice), silu, down in one launch
 int gemm_launch_moe(cudaStream_t s, int fmt, bool down, const XPlanes &xp, MoeArgs &m, int *ksplit, const float *wt_silu);   // moe.cuh
 
+// api.cu: from the first to the last of a series of uploads, the staging buffer of those from host memory is kept
+void upload_hold(bool from_host);
+int upload_release(void);
+
 // ops.cu
 int backend_graph_bail(void);   // ends a launch recording in progress by running it (the memory primitives call it first)
 int ops_xp_from_f32(cudaStream_t s, const float *x, int T, int planes, XPlanes xp);

@@ -77,3 +77,17 @@ def test_a_gemm_behind_an_upload_sees_it(llb, packs, dev, ty):
     for i in range(n):
         assert np.array_equal(got[i], got[i & 1])
     assert np.array_equal(got[0], got[1][:, ::-1])
+
+
+@pytest.mark.parametrize("ty,cols", [("Q6_K", 4096), ("Q4_K", 32 * 256)])
+def test_host_uploads_larger_than_the_staging_buffer(llb, packs, dev, ty, cols):
+    """More than 32 MB go through the buffer in whole row tiles; the last piece ends inside one."""
+    L, rows = llb.lib(), (70 << 20) // packs.row_bytes(ty, cols) | 1
+    raw = _raw(packs, ty, 33, cols).repeat(-(-rows // 33), 1)[:rows].contiguous()
+    w = dev(L.llb_b200_weight_bytes(packs.FMT[ty], rows, cols))
+    llb.check(L.llb_b200_weight_upload(packs.FMT[ty], rows, cols, raw.numpy().ctypes.data, 0, w.ptr), "weight_upload")
+    ids = np.array(sorted({0, 1, 15, 16, rows // 3, rows // 2, rows - 17, rows - 1} | set(range(0, rows, 97))), np.int32)
+    d, out = dev(ids.nbytes).write(ids), dev(len(ids) * cols * 4)
+    llb.check(L.llb_b200_dequant(packs.FMT[ty], rows, cols, w.ptr, d.ptr, len(ids), out.ptr), "dequant")
+    ref = packs.dequant(ty, raw[torch.from_numpy(ids).long()].contiguous(), len(ids), cols).numpy()
+    assert np.array_equal(out.read((len(ids), cols), np.float32).view(np.uint32), ref.view(np.uint32))
