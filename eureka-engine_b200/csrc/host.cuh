@@ -68,7 +68,6 @@ int backend_graph_bail(void);   // ends a launch recording in progress by runnin
 int ops_xp_from_f32(cudaStream_t s, const float *x, int T, int planes, XPlanes xp);
 int ops_xp_from_bf16(cudaStream_t s, const void *x, int T, XPlanes xp);
 int ops_dequant_rows(cudaStream_t s, int fmt, const uint8_t *W, int rows, int cols, const int *row_ids, int nrows, float *out);
-int ops_repack_q6k(cudaStream_t s, const uint8_t *src210, uint8_t *dst224, size_t nblocks);
 int ops_setup(void);   // at init
 int ops_fence_hold(bool on);
 int ops_to_tiles(cudaStream_t s, int fmt, const uint8_t *src, int rows, int cols, uint8_t *dst);

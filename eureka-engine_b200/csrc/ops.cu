@@ -72,27 +72,6 @@ int ops_dequant_rows(cudaStream_t s, int fmt, const uint8_t *W, int rows, int co
   return 0;
 }
 
-// ---- Q6_K: 210-byte stored super-blocks -> 224-byte device super-blocks ------------------------
-__global__ void k_repack_q6k(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, size_t nblocks) {
-  pdl_trigger();
-  pdl_wait();
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t n = nblocks * 224;
-  for (; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    size_t b = i / 224;
-    int o = (int)(i - b * 224);
-    dst[i] = o < 210 ? src[b * 210 + o] : 0;
-  }
-}
-int ops_repack_q6k(cudaStream_t s, const uint8_t *src210, uint8_t *dst224, size_t nblocks) {
-  if (!nblocks) return 0;
-  size_t n = nblocks * 224;
-  int grid = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-  CU_OK(llb_launch(k_repack_q6k, dim3(grid), dim3(256), (size_t)(0), s, src210, dst224, nblocks));
-  CU_OK(cudaGetLastError());
-  return 0;
-}
-
 // A GEMM's first weight copies do not wait for the kernel in front of it (programmatic launch), so weights that a kernel has
 // just written need something between the two that is no kernel: what comes behind it starts when it is done.
 static unsigned int *g_fence = nullptr;
@@ -230,8 +209,8 @@ struct llb_b200_kernel { const char *name; const void *fn; int nparams; };
 static const llb_b200_kernel g_kernels[] = {
     {"llb_b200_k_dequant_rows", (const void *)k_dequant_rows, 5},   // (int fmt, const u8 *W, int cols, const int *row_ids, float *out), grid (x, rows)
     {"llb_b200_k_sum_parts", (const void *)k_sum_parts, 5},         // (const float *parts, int nsplit, long long stride, int n, float *out)
-    {"llb_b200_k_repack_q6k", (const void *)k_repack_q6k, 3},       // (const u8 *src210, u8 *dst224, size_t nblocks)
-    {"llb_b200_k_xp_from_f32", (const void *)k_xp_from_f32, 4},     // (const float *x, int K, int planes, XPlanes xp), grid (K / 256, T)
+    {"llb_b200_k_to_tiles", (const void *)k_to_tiles<uint8_t>, 5},  // (int fmt, const u8 *pack rows, int rows, int cols, u8 *device layout), any grid x
+    {"llb_b200_k_xp_from_f32", (const void *)k_xp_from_f32, 4},     // (const float *x, int K, int planes, XPlanes xp), grid ((K + 1023) / 1024, T)
 };
 
 #define GRAPH_SLOTS 16      // cached kernel sequences (LLB_GSLOT of the reference)
@@ -282,7 +261,7 @@ __attribute__((visibility("default"))) int llb_b200_launch(const llb_b200_kernel
   }
   const cudaError_t e = cudaLaunchKernel(k->fn, dim3(gx, gy, 1), dim3(bx, 1, 1), args, sm, g_llb.stream);
   if (e != cudaSuccess) return llb_fail("launch of %s: %s", k->name, cudaGetErrorString(e));
-  return 0;
+  return k->fn == (const void *)k_to_tiles<uint8_t> ? ops_fence(g_llb.stream) : 0;
 }
 
 __attribute__((visibility("default"))) int llb_b200_graph_begin(void) {

@@ -55,8 +55,8 @@ LLB_API llb_b200_dptr llb_b200_stream(void);                  /* the cudaStream_
  * name are the library's leaves with plain argument lists:
  *   llb_b200_k_dequant_rows (int fmt, W, int cols, const int *row_ids or 0, float *out)     grid (<= 64, rows), block 256
  *   llb_b200_k_sum_parts    (const float *parts, int nsplit, long long stride, int n, float *out)   grid ((n + 255) / 256, 1), block 256
- *   llb_b200_k_repack_q6k   (src 210-byte blocks, dst 224-byte blocks, size_t nblocks)
- *   llb_b200_k_xp_from_f32  (const float *x, int K, int planes, planes descriptor by value)
+ *   llb_b200_k_to_tiles     (int fmt, pack rows, int rows, int cols, W in the device layout)        grid (tiles or fewer, 1), block 256
+ *   llb_b200_k_xp_from_f32  (const float *x, int K, int planes, planes descriptor by value)         grid ((K + 1023) / 1024, T), block 256
  * Any other name -- the reference's kernel names included, whose argument lists carry its two-plane int8
  * activations -- returns NULL; a launch with a NULL kernel or a wrong argument count returns -1 and queues nothing. */
 typedef struct llb_b200_kernel llb_b200_kernel;
