@@ -145,6 +145,9 @@ struct llb_spec {
   double pf_rows = 0;     // prompt rows the dense path has processed since the engine was opened
   // graphs
   cudaGraphExec_t g_spec = nullptr, g_prefill = nullptr, g_verify = nullptr;
+  // where the logits of a captured pass lie: K-slices, their stride, a stream's rows (the head's split follows the pass's width)
+  struct LogitsAt { int ns = 1; long long stride = 0; int per = 1; } lg_at[3];
+  int last_pass = 0;   // 0 the speculative cycle, 1 a prompt chunk, 2 the verify pass
   size_t n_spec_nodes = 0, n_verify_nodes = 0;
   std::vector<SeqHost> sq;   // one per stream
   // sampling-mode verify (sampler.cu): off while the parameters leave the argmax untouched
@@ -738,10 +741,17 @@ static int capture(llb_spec *m, int which, cudaGraphExec_t *out, size_t *nodes) 
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (rc) { if (g) cudaGraphDestroy(g); return -1; }
   if (e != cudaSuccess) return llb_fail("graph capture: %s", cudaGetErrorString(e));
+  m->lg_at[which] = {m->b_lg.ns, m->b_lg.stride, m->per};
   if (nodes) cudaGraphGetNodes(g, nullptr, nodes);
   e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return llb_fail("graph instantiate: %s", cudaGetErrorString(e));
+  return 0;
+}
+
+static int launch_pass(llb_spec *m, int which) {
+  CU_OK(cudaGraphLaunch(which == 0 ? m->g_spec : which == 1 ? m->g_prefill : m->g_verify, g_llb.stream));
+  m->last_pass = which;
   return 0;
 }
 
@@ -1490,7 +1500,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
       CU_OK(cudaMemcpyAsync(&ctl_of(m, b)->forced, tail, sizeof tail, cudaMemcpyHostToDevice, g_llb.stream));
     }
     if (!live) break;
-    CU_OK(cudaGraphLaunch(m->g_prefill, g_llb.stream));
+    CK(launch_pass(m, 1));
     for (int i = 0; i < nb; i++) {
       if (!rows_of[i]) continue;
       SpecResult r;
@@ -1500,7 +1510,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
       if (p[i] >= ns[i] - 1 && live > 1) CK(park(bs[i]));   // through, while others still have rows to feed
     }
   }
-  if (m->B > 1 && m->has_mtp)   // the rows that the first speculative cycle's drafter catches up over, where that cycle looks for them
+  if (m->B > 1)   // the rows that the first speculative cycle's drafter catches up over, where that cycle (and read_state) looks for them
     for (int i = 0; i < nb; i++)
       CU_OK(cudaMemcpyAsync(m->hn + (size_t)bs[i] * m->Tspec * m->d, m->hn_pf + (size_t)bs[i] * m->Tpf * m->d, (size_t)m->Tspec * m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
   for (int o = 0; o < m->B; o++) if (kept[o]) CK(ctl_write(m, o, keep[o]));
@@ -1536,7 +1546,7 @@ LLB_API int llb_spec_cycle(llb_spec *m, int *ids_out, int *n_out, uint32_t *top2
   // every row of the cycle, and the drafter's chained rows, must fit: no clipped cycles
   if (q.pos + m->Tmax >= m->max_ctx) return llb_fail("context of %d positions is full", m->max_ctx);
   if (m->tp.size > 1) CK(tp_host_barrier());
-  CU_OK(cudaGraphLaunch(m->g_spec, g_llb.stream));
+  CK(launch_pass(m, 0));
   SpecResult r;
   CK(wait_result(m, 0, &r));
   if (r.p0 != q.pos) return llb_fail("cycle ran at position %d, host expected %d", r.p0, q.pos);
@@ -1561,7 +1571,7 @@ LLB_API int llb_spec_cycle_streams(llb_spec *m, int *ids_out, int *n_out, uint32
     live++;
   }
   if (!live) return llb_fail("llb_spec_cycle_streams: no stream has a prompt");
-  CU_OK(cudaGraphLaunch(m->g_spec, g_llb.stream));
+  CK(launch_pass(m, 0));
   for (int b = 0; b < m->B; b++) {
     n_out[b] = 0;
     SeqHost &q = m->sq[b];
@@ -1587,7 +1597,7 @@ LLB_API int llb_spec_run_cycles_streams(llb_spec *m, int n, int *tokens) {
     const SeqHost &q = m->sq[b];
     if (q.primed && q.pos + n * m->per >= m->max_ctx) return llb_fail("stream %d: context of %d positions cannot take %d more cycles", b, m->max_ctx, n);
   }
-  for (int i = 0; i < n; i++) CU_OK(cudaGraphLaunch(m->g_spec, g_llb.stream));
+  for (int i = 0; i < n; i++) CK(launch_pass(m, 0));
   for (int i = 0; i < n; i++)
     for (int b = 0; b < m->B; b++) {
       SeqHost &q = m->sq[b];
@@ -1654,7 +1664,7 @@ LLB_API int llb_spec_run_cycles(llb_spec *m, int n, int *ids, int cap) {
   if (n > m->res_n) return llb_fail("at most %d cycles per call", m->res_n);
   if (q.pos + n * m->Tmax >= m->max_ctx) return llb_fail("context of %d positions cannot take %d more cycles", m->max_ctx, n);
   if (m->tp.size > 1) CK(tp_host_barrier());
-  for (int i = 0; i < n; i++) CU_OK(cudaGraphLaunch(m->g_spec, g_llb.stream));
+  for (int i = 0; i < n; i++) CK(launch_pass(m, 0));
   int total = 0;
   for (int i = 0; i < n; i++) {
     SpecResult r;
@@ -1672,9 +1682,9 @@ LLB_API int llb_spec_time_verify(llb_spec *m, int iters, float *ms_per_pass) {
   if (m->tp.size > 1) CK(tp_host_barrier());
   cudaEvent_t a, b;
   CU_OK(cudaEventCreate(&a)); CU_OK(cudaEventCreate(&b));
-  CU_OK(cudaGraphLaunch(m->g_verify, g_llb.stream));
+  CK(launch_pass(m, 2));
   CU_OK(cudaEventRecord(a, g_llb.stream));
-  for (int i = 0; i < iters; i++) CU_OK(cudaGraphLaunch(m->g_verify, g_llb.stream));
+  for (int i = 0; i < iters; i++) CK(launch_pass(m, 2));
   CU_OK(cudaEventRecord(b, g_llb.stream));
   CU_OK(cudaEventSynchronize(b));
   float ms = 0;
@@ -1738,6 +1748,7 @@ LLB_API int llb_spec_profile_verify(llb_spec *m, char *buf, int cap) {
     prof_mark("start");
     StreamScope scope(m);
     int rc = enq_verify(m, m->hn);
+    m->last_pass = 2;
     g_prof_on = false;
     if (rc) return -1;
     CU_OK(cudaStreamSynchronize(g_llb.stream));
@@ -1911,9 +1922,12 @@ LLB_API int llb_spec_read_logits(llb_spec *m, int r, float *out) {
   if (r < 0 || r >= m->Tmax || !m->b_lg.p) return llb_fail("read_logits: row %d of a pass of %d rows", r, m->Tmax);
   CU_OK(cudaStreamSynchronize(g_llb.stream));
   std::vector<float> tmp(m->V);
+  // several streams: row r is row r % (k + 1) of stream r / (k + 1), whatever the pass's width was
+  const auto &at = m->lg_at[m->last_pass];
+  const size_t row = m->B > 1 ? (size_t)(r / m->Tspec) * at.per + r % m->Tspec : (size_t)r;
   for (int i = 0; i < m->V; i++) out[i] = 0.0f;
-  for (int k = 0; k < m->b_lg.ns; k++) {
-    CU_OK(cudaMemcpy(tmp.data(), m->b_lg.p + (size_t)k * m->b_lg.stride + (size_t)r * m->V, (size_t)m->V * 4, cudaMemcpyDeviceToHost));
+  for (int k = 0; k < at.ns; k++) {
+    CU_OK(cudaMemcpy(tmp.data(), m->b_lg.p + (size_t)k * at.stride + row * m->V, (size_t)m->V * 4, cudaMemcpyDeviceToHost));
     for (int i = 0; i < m->V; i++) out[i] += tmp[i];
   }
   return 0;
