@@ -13,10 +13,10 @@ unsigned int *gemm_err_word(void) { return g_g3_err; }
 // Cost model of a launch, in cycles of one SM.  The work of its tiles is about 45 + 6.3 cycles a plane column and
 // 16 x 256 tile, 65 + for Q5_K with its fifth bits (measured with the copies left out on the 27B shape's gate|up launch at 4, 8 and 16 rows); a warp's own
 // chain, where that is longer, about 1200 cycles a tile (two stages of copies in flight), with 350 for adding up the parts of
-// a row tile that warps share.  nc: plane columns that are multiplied
-static double gemm_stream_cost(int fmt, int warps, int nc, int tiles, int slice, int parts) {
+// a row tile that warps share (each of them where per_tile is the operator's).  nc: plane columns that are multiplied
+static double gemm_stream_cost(int fmt, int warps, int nc, int tiles, int slice, int parts, double per_tile = 1200.0) {
   const int rounds = (tiles * parts + warps - 1) / warps;
-  const double work = (double)tiles * slice * ((fmt == LLB_FM_Q5_K ? 65.0 : 45.0) + 6.3 * nc), chain = rounds * ((slice + parts - 1) / parts * 1200.0 + (parts > 1 ? 350.0 : 0.0));
+  const double work = (double)tiles * slice * ((fmt == LLB_FM_Q5_K ? 65.0 : 45.0) + 6.3 * nc), chain = rounds * ((slice + parts - 1) / parts * per_tile + (per_tile > 1200.0 ? 350.0 * (parts - 1) : parts > 1 ? 350.0 : 0.0));
   return work > chain ? work : chain;
 }
 // Parts of a row tile's K-slice (g2_phase): the power of two with the lowest cost that divides the warps, leaves every part a
@@ -39,7 +39,8 @@ template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
   const size_t smem = g2_smem(FMT, nsl, NC, a.parts, NT, ring);
   if (smem > G2_SMEM_MAX) return llb_fail("k_gemm2: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   const bool fold = (long long)a.tile0[a.nmat] * a.nsb >= G2_FOLD_TILES;
-  cudaError_t e = llb_launch(ring ? k_gemm2<FMT, NT, false, g2_has_short(FMT, 8 * NT)> : fold ? k_gemm2<FMT, NT, g2_folds(FMT, NT), 0> : k_gemm2<FMT, NT, false, 0>,
+  constexpr int RS = g2_small_ring(FMT, 8 * NT);
+  cudaError_t e = llb_launch(ring ? k_gemm2<FMT, NT, false, RS ? RS : g2_has_short(FMT, 8 * NT)> : fold && g2_folds(FMT, NT) ? k_gemm2<FMT, NT, g2_folds(FMT, NT), 0> : k_gemm2<FMT, NT, false, RS>,
                              dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, cps);
   if (e != cudaSuccess) return llb_fail("k_gemm2 launch: %s", cudaGetErrorString(e));
   return 0;
@@ -118,7 +119,8 @@ template <typename K> static int setup_smem(K k) {
   return 0;
 }
 template <int FMT, int NT> static int setup_fmt2() {
-  return setup_smem(k_gemm2<FMT, NT, false, 0>) || setup_smem(k_gemm2<FMT, NT, g2_folds(FMT, NT), 0>) || setup_smem(k_gemm2<FMT, NT, false, g2_has_short(FMT, 8 * NT)>);
+  constexpr int RS = g2_small_ring(FMT, 8 * NT);
+  return setup_smem(k_gemm2<FMT, NT, false, RS>) || setup_smem(k_gemm2<FMT, NT, g2_folds(FMT, NT), 0>) || setup_smem(k_gemm2<FMT, NT, false, RS ? RS : g2_has_short(FMT, 8 * NT)>);
 }
 template <int FMT, int NT> static int setup_moe() {
   constexpr int SH = g2_has_short(FMT, 8 * NT);
@@ -167,10 +169,13 @@ int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks) {
 int gemm_longest_slice(int fmt, int NC) { return g2_longest_slice(fmt, NC); }
 
 // K-slices per row tile: streaming, the staging of the slice, and a charge per slice for the partial sums that the consumer
-// has to add (direct: a launch of its own adds them, 1.5 us).
+// has to add (direct: a launch of its own adds them, 1.5 us).  At 32 plane columns a warp's chain is nearer 3000 cycles a tile
+// (fitted on fifteen shapes, four formats, one to eight slices; with 1200 the operator's choices were 4.5 % off the best of those,
+// now 1 %: Q4_K 8192 x 3072 at sixteen rows 18.0 -> 15.8 us, 5120 x 5120 18.5 -> 15.9).  The operator alone goes by it: a
+// split decides the order of a model's sums, and the passes were timed with the splits they have.
 static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool direct, double stage) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps;
-  const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, NC / 8, tiles, nsb, ks));
+  const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, NC / 8, tiles, nsb, ks), direct && NC >= 32 ? 3000.0 : 1200.0);
   return (stream + stage * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {

@@ -37,9 +37,14 @@
 // (their epilogue needs whole sums), and matrices of more than GEMM_MAXSPLIT of the usual slices.
 __host__ __device__ constexpr int g2_chunk(int fmt, int ring = 0) { return fmt == LLB_FM_Q4_K && !ring ? 2 : 1; }
 __host__ __device__ constexpr int g2_stages(int fmt, int NC, int ring = 0) {
+  if (ring == 2) return 2;
   if (ring) return fmt == LLB_FM_Q4_K ? 3 : NC >= 32 ? 1 : 2;
   return fmt == LLB_FM_Q4_K ? (NC >= 32 ? 1 : 2) : NC >= 32 || fmt == LLB_FM_Q8_0 ? 2 : 3;
 }
+// ring 2: Q4_K at 32 columns with the bytes of ring 0 as two stages of one super-block: a warp with few tiles then has the next one
+// on its way while it multiplies (3072 x 8192 at sixteen rows 21.7 -> 20.3 us).  Large launches have other warps' copies for
+// that and want the larger ones (FOLD).
+__host__ __device__ constexpr int g2_small_ring(int fmt, int NC) { return fmt == LLB_FM_Q4_K && NC >= 32 ? 2 : 0; }
 __host__ __device__ constexpr bool g2_has_short(int fmt, int NC) { return NC < 32 ? fmt == LLB_FM_Q4_K : fmt == LLB_FM_Q6_K; }
 // Warps of a CTA: sixteen (128 registers a thread), fewer where the rings of sixteen would leave the activation slice less than
 // the widths in use need: Q8_0's tiles are twice the size, and 32 plane columns take half of the memory.
