@@ -386,6 +386,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1) k_pfm
       if (lane == 0) mbar_arrive_cluster(t5_map_rank(acc_empty, 0));
     }
   }
+  // after a wait ran out nothing is requested any more, but copies may be on their way into this CTA's ring: they land within
+  // microseconds, and their barriers count others too, so the CTA gives them 64
+  if (*dead) for (int i = 0; i < 64; i++) __nanosleep(1000);
   __syncwarp();
   t5_fence_before();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // no CTA leaves while the other still arrives here or reads its memory
