@@ -125,8 +125,7 @@ struct llb_spec {
   SpecResult *res_host = nullptr, *res_dev = nullptr;
   int res_n = 256;
   // activations
-  float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *beta = nullptr, *decay = nullptr,
-        *logits = nullptr, *t2part = nullptr, *pm = nullptr, *pl = nullptr, *po = nullptr;
+  float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *logits = nullptr, *t2part = nullptr, *pm = nullptr, *pl = nullptr, *po = nullptr;
   // the trunk's normed rows that the drafter pairs with: hn after a speculative pass (stream b's from row b * Tspec), hn_pf after a
   // prompt pass (from row b * Tpf); one buffer where there is one stream
   float *hn_pf = nullptr;
@@ -1026,10 +1025,9 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
   if (!m->hist) return -1;
 
   // activations
-  int big = m->f > m->convd ? m->f : m->convd;
   const int Tc = T > SPEC_MAXT ? T : SPEC_MAXT;
   m->x = falloc(m, (size_t)T * d); m->x1 = falloc(m, (size_t)T * d); m->hn = falloc(m, (size_t)Tc * d); m->hn_pf = B > 1 ? falloc(m, (size_t)Tc * d) : m->hn; m->e = falloc(m, (size_t)T * d);
-  m->qn = falloc(m, (size_t)T * qa); m->y = falloc(m, (size_t)T * big); m->beta = falloc(m, (size_t)T * m->TR); m->decay = falloc(m, (size_t)T * m->TR);
+  m->qn = falloc(m, (size_t)T * qa);
   m->t2part = falloc(m, (size_t)2 * Tc * TOP2_NB * 4);
   m->mt_x = falloc(m, (size_t)T * d); m->mt_hn = falloc(m, (size_t)T * d); m->chain_h = falloc(m, (size_t)T * d);
   m->att_split = g_llb.sms / (m->KV * B);   // one wave of blocks: the kernel takes a whole SM's shared memory

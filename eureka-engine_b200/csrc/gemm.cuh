@@ -63,8 +63,7 @@ struct MoeArgs {
   int ne;               // block ne is the shared expert; ids are clamped to 0..ne
   int ef, d, T;
   const int *live;      // rows of the pass in use: how many, then which, ascending (rows without a token cost nothing)
-  float *g, *u;         // gate|up: [K-slice][T][nslot * ef]
-  long long gu_stride;  // floats between their K-slices (one slice: any)
+  float *g, *u;         // gate|up: [T][nslot * ef]
   float *out;           // k_moe_dn: [ksplit][T][d]
   long long split_stride;
 };

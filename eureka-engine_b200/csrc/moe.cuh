@@ -90,7 +90,7 @@ template <int FMT> struct MoeGuMats {
     moe_col<NT>(acc, t, lane, v0, v1, mine);
     if (!mine) return;
     const int r = (tile - slot * tps) * 16 + g2_row<FMT, false>(lane >> 2);          // rows r and r + 8 of [gate | up]; a tile is all gate or all up
-    float *dst = (r < m.ef ? m.g : m.u) + (size_t)ks * m.gu_stride + (size_t)t * m.nslot * m.ef + (size_t)jx * m.ef + (r < m.ef ? r : r - m.ef);
+    float *dst = (r < m.ef ? m.g : m.u) + (size_t)t * m.nslot * m.ef + (size_t)jx * m.ef + (r < m.ef ? r : r - m.ef);
     dst[0] = v0; dst[8] = v1;
   }
 };
