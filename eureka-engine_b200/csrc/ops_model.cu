@@ -401,8 +401,9 @@ k_delta(float *__restrict__ S, const SpecCtl *__restrict__ ctl, PartIn ring, con
   // history row r is position pos0 - (KC - 1) + r.  Item = (row, four channels); a stream's ring is [K-slice][CONV_RING slots].
   // (Every thread makes one trip at least: the last warp's gates are in it, however few items a short conv kernel leaves.)
   const float *rp = ring.p + (size_t)blockIdx.z * ring.ns * CONV_RING * sh.convd;
+  const int items = KC > 3 ? nr * 72 : max(nr * 72, DL_THREADS);
 #pragma unroll 1
-  for (int i0 = tid; i0 < max(nr * 72, DL_THREADS); i0 += 2 * DL_THREADS) {
+  for (int i0 = tid; i0 < items; i0 += 2 * DL_THREADS) {
     float4 v[2], l[4][2];
     const float *p[2];
 #pragma unroll
