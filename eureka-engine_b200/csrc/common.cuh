@@ -45,9 +45,9 @@ __host__ __device__ inline size_t pack_row_bytes(int fmt, int cols) {
 }
 
 // ---- activation planes -------------------------------------------------------------------------
-// A GEMM reads its T <= 8 activation rows as fp16 "planes": column t (< NH) holds hi = fp16(x),
+// A GEMM reads its T <= 16 activation rows as fp16 "planes": column t (< NH) holds hi = fp16(x),
 // column NH + t holds lo = fp16((x - hi) * 2048), NH = NC / 2, so hi + lo/2048 carries about 22
-// bits of x.  NC is 8 (T <= 4) or 16 (T <= 8).  With planes == 1 all NC columns are independent
+// bits of x.  NC is 8 (T <= 4), 16 (T <= 8) or 32 (T <= 16).  With planes == 1 all NC columns are independent
 // rows (bf16/fp16 inputs that need no second plane).
 //   xh   [NC][K]    fp16, K-index permuted inside every aligned group of 8: stored order
 //                   0 2 1 3 4 6 5 7, which is the order the tensor-core B fragments consume

@@ -1529,7 +1529,7 @@ LLB_API int llb_spec_prefill(llb_spec *m, const int *ids, int n) { return prefil
 // The same for stream b of an engine opened with llb_spec_open_streams; the other streams keep their state.
 LLB_API int llb_spec_prefill_stream(llb_spec *m, int stream, const int *ids, int n) { return prefill_stream(m, stream, ids, n); }
 // Several streams' prompts at once (streams[i] gets ids[i][0 .. n[i]-1]): the prompts' rows share the prompt passes, each
-// stream feeding its own k + 1 rows of a pass; results are those of llb_spec_prefill_stream on each stream in turn.
+// stream feeding its share of a pass's sixteen rows; results are those of llb_spec_prefill_stream on each stream in turn.
 LLB_API int llb_spec_prefill_streams(llb_spec *m, int n_prompts, const int *streams, const int *const *ids, const int *n) {
   if (!m || !streams || !ids || !n) return llb_fail("llb_spec_prefill_streams: null argument");
   return prefill_many(m, n_prompts, streams, ids, n);
@@ -1815,7 +1815,7 @@ LLB_API int llb_spec_position(const llb_spec *m) { return m->sq[0].pos; }
 LLB_API int llb_spec_position_stream(const llb_spec *m, int stream) { return stream >= 0 && stream < m->B ? m->sq[stream].pos : -1; }
 LLB_API int llb_spec_streams(const llb_spec *m) { return m->B; }
 
-// mode 1: prompts go through the dense tcgen05 path in chunks of 128 rows (all but their last k + 1 rows); mode 0: every
+// mode 1: prompts go through the dense tcgen05 path in chunks of 256 rows (all but their last k + 1 rows); mode 0: every
 // row through the T-row pass.  Returns the previous mode.
 LLB_API int llb_spec_set_prefill(llb_spec *m, int mode) {
   const int was = m->prefill_mode;

@@ -9,10 +9,9 @@
 //    min/offset are applied to that partial sum in fp32.  No weight is ever rounded;
 //  * activations are fp16 hi/lo planes (common.cuh), T <= 4 rows fill the n = 8 tile exactly; 8 rows take two
 //    n-tiles, 16 rows four (the rows of several streams verified in one pass);
-//  * every warp streams its own 16-row weight tiles through a private cp.async ring in shared
-//    memory (16-byte coalesced copies of the packed super-blocks, bank-conflict-free row stride),
-//    prefetching across tile boundaries so HBM requests never drain between tiles (the kernel
-//    itself is k_gemm2 in gemm2.cuh; this file holds the arithmetic of a staged chunk and the epilogue);
+//  * every warp streams its own 16 x 256 weight tiles through a private ring of bulk copies in shared memory (a tile is
+//    contiguous, common.cuh), prefetching across row tiles so HBM requests never drain between them (the kernel itself
+//    is k_gemm2 in gemm2.cuh; this file holds what its launches share and the epilogue);
 //  * up to four matrices that share the activations run in one launch (gate|up, q|k|v,
 //    qkv|z|beta|alpha), and K can be split into slices whose partial sums the consumer adds in a
 //    fixed order (deterministic, no atomics).

@@ -29,8 +29,8 @@
 
 // XPAD: padding of a plane column in shared memory (column stride = 64 mod 128 bytes for the 16-byte B reads of Q4_K / Q5_K /
 // Q8_0, 32 mod 128 for the 8-byte ones of Q6_K), AUX: bytes per (super-block, column) of the sub-block means
-// Ring depth: 90 to 160 KB an SM in flight (44 KB cover HBM's latency at full rate), less beside 32 plane columns, whose whole
-// d = 2048 slice must fit.
+// Ring depth: 104 to 161 KB an SM (44 KB in flight cover HBM's latency at full rate), 55 to 104 KB beside 32 plane columns,
+// whose whole d = 2048 slice must fit.
 // Super-blocks a copy brings.  A bulk copy costs about 85 cycles of the SM's copy engine on top of its bytes (copies alone, no
 // arithmetic, gate|up of the 27B shape: 19.6 us at 2304 bytes, 11.8 us at 4608), so Q4_K takes two at a time.
 // ring 1: a shorter ring for K-slices that do not fit beside the usual one (ring 0): one K-slice of wide routed-expert models

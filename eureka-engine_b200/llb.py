@@ -384,7 +384,7 @@ class SpecEngine:
                 "drafted": [int(v) for v in out[3:11]], "accepted": [int(v) for v in out[11:19]]}
 
     def set_prefill(self, fast: bool) -> int:
-        """True: prompts go through the dense tcgen05 path in chunks of 128 rows; returns the previous mode."""
+        """True: prompts go through the dense tcgen05 path in chunks of 256 rows; returns the previous mode."""
         return self.L.llb_spec_set_prefill(self.h, 1 if fast else 0)
 
     def fast_rows(self) -> float:

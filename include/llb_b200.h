@@ -230,7 +230,7 @@ LLB_API llb_spec *llb_spec_open_sibling(llb_spec *first, int k, int max_ctx, int
 LLB_API size_t llb_spec_weight_bytes(const llb_spec *m);
 LLB_API int llb_spec_prefill_stream(llb_spec *m, int stream, const int *ids, int n);
 /* The prompts of several streams at once: streams[i] gets ids[i][0 .. n[i]-1].  The prompts' rows share the prompt passes
- * (every stream feeds its own k + 1 rows of a pass), so n_prompts prompts take about the passes of the longest one; each
+ * (every stream feeds its share of a pass's sixteen rows, k + 1 at least), so n_prompts prompts take about the passes of the longest one; each
  * stream ends in the state llb_spec_prefill_stream would have left it in.  A stream named twice is refused. */
 LLB_API int llb_spec_prefill_streams(llb_spec *m, int n_prompts, const int *streams, const int *const *ids, const int *n);
 /* One cycle of every stream that has a prompt, as one graph launch: ids_out[stream * 8 + i], i < n_out[stream], are that
@@ -270,7 +270,7 @@ LLB_API int llb_spec_pass(llb_spec *m, int pos, int tok, float *y);
 LLB_API int llb_spec_position(const llb_spec *m);
 /* How llb_spec_prefill feeds a prompt.  mode 0 (default): every row through the T-row verify pass, eight rows a pass, at
  * the verify path's precision.  mode 1 (also LLB_PREFILL=fast in the environment at open, the reference's switch,
- * host/llb_host.c:206): all but the last k + 1 rows in chunks of 128 rows through dense tcgen05 GEMMs (operands as two fp16 planes)
+ * host/llb_host.c:206): all but the last k + 1 rows in chunks of 256 rows through dense tcgen05 GEMMs (operands as two fp16 planes)
  * (replaces pf_take / spec_pf / spec_take, host/llb_pf.h:551, host/llb_host.c:1831-1899): trunk K/V, conv history and
  * DeltaNet state, and the drafter's K/V rows, are left as the T-row pass would have left them, within the path's
  * tolerance.  Models with routed experts always take mode 0.  Returns the previous mode.
