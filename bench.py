@@ -34,8 +34,8 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# DRAM bytes one gate|up launch moved under ncu (102.1 MB read + 4.3 MB written; algorithmic 100.9 MB)
-GEMM_DRAM_TRAFFIC = 106.4e6
+# DRAM bytes one gate|up launch moved under ncu (100.4 MB read + 3.6 MB written; algorithmic 100.9 MB)
+GEMM_DRAM_TRAFFIC = 104.0e6
 METRIC = "spec-decode tok/s per B200, 27B-shape Q4_K_M MTP k=3; verify-step HBM GB/s"
 WORKLOAD = "config 2: 27B-shape hybrid (d 5120, 64 layers, f 17408, V 151936), Q4_K_M, batch 1, MTP k=3 greedy, prompt 3011"
 PROMPT, GEN_CAP, K_DRAFT = 3011, 1200, 3
