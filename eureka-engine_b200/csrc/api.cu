@@ -278,7 +278,7 @@ int llb_b200_smp_rows(const llb_smp_params *p, llb_b200_dptr logits, int T, int 
   if (smp_prepare(p, &d, &argmax_only)) return -1;
   if (backend_graph_bail()) return -1;
   void *buf = nullptr;
-  const size_t b_adj = (size_t)T * V * 4, b_win = (size_t)T * SMP_MAX_WIN * 4, b_i = (size_t)T * 4, b_l = (size_t)T * 8;
+  const size_t b_adj = (size_t)T * smp_row_floats(V) * 4, b_win = (size_t)T * SMP_MAX_WIN * 4, b_i = (size_t)T * 4, b_l = (size_t)T * 8;
   CU_OK(cudaMalloc(&buf, b_adj + b_win + 5 * b_i + b_l + 16));
   char *c = (char *)buf;
   float *adj = (float *)c; c += b_adj;

@@ -152,7 +152,7 @@ struct llb_spec {
   // sampling-mode verify (sampler.cu): off while the parameters leave the argmax untouched
   bool smp_on = false;
   SmpDev smp;
-  float *smp_adj = nullptr, *smp_val = nullptr;   // biased / penalised logits of every row; the emitted tokens' raw logits
+  float *smp_adj = nullptr, *smp_val = nullptr;   // every row's biased / penalised logits or its candidates; the emitted tokens' raw logits
   int *smp_tok = nullptr;
   unsigned int *smp_err = nullptr;
 };
@@ -1781,7 +1781,7 @@ LLB_API int llb_spec_set_sampler(llb_spec *m, const llb_smp_params *p) {
   if (m->tp.size > 1 && !argmax_only) return llb_fail("set_sampler: a tensor-parallel engine decodes greedily");
   const int rows = m->B * m->Tspec;
   if (!argmax_only && !m->smp_adj) {
-    m->smp_adj = falloc(m, (size_t)rows * m->V); m->smp_val = falloc(m, rows); m->smp_tok = (int *)dalloc(m, (size_t)rows * 4);
+    m->smp_adj = falloc(m, (size_t)rows * smp_row_floats(m->V)); m->smp_val = falloc(m, rows); m->smp_tok = (int *)dalloc(m, (size_t)rows * 4);
     m->smp_err = (unsigned int *)dalloc(m, 4);
     if (!m->smp_adj || !m->smp_val || !m->smp_tok || !m->smp_err) return -1;
   }

@@ -20,7 +20,8 @@ struct SmpDev {
 };
 
 int smp_prepare(const llb_smp_params *p, SmpDev *d, bool *argmax_only);
-// rows blocks: engine mode takes draft / position / window of every row from the control blocks at ctl (stream geometry
+size_t smp_row_floats(int V);   // floats of adj that a row takes
+// engine mode takes draft / position / window of every row from the control blocks at ctl (stream geometry
 // as set by ops_set_streams); test mode (ctl == null) from t_draft[rows], t_pos[rows], t_win[rows][SMP_MAX_WIN], t_nwin[rows]
 int op_smp_rows(cudaStream_t s, const SmpDev &P, PartIn lg, int V, float *adj, const SpecCtl *ctl, int rows, const int *t_draft, const long long *t_pos,
                 const int *t_win, const int *t_nwin, int *tok_out, float *val_out, int *acc_out, unsigned int *err);

@@ -77,6 +77,31 @@ def test_vocabulary_sized_rows_against_the_oracle(llb, oracle, dev, case):
     assert hits >= T - 1
 
 
+@pytest.mark.parametrize("V", [1, 40, 2047, 2049, 6145, 263001])
+@pytest.mark.parametrize("top_k", [1, 7, 256])
+def test_the_largest_of_rows_with_ties_and_holes(llb, oracle, dev, V, top_k):
+    """Vocabularies around the edges of a chunk of ids and of a batch of candidates, logits on a coarse grid (hundreds of equal ones
+    across every line that a selection draws), banned ids (-inf), biases that name an id twice, a list longer than the row."""
+    from oracle import bindings
+    rng = np.random.default_rng(1000 * top_k + V)
+    T = 4
+    lg = (np.round(rng.standard_normal((T, V)) * 4) / 4).astype(np.float32)
+    lg[1, 1: V - V // 3] = -np.inf
+    lg[2] = 0.0                                             # one tie of the whole row, both signs of zero
+    lg[2, ::2] = -0.0
+    bias = [(int(i), float(b)) for i, b in zip(rng.integers(0, V, 8), rng.integers(-3, 4, 8))] + [(V // 2, 1.0), (V // 2, 0.5)]
+    op = bindings.SmpParams.make(temp=0.7, top_k=top_k, top_p=0.95 if top_k > 1 else 1.0, repeat_penalty=1.1, repeat_last_n=64, seed=5, bias=bias)
+    hists = [rng.integers(0, V, 80).astype(np.int32) for _ in range(T)]
+    drafts = [-1, int(V - 1), int(rng.integers(0, V)), int(np.argmax(lg[3]))]
+    pos = [int(rng.integers(1, 1 << 24)) for _ in range(T)]
+    buf = dev(lg.nbytes).write(lg)
+    tok, acc, val = llb.smp_rows(_dev_params(llb, op), buf.ptr, T, V, drafts, pos, [h[-64:] for h in hists])
+    for r in range(T):
+        t, a, margin = bindings.smp_row(op, lg[r], hists[r], drafts[r], pos[r])
+        assert (tok[r], acc[r]) == (t, a) or margin < 1e-6, (r, int(tok[r]), int(acc[r]), t, a, margin)
+        assert val[r] == lg[r, tok[r]]
+
+
 def test_what_has_no_device_path_is_refused_by_name(llb, dev):
     lg = np.zeros((1, 64), np.float32)
     buf = dev(lg.nbytes).write(lg)
