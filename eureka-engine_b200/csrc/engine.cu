@@ -72,8 +72,8 @@ struct llb_spec {
   float rope_base = 1e7f, eps = 1e-6f;
   int ne = 0, nk = 0, ef = 0, sf = 0;   // routed experts, experts per token, expert width, shared expert width (ne = 0: dense FFN)
   float *moe_lg = nullptr, *moe_wt = nullptr, *moe_g = nullptr, *moe_u = nullptr, *hn2 = nullptr;
-  int *moe_ids = nullptr, *moe_live = nullptr;   // moe_live: how many rows of the pass are in use, then which
-  XPlanes xp_e;
+  int *moe_ids = nullptr;
+  int4 *moe_units = nullptr;   // the pass's (expert, rows) units (moe.cuh)
   size_t pack_bytes = 0;   // size of the pack the index describes: every tensor range is checked against it
   int k = 0, Tmax = 1, R = 2, max_ctx = 0, NC = 8;   // Tmax / NC: rows and plane columns of the pass being enqueued
   // Several streams (sequences) per engine share every weight read: a pass has B x per rows, row t belonging to stream
@@ -85,7 +85,7 @@ struct llb_spec {
   // the weights stream once per pass whatever its rows, so a wider chunk halves the prompt's time).  The two widths
   // share every buffer; the planes have one view per column count.
   int Tspec = 1, Tpf = 1;
-  XPlanes xpv[3][6];   // [NC 8 / 16 / 32][xp_d, xp_f, xp_qa, xp_v, xp_2d, xp_e]
+  XPlanes xpv[3][5];   // [NC 8 / 16 / 32][xp_d, xp_f, xp_qa, xp_v, xp_2d]
   // weights
   std::vector<void *> allocs;
   // An engine opened by llb_spec_open_sibling uses the weights of the engine it names (`share`) and owns only its
@@ -230,7 +230,7 @@ static void set_width(llb_spec *m, int T) {
   m->Tmax = T; m->NC = nc_of(T);
   m->per = T / m->B;
   const XPlanes *v = m->xpv[m->NC == 8 ? 0 : m->NC == 16 ? 1 : 2];
-  m->xp_d = v[0]; m->xp_f = v[1]; m->xp_qa = v[2]; m->xp_v = v[3]; m->xp_2d = v[4]; m->xp_e = v[5];
+  m->xp_d = v[0]; m->xp_f = v[1]; m->xp_qa = v[2]; m->xp_v = v[3]; m->xp_2d = v[4];
 }
 
 static int fmt_of(const std::string &ty) {
@@ -462,7 +462,7 @@ static int load_moe(llb_spec *m, FfnW &w, const std::string &p, const std::unord
 }
 
 // Does a pass of T rows fit the GEMMs' shared memory?  Every matrix of the index in the K-slices it may have: sixteen, those of
-// the conv ring's launch RING_MAXSPLIT, one for the experts' gate and up.
+// the conv ring's launch RING_MAXSPLIT.
 static bool width_fits(const llb_spec *m, const std::unordered_map<std::string, TensorRec> &tab, int T) {
   const int NC = nc_of(T);
   auto fits = [&](int fmt, int nsb, int cap) {
@@ -472,10 +472,8 @@ static bool width_fits(const llb_spec *m, const std::unordered_map<std::string, 
   for (const auto &kv : tab) {
     const TensorRec &t = kv.second;
     const std::string &n = kv.first;
-    if (t.fmt == LLB_FM_F32 || n.find("_shexp") != std::string::npos) continue;   // (the shared expert is a block of the stacks)
-    if (n.find("down_exps") != std::string::npos) { if (!fits(t.fmt, (m->nk + 1) * m->ef / 256, 16)) return false; }
-    else if (n.find("_exps") != std::string::npos) { if (!fits(t.fmt, m->d / 256, 1)) return false; }
-    else if (!fits(t.fmt, (t.cols + 255) / 256, n.find("attn_qkv") != std::string::npos ? RING_MAXSPLIT : 16)) return false;
+    if (t.fmt == LLB_FM_F32 || n.find("_shexp") != std::string::npos || n.find("_exps") != std::string::npos) continue;   // (the experts' launches stage four rows at a time, however many a pass has)
+    if (!fits(t.fmt, (t.cols + 255) / 256, n.find("attn_qkv") != std::string::npos ? RING_MAXSPLIT : 16)) return false;
   }
   return fits(LLB_FM_Q8_0, 2 * m->d / 256, 16);   // a drafter's input projection, whatever its format
 }
@@ -580,9 +578,9 @@ static int enq_attn(llb_spec *m, const AttnW &w, float *Kc, float *Vc, const Row
 }
 
 // x1 = xin + sum(b_a); h = rms(x1) * post -> planes; x1 + down(silu(gate h) * up h) stays split in b_dn
-// The routed-expert FFN: router logits and top k on the normed rows, gate|up of every (row, slot), the slots'
-// weights folded into silu(gate) * up, and one down launch per pass whose accumulation order is the rank order;
-// like the dense FFN it leaves x1 + (its output) as x1 and K-slice partial sums in b_dn.
+// The routed-expert FFN: router logits on the normed rows, top k and gate|up of the chosen experts, and a down launch on silu(gate) *
+// up times the slots' weights; like the dense FFN it leaves x1 + (its output) as x1 and partial sums, here one a slot in rank
+// order, in b_dn.
 static int enq_moe_core(llb_spec *m, const FfnW &w, const RowSet *rs);
 static int enq_moe_ffn(llb_spec *m, const FfnW &w, const float *xin, float *x1, const RowSet *rs) {
   cudaStream_t s = g_llb.stream;
@@ -592,20 +590,18 @@ static int enq_moe_ffn(llb_spec *m, const FfnW &w, const float *xin, float *x1, 
 // ... from the normed rows on: planes in xp_d, the same rows as F32 in hn2
 static int enq_moe_core(llb_spec *m, const FfnW &w, const RowSet *rs) {
   cudaStream_t s = g_llb.stream;
-  const int ns = m->nk + 1, fe = ns * m->ef;
-  PK("moe route", op_moe_route(s, w.router, m->hn2, m->d, m->ne, m->nk, m->moe_lg, m->moe_ids, m->moe_wt, m->moe_live, rs, m->Tmax));
+  PK("moe route", op_moe_logits(s, w.router, m->hn2, m->d, m->ne, m->moe_lg, rs, m->Tmax));
+  const Streams sg = ops_streams();
   MoeArgs a;
   memset(&a, 0, sizeof a);
-  a.ids = m->moe_ids; a.nslot = ns; a.ne = m->ne; a.ef = m->ef; a.d = m->d; a.T = m->Tmax; a.live = m->moe_live;
+  a.nslot = m->nk + 1; a.ne = m->ne; a.ef = m->ef; a.d = m->d; a.T = m->Tmax;
+  a.lg = m->moe_lg; a.rs = rs; a.per = sg.per; a.stride = sg.stride; a.ids = m->moe_ids; a.wt = m->moe_wt; a.units = m->moe_units;
   a.W = w.gu; a.es = w.es_gu; a.g = m->moe_g; a.u = m->moe_u;
-  int one = 1;
-  PK("moe gate|up", gemm_launch_moe(s, w.fmt_gu, false, m->xp_d, a, &one, nullptr));
-  const bool silu_in_down = m->NC == 8;
-  if (!silu_in_down) PK("moe silu", op_silu_scaled_xp(s, PartIn{m->moe_g, 1, 0}, PartIn{m->moe_u, 1, 0}, fe, m->xp_e, rs, m->Tmax, m->moe_wt, m->ef));
-  int ks = gemm_fix_ksplit(w.fmt_dn, m->NC, fe / 256, gemm_pick_ksplit(w.fmt_dn, m->NC, m->Tmax * (m->d / 16), fe / 256, g_llb.sms, false, silu_in_down ? 96.0 : 24.0));
-  CK(out_prepare(m, m->b_dn, m->d, ks));
+  PK("moe gate|up", gemm_launch_moe_gu(s, w.fmt_gu, m->xp_d, a));
+  const int ks = gemm_moe_dn_ksplit(w.fmt_dn, a);
+  CK(out_prepare(m, m->b_dn, m->d, a.nslot * (ks < 1 ? 1 : ks)));
   a.W = w.dn; a.es = w.es_dn; a.out = m->b_dn.p; a.split_stride = m->b_dn.stride;
-  PK("moe down", gemm_launch_moe(s, w.fmt_dn, true, m->xp_e, a, &ks, silu_in_down ? m->moe_wt : nullptr));
+  PK("moe down", gemm_launch_moe_dn(s, w.fmt_dn, a, ks));
   return 0;
 }
 
@@ -1037,13 +1033,11 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
   m->po = falloc(m, (size_t)m->H * T * m->att_split * m->hd);
   CK(xp_alloc(m, 0, d)); CK(xp_alloc(m, 1, m->f)); CK(xp_alloc(m, 2, qa)); CK(xp_alloc(m, 3, m->vdc));
   CK(xp_alloc(m, 4, 2 * d));
-  for (int v = 0; v < 3; v++) m->xpv[v][5] = m->xpv[v][0];   // placeholder where there are no routed experts
   if (m->ne > 0) {
     const int ns = m->nk + 1;
-    m->moe_lg = falloc(m, (size_t)T * (m->ne + 1)); m->moe_wt = falloc(m, (size_t)T * ns); m->moe_ids = (int *)dalloc(m, ((size_t)T * ns * 4 + 15) & ~(size_t)15); m->moe_live = (int *)dalloc(m, 4 * 64);
+    m->moe_lg = falloc(m, (size_t)T * (m->ne + 1)); m->moe_wt = falloc(m, (size_t)T * ns); m->moe_ids = (int *)dalloc(m, (size_t)T * ns * 4); m->moe_units = (int4 *)dalloc(m, (size_t)(T * ns + 1) * sizeof(int4));
     m->moe_g = falloc(m, (size_t)T * ns * m->ef); m->moe_u = falloc(m, (size_t)T * ns * m->ef); m->hn2 = falloc(m, (size_t)T * d);
-    CK(xp_alloc(m, 5, ns * m->ef));
-    if (!m->moe_lg || !m->moe_wt || !m->moe_ids || !m->moe_live || !m->moe_g || !m->moe_u || !m->hn2) return -1;
+    if (!m->moe_lg || !m->moe_wt || !m->moe_ids || !m->moe_units || !m->moe_g || !m->moe_u || !m->hn2) return -1;
   }
   m->ctl = (SpecCtl *)dalloc(m, sizeof(SpecCtl) * B);
   if (!m->x || !m->po || !m->ctl || !m->hn_pf) return -1;

@@ -116,10 +116,10 @@ __global__ void __launch_bounds__(G2_MAXWARPS * 32, 1) k_ffn(const GemmArgs a1, 
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   G2Ring rg = g2_ring_init(smem, FFN_RING / G2_MAXWARPS);
-  g2_phase<LLB_FM_Q4_K, 1, G2StagePlanes<LLB_FM_Q4_K, 1>, G2MatsPlain<LLB_FM_Q4_K>, 1, false, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + FFN_RING,
+  g2_phase<LLB_FM_Q4_K, 1, G2StagePlanes<LLB_FM_Q4_K, 1>, G2MatsPlain<LLB_FM_Q4_K>, false, 1>(a1, cps1, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + FFN_RING,
                                                                                                 G2StagePlanes<LLB_FM_Q4_K, 1>{a1}, G2MatsPlain<LLB_FM_Q4_K>{a1});
   __syncthreads();   // the CTA is done with the first launch's planes
-  g2_phase<FMT2, 1, FfnStageSilu<FMT2>, G2MatsPlain<FMT2>, 1, false, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + FFN_RING,
+  g2_phase<FMT2, 1, FfnStageSilu<FMT2>, G2MatsPlain<FMT2>, false, 1>(a2, cps2, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + FFN_RING,
                                                                        FfnStageSilu<FMT2>{a1.m[0].out, a1.m[1].out, a1.m[0].rows, a1.T, sync, err}, G2MatsPlain<FMT2>{a2});
   g2_drain(rg);
 }

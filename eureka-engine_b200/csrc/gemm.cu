@@ -122,14 +122,8 @@ template <int FMT, int NT> static int setup_fmt2() {
   constexpr int RS = g2_small_ring(FMT, 8 * NT);
   return setup_smem(k_gemm2<FMT, NT, false, RS>) || setup_smem(k_gemm2<FMT, NT, g2_folds(FMT, NT), 0>) || setup_smem(k_gemm2<FMT, NT, false, RS ? RS : g2_has_short(FMT, 8 * NT)>);
 }
-template <int FMT, int NT> static int setup_moe() {
-  constexpr int SH = g2_has_short(FMT, 8 * NT);
-  return setup_smem(k_moe_gu<FMT, NT, 0>) || setup_smem(k_moe_gu<FMT, NT, SH>) || setup_smem(k_moe_dn<FMT, NT, 0>) || setup_smem(k_moe_dn<FMT, NT, SH>);
-}
 template <int FMT> static int setup_fmt() { return setup_fmt2<FMT, 1>() || setup_fmt2<FMT, 2>() || setup_fmt2<FMT, 4>(); }
-template <int FMT> static int setup_experts() {
-  return setup_moe<FMT, 1>() || setup_moe<FMT, 2>() || setup_moe<FMT, 4>() || setup_smem(k_moe_dn_silu<FMT, 0>) || setup_smem(k_moe_dn_silu<FMT, g2_has_short(FMT, 8)>);
-}
+template <int FMT> static int setup_experts() { return setup_smem(k_moe_gu<FMT, 8>) || setup_smem(k_moe_gu<FMT, 32>) || setup_smem(k_moe_dn<FMT>); }
 
 int gemm_setup(void) {
   if (setup_fmt<LLB_FM_Q4_K>() || setup_fmt<LLB_FM_Q5_K>() || setup_fmt<LLB_FM_Q6_K>() || setup_fmt<LLB_FM_Q8_0>()) return -1;
@@ -265,52 +259,73 @@ int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2) {
 }
 
 // ---- the routed experts' GEMMs (moe.cuh) ---------------------------------------------------------
-template <int FMT, int NT> static int launch_moe(cudaStream_t s, bool down, GemmArgs &a, const MoeArgs &m, int ntiles, const float *wt_silu) {
-  const int NC = 8 * NT, nsl = (a.nsb + a.ksplit - 1) / a.ksplit;
-  int cps = g_llb.sms / a.ksplit;
-  if (cps < 1) cps = 1;
-  if (cps > ntiles) cps = ntiles;
-  // from the capacity of the launch, whatever rows are in use: a row's sums do not depend on its neighbours
-  a.parts = gemm_pick_parts(FMT, NC, moe_ntc<NT>(), (ntiles + cps - 1) / cps, a.nsb, a.ksplit);
-  constexpr int SH = g2_has_short(FMT, 8 * NT);
-  const int ring = g2_ring_of(FMT, NC, nsl);
-  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, moe_ntc<NT>(), ring);
-  if (smem > G2_SMEM_MAX) return llb_fail("moe gemm: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
-  cudaError_t e;
-  if (down && wt_silu) {
-    if constexpr (NT == 1) e = llb_launch(ring ? k_moe_dn_silu<FMT, SH> : k_moe_dn_silu<FMT, 0>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, wt_silu, cps);
-    else return llb_fail("moe gemm: the down launch builds its own activations for T <= 4 only");
-  } else {
-    e = down ? llb_launch(ring ? k_moe_dn<FMT, NT, SH> : k_moe_dn<FMT, NT, 0>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps)
-             : llb_launch(ring ? k_moe_gu<FMT, NT, SH> : k_moe_gu<FMT, NT, 0>, dim3(cps * a.ksplit), dim3(g2_warps(FMT, NC) * 32), smem, s, a, m, cps);
-  }
-  if (e != cudaSuccess) return llb_fail("moe gemm launch: %s", cudaGetErrorString(e));
-  return 0;
+// Shape of a launch of `units` units at most (tpu tiles of nsl super-blocks each), with `sel` bytes in front of the planes: CTAs,
+// parts of a row tile, the rings, and how many units are staged at a time -- all that a CTA meets where they fit.  It depends on the
+// pass's capacity, not on the rows in use or their experts: a row's sums do not depend on its neighbours.
+struct MoeShape { int cps, parts, st, ch, ub; size_t smem; };
+static bool moe_shape(int fmt, int units, int tpu, int nsl, int sel, MoeShape &o) {
+  const long long tiles = (long long)units * tpu;
+  o.cps = tiles < g_llb.sms ? (int)tiles : g_llb.sms;
+  const int mine = (int)((tiles + o.cps - 1) / o.cps), need = mine / tpu + 2 < units ? mine / tpu + 2 : units;
+  o.parts = 1;
+  for (int p = 2; p <= MOE_WARPS && p <= nsl; p *= 2)
+    if (gemm_stream_cost(fmt, MOE_WARPS, 8, mine, nsl, p) < gemm_stream_cost(fmt, MOE_WARPS, 8, mine, nsl, o.parts)) o.parts = p;
+  static const int rings[4][2] = {{2, 2}, {3, 1}, {2, 1}, {1, 1}};
+  for (o.ub = need < 4 ? need : 4; o.ub >= 1; o.ub--)
+    for (int r = fmt == LLB_FM_Q4_K ? 0 : 1; r < (o.ub > 1 ? 3 : 4); r++) {
+      o.st = rings[r][0]; o.ch = rings[r][1];
+      o.smem = G2_BAR_BYTES + (size_t)MOE_WARPS * o.st * o.ch * tile_bytes(fmt) + sel + (size_t)o.ub * moe_unit_bytes(fmt, nsl) + (o.parts > 1 ? MOE_WARPS * 512 : 0);
+      if (o.smem <= G2_SMEM_MAX) return true;
+    }
+  return false;
 }
-// down == false: gate|up of every (token, slot) on planes of K = d columns, one K-slice (the epilogue needs whole sums);
-// down == true: the per-token virtual matrices of K = nslot * ef columns, *ksplit slices (0: chosen here) into m.out
-// wt_silu (down only, T <= 4): the launch builds wt * silu(m.g) * m.u in shared memory itself; xp then only gives K and NC
-int gemm_launch_moe(cudaStream_t s, int fmt, bool down, const XPlanes &xp, MoeArgs &m, int *ksplit, const float *wt_silu) {
+static int moe_check(int fmt, const MoeArgs &m) {
   if (fmt != LLB_FM_Q4_K && fmt != LLB_FM_Q5_K && fmt != LLB_FM_Q6_K) return llb_fail("moe gemm: expert stacks of format %d have no kernel", fmt);
   if (m.ef % 256 || m.d % 256) return llb_fail("moe gemm: widths %d, %d are not multiples of 256", m.ef, m.d);
-  GemmArgs a;
+  if (m.T < 1 || m.T > MOE_MAXROWS || m.ne < 1 || m.ne > 1024 || m.nslot < 2 || m.nslot > 33 || m.nslot - 1 > m.ne) return llb_fail("moe gemm: %d rows, %d experts, top %d", m.T, m.ne, m.nslot - 1);
+  return 0;
+}
+static void moe_gemm_args(GemmArgs &a, int K, int ks, const MoeArgs &m, const MoeShape &o) {
   memset(&a, 0, sizeof a);
-  a.K = down ? m.nslot * m.ef : m.d;
-  if (xp.K != a.K || (xp.NC != 8 && xp.NC != 16 && xp.NC != 32)) return llb_fail("moe gemm: planes of %d x %d columns, K is %d", xp.K, xp.NC, a.K);
-  a.err = g_g3_err; a.nsb = a.K / 256; a.xp = xp; a.planes = 2; a.T = m.T; a.nmat = 0;
-  const int ntiles = down ? m.T * (m.d / 16) : m.T * m.nslot * (m.ef / 8);
-  int ks = 1;
-  if (down) ks = *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, xp.NC, ntiles, a.nsb, g_llb.sms);
-  if (down) ks = gemm_fix_ksplit(fmt, xp.NC, a.nsb, ks);
-  else if (a.nsb > g2_longest_slice(fmt, xp.NC)) return llb_fail("moe gemm: %d columns do not fit one K-slice", a.K);
-  a.ksplit = ks;
-  if (ksplit) *ksplit = ks;
-  const int NT = xp.NC / 8;
-#define MOE_GO(F) return NT == 1 ? launch_moe<F, 1>(s, down, a, m, ntiles, wt_silu) : NT == 2 ? launch_moe<F, 2>(s, down, a, m, ntiles, wt_silu) : launch_moe<F, 4>(s, down, a, m, ntiles, wt_silu)
+  a.K = K; a.nsb = K / 256; a.ksplit = ks; a.parts = o.parts; a.planes = 2; a.T = m.T; a.err = g_g3_err;
+}
+// the choice, then gate|up of every unit on planes of d columns (whole sums: one K-slice)
+int gemm_launch_moe_gu(cudaStream_t s, int fmt, const XPlanes &xp, const MoeArgs &m) {
+  if (moe_check(fmt, m)) return -1;
+  if (xp.K != m.d) return llb_fail("moe gemm: planes of %d columns, the experts take %d", xp.K, m.d);
+  MoeShape o;
+  if (!moe_shape(fmt, m.T * m.nslot, m.ef / 8, m.d / 256, moe_sel_bytes(m.T * m.nslot), o)) return llb_fail("moe gemm: %d columns do not fit one K-slice", m.d);
+  GemmArgs a;
+  moe_gemm_args(a, m.d, 1, m, o);
+  a.xp = xp;
+  const bool wide = m.ne > 256;
+#define MOE_GO(F) CU_OK(llb_launch(wide ? k_moe_gu<F, 32> : k_moe_gu<F, 8>, dim3(o.cps), dim3(MOE_WARPS * 32), o.smem, s, a, m, o.st, o.ch, o.ub))
   if (fmt == LLB_FM_Q4_K) MOE_GO(LLB_FM_Q4_K);
-  if (fmt == LLB_FM_Q5_K) MOE_GO(LLB_FM_Q5_K);
-  MOE_GO(LLB_FM_Q6_K);
+  else if (fmt == LLB_FM_Q5_K) MOE_GO(LLB_FM_Q5_K);
+  else MOE_GO(LLB_FM_Q6_K);
 #undef MOE_GO
+  return 0;
+}
+// K-slices of an expert's ef columns in the down launch: one, or where a unit's activations do not fit the fewest equal ones that do
+int gemm_moe_dn_ksplit(int fmt, const MoeArgs &m) {
+  MoeShape o;
+  for (int ks = 1; ks <= m.ef / 256; ks++)
+    if (m.ef / 256 % ks == 0 && moe_shape(fmt, m.T * m.nslot * ks, m.d / 16, m.ef / 256 / ks, m.T * m.nslot * 16, o)) return ks;
+  return 0;
+}
+// the units' down matrices on wt * silu(g) * u; slice slot * ks + k of m.out is K-slice k of that slot
+int gemm_launch_moe_dn(cudaStream_t s, int fmt, const MoeArgs &m, int ks) {
+  if (moe_check(fmt, m)) return -1;
+  MoeShape o;
+  if (ks < 1 || m.ef / 256 % ks || !moe_shape(fmt, m.T * m.nslot * ks, m.d / 16, m.ef / 256 / ks, m.T * m.nslot * 16, o)) return llb_fail("moe gemm: %d K-slices of %d columns", ks, m.ef);
+  GemmArgs a;
+  moe_gemm_args(a, m.ef, ks, m, o);
+#define MOE_GO(F) CU_OK(llb_launch(k_moe_dn<F>, dim3(o.cps), dim3(MOE_WARPS * 32), o.smem, s, a, m, o.st, o.ch, o.ub))
+  if (fmt == LLB_FM_Q4_K) MOE_GO(LLB_FM_Q4_K);
+  else if (fmt == LLB_FM_Q5_K) MOE_GO(LLB_FM_Q5_K);
+  else MOE_GO(LLB_FM_Q6_K);
+#undef MOE_GO
+  return 0;
 }
 
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a) {

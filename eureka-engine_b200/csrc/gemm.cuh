@@ -57,13 +57,17 @@ struct GemmArgs {
 struct MoeArgs {
   const uint8_t *W;     // GU or D stack
   long long es;         // bytes per expert block
-  const int *ids;       // [live rows][nslot]
   int nslot;            // k + 1
   int ne;               // block ne is the shared expert; ids are clamped to 0..ne
   int ef, d, T;
-  const int *live;      // rows of the pass in use: how many, then which, ascending (rows without a token cost nothing)
+  const float *lg;      // router logits [T][ne + 1]
+  const void *rs;       // the rows of the pass (RowSet), `per` to a stream, `stride` bytes from one stream's set to the next
+  int per, stride;
+  int *ids;             // [live rows][nslot]: the choice, left by the gate|up launch
+  float *wt;            // [T][nslot]
+  int4 *units;          // how many, then the units (moe.cuh)
   float *g, *u;         // gate|up: [T][nslot * ef]
-  float *out;           // k_moe_dn: [ksplit][T][d]
+  float *out;           // down: [nslot * ksplit][T][d]
   long long split_stride;
 };
 

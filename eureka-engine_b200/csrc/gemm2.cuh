@@ -33,8 +33,8 @@
 // whose whole d = 2048 slice must fit.
 // Super-blocks a copy brings.  A bulk copy costs about 85 cycles of the SM's copy engine on top of its bytes (copies alone, no
 // arithmetic, gate|up of the 27B shape: 19.6 us at 2304 bytes, 11.8 us at 4608), so Q4_K takes two at a time.
-// ring 1: a shorter ring for K-slices that do not fit beside the usual one (ring 0): one K-slice of wide routed-expert models
-// (their epilogue needs whole sums), and matrices of more than GEMM_MAXSPLIT of the usual slices.
+// ring 1: a shorter ring for K-slices that do not fit beside the usual one (ring 0): matrices of more than GEMM_MAXSPLIT of the
+// usual slices.
 __host__ __device__ constexpr int g2_chunk(int fmt, int ring = 0) { return fmt == LLB_FM_Q4_K && !ring ? 2 : 1; }
 __host__ __device__ constexpr int g2_stages(int fmt, int NC, int ring = 0) {
   if (ring == 2) return 2;
@@ -54,8 +54,7 @@ __host__ __device__ constexpr int g2_warps(int fmt, int NC) {
 __host__ __device__ constexpr int g2_ring_bytes(int fmt, int NC, int ring = 0) { return g2_warps(fmt, NC) * g2_stages(fmt, NC, ring) * g2_chunk(fmt, ring) * tile_bytes(fmt); }
 __host__ __device__ constexpr int g2_aux(int fmt) { return fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K ? 32 : 0; }
 __host__ __device__ constexpr int g2_xpad(int fmt) { return fmt == LLB_FM_Q6_K ? 32 : 64; }
-// bytes of shared memory of a launch whose K-slices have nsl super-blocks in `parts` parts, for NC activation columns (ntc
-// n-tiles of which are summed over the parts)
+// bytes of shared memory of a launch whose K-slices have nsl super-blocks in `parts` parts, for NC activation columns (ntc of them in n-tiles that are summed over the parts)
 __host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC, int parts = 1, int ntc = 4, int ring = 0) {
   return (size_t)(parts > 1 ? g2_warps(fmt, NC) * ntc * 512 : 0) + G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC, ring);
 }
@@ -121,14 +120,13 @@ __device__ __forceinline__ void g2_group_scales(uint32_t u0, uint32_t u1, uint32
 }
 
 // One staged tile times the staged planes of super-block c_c of the slice: acc[nt] += the tile's contribution to n-tile nt.
-//   st     the tile (shared memory);  xh_s, xsf_s, CS  the staged planes, means and column stride;  cb  first plane column
-//   NTS    plane columns from one computed n-tile to the next
-template <int FMT, int NT, int NTC, bool FOLD>
-__device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, const uint8_t *xsf_s, const int CS, const int c_c, const int cb, const int lane, float (&acc)[NTC][4]) {
-  constexpr int NC = 8 * NT, NTS = NTC == NT ? 8 : NC / 2;
+//   st     the tile (shared memory);  xh_s, xsf_s, CS  the staged planes, means and column stride
+template <int FMT, int NT, bool FOLD>
+__device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, const uint8_t *xsf_s, const int CS, const int c_c, const int lane, float (&acc)[NT][4]) {
+  constexpr int NC = 8 * NT;
   const int gid = lane >> 2, j = lane & 3, r0 = g2_row<FMT, FOLD>(gid);
   const uint8_t *b0 = st + r0 * tile_row(FMT), *b1 = b0 + 8 * tile_row(FMT);
-  const uint8_t *xb = xh_s + (gid + cb) * CS + (size_t)c_c * 512;
+  const uint8_t *xb = xh_s + gid * CS + (size_t)c_c * 512;
   if constexpr (FMT == LLB_FM_Q8_0) {
     // eight blocks of 32 codes, two MMAs each; lane j holds columns 8 j .. 8 j + 7 of a block
     const uint4 sw0 = *(const uint4 *)(b0 + 256), sw1 = *(const uint4 *)(b1 + 256);
@@ -149,8 +147,8 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
       const float2 f0 = __half22float2(*(const __half2 *)&d0w[blk >> 1]), f1 = __half22float2(*(const __half2 *)&d1w[blk >> 1]);
       const float d0 = (blk & 1) ? f0.y : f0.x, d1 = (blk & 1) ? f1.y : f1.x;
 #pragma unroll
-      for (int nt = 0; nt < NTC; nt++) {
-        const uint4 bx = *(const uint4 *)(xb + (size_t)nt * NTS * CS + 64 * blk);
+      for (int nt = 0; nt < NT; nt++) {
+        const uint4 bx = *(const uint4 *)(xb + (size_t)nt * 8 * CS + 64 * blk);
         float p[4];
         mma16816_z(p, A[0][0], A[0][1], A[0][2], A[0][3], bx.x, bx.y);
         mma16816(p, A[1][0], A[1][1], A[1][2], A[1][3], bx.z, bx.w);
@@ -164,9 +162,9 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
     const uint32_t sc0w[4] = {sw0.x ^ 0x80808080u, sw0.y ^ 0x80808080u, sw0.z ^ 0x80808080u, sw0.w ^ 0x80808080u};
     const uint32_t sc1w[4] = {sw1.x ^ 0x80808080u, sw1.y ^ 0x80808080u, sw1.z ^ 0x80808080u, sw1.w ^ 0x80808080u};
     xb += 8 * j;
-    float sS[NTC][4];
+    float sS[NT][4];
 #pragma unroll
-    for (int nt = 0; nt < NTC; nt++) sS[nt][0] = sS[nt][1] = sS[nt][2] = sS[nt][3] = 0.0f;
+    for (int nt = 0; nt < NT; nt++) sS[nt][0] = sS[nt][1] = sS[nt][2] = sS[nt][3] = 0.0f;
 #pragma unroll
     for (int hf = 0; hf < 2; hf++) {
 #pragma unroll
@@ -194,8 +192,8 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
           if (qd >= 2) { s0 *= 0.0625f; s1 *= 0.0625f; }
           const int kl = 128 * hf + 32 * qd + 16 * u;
 #pragma unroll
-          for (int nt = 0; nt < NTC; nt++) {
-            const uint2 bx = *(const uint2 *)(xb + (size_t)nt * NTS * CS + kl * 2);
+          for (int nt = 0; nt < NT; nt++) {
+            const uint2 bx = *(const uint2 *)(xb + (size_t)nt * 8 * CS + kl * 2);
             float p[4];
             mma16816_z(p, e0, e1, o0, o1, bx.x, bx.y);
             sS[nt][0] += s0 * p[0]; sS[nt][1] += s0 * p[1]; sS[nt][2] += s1 * p[2]; sS[nt][3] += s1 * p[3];
@@ -204,7 +202,7 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
       }
     }
 #pragma unroll
-    for (int nt = 0; nt < NTC; nt++) { acc[nt][0] += d0 * sS[nt][0]; acc[nt][1] += d0 * sS[nt][1]; acc[nt][2] += d1 * sS[nt][2]; acc[nt][3] += d1 * sS[nt][3]; }
+    for (int nt = 0; nt < NT; nt++) { acc[nt][0] += d0 * sS[nt][0]; acc[nt][1] += d0 * sS[nt][1]; acc[nt][2] += d1 * sS[nt][2]; acc[nt][3] += d1 * sS[nt][3]; }
   } else {
     constexpr int QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
     const uint4 h0 = *(const uint4 *)b0, h1 = *(const uint4 *)b1;
@@ -216,10 +214,10 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
       const uint32_t at0 = __byte_perm(j < 2 ? mnA0 : mnB0, 0x64646464u, ms), at1 = __byte_perm(j < 2 ? mnA1 : mnB1, 0x64646464u, ms);
       const uint32_t am0 = g2_hfma2(at0, 0x3c003c00u, 0xe400e400u), am1 = g2_hfma2(at1, 0x3c003c00u, 0xe400e400u);       // * 1 - 1024
       const uint32_t al0 = g2_hfma2(at0, 0x10001000u, 0xb800b800u), al1 = g2_hfma2(at1, 0x10001000u, 0xb800b800u);       // * 2^-11 - 0.5
-      float sS[NTC][4], pm[NTC][4];
+      float sS[NT][4], pm[NT][4];
 #pragma unroll
-      for (int nt = 0; nt < NTC; nt++) {
-        const uint2 xf = *(const uint2 *)(xsf_s + ((size_t)c_c * NC + nt * NTS + cb + gid) * 32 + 8 * j);
+      for (int nt = 0; nt < NT; nt++) {
+        const uint2 xf = *(const uint2 *)(xsf_s + ((size_t)c_c * NC + nt * 8 + gid) * 32 + 8 * j);
         mma16816_z(pm[nt], am0, am1, al0, al1, xf.x, xf.y);
         sS[nt][0] = sS[nt][1] = sS[nt][2] = sS[nt][3] = 0.0f;
       }
@@ -249,8 +247,8 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
         const float sc0l = byte_f(s0, (2 * g) & 3), sc0h = byte_f_scaled(s0, (2 * g + 1) & 3, 0.0625f);
         const float sc1l = byte_f(s1, (2 * g) & 3), sc1h = byte_f_scaled(s1, (2 * g + 1) & 3, 0.0625f);
 #pragma unroll
-        for (int nt = 0; nt < NTC; nt++) {
-          const uint8_t *xr = xb + (size_t)nt * NTS * CS + 128 * g;
+        for (int nt = 0; nt < NT; nt++) {
+          const uint8_t *xr = xb + (size_t)nt * 8 * CS + 128 * g;
           const uint4 bl = *(const uint4 *)xr, bh = *(const uint4 *)(xr + 64);
           float pl[4], ph[4];
           mma16816_z(pl, A[0][0][0], A[0][0][1], A[0][0][2], A[0][0][3], bl.x, bl.y);
@@ -266,7 +264,7 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
       const float d0 = h2f_bits(h0.x & 0xffffu) * TWO24, dm0 = h2f_bits(h0.x >> 16) * 32.0f;
       const float d1 = h2f_bits(h1.x & 0xffffu) * TWO24, dm1 = h2f_bits(h1.x >> 16) * 32.0f;
 #pragma unroll
-      for (int nt = 0; nt < NTC; nt++) {
+      for (int nt = 0; nt < NT; nt++) {
         acc[nt][0] += d0 * sS[nt][0] - dm0 * pm[nt][0];
         acc[nt][1] += d0 * sS[nt][1] - dm0 * pm[nt][1];
         acc[nt][2] += d1 * sS[nt][2] - dm1 * pm[nt][2];
@@ -287,10 +285,10 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
     const uint32_t at0 = __byte_perm(mn0, 0x64646464u, 0x4140), at1 = __byte_perm(mn1, 0x64646464u, 0x4140);
     const uint32_t am0 = g2_hfma2(at0, 0x3c003c00u, 0xe400e400u), am1 = g2_hfma2(at1, 0x3c003c00u, 0xe400e400u);       // * 1 - 1024
     const uint32_t al0 = g2_hfma2(at0, 0x10001000u, 0xb800b800u), al1 = g2_hfma2(at1, 0x10001000u, 0xb800b800u);       // * 2^-11 - 0.5
-    float pl[NTC][4], ph[NTC][4], pm[NTC][4];
+    float pl[NT][4], ph[NT][4], pm[NT][4];
 #pragma unroll
-    for (int nt = 0; nt < NTC; nt++) {
-      const uint2 xf = *(const uint2 *)(xsf_s + ((size_t)c_c * NC + nt * NTS + cb + gid) * 32 + 8 * j);
+    for (int nt = 0; nt < NT; nt++) {
+      const uint2 xf = *(const uint2 *)(xsf_s + ((size_t)c_c * NC + nt * 8 + gid) * 32 + 8 * j);
       mma16816_z(pm[nt], am0, am1, al0, al1, xf.x, xf.y);
     }
     xb += 16 * j;
@@ -307,8 +305,8 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
         A[w][1][2] = g2_hmul2(y0 & 0x00f000f0u, H0); A[w][1][3] = g2_hmul2(y1 & 0x00f000f0u, H1);
       }
 #pragma unroll
-      for (int nt = 0; nt < NTC; nt++) {
-        const uint8_t *xr = xb + (size_t)nt * NTS * CS + 64 * q;
+      for (int nt = 0; nt < NT; nt++) {
+        const uint8_t *xr = xb + (size_t)nt * 8 * CS + 64 * q;
         const uint4 bl = *(const uint4 *)xr, bh = *(const uint4 *)(xr + 256);
         if (q == 0) {
           mma16816_z(pl[nt], A[0][0][0], A[0][0][1], A[0][0][2], A[0][0][3], bl.x, bl.y);
@@ -324,7 +322,7 @@ __device__ __forceinline__ void g2_tile(const uint8_t *st, const uint8_t *xh_s, 
     const float d0 = h2f_bits(h0.x & 0xffffu) * 16384.0f, dm0 = h2f_bits(h0.x >> 16) * 32.0f;
     const float d1 = h2f_bits(h1.x & 0xffffu) * 16384.0f, dm1 = h2f_bits(h1.x >> 16) * 32.0f;
 #pragma unroll
-    for (int nt = 0; nt < NTC; nt++) {
+    for (int nt = 0; nt < NT; nt++) {
       acc[nt][0] += d0 * (pl[nt][0] + ph[nt][0]) - dm0 * pm[nt][0];
       acc[nt][1] += d0 * (pl[nt][1] + ph[nt][1]) - dm0 * pm[nt][1];
       acc[nt][2] += d1 * (pl[nt][2] + ph[nt][2]) - dm1 * pm[nt][2];
@@ -366,11 +364,9 @@ __device__ __forceinline__ void g2_drain(const G2Ring &r) {
 
 // Where a launch's row tiles live.  A policy says how many 16-row tiles there are, where tile i's 16 x 256 tiles in the
 // CTA's K-slice are, and what to do with a finished row tile.  G2MatsPlain is the launch of up to four matrices that
-// GemmArgs describes; the routed-expert launches (moe.cuh) find their matrices through the expert ids an earlier kernel chose.
-//   EARLY   the weight addresses depend on no earlier kernel: the ring's prologue is issued before the wait
+// GemmArgs describes.
 //   Cur     cursor of the row tile being copied;  locate  row tile -> cursor;  src  tile of super-block sb0 + c of the slice
 template <int FMT, bool FOLD = false> struct G2MatsPlain {
-  static constexpr bool EARLY = true, CONTIG = true;
   const GemmArgs &a;
   struct Cur { const uint8_t *W; };
   __device__ __forceinline__ int ntiles() const { return a.tile0[a.nmat]; }
@@ -379,7 +375,7 @@ template <int FMT, bool FOLD = false> struct G2MatsPlain {
     while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
     c.W = a.m[m].W + ((size_t)(tile - a.tile0[m]) * a.nsb + sb0) * tile_bytes(FMT);
   }
-  __device__ __forceinline__ const uint8_t *src(const Cur &c, int sb0, int pc) const { return c.W + (size_t)pc * tile_bytes(FMT); }
+  __device__ __forceinline__ const uint8_t *src(const Cur &c, int pc) const { return c.W + (size_t)pc * tile_bytes(FMT); }
   template <int NT> __device__ __forceinline__ void epilogue(int ks, int tile, float (&acc)[NT][4], int lane) const {
     int m = 0;
     while (m + 1 < a.nmat && tile >= a.tile0[m + 1]) m++;
@@ -399,13 +395,9 @@ template <int FMT, bool FOLD = false> struct G2MatsPlain {
 //
 // Tile of (CTA ci, warp group w, round n) = (n * groups + w) * cps + ci: consecutive tiles go to different SMs, so the SMs'
 // tile counts differ by one at most.
-// NTC < NT (the routed-expert launches at 16 rows): a weight tile is multiplied with NTC = 2 of the NT staged n-tiles only,
-// the hi and lo tiles of the eight rows its own row is among (Mats::col0(tile) = first plane column of the hi tile; the
-// lo tile is NC / 2 columns on), since the epilogue keeps one row of the tile.
-template <int FMT, int NT, class Stage, class Mats, int NTC = NT, bool FOLD = false, int RING = 0>
+template <int FMT, int NT, class Stage, class Mats, bool FOLD = false, int RING = 0>
 __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const int bid, G2Ring &rg, uint8_t *planes, Stage stage, const Mats mats) {
   constexpr int NC = 8 * NT, WARPS = g2_warps(FMT, NC), TB = tile_bytes(FMT), ST = g2_stages(FMT, NC, RING), CH = g2_chunk(FMT, RING);
-  static_assert(NTC == NT || NTC == 2, "a column selection computes one hi and one lo n-tile");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool live = bid < cps * a.ksplit && warp < WARPS;
   const int ks = bid % a.ksplit, ci = bid / a.ksplit;
@@ -414,7 +406,6 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
   uint8_t *xh_s = planes, *xsf_s = planes + NC * CS;
   const int P = a.parts, lp = 31 - __clz(P), grp = warp >> lp, mine = warp & (P - 1), nws = (WARPS >> lp) * cps;
   const int tile0 = grp * cps + ci, c0 = (mine * nsl) >> lp, c1 = ((mine + 1) * nsl) >> lp;   // this warp's tiles; its part
-  if constexpr (!Mats::EARLY) stage(xh_s, xsf_s, CS, sb0, nsl);   // the weight addresses come from an earlier kernel's choice: the wait comes first
   const int ntiles = live ? mats.ntiles() : 0;                    // a warp that is not live sees no tiles
   int p_tile = tile0, p_c = c0;                                   // producer: (tile, super-block) of the next copy
   typename Mats::Cur p_cur;
@@ -425,8 +416,7 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
     if (lane == 0) {
       const uint32_t bar = rg.bar_s + 8 * s, dst = rg.ring_s + s * CH * TB;
       mbar_expect(bar, n * TB);
-      if (Mats::CONTIG || CH == 1) bulk_load(dst, mats.src(p_cur, sb0, p_c), n * TB, bar);
-      else for (int u = 0; u < n; u++) bulk_load(dst + u * TB, mats.src(p_cur, sb0, p_c + u), TB, bar);
+      bulk_load(dst, mats.src(p_cur, p_c), n * TB, bar);
     }
     p_c += n;
     if (p_c == c1) {
@@ -438,21 +428,19 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
   // still runs, and while the activation slice is staged
 #pragma unroll 1
   for (int s = 0; s < ST; s++) issue(s);
-  if constexpr (Mats::EARLY) stage(xh_s, xsf_s, CS, sb0, nsl);
-  float4 *red = (float4 *)(planes + NC * (((a.nsb + a.ksplit - 1) / a.ksplit) * (512 + g2_aux(FMT)) + g2_xpad(FMT))) + warp * NTC * 32 + lane;
+  stage(xh_s, xsf_s, CS, sb0, nsl);
+  float4 *red = (float4 *)(planes + NC * (((a.nsb + a.ksplit - 1) / a.ksplit) * (512 + g2_aux(FMT)) + g2_xpad(FMT))) + warp * NT * 32 + lane;
   int s = 0;
 #pragma unroll 1
   for (int tile = tile0; tile < ntiles; tile += nws) {
-    int cb = 0;                                            // first plane column of the computed n-tiles
-    if constexpr (NTC != NT) cb = mats.col0(tile);
-    float acc[NTC][4];
+    float acc[NT][4];
 #pragma unroll
-    for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
+    for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
 #pragma unroll 1
     for (int c = c0; c < c1; c += CH) {
       g2_wait(rg, s, G2_WAIT_LIMIT, a.err);
 #pragma unroll 1
-      for (int u = 0; u < CH && c + u < c1; u++) g2_tile<FMT, NT, NTC, FOLD>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, cb, lane, acc);
+      for (int u = 0; u < CH && c + u < c1; u++) g2_tile<FMT, NT, FOLD>(rg.ring + (s * CH + u) * TB, xh_s, xsf_s, CS, c + u, lane, acc);
       __syncwarp();                                        // every lane has read the stage
       issue(s);
       s = s + 1 == ST ? 0 : s + 1;
@@ -460,21 +448,21 @@ __device__ __forceinline__ void g2_phase(const GemmArgs &a, const int cps, const
     if (P > 1) {
       if (mine) {
 #pragma unroll
-        for (int nt = 0; nt < NTC; nt++) red[nt * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+        for (int nt = 0; nt < NT; nt++) red[nt * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
       }
       asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * P) : "memory");
       if (!mine) {
 #pragma unroll 1
         for (int q = 1; q < P; q++)
 #pragma unroll
-          for (int nt = 0; nt < NTC; nt++) {
-            const float4 v = red[(q * NTC + nt) * 32];
+          for (int nt = 0; nt < NT; nt++) {
+            const float4 v = red[(q * NT + nt) * 32];
             acc[nt][0] += v.x; acc[nt][1] += v.y; acc[nt][2] += v.z; acc[nt][3] += v.w;
           }
       }
       if (tile + nws < ntiles) asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * P) : "memory");   // read before it is written again
     }
-    if (!mine) mats.template epilogue<NTC>(ks, tile, acc, lane);
+    if (!mine) mats.template epilogue<NT>(ks, tile, acc, lane);
   }
 }
 
@@ -507,7 +495,7 @@ __global__ void __launch_bounds__(g2_warps(FMT, 8 * NT) * 32, 1) k_gemm2(const G
   pdl_trigger();
   constexpr int RB = g2_ring_bytes(FMT, 8 * NT, RING);
   G2Ring rg = g2_ring_init(smem, RB / g2_warps(FMT, 8 * NT));
-  g2_phase<FMT, NT, G2StagePlanes<FMT, NT, FOLD>, G2MatsPlain<FMT, FOLD>, NT, FOLD, RING>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<FMT, NT, FOLD>{a},
+  g2_phase<FMT, NT, G2StagePlanes<FMT, NT, FOLD>, G2MatsPlain<FMT, FOLD>, FOLD, RING>(a, cps, (int)blockIdx.x, rg, smem + G2_BAR_BYTES + RB, G2StagePlanes<FMT, NT, FOLD>{a},
                                                                                          G2MatsPlain<FMT, FOLD>{a});
   g2_drain(rg);
 }

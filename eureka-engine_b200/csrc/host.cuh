@@ -57,7 +57,9 @@ int gemm_wait_errors_clear(void);
 int gemm_wait_selftest(cudaStream_t s, int which, int limit);
 bool gemm_ffn_fusable(int fmt_gu, int fmt_dn, int NC, int d, int f, int *ks2);
 int gemm_launch_ffn(cudaStream_t s, GemmArgs &a1, int fmt2, GemmArgs &a2);   // gate|up (Q4_K, one K-slice), silu, down in one launch
-int gemm_launch_moe(cudaStream_t s, int fmt, bool down, const XPlanes &xp, MoeArgs &m, int *ksplit, const float *wt_silu);   // moe.cuh
+int gemm_launch_moe_gu(cudaStream_t s, int fmt, const XPlanes &xp, const MoeArgs &m);   // moe.cuh
+int gemm_moe_dn_ksplit(int fmt, const MoeArgs &m);
+int gemm_launch_moe_dn(cudaStream_t s, int fmt, const MoeArgs &m, int ks);
 
 // api.cu: from the first to the last of a series of uploads, the staging buffer of those from host memory is kept
 void upload_hold(bool from_host);

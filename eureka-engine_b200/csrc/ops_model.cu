@@ -131,9 +131,7 @@ int op_norm_xp(cudaStream_t s, const float *xin, PartIn add, const float *w, flo
 }
 
 // ---- silu(gate) * up -> planes (llb_t_siluq, tools/payload-spec2.patch:114-124) -----------------
-// scale (optional): the product of row t, columns [j seg, (j+1) seg) is multiplied by scale[t * (f / seg) + j]
-// (the routed experts' weights, folded into the activations the down matrices see)
-__global__ void __launch_bounds__(256) k_silu_xp(PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, Streams sg, const float *__restrict__ scale, int seg) {
+__global__ void __launch_bounds__(256) k_silu_xp(PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, Streams sg) {
   int rs_n, rs_p0, tl;
   const int t = blockIdx.y, lane = threadIdx.x & 31;
   rs = rs_begin_row(rs, sg, t, rs_n, rs_p0, tl);
@@ -160,37 +158,27 @@ __global__ void __launch_bounds__(256) k_silu_xp(PartIn g, PartIn u, int f, XPla
         uv.x += m[q].x; uv.y += m[q].y; uv.z += m[q].z; uv.w += m[q].w;
       }
     }
-    const float w = scale ? __ldcg(scale + (size_t)t * (f / seg) + c / seg) : 1.0f;
-    h[0] = silu_f(gv.x) * uv.x * w; h[1] = silu_f(gv.y) * uv.y * w; h[2] = silu_f(gv.z) * uv.z * w; h[3] = silu_f(gv.w) * uv.w * w;
+    h[0] = silu_f(gv.x) * uv.x; h[1] = silu_f(gv.y) * uv.y; h[2] = silu_f(gv.z) * uv.z; h[3] = silu_f(gv.w) * uv.w;
   }
   xp_store4(xp, t, 2, c, h, lane, on);
 }
 int op_silu_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, int Tmax) {
   if (f % 32) return llb_fail("silu: f %d", f);
-  CU_OK(llb_launch(k_silu_xp, dim3((f / 4 + 255) / 256, Tmax), dim3(256), (size_t)(0), s, g, u, f, xp, rs, g_streams, (const float *)nullptr, f));
-  CU_OK(cudaGetLastError());
-  return 0;
-}
-int op_silu_scaled_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, int Tmax, const float *scale, int seg) {
-  if (f % 32 || seg % 4 || f % seg) return llb_fail("silu: f %d, segments of %d", f, seg);
-  CU_OK(llb_launch(k_silu_xp, dim3((f / 4 + 255) / 256, Tmax), dim3(256), (size_t)(0), s, g, u, f, xp, rs, g_streams, scale, seg));
+  CU_OK(llb_launch(k_silu_xp, dim3((f / 4 + 255) / 256, Tmax), dim3(256), (size_t)(0), s, g, u, f, xp, rs, g_streams));
   CU_OK(cudaGetLastError());
   return 0;
 }
 
-// ---- the router of a routed-expert layer (host/llb_host.c:622-724; llb_moe_topk of tools/payload-moeany.patch; the top k of a
-// row is moe_route_row, rowops.cuh) ----
+// ---- the router of a routed-expert layer (host/llb_host.c:622-724; llb_moe_topk of tools/payload-moeany.patch) ----
 // Router logits lg[t][r] = W[r] . h[t] for the ne router rows and the shared expert's gate row (row ne): F32
-// weights, a block per row (every load of the row in flight at once), all rows of the pass.  The block that
-// finishes last (a counter, no waiting) then routes: its warp t takes row t of the pass.
-#define MOE_MAXROWS 16   // rows of a pass the router takes (several streams of k + 1 rows)
-template <int NQ, int MR>   // MR: the most rows of a pass (8 or 16); two resident blocks a multiprocessor, so that the ne + 1 blocks are one wave
-__global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__ W, const float *__restrict__ h, int d, int ne, int nk, float *__restrict__ lg,
-                                                    int *__restrict__ ids, float *__restrict__ wt, unsigned int *__restrict__ ctr, int *__restrict__ live, const RowSet *rs, Streams sg, int n_all) {
+// weights, a block per row, all rows of the pass; the gate|up launch makes the choice from them (moe.cuh).  Bound by the one trip
+// to L2 for the rows of h, so four rows are in flight at a time: row by row, each trip behind the last, sixteen rows
+// took 21 us.
+#define MOE_MAXROWS 16   // rows of a pass (several streams of k + 1 rows)
+__global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__ W, const float *__restrict__ h, int d, int ne, float *__restrict__ lg, const RowSet *rs, int n_all) {
   int rs_n, rs_p0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.x, nrows = ne + 1;
-  __shared__ float red[8][MR];
-  __shared__ unsigned int last;
+  __shared__ float red[8][MOE_MAXROWS];
   // the row's weights depend on no kernel: fetched before the wait (two float4 per thread cover d <= 2048)
   const float4 *wr = (const float4 *)(W + (size_t)r * d);
   const int c0 = threadIdx.x, c1 = threadIdx.x + 256, nc = d / 4;
@@ -198,25 +186,33 @@ __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__
   const float4 w0 = c0 < nc ? __ldg(wr + c0) : z4, w1 = c1 < nc ? __ldg(wr + c1) : z4;
   rs = rs_begin(rs, rs_n, rs_p0);
   if (n_all > 0) rs_n = n_all;   // a pass over several streams: every row of the pass (a stream's idle rows cost nothing that matters)
-  float acc[MR];
+#pragma unroll 1
+  for (int t0 = 0; t0 < rs_n; t0 += 4) {
+    float4 a[4], b[4];
+    float acc[4];
 #pragma unroll
-  for (int t = 0; t < MR; t++) {
-    acc[t] = 0.0f;
-    if (t < rs_n) {
-      const float4 *x = (const float4 *)(h + (size_t)t * d);
-      if (c0 < nc) { const float4 v = __ldcg(x + c0); acc[t] += (w0.x * v.x + w0.y * v.y) + (w0.z * v.z + w0.w * v.w); }
-      if (c1 < nc) { const float4 v = __ldcg(x + c1); acc[t] += (w1.x * v.x + w1.y * v.y) + (w1.z * v.z + w1.w * v.w); }
-      for (int c = threadIdx.x + 512; c < nc; c += 256) {
-        const float4 w = __ldg(wr + c), v = __ldcg(x + c);
-        acc[t] += (w.x * v.x + w.y * v.y) + (w.z * v.z + w.w * v.w);
+    for (int q = 0; q < 4; q++) {
+      const float4 *x = (const float4 *)(h + (size_t)min(t0 + q, rs_n - 1) * d);
+      a[q] = c0 < nc ? __ldcg(x + c0) : z4;
+      b[q] = c1 < nc ? __ldcg(x + c1) : z4;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      acc[q] = (w0.x * a[q].x + w0.y * a[q].y) + (w0.z * a[q].z + w0.w * a[q].w);
+      acc[q] += (w1.x * b[q].x + w1.y * b[q].y) + (w1.z * b[q].z + w1.w * b[q].w);
+    }
+    for (int c = threadIdx.x + 512; c < nc; c += 256) {
+      const float4 w = __ldg(wr + c);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float4 v = __ldcg((const float4 *)(h + (size_t)min(t0 + q, rs_n - 1) * d) + c);
+        acc[q] += (w.x * v.x + w.y * v.y) + (w.z * v.z + w.w * v.w);
       }
     }
-  }
 #pragma unroll
-  for (int t = 0; t < MR; t++) {
-    if (t < rs_n) {   // the same for every thread of the launch
-      const float v = warp_sum(acc[t]);
-      if (lane == 0) red[warp][t] = v;
+    for (int q = 0; q < 4; q++) {
+      const float v = warp_sum(acc[q]);
+      if (lane == 0) red[warp][t0 + q] = v;
     }
   }
   __syncthreads();
@@ -225,39 +221,12 @@ __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__
 #pragma unroll
     for (int w = 0; w < 8; w++) v += red[w][threadIdx.x];
     lg[(size_t)threadIdx.x * nrows + r] = v;
-    __threadfence();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ctr, 1u);
-  __syncthreads();
-  if (last != gridDim.x - 1) return;
-  __threadfence();
-  if (threadIdx.x == 0) *ctr = 0;   // ready for the next launch (launches of one stream do not overlap here)
-  // which rows are in use: all of them in a pass of one stream, else the first n of every stream's
-  bool on = lane < rs_n;
-  if (n_all > 0 && on) { const int z = lane / sg.per; on = lane - z * sg.per < __ldcg(&((const RowSet *)((const char *)rs + (size_t)z * sg.stride))->n); }
-  const unsigned int mask = __ballot_sync(0xffffffffu, on);
-  if (warp == 0) {
-    if (lane == 0) live[0] = __popc(mask);
-    if (on) live[1 + __popc(mask & ((1u << lane) - 1))] = lane;
-  }
-  for (int t = warp; t < rs_n; t += 8)
-    if ((mask >> t) & 1) moe_route_row<NQ>(lg + (size_t)t * nrows, ne, nk, ids + (size_t)__popc(mask & ((1u << t) - 1)) * (nk + 1), wt + (size_t)t * (nk + 1), lane);
 }
-static unsigned int *g_moe_ctr = nullptr;
-int op_moe_route(cudaStream_t s, const float *Wr, const float *h, int d, int ne, int nk, float *lg, int *ids, float *wt, int *live, const RowSet *rs, int Tmax) {
-  const int n_all = g_streams.stride ? Tmax : 0;
+int op_moe_logits(cudaStream_t s, const float *Wr, const float *h, int d, int ne, float *lg, const RowSet *rs, int Tmax) {
   if (Tmax > MOE_MAXROWS) return llb_fail("moe route: %d rows in a pass (at most %d)", Tmax, MOE_MAXROWS);
-  if (ne < 1 || ne > 1024 || nk < 1 || nk > 32 || nk > ne || d % 4) return llb_fail("moe route: %d experts, top %d, d %d", ne, nk, d);
-  if (!g_moe_ctr) {
-    CU_OK(cudaMalloc(&g_moe_ctr, 4));
-    CU_OK(cudaMemset(g_moe_ctr, 0, 4));
-  }
-#define ROUTE_GO(NQ, MR) CU_OK(llb_launch(k_moe_router<NQ, MR>, dim3(ne + 1), dim3(256), (size_t)(0), s, Wr, h, d, ne, nk, lg, ids, wt, g_moe_ctr, live, rs, g_streams, n_all))
-  if (ne <= 256) { if (Tmax <= 8) ROUTE_GO(8, 8); else ROUTE_GO(8, MOE_MAXROWS); }
-  else { if (Tmax <= 8) ROUTE_GO(32, 8); else ROUTE_GO(32, MOE_MAXROWS); }
-#undef ROUTE_GO
-  CU_OK(cudaGetLastError());
+  if (ne < 1 || ne > 1024 || d % 4) return llb_fail("moe route: %d experts, d %d", ne, d);
+  CU_OK(llb_launch(k_moe_router, dim3(ne + 1), dim3(256), (size_t)(0), s, Wr, h, d, ne, lg, rs, g_streams.stride ? Tmax : 0));
   return 0;
 }
 

@@ -17,6 +17,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // One warp per row of the pass: softmax over the ne logits, the k largest probabilities in descending order with
 // ties to the lower index, their weights divided by their sum clamped at 6.103515625e-5; slot k is the shared
 // expert (id ne) with weight sigmoid(its gate logit).
+// (wt null: the weights are not wanted.)  A round of the selection is two warp-wide reductions of integers: the probabilities are not
+// negative, so their bits order as they do.
 template <int NQ> __device__ __forceinline__ void moe_route_row(const float *l, int ne, int nk, int *ids, float *wt, int lane) {
   float p[NQ];   // experts lane, lane + 32, ...: ne <= 32 NQ
   float mx = -INFINITY;
@@ -26,46 +28,43 @@ template <int NQ> __device__ __forceinline__ void moe_route_row(const float *l, 
     p[q] = e < ne ? __ldcg(l + e) : -INFINITY;
     mx = fmaxf(mx, p[q]);
   }
+  const float gate = __ldcg(l + ne);
   mx = warp_max(mx);
   float sm = 0.0f;
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
     const int e = lane + 32 * q;
     if (e < ne) { p[q] = expf(p[q] - mx); sm += p[q]; }
-    else p[q] = -1.0f;
   }
   sm = warp_sum(sm);
   const float inv = 1.0f / sm;
+  unsigned int key[NQ];   // the probability's bits + 1; 0: none, taken, or not a number
 #pragma unroll
-  for (int q = 0; q < NQ; q++)
-    if (p[q] >= 0.0f) p[q] *= inv;
+  for (int q = 0; q < NQ; q++) {
+    const float v = p[q] * inv;
+    key[q] = lane + 32 * q < ne && v >= 0.0f ? __float_as_uint(v) + 1u : 0u;
+  }
   float s = 0.0f, mine_w = 0.0f;   // lane j keeps the weight of rank j
   int mine_id = 0;
   for (int j = 0; j < nk; j++) {
-    float bv = -1.0f;
-    int bi = 0x7fffffff;
+    unsigned int bk = 0, bi = 0x7fffffffu;
 #pragma unroll
     for (int q = 0; q < NQ; q++)
-      if (p[q] > bv) { bv = p[q]; bi = lane + 32 * q; }   // ascending q: the lane's lowest index among equals
+      if (key[q] > bk) { bk = key[q]; bi = lane + 32 * q; }   // ascending q: the lane's lowest index among equals
+    const unsigned int k = __reduce_max_sync(0xffffffffu, bk);
+    const unsigned int i = __reduce_min_sync(0xffffffffu, bk == k && k > 0 ? bi : 0x7fffffffu);
 #pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, m);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, m);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if ((bi & 31) == lane) {
-#pragma unroll
-      for (int q = 0; q < NQ; q++)
-        if (q == (bi >> 5)) p[q] = -2.0f;
-    }
+    for (int q = 0; q < NQ; q++)
+      if (i == (unsigned int)(lane + 32 * q)) key[q] = 0;
+    const float bv = k > 0 ? __uint_as_float(k - 1u) : -1.0f;
     s += bv;
-    if (j == lane) { mine_w = bv; mine_id = bi; }
+    if (j == lane) { mine_w = bv; mine_id = (int)i; }
   }
   s = s < 6.103515625e-5f ? 6.103515625e-5f : s;
-  if (lane < nk) { ids[lane] = mine_id; wt[lane] = mine_w / s; }
+  if (lane < nk) { ids[lane] = mine_id; if (wt) wt[lane] = mine_w / s; }
   if (lane == 0) {
     ids[nk] = ne;
-    wt[nk] = 1.0f / (1.0f + expf(-__ldcg(l + ne)));
+    if (wt) wt[nk] = 1.0f / (1.0f + expf(-gate));
   }
 }
 

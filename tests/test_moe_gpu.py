@@ -107,6 +107,30 @@ def test_moe_ffn_sixteen_rows_of_several_streams(pkg, packs, oracle, llb, T, k, 
         orc.close()
 
 
+@pytest.mark.parametrize("ne,top,T,de", [(300, 32, 16, 256), (5, 5, 16, 256), (257, 1, 3, 768), (1, 1, 16, 512)])
+def test_moe_ffn_units_at_their_limits(pkg, packs, oracle, llb, ne, top, T, de):
+    """The most pairs of a pass (sixteen rows of 32 experts and the shared one, more than 256 experts), every expert chosen by every
+    row (units of four rows each), hardly any shared, one expert; an expert of three super-blocks."""
+    cfg = packs.cfg_tiny_moe(n_layers=2, n_experts=ne, n_experts_used=top, d_expert=de, d_shared=de)
+    pack = packs.build_pack(cfg)
+    orc = oracle.Oracle(pack.index_text(), pack.data.numpy(), cap=8)
+    eng = pkg.llb.SpecEngine(pack, None, k=T - 1 if T <= 8 else 0, max_ctx=64, streams=1 if T <= 8 else T)
+    try:
+        h2 = np.random.default_rng(ne + T).standard_normal((T, cfg.d_model)).astype(np.float32)
+        out, ids, wt = eng.moe_ffn(1, h2)
+        for t in range(T):
+            ro, rid, rw = orc.moe_ffn(1, h2[t])
+            assert list(ids[t, :-1]) == list(rid)
+            assert np.abs(wt[t] - rw).max() < 1e-6
+            assert np.linalg.norm(out[t] - ro) / np.linalg.norm(ro) < 2e-5
+        alone, _, _ = eng.moe_ffn(1, h2[T - 1:T])
+        assert np.array_equal(alone[0].view(np.uint32), out[T - 1].view(np.uint32))
+        assert llb.lib().llb_b200_wait_errors() == 0
+    finally:
+        eng.close()
+        orc.close()
+
+
 @pytest.mark.parametrize("k", [0, 3])
 def test_tiny_moe_model_ids_match_oracle(pkg, packs, oracle, llb, k):
     """A hybrid model whose every FFN is routed: plain greedy (k = 0) and the prompt-lookup speculative loop."""
