@@ -5,8 +5,13 @@
 #include "moe.cuh"
 #include "host.cuh"
 
-// the tcgen05 kernel takes Q4_K with T <= 4 (8 plane columns)
-static bool is_g3(int fmt, int NC) { return g_llb.gemm3 && fmt == LLB_FM_Q4_K && NC == 8; }
+#define G3_SCALE 1.0
+
+// can the tcgen05 kernel take this K-split?  (a super-block of every tile for each of its groups, two stages beside the planes)
+static bool g3_fits(int fmt, int NC, int nsb, int ks) {
+  if (g_llb.gemm3 < 0 || fmt != LLB_FM_Q4_K) return false;
+  return ks >= 1 && nsb / ks >= g3_groups(NC) && g3_stages(NC, (nsb + ks - 1) / ks) >= 2;
+}
 static unsigned int *g_ffn_sync = nullptr;   // the fused FFN's grid barrier: two counters
 static unsigned int *g_g3_err = nullptr;   // device word: set when a bounded wait of a kernel ran out
 unsigned int *gemm_err_word(void) { return g_g3_err; }
@@ -46,16 +51,15 @@ template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
   return 0;
 }
 
-static int launch_three(cudaStream_t s, const GemmArgs &a) {
-  const int nsl = (a.nsb + a.ksplit - 1) / a.ksplit;
+template <int NC> static int launch_three(cudaStream_t s, const GemmArgs &a) {
+  const int nsl = (a.nsb + a.ksplit - 1) / a.ksplit, st = g3_stages(NC, nsl);
   int ntiles = 0;
   for (int i = 0; i < a.nmat; i++) ntiles += (a.m[i].rows + 127) / 128;
   int cps = g_llb.sms / a.ksplit;
   if (cps < 1) cps = 1;
   if (cps > ntiles) cps = ntiles;
-  const size_t smem = (size_t)g3_smem_bytes(nsl);
-  if (smem > G3_SMEM_MAX) return llb_fail("k_gemm3: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
-  cudaError_t e = llb_launch(k_gemm3, dim3(cps * a.ksplit), dim3(G3_BLOCK), smem, s, a, cps, g_g3_err);
+  const size_t smem = (size_t)G3_HDR + g3_xp_bytes(NC, nsl) + g3_red_bytes(NC) + (size_t)st * G3_STAGE;
+  cudaError_t e = llb_launch(k_gemm3<NC>, dim3(cps * a.ksplit), dim3(g3_threads(NC)), smem, s, a, cps, st);
   if (e != cudaSuccess) return llb_fail("k_gemm3 launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -125,9 +129,14 @@ template <int FMT, int NT> static int setup_fmt2() {
 template <int FMT> static int setup_fmt() { return setup_fmt2<FMT, 1>() || setup_fmt2<FMT, 2>() || setup_fmt2<FMT, 4>(); }
 template <int FMT> static int setup_experts() { return setup_smem(k_moe_gu<FMT, 8>) || setup_smem(k_moe_gu<FMT, 32>) || setup_smem(k_moe_dn<FMT>); }
 
+template <int NC> static int setup_three() {
+  CU_OK(cudaFuncSetAttribute(k_gemm3<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM_MAX));
+  return 0;
+}
+
 int gemm_setup(void) {
   if (setup_fmt<LLB_FM_Q4_K>() || setup_fmt<LLB_FM_Q5_K>() || setup_fmt<LLB_FM_Q6_K>() || setup_fmt<LLB_FM_Q8_0>()) return -1;
-  CU_OK(cudaFuncSetAttribute(k_gemm3, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM_MAX));
+  if (setup_three<8>() || setup_three<16>() || setup_three<32>()) return -1;
   if (setup_experts<LLB_FM_Q4_K>() || setup_experts<LLB_FM_Q5_K>() || setup_experts<LLB_FM_Q6_K>()) return -1;
   CU_OK(cudaFuncSetAttribute(k_ffn<LLB_FM_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
   CU_OK(cudaFuncSetAttribute(k_ffn<LLB_FM_Q5_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_MAX));
@@ -143,16 +152,16 @@ int gemm_setup(void) {
   return 0;
 }
 
+// the fewest K-slices that the mma.sync kernel can take: the activation slice of a CTA has to fit in shared memory, beside the usual
+// ring, or where that would take too many slices, beside the shorter one
+static int g2_least_ksplit(int fmt, int NC, int nsb) {
+  const int mx = g2_max_slice_sb(fmt, NC), most = g2_longest_slice(fmt, NC), lo = (nsb + mx - 1) / mx;
+  return lo <= GEMM_MAXSPLIT ? lo : (nsb + most - 1) / most;
+}
 int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks) {
   if (ks < 1) ks = 1;
-  if (is_g3(fmt, NC)) {
-    const int mx = g3_max_slice_sb();
-    const int lo = (nsb + mx - 1) / mx;
-    if (ks < lo) ks = lo;
-  } else {
-    // the activation slice of a CTA has to fit in shared memory: beside the usual ring, or where that would take too many
-    // slices, beside the shorter one
-    const int mx = g2_max_slice_sb(fmt, NC), most = g2_longest_slice(fmt, NC), lo = (nsb + mx - 1) / mx, least = lo <= GEMM_MAXSPLIT ? lo : (nsb + most - 1) / most;
+  if (!g3_fits(fmt, NC, nsb, ks)) {
+    const int least = g2_least_ksplit(fmt, NC, nsb);
     if (ks < least) ks = least;
   }
   if (ks > GEMM_MAXSPLIT) ks = GEMM_MAXSPLIT;
@@ -172,20 +181,24 @@ static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int 
   const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, NC / 8, tiles, nsb, ks), direct && NC >= 32 ? 3000.0 : 1200.0);
   return (stream + stage * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
+// The tcgen05 kernel's cost on the same scale (fitted to its gains over the other one, which that scale flatters): a super-block of
+// 128 rows in a CTA, the slice's activations, the pipeline's fill and the last tile's way out.
+static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
+  const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
+  return G3_SCALE * (tiles * (double)slice * (820.0 + (NC >= 32 ? 150.0 : 0.0)) * (1.0 + 0.02 * (ks - 1)) + 3000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
+}
+// Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
+static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks) {
+  if (!g3_fits(fmt, NC, nsb, ks)) return false;
+  if (g_llb.gemm3 > 0 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
+  return g3_cost(NC, ntiles, nsb, ks, g_llb.sms, false) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, g_llb.sms, false, 24.0);
+}
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
     if (gemm_fix_ksplit(fmt, NC, nsb, ks) != ks) continue;
-    const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks;
-    double cost;
-    if (is_g3(fmt, NC)) {
-      // 128-row tiles, one CTA per (tile, slice) at a time; 1.5 super-blocks of pipeline fill per tile
-      const int nt128 = (ntiles + 7) / 8;
-      cost = (double)((nt128 + cps - 1) / cps) * (slice + 1.5) * (1.0 + 0.02 * (ks - 1));
-    } else {
-      cost = gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
-    }
+    const double cost = g3_use(fmt, NC, ntiles, nsb, ks) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
   }
   return gemm_fix_ksplit(fmt, NC, nsb, best);
@@ -332,7 +345,7 @@ int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a) {
   if (gemm_prepare(fmt, a)) return -1;
   if (a.tile0[a.nmat] < 1) return 0;
   const int NT = a.xp.NC / 8;
-  if (is_g3(fmt, a.xp.NC)) return launch_three(s, a);
+  if (g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
   if (fmt == LLB_FM_Q4_K) return NT == 1 ? launch_two<LLB_FM_Q4_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q4_K, 2>(s, a) : launch_two<LLB_FM_Q4_K, 4>(s, a);
   if (fmt == LLB_FM_Q5_K) return NT == 1 ? launch_two<LLB_FM_Q5_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q5_K, 2>(s, a) : launch_two<LLB_FM_Q5_K, 4>(s, a);
   if (fmt == LLB_FM_Q6_K) return NT == 1 ? launch_two<LLB_FM_Q6_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q6_K, 2>(s, a) : launch_two<LLB_FM_Q6_K, 4>(s, a);

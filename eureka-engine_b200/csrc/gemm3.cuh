@@ -1,295 +1,339 @@
-// gemm3.cuh -- the Q4_K skinny GEMM on the fifth-generation tensor cores (tcgen05), T <= 4.
+// gemm3.cuh -- the skinny GEMM of large Q4_K launches on the fifth-generation tensor cores (tcgen05), T <= 16.
 //
-// Same arithmetic as gemm2.cuh -- 4-bit codes as fp16 subnormal integers, fp16 hi/lo activation
-// planes, sub-block scales applied to fp32 partial sums, the "min" term as one extra MMA per
-// super-block -- but the multiply runs as tcgen05.mma (M = 128 rows, N = 16, K = 16) with the weight
-// operand in TENSOR MEMORY: a thread owns one row and a pair of sub-blocks, unpacks its 32 bytes of
-// nibbles into 32 registers (five instructions per four) and stores them with tcgen05.st; one thread
-// issues the 17 MMAs of a 128-row x 256-column super-block; the accumulators come back with
-// tcgen05.ld, one row per thread, so the scale step is 18 FMAs per thread and super-block.  The mma.sync
-// kernel spends 380 warp instructions per 16 rows x 256 columns; this one about 250 for the same bytes.
+// The mma.sync kernel (gemm2.cuh) is bound by its instructions, not by the weights' bytes: gate|up of the 27B shape takes as
+// long when its weights come from L2 as from HBM (23 us; 15.4 at the measured copy rate), and the work around its
+// MMAs grows with the rows (60 us at sixteen).  Here
+//   * the multiply is tcgen05.mma (M = 128 weight rows, N = 16 or 32 plane columns, K = 16) with the weight operand in TENSOR
+//     MEMORY, which costs the SM's issue slots nothing and does not grow with the rows;
+//   * the six-bit scale is multiplied into the code: sc * q <= 63 * 15 is an exact fp16 number, so a whole super-block of 256
+//     columns accumulates into ONE fp32 accumulator and d comes in once per super-block.  A row of a super-block is 32 words,
+//     nine instructions each for eight products: about 200 warp instructions a 16 x 256 tile against 351;
+//   * the "min" term is one extra MMA a super-block into an accumulator of its own, as in gemm2.cuh.
+// gate|up, operator alone, cold weights: 28.2 -> 24.5 us at one row, 28.2 -> 27 at four, 37.3 -> 32 at eight, 60 -> 46.5 at
+// sixteen.  What is left: the activations, which every SM reads from L2 at about 10 bytes a cycle (4 us for four rows of 5120
+// columns; cp.async or plain loads, in one order or a different one in every CTA), the groups' chains (2300 cycles a super-block, three groups),
+// and tiles of 128 rows that do not divide evenly.
 //
-//   TMEM columns (512 allocated):  A buffers at 0 and 136 (128 columns of codes + 8 of mins),
-//   D buffers at 272 and 376.  Issuing a tcgen05.mma costs one thread about 100 cycles, so four warps
-//   issue, each the four MMAs of one sub-block pair (the last also the min term).  The MMA's N is 16 but
-//   only 8 columns are real (4 tokens x hi/lo): issuer i accumulates sub-block 2i at D + 24i and
-//   2i + 1 at D + 24i + 8, whose first MMA overwrites the unused upper half of the one before (the MMAs
-//   of one thread execute in issue order); the min term sits at D + 88.
-//   Shared memory: activation planes of the CTA's K-slice as K-major core matrices
-//   [k/8][column][8 halves] (the planes' stored k-order 0 2 1 3 4 6 5 7 is the order the unpack
-//   produces), the sub-block means for the min term, a ring of raw 128-row x 144-byte stages filled
-//   with cp.async, and the buffer the four threads of a row reduce through.
-//   Every wait on an mbarrier is bounded; a wait that runs out sets *err and the kernel drains, frees
-//   its tensor memory and returns.
+// Roles of a CTA (one an SM): GROUPS of four warps, a thread a weight row, take the super-blocks of the CTA's tiles in turn:
+// unpack into the group's operand buffer, and before the next one read the accumulators of the last and scale them into the
+// row's sums.  A group has its own operand and accumulators, so groups wait for nothing but their own MMAs; a warp a group issues
+// them (all lanes walk, an elected one issues: descriptors stay in uniform registers; one warp for all groups paced the
+// kernel, 990 cycles a super-block, a third of them in waits that find their phase complete), one requests the weights (two
+// super-blocks of eight 16-row tiles a stage, a bulk copy a tile).  At the end of a tile the other groups leave their sums in shared memory
+// and the group that came last adds them in order and writes.
+//   Tensor memory (512 columns): the groups' operands (128 columns of products, 8 of mins), then their accumulators (N + N).
+//   Three groups where that fits (N = 16), two at N = 32.
+//   Shared memory: activation planes of the K-slice as K-major core matrices [k / 8][column][8 halves] (their k-order 0 2 1 3 4 6
+//   5 7 is the one the unpack produces), the sub-block means likewise, the groups' sums, the ring.
+//   N is 16 at least, and with 8 plane columns the upper half of an accumulator is whatever the next k-group's columns give; nobody
+//   reads it.
+// Every wait is bounded; one that runs out sets *err, all roles then run through without waiting, copies in flight get time to
+// land, tensor memory is freed and the kernel returns.
 #pragma once
-#include "gemm.cuh"
-#include "tc5.cuh"
+#include "gemm2.cuh"
 static_assert(GEMM_MAXMAT == 4, "k_gemm3 finds a tile's matrix with three compares");
 
-#define G3_THREADS 512        // worker threads; four more warps issue the MMAs
-#define G3_BLOCK (G3_THREADS + 128)
-#define G3_STAGES 6
-#define G3_STAGE_BYTES (128 * 144)
-#define G3_RED_BYTES (5 * 128 * 8 * 4)   // four partial sums per row and column, and the row's min terms
-#define G3_HDR_BYTES 128
-#define G3_SMEM_MAX 232448
-#define G3_TMEM_COLS 512
+#define G3_HDR 256
+#define G3_SMEM_MAX 231424
 #define G3_A_COLS 136
-#define G3_D0 272
-#define G3_D_COLS 104
-#define G3_IDESC 0x08040010u   // kind::f16: D f32, A/B f16 K-major, N = 16, M = 128
+#define G3_CH 2                // super-blocks a copy brings
+#define G3_STAGE (8 * G3_CH * tile_bytes(LLB_FM_Q4_K))
+__host__ __device__ constexpr int g3_groups(int NC) { return NC <= 16 ? 3 : 2; }
+__host__ __device__ constexpr int g3_n(int NC) { return NC <= 16 ? 16 : 32; }
+__host__ __device__ constexpr int g3_threads(int NC) { return g3_groups(NC) * 160 + 32; }
+__host__ __device__ constexpr int g3_red_bytes(int NC) { return (NC <= 16 ? 2 : 1) * (g3_groups(NC) - 1) * 128 * NC * 4; }
+// planes and means of a K-slice of nsl super-blocks (and what the MMAs read beyond the last column)
+__host__ __device__ inline int g3_xp_bytes(int NC, int nsl) { return nsl * NC * (512 + 32) + 512; }
+__host__ __device__ inline int g3_stages(int NC, int nsl) {
+  const int left = G3_SMEM_MAX - G3_HDR - g3_red_bytes(NC) - g3_xp_bytes(NC, nsl), st = left / G3_STAGE;
+  return st > 4 ? 4 : st;
+}
+__host__ __device__ constexpr uint32_t g3_idesc(int N) { return 0x08000010u | ((uint32_t)(N >> 3) << 17); }   // kind::f16: D f32, A / B f16 K-major, M = 128
 
-// bytes of shared memory for a K-slice of nsl super-blocks (NC = 8 activation columns)
-__host__ __device__ inline int g3_xp_bytes(int nsl) { return nsl * (32 * 8 * 16 + 2 * 8 * 16) + 256; }
-inline int g3_smem_bytes(int nsl) { return G3_HDR_BYTES + g3_xp_bytes(nsl) + G3_RED_BYTES + G3_STAGES * G3_STAGE_BYTES; }
-inline int g3_max_slice_sb() { return (G3_SMEM_MAX - G3_HDR_BYTES - 256 - G3_RED_BYTES - G3_STAGES * G3_STAGE_BYTES) / (32 * 8 * 16 + 2 * 8 * 16); }
-
-__device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(G3_THREADS) : "memory"); }
-__device__ __forceinline__ void quarter_sync(int q) { asm volatile("bar.sync %0, 128;" ::"r"(2 + q) : "memory"); }
-
-__global__ void __launch_bounds__(G3_BLOCK, 1) k_gemm3(const GemmArgs a, const int cps, unsigned int *__restrict__ err) {
+template <int NC>
+__global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, const int cps, const int st) {
+  constexpr int NG = g3_groups(NC), N = g3_n(NC), TB = tile_bytes(LLB_FM_Q4_K), RPB = NC <= 16 ? 2 : 1;
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q = warp & 3, c = (warp >> 2) & 3, r = 32 * q + lane;   // TMEM lane quarter, sub-block pair, row of the tile
   const int ks = blockIdx.x % a.ksplit, ci = blockIdx.x / a.ksplit;
   const int sb0 = (int)(((long long)ks * a.nsb) / a.ksplit), nsl = (int)(((long long)(ks + 1) * a.nsb) / a.ksplit) - sb0;
-  uint32_t *tmem_slot = (uint32_t *)(smem + 40);
-  volatile uint32_t *dead = (volatile uint32_t *)(smem + 44);
-  uint8_t *Bp = smem + G3_HDR_BYTES, *Bm = Bp + (size_t)nsl * 4096 + 128;
-  float *red = (float *)(Bm + (size_t)nsl * 256 + 128);
-  uint8_t *ring = (uint8_t *)red + G3_RED_BYTES;
-  // barriers: D_full[2] at +0, +8 (one commit per issuing warp), A_full[2] at +24, +32 (16 worker warps)
-  const uint32_t bar_s = smem_u32(smem), Bp_s = smem_u32(Bp), Bm_s = smem_u32(Bm);
-  auto dfull = [&](int i) { return bar_s + 8u * (uint32_t)i; };
-  auto afull = [&](int i) { return bar_s + 24u + 8u * (uint32_t)i; };
+  // header: raw_full[4] +0, raw_empty[4] +32, a_full[3][2] +64, d_full[3] +112, red_full[2] +136, red_empty[2] +152, tmem +168, dead +172, xp_full +176
+  const uint32_t bar_s = smem_u32(smem);
+  auto raw_full = [&](int i) { return bar_s + 8u * i; };
+  auto raw_empty = [&](int i) { return bar_s + 32u + 8u * i; };
+  auto a_full = [&](int g, int h) { return bar_s + 64u + 16u * g + 8u * h; };
+  auto d_full = [&](int g) { return bar_s + 112u + 8u * g; };
+  auto red_full = [&](int p) { return bar_s + 136u + 8u * p; };
+  auto red_empty = [&](int p) { return bar_s + 152u + 8u * p; };
+  const uint32_t xp_full = bar_s + 176u;
+  uint32_t *tmem_slot = (uint32_t *)(smem + 168);
+  volatile uint32_t *dead = (volatile uint32_t *)(smem + 172);
+  uint8_t *Bp = smem + G3_HDR, *Bm = Bp + (size_t)nsl * NC * 512 + 256;
+  float *red = (float *)(smem + G3_HDR + g3_xp_bytes(NC, (a.nsb + a.ksplit - 1) / a.ksplit));
+  uint8_t *ring = (uint8_t *)red + g3_red_bytes(NC);
+  const uint32_t Bp_s = smem_u32(Bp), Bm_s = smem_u32(Bm), ring_s = smem_u32(ring);
   int t128[GEMM_MAXMAT + 1];
   t128[0] = 0;
 #pragma unroll
-  for (int m = 0; m < GEMM_MAXMAT; m++) t128[m + 1] = t128[m] + (m < a.nmat ? (a.m[m].rows + 127) / 128 : 0);
-  const int ntiles = t128[GEMM_MAXMAT];
-  const int my_tiles = ci < ntiles ? (ntiles - ci + cps - 1) / cps : 0, n_items = my_tiles * nsl;
-
-  // The four warps of a lane quarter load the quarter's 32 rows x 144 bytes of a super-block together:
-  // 288 sixteen-byte pieces, piece i = tq + 128 * it of thread tq = 32 c + lane, nine consecutive pieces per row.
-  const int tq = 32 * c + lane;
-  uint8_t *qring = ring + (size_t)q * 4608;
-  const uint32_t qring_s = smem_u32(qring);
-  int p_tile = ci, p_c = 0, p_stage = 0, p_left = n_items;
-  const uint8_t *p_W = nullptr;
-  uint32_t p_off[3];
-  auto plan_tile = [&](int tile) {
-    if (tile >= ntiles) return;
-    const int m = (tile >= t128[1]) + (tile >= t128[2]) + (tile >= t128[3]);   // t128[k] = ntiles beyond the last matrix
-    const int row0 = (tile - (m == 0 ? 0 : m == 1 ? t128[1] : m == 2 ? t128[2] : t128[3])) * 128 + 32 * q, rows = a.m[m].rows;
-    p_W = a.m[m].W + (size_t)sb0 * tile_bytes(LLB_FM_Q4_K);
-#pragma unroll
-    for (int it = 0; it < 3; it++) {
-      const int i = tq + 128 * it, rr = i / 9, pp = i - rr * 9;
-      const int r = min(row0 + rr, rows - 1);
-      p_off[it] = (uint32_t)(r >> 4) * (uint32_t)(a.nsb * tile_bytes(LLB_FM_Q4_K)) + (r & 15) * 144 + pp * 16;
-    }
+  for (int m = 0; m < GEMM_MAXMAT; m++) t128[m + 1] = t128[m] + (m < a.nmat ? (a.m[m].rows + 127) >> 7 : 0);
+  const int ntiles = t128[GEMM_MAXMAT], my_tiles = ci < ntiles ? (ntiles - ci + cps - 1) / cps : 0, nch = (nsl + G3_CH - 1) / G3_CH;
+  // first row of tile t in its matrix m
+  auto locate = [&](int t, int &m) {
+    m = (t >= t128[1]) + (t >= t128[2]) + (t >= t128[3]);   // t128[k] = ntiles beyond the last matrix
+    return (t - (m == 0 ? 0 : m == 1 ? t128[1] : m == 2 ? t128[2] : t128[3])) * 128;
   };
-  auto issue = [&]() {
-    if (p_left > 0) {
-      const uint8_t *src = p_W + (size_t)p_c * tile_bytes(LLB_FM_Q4_K);
-      const uint32_t dst = qring_s + p_stage * G3_STAGE_BYTES + tq * 16;
-      cp_async16(dst, src + p_off[0]);
-      cp_async16(dst + 2048, src + p_off[1]);
-      if (tq < 32) cp_async16(dst + 4096, src + p_off[2]);
-      p_left--;
-      if (++p_c == nsl) { p_c = 0; p_tile += cps; plan_tile(p_tile); }
-      p_stage = p_stage + 1 == G3_STAGES ? 0 : p_stage + 1;
-    }
-    cp_async_commit();
-  };
-  const bool worker = warp < G3_THREADS / 32;
   pdl_trigger();
-  if (worker) {
-    plan_tile(p_tile);
-#pragma unroll 1
-    for (int s = 0; s < G3_STAGES - 1; s++) issue();   // weights depend on no kernel: in flight before the wait
-  }
   if (tid == 0) {
-    mbar_init(dfull(0), 4);
-    mbar_init(dfull(1), 4);
-    mbar_init(afull(0), 16);
-    mbar_init(afull(1), 16);
+    for (int i = 0; i < 4; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), 4 * G3_CH); }
+    for (int g = 0; g < NG; g++) { mbar_init(a_full(g, 0), 4); mbar_init(a_full(g, 1), 4); mbar_init(d_full(g), 1); }
+    for (int p = 0; p < 2; p++) { mbar_init(red_full(p), 4 * (NG - 1)); mbar_init(red_empty(p), 4); }
+    mbar_init(xp_full, NG * 128);
     *dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)G3_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  pdl_wait();
-  if (worker) {
-    const int per_col = nsl * 32;   // k-groups of the slice
-    for (int i = tid; i < 8 * per_col; i += G3_THREADS) {
-      const int n = i / per_col, g = i - n * per_col;
-      cp_async16(Bp_s + (g * 8 + n) * 16, (const uint8_t *)(a.xp.xh + (size_t)n * a.K + (size_t)sb0 * 256) + g * 16);
-    }
-    for (int i = tid; i < nsl * 16; i += G3_THREADS) {   // (sb, n, h): 16 halves of means -> chunk h of column n
-      const int sb = i >> 4, n = (i >> 1) & 7, h = i & 1;
-      cp_async16(Bm_s + ((sb * 2 + h) * 8 + n) * 16, (const uint8_t *)(a.xp.xsf + ((size_t)(sb0 + sb) * 8 + n) * 16) + h * 16);
-    }
-    if (tid < 8) *(uint4 *)(Bp + (size_t)nsl * 4096 + tid * 16) = make_uint4(0, 0, 0, 0);
-    else if (tid < 16) *(uint4 *)(Bm + (size_t)nsl * 256 + (tid - 8) * 16) = make_uint4(0, 0, 0, 0);
-    cp_async_commit();
-    cp_async_wait<0>();
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read these bytes through the async proxy
   }
   t5_fence_before();
   __syncthreads();
   t5_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  if (!worker) {
-    // ---- four issuing warps: lane 0 of warp 16 + i feeds the tensor core sub-block pair i ---------
-    if (lane == 0) {
-      const int i4 = warp - G3_THREADS / 32;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      int c_c = 0;
-      for (int s = 0; s < n_items; s++) {
-        const int buf = s & 1;
-        if (!*dead && !mbar_wait(afull(buf), (uint32_t)(s >> 1) & 1u)) {
-          *dead = 1;
-          if (err) atomicExch(err, 1u);
-        }
-        t5_fence_after();
-        const uint32_t abuf = tmem_base + (uint32_t)(buf * G3_A_COLS + 32 * i4), dbuf = tmem_base + (uint32_t)(G3_D0 + buf * G3_D_COLS + 24 * i4);
-        const uint64_t bd = g3_desc(Bp_s + c_c * 4096 + i4 * 1024, 128, 128);   // + 8 per 128 bytes: the address field counts 16-byte units
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-          for (int u = 0; u < 2; u++) t5_mma_f16_ts(dbuf + 8 * h, abuf + 16 * h + 8 * u, bd + (uint64_t)((4 * h + 2 * u) * 8), G3_IDESC, u);
-        if (i4 == 3) t5_mma_f16_ts(dbuf + 16, tmem_base + (uint32_t)(buf * G3_A_COLS + 128), g3_desc(Bm_s + c_c * 256, 128, 128), G3_IDESC, 0);
-        t5_commit(dfull(buf));
-        if (++c_c == nsl) c_c = 0;
-      }
-      // nothing of this CTA may still be running on the tensor core when its tensor memory is freed
-      if (n_items > 0 && !*dead) mbar_wait(dfull((n_items - 1) & 1), (uint32_t)((n_items - 1) >> 1) & 1u);
+  const uint32_t tmem = *tmem_slot;
+  auto wait = [&](uint32_t bar, uint32_t parity) {   // gives up for the whole CTA
+    for (uint32_t n = 0; !mbar_wait(bar, parity, 4); n += 4) {
+      if (*dead) return;
+      if (n >= T5_WAIT_LIMIT) { *dead = 1; if (a.err) atomicExch(a.err, 1u); return; }
     }
-  } else {
-    // ---- 512 workers: unpack super-block s into tensor memory, scale super-block s - 1 out of it ---
+  };
+
+  if (warp < 4 * NG) {
+    // ---- workers: group g, row r of the tile ----
+    const int g = warp >> 2, q = warp & 3, r = 32 * q + lane;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
-    float acc[8], accm[2] = {0.0f, 0.0f};
+    const uint32_t abuf = tmem + lane_off + (uint32_t)(g * G3_A_COLS), dbuf = tmem + lane_off + (uint32_t)(NG * G3_A_COLS + g * 2 * N);
+    const uint32_t roff = (uint32_t)(r >> 4) * (G3_CH * TB) + (r & 15) * tile_row(LLB_FM_Q4_K);
+    float acc[NC];
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc[j] = 0.0f;
-    float s0_p = 0.0f, s1_p = 0.0f, dm_p = 0.0f;
-    int c_stage = 0;             // ring stage of the item being unpacked
-    int e_tile = ci, e_c = 0;    // the item whose accumulators are read (one behind)
-#pragma unroll 1
-    for (int s = 0; s <= n_items; s++) {
-      const int buf = s & 1;
-      float s0 = 0.0f, s1 = 0.0f, dm = 0.0f;
-      if (s < n_items) {
-        cp_async_wait<G3_STAGES - 2>();   // this thread's pieces of item s have landed
-        quarter_sync(q);                  // ... and those of the quarter's other three warps; they are done with item s - 1
-        issue();                          // item s + G3_STAGES - 1 into the stage item s - 1 left
-        const uint8_t *rowp = qring + (size_t)c_stage * G3_STAGE_BYTES + lane * 144;
-        const uint4 hdr = *(const uint4 *)rowp, qa = *(const uint4 *)(rowp + 16 + 32 * c), qb = *(const uint4 *)(rowp + 32 + 32 * c);
-        c_stage = c_stage + 1 == G3_STAGES ? 0 : c_stage + 1;
-        uint32_t sc0, sc1, mn0, mn1;
-        if (c < 2) {
-          const uint32_t sv = hdr.y >> (16 * c), mv = hdr.z >> (16 * c);
-          sc0 = sv & 63; sc1 = (sv >> 8) & 63; mn0 = mv & 63; mn1 = (mv >> 8) & 63;
-        } else {
-          const uint32_t hv = hdr.w >> (16 * (c - 2)), lo = hdr.y >> (16 * (c - 2)), mi = hdr.z >> (16 * (c - 2));
-          sc0 = (hv & 15) | ((lo >> 2) & 0x30); sc1 = ((hv >> 8) & 15) | ((lo >> 10) & 0x30);
-          mn0 = ((hv >> 4) & 15) | ((mi >> 2) & 0x30); mn1 = ((hv >> 12) & 15) | ((mi >> 10) & 0x30);
+    for (int j = 0; j < NC; j++) acc[j] = 0.0f;
+    float d_p = 0.0f, dm_p = 0.0f;      // scales of the super-block whose accumulators are read next
+    int ti = 0, c = g;                  // the item: tile of this CTA, super-block of the slice (nsl >= NG)
+    int it = 0, ti_p = 0;               // items so far; the tile of the last one
+    int slot = (g / G3_CH) % st;        // the item's stage, and the parity of its use
+    uint32_t rpar = (uint32_t)((g / G3_CH) / st) & 1u;
+    bool staged = false;
+    // the accumulators of the last item into the row's sums
+    auto drain = [&]() {
+      wait(d_full(g), (uint32_t)(it - 1) & 1u);
+      t5_fence_after();
+#pragma unroll
+      for (int j0 = 0; j0 < NC; j0 += 8) {
+        float v[8], p[8];
+        t5_ld8(dbuf + j0, v);
+        t5_ld8(dbuf + N + j0, p);
+        t5_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[j0 + j] += d_p * v[j] - dm_p * p[j];
+      }
+      t5_fence_before();
+    };
+    // A finished tile: the group that has its last super-block (which comes here last) adds the others' sums to its own in group
+    // order, then hi + lo / 2048.  (Nothing but loads, sums and stores: with the matrix's fields read at every store a tile of
+    // sixteen rows took 4700 cycles.)
+    auto flush = [&](int t) {
+      const int p = RPB == 2 ? t & 1 : 0, n = RPB == 2 ? t >> 1 : t, og = ((t + 1) * nsl - 1) % NG;      // buffer, its use so far; that group
+      if (g != og) {
+        if (n > 0) wait(red_empty(p), (uint32_t)(n - 1) & 1u);
+        float *w = red + (size_t)(p * (NG - 1) + (g > og ? g - 1 : g)) * 128 * NC + r;
+#pragma unroll
+        for (int j = 0; j < NC; j++) w[j * 128] = acc[j];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(red_full(p));
+      } else {
+        int m;
+        const int row = locate(ci + t * cps, m) + r, T = a.T, os = a.m[m].ostride, rows = a.m[m].rows, per = a.m[m].tok_per, tst = a.m[m].tok_stride, tadd = a.m[m].tok_add;
+        float *out = a.m[m].out + (size_t)ks * a.m[m].split_stride + row;
+        const int *ts = a.m[m].tok_slot;
+        wait(red_full(p), (uint32_t)n & 1u);
+#pragma unroll
+        for (int k = 0; k < NG - 1; k++) {
+          const float *w = red + (size_t)(p * (NG - 1) + k) * 128 * NC + r;
+#pragma unroll
+          for (int j = 0; j < NC; j++) acc[j] += w[j * 128];
         }
-        const float d = h2f_bits(hdr.x & 0xffffu), dmin = h2f_bits(hdr.x >> 16);
-        s0 = d * (float)sc0 * TWO24; s1 = d * (float)sc1 * (TWO24 * 0.0625f); dm = dmin * 32.0f;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(red_empty(p));
+        if (a.planes == 2) {
+#pragma unroll
+          for (int j = 0; j < NC / 2; j++) acc[j] += acc[j + NC / 2] * XP_LO_INV;
+        }
+        if (row < rows) {
+          if (!ts) {
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+              if (j < T) *out = acc[j];
+              out += os;
+            }
+          } else {
+            int blk[NC];                        // every slot's load in flight at once
+#pragma unroll
+            for (int j = 0; j < NC; j++) { const int z = per > 0 ? j / per : 0; blk[j] = j < T ? ts[(size_t)z * tst + (j - z * per)] + z * tadd : 0; }
+#pragma unroll
+            for (int j = 0; j < NC; j++) if (j < T) out[(size_t)blk[j] * os] = acc[j];
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NC; j++) acc[j] = 0.0f;
+    };
+#pragma unroll 1
+    while (ti < my_tiles) {
+      const int sub = c % G3_CH;
+      wait(raw_full(slot), rpar);
+      const uint8_t *row = ring + (size_t)slot * G3_STAGE + roff + sub * TB;
+      const uint4 hd = *(const uint4 *)row;
+      uint32_t scA, scB, mnA, mnB;
+      k4_scales(hd.y, hd.z, hd.w, scA, scB, mnA, mnB);
+#pragma unroll
+      for (int gq = 0; gq < 4; gq++) {            // 64 columns: sub-block 2 gq in the low nibbles, 2 gq + 1 in the high ones
+        const uint8_t *qs = row + 16 + 32 * gq;
+        const uint4 qa = *(const uint4 *)qs, qb = *(const uint4 *)(qs + 16);
         const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+        // the scales as fp16 (0x6400 | s is 1024 + s) times 2^5 for the low nibbles and 2 for the high ones, which stay four bits
+        // up: q 2^-24 * s 2^5 = 16 q 2^-24 * s 2 = s q 2^-19, exact
+        const uint32_t sw = gq < 2 ? scA : scB;
+        const uint32_t L = g2_hfma2(__byte_perm(sw, 0x64646464u, gq & 1 ? 0x4242 : 0x4040), 0x50005000u, 0xf800f800u);
+        const uint32_t H = g2_hfma2(__byte_perm(sw, 0x64646464u, gq & 1 ? 0x4343 : 0x4141), 0x40004000u, 0xe800e800u);
         uint32_t v[32];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          const uint32_t w8 = w[i] >> 8;
-          v[2 * i] = w[i] & 0x000f000fu; v[2 * i + 1] = w8 & 0x000f000fu;            // sub-block 2c: low nibbles
-          v[16 + 2 * i] = w[i] & 0x00f000f0u; v[16 + 2 * i + 1] = w8 & 0x00f000f0u;  // sub-block 2c+1: high nibbles, x16
+          const uint32_t y = w[i] >> 8;
+          v[2 * i] = g2_hmul2(w[i] & 0x000f000fu, L); v[2 * i + 1] = g2_hmul2(y & 0x000f000fu, L);
+          v[16 + 2 * i] = g2_hmul2(w[i] & 0x00f000f0u, H); v[17 + 2 * i] = g2_hmul2(y & 0x00f000f0u, H);
         }
-        // A[buf] is free: this thread waited for the MMAs of item s - 2 when it read their accumulators
-        const uint32_t abuf = tmem_base + lane_off + (uint32_t)(buf * G3_A_COLS);
-        t5_st32(abuf + 32 * c, v);
-        // the pair's mins as fp16 numbers (0x6400 | m is 1024 + m): m against the means' hi halves, m / 2048 against
-        // their lo halves, which are stored times 2048
-        const uint32_t mt = mn0 | (mn1 << 16) | 0x64006400u;
-        t5_st2(abuf + 128 + 2 * c, g2_hfma2(mt, 0x3c003c00u, 0xe400e400u), g2_hfma2(mt, 0x10001000u, 0xb800b800u));
-        t5_wait_st();
-        t5_fence_before();
-        __syncwarp();
-        // also says: this warp has read the accumulators of item s - 2, whose buffer item s takes
-        if (lane == 0) mbar_arrive(afull(buf));
-      } else {
-        cp_async_wait<0>();
-      }
-      if (s >= 1) {
-        const int it = s - 1, eb = it & 1;
-        if (!*dead && !mbar_wait(dfull(eb), (uint32_t)(it >> 1) & 1u)) {
-          *dead = 1;
-          if (err) atomicExch(err, 1u);
-        }
-        t5_fence_after();
-        float v[16], vm[2];
-        const uint32_t dcol = tmem_base + lane_off + (uint32_t)(G3_D0 + eb * G3_D_COLS);
-        t5_ld16(dcol + 24 * c, v);
-        t5_ld2(dcol + 88 + 2 * c, vm);
-        t5_wait_ld();
-        t5_fence_before();
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] += s0_p * v[j] + s1_p * v[8 + j];
-        accm[0] += dm_p * vm[0];
-        accm[1] += dm_p * vm[1];
-        if (++e_c == nsl) {
-          // tile done: the four threads of a row add up through shared memory
-          // (the min term of a column is subtracted after the four partial sums are added, so that a
-          // column's result does not depend on which column of the launch it is)
-          float4 *rp = (float4 *)(red + ((size_t)c * 128 + r) * 8);
-          rp[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-          rp[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-          *(float2 *)(red + (size_t)(4 * 128 + r) * 8 + 2 * c) = make_float2(accm[0], accm[1]);
-          quarter_sync(q);
-          if (c == 0) {
-            float sum[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) sum[j] = 0.0f;
-#pragma unroll
-            for (int cc = 0; cc < 4; cc++) {
-              const float4 x0 = *(const float4 *)(red + ((size_t)cc * 128 + r) * 8), x1 = *(const float4 *)(red + ((size_t)cc * 128 + r) * 8 + 4);
-              sum[0] += x0.x; sum[1] += x0.y; sum[2] += x0.z; sum[3] += x0.w; sum[4] += x1.x; sum[5] += x1.y; sum[6] += x1.z; sum[7] += x1.w;
-            }
-            {
-              const float4 m0 = *(const float4 *)(red + (size_t)(4 * 128 + r) * 8), m1 = *(const float4 *)(red + (size_t)(4 * 128 + r) * 8 + 4);
-              sum[0] -= m0.x; sum[1] -= m0.y; sum[2] -= m0.z; sum[3] -= m0.w; sum[4] -= m1.x; sum[5] -= m1.y; sum[6] -= m1.z; sum[7] -= m1.w;
-            }
-            const int m = (e_tile >= t128[1]) + (e_tile >= t128[2]) + (e_tile >= t128[3]);
-            const GemmMat &M = a.m[m];
-            const int row = (e_tile - (m == 0 ? 0 : m == 1 ? t128[1] : m == 2 ? t128[2] : t128[3])) * 128 + r;
-            if (row < M.rows) {
-              float *out = M.out + (size_t)ks * M.split_stride;
-#pragma unroll
-              for (int t = 0; t < 8; t++) {
-                if (t < a.T && (a.planes == 1 || t < 4)) {
-                  const float val = a.planes == 2 ? sum[t & 3] + sum[4 + (t & 3)] * XP_LO_INV : sum[t];
-                  out[(size_t)gemm_out_block(M, t) * M.ostride + row] = val;
-                }
-              }
-            }
+        if (gq == 0) {
+          // the operand buffer and the accumulators are free once the last item's MMAs are done and its sums are read
+          if (it > 0) {
+            drain();
+            if (ti != ti_p) flush(ti_p);
           }
-          quarter_sync(q);   // the quarter's part of red is free again
+          // the mins as fp16 numbers: m against the means' hi halves, m / 2048 against their lo halves, which are stored times 2048
+          uint32_t mm[8];
 #pragma unroll
-          for (int j = 0; j < 8; j++) acc[j] = 0.0f;
-          accm[0] = accm[1] = 0.0f;
-          e_c = 0;
-          e_tile += cps;
+          for (int j = 0; j < 4; j++) {
+            const uint32_t at = __byte_perm(j < 2 ? mnA : mnB, 0x64646464u, (j & 1) ? 0x4342u : 0x4140u);
+            mm[2 * j] = g2_hfma2(at, 0x3c003c00u, 0xe400e400u); mm[2 * j + 1] = g2_hfma2(at, 0x10001000u, 0xb800b800u);
+          }
+          t5_st8(abuf + 128, mm);
+        }
+        t5_st32(abuf + 32 * gq, v);
+        if (gq & 1) {
+          t5_wait_st();
+          t5_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(a_full(g, gq >> 1));
         }
       }
-      s0_p = s0; s1_p = s1; dm_p = dm;
+      if (lane == 0) mbar_arrive_n(raw_empty(slot), c + 1 == nsl && !sub ? G3_CH : 1);   // (a stage with one super-block stands for two)
+      d_p = h2f_bits(hd.x & 0xffffu) * 524288.0f; dm_p = h2f_bits(hd.x >> 16) * 32.0f;
+      ti_p = ti;
+      it++;
+      {
+        // NG super-blocks on: as many stages as chunk boundaries lie between (a tile's last chunk may hold one)
+        int step = -(c / G3_CH);
+        c += NG;
+        if (c >= nsl) { c -= nsl; ti++; step += nch; }
+        slot += step + c / G3_CH;
+        if (slot >= st) { slot -= st; rpar ^= 1u; }
+      }
+      if (!staged) {
+        // ---- the activation slice: eight pieces of sixteen bytes in flight a thread ----
+        staged = true;
+        pdl_wait();
+        const int half = NC / 2, T = a.T, np = nsl * 32 * NC, nm = nsl * 2 * NC;
+        const bool two = a.planes == 2;
+        const uint8_t *xh = (const uint8_t *)(a.xp.xh + (size_t)sb0 * 256), *xf = (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
+        const size_t cs = (size_t)a.K * 2;
+        auto live = [&](int col) { return (two && col >= half ? col - half : col) < T; };
+        // (four k-groups of eight columns a warp: whole sectors of the source, whole rows of core matrices at the destination)
+#pragma unroll 1
+        for (int i0 = tid; i0 < np; i0 += 8 * NG * 128) {
+          uint4 x[8];
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            const int i = i0 + u * NG * 128, blk = i >> 5, col = blk % (NC / 8) * 8 + (i & 7), kg = blk / (NC / 8) * 4 + ((i >> 3) & 3);
+            x[u] = i < np && live(col) ? __ldcg((const uint4 *)(xh + col * cs + kg * 16)) : make_uint4(0, 0, 0, 0);
+          }
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            const int i = i0 + u * NG * 128, blk = i >> 5, col = blk % (NC / 8) * 8 + (i & 7), kg = blk / (NC / 8) * 4 + ((i >> 3) & 3);
+            if (i < np) *(uint4 *)(Bp + (kg * NC + col) * 16) = x[u];
+          }
+        }
+#pragma unroll 1
+        for (int i = tid; i < nm; i += NG * 128) {   // (super-block, column, half of its means)
+          const int sb = i / (2 * NC), col = (i >> 1) % NC, h = i & 1;
+          if (live(col)) *(uint4 *)(Bm + ((sb * 2 + h) * NC + col) * 16) = __ldcg((const uint4 *)(xf + ((size_t)sb * NC + col) * 32 + h * 16));
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read these bytes through the async proxy
+        mbar_arrive(xp_full);
+      }
+    }
+    if (it > 0) { drain(); flush(ti_p); }
+  } else if (warp == 4 * NG) {
+    // ---- weights: lane t requests the t-th 16-row tile of every chunk ----
+    int slot = 0;
+    uint32_t par = 1;                   // a fresh barrier's "previous" phase is complete
+    for (int t = 0; t < my_tiles; t++) {
+      int m;
+      const int row0 = locate(ci + t * cps, m), have = min(8, ((a.m[m].rows + 15) >> 4) - (row0 >> 4));
+      const uint8_t *src = a.m[m].W + ((size_t)((row0 >> 4) + lane) * a.nsb + sb0) * TB;
+      for (int k = 0; k < nch; k++) {
+        const int n = min(G3_CH, nsl - k * G3_CH);
+        wait(raw_empty(slot), par);
+        if (!*dead) {
+          if (lane == 0) mbar_expect(raw_full(slot), (uint32_t)(have * n * TB));
+          __syncwarp();
+          if (lane < have) bulk_load(ring_s + slot * G3_STAGE + lane * (G3_CH * TB), src + (size_t)k * G3_CH * TB, (uint32_t)(n * TB), raw_full(slot));
+        }
+        __syncwarp();
+        if (++slot == st) { slot = 0; par ^= 1u; }
+      }
+    }
+  } else {
+    // ---- the tensor core: a warp issues a group's MMAs ----
+    const int g = __shfl_sync(0xffffffffu, warp - 4 * NG - 1, 0);
+    const bool el = t5_elect();
+    const uint32_t ab = tmem + (uint32_t)(g * G3_A_COLS), db = tmem + (uint32_t)(NG * G3_A_COLS + g * 2 * N);
+    const int items = my_tiles * nsl;
+    int c = g;
+    uint32_t par = 0;
+    for (int s = g; s < items; s += NG) {
+      if (s == g) wait(xp_full, 0);
+      const uint64_t bd = g3_desc(Bp_s + c * NC * 512, NC * 16, 128), md = g3_desc(Bm_s + c * NC * 32, NC * 16, 128);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        wait(a_full(g, h), par);
+        t5_fence_after();
+        if (el) {
+          if (h == 0) t5_mma_f16_ts(db + N, ab + 128, md, g3_idesc(N), 0);
+#pragma unroll
+          for (int k = 0; k < 8; k++) t5_mma_f16_ts(db, ab + 64 * h + 8 * k, bd + (uint64_t)((8 * h + k) * 2 * NC), g3_idesc(N), (h | k) != 0);
+          if (h == 1) t5_commit(d_full(g));
+        }
+        __syncwarp();
+      }
+      c += NG;
+      if (c >= nsl) c -= nsl;
+      par ^= 1u;
     }
   }
+  // After a wait ran out: copies in flight land, and nothing of this CTA may still run on the tensor core when its tensor memory
+  // is freed.  (Otherwise the workers have waited for all of both.)
+  if (*dead) for (int i = 0; i < 64; i++) __nanosleep(1000);
   t5_fence_before();
   __syncthreads();
   if (warp == 0) {
     t5_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)G3_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
 }

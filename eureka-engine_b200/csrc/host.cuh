@@ -12,7 +12,7 @@ struct LlbCtx {
   int device = -1;
   int sms = 0;
   int ffn_fused = 0;   // the FFN as one launch with a grid barrier (LLB_FFN_FUSED=1)
-  int gemm3 = 0;   // Q4_K, T <= 4 on the tcgen05 kernel (LLB_GEMM3=1)
+  int gemm3 = 0;   // the tcgen05 kernel of Q4_K launches: 0 where it is the faster one, 1 wherever it can run (LLB_GEMM3=1), -1 never (LLB_GEMM3=0)
   int pdl = 1;     // programmatic dependent launch on every kernel of a pass (LLB_PDL=0 turns it off)
   cudaStream_t stream = nullptr;
   char err[512] = {0};
