@@ -5,8 +5,6 @@
 #include "moe.cuh"
 #include "host.cuh"
 
-#define G3_SCALE 1.0
-
 // can the tcgen05 kernel take this K-split?  (a super-block of every tile for each of its groups, two stages beside the planes)
 static bool g3_fits(int fmt, int NC, int nsb, int ks) {
   if (g_llb.gemm3 < 0 || fmt != LLB_FM_Q4_K) return false;
@@ -181,11 +179,14 @@ static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int 
   const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, NC / 8, tiles, nsb, ks), direct && NC >= 32 ? 3000.0 : 1200.0);
   return (stream + stage * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
-// The tcgen05 kernel's cost on the same scale (fitted to its gains over the other one, which that scale flatters): a super-block of
-// 128 rows in a CTA, the slice's activations, the pipeline's fill and the last tile's way out.
+// The tcgen05 kernel's cost on the same scale: a super-block of 128 rows in a CTA, a tile's way out, the slice's activations, the
+// pipeline's fill -- times 0.7, because that scale flatters the other kernel (27B shape, milliseconds a pass of one, four, eight
+// and sixteen rows: 4.99, 5.33, 6.56, 9.82 with this factor; 5.21, 5.44, 6.62, 9.83 with 1; 5.15, 5.52, 6.56, 9.73 with 0.4; 5.21, 5.39, 7.08,
+// 11.19 without the kernel).
 static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
-  return G3_SCALE * (tiles * (double)slice * (820.0 + (NC >= 32 ? 150.0 : 0.0)) * (1.0 + 0.02 * (ks - 1)) + 3000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
+  const double sb = NC >= 32 ? 970.0 : 820.0;
+  return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
 static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks) {
