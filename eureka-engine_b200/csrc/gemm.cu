@@ -5,9 +5,12 @@
 #include "moe.cuh"
 #include "host.cuh"
 
-// can the tcgen05 kernel take this K-split?  (a super-block of every tile for each of its groups, two stages beside the planes)
-static bool g3_fits(int fmt, int NC, int nsb, int ks) {
-  if (g_llb.gemm3 < 0 || fmt != LLB_FM_Q4_K) return false;
+// Can the tcgen05 kernel take this K-split?  (a super-block of every tile for each of its groups, two stages beside the planes)
+// At 8 plane columns it is for launches on their own: between the small kernels of a pass, where the mma.sync kernel's ring and first
+// tiles are ready when the activations come, it is the slower one (27B shape, 24 cycles of four rows 143.6 ms without it, 151 with
+// it; 24 passes of one row 121.7 and 123.4), alone the faster (gate|up at four rows 28.1 and 26.5 us, at one 28.2 and 24.6).
+static bool g3_fits(int fmt, int NC, int nsb, int ks, bool alone) {
+  if (g_llb.gemm3 < 0 || fmt != LLB_FM_Q4_K || (NC == 8 && !alone && g_llb.gemm3 == 0)) return false;
   return ks >= 1 && nsb / ks >= g3_groups(NC) && g3_stages(NC, (nsb + ks - 1) / ks) >= 2;
 }
 static unsigned int *g_ffn_sync = nullptr;   // the fused FFN's grid barrier: two counters
@@ -156,9 +159,9 @@ static int g2_least_ksplit(int fmt, int NC, int nsb) {
   const int mx = g2_max_slice_sb(fmt, NC), most = g2_longest_slice(fmt, NC), lo = (nsb + mx - 1) / mx;
   return lo <= GEMM_MAXSPLIT ? lo : (nsb + most - 1) / most;
 }
-int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks) {
+int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone) {
   if (ks < 1) ks = 1;
-  if (!g3_fits(fmt, NC, nsb, ks)) {
+  if (!g3_fits(fmt, NC, nsb, ks, alone)) {
     const int least = g2_least_ksplit(fmt, NC, nsb);
     if (ks < least) ks = least;
   }
@@ -180,17 +183,16 @@ static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int 
   return (stream + stage * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
 // The tcgen05 kernel's cost on the same scale: a super-block of 128 rows in a CTA, a tile's way out, the slice's activations, the
-// pipeline's fill -- times 0.7, because that scale flatters the other kernel (27B shape, milliseconds a pass of one, four, eight
-// and sixteen rows: 4.99, 5.33, 6.56, 9.82 with this factor; 5.21, 5.44, 6.62, 9.83 with 1; 5.15, 5.52, 6.56, 9.73 with 0.4; 5.21, 5.39, 7.08,
-// 11.19 without the kernel).
+// pipeline's fill -- times 0.7, because that scale flatters the other kernel (27B shape, a prompt of 48 tokens in passes of eight rows
+// 51.7 ms without the kernel, 49.2 with this factor 1, 48.5 with 0.7; ten cycles of sixteen rows 125.2, 114.6, 114.2).
 static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
   const double sb = NC >= 32 ? 970.0 : 820.0;
   return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
-static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks) {
-  if (!g3_fits(fmt, NC, nsb, ks)) return false;
+static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, bool alone) {
+  if (!g3_fits(fmt, NC, nsb, ks, alone)) return false;
   if (g_llb.gemm3 > 0 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
   return g3_cost(NC, ntiles, nsb, ks, g_llb.sms, false) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, g_llb.sms, false, 24.0);
 }
@@ -198,11 +200,11 @@ int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct,
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
-    if (gemm_fix_ksplit(fmt, NC, nsb, ks) != ks) continue;
-    const double cost = g3_use(fmt, NC, ntiles, nsb, ks) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
+    if (gemm_fix_ksplit(fmt, NC, nsb, ks, direct) != ks) continue;
+    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
   }
-  return gemm_fix_ksplit(fmt, NC, nsb, best);
+  return gemm_fix_ksplit(fmt, NC, nsb, best, direct);
 }
 
 // One K-split for a launch whose partial sums outlive the pass (attn_qkv into the conv ring): valid at both
@@ -230,7 +232,7 @@ static int gemm_prepare(int fmt, GemmArgs &a, bool fused = false) {
   a.tile0[0] = 0;
   for (int i = 0; i < a.nmat; i++) a.tile0[i + 1] = a.tile0[i] + (a.m[i].rows + 15) / 16;
   for (int i = a.nmat; i < GEMM_MAXMAT; i++) a.tile0[i + 1] = a.tile0[a.nmat];
-  if (!fused && a.ksplit != gemm_fix_ksplit(fmt, a.xp.NC, a.nsb, a.ksplit)) return llb_fail("gemm: ksplit %d is not valid for this shape", a.ksplit);
+  if (!fused && a.ksplit != gemm_fix_ksplit(fmt, a.xp.NC, a.nsb, a.ksplit, a.alone)) return llb_fail("gemm: ksplit %d is not valid for this shape", a.ksplit);
   return 0;
 }
 
@@ -346,7 +348,7 @@ int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a) {
   if (gemm_prepare(fmt, a)) return -1;
   if (a.tile0[a.nmat] < 1) return 0;
   const int NT = a.xp.NC / 8;
-  if (g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
+  if (g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit, a.alone)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
   if (fmt == LLB_FM_Q4_K) return NT == 1 ? launch_two<LLB_FM_Q4_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q4_K, 2>(s, a) : launch_two<LLB_FM_Q4_K, 4>(s, a);
   if (fmt == LLB_FM_Q5_K) return NT == 1 ? launch_two<LLB_FM_Q5_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q5_K, 2>(s, a) : launch_two<LLB_FM_Q5_K, 4>(s, a);
   if (fmt == LLB_FM_Q6_K) return NT == 1 ? launch_two<LLB_FM_Q6_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q6_K, 2>(s, a) : launch_two<LLB_FM_Q6_K, 4>(s, a);

@@ -47,7 +47,7 @@ inline cudaError_t llb_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
 
 // gemm.cu
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct = false, double stage = 24.0);   // direct: the caller adds the slices with a launch of its own; stage: cycles to stage a plane column of a super-block
-int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks);   // clamps a requested K-split to what the format's kernel can take
+int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone = false);   // clamps a requested K-split to what a kernel can take; alone: not one of a pass's launches
 int gemm_longest_slice(int fmt, int NC);   // super-blocks of the longest K-slice a launch takes
 int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int sms, int cap);
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a);   // fills tile0 / nsb, picks NT from xp.NC
