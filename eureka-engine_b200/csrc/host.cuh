@@ -45,6 +45,21 @@ inline cudaError_t llb_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
   return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
 }
 
+// ... in clusters of n blocks along x
+template <typename... KArgs, typename... Args>
+inline cudaError_t llb_launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, int n, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned int)n; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = g_llb.pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
+}
+
 // gemm.cu
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct = false, double stage = 24.0);   // direct: the caller adds the slices with a launch of its own; stage: cycles to stage a plane column of a super-block
 int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone = false);   // clamps a requested K-split to what a kernel can take; alone: not one of a pass's launches
@@ -52,6 +67,7 @@ int gemm_longest_slice(int fmt, int NC);   // super-blocks of the longest K-slic
 int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int sms, int cap);
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a);   // fills tile0 / nsb, picks NT from xp.NC
 int gemm_setup(void);
+unsigned int *gemm_err_word(void);   // device word that a bounded wait sets when it runs out
 int gemm_wait_errors(void);
 int gemm_wait_errors_clear(void);
 int gemm_wait_selftest(cudaStream_t s, int which, int limit);

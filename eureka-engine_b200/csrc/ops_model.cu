@@ -6,6 +6,7 @@
 
 #include "model.cuh"
 #include "rowops.cuh"
+#include "tc5.cuh"
 namespace cg = cooperative_groups;
 
 // sum over the block; every thread gets the result (red: >= 32 floats of shared memory)
@@ -45,32 +46,49 @@ int op_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const RowSet *rs,
 // tools/payload-spec2.patch:35-112; rms_norm tools/qwen35_engine.c:510-515) ----------------------
 // v = xin + sum(partials); xout = v (optional); h = (v * s) * w, s = 1/sqrt(mean(v^2) + eps);
 // h goes to the planes at column offset xp_col0 and, optionally, to hn_out as f32.
-// One block per row; a thread holds NI groups of four consecutive columns (float4 loads and stores).
+// A row is a cluster of CL blocks (one, where the row is short), each with its part of the columns, four consecutive ones a
+// thread (float4 loads and stores).  What bounds it is one SM's way to L2: a row of 5120 columns in eleven K-slices is 245 KB, 1.9 us
+// through one SM's port; in four it and the blocks' sums, pushed to the peers with st.async, take less.  The 27B shape's passes took
+// 1.2 % longer with a block a row, the 35B-A3B shape's (2048 columns) 1.3 %.
 #define NORM_MAXT 1024
-template <int NI>
+#define NORM_CL 4
+template <int NI, int CL>
 __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__ xin, PartIn add, const float *__restrict__ w, float eps, int d,
                                                        float *__restrict__ xout, XPlanes xp, int xp_col0, float *__restrict__ hn_out,
-                                                       const RowSet *rs, Streams sg, int zero_if_pos0) {
+                                                       const RowSet *rs, Streams sg, int zero_if_pos0, unsigned int *err) {
+  __shared__ float red[32], part[CL];
+  __shared__ __align__(8) uint64_t bar;
+  const uint32_t bar_s = smem_u32(&bar);
+  const int rank = CL > 1 ? blockIdx.x % CL : 0, dc = CL > 1 ? d / CL : d, cb = rank * dc;   // this block's columns cb .. cb + dc - 1
+  if constexpr (CL > 1) {
+    if (threadIdx.x == 0) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_s) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_s), "r"(4u * CL) : "memory");
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  }
   // the norm weights depend on no kernel: their trip to DRAM overlaps the wait on the producer
   float4 wv[NI], v[NI];
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
     v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    wv[i] = c < d ? __ldg((const float4 *)(w + c)) : v[i];
+    wv[i] = c < dc ? __ldg((const float4 *)(w + cb + c)) : v[i];
   }
   int rs_n, rs_p0, tl;
-  const int t = blockIdx.x;
+  const int t = blockIdx.x / CL;
   rs = rs_begin_row(rs, sg, t, rs_n, rs_p0, tl);
-  __shared__ float red[32];
-  if (tl >= rs_n) return;
+  if constexpr (CL > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer's barrier is there
+  if (tl >= rs_n) return;   // every block of the row takes this exit
   const bool zero = zero_if_pos0 && (rs_p0 + tl == 0);
-  const size_t row = (size_t)t * d;
+  const size_t row = (size_t)t * d + cb;
   if (xin && !zero) {
 #pragma unroll
     for (int i = 0; i < NI; i++) {
       const int c = 4 * (threadIdx.x + i * blockDim.x);
-      if (c < d) v[i] = __ldcg((const float4 *)(xin + row + c));
+      if (c < dc) v[i] = __ldcg((const float4 *)(xin + row + c));
     }
   }
   if (add.p && !zero) {
@@ -84,7 +102,7 @@ __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__
 #pragma unroll
         for (int i = 0; i < NI; i++) {
           const int c = 4 * (threadIdx.x + i * blockDim.x);
-          l[q][i] = (c < d && k + q < add.ns) ? __ldcg((const float4 *)(pk + (size_t)q * add.stride + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          l[q][i] = (c < dc && k + q < add.ns) ? __ldcg((const float4 *)(pk + (size_t)q * add.stride + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
       for (int q = 0; q < 4; q++)
@@ -96,7 +114,7 @@ __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
-    if (xout && c < d) *(float4 *)(xout + row + c) = v[i];
+    if (xout && c < dc) *(float4 *)(xout + row + c) = v[i];
     ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;   // (zeros past the row's end)
   }
   const int lane = threadIdx.x & 31, nwp = blockDim.x >> 5;
@@ -104,21 +122,35 @@ __global__ void __launch_bounds__(NORM_MAXT) k_norm_xp(const float *__restrict__
   if (lane == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
   ss = warp_sum(lane < nwp ? red[lane] : 0.0f);
+  if constexpr (CL > 1) {
+    if (threadIdx.x < CL) cl_push(smem_u32(&part[rank]), ss, bar_s, lane);
+    if (!cl_wait(bar_s) && threadIdx.x == 0) atomicExch(err, 1u);   // (a block leaves when every push to it is there)
+    ss = part[0];
+#pragma unroll
+    for (int i = 1; i < CL; i++) ss += part[i];
+  }
   const float sc = 1.0f / sqrtf(ss / (float)d + eps);
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);   // eight lanes hold 32 consecutive columns
     const float h[4] = {v[i].x * sc * wv[i].x, v[i].y * sc * wv[i].y, v[i].z * sc * wv[i].z, v[i].w * sc * wv[i].w};
-    if (c < d && hn_out) *(float4 *)(hn_out + row + c) = make_float4(h[0], h[1], h[2], h[3]);
-    xp_store4(xp, t, 2, xp_col0 + c, h, lane, c < d);
+    if (c < dc && hn_out) *(float4 *)(hn_out + row + c) = make_float4(h[0], h[1], h[2], h[3]);
+    xp_store4(xp, t, 2, xp_col0 + cb + c, h, lane, c < dc);
   }
 }
+// Four blocks a row from NORM_SPLIT columns on (whole groups of 32 columns to each), one below: 1024 columns are one trip of one block.
+#define NORM_SPLIT 2048
 int op_norm_xp(cudaStream_t s, const float *xin, PartIn add, const float *w, float eps, int d, float *xout, XPlanes xp,
                int xp_col0, float *hn_out, const RowSet *rs, int Tmax, int zero_if_pos0) {
   if (d % 32 || xp_col0 % 32 || d > 4 * 4 * NORM_MAXT) return llb_fail("norm: d %d at column %d", d, xp_col0);
-  const int d4 = d / 4, ni = (d4 + NORM_MAXT - 1) / NORM_MAXT;
+  const bool split = d >= NORM_SPLIT && d % (32 * NORM_CL) == 0;
+  const int d4 = d / 4 / (split ? NORM_CL : 1), ni = (d4 + NORM_MAXT - 1) / NORM_MAXT;
   const int threads = (((d4 + ni - 1) / ni) + 31) & ~31;
-#define NORM_GO(NI) CU_OK(llb_launch(k_norm_xp<NI>, dim3(Tmax), dim3(threads), (size_t)(0), s, xin, add, w, eps, d, xout, xp, xp_col0, hn_out, rs, g_streams, zero_if_pos0))
+  if (split) {   // (d / 4 / NORM_CL <= NORM_MAXT)
+    CU_OK(llb_launch_cluster(k_norm_xp<1, NORM_CL>, dim3(Tmax * NORM_CL), dim3(threads), NORM_CL, s, xin, add, w, eps, d, xout, xp, xp_col0, hn_out, rs, g_streams, zero_if_pos0, gemm_err_word()));
+    return 0;
+  }
+#define NORM_GO(NI) CU_OK(llb_launch(k_norm_xp<NI, 1>, dim3(Tmax), dim3(threads), (size_t)(0), s, xin, add, w, eps, d, xout, xp, xp_col0, hn_out, rs, g_streams, zero_if_pos0, gemm_err_word()))
   switch (ni) {
     case 1: NORM_GO(1); break;
     case 2: NORM_GO(2); break;
@@ -126,7 +158,6 @@ int op_norm_xp(cudaStream_t s, const float *xin, PartIn add, const float *w, flo
     default: NORM_GO(4); break;
   }
 #undef NORM_GO
-  CU_OK(cudaGetLastError());
   return 0;
 }
 
@@ -531,8 +562,24 @@ __global__ void __launch_bounds__(256) k_top2_part(PartIn logits, int V, long lo
   const size_t z0 = (size_t)t * row_stride;
   const int per = (V + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * per, i1 = min(V, i0 + per);
   Top2 a = {0.f, -1, 0.f, -1};
+  // (four values of a thread in flight at a time: one by one, a vocabulary of 151936 took nine trips to L2)
 #pragma unroll 1
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) t2_push(a, part_get(logits, z0 + i), i);
+  for (int i = i0 + threadIdx.x; i < i1; i += 4 * blockDim.x) {
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[q] = i + q * blockDim.x < i1 ? __ldcg(logits.p + z0 + i + q * blockDim.x) : 0.0f;
+#pragma unroll 1
+    for (int k = 1; k < logits.ns; k++) {
+      const float *pk = logits.p + (size_t)k * logits.stride + z0 + i;
+      float l[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) l[q] = i + q * blockDim.x < i1 ? __ldcg(pk + q * blockDim.x) : 0.0f;
+#pragma unroll
+      for (int q = 0; q < 4; q++) v[q] += l[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) t2_push(a, v[q], i + q * blockDim.x < i1 ? i + q * (int)blockDim.x : -1);
+  }
   a = t2_warp(a);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
   __syncthreads();
@@ -552,11 +599,11 @@ int op_top2_part(cudaStream_t s, PartIn logits, int V, long long row_stride, flo
 }
 __device__ __forceinline__ Top2 t2_final(const float *part, int t, int lane) {
   Top2 a = {0.f, -1, 0.f, -1};
-  for (int b = lane; b < TOP2_NB; b += 32) {
-    const float4 p = __ldcg((const float4 *)part + (size_t)t * TOP2_NB + b);   // (to L2: every drafter step writes the same partials)
-    t2_push(a, p.x, __float_as_int(p.y));
-    t2_push(a, p.z, __float_as_int(p.w));
-  }
+  float4 p[TOP2_NB / 32];
+#pragma unroll
+  for (int q = 0; q < TOP2_NB / 32; q++) p[q] = __ldcg((const float4 *)part + (size_t)t * TOP2_NB + lane + 32 * q);   // (to L2: every drafter step writes the same partials)
+#pragma unroll
+  for (int q = 0; q < TOP2_NB / 32; q++) { t2_push(a, p[q].x, __float_as_int(p[q].y)); t2_push(a, p[q].z, __float_as_int(p[q].w)); }
   return t2_warp(a);
 }
 
@@ -687,36 +734,39 @@ int op_lookup_draft(cudaStream_t s, SpecCtl *ctl, int nz) {
 // After a drafter pass: the head argmax of its last row is draft j (mapped through the draft-vocab ids,
 // host/llb_host.c:1800-1807); it becomes verify input j and the token of the next chained row, whose hidden
 // is the drafter's own normed hidden of that last row (host/llb_host.c:1824-1827).
-__global__ void k_draft_pick(const float *__restrict__ part, const int *__restrict__ ids, SpecCtl *__restrict__ ctl,
+#define PICK_THREADS 512
+__global__ void __launch_bounds__(PICK_THREADS) k_draft_pick(const float *__restrict__ part, const int *__restrict__ ids, SpecCtl *__restrict__ ctl,
                              int from_chain, int j, const float *__restrict__ mt_hn, float *__restrict__ chain_h, int d, int per) {
   pdl_trigger();
   pdl_wait();
-  __shared__ int s_tok;
   // one block per stream: its control block and its rows of the drafter pass; the chained row is the stream's row 0
   ctl += blockIdx.x;
   const size_t row0 = (size_t)blockIdx.x * per;
   part += row0 * TOP2_NB * 4; mt_hn += row0 * d; chain_h += row0 * d;
   const RowSet *rs = from_chain ? &ctl->chain : &ctl->catchup;
-  const int last = __ldcg(&rs->n) - 1;
-  if (last < 0) return;
-  if (threadIdx.x < 32) {
-    Top2 a = t2_final(part, last, threadIdx.x);
-    if (threadIdx.x == 0) s_tok = a.i1 < 0 ? 0 : ids ? ids[a.i1] : a.i1;
-  }
+  const int last = __ldcg(&rs->n) - 1, p = __ldcg(&ctl->verify.pos0), n = __ldcg(&ctl->verify.n);
+  // (every thread has read the row count before the first one writes it: in the drafter's later steps the chain is the row set)
   __syncthreads();
-  for (int c = threadIdx.x; c < d; c += blockDim.x) chain_h[c] = __ldcg(mt_hn + (size_t)last * d + c);
+  if (last < 0) return;
+  if (threadIdx.x >= 32) {   // the first warp picks while the others copy (d is a multiple of 32)
+    const float4 *src = (const float4 *)(mt_hn + (size_t)last * d);
+#pragma unroll 4
+    for (int c = threadIdx.x - 32; c < d / 4; c += PICK_THREADS - 32) ((float4 *)chain_h)[c] = __ldcg(src + c);
+    return;
+  }
+  const Top2 a = t2_final(part, last, threadIdx.x);
   if (threadIdx.x == 0) {
-    const int p = __ldcg(&ctl->verify.pos0);
-    if (j < __ldcg(&ctl->verify.n)) ctl->verify.tok[j] = s_tok;
+    const int tok = a.i1 < 0 ? 0 : ids ? ids[a.i1] : a.i1;
+    if (j < n) ctl->verify.tok[j] = tok;
     ctl->chain.n = 1;
     ctl->chain.pos0 = p + j;
-    ctl->chain.tok[0] = s_tok;
+    ctl->chain.tok[0] = tok;
     ctl->chain.slot[0] = 0;
   }
 }
 int op_draft_pick(cudaStream_t s, const float *part, const int *ids, SpecCtl *ctl, int from_chain, int j, const float *mt_hn,
                   float *chain_h, int d, int nz, int per) {
-  CU_OK(llb_launch(k_draft_pick, dim3(nz), dim3(256), (size_t)(0), s, part, ids, ctl, from_chain, j, mt_hn, chain_h, d, per));
+  CU_OK(llb_launch(k_draft_pick, dim3(nz), dim3(PICK_THREADS), (size_t)(0), s, part, ids, ctl, from_chain, j, mt_hn, chain_h, d, per));
   CU_OK(cudaGetLastError());
   return 0;
 }

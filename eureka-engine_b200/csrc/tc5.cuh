@@ -91,6 +91,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar_s, uint32_t parity, uint3
   }
   return false;
 }
+// bounded wait for the first phase of a barrier that blocks of the cluster complete (cl_push): their words are visible after it
+__device__ __forceinline__ bool cl_wait(uint32_t bar_s) {
+#pragma unroll 1
+  for (uint32_t it = 0; it < (1u << 20); it++) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(ok) : "r"(bar_s) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// one word into shared memory of block `rank` of the cluster, counted on that block's barrier
+__device__ __forceinline__ void cl_push(uint32_t dst_s, float v, uint32_t bar_s, uint32_t rank) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(t5_map_rank(dst_s, rank)), "r"(__float_as_uint(v)), "r"(t5_map_rank(bar_s, rank))
+               : "memory");
+}
 // K-major, no swizzle: 8 rows x 16 bytes per core matrix; LBO = step between the two k-chunks of an
 // MMA, SBO = step between 8-row groups (bytes, both multiples of 16); descriptor version 1 (sm_100)
 __device__ __forceinline__ uint64_t g3_desc(uint32_t addr_s, uint32_t lbo, uint32_t sbo) {
