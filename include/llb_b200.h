@@ -98,10 +98,10 @@ LLB_API int llb_b200_xp_set_bf16(llb_xp *xp, llb_b200_dptr x_bf16 /* [T][K] */);
  * out_i: f32 [T][rows_i].  ksplit = 0 picks the K-split; scratch for the partial sums is internal. */
 LLB_API int llb_b200_gemm(int fmt, int nmat, const llb_b200_dptr *w, const int *rows, const llb_b200_dptr *out, int K, const llb_xp *xp,
                   int ksplit);
-/* Q4_K GEMMs with T <= 4 on the tcgen05 kernel (weights unpacked into tensor memory, tcgen05.mma) instead
- * of the mma.sync one; returns the previous setting.  Also set by LLB_GEMM3=1 at llb_b200_init.  Off by
- * default: at the 27B shapes the mma.sync kernel is the faster of the two.  A speculative engine keeps the
- * kernels it was opened with. */
+/* Every Q4_K GEMM that can run there on the tcgen05 kernel (weights unpacked into tensor memory, tcgen05.mma) instead
+ * of the mma.sync one; returns the previous setting.  Also set by LLB_GEMM3=1 at llb_b200_init.  Off (0) by
+ * default: each launch then takes the kernel that is the faster one at its size (LLB_GEMM3=0 at llb_b200_init keeps all of them
+ * on mma.sync).  A speculative engine keeps the kernels it was opened with. */
 LLB_API int llb_b200_use_tcgen05(int on);
 /* The SwiGLU FFN of engines opened from now on as ONE launch (gate|up GEMM, grid-wide barrier, silu(gate) * up built in
  * shared memory, down GEMM) instead of three; returns the previous setting.  Also LLB_FFN_FUSED=1 at llb_b200_init.  Off by

@@ -167,7 +167,7 @@ def test_row_independence_at_sixteen_rows(llb, packs, dev, ty):
 
 @pytest.fixture
 def tcgen05(llb):
-    """Q4_K, T <= 4 GEMMs of this test run on the tcgen05 kernel (weights in tensor memory)."""
+    """Q4_K GEMMs of three super-blocks a K-slice and more run on the tcgen05 kernel in this test (weights in tensor memory)."""
     L = llb.lib()
     was = L.llb_b200_use_tcgen05(1)
     yield
@@ -196,3 +196,14 @@ def test_tcgen05_gemm_many_tiles(llb, packs, oracle, dev, tcgen05):
     # more 128-row tiles than CTAs: a CTA walks several tiles and prefetches across them
     _gemm_case(llb, packs, oracle, dev, "Q4_K", [40000], 512, 4, 2, 0, seed=9)
     _gemm_case(llb, packs, oracle, dev, "Q4_K", [20000], 1024, 4, 2, 2, seed=10)
+
+
+@pytest.mark.parametrize("rows,K,ksplit", [([1], 768, 1), ([127, 129], 1280, 1), ([128], 2304, 3), ([300, 16, 1, 260], 1792, 2), ([20000], 1280, 1), ([515], 17408, 13)])
+@pytest.mark.parametrize("T", [1, 4, 5, 8, 9, 16])
+def test_tcgen05_edges_of_tiles_and_slices(llb, packs, oracle, dev, tcgen05, rows, K, ksplit, T):
+    """One row, rows around a tile of 128, matrices that share a launch, a CTA of several tiles, K-slices of odd lengths (a stage with one
+    super-block, slices one longer than others, the three of the shortest), every plane width: against the oracle's dequantisation at
+    1e-5 of the dot mass."""
+    if K // 256 // ksplit < 3 or (T > 8 and K // 256 // ksplit > 8):
+        ksplit = max(1, K // 256 // 5)
+    _gemm_case(llb, packs, oracle, dev, "Q4_K", rows, K, T, 2, ksplit, seed=K + T)
