@@ -136,6 +136,10 @@ def run_reference(args, rank):
     if rank != 0:
         return
     import torch
+    from oracle import bindings
+    if not os.path.exists(bindings.REF_SO):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference engine's library has not been built: its sources are not on this machine"}), flush=True)
+        return
     cores = os.cpu_count() or 1
     dev = "cuda:0" if torch.cuda.is_available() else "cpu"
     packs, pack, mtp, prompt = build_model(dev)
@@ -387,7 +391,7 @@ def run_gemm_case(args, local):
     peak, peak_src = peaks()
     nc = 8 if T <= 4 else 16 if T <= 8 else 32
     nbytes = per_copy + nc * K * 2 + sum(T * r * 4 for r in rows)
-    print(json.dumps({"case": "gemm", "kernel": f"k_gemm2<{ty}>", "rows": rows, "cols": K, "T": T, "plane_columns": nc, "launches": args.steps,
+    print(json.dumps({"case": "gemm", "kernel": f"skinny GEMM, {ty}", "rows": rows, "cols": K, "T": T, "plane_columns": nc, "launches": args.steps,
                       "weight_copies": copies, "us_per_launch": us, "bytes_per_launch": nbytes, "GBs": nbytes / us / 1e3, "frac": nbytes / us / 1e3 / peak,
                       "peak": peak, "peak_source": peak_src, "ksplit": L.llb_b200_gemm_ksplit(fmt, nc, sum((r + 15) // 16 for r in rows), K // 256, L.llb_b200_sm_count()) if args.ksplit == 0 else args.ksplit,
                       "wait_errors": L.llb_b200_wait_errors()}), flush=True)
