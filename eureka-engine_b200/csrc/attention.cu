@@ -331,6 +331,7 @@ template <int HD, int NQG> static int att_attr() {
   return 0;
 }
 int ops_model_setup(void) {
+  if (delta_setup()) return -1;
   if (att_attr<128, 1>() || att_attr<128, 2>() || att_attr<128, 3>() || att_attr<128, 4>() || att_attr<128, 5>() || att_attr<128, 6>()) return -1;
   if (att_attr<256, 1>() || att_attr<256, 2>() || att_attr<256, 3>() || att_attr<256, 4>() || att_attr<256, 5>() || att_attr<256, 6>()) return -1;
   return 0;

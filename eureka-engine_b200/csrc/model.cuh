@@ -158,4 +158,5 @@ int op_accept(cudaStream_t s, const float *part, SpecCtl *ctl, SpecResult *ring,
               const int *smp_tok = nullptr, const float *smp_val = nullptr);
 int op_draft_pick(cudaStream_t s, const float *part, const int *ids, SpecCtl *ctl, int from_chain, int j, const float *mt_hn,
                   float *chain_h, int d, int nz = 1, int per = 0);
+int delta_setup(void);
 int ops_model_setup(void);

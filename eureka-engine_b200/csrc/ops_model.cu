@@ -339,6 +339,7 @@ int op_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, c
 // sums of squares of the gated norm are pushed into the peers' shared memory and cost one cluster barrier, behind which
 // the gate factors are made.
 #define DL_THREADS 256
+#define DL_ALONE (104 * 1024)   // dynamic shared memory of a block that wants its SM for itself
 #define DL_MAXR (SPEC_MAXT + CONV_RING / 2 - 1)   // history rows of a pass: n + KC - 1
 __device__ __forceinline__ float4 dl_slice(const PartIn &a, size_t i, int k) {
   return k < a.ns ? __ldcg((const float4 *)(a.p + i + k * a.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -542,11 +543,19 @@ k_delta(float *__restrict__ S, const SpecCtl *__restrict__ ctl, PartIn ring, con
     xp_store4(xp, row0 + zt, 2, col, h, lane, zon);
   }
 }
+int delta_setup(void) {
+  CU_OK(cudaFuncSetAttribute(k_delta, cudaFuncAttributeMaxDynamicSharedMemorySize, DL_ALONE));
+  return 0;
+}
 int op_delta(cudaStream_t s, float *S, const SpecCtl *ctl, PartIn ring, const float *cw, PartIn bp, PartIn ap, const float *dt, const float *sa,
              PartIn z, const float *nw, DeltaShape sh, XPlanes xp, const RowSet *rs, int nz, long long s_group) {
   if (sh.SZ != 128) return llb_fail("DeltaNet state size %d (only 128, as host/llb_host.c:1608)", sh.SZ);
   if (sh.KC > CONV_RING / 2) return llb_fail("conv kernel %d", sh.KC);
-  CU_OK(llb_launch(k_delta, dim3(sh.TR, 4, nz), dim3(DL_THREADS), (size_t)0, s, S, ctl, ring, cw, bp, ap, dt, sa, z, nw, sh, xp, rs, g_streams, s_group));
+  // An SM's stores leave it at about 32 bytes a cycle, and two of a cluster's blocks on one SM share them (a row of the scan 0.64 us
+  // there): where every block can have an SM, each asks for nearly half of the shared memory. 0.8B shape (32 blocks) 26.2 -> 25.3 ms a
+  // chat turn, 35B-A3B shape (128 blocks) 107.8 -> 105.9; with more blocks than SMs there is nothing to spread.
+  const size_t alone = 4 * sh.TR * nz <= g_llb.sms ? DL_ALONE : 0;
+  CU_OK(llb_launch(k_delta, dim3(sh.TR, 4, nz), dim3(DL_THREADS), alone, s, S, ctl, ring, cw, bp, ap, dt, sa, z, nw, sh, xp, rs, g_streams, s_group));
   return 0;
 }
 
