@@ -185,16 +185,18 @@ static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int 
 // The tcgen05 kernel's cost on the same scale: a super-block of 128 rows in a CTA, a tile's way out, the slice's activations, the
 // pipeline's fill -- times 0.7, because that scale flatters the other kernel (27B shape, a prompt of 48 tokens in passes of eight rows
 // 51.7 ms without the kernel, 49.2 with this factor 1, 48.5 with 0.7; ten cycles of sixteen rows 125.2, 114.6, 114.2).
+// In a pass (not direct) 4000 cycles more: its first MMA waits for all activations, and what the mma.sync kernel has ready by then is
+// worth that much; without it the 2048-column launches of the 35B-A3B shape came here and eight of its streams took 156 ms instead of 147.
 static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
   const double sb = NC >= 32 ? 970.0 : 820.0;
-  return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
+  return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0) + (direct ? 0.0 : 4000.0);
 }
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
 static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, bool alone) {
   if (!g3_fits(fmt, NC, nsb, ks, alone)) return false;
   if (g_llb.gemm3 > 0 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
-  return g3_cost(NC, ntiles, nsb, ks, g_llb.sms, false) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, g_llb.sms, false, 24.0);
+  return g3_cost(NC, ntiles, nsb, ks, g_llb.sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, g_llb.sms, false, 24.0);
 }
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {
   int best = 1;
