@@ -247,6 +247,8 @@ int llb_b200_gemm_ksplit(int fmt, int nc, int ntiles, int nsb, int sms) { return
 int llb_b200_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_prefill, int sms) {
   return gemm_ring_ksplit(fmt, nsb, ntiles, nc_spec, nc_prefill, sms, 8);
 }
+int llb_b200_gemm3_trace(int nc, int nsl, int tiles, int agent, int *ops, int cap) { return gemm3_trace(nc, nsl, tiles, agent, ops, cap); }
+int llb_b200_gemm3_bar_count(int nc, int bar) { return gemm3_bar_count(nc, bar); }
 
 int llb_b200_use_tcgen05(int on) {
   NEED_INIT(-1)

@@ -64,6 +64,44 @@ template <int NC> static int launch_three(cudaStream_t s, const GemmArgs &a) {
   if (e != cudaSuccess) return llb_fail("k_gemm3 launch: %s", cudaGetErrorString(e));
   return 0;
 }
+// What one agent of a CTA of k_gemm3 does with the CTA's barriers, in its order: a warp of group `agent`, behind the groups the warp
+// that requests the weights, then a group's issuing warp.  ops: {0 wait, barrier, phase}, {1 arrive, barrier, times}, {2 arrive, barrier,
+// once a copy requested here has landed or an MMA issued here is done}.  Returns their number, -1 where the kernel takes no such slice.
+int gemm3_trace(int NC, int nsl, int tiles, int agent, int *ops, int cap) {
+  const int NG = g3_groups(NC), st = g3_stages(NC, nsl);
+  if ((NC != 8 && NC != 16 && NC != 32) || nsl < NG || st < 2 || tiles < 1 || agent < 0 || agent > 2 * NG) return -1;
+  int n = 0;
+  auto op = [&](int kind, int b, int v) { if (3 * n + 2 < cap) { ops[3 * n] = kind; ops[3 * n + 1] = b; ops[3 * n + 2] = v; } n++; };
+  if (agent < NG) {
+    G3Walk wk;
+    int it = 0;
+    for (wk.start(agent, st); wk.ti < tiles; wk.next(NG, nsl, st)) {
+      op(0, wk.full(), wk.phase());
+      if (it > 0) op(0, G3_D_FULL + agent, it - 1);
+      for (int h = 0; h < 2; h++) op(1, G3_A_FULL + 2 * agent + h, 1);
+      op(1, G3_RAW_EMPTY + wk.slot, wk.owed(nsl));
+      if (it++ == 0) op(1, G3_XP_FULL, 32);
+    }
+    op(0, G3_D_FULL + agent, it - 1);
+  } else if (agent == NG) {
+    const int nch = (nsl + G3_CH - 1) / G3_CH;
+    for (int k = 0; k < tiles * nch; k++) {
+      const int slot = k % st, use = k / st;
+      if (use > 0) op(0, G3_RAW_EMPTY + slot, use - 1);
+      op(2, G3_RAW_FULL + 4 * (use & 1) + slot, 1);
+    }
+  } else {
+    const int g = agent - NG - 1;
+    for (int s = g, k = 0; s < tiles * nsl; s += NG, k++) {
+      if (k == 0) op(0, G3_XP_FULL, 0);
+      for (int h = 0; h < 2; h++) op(0, G3_A_FULL + 2 * g + h, k);
+      op(2, G3_D_FULL + g, 1);
+    }
+  }
+  return n;
+}
+int gemm3_bar_count(int NC, int b) { return (NC != 8 && NC != 16 && NC != 32) || b < 0 || b >= G3_BARS ? -1 : g3_bar_count(NC, b); }
+
 // 1 when a bounded wait of the tcgen05 kernel or of the fused FFN's barrier has run out since the library was
 // initialised (or since the word was last cleared)
 int gemm_wait_errors(void) {

@@ -48,6 +48,33 @@ __host__ __device__ inline int g3_stages(int NC, int nsl) {
   const int left = G3_SMEM_MAX - G3_HDR - g3_red_bytes(NC) - g3_xp_bytes(NC, nsl), st = left / G3_STAGE;
   return st > 4 ? 4 : st;
 }
+// A CTA's barriers by number, eight bytes each from the front of its shared memory, and the arrivals that complete a phase.
+// A stage has two raw_full barriers that its uses take in turn: a group passes over chunks, and bulk copies land in any order, so
+// it comes to use u of a stage without having seen use u - 1 land; with one barrier the parity of a phase that is still
+// pending reads as use u complete.  Use u - 2 of the stage it knows to have landed (g3_walk below).
+enum { G3_RAW_FULL = 0 /* [2][4] */, G3_RAW_EMPTY = 8, G3_A_FULL = 12 /* [3][2] */, G3_D_FULL = 18, G3_RED_FULL = 21, G3_RED_EMPTY = 23, G3_XP_FULL = 25, G3_BARS = 26 };
+__host__ __device__ constexpr int g3_bar_count(int NC, int b) {
+  return b < G3_RAW_EMPTY ? 1 : b < G3_A_FULL ? 4 * G3_CH : b < G3_D_FULL ? 4 : b < G3_RED_FULL ? 1 : b < G3_RED_EMPTY ? 4 * (g3_groups(NC) - 1) : b < G3_XP_FULL ? 4 : g3_groups(NC) * 128;
+}
+// A group's walk: the item (tile of the CTA, super-block of the slice), the stage it lies in and which use of that stage.  nsl >= NG,
+// so that every group has an item in every tile; st >= 2.  NG super-blocks on are two chunks on at most (a tile's last chunk may hold
+// one): the chunk a group comes from was requested behind use u - 1 of the stage it goes to or is that use, which was requested when
+// every group had read use u - 2.
+struct G3Walk {
+  int ti, c, slot, use;
+  __host__ __device__ __forceinline__ void start(int g, int st) { ti = 0; c = g; slot = (g / G3_CH) % st; use = (g / G3_CH) / st; }
+  __host__ __device__ __forceinline__ void next(int NG, int nsl, int st) {
+    int step = -(c / G3_CH);            // as many stages as chunk boundaries lie between
+    c += NG;
+    if (c >= nsl) { c -= nsl; ti++; step += (nsl + G3_CH - 1) / G3_CH; }
+    slot += step + c / G3_CH;
+    if (slot >= st) { slot -= st; use++; }
+  }
+  __host__ __device__ __forceinline__ int full() const { return G3_RAW_FULL + 4 * (use & 1) + slot; }   // its barrier and the phase of that
+  __host__ __device__ __forceinline__ int phase() const { return use >> 1; }
+  // arrivals a warp owes its stage for the item (a stage with one super-block stands for two)
+  __host__ __device__ __forceinline__ int owed(int nsl) const { return c + 1 == nsl && c % G3_CH == 0 ? G3_CH : 1; }
+};
 __host__ __device__ constexpr uint32_t g3_idesc(int N) { return 0x08000010u | ((uint32_t)(N >> 3) << 17); }   // kind::f16: D f32, A / B f16 K-major, M = 128
 
 template <int NC>
@@ -57,17 +84,17 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ks = blockIdx.x % a.ksplit, ci = blockIdx.x / a.ksplit;
   const int sb0 = (int)(((long long)ks * a.nsb) / a.ksplit), nsl = (int)(((long long)(ks + 1) * a.nsb) / a.ksplit) - sb0;
-  // header: raw_full[4] +0, raw_empty[4] +32, a_full[3][2] +64, d_full[3] +112, red_full[2] +136, red_empty[2] +152, tmem +168, dead +172, xp_full +176
+  // header: the barriers, tmem, dead
   const uint32_t bar_s = smem_u32(smem);
-  auto raw_full = [&](int i) { return bar_s + 8u * i; };
-  auto raw_empty = [&](int i) { return bar_s + 32u + 8u * i; };
-  auto a_full = [&](int g, int h) { return bar_s + 64u + 16u * g + 8u * h; };
-  auto d_full = [&](int g) { return bar_s + 112u + 8u * g; };
-  auto red_full = [&](int p) { return bar_s + 136u + 8u * p; };
-  auto red_empty = [&](int p) { return bar_s + 152u + 8u * p; };
-  const uint32_t xp_full = bar_s + 176u;
-  uint32_t *tmem_slot = (uint32_t *)(smem + 168);
-  volatile uint32_t *dead = (volatile uint32_t *)(smem + 172);
+  auto bar = [&](int b) { return bar_s + 8u * b; };
+  auto raw_empty = [&](int i) { return bar(G3_RAW_EMPTY + i); };
+  auto a_full = [&](int g, int h) { return bar(G3_A_FULL + 2 * g + h); };
+  auto d_full = [&](int g) { return bar(G3_D_FULL + g); };
+  auto red_full = [&](int p) { return bar(G3_RED_FULL + p); };
+  auto red_empty = [&](int p) { return bar(G3_RED_EMPTY + p); };
+  const uint32_t xp_full = bar(G3_XP_FULL);
+  uint32_t *tmem_slot = (uint32_t *)(smem + 8 * G3_BARS);
+  volatile uint32_t *dead = (volatile uint32_t *)(smem + 8 * G3_BARS + 4);
   uint8_t *Bp = smem + G3_HDR, *Bm = Bp + (size_t)nsl * NC * 512 + 256;
   float *red = (float *)(smem + G3_HDR + g3_xp_bytes(NC, (a.nsb + a.ksplit - 1) / a.ksplit));
   uint8_t *ring = (uint8_t *)red + g3_red_bytes(NC);
@@ -84,10 +111,8 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
   };
   pdl_trigger();
   if (tid == 0) {
-    for (int i = 0; i < 4; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), 4 * G3_CH); }
-    for (int g = 0; g < NG; g++) { mbar_init(a_full(g, 0), 4); mbar_init(a_full(g, 1), 4); mbar_init(d_full(g), 1); }
-    for (int p = 0; p < 2; p++) { mbar_init(red_full(p), 4 * (NG - 1)); mbar_init(red_empty(p), 4); }
-    mbar_init(xp_full, NG * 128);
+#pragma unroll
+    for (int b = 0; b < G3_BARS; b++) mbar_init(bar(b), g3_bar_count(NC, b));
     *dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -116,10 +141,9 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
 #pragma unroll
     for (int j = 0; j < NC; j++) acc[j] = 0.0f;
     float d_p = 0.0f, dm_p = 0.0f;      // scales of the super-block whose accumulators are read next
-    int ti = 0, c = g;                  // the item: tile of this CTA, super-block of the slice (nsl >= NG)
+    G3Walk wk;
+    wk.start(g, st);
     int it = 0, ti_p = 0;               // items so far; the tile of the last one
-    int slot = (g / G3_CH) % st;        // the item's stage, and the parity of its use
-    uint32_t rpar = (uint32_t)((g / G3_CH) / st) & 1u;
     bool staged = false;
     // the accumulators of the last item into the row's sums
     auto drain = [&]() {
@@ -186,10 +210,9 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
       for (int j = 0; j < NC; j++) acc[j] = 0.0f;
     };
 #pragma unroll 1
-    while (ti < my_tiles) {
-      const int sub = c % G3_CH;
-      wait(raw_full(slot), rpar);
-      const uint8_t *row = ring + (size_t)slot * G3_STAGE + roff + sub * TB;
+    while (wk.ti < my_tiles) {
+      wait(bar(wk.full()), (uint32_t)wk.phase() & 1u);
+      const uint8_t *row = ring + (size_t)wk.slot * G3_STAGE + roff + wk.c % G3_CH * TB;
       const uint4 hd = *(const uint4 *)row;
       uint32_t scA, scB, mnA, mnB;
       k4_scales(hd.y, hd.z, hd.w, scA, scB, mnA, mnB);
@@ -214,7 +237,7 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
           // the operand buffer and the accumulators are free once the last item's MMAs are done and its sums are read
           if (it > 0) {
             drain();
-            if (ti != ti_p) flush(ti_p);
+            if (wk.ti != ti_p) flush(ti_p);
           }
           // the mins as fp16 numbers: m against the means' hi halves, m / 2048 against their lo halves, which are stored times 2048
           uint32_t mm[8];
@@ -233,18 +256,11 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
           if (lane == 0) mbar_arrive(a_full(g, gq >> 1));
         }
       }
-      if (lane == 0) mbar_arrive_n(raw_empty(slot), c + 1 == nsl && !sub ? G3_CH : 1);   // (a stage with one super-block stands for two)
+      if (lane == 0) mbar_arrive_n(raw_empty(wk.slot), wk.owed(nsl));
       d_p = h2f_bits(hd.x & 0xffffu) * 524288.0f; dm_p = h2f_bits(hd.x >> 16) * 32.0f;
-      ti_p = ti;
+      ti_p = wk.ti;
       it++;
-      {
-        // NG super-blocks on: as many stages as chunk boundaries lie between (a tile's last chunk may hold one)
-        int step = -(c / G3_CH);
-        c += NG;
-        if (c >= nsl) { c -= nsl; ti++; step += nch; }
-        slot += step + c / G3_CH;
-        if (slot >= st) { slot -= st; rpar ^= 1u; }
-      }
+      wk.next(NG, nsl, st);
       if (!staged) {
         // ---- the activation slice: eight pieces of sixteen bytes in flight a thread ----
         staged = true;
@@ -281,22 +297,22 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
     if (it > 0) { drain(); flush(ti_p); }
   } else if (warp == 4 * NG) {
     // ---- weights: lane t requests the t-th 16-row tile of every chunk ----
-    int slot = 0;
-    uint32_t par = 1;                   // a fresh barrier's "previous" phase is complete
+    int slot = 0, use = 0;
     for (int t = 0; t < my_tiles; t++) {
       int m;
       const int row0 = locate(ci + t * cps, m), have = min(8, ((a.m[m].rows + 15) >> 4) - (row0 >> 4));
       const uint8_t *src = a.m[m].W + ((size_t)((row0 >> 4) + lane) * a.nsb + sb0) * TB;
       for (int k = 0; k < nch; k++) {
         const int n = min(G3_CH, nsl - k * G3_CH);
-        wait(raw_empty(slot), par);
+        const uint32_t full = bar(G3_RAW_FULL + 4 * (use & 1) + slot);
+        if (use > 0) wait(raw_empty(slot), (uint32_t)(use - 1) & 1u);
         if (!*dead) {
-          if (lane == 0) mbar_expect(raw_full(slot), (uint32_t)(have * n * TB));
+          if (lane == 0) mbar_expect(full, (uint32_t)(have * n * TB));
           __syncwarp();
-          if (lane < have) bulk_load(ring_s + slot * G3_STAGE + lane * (G3_CH * TB), src + (size_t)k * G3_CH * TB, (uint32_t)(n * TB), raw_full(slot));
+          if (lane < have) bulk_load(ring_s + slot * G3_STAGE + lane * (G3_CH * TB), src + (size_t)k * G3_CH * TB, (uint32_t)(n * TB), full);
         }
         __syncwarp();
-        if (++slot == st) { slot = 0; par ^= 1u; }
+        if (++slot == st) { slot = 0; use++; }
       }
     }
   } else {

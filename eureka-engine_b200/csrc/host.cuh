@@ -68,6 +68,8 @@ int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int s
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a);   // fills tile0 / nsb, picks NT from xp.NC
 int gemm_setup(void);
 unsigned int *gemm_err_word(void);   // device word that a bounded wait sets when it runs out
+int gemm3_trace(int NC, int nsl, int tiles, int agent, int *ops, int cap);
+int gemm3_bar_count(int NC, int b);
 int gemm_wait_errors(void);
 int gemm_wait_errors_clear(void);
 int gemm_wait_selftest(cudaStream_t s, int which, int limit);

@@ -258,6 +258,13 @@ LLB_API int llb_spec_check_index(const char *index_text, size_t pack_bytes);
  * the conv ring across passes of both widths (0: none fits). */
 LLB_API int llb_b200_gemm_ksplit(int fmt, int nc, int ntiles, int nsb, int sms);
 LLB_API int llb_b200_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_prefill, int sms);
+/* Test entry (no GPU needed): what one agent of a CTA of the tcgen05 skinny GEMM does with the CTA's barriers, for a K-slice of nsl
+ * super-blocks and `tiles` row tiles at nc plane columns.  Agents: a warp of each group of workers (three groups, two at nc 32), then the
+ * warp that requests weights, then each group's issuing warp.  ops[3 i ..]: {0 wait, barrier, phase}, {1 arrive, barrier, times}, {2
+ * arrive, barrier, when what was requested here is done}.  Returns how many (at most cap ints are written), -1: no such slice.
+ * _bar_count: the arrivals that complete a phase of a barrier; -1 beyond the last. */
+LLB_API int llb_b200_gemm3_trace(int nc, int nsl, int tiles, int agent, int *ops, int cap);
+LLB_API int llb_b200_gemm3_bar_count(int nc, int bar);
 LLB_API void llb_spec_close(llb_spec *m);
 LLB_API int llb_spec_reset(llb_spec *m);                       /* host/llb_host.c:1915-1928 */
 LLB_API int llb_spec_prefill(llb_spec *m, const int *ids, int n);
