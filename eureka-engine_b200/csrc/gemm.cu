@@ -74,15 +74,23 @@ int gemm3_trace(int NC, int nsl, int tiles, int agent, int *ops, int cap) {
   auto op = [&](int kind, int b, int v) { if (3 * n + 2 < cap) { ops[3 * n] = kind; ops[3 * n + 1] = b; ops[3 * n + 2] = v; } n++; };
   if (agent < NG) {
     G3Walk wk;
-    int it = 0;
+    int it = 0, ti_p = 0;
+    auto flush = [&](int t) {
+      const G3Sum sm = g3_sum(NC, nsl, t);
+      if (sm.n > 0) op(0, G3_RED_EMPTY + sm.p, sm.n - 1);
+      if (agent != sm.owner) op(1, G3_RED_FULL + sm.p, 1);
+      else { op(0, G3_RED_FULL + sm.p, sm.n); op(1, G3_RED_EMPTY + sm.p, 1); }
+    };
     for (wk.start(agent, st); wk.ti < tiles; wk.next(NG, nsl, st)) {
       op(0, wk.full(), wk.phase());
-      if (it > 0) op(0, G3_D_FULL + agent, it - 1);
+      if (it > 0) { op(0, G3_D_FULL + agent, it - 1); if (wk.ti != ti_p) flush(ti_p); }
+      ti_p = wk.ti;
       for (int h = 0; h < 2; h++) op(1, G3_A_FULL + 2 * agent + h, 1);
       op(1, G3_RAW_EMPTY + wk.slot, wk.owed(nsl));
       if (it++ == 0) op(1, G3_XP_FULL, 32);
     }
     op(0, G3_D_FULL + agent, it - 1);
+    flush(ti_p);
   } else if (agent == NG) {
     const int nch = (nsl + G3_CH - 1) / G3_CH;
     for (int k = 0; k < tiles * nch; k++) {

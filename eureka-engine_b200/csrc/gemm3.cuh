@@ -75,11 +75,19 @@ struct G3Walk {
   // arrivals a warp owes its stage for the item (a stage with one super-block stands for two)
   __host__ __device__ __forceinline__ int owed(int nsl) const { return c + 1 == nsl && c % G3_CH == 0 ? G3_CH : 1; }
 };
+// The sums of a tile: the buffer where the other groups leave theirs, which use of the buffer that is, and the group that adds them up
+// (it has the tile's last super-block).  From the second use on EVERY group waits until the use before has been read, the adding group
+// too: it may have been a writer then and not know that the other writer had arrived, and the parity of that phase of red_full, still
+// pending, would read as this one's.
+struct G3Sum { int p, n, owner; };
+__host__ __device__ __forceinline__ G3Sum g3_sum(int NC, int nsl, int t) {
+  return G3Sum{NC <= 16 ? t & 1 : 0, NC <= 16 ? t >> 1 : t, ((t + 1) * nsl - 1) % g3_groups(NC)};
+}
 __host__ __device__ constexpr uint32_t g3_idesc(int N) { return 0x08000010u | ((uint32_t)(N >> 3) << 17); }   // kind::f16: D f32, A / B f16 K-major, M = 128
 
 template <int NC>
 __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, const int cps, const int st) {
-  constexpr int NG = g3_groups(NC), N = g3_n(NC), TB = tile_bytes(LLB_FM_Q4_K), RPB = NC <= 16 ? 2 : 1;
+  constexpr int NG = g3_groups(NC), N = g3_n(NC), TB = tile_bytes(LLB_FM_Q4_K);
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ks = blockIdx.x % a.ksplit, ci = blockIdx.x / a.ksplit;
@@ -164,9 +172,10 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
     // order, then hi + lo / 2048.  (Nothing but loads, sums and stores: with the matrix's fields read at every store a tile of
     // sixteen rows took 4700 cycles.)
     auto flush = [&](int t) {
-      const int p = RPB == 2 ? t & 1 : 0, n = RPB == 2 ? t >> 1 : t, og = ((t + 1) * nsl - 1) % NG;      // buffer, its use so far; that group
+      const G3Sum sm = g3_sum(NC, nsl, t);
+      const int p = sm.p, n = sm.n, og = sm.owner;
+      if (n > 0) wait(red_empty(p), (uint32_t)(n - 1) & 1u);
       if (g != og) {
-        if (n > 0) wait(red_empty(p), (uint32_t)(n - 1) & 1u);
         float *w = red + (size_t)(p * (NG - 1) + (g > og ? g - 1 : g)) * 128 * NC + r;
 #pragma unroll
         for (int j = 0; j < NC; j++) w[j * 128] = acc[j];
