@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
         const int n = min(G3_CH, nsl - k * G3_CH);
         const uint32_t full = bar(G3_RAW_FULL + 4 * (use & 1) + slot);
         if (use > 0) wait(raw_empty(slot), (uint32_t)(use - 1) & 1u);
-        if (!*dead) {
+        // (one answer for the warp: lanes that saw the word differently would leave bytes expected that nobody requests)
+        if (!__any_sync(0xffffffffu, *dead != 0)) {
           if (lane == 0) mbar_expect(full, (uint32_t)(have * n * TB));
           __syncwarp();
           if (lane < have) bulk_load(ring_s + slot * G3_STAGE + lane * (G3_CH * TB), src + (size_t)k * G3_CH * TB, (uint32_t)(n * TB), full);
