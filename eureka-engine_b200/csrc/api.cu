@@ -74,7 +74,7 @@ int llb_b200_init(int device) {
   CU_OK(cudaGetDeviceProperties(&pr, device));
   if (pr.major < 10) return llb_fail("device %d is sm_%d%d; this library is built for sm_100a only", device, pr.major, pr.minor);
   { const char *e = getenv("LLB_PDL"); g_llb.pdl = !(e && e[0] == '0'); }
-  { const char *e = getenv("LLB_GEMM3"); g_llb.gemm3 = e && e[0] == '1' ? 1 : e && e[0] == '0' ? -1 : 0; }
+  { const char *e = getenv("LLB_GEMM3"); g_llb.gemm3 = e && e[0] == '1' ? 1 : e && e[0] == '0' ? 0 : 2; }
   { const char *e = getenv("LLB_FFN_FUSED"); g_llb.ffn_fused = e && e[0] == '1'; }
   g_llb.sms = pr.multiProcessorCount;
   // a blocking stream: ordered after work a caller queued on the legacy default stream (torch's), so
@@ -247,13 +247,16 @@ int llb_b200_gemm_ksplit(int fmt, int nc, int ntiles, int nsb, int sms) { return
 int llb_b200_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_prefill, int sms) {
   return gemm_ring_ksplit(fmt, nsb, ntiles, nc_spec, nc_prefill, sms, 8);
 }
+int llb_b200_gemm_kernel(int fmt, int nc, int ntiles, int nsb, int sms, int alone, int *ksplit) {
+  return gemm_which(fmt, nc, ntiles, nsb, sms, alone != 0, ksplit);
+}
 int llb_b200_gemm3_trace(int nc, int nsl, int tiles, int agent, int *ops, int cap) { return gemm3_trace(nc, nsl, tiles, agent, ops, cap); }
 int llb_b200_gemm3_bar_count(int nc, int bar) { return gemm3_bar_count(nc, bar); }
 
 int llb_b200_use_tcgen05(int on) {
   NEED_INIT(-1)
   const int was = g_llb.gemm3;
-  g_llb.gemm3 = on < 0 ? -1 : on != 0;
+  g_llb.gemm3 = on == 2 ? 2 : on != 0;
   return was;
 }
 int llb_b200_use_fused_ffn(int on) {

@@ -10,7 +10,7 @@
 // tiles are ready when the activations come, it is the slower one (27B shape, 24 cycles of four rows 143.6 ms without it, 151 with
 // it; 24 passes of one row 121.7 and 123.4), alone the faster (gate|up at four rows 28.1 and 26.5 us, at one 28.2 and 24.6).
 static bool g3_fits(int fmt, int NC, int nsb, int ks, bool alone) {
-  if (g_llb.gemm3 < 0 || fmt != LLB_FM_Q4_K || (NC == 8 && !alone && g_llb.gemm3 == 0)) return false;
+  if (g_llb.gemm3 == 0 || fmt != LLB_FM_Q4_K || (NC == 8 && !alone && g_llb.gemm3 == 2)) return false;
   return ks >= 1 && nsb / ks >= g3_groups(NC) && g3_stages(NC, (nsb + ks - 1) / ks) >= 2;
 }
 static unsigned int *g_ffn_sync = nullptr;   // the fused FFN's grid barrier: two counters
@@ -241,7 +241,7 @@ static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct)
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
 static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, bool alone) {
   if (!g3_fits(fmt, NC, nsb, ks, alone)) return false;
-  if (g_llb.gemm3 > 0 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
+  if (g_llb.gemm3 == 1 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
   return g3_cost(NC, ntiles, nsb, ks, g_llb.sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, g_llb.sms, false, 24.0);
 }
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {
@@ -249,10 +249,19 @@ int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct,
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
     if (gemm_fix_ksplit(fmt, NC, nsb, ks, direct) != ks) continue;
+    if (g_llb.gemm3 == 1 && best_cost < 1e30 && !g3_fits(fmt, NC, nsb, ks, direct) && g3_fits(fmt, NC, nsb, best, direct)) continue;
     const double cost = g3_use(fmt, NC, ntiles, nsb, ks, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
-    if (cost < best_cost - 1e-9) { best_cost = cost; best = ks; }
+    // (the tcgen05 kernel asked for: before any split that it cannot take comes one that it can)
+    const bool asked = g_llb.gemm3 == 1 && g3_fits(fmt, NC, nsb, ks, direct) && !g3_fits(fmt, NC, nsb, best, direct);
+    if (cost < best_cost - 1e-9 || asked) { best_cost = cost; best = ks; }
   }
   return gemm_fix_ksplit(fmt, NC, nsb, best, direct);
+}
+
+int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit) {
+  const int ks = gemm_fix_ksplit(fmt, NC, nsb, *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, NC, ntiles, nsb, sms, alone), alone);
+  *ksplit = ks;
+  return g3_use(fmt, NC, ntiles, nsb, ks, alone) ? 3 : 2;
 }
 
 // One K-split for a launch whose partial sums outlive the pass (attn_qkv into the conv ring): valid at both

@@ -12,7 +12,7 @@ struct LlbCtx {
   int device = -1;
   int sms = 0;
   int ffn_fused = 0;   // the FFN as one launch with a grid barrier (LLB_FFN_FUSED=1)
-  int gemm3 = 0;   // the tcgen05 kernel of Q4_K launches: 0 where it is the faster one, 1 wherever it can run (LLB_GEMM3=1), -1 never (LLB_GEMM3=0)
+  int gemm3 = 2;   // the tcgen05 kernel of Q4_K launches: 0 never (LLB_GEMM3=0), 1 wherever it can run (LLB_GEMM3=1), 2 where it is the faster one
   int pdl = 1;     // programmatic dependent launch on every kernel of a pass (LLB_PDL=0 turns it off)
   cudaStream_t stream = nullptr;
   char err[512] = {0};
@@ -63,6 +63,7 @@ inline cudaError_t llb_launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block
 // gemm.cu
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct = false, double stage = 24.0);   // direct: the caller adds the slices with a launch of its own; stage: cycles to stage a plane column of a super-block
 int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone = false);   // clamps a requested K-split to what a kernel can take; alone: not one of a pass's launches
+int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit);   // 2 mma.sync, 3 tcgen05; *ksplit 0: picked here
 int gemm_longest_slice(int fmt, int NC);   // super-blocks of the longest K-slice a launch takes
 int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int sms, int cap);
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a);   // fills tile0 / nsb, picks NT from xp.NC

@@ -98,10 +98,10 @@ LLB_API int llb_b200_xp_set_bf16(llb_xp *xp, llb_b200_dptr x_bf16 /* [T][K] */);
  * out_i: f32 [T][rows_i].  ksplit = 0 picks the K-split; scratch for the partial sums is internal. */
 LLB_API int llb_b200_gemm(int fmt, int nmat, const llb_b200_dptr *w, const int *rows, const llb_b200_dptr *out, int K, const llb_xp *xp,
                   int ksplit);
-/* Every Q4_K GEMM that can run there on the tcgen05 kernel (weights unpacked into tensor memory, tcgen05.mma) instead
- * of the mma.sync one; returns the previous setting.  Also set by LLB_GEMM3=1 at llb_b200_init.  Off (0) by
- * default: each launch then takes the kernel that is the faster one at its size (LLB_GEMM3=0 at llb_b200_init keeps all of them
- * on mma.sync).  A speculative engine keeps the kernels it was opened with. */
+/* Which of the two kernels Q4_K GEMMs take: 0 the mma.sync one, all of them; 1 the tcgen05 one (weights unpacked into tensor
+ * memory, tcgen05.mma) wherever it can run: three super-blocks a K-slice and more, two at nine to sixteen rows; 2, the default, the one
+ * that is the faster at the launch's size.  Returns the previous setting.  LLB_GEMM3=0 or 1 in the environment of llb_b200_init sets
+ * 0 or 1.  A speculative engine keeps the kernels it was opened with. */
 LLB_API int llb_b200_use_tcgen05(int on);
 /* The SwiGLU FFN of engines opened from now on as ONE launch (gate|up GEMM, grid-wide barrier, silu(gate) * up built in
  * shared memory, down GEMM) instead of three; returns the previous setting.  Also LLB_FFN_FUSED=1 at llb_b200_init.  Off by
@@ -258,6 +258,9 @@ LLB_API int llb_spec_check_index(const char *index_text, size_t pack_bytes);
  * the conv ring across passes of both widths (0: none fits). */
 LLB_API int llb_b200_gemm_ksplit(int fmt, int nc, int ntiles, int nsb, int sms);
 LLB_API int llb_b200_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_prefill, int sms);
+/* Test entry (no GPU needed): the kernel of such a launch, 2 mma.sync, 3 tcgen05, of the operator (alone != 0) or of a pass, and in
+ * *ksplit its K-slices: on entry what is asked for, 0 for the launch's own choice. */
+LLB_API int llb_b200_gemm_kernel(int fmt, int nc, int ntiles, int nsb, int sms, int alone, int *ksplit);
 /* Test entry (no GPU needed): what one agent of a CTA of the tcgen05 skinny GEMM does with the CTA's barriers, for a K-slice of nsl
  * super-blocks and `tiles` row tiles at nc plane columns.  Agents: a warp of each group of workers (three groups, two at nc 32), then the
  * warp that requests weights, then each group's issuing warp.  ops[3 i ..]: {0 wait, barrier, phase}, {1 arrive, barrier, times}, {2
