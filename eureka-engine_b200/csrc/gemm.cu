@@ -239,10 +239,10 @@ static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct)
   return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0) + (direct ? 0.0 : 4000.0);
 }
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
-static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, bool alone) {
+static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool alone) {
   if (!g3_fits(fmt, NC, nsb, ks, alone)) return false;
   if (g_llb.gemm3 == 1 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
-  return g3_cost(NC, ntiles, nsb, ks, g_llb.sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, g_llb.sms, false, 24.0);
+  return g3_cost(NC, ntiles, nsb, ks, sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, false, 24.0);
 }
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {
   int best = 1;
@@ -250,7 +250,7 @@ int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct,
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
     if (gemm_fix_ksplit(fmt, NC, nsb, ks, direct) != ks) continue;
     if (g_llb.gemm3 == 1 && best_cost < 1e30 && !g3_fits(fmt, NC, nsb, ks, direct) && g3_fits(fmt, NC, nsb, best, direct)) continue;
-    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
+    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, sms, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
     // (the tcgen05 kernel asked for: before any split that it cannot take comes one that it can)
     const bool asked = g_llb.gemm3 == 1 && g3_fits(fmt, NC, nsb, ks, direct) && !g3_fits(fmt, NC, nsb, best, direct);
     if (cost < best_cost - 1e-9 || asked) { best_cost = cost; best = ks; }
@@ -261,7 +261,7 @@ int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct,
 int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit) {
   const int ks = gemm_fix_ksplit(fmt, NC, nsb, *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, NC, ntiles, nsb, sms, alone), alone);
   *ksplit = ks;
-  return g3_use(fmt, NC, ntiles, nsb, ks, alone) ? 3 : 2;
+  return g3_use(fmt, NC, ntiles, nsb, ks, sms, alone) ? 3 : 2;
 }
 
 // One K-split for a launch whose partial sums outlive the pass (attn_qkv into the conv ring): valid at both
@@ -405,7 +405,7 @@ int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a) {
   if (gemm_prepare(fmt, a)) return -1;
   if (a.tile0[a.nmat] < 1) return 0;
   const int NT = a.xp.NC / 8;
-  if (g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit, a.alone)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
+  if (g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit, g_llb.sms, a.alone)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
   if (fmt == LLB_FM_Q4_K) return NT == 1 ? launch_two<LLB_FM_Q4_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q4_K, 2>(s, a) : launch_two<LLB_FM_Q4_K, 4>(s, a);
   if (fmt == LLB_FM_Q5_K) return NT == 1 ? launch_two<LLB_FM_Q5_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q5_K, 2>(s, a) : launch_two<LLB_FM_Q5_K, 4>(s, a);
   if (fmt == LLB_FM_Q6_K) return NT == 1 ? launch_two<LLB_FM_Q6_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q6_K, 2>(s, a) : launch_two<LLB_FM_Q6_K, 4>(s, a);

@@ -27,3 +27,20 @@ def test_the_setting_decides_for_every_launch(llb, nc, rows, K):
         assert L.llb_b200_use_tcgen05(was) == 1
     assert kernel(L, nc, 34816, 5120)[0] == 3 and kernel(L, nc, 16, 1024)[0] == 2
     assert kernel(L, 8, rows, K, alone=False)[0] == 2       # a pass of up to four rows
+
+
+def test_the_number_of_sms_asked_about_decides(pkg):
+    """The launch's kernel and K-slices on 148 SMs, without a device: the same as where such a device is in use."""
+    L = pkg.llb.lib()
+    assert L.llb_b200_gemm_ksplit(Q4_K, 16, 320, 20, 148) == kernel(L, 16, 5120, 5120, alone=False)[1] == 4
+    assert L.llb_b200_gemm_ksplit(Q4_K, 16, 256, 16, 148) == 4
+    assert kernel(L, 16, 17408, 5120, alone=False)[0] == 3
+    # on few SMs a launch has tiles for all of them whatever the kernel; on very many the tcgen05 kernel's 128-row tiles leave most idle
+    assert kernel(L, 16, 2048, 2048, sms=16)[0] == 3 and kernel(L, 16, 2048, 2048, sms=2000)[0] == 2
+
+
+@pytest.mark.gpu
+def test_the_device_in_use_decides_nothing_about_others(llb):
+    L = llb.lib()
+    assert L.llb_b200_sm_count() == 148
+    test_the_number_of_sms_asked_about_decides(type("P", (), {"llb": llb}))
