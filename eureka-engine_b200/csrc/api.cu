@@ -250,6 +250,7 @@ int llb_b200_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_prefi
 int llb_b200_gemm_kernel(int fmt, int nc, int ntiles, int nsb, int sms, int alone, int *ksplit) {
   return gemm_which(fmt, nc, ntiles, nsb, sms, alone != 0, ksplit);
 }
+int llb_b200_gemm_fits(int fmt, int nc, int nsb, int cap) { return gemm_fits(fmt, nc, nsb, cap); }
 int llb_b200_gemm3_trace(int nc, int nsl, int tiles, int agent, int *ops, int cap) { return gemm3_trace(nc, nsl, tiles, agent, ops, cap); }
 int llb_b200_gemm3_bar_count(int nc, int bar) { return gemm3_bar_count(nc, bar); }
 

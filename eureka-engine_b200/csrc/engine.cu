@@ -465,10 +465,7 @@ static int load_moe(llb_spec *m, FfnW &w, const std::string &p, const std::unord
 // the conv ring's launch RING_MAXSPLIT.
 static bool width_fits(const llb_spec *m, const std::unordered_map<std::string, TensorRec> &tab, int T) {
   const int NC = nc_of(T);
-  auto fits = [&](int fmt, int nsb, int cap) {
-    const int ks = cap > 1 ? gemm_fix_ksplit(fmt, NC, nsb, 1) : 1;
-    return ks <= cap && (nsb + ks - 1) / ks <= gemm_longest_slice(fmt, NC);
-  };
+  auto fits = [&](int fmt, int nsb, int cap) { return gemm_fits(fmt, NC, nsb, cap); };
   for (const auto &kv : tab) {
     const TensorRec &t = kv.second;
     const std::string &n = kv.first;

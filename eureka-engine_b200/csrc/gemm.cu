@@ -216,7 +216,11 @@ int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone) {
   return ks;
 }
 
-int gemm_longest_slice(int fmt, int NC) { return g2_longest_slice(fmt, NC); }
+// (the fewest slices that either kernel takes, held against the room of the kernel that takes them)
+bool gemm_fits(int fmt, int NC, int nsb, int cap) {
+  const int ks = gemm_fix_ksplit(fmt, NC, nsb, 1);
+  return ks <= cap && (g3_fits(fmt, NC, nsb, ks, false) || (nsb + ks - 1) / ks <= g2_longest_slice(fmt, NC));
+}
 
 // K-slices per row tile: streaming, the staging of the slice, and a charge per slice for the partial sums that the consumer
 // has to add (direct: a launch of its own adds them, 1.5 us).  At 32 plane columns a warp's chain is nearer 3000 cycles a tile

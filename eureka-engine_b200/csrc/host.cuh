@@ -64,7 +64,7 @@ inline cudaError_t llb_launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block
 int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct = false, double stage = 24.0);   // direct: the caller adds the slices with a launch of its own; stage: cycles to stage a plane column of a super-block
 int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone = false);   // clamps a requested K-split to what a kernel can take; alone: not one of a pass's launches
 int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit);   // 2 mma.sync, 3 tcgen05; *ksplit 0: picked here
-int gemm_longest_slice(int fmt, int NC);   // super-blocks of the longest K-slice a launch takes
+bool gemm_fits(int fmt, int NC, int nsb, int cap);   // whether a pass's launch can take nsb super-blocks in at most cap K-slices
 int gemm_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int nc_pf, int sms, int cap);
 int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a);   // fills tile0 / nsb, picks NT from xp.NC
 int gemm_setup(void);

@@ -261,6 +261,8 @@ LLB_API int llb_b200_ring_ksplit(int fmt, int nsb, int ntiles, int nc_spec, int 
 /* Test entry (no GPU needed): the kernel of such a launch, 2 mma.sync, 3 tcgen05, of the operator (alone != 0) or of a pass, and in
  * *ksplit its K-slices: on entry what is asked for, 0 for the launch's own choice. */
 LLB_API int llb_b200_gemm_kernel(int fmt, int nc, int ntiles, int nsb, int sms, int alone, int *ksplit);
+/* ... and whether a pass's launch of nc plane columns can take nsb super-blocks in at most cap K-slices: 1 or 0. */
+LLB_API int llb_b200_gemm_fits(int fmt, int nc, int nsb, int cap);
 /* Test entry (no GPU needed): what one agent of a CTA of the tcgen05 skinny GEMM does with the CTA's barriers, for a K-slice of nsl
  * super-blocks and `tiles` row tiles at nc plane columns.  Agents: a warp of each group of workers (three groups, two at nc 32), then the
  * warp that requests weights, then each group's issuing warp.  ops[3 i ..]: {0 wait, barrier, phase}, {1 arrive, barrier, times}, {2

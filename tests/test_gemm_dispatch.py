@@ -44,3 +44,17 @@ def test_the_device_in_use_decides_nothing_about_others(llb):
     L = llb.lib()
     assert L.llb_b200_sm_count() == 148
     test_the_number_of_sms_asked_about_decides(type("P", (), {"llb": llb}))
+
+
+@pytest.mark.parametrize("cap", [8, 16])
+@pytest.mark.parametrize("nc", [8, 16, 32])
+@pytest.mark.parametrize("fmt", [Q4_K, 9, 4, 1])
+def test_a_width_fits_where_a_launch_can_be_made(pkg, fmt, nc, cap):
+    """Columns up to 512 super-blocks: no narrower matrix is refused than one that is taken, and each kernel's slices are held against its
+    own room."""
+    L = pkg.llb.lib()
+    fits = [bool(L.llb_b200_gemm_fits(fmt, nc, n, cap)) for n in range(1, 513)]
+    assert fits == sorted(fits, reverse=True)
+    assert fits[:cap * {8: 13, 16: 7, 32: 4}[nc]] == [True] * (cap * {8: 13, 16: 7, 32: 4}[nc])
+    if fmt == Q4_K and nc == 16:
+        assert L.llb_b200_gemm_fits(fmt, nc, 14, cap) == 1   # 3584 columns: one slice of the tcgen05 kernel, two of the other one
