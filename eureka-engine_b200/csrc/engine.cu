@@ -70,6 +70,7 @@ struct llb_spec {
   int L = 0, d = 0, H = 0, KV = 0, hd = 0, f = 0, V = 0, interval = 4, KC = 4, SZ = 128, GK = 0, TR = 0, vdc = 0, kdc = 0,
       convd = 0, rope_dim = 64;
   float rope_base = 1e7f, eps = 1e-6f;
+  const int gemm3 = g_llb.gemm3;   // llb_b200_use_tcgen05's setting at open: the engine's launches keep to it
   int ne = 0, nk = 0, ef = 0, sf = 0;   // routed experts, experts per token, expert width, shared expert width (ne = 0: dense FFN)
   float *moe_lg = nullptr, *moe_wt = nullptr, *moe_g = nullptr, *moe_u = nullptr, *hn2 = nullptr;
   int *moe_ids = nullptr;
@@ -162,13 +163,15 @@ static inline float *kc_of(const llb_spec *m, float *base, int b) { return base 
 static inline float *ring_of(const llb_spec *m, int il, int b) { return m->ring[il] + (size_t)b * m->ring_ks[il] * CONV_RING * m->convd; }
 static inline float *state_of(const llb_spec *m, int il, int b) { return m->S[il] + (size_t)b * m->s_group; }
 static inline int *hist_of(const llb_spec *m, int b) { return m->hist ? m->hist + (size_t)b * (m->max_ctx + 16) : nullptr; }
-// the launchers' stream geometry while this engine enqueues (engines of different shapes may coexist)
+// the launchers' stream geometry and GEMM kernels while this engine enqueues (engines of different shapes may coexist)
 struct StreamScope {
   Streams was;
-  explicit StreamScope(const llb_spec *m, bool single = false) : was(ops_streams()) {
+  const int was_gemm3;
+  explicit StreamScope(const llb_spec *m, bool single = false) : was(ops_streams()), was_gemm3(g_llb.gemm3) {
     if (m->B > 1 && !single) ops_set_streams(m->per, (int)sizeof(SpecCtl)); else ops_set_streams(0, 0);
+    g_llb.gemm3 = m->gemm3;
   }
-  ~StreamScope() { ops_set_streams(was.per, was.stride); }
+  ~StreamScope() { ops_set_streams(was.per, was.stride); g_llb.gemm3 = was_gemm3; }
 };
 
 #define CK(call) do { if ((call)) return -1; } while (0)

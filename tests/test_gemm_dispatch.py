@@ -58,3 +58,30 @@ def test_a_width_fits_where_a_launch_can_be_made(pkg, fmt, nc, cap):
     assert fits[:cap * {8: 13, 16: 7, 32: 4}[nc]] == [True] * (cap * {8: 13, 16: 7, 32: 4}[nc])
     if fmt == Q4_K and nc == 16:
         assert L.llb_b200_gemm_fits(fmt, nc, 14, cap) == 1   # 3584 columns: one slice of the tcgen05 kernel, two of the other one
+
+
+@pytest.mark.gpu
+def test_an_engine_keeps_the_kernels_it_was_opened_with(pkg, packs, llb):
+    """Six rows a pass of a Q4_K model of three super-blocks' width, opened with the tcgen05 kernel asked for; the setting then changes, and
+    the cycle graph is captured again for a sampler: the same bits as without the change."""
+    import numpy as np
+    L = llb.lib()
+    cfg = packs.cfg_tiny(d_model=768, d_ff=1024, quant="q4_k_s")
+    pack = packs.build_pack(cfg)
+    prompt = packs.synth_prompt(3, 21, cfg.vocab_size)
+    out = []
+    for later in (1, 0, 2):
+        was = L.llb_b200_use_tcgen05(1)
+        eng = pkg.llb.SpecEngine(pack, None, k=5, max_ctx=96)
+        try:
+            L.llb_b200_use_tcgen05(later)
+            eng.set_sampler(pkg.llb.SmpParams.make(temp=0.8, top_k=20, seed=9))
+            eng.prefill(prompt)
+            out.append(eng.generate(24))
+            assert L.llb_b200_use_tcgen05(later) == later
+        finally:
+            L.llb_b200_use_tcgen05(was)
+            eng.close()
+    for ids, top2 in out[1:]:
+        assert np.array_equal(ids, out[0][0]) and np.array_equal(top2, out[0][1])
+    assert L.llb_b200_wait_errors() == 0
