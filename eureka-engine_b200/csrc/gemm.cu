@@ -8,7 +8,7 @@
 // Can the tcgen05 kernel take this K-split?  (a super-block of every tile for each of its groups, two stages beside the planes)
 // At 8 plane columns it is for launches on their own: between the small kernels of a pass, where the mma.sync kernel's ring and first
 // tiles are ready when the activations come, it is the slower one (27B shape, 24 cycles of four rows 143.6 ms without it, 151 with
-// it; 24 passes of one row 121.7 and 123.4), alone the faster (gate|up at four rows 28.1 and 26.5 us, at one 28.2 and 24.6).
+// it; 24 passes of one row 121.7 and 123.4), alone the faster (gate|up at four rows 28.3 and 27.1 us, at one 28.1 and 25.1).
 static bool g3_fits(int fmt, int NC, int nsb, int ks, bool alone) {
   if (g_llb.gemm3 == 0 || fmt != LLB_FM_Q4_K || (NC == 8 && !alone && g_llb.gemm3 == 2)) return false;
   return ks >= 1 && nsb / ks >= g3_groups(NC) && g3_stages(NC, (nsb + ks - 1) / ks) >= 2;
@@ -85,9 +85,11 @@ int gemm3_trace(int NC, int nsl, int tiles, int agent, int *ops, int cap) {
       op(0, wk.full(), wk.phase());
       if (it > 0) { op(0, G3_D_FULL + agent, it - 1); if (wk.ti != ti_p) flush(ti_p); }
       ti_p = wk.ti;
-      for (int h = 0; h < 2; h++) op(1, G3_A_FULL + 2 * agent + h, 1);
+      op(1, G3_A_FULL + 2 * agent, 1);
+      if (g3_reuse(NC)) { if (it == 0) op(1, G3_XP_FULL, 32); op(0, G3_HALF + agent, it); }
+      op(1, G3_A_FULL + 2 * agent + 1, 1);
       op(1, G3_RAW_EMPTY + wk.slot, wk.owed(nsl));
-      if (it++ == 0) op(1, G3_XP_FULL, 32);
+      if (it++ == 0 && !g3_reuse(NC)) op(1, G3_XP_FULL, 32);
     }
     op(0, G3_D_FULL + agent, it - 1);
     flush(ti_p);
@@ -102,7 +104,9 @@ int gemm3_trace(int NC, int nsl, int tiles, int agent, int *ops, int cap) {
     const int g = agent - NG - 1;
     for (int s = g, k = 0; s < tiles * nsl; s += NG, k++) {
       if (k == 0) op(0, G3_XP_FULL, 0);
-      for (int h = 0; h < 2; h++) op(0, G3_A_FULL + 2 * g + h, k);
+      op(0, G3_A_FULL + 2 * g, k);
+      if (g3_reuse(NC)) op(2, G3_HALF + g, 1);
+      op(0, G3_A_FULL + 2 * g + 1, k);
       op(2, G3_D_FULL + g, 1);
     }
   }
@@ -239,7 +243,7 @@ static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int 
 // worth that much; without it the 2048-column launches of the 35B-A3B shape came here and eight of its streams took 156 ms instead of 147.
 static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
-  const double sb = NC >= 32 ? 970.0 : 820.0;
+  const double sb = NC >= 32 ? 990.0 : NC >= 16 ? 860.0 : 835.0;
   return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0) + (direct ? 0.0 : 4000.0);
 }
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).

@@ -5,12 +5,17 @@
 // MMAs grows with the rows (60 us at sixteen).  Here
 //   * the multiply is tcgen05.mma (M = 128 weight rows, N = 16 or 32 plane columns, K = 16) with the weight operand in TENSOR
 //     MEMORY, which costs the SM's issue slots nothing and does not grow with the rows;
-//   * the six-bit scale is multiplied into the code: sc * q <= 63 * 15 is an exact fp16 number, so a whole super-block of 256
+//   * the six-bit scale is multiplied into the code: sc * (q - 8) is an exact fp16 number, so a whole super-block of 256
 //     columns accumulates into ONE fp32 accumulator and d comes in once per super-block.  A row of a super-block is 32 words,
-//     nine instructions each for eight products: about 200 warp instructions a 16 x 256 tile against 351;
-//   * the "min" term is one extra MMA a super-block into an accumulator of its own, as in gemm2.cuh.
-// gate|up, operator alone, cold weights: 28.2 -> 24.5 us at one row, 28.2 -> 27 at four, 37.3 -> 32 at eight, 60 -> 46.5 at
-// sixteen.  What is left: the activations, which every SM reads from L2 at about 10 bytes a cycle (4 us for four rows of 5120
+//     nine instructions each for eight products: about 210 warp instructions a 16 x 256 tile against 351;
+//   * what the 8 took, and the "min" term, are an MMA each against the means of the sub-blocks, the second into an accumulator of its
+//     own, as in gemm2.cuh.  The tensor core truncates where it adds to an accumulator.  With q from 0 to 15 the sixteen MMAs of a
+//     super-block climb, for activations with a mean, to a sum that the min term then all but cancels, and sixteen truncations of one
+//     sign are left: x = 1 + 0.1 N against quantised Gaussian weights, 5120 columns, 6.5e-5 of the result's norm off 64 bits (k_gemm2 3.5e-6).
+//     Centred, the climb is one MMA, the chain's last: 2.3e-6; N(0, 1) 7e-7 -> 3.1e-7 (3.4e-7 to 1.2e-6), silu(g) u 7e-7 -> 3.8e-7 (4e-7 to
+//     5e-6); |N| 2.3e-6 at 5120 columns and 3.7e-6 at 17408 (1.7e-6 and 2.1e-6; at sixteen rows 2.3e-5 and 4.2e-5).
+// gate|up of the 27B shape, operator alone, cold weights: 28.1 -> 25.1 us at one row, 28.3 -> 27.1 at four, 37.3 -> 34.3 at eight, 60.2 -> 53.9
+// at sixteen (not centred 24.7, 26.7, 32.8, 52.8).  What is left: the activations, which every SM reads from L2 at about 10 bytes a cycle (4 us for four rows of 5120
 // columns; cp.async or plain loads, in one order or a different one in every CTA), the groups' chains (2300 cycles a super-block, three groups),
 // and tiles of 128 rows that do not divide evenly.
 //
@@ -21,11 +26,10 @@
 // kernel, 990 cycles a super-block, a third of them in waits that find their phase complete), one requests the weights (two
 // super-blocks of eight 16-row tiles a stage, a bulk copy a tile).  At the end of a tile the other groups leave their sums in shared memory
 // and the group that came last adds them in order and writes.
-//   Tensor memory (512 columns): the groups' operands (128 columns of products, 8 of mins), then their accumulators (N + N).
-//   Three groups where that fits (N = 16), two at N = 32.
+//   Tensor memory: see g3_reuse.  Three groups at N = 16, two at N = 32.
 //   Shared memory: activation planes of the K-slice as K-major core matrices [k / 8][column][8 halves] (their k-order 0 2 1 3 4 6
 //   5 7 is the one the unpack produces), the sub-block means likewise, the groups' sums, the ring.
-//   N is 16 at least, and with 8 plane columns the upper half of an accumulator is whatever the next k-group's columns give; nobody
+//   N is 16 at least, and with 8 plane columns half of an accumulator is whatever a neighbouring k-group's columns give; nobody
 //   reads it.
 // Every wait is bounded; one that runs out sets *err, all roles then run through without waiting, copies in flight get time to
 // land, tensor memory is freed and the kernel returns.
@@ -35,11 +39,21 @@ static_assert(GEMM_MAXMAT == 4, "k_gemm3 finds a tile's matrix with three compar
 
 #define G3_HDR 256
 #define G3_SMEM_MAX 231424
-#define G3_A_COLS 136
 #define G3_CH 2                // super-blocks a copy brings
 #define G3_STAGE (8 * G3_CH * tile_bytes(LLB_FM_Q4_K))
 __host__ __device__ constexpr int g3_groups(int NC) { return NC <= 16 ? 3 : 2; }
 __host__ __device__ constexpr int g3_n(int NC) { return NC <= 16 ? 16 : 32; }
+// Tensor memory: the groups' operands -- 128 columns of products, behind them 16 of scales and mins --, then the groups' accumulators, D of
+// the products and the scales' part, P of the mins.  Three groups are short of room:
+//   8 plane columns: half of each N = 16 is nothing anybody reads.  D's is the upper half; P's B operand starts a column group
+//     early, so that its own is the lower one, and the two lie over one another: 24 columns.
+//   16: scales and mins take the place of the first half of the products once that half's MMAs are done (a wait more an item: 4 % of
+//     the operator's time where it was measured, at 8).
+__host__ __device__ constexpr bool g3_reuse(int NC) { return NC == 16; }
+__host__ __device__ constexpr int g3_a_cols(int NC) { return g3_reuse(NC) ? 128 : 144; }
+__host__ __device__ constexpr int g3_p_col(int NC) { return NC == 8 ? 8 : g3_n(NC); }    // P behind D
+__host__ __device__ constexpr int g3_d_cols(int NC) { return g3_p_col(NC) + g3_n(NC); }
+static_assert(3 * (g3_a_cols(8) + g3_d_cols(8)) <= 512 && 3 * (g3_a_cols(16) + g3_d_cols(16)) <= 512 && 2 * (g3_a_cols(32) + g3_d_cols(32)) <= 512, "tensor memory");
 __host__ __device__ constexpr int g3_threads(int NC) { return g3_groups(NC) * 160 + 32; }
 __host__ __device__ constexpr int g3_red_bytes(int NC) { return (NC <= 16 ? 2 : 1) * (g3_groups(NC) - 1) * 128 * NC * 4; }
 // planes and means of a K-slice of nsl super-blocks (and what the MMAs read beyond the last column)
@@ -52,9 +66,9 @@ __host__ __device__ inline int g3_stages(int NC, int nsl) {
 // A stage has two raw_full barriers that its uses take in turn: a group passes over chunks, and bulk copies land in any order, so
 // it comes to use u of a stage without having seen use u - 1 land; with one barrier the parity of a phase that is still
 // pending reads as use u complete.  Use u - 2 of the stage it knows to have landed (g3_walk below).
-enum { G3_RAW_FULL = 0 /* [2][4] */, G3_RAW_EMPTY = 8, G3_A_FULL = 12 /* [3][2] */, G3_D_FULL = 18, G3_RED_FULL = 21, G3_RED_EMPTY = 23, G3_XP_FULL = 25, G3_BARS = 26 };
+enum { G3_RAW_FULL = 0 /* [2][4] */, G3_RAW_EMPTY = 8, G3_A_FULL = 12 /* [3][2] */, G3_D_FULL = 18, G3_RED_FULL = 21, G3_RED_EMPTY = 23, G3_XP_FULL = 25, G3_HALF = 26 /* [3] */, G3_BARS = 29 };
 __host__ __device__ constexpr int g3_bar_count(int NC, int b) {
-  return b < G3_RAW_EMPTY ? 1 : b < G3_A_FULL ? 4 * G3_CH : b < G3_D_FULL ? 4 : b < G3_RED_FULL ? 1 : b < G3_RED_EMPTY ? 4 * (g3_groups(NC) - 1) : b < G3_XP_FULL ? 4 : g3_groups(NC) * 128;
+  return b < G3_RAW_EMPTY ? 1 : b < G3_A_FULL ? 4 * G3_CH : b < G3_D_FULL ? 4 : b < G3_RED_FULL ? 1 : b < G3_RED_EMPTY ? 4 * (g3_groups(NC) - 1) : b < G3_XP_FULL ? 4 : b < G3_HALF ? g3_groups(NC) * 128 : 1;
 }
 // A group's walk: the item (tile of the CTA, super-block of the slice), the stage it lies in and which use of that stage.  nsl >= NG,
 // so that every group has an item in every tile; st >= 2.  NG super-blocks on are two chunks on at most (a tile's last chunk may hold
@@ -97,6 +111,7 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
   auto bar = [&](int b) { return bar_s + 8u * b; };
   auto raw_empty = [&](int i) { return bar(G3_RAW_EMPTY + i); };
   auto a_full = [&](int g, int h) { return bar(G3_A_FULL + 2 * g + h); };
+  auto half_done = [&](int g) { return bar(G3_HALF + g); };
   auto d_full = [&](int g) { return bar(G3_D_FULL + g); };
   auto red_full = [&](int p) { return bar(G3_RED_FULL + p); };
   auto red_empty = [&](int p) { return bar(G3_RED_EMPTY + p); };
@@ -143,7 +158,7 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
     // ---- workers: group g, row r of the tile ----
     const int g = warp >> 2, q = warp & 3, r = 32 * q + lane;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
-    const uint32_t abuf = tmem + lane_off + (uint32_t)(g * G3_A_COLS), dbuf = tmem + lane_off + (uint32_t)(NG * G3_A_COLS + g * 2 * N);
+    const uint32_t abuf = tmem + lane_off + (uint32_t)(g * g3_a_cols(NC)), dbuf = tmem + lane_off + (uint32_t)(NG * g3_a_cols(NC) + g * g3_d_cols(NC));
     const uint32_t roff = (uint32_t)(r >> 4) * (G3_CH * TB) + (r & 15) * tile_row(LLB_FM_Q4_K);
     float acc[NC];
 #pragma unroll
@@ -152,7 +167,19 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
     G3Walk wk;
     wk.start(g, st);
     int it = 0, ti_p = 0;               // items so far; the tile of the last one
-    bool staged = false;
+    // What stands against the means of the activations' sub-blocks (hi halves, and lo halves, which are stored times 2048), as fp16:
+    // 8 s 32 2^-19 = s / 2048 and that over 2048, the products' offset; m and m / 2048
+    auto store_means = [&](uint32_t at, uint32_t scA, uint32_t scB, uint32_t mnA, uint32_t mnB) {
+      uint32_t s8[8], mm[8];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const uint32_t sel = (j & 1) ? 0x4342u : 0x4140u, s = __byte_perm(j < 2 ? scA : scB, 0x64646464u, sel), m = __byte_perm(j < 2 ? mnA : mnB, 0x64646464u, sel);
+        s8[2 * j] = g2_hfma2(s, 0x10001000u, 0xb800b800u); s8[2 * j + 1] = g2_hfma2(s, 0x00040004u, 0x8c008c00u);
+        mm[2 * j] = g2_hfma2(m, 0x3c003c00u, 0xe400e400u); mm[2 * j + 1] = g2_hfma2(m, 0x10001000u, 0xb800b800u);
+      }
+      t5_st8(at, s8);
+      t5_st8(at + 8, mm);
+    };
     // the accumulators of the last item into the row's sums
     auto drain = [&]() {
       wait(d_full(g), (uint32_t)(it - 1) & 1u);
@@ -161,7 +188,7 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
       for (int j0 = 0; j0 < NC; j0 += 8) {
         float v[8], p[8];
         t5_ld8(dbuf + j0, v);
-        t5_ld8(dbuf + N + j0, p);
+        t5_ld8(dbuf + g3_p_col(NC) + (NC == 8 ? 8 : 0) + j0, p);
         t5_wait_ld();
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[j0 + j] += d_p * v[j] - dm_p * p[j];
@@ -218,6 +245,37 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
 #pragma unroll
       for (int j = 0; j < NC; j++) acc[j] = 0.0f;
     };
+    // the activation slice: eight pieces of sixteen bytes in flight a thread
+    auto stage = [&]() {
+      pdl_wait();
+      const int half = NC / 2, T = a.T, np = nsl * 32 * NC, nm = nsl * 2 * NC;
+      const bool two = a.planes == 2;
+      const uint8_t *xh = (const uint8_t *)(a.xp.xh + (size_t)sb0 * 256), *xf = (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
+      const size_t cs = (size_t)a.K * 2;
+      auto live = [&](int col) { return (two && col >= half ? col - half : col) < T; };
+      // (four k-groups of eight columns a warp: whole sectors of the source, whole rows of core matrices at the destination)
+#pragma unroll 1
+      for (int i0 = tid; i0 < np; i0 += 8 * NG * 128) {
+        uint4 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const int i = i0 + u * NG * 128, blk = i >> 5, col = blk % (NC / 8) * 8 + (i & 7), kg = blk / (NC / 8) * 4 + ((i >> 3) & 3);
+          x[u] = i < np && live(col) ? __ldcg((const uint4 *)(xh + col * cs + kg * 16)) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const int i = i0 + u * NG * 128, blk = i >> 5, col = blk % (NC / 8) * 8 + (i & 7), kg = blk / (NC / 8) * 4 + ((i >> 3) & 3);
+          if (i < np) *(uint4 *)(Bp + (kg * NC + col) * 16) = x[u];
+        }
+      }
+#pragma unroll 1
+      for (int i = tid; i < nm; i += NG * 128) {   // (super-block, column, half of its means)
+        const int sb = i / (2 * NC), col = (i >> 1) % NC, h = i & 1;
+        if (live(col)) *(uint4 *)(Bm + ((sb * 2 + h) * NC + col) * 16) = __ldcg((const uint4 *)(xf + ((size_t)sb * NC + col) * 32 + h * 16));
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read these bytes through the async proxy
+      mbar_arrive(xp_full);
+    };
 #pragma unroll 1
     while (wk.ti < my_tiles) {
       wait(bar(wk.full()), (uint32_t)wk.phase() & 1u);
@@ -231,16 +289,17 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
         const uint4 qa = *(const uint4 *)qs, qb = *(const uint4 *)(qs + 16);
         const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
         // the scales as fp16 (0x6400 | s is 1024 + s) times 2^5 for the low nibbles and 2 for the high ones, which stay four bits
-        // up: q 2^-24 * s 2^5 = 16 q 2^-24 * s 2 = s q 2^-19, exact
+        // up: q 2^-24 * s 2^5 - 8 s 2^-19 = 16 q 2^-24 * s 2 - 8 s 2^-19 = s (q - 8) 2^-19, exact
         const uint32_t sw = gq < 2 ? scA : scB;
         const uint32_t L = g2_hfma2(__byte_perm(sw, 0x64646464u, gq & 1 ? 0x4242 : 0x4040), 0x50005000u, 0xf800f800u);
         const uint32_t H = g2_hfma2(__byte_perm(sw, 0x64646464u, gq & 1 ? 0x4343 : 0x4141), 0x40004000u, 0xe800e800u);
+        const uint32_t L8 = g2_hmul2(L, 0x80088008u), H8 = g2_hmul2(H, 0x80808080u);   // * -2^-21, * -2^-17
         uint32_t v[32];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const uint32_t y = w[i] >> 8;
-          v[2 * i] = g2_hmul2(w[i] & 0x000f000fu, L); v[2 * i + 1] = g2_hmul2(y & 0x000f000fu, L);
-          v[16 + 2 * i] = g2_hmul2(w[i] & 0x00f000f0u, H); v[17 + 2 * i] = g2_hmul2(y & 0x00f000f0u, H);
+          v[2 * i] = g2_hfma2(w[i] & 0x000f000fu, L, L8); v[2 * i + 1] = g2_hfma2(y & 0x000f000fu, L, L8);
+          v[16 + 2 * i] = g2_hfma2(w[i] & 0x00f000f0u, H, H8); v[17 + 2 * i] = g2_hfma2(y & 0x00f000f0u, H, H8);
         }
         if (gq == 0) {
           // the operand buffer and the accumulators are free once the last item's MMAs are done and its sums are read
@@ -248,16 +307,15 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
             drain();
             if (wk.ti != ti_p) flush(ti_p);
           }
-          // the mins as fp16 numbers: m against the means' hi halves, m / 2048 against their lo halves, which are stored times 2048
-          uint32_t mm[8];
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint32_t at = __byte_perm(j < 2 ? mnA : mnB, 0x64646464u, (j & 1) ? 0x4342u : 0x4140u);
-            mm[2 * j] = g2_hfma2(at, 0x3c003c00u, 0xe400e400u); mm[2 * j + 1] = g2_hfma2(at, 0x10001000u, 0xb800b800u);
-          }
-          t5_st8(abuf + 128, mm);
+          if (!g3_reuse(NC)) store_means(abuf + 128, scA, scB, mnA, mnB);
         }
         t5_st32(abuf + 32 * gq, v);
+        if (g3_reuse(NC) && gq == 3) {
+          if (it == 0) stage();
+          wait(half_done(g), (uint32_t)it & 1u);
+          t5_fence_after();
+          store_means(abuf, scA, scB, mnA, mnB);
+        }
         if (gq & 1) {
           t5_wait_st();
           t5_fence_before();
@@ -270,38 +328,7 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
       ti_p = wk.ti;
       it++;
       wk.next(NG, nsl, st);
-      if (!staged) {
-        // ---- the activation slice: eight pieces of sixteen bytes in flight a thread ----
-        staged = true;
-        pdl_wait();
-        const int half = NC / 2, T = a.T, np = nsl * 32 * NC, nm = nsl * 2 * NC;
-        const bool two = a.planes == 2;
-        const uint8_t *xh = (const uint8_t *)(a.xp.xh + (size_t)sb0 * 256), *xf = (const uint8_t *)(a.xp.xsf + (size_t)sb0 * NC * 16);
-        const size_t cs = (size_t)a.K * 2;
-        auto live = [&](int col) { return (two && col >= half ? col - half : col) < T; };
-        // (four k-groups of eight columns a warp: whole sectors of the source, whole rows of core matrices at the destination)
-#pragma unroll 1
-        for (int i0 = tid; i0 < np; i0 += 8 * NG * 128) {
-          uint4 x[8];
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const int i = i0 + u * NG * 128, blk = i >> 5, col = blk % (NC / 8) * 8 + (i & 7), kg = blk / (NC / 8) * 4 + ((i >> 3) & 3);
-            x[u] = i < np && live(col) ? __ldcg((const uint4 *)(xh + col * cs + kg * 16)) : make_uint4(0, 0, 0, 0);
-          }
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const int i = i0 + u * NG * 128, blk = i >> 5, col = blk % (NC / 8) * 8 + (i & 7), kg = blk / (NC / 8) * 4 + ((i >> 3) & 3);
-            if (i < np) *(uint4 *)(Bp + (kg * NC + col) * 16) = x[u];
-          }
-        }
-#pragma unroll 1
-        for (int i = tid; i < nm; i += NG * 128) {   // (super-block, column, half of its means)
-          const int sb = i / (2 * NC), col = (i >> 1) % NC, h = i & 1;
-          if (live(col)) *(uint4 *)(Bm + ((sb * 2 + h) * NC + col) * 16) = __ldcg((const uint4 *)(xf + ((size_t)sb * NC + col) * 32 + h * 16));
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read these bytes through the async proxy
-        mbar_arrive(xp_full);
-      }
+      if (!g3_reuse(NC) && it == 1) stage();
     }
     if (it > 0) { drain(); flush(ti_p); }
   } else if (warp == 4 * NG) {
@@ -329,7 +356,7 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
     // ---- the tensor core: a warp issues a group's MMAs ----
     const int g = __shfl_sync(0xffffffffu, warp - 4 * NG - 1, 0);
     const bool el = t5_elect();
-    const uint32_t ab = tmem + (uint32_t)(g * G3_A_COLS), db = tmem + (uint32_t)(NG * G3_A_COLS + g * 2 * N);
+    const uint32_t ab = tmem + (uint32_t)(g * g3_a_cols(NC)), db = tmem + (uint32_t)(NG * g3_a_cols(NC) + g * g3_d_cols(NC)), mb = ab + (g3_reuse(NC) ? 0u : 128u);
     const int items = my_tiles * nsl;
     int c = g;
     uint32_t par = 0;
@@ -341,10 +368,13 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
         wait(a_full(g, h), par);
         t5_fence_after();
         if (el) {
-          if (h == 0) t5_mma_f16_ts(db + N, ab + 128, md, g3_idesc(N), 0);
 #pragma unroll
           for (int k = 0; k < 8; k++) t5_mma_f16_ts(db, ab + 64 * h + 8 * k, bd + (uint64_t)((8 * h + k) * 2 * NC), g3_idesc(N), (h | k) != 0);
-          if (h == 1) t5_commit(d_full(g));
+          if (h == 1) {
+            t5_mma_f16_ts(db, mb, md, g3_idesc(N), 1);
+            t5_mma_f16_ts(db + g3_p_col(NC), mb + 8, NC == 8 ? md - 8 : md, g3_idesc(N), 0);   // (128 bytes early)
+            t5_commit(d_full(g));
+          } else if (g3_reuse(NC)) t5_commit(half_done(g));
         }
         __syncwarp();
       }

@@ -207,3 +207,41 @@ def test_tcgen05_edges_of_tiles_and_slices(llb, packs, oracle, dev, tcgen05, row
     if K // 256 // ksplit < 3 or (T > 8 and K // 256 // ksplit > 8):
         ksplit = max(1, K // 256 // 5)
     _gemm_case(llb, packs, oracle, dev, "Q4_K", rows, K, T, 2, ksplit, seed=K + T)
+
+
+@pytest.mark.parametrize("rows,K,T", [(2000, 1024, 4), (2048, 5120, 4), (2048, 5120, 8), (2048, 5120, 16), (600, 17408, 4)])
+def test_tcgen05_sums_keep_their_precision(llb, packs, rows, K, T):
+    """Both kernels against 64-bit sums.  Zero-mean activations: the tcgen05 kernel is no further off than the other.  Activations with a
+    mean: the scales' part and the min term of such a row all but cancel; both are truncated once at 2^-23 and up to four times the mass of
+    what they cancel to, so 2^-20 of the dot mass bounds a value; it stays within three times the other kernel's error."""
+    L = llb.lib()
+    g = torch.Generator(device="cuda").manual_seed(K + T)
+    raw = packs.QUANT["Q4_K"](torch.randn(rows, K, device="cuda", generator=g) * 0.02).contiguous()
+    W = packs.dequant("Q4_K", raw, rows, K).double()
+    w = llb.alloc(L.llb_b200_weight_bytes(3, rows, K))
+    llb.check(L.llb_b200_weight_upload(3, rows, K, raw.data_ptr(), 1, w), "weight_upload")
+    r, r2 = (torch.randn(T, K, device="cuda", generator=g) for _ in range(2))
+    cases = {"normal": r, "cube": r ** 3, "silu": torch.nn.functional.silu(r) * r2, "offset": 1 + 0.1 * r, "positive": r.abs()}
+    was = L.llb_b200_use_tcgen05(2)
+    try:
+        for name, x in cases.items():
+            x = x.contiguous()
+            ref, mass = x.double() @ W.T, x.double().abs() @ W.abs().T
+            err = []
+            for mode in (0, 1):
+                L.llb_b200_use_tcgen05(mode)
+                xp = llb.handle(L.llb_b200_xp_new(K, T, 2), "xp_new")
+                y = torch.zeros(T, rows, device="cuda")
+                torch.cuda.synchronize()
+                llb.check(L.llb_b200_xp_set_f32(xp, x.data_ptr()), "xp_set")
+                llb.gemm(3, [w], [rows], [y.data_ptr()], K, xp, 0)
+                llb.check(L.llb_b200_sync(), "sync")
+                L.llb_b200_xp_free(xp)
+                d = y.double() - ref
+                err.append(float(d.norm() / ref.norm()))
+                assert mode == 0 or bool((d.abs() <= 2.0 ** -20 * mass).all()), (name, float((d.abs() / mass).max()))
+            assert err[1] <= (3.0 if name in ("offset", "positive") else 1.2) * err[0], (name, err)
+    finally:
+        L.llb_b200_use_tcgen05(was)
+        L.llb_b200_free(w)
+    assert L.llb_b200_wait_errors() == 0
