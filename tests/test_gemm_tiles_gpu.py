@@ -24,10 +24,19 @@ def test_tiles_hold_every_weight(llb, packs, dev, ty, rows, cols):
     assert np.array_equal(out.read((rows, cols), np.float32).view(np.uint32), ref.view(np.uint32))
 
 
+@pytest.fixture
+def mma_sync(llb):
+    """Q4_K launches stay on the mma.sync kernel, whose tiles, rings and folded form these are."""
+    was = llb.lib().llb_b200_use_tcgen05(0)
+    yield
+    llb.lib().llb_b200_use_tcgen05(was)
+
+
 @pytest.mark.parametrize("ksplit", [0, 1, 3])
 @pytest.mark.parametrize("rows,K,T", [(1, 256, 1), (16, 1024, 1), (17, 3328, 3), (100, 2048, 8), (2500, 1280, 4), (40, 4096, 16), (19200, 2560, 9), (19216, 2560, 16)])
 @pytest.mark.parametrize("ty", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
-def test_row_tiles_shared_by_warps(llb, packs, dev, ty, rows, K, T, ksplit):
+def test_row_tiles_shared_by_warps(llb, packs, dev, mma_sync, ty, rows, K, T, ksplit):
+    """(19200 rows of ten super-blocks are the most tiles before Q4_K's scales go into the codes at nine rows and more, 19216 the fewest behind)"""
     rng = np.random.default_rng(rows + K)
     raw = packs.QUANT[ty](torch.from_numpy(rng.standard_normal((rows, K), dtype=np.float32) * 0.05))
     x = rng.standard_normal((T, K), dtype=np.float32)
