@@ -1,5 +1,7 @@
 """GPU parity of the dequant-fused skinny GEMM and of row dequantisation, through the C ABI,
 against the CPU oracle on the same seeded inputs."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -175,8 +177,15 @@ def tcgen05(llb):
     assert L.llb_b200_wait_errors() == 0      # no bounded wait on an mbarrier ran out
 
 
+def _kernel(llb, rows, K, T, planes, ksplit):
+    """2 mma.sync, 3 tcgen05: what a Q4_K launch takes under the present setting"""
+    ks, cols = C.c_int(ksplit), T * planes
+    return llb.lib().llb_b200_gemm_kernel(3, 8 if cols <= 8 else 16 if cols <= 16 else 32, sum((r + 15) // 16 for r in rows), K // 256, llb.lib().llb_b200_sm_count(), 1, C.byref(ks))
+
+
 @pytest.mark.parametrize("K,ksplit", [(256, 1), (768, 1), (1280, 0), (2560, 3), (5120, 0)])
 def test_tcgen05_gemm_vs_oracle(llb, packs, oracle, dev, tcgen05, K, ksplit):
+    assert _kernel(llb, [80], K, 4, 2, ksplit) == (3 if K > 256 else 2)     # (one super-block is not enough for its groups)
     _gemm_case(llb, packs, oracle, dev, "Q4_K", [80], K, 4, 2, ksplit, seed=K)
     _gemm_case(llb, packs, oracle, dev, "Q4_K", [300], K, 3, 2, ksplit, seed=K + 1)
 
@@ -192,10 +201,32 @@ def test_tcgen05_gemm_ragged_cat_and_planes(llb, packs, oracle, dev, tcgen05):
         _gemm_case(llb, packs, oracle, dev, "Q4_K", [64], 1536, T, planes, 0, seed=T + planes)
 
 
-def test_tcgen05_gemm_many_tiles(llb, packs, oracle, dev, tcgen05):
-    # more 128-row tiles than CTAs: a CTA walks several tiles and prefetches across them
-    _gemm_case(llb, packs, oracle, dev, "Q4_K", [40000], 512, 4, 2, 0, seed=9)
-    _gemm_case(llb, packs, oracle, dev, "Q4_K", [20000], 1024, 4, 2, 2, seed=10)
+@pytest.mark.parametrize("T", [4, 8, 16])
+@pytest.mark.parametrize("nsl,ksplit", [(3, 1), (3, 5), (4, 4), (5, 3), (7, 2), (12, 2)])
+def test_tcgen05_gemm_many_tiles(llb, packs, tcgen05, nsl, ksplit, T):
+    """Five 128-row tiles a CTA and six for some: rings and buffers of sums go round several times, across tiles, K-slices as long as the ring
+    and the groups' walk can meet them (a stage with one super-block, a tile of one round of the groups).  All rows, at 1e-5 of the dot mass."""
+    if T > 8:
+        nsl, ksplit = min(nsl, 7), max(ksplit, 2)
+    L, K = llb.lib(), 256 * nsl * ksplit
+    rows = (L.llb_b200_sm_count() // ksplit * 5 + 3) * 128 - 40
+    assert _kernel(llb, [rows], K, T, 2, ksplit) == 3
+    g = torch.Generator(device="cuda").manual_seed(K + T)
+    raw = packs.q4k_random_blocks(rows, K, seed=K, device="cuda").contiguous()
+    w = llb.alloc(L.llb_b200_weight_bytes(3, rows, K))
+    llb.check(L.llb_b200_weight_upload(3, rows, K, raw.data_ptr(), 1, w), "weight_upload")
+    x, y = torch.randn(T, K, device="cuda", generator=g), torch.zeros(T, rows, device="cuda")
+    torch.cuda.synchronize()
+    xp = llb.handle(L.llb_b200_xp_new(K, T, 2), "xp_new")
+    llb.check(L.llb_b200_xp_set_f32(xp, x.data_ptr()), "xp_set")
+    llb.gemm(3, [w], [rows], [y.data_ptr()], K, xp, ksplit)
+    llb.check(L.llb_b200_sync(), "sync")
+    L.llb_b200_xp_free(xp)
+    L.llb_b200_free(w)
+    for r0 in range(0, rows, 8192):
+        W = packs.dequant("Q4_K", raw[r0:r0 + 8192], min(8192, rows - r0), K).double()
+        ref, mass = x.double() @ W.T, x.double().abs() @ W.abs().T
+        assert bool(((y[:, r0:r0 + 8192].double() - ref).abs() <= 1e-5 * mass).all()), r0
 
 
 @pytest.mark.parametrize("rows,K,ksplit", [([1], 768, 1), ([127, 129], 1280, 1), ([128], 2304, 3), ([300, 16, 1, 260], 1792, 2), ([20000], 1280, 1), ([515], 17408, 13)])
@@ -206,6 +237,7 @@ def test_tcgen05_edges_of_tiles_and_slices(llb, packs, oracle, dev, tcgen05, row
     1e-5 of the dot mass."""
     if K // 256 // ksplit < 3 or (T > 8 and K // 256 // ksplit > 8):
         ksplit = max(1, K // 256 // 5)
+    assert _kernel(llb, rows, K, T, 2, ksplit) == 3
     _gemm_case(llb, packs, oracle, dev, "Q4_K", rows, K, T, 2, ksplit, seed=K + T)
 
 
