@@ -22,6 +22,7 @@ path, weak scaling.  `--impl reference` times the reference CPU engine alone (ra
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import statistics
@@ -391,9 +392,11 @@ def run_gemm_case(args, local):
     peak, peak_src = peaks()
     nc = 8 if T <= 4 else 16 if T <= 8 else 32
     nbytes = per_copy + nc * K * 2 + sum(T * r * 4 for r in rows)
-    print(json.dumps({"case": "gemm", "kernel": f"skinny GEMM, {ty}", "rows": rows, "cols": K, "T": T, "plane_columns": nc, "launches": args.steps,
+    ks = ctypes.c_int(args.ksplit)
+    kernel = L.llb_b200_gemm_kernel(fmt, nc, sum((r + 15) // 16 for r in rows), K // 256, L.llb_b200_sm_count(), 1, ctypes.byref(ks))
+    print(json.dumps({"case": "gemm", "kernel": f"k_gemm{kernel}, {ty}", "rows": rows, "cols": K, "T": T, "plane_columns": nc, "launches": args.steps,
                       "weight_copies": copies, "us_per_launch": us, "bytes_per_launch": nbytes, "GBs": nbytes / us / 1e3, "frac": nbytes / us / 1e3 / peak,
-                      "peak": peak, "peak_source": peak_src, "ksplit": L.llb_b200_gemm_ksplit(fmt, nc, sum((r + 15) // 16 for r in rows), K // 256, L.llb_b200_sm_count()) if args.ksplit == 0 else args.ksplit,
+                      "peak": peak, "peak_source": peak_src, "ksplit": ks.value,
                       "wait_errors": L.llb_b200_wait_errors()}), flush=True)
 
 
