@@ -27,11 +27,11 @@ static double gemm_stream_cost(int fmt, int warps, int nc, int tiles, int slice,
 }
 // Parts of a row tile's K-slice (g2_phase): the power of two with the lowest cost that divides the warps, leaves every part a
 // super-block and whose sums fit beside the activation slice.  tiles: row tiles of a CTA, nsb in ks slices
-static int gemm_pick_parts(int fmt, int NC, int ntc, int tiles, int nsb, int ks) {
+static int gemm_pick_parts(int fmt, int NC, int tiles, int nsb, int ks) {
   const int warps = g2_warps(fmt, NC), slice = (nsb + ks - 1) / ks, ring = g2_ring_of(fmt, NC, slice);
   int best = 1;
   for (int p = 2; p <= 16 && p <= nsb / ks && warps % p == 0; p *= 2)
-    if (g2_smem(fmt, slice, NC, p, ntc, ring) <= G2_SMEM_MAX && gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, p) < gemm_stream_cost(fmt, warps, 8 * ntc, tiles, slice, best)) best = p;
+    if (g2_smem(fmt, slice, NC, p, ring) <= G2_SMEM_MAX && gemm_stream_cost(fmt, warps, NC, tiles, slice, p) < gemm_stream_cost(fmt, warps, NC, tiles, slice, best)) best = p;
   return best;
 }
 template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
@@ -40,9 +40,9 @@ template <int FMT, int NT> static int launch_two(cudaStream_t s, GemmArgs &a) {
   if (cps < 1) cps = 1;
   // every SM takes part as long as there is a tile for it: the tiles are dealt out one per CTA in turn
   if (cps > a.tile0[a.nmat]) cps = a.tile0[a.nmat];
-  a.parts = gemm_pick_parts(FMT, NC, NT, (a.tile0[a.nmat] + cps - 1) / cps, a.nsb, a.ksplit);
+  a.parts = gemm_pick_parts(FMT, NC, (a.tile0[a.nmat] + cps - 1) / cps, a.nsb, a.ksplit);
   const int ring = g2_ring_of(FMT, NC, nsl);
-  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, NT, ring);
+  const size_t smem = g2_smem(FMT, nsl, NC, a.parts, ring);
   if (smem > G2_SMEM_MAX) return llb_fail("k_gemm2: a K-slice of %d super-blocks needs %zu bytes of shared memory", nsl, smem);
   const bool fold = (long long)a.tile0[a.nmat] * a.nsb >= G2_FOLD_TILES;
   constexpr int RS = g2_small_ring(FMT, 8 * NT);
@@ -226,15 +226,15 @@ bool gemm_fits(int fmt, int NC, int nsb, int cap) {
   return ks <= cap && (g3_fits(fmt, NC, nsb, ks, false) || (nsb + ks - 1) / ks <= g2_longest_slice(fmt, NC));
 }
 
-// K-slices per row tile: streaming, the staging of the slice, and a charge per slice for the partial sums that the consumer
+// K-slices per row tile: streaming, the staging of the slice (24 cycles a plane column of a super-block), and a charge per slice for the partial sums that the consumer
 // has to add (direct: a launch of its own adds them, 1.5 us).  At 32 plane columns a warp's chain is nearer 3000 cycles a tile
 // (fitted on fifteen shapes, four formats, one to eight slices; with 1200 the operator's choices were 4.5 % off the best of those,
 // now 1 %: Q4_K 8192 x 3072 at sixteen rows 18.0 -> 15.8 us, 5120 x 5120 18.5 -> 15.9).  The operator alone goes by it: a
 // split decides the order of a model's sums, and the passes were timed with the splits they have.
-static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool direct, double stage) {
+static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps;
-  const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, NC / 8, tiles, nsb, ks), direct && NC >= 32 ? 3000.0 : 1200.0);
-  return (stream + stage * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
+  const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, tiles, nsb, ks), direct && NC >= 32 ? 3000.0 : 1200.0);
+  return (stream + 24.0 * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
 // The tcgen05 kernel's cost on the same scale: a super-block of 128 rows in a CTA, a tile's way out, the slice's activations, the
 // pipeline's fill -- times 0.7, because that scale flatters the other kernel (27B shape, a prompt of 48 tokens in passes of eight rows
@@ -250,15 +250,15 @@ static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct)
 static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool alone) {
   if (!g3_fits(fmt, NC, nsb, ks, alone)) return false;
   if (g_llb.gemm3 == 1 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
-  return g3_cost(NC, ntiles, nsb, ks, sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, false, 24.0);
+  return g3_cost(NC, ntiles, nsb, ks, sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, false);
 }
-int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct, double stage) {
+int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct) {
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
     if (gemm_fix_ksplit(fmt, NC, nsb, ks, direct) != ks) continue;
     if (g_llb.gemm3 == 1 && best_cost < 1e30 && !g3_fits(fmt, NC, nsb, ks, direct) && g3_fits(fmt, NC, nsb, best, direct)) continue;
-    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, sms, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct, stage);
+    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, sms, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct);
     // (the tcgen05 kernel asked for: before any split that it cannot take comes one that it can)
     const bool asked = g_llb.gemm3 == 1 && g3_fits(fmt, NC, nsb, ks, direct) && !g3_fits(fmt, NC, nsb, best, direct);
     if (cost < best_cost - 1e-9 || asked) { best_cost = cost; best = ks; }
@@ -304,7 +304,7 @@ static int gemm_prepare(int fmt, GemmArgs &a, bool fused = false) {
 // ---- the fused FFN launch (ffn_fused.cuh) ------------------------------------------------------
 // shared memory of the launch: the ring, and the larger of gate|up's planes (nsb1 super-blocks) and a down slice's (nsl2)
 static size_t ffn_smem(int fmt2, int nsb1, int nsl2) {
-  const size_t s1 = g2_smem(LLB_FM_Q4_K, nsb1, 8, 1, 1, 1), s2 = g2_smem(fmt2, nsl2, 8, 1, 1, 1) - g2_ring_bytes(fmt2, 8, 1) + FFN_RING;
+  const size_t s1 = g2_smem(LLB_FM_Q4_K, nsb1, 8, 1, 1), s2 = g2_smem(fmt2, nsl2, 8, 1, 1) - g2_ring_bytes(fmt2, 8, 1) + FFN_RING;
   return s1 > s2 ? s1 : s2;
 }
 template <int FMT2> static int launch_ffn(cudaStream_t s, const GemmArgs &a1, const GemmArgs &a2) {

@@ -7,7 +7,8 @@
 //    16-byte copies took 30 of the loop's 397 instructions, most of them integer adds;
 //  * Q4_K / Q5_K: a code in the low bits of an fp16 lane is the subnormal code * 2^-24, so two MMAs sum
 //    code * x of a 32-column sub-block exactly; the six-bit scale multiplies that fp32 sum, d the super-block's;
-//  * Q4_K, 16 rows (four n-tiles), large launches: the scale is multiplied into the codes instead (FOLD), since sc * q <=
+//  * Q4_K, 16 rows (four n-tiles), large launches that the tcgen05 kernel (gemm3.cuh) cannot take or is kept from (a matrix of
+//    one super-block's columns; LLB_GEMM3=0, llb_b200_use_tcgen05(0)): the scale is multiplied into the codes instead (FOLD), since sc * q <=
 //    63 * 15 is an exact fp16 integer: one HMUL2 a fragment register, shared by the n-tiles, and the MMAs of a whole super-block
 //    accumulate into one fragment.  Lane j of a row's four lanes then holds the k indices of column group j (64 columns, two
 //    sub-blocks) and needs that group's scales only.  The chain of MMAs into one fragment is longer, so it takes enough
@@ -54,9 +55,9 @@ __host__ __device__ constexpr int g2_warps(int fmt, int NC) {
 __host__ __device__ constexpr int g2_ring_bytes(int fmt, int NC, int ring = 0) { return g2_warps(fmt, NC) * g2_stages(fmt, NC, ring) * g2_chunk(fmt, ring) * tile_bytes(fmt); }
 __host__ __device__ constexpr int g2_aux(int fmt) { return fmt == LLB_FM_Q4_K || fmt == LLB_FM_Q5_K ? 32 : 0; }
 __host__ __device__ constexpr int g2_xpad(int fmt) { return fmt == LLB_FM_Q6_K ? 32 : 64; }
-// bytes of shared memory of a launch whose K-slices have nsl super-blocks in `parts` parts, for NC activation columns (ntc of them in n-tiles that are summed over the parts)
-__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC, int parts = 1, int ntc = 4, int ring = 0) {
-  return (size_t)(parts > 1 ? g2_warps(fmt, NC) * ntc * 512 : 0) + G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC, ring);
+// bytes of shared memory of a launch whose K-slices have nsl super-blocks in `parts` parts, for NC activation columns
+__host__ __device__ inline size_t g2_smem(int fmt, int nsl, int NC, int parts = 1, int ring = 0) {
+  return (size_t)(parts > 1 ? g2_warps(fmt, NC) * (NC / 8) * 512 : 0) + G2_BAR_BYTES + NC * (nsl * 512 + g2_xpad(fmt)) + nsl * NC * g2_aux(fmt) + g2_ring_bytes(fmt, NC, ring);
 }
 inline int g2_max_slice_sb(int fmt, int NC, int ring = 0) {
   const int left = G2_SMEM_MAX - G2_BAR_BYTES - g2_ring_bytes(fmt, NC, ring) - NC * g2_xpad(fmt);

@@ -31,7 +31,6 @@
 #include "rowops.cuh"
 
 #define MOE_WARPS G2_MAXWARPS
-#define MOE_MAXROWS 16
 // shared memory that the choice takes: units, chosen ids, per 32 pairs those that open a unit, the rows in use
 __host__ __device__ inline int moe_sel_bytes(int pairs) { return pairs * 16 + ((pairs * 4 + 15) & ~15) + 96 + 64; }
 // bytes of a unit's staged activations: eight plane columns of nsl super-blocks and their means

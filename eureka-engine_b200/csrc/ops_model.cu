@@ -205,7 +205,6 @@ int op_silu_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, const RowS
 // weights, a block per row, all rows of the pass; the gate|up launch makes the choice from them (moe.cuh).  Bound by the one trip
 // to L2 for the rows of h, so four rows are in flight at a time: row by row, each trip behind the last, sixteen rows
 // took 21 us.
-#define MOE_MAXROWS 16   // rows of a pass (several streams of k + 1 rows)
 __global__ void __launch_bounds__(256, 2) k_moe_router(const float *__restrict__ W, const float *__restrict__ h, int d, int ne, float *__restrict__ lg, const RowSet *rs, int n_all) {
   int rs_n, rs_p0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.x, nrows = ne + 1;

@@ -14,6 +14,7 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // ---- top k of a routed-expert layer's router (host/llb_host.c:651-667; llb_moe_topk of tools/payload-moeany.patch) ----
+#define MOE_MAXROWS 16   // rows of a pass (several streams of k + 1 rows)
 // One warp per row of the pass: softmax over the ne logits, the k largest probabilities in descending order with
 // ties to the lower index, their weights divided by their sum clamped at 6.103515625e-5; slot k is the shared
 // expert (id ne) with weight sigmoid(its gate logit).
