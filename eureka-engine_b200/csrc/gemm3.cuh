@@ -234,11 +234,16 @@ __global__ void __launch_bounds__(g3_threads(NC), 1) k_gemm3(const GemmArgs a, c
               out += os;
             }
           } else {
-            int blk[NC];                        // every slot's load in flight at once
+            // every slot's load in flight at once, row j of stream z counted along: a division a column took longer than all the rest of a
+            // tile (the DeltaNet inputs of the 35B-A3B shape, sixteen rows of four streams, 31 us a launch where the mma.sync kernel takes 20)
+            int blk[NC / 2], z = 0, tl = 0;     // (passes only: two planes, T <= NC / 2)
 #pragma unroll
-            for (int j = 0; j < NC; j++) { const int z = per > 0 ? j / per : 0; blk[j] = j < T ? ts[(size_t)z * tst + (j - z * per)] + z * tadd : 0; }
+            for (int j = 0; j < NC / 2; j++) {
+              blk[j] = j < T ? __ldcg(ts + z * tst + tl) + z * tadd : 0;
+              if (++tl == per) { tl = 0; z++; }
+            }
 #pragma unroll
-            for (int j = 0; j < NC; j++) if (j < T) out[(size_t)blk[j] * os] = acc[j];
+            for (int j = 0; j < NC / 2; j++) if (j < T) out[(size_t)blk[j] * os] = acc[j];
           }
         }
       }
