@@ -214,8 +214,8 @@ int llb_b200_gemm(int fmt, int nmat, const llb_b200_dptr *w, const int *rows, co
   a.nmat = nmat; a.K = K; a.xp = xp->p; a.planes = xp->planes; a.T = xp->T;
   int ntiles = 0, total_rows = 0;
   for (int i = 0; i < nmat; i++) { ntiles += (rows[i] + 15) / 16; total_rows += rows[i]; }
-  a.alone = true;
-  a.ksplit = gemm_fix_ksplit(fmt, xp->p.NC, K / 256, ksplit > 0 ? ksplit : gemm_pick_ksplit(fmt, xp->p.NC, ntiles, K / 256, g_llb.sms, true), true);
+  a.alone = true; a.ksplit = ksplit;
+  a.g3 = gemm_which(fmt, xp->p.NC, ntiles, K / 256, g_llb.sms, true, &a.ksplit) == 3;
   const size_t per_split = (size_t)xp->T * total_rows;
   if (a.ksplit > 1 && per_split * a.ksplit > g_parts_floats) {
     if (g_parts) {

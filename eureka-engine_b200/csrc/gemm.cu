@@ -236,40 +236,81 @@ static double gemm_split_cost(int fmt, int NC, int ntiles, int nsb, int ks, int 
   const double stream = gemm_stream_cost(fmt, g2_warps(fmt, NC), NC, tiles, slice, gemm_pick_parts(fmt, NC, tiles, nsb, ks), direct && NC >= 32 ? 3000.0 : 1200.0);
   return (stream + 24.0 * NC * slice) * (1.0 + 0.02 * (ks - 1)) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0);
 }
-// The tcgen05 kernel's cost on the same scale: a super-block of 128 rows in a CTA, a tile's way out, the slice's activations, the
+// The tcgen05 kernel's cost on the same scale, in a pass: a super-block of 128 rows in a CTA, a tile's way out, the slice's activations, the
 // pipeline's fill -- times 0.7, because that scale flatters the other kernel (27B shape, a prompt of 48 tokens in passes of eight rows
 // 51.7 ms without the kernel, 49.2 with this factor 1, 48.5 with 0.7; ten cycles of sixteen rows 125.2, 114.6, 114.2).
-// In a pass (not direct) 4000 cycles more: its first MMA waits for all activations, and what the mma.sync kernel has ready by then is
-// worth that much; without it the 2048-column launches of the 35B-A3B shape came here and eight of its streams took 156 ms instead of 147.
-static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms, bool direct) {
+// 4000 cycles more: its first MMA waits for all activations, and what the mma.sync kernel has ready by then is worth that much.
+static double g3_cost(int NC, int ntiles, int nsb, int ks, int sms) {
   const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
-  const double sb = NC >= 32 ? 990.0 : NC >= 16 ? 860.0 : 835.0;
-  return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + (direct && ks > 1 ? 3000.0 : 0.0) + (direct ? 0.0 : 4000.0);
+  const double sb = NC >= 32 ? 970.0 : 820.0;
+  return 0.7 * (tiles * (slice * sb + 900.0) * (1.0 + 0.02 * (ks - 1)) + 4000.0 + 12.0 * NC * slice) + 25.0 * NC * (ks - 1) + 4000.0;
+}
+// Microseconds of the operator's launch and its sums with either kernel, for a width's most rows (the choice may not depend on the
+// rows: a row's bits do not).  Fitted on 56 shapes of 4 to 68 super-blocks and 512 to 40000 rows, 148 SMs, weights cold, every K-split: half
+// of the launches within 5 %, nine in ten within 12 %.  The scale of gemm_split_cost, whose costs the passes go by, is too kind to the
+// tcgen05 kernel here by up to a third: 6144 x 5120 at eight rows went there and took 12.9 us for 10.7, 17408 x 5120 at four 17.6 for 15.6.
+static double g3_us(int NC, int ntiles, int nsb, int ks, int sms) {
+  static const double c[3][6] = {{2.24, 0.0324, 0.1108, 0.87, 1.94, 0.1536}, {2.38, 0.0327, 0.1378, 0.86, 1.27, 0.1711}, {3.16, 0.0225, 0.1268, 1.10, 0.86, 0.2106}};
+  const double *k = c[NC / 16];
+  const int cps = sms / ks > 0 ? sms / ks : 1, slice = (nsb + ks - 1) / ks, tiles = ((ntiles + 7) / 8 + cps - 1) / cps;
+  return k[0] + k[1] * NC * slice + k[2] * tiles * slice + (ks > 1 ? k[3] + k[4] * 32e-6 * NC * ks * ntiles : 0.0) + k[5] * 2304e-6 * ntiles * nsb;
+}
+static double g2_us(int NC, int ntiles, int nsb, int ks, int sms) {
+  static const double c[3][9] = {{1.76, 0.0089, 0.0319, 0.0406, 0.196, 0.87, 0.75, 0.1295, 0.4115}, {1.75, 0.0169, 0.0474, 0.1672, 0.0, 1.27, 0.86, 0.1168, 0.2108}, {2.59, 0.0122, 0.0451, 0.8476, 0.0, 0.97, 1.02, 0.0930, 0.0}};
+  const double *k = c[NC / 16];
+  int cps = sms / ks > 0 ? sms / ks : 1;
+  if (cps > ntiles) cps = ntiles;
+  const int slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps, p = gemm_pick_parts(LLB_FM_Q4_K, NC, tiles, nsb, ks), w = g2_warps(LLB_FM_Q4_K, NC);
+  const int rounds = (tiles * p + w - 1) / w;
+  return k[0] + k[1] * NC * slice + k[2] * tiles * slice + k[3] * rounds * ((slice + p - 1) / p) + (p > 1 ? k[4] * rounds : 0.0) + (ks > 1 ? k[5] + k[6] * 32e-6 * NC * ks * ntiles : 0.0) +
+         k[7] * 2304e-6 * ntiles * nsb + k[8] * rounds;
+}
+// Whether the tcgen05 kernel in k3 slices is the operator's choice over the other in k2: where it is faster by more than the fit is off at
+// shapes that are near.  At 8 plane columns, where the two are, a slice more counts 0.3 us.  Of the 56 shapes eleven, sixteen and forty-six
+// change kernels at 8, 16 and 32 columns; none is more than 3.7 % slower for it, on average they are 1.6, 3.3 and 16 % faster.
+static bool g3_better(int NC, int ntiles, int nsb, int k3, int k2, int sms) {
+  const double slice = NC == 8 ? 0.3 : 0.0, margin = NC == 8 ? 0.97 : NC == 16 ? 0.95 : 0.96;
+  return g3_us(NC, ntiles, nsb, k3, sms) + slice * k3 < margin * (g2_us(NC, ntiles, nsb, k2, sms) + slice * k2);
 }
 // Which kernel a launch takes at this K-split: the tcgen05 one where it can and costs less (or has been asked for).
 static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool alone) {
   if (!g3_fits(fmt, NC, nsb, ks, alone)) return false;
   if (g_llb.gemm3 == 1 || ks < g2_least_ksplit(fmt, NC, nsb)) return true;
-  return g3_cost(NC, ntiles, nsb, ks, sms, alone) - (alone && ks > 1 ? 3000.0 : 0.0) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, false);
+  if (alone) return g3_better(NC, ntiles, nsb, ks, ks, sms);
+  return g3_cost(NC, ntiles, nsb, ks, sms) < gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, false);
 }
-int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct) {
+// The operator's K-slices where the caller names none, and in *g3 its kernel: each kernel's own best, then the better of the two.
+static int gemm_pick_alone(int fmt, int NC, int ntiles, int nsb, int sms, bool *g3) {
+  int k2 = 0, k3 = 0;
+  for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
+    if (ks >= g2_least_ksplit(fmt, NC, nsb) && (!k2 || gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, true) < gemm_split_cost(fmt, NC, ntiles, nsb, k2, sms, true) - 1e-9)) k2 = ks;
+    if (g3_fits(fmt, NC, nsb, ks, true) && (!k3 || g3_us(NC, ntiles, nsb, ks, sms) + (NC == 8 ? 0.3 : 0.0) * (ks - k3) < g3_us(NC, ntiles, nsb, k3, sms))) k3 = ks;
+  }
+  *g3 = k3 && (!k2 || g_llb.gemm3 == 1 || g3_better(NC, ntiles, nsb, k3, k2, sms));
+  return *g3 ? k3 : k2 ? k2 : gemm_fix_ksplit(fmt, NC, nsb, 1, true);
+}
+int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms) {
   int best = 1;
   double best_cost = 1e30;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
-    if (gemm_fix_ksplit(fmt, NC, nsb, ks, direct) != ks) continue;
-    if (g_llb.gemm3 == 1 && best_cost < 1e30 && !g3_fits(fmt, NC, nsb, ks, direct) && g3_fits(fmt, NC, nsb, best, direct)) continue;
-    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, sms, direct) ? g3_cost(NC, ntiles, nsb, ks, sms, direct) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, direct);
+    if (gemm_fix_ksplit(fmt, NC, nsb, ks) != ks) continue;
+    if (g_llb.gemm3 == 1 && best_cost < 1e30 && !g3_fits(fmt, NC, nsb, ks, false) && g3_fits(fmt, NC, nsb, best, false)) continue;
+    const double cost = g3_use(fmt, NC, ntiles, nsb, ks, sms, false) ? g3_cost(NC, ntiles, nsb, ks, sms) : gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, false);
     // (the tcgen05 kernel asked for: before any split that it cannot take comes one that it can)
-    const bool asked = g_llb.gemm3 == 1 && g3_fits(fmt, NC, nsb, ks, direct) && !g3_fits(fmt, NC, nsb, best, direct);
+    const bool asked = g_llb.gemm3 == 1 && g3_fits(fmt, NC, nsb, ks, false) && !g3_fits(fmt, NC, nsb, best, false);
     if (cost < best_cost - 1e-9 || asked) { best_cost = cost; best = ks; }
   }
-  return gemm_fix_ksplit(fmt, NC, nsb, best, direct);
+  return gemm_fix_ksplit(fmt, NC, nsb, best);
 }
 
 int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit) {
-  const int ks = gemm_fix_ksplit(fmt, NC, nsb, *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, NC, ntiles, nsb, sms, alone), alone);
-  *ksplit = ks;
-  return g3_use(fmt, NC, ntiles, nsb, ks, sms, alone) ? 3 : 2;
+  bool g3 = false;
+  if (alone && *ksplit <= 0) *ksplit = gemm_pick_alone(fmt, NC, ntiles, nsb, sms, &g3);
+  else {
+    *ksplit = gemm_fix_ksplit(fmt, NC, nsb, *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, NC, ntiles, nsb, sms), alone);
+    g3 = g3_use(fmt, NC, ntiles, nsb, *ksplit, sms, alone);
+  }
+  return g3 ? 3 : 2;
 }
 
 // One K-split for a launch whose partial sums outlive the pass (attn_qkv into the conv ring): valid at both
@@ -413,7 +454,7 @@ int gemm_launch(cudaStream_t s, int fmt, GemmArgs &a) {
   if (gemm_prepare(fmt, a)) return -1;
   if (a.tile0[a.nmat] < 1) return 0;
   const int NT = a.xp.NC / 8;
-  if (g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit, g_llb.sms, a.alone)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
+  if (a.alone ? a.g3 : g3_use(fmt, a.xp.NC, a.tile0[a.nmat], a.nsb, a.ksplit, g_llb.sms, false)) return NT == 1 ? launch_three<8>(s, a) : NT == 2 ? launch_three<16>(s, a) : launch_three<32>(s, a);
   if (fmt == LLB_FM_Q4_K) return NT == 1 ? launch_two<LLB_FM_Q4_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q4_K, 2>(s, a) : launch_two<LLB_FM_Q4_K, 4>(s, a);
   if (fmt == LLB_FM_Q5_K) return NT == 1 ? launch_two<LLB_FM_Q5_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q5_K, 2>(s, a) : launch_two<LLB_FM_Q5_K, 4>(s, a);
   if (fmt == LLB_FM_Q6_K) return NT == 1 ? launch_two<LLB_FM_Q6_K, 1>(s, a) : NT == 2 ? launch_two<LLB_FM_Q6_K, 2>(s, a) : launch_two<LLB_FM_Q6_K, 4>(s, a);

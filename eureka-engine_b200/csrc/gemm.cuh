@@ -50,7 +50,7 @@ struct GemmArgs {
   XPlanes xp;
   int planes;                  // 2: hi/lo columns are folded into T = NC/2 tokens; 1: NC independent tokens
   int T;                       // tokens actually written
-  bool alone;                  // the operator's launch, not one of a pass's
+  bool alone, g3;              // the operator's launch, not one of a pass's; its kernel: the tcgen05 one
   unsigned int *err;           // device word set when a bounded wait runs out
 };
 

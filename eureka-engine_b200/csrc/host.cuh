@@ -61,7 +61,7 @@ inline cudaError_t llb_launch_cluster(void (*k)(KArgs...), dim3 grid, dim3 block
 }
 
 // gemm.cu
-int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms, bool direct = false);   // direct: the caller adds the slices with a launch of its own
+int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms);   // of a launch of a pass
 int gemm_fix_ksplit(int fmt, int NC, int nsb, int ks, bool alone = false);   // clamps a requested K-split to what a kernel can take; alone: not one of a pass's launches
 int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit);   // 2 mma.sync, 3 tcgen05; *ksplit 0: picked here
 bool gemm_fits(int fmt, int NC, int nsb, int cap);   // whether a pass's launch can take nsb super-blocks in at most cap K-slices
