@@ -259,7 +259,7 @@ static double g2_us(int NC, int ntiles, int nsb, int ks, int sms) {
   static const double c[3][9] = {{1.76, 0.0089, 0.0319, 0.0406, 0.196, 0.87, 0.75, 0.1295, 0.4115}, {1.75, 0.0169, 0.0474, 0.1672, 0.0, 1.27, 0.86, 0.1168, 0.2108}, {2.59, 0.0122, 0.0451, 0.8476, 0.0, 0.97, 1.02, 0.0930, 0.0}};
   const double *k = c[NC / 16];
   int cps = sms / ks > 0 ? sms / ks : 1;
-  if (cps > ntiles) cps = ntiles;
+  if (cps > ntiles) cps = ntiles > 0 ? ntiles : 1;
   const int slice = (nsb + ks - 1) / ks, tiles = (ntiles + cps - 1) / cps, p = gemm_pick_parts(LLB_FM_Q4_K, NC, tiles, nsb, ks), w = g2_warps(LLB_FM_Q4_K, NC);
   const int rounds = (tiles * p + w - 1) / w;
   return k[0] + k[1] * NC * slice + k[2] * tiles * slice + k[3] * rounds * ((slice + p - 1) / p) + (p > 1 ? k[4] * rounds : 0.0) + (ks > 1 ? k[5] + k[6] * 32e-6 * NC * ks * ntiles : 0.0) +

@@ -94,3 +94,11 @@ def test_an_engine_keeps_the_kernels_it_was_opened_with(pkg, packs, llb):
     (32, 34816, 5120, 3), (32, 5120, 17408, 3), (32, 5120, 5120, 3), (32, 16384, 2048, 3), (32, 2048, 2048, 2)])
 def test_the_operator_takes_the_faster_kernel(pkg, nc, rows, K, which):
     assert kernel(pkg.llb.lib(), nc, rows, K)[0] == which
+
+
+def test_no_rows_and_no_sms_are_questions_too(pkg):
+    L = pkg.llb.lib()
+    for nc in (8, 16, 32):
+        for alone in (False, True):
+            assert kernel(L, nc, 0, 5120, alone=alone)[1] >= 1 and kernel(L, nc, 0, 5120, ksplit=4, alone=alone)[1] == 4
+            assert kernel(L, nc, 5120, 5120, sms=0, alone=alone)[1] >= 1
