@@ -551,8 +551,9 @@ int op_delta(cudaStream_t s, float *S, const SpecCtl *ctl, PartIn ring, const fl
   if (sh.SZ != 128) return llb_fail("DeltaNet state size %d (only 128, as host/llb_host.c:1608)", sh.SZ);
   if (sh.KC > CONV_RING / 2) return llb_fail("conv kernel %d", sh.KC);
   // An SM's stores leave it at about 32 bytes a cycle, and two of a cluster's blocks on one SM share them (a row of the scan 0.64 us
-  // there): where every block can have an SM, each asks for nearly half of the shared memory. 0.8B shape (32 blocks) 26.2 -> 25.3 ms a
-  // chat turn, 35B-A3B shape (128 blocks) 107.8 -> 105.9; with more blocks than SMs there is nothing to spread.
+  // there): where every block can have an SM, each asks for nearly half of the shared memory. 0.8B shape (32 blocks) 26.6 -> 25.7 and
+  // 23.5 -> 22.7 ms a chat turn, both sides in turn on two machines, 35B-A3B shape (128 blocks) 109.2 -> 107.8 and 104.4 -> 102.5; with
+  // more blocks than SMs there is nothing to spread.
   const size_t alone = 4 * sh.TR * nz <= g_llb.sms ? DL_ALONE : 0;
   CU_OK(llb_launch(k_delta, dim3(sh.TR, 4, nz), dim3(DL_THREADS), alone, s, S, ctl, ring, cw, bp, ap, dt, sa, z, nw, sh, xp, rs, g_streams, s_group));
   return 0;
