@@ -8,7 +8,7 @@
 // Can the tcgen05 kernel take this K-split?  (a super-block of every tile for each of its groups, two stages beside the planes)
 // At 8 plane columns it is for launches on their own: between the small kernels of a pass, where the mma.sync kernel's ring and first
 // tiles are ready when the activations come, it is the slower one (27B shape, 24 cycles of four rows 143.6 ms without it, 151 with
-// it; 24 passes of one row 121.7 and 123.4), alone the faster (gate|up at four rows 28.3 and 27.1 us, at one 28.1 and 25.1).
+// it; 24 passes of one row 121.7 and 123.4), alone the faster (gate|up at four rows 27.5 and 27.4 us, at one 27.0 and 25.4).
 static bool g3_fits(int fmt, int NC, int nsb, int ks, bool alone) {
   if (g_llb.gemm3 == 0 || fmt != LLB_FM_Q4_K || (NC == 8 && !alone && g_llb.gemm3 == 2)) return false;
   return ks >= 1 && nsb / ks >= g3_groups(NC) && g3_stages(NC, (nsb + ks - 1) / ks) >= 2;

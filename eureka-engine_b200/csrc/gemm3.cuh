@@ -14,10 +14,10 @@
 //     sign are left: x = 1 + 0.1 N against quantised Gaussian weights, 5120 columns, 6.5e-5 of the result's norm off 64 bits (k_gemm2 3.5e-6).
 //     Centred, the climb is one MMA, the chain's last: 2.3e-6; N(0, 1) 7e-7 -> 3.1e-7 (3.4e-7 to 1.2e-6), silu(g) u 7e-7 -> 3.8e-7 (4e-7 to
 //     5e-6); |N| 2.3e-6 at 5120 columns and 3.7e-6 at 17408 (1.7e-6 and 2.1e-6; at sixteen rows 2.3e-5 and 4.2e-5).
-// gate|up of the 27B shape, operator alone, cold weights: 28.1 -> 25.1 us at one row, 28.3 -> 27.1 at four, 37.3 -> 34.3 at eight, 60.2 -> 53.9
-// at sixteen (not centred 24.7, 26.7, 32.8, 52.8).  What is left: the activations, which every SM reads from L2 at about 10 bytes a cycle (4 us for four rows of 5120
-// columns; cp.async or plain loads, in one order or a different one in every CTA), the groups' chains (2300 cycles a super-block, three groups),
-// and tiles of 128 rows that do not divide evenly.
+// gate|up of the 27B shape, launches of a graph over cold weights: 27.0 -> 25.4 us at one row, 27.5 -> 27.4 at four, 36.4 -> 33.3 at eight, 58.8 ->
+// 46.5 at sixteen; centring cost 0.4 us at one and four rows, 1.5 at eight.  What is left: the activations, which every SM reads before its first
+// MMA (about 4 us for four rows of 5120 columns; cp.async or plain loads, in one order or a different one in every CTA, take the same),
+// the groups' chains of waits, 16 warps an SM deep at most (half of the issue slots are in use), and tiles of 128 rows that do not divide evenly.
 //
 // Roles of a CTA (one an SM): GROUPS of four warps, a thread a weight row, take the super-blocks of the CTA's tiles in turn:
 // unpack into the group's operand buffer, and before the next one read the accumulators of the last and scale them into the
