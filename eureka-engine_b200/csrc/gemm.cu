@@ -281,10 +281,18 @@ static bool g3_use(int fmt, int NC, int ntiles, int nsb, int ks, int sms, bool a
 }
 // The operator's K-slices where the caller names none, and in *g3 its kernel: each kernel's own best, then the better of the two.
 static int gemm_pick_alone(int fmt, int NC, int ntiles, int nsb, int sms, bool *g3) {
+  const int least = g2_least_ksplit(fmt, NC, nsb);
   int k2 = 0, k3 = 0;
+  double c2 = 0.0, c3 = 0.0;
   for (int ks = 1; ks <= GEMM_MAXSPLIT && ks <= nsb; ks++) {
-    if (ks >= g2_least_ksplit(fmt, NC, nsb) && (!k2 || gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, true) < gemm_split_cost(fmt, NC, ntiles, nsb, k2, sms, true) - 1e-9)) k2 = ks;
-    if (g3_fits(fmt, NC, nsb, ks, true) && (!k3 || g3_us(NC, ntiles, nsb, ks, sms) + (NC == 8 ? 0.3 : 0.0) * (ks - k3) < g3_us(NC, ntiles, nsb, k3, sms))) k3 = ks;
+    if (ks >= least) {
+      const double c = gemm_split_cost(fmt, NC, ntiles, nsb, ks, sms, true);
+      if (!k2 || c < c2 - 1e-9) { k2 = ks; c2 = c; }
+    }
+    if (g3_fits(fmt, NC, nsb, ks, true)) {
+      const double c = g3_us(NC, ntiles, nsb, ks, sms) + (NC == 8 ? 0.3 : 0.0) * ks;
+      if (!k3 || c < c3) { k3 = ks; c3 = c; }
+    }
   }
   *g3 = k3 && (!k2 || g_llb.gemm3 == 1 || g3_better(NC, ntiles, nsb, k3, k2, sms));
   return *g3 ? k3 : k2 ? k2 : gemm_fix_ksplit(fmt, NC, nsb, 1, true);
