@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(2 * HD, HD > 128 ? 1 : 2) k_attn_mma(const flo
 // (llb_attn4_combine + llb_t_ogq, tools/payload-sk8add.patch, tools/payload-spec2.patch:149-156)
 // block = (head, row); thread (sg, i4): split group sg, dims 4*i4 .. 4*i4+3
 __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm, const float *__restrict__ pl, const float *__restrict__ po, PartIn qg,
-                                                   AttnShape sh, int nsplit, int Tmax, XPlanes xp, const RowSet *rs, __half *__restrict__ kg, int kg_row0) {
+                                                   AttnShape sh, int nsplit, int Tmax, XPlanes xp, const RowSet *rs, __half *__restrict__ kg, int kg_row0, int kg_ru) {
   {
     const size_t z = blockIdx.z, per = (size_t)sh.H * Tmax * nsplit;
     rs = (const RowSet *)((uintptr_t)rs + z * sh.rs_stride);
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm,
     const float hv[4] = {(a.x / L) / (1.0f + expf(-gate.x)), (a.y / L) / (1.0f + expf(-gate.y)), (a.z / L) / (1.0f + expf(-gate.z)),
                          (a.w / L) / (1.0f + expf(-gate.w))};
     // the prompt path takes the rows as fp16 in the dense GEMM's k-group-major order instead of the T-row planes
-    if (kg) pf_kg_store4(kg, sh.H * hd, kg_row0 + t, h * hd + 4 * i, hv[0], hv[1], hv[2], hv[3]);
+    if (kg) pf_kg_store4(kg, sh.H * hd, kg_ru, kg_row0 + t, h * hd + 4 * i, hv[0], hv[1], hv[2], hv[3]);
     else xp_store4(xp, xrow0 + t, 2, h * hd + 4 * i, hv, lane, true);
   }
 }
@@ -312,7 +312,7 @@ int att_prompt_split(int KV, int hd, int nz, int total, int sms, int cap) {
 }
 
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,
-                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg, int kg_row0, int nz) {
+                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg, int kg_ru, int nz) {
   const int G = sh.H / sh.KV, NQ = G * Tmax, nqg = (NQ + 7) / 8;
   dim3 grid(sh.KV, nsplit, nz);
   int rc;
@@ -321,7 +321,7 @@ int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *V
   else return llb_fail("attention: head_dim %d", sh.hd);
   if (rc) return rc;
   CU_OK(cudaGetLastError());
-  CU_OK(llb_launch(k_attn_comb, dim3(sh.H, Tmax, nz), dim3(256), (size_t)(0), s, pm, pl, po, qg, sh, nsplit, Tmax, xp, rs, kg, kg_row0));
+  CU_OK(llb_launch(k_attn_comb, dim3(sh.H, Tmax, nz), dim3(256), (size_t)(0), s, pm, pl, po, qg, sh, nsplit, Tmax, xp, rs, kg, 0, kg_ru));
   CU_OK(cudaGetLastError());
   return 0;
 }

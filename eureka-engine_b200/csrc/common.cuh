@@ -107,23 +107,35 @@ __device__ __forceinline__ void xp_store4(const XPlanes &xp, int t, int planes, 
 }
 
 // ---- activations of a prompt chunk ----------------------------------------------------------------
-#define PF_R 128              // rows of a unit of a prompt chunk: the half of the dense GEMM's N = 256 that one CTA of a pair holds (pfmm.cuh)
+#define PF_R 128              // most rows of a unit of a prompt chunk: the half of the dense GEMM's N = 256 that one CTA of a pair holds (pfmm.cuh)
 #define PF_RMAX 256           // rows of a chunk, PF_RMAX / PF_R units
-// Activations of a chunk for the dense GEMM, "k-group major", as two fp16 planes like the T-row planes: hi = fp16(x),
-// lo = fp16((x - hi) * 2048), about 22 bits of x.  Element (row r, column k) of a [PF_R][K] matrix sits at half index
-// ((k >> 3) * PF_R + r) * 8 + (k & 7) of its plane; the lo plane follows the hi plane (K * PF_R halves further on).  Eight
-// consecutive columns of one row are one 16-byte core-matrix row, the PF_R rows of a k-group are contiguous (2 KB), and
-// a 64-column stage of one plane is one contiguous run (16 KB).  A chunk of more than PF_R rows is two such matrices one after the other.
-__host__ __device__ inline size_t pf_kg_halves(int K) { return (size_t)2 * K * PF_R; }
-// four consecutive columns k .. k+3 (k a multiple of 4) of row r into both planes
-__device__ __forceinline__ void pf_kg_store4(__half *x, int K, int r, int k, float v0, float v1, float v2, float v3) {
-  if (r >= PF_R) { x += pf_kg_halves(K); r -= PF_R; }   // a second unit of a chunk follows the first
-  const size_t i = ((size_t)(k >> 3) * PF_R + r) * 8 + (k & 4);
-  const __half2 a = __floats2half2_rn(v0, v1), b = __floats2half2_rn(v2, v3);
+// Activations of a chunk for the dense GEMMs, "k-group major": one or two units of ru = 32, 64 or 128 rows (pf_unit_rows), each as two
+// fp16 planes like the T-row planes: hi = fp16(x), lo = fp16((x - hi) * 2048), about 22 bits of x.  Element (row r, column k) of a
+// unit sits at half index ((k >> 3) * ru + r) * 8 + xp_perm(k & 7) of its plane, the lo plane K * ru halves further on: eight
+// consecutive columns of a row are one 16-byte core-matrix row in the order the unpacked codes have, the rows of a k-group are
+// contiguous, and so is a plane's 64-column stage.  Behind the planes of a unit the means of every 32 columns, hi and then lo
+// likewise: the eight of a super-block are a core-matrix row, stored twice (the two k-groups of a K = 16 step): [super-block][2][row][8].
+__host__ __device__ inline int pf_unit_rows(int R) { return R > 64 ? 128 : R > 32 ? 64 : 32; }
+__host__ __device__ inline size_t pf_sum_halves(int K, int ru) { return (size_t)K / 16 * ru; }               // of one plane's means
+__host__ __device__ inline size_t pf_kg_halves(int K, int ru) { return (size_t)2 * K * ru + 2 * pf_sum_halves(K, ru); }
+// Four consecutive columns k .. k+3 (k a multiple of 4) of row r into both planes, and the mean of the 32 that lanes 8 j .. 8 j + 7 of the warp hold
+__device__ __forceinline__ void pf_kg_store4(__half *x, int K, int ru, int r, int k, float v0, float v1, float v2, float v3) {
+  if (r >= ru) { x += pf_kg_halves(K, ru); r -= ru; }   // a second unit of a chunk follows the first
+  const size_t i = ((size_t)(k >> 3) * ru + r) * 8 + (k & 4);
+  const __half2 a = __floats2half2_rn(v0, v2), b = __floats2half2_rn(v1, v3);
   const float2 af = __half22float2(a), bf = __half22float2(b);
-  const __half2 c = __floats2half2_rn((v0 - af.x) * XP_LO_SCALE, (v1 - af.y) * XP_LO_SCALE), d = __floats2half2_rn((v2 - bf.x) * XP_LO_SCALE, (v3 - bf.y) * XP_LO_SCALE);
+  const __half2 c = __floats2half2_rn((v0 - af.x) * XP_LO_SCALE, (v2 - af.y) * XP_LO_SCALE), d = __floats2half2_rn((v1 - bf.x) * XP_LO_SCALE, (v3 - bf.y) * XP_LO_SCALE);
   *(uint2 *)(x + i) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
-  *(uint2 *)(x + (size_t)K * PF_R + i) = make_uint2(*(const uint32_t *)&c, *(const uint32_t *)&d);
+  *(uint2 *)(x + (size_t)K * ru + i) = make_uint2(*(const uint32_t *)&c, *(const uint32_t *)&d);
+  float m = ((v0 + v1) + v2) + v3;
+#pragma unroll
+  for (int s = 1; s < 8; s <<= 1) m += __shfl_xor_sync(0xffffffffu, m, s);
+  m *= 0.03125f;
+  const int l = threadIdx.x & 7;
+  if (l < 4) {   // (plane, k-group)
+    const __half h = __float2half_rn(m);
+    x[(size_t)2 * K * ru + (l >> 1) * pf_sum_halves(K, ru) + ((size_t)(k >> 8) * 2 + (l & 1)) * ru * 8 + r * 8 + ((k >> 5) & 7)] = l >> 1 ? __float2half_rn((m - __half2float(h)) * XP_LO_SCALE) : h;
+  }
 }
 // ---- programmatic dependent launch --------------------------------------------------------------
 // Every kernel of a pass is launched with the programmatic-serialization attribute: the next kernel's

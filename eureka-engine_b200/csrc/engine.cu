@@ -1056,7 +1056,7 @@ static int pf_alloc(llb_spec *m) {
   if (f.ready) return 0;
   CK(pf_setup());
   const int d = m->d, qa = m->H * m->hd;
-  auto kg = [&](int K) { return (__half *)dalloc(m, (PF_RMAX / PF_R) * pf_kg_halves(K) * 2); };   // the chunk's units one after the other
+  auto kg = [&](int K) { return (__half *)dalloc(m, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
   f.x = falloc(m, (size_t)PF_RMAX * d); f.x1 = falloc(m, (size_t)PF_RMAX * d); f.hn = falloc(m, (size_t)(PF_RMAX + 1) * d); f.e = falloc(m, (size_t)PF_RMAX * d);
   f.qn = falloc(m, (size_t)PF_RMAX * qa); f.y = falloc(m, (size_t)PF_RMAX * m->convd); f.beta = falloc(m, (size_t)PF_RMAX * m->TR); f.gram = falloc(m, (size_t)PF_RMAX / 8 * 64 * m->GK);
   f.decay = falloc(m, (size_t)PF_RMAX * m->TR); f.o = falloc(m, (size_t)PF_RMAX * m->vdc);
@@ -1162,7 +1162,7 @@ static int pf_chunk(llb_spec *m, int b, const int *ids, int p0, int R) {
       PFK("gemm qkv", pf_site(m, {{&l.at.q, &f.q}, {&l.at.k, &f.k}, {&l.at.v, &f.v}}, f.kg_d, d, R));
       PFK("qkrope", op_qkrope(s, as_in(f.q), as_in(f.k), as_in(f.v), l.at.qn, l.at.kn, m->invfreq, ash, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), &f.rs[0], R));
       // every group of gsz rows in one launch (grid z): each streams the K/V rows up to its own last position
-      PFK("attention", op_attention(s, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), as_in(f.q), ash, nsp, f.pm, f.pl, f.po, m->xp_qa, &f.rs[1], gsz, f.kg_qa, 0, ngrp));
+      PFK("attention", op_attention(s, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), as_in(f.q), ash, nsp, f.pm, f.pl, f.po, m->xp_qa, &f.rs[1], gsz, f.kg_qa, pf_unit_rows(R), ngrp));
       PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
     } else {
       PFK("gemm qkv|z|b|a", pf_site(m, {{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));

@@ -7,6 +7,7 @@
 // differs is the GEMM operand precision (fp16, see pfmm.cuh) and that a DeltaNet layer scans the chunk's rows in one
 // kernel with the state in registers, writing the state once.
 #include "pfmm.cuh"
+#include "pfx.cuh"
 #include "model.cuh"
 #include "pf.cuh"
 
@@ -16,13 +17,27 @@ template <int FMT> static int pf_attr() {
   CU_OK(cudaFuncSetAttribute(k_pfmm<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
   return 0;
 }
+template <int FMT> static int px_attr1() {
+  CU_OK(cudaFuncSetAttribute(k_pfx1<FMT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, px_smem(FMT, 32)));
+  CU_OK(cudaFuncSetAttribute(k_pfx1<FMT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, px_smem(FMT, 64)));
+  CU_OK(cudaFuncSetAttribute(k_pfx1<FMT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, px_smem(FMT, 128)));
+  return 0;
+}
+template <int FMT> static int px_attr2() {
+  CU_OK(cudaFuncSetAttribute(k_pfx2<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, px2_smem(FMT)));
+  cudaFuncAttributes at;   // its warpgroups trade registers: a launch with fewer than they were counted with would wait for ever
+  CU_OK(cudaFuncGetAttributes(&at, k_pfx2<FMT>));
+  if (at.numRegs != PX_REG_LAUNCH) return llb_fail("k_pfx2: built with %d registers a thread, its register split needs %d", at.numRegs, PX_REG_LAUNCH);
+  return 0;
+}
 #define PF_SCAN_NW 4                            // warps of a scan block, 8 state rows each
 #define PF_SCAN_BLOCKS (128 / (8 * PF_SCAN_NW)) // blocks of a head
 #define PF_SCAN_SMEM (220 * 1024)
 __global__ void k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
                           const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R);
 int pf_setup(void) {
-  if (pf_attr<LLB_FM_Q4_K>() || pf_attr<LLB_FM_Q5_K>() || pf_attr<LLB_FM_Q6_K>() || pf_attr<LLB_FM_Q8_0>()) return -1;
+  if (pf_attr<LLB_FM_Q6_K>() || pf_attr<LLB_FM_Q8_0>()) return -1;
+  if (px_attr1<LLB_FM_Q4_K>() || px_attr1<LLB_FM_Q5_K>() || px_attr1<LLB_FM_Q6_K>() || px_attr1<LLB_FM_Q8_0>() || px_attr2<LLB_FM_Q4_K>() || px_attr2<LLB_FM_Q5_K>()) return -1;
   CU_OK(cudaFuncSetAttribute(k_pf_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SCAN_SMEM - 24 * 1024));
   if (!g_pf_err) {
     CU_OK(cudaMalloc(&g_pf_err, 4));
@@ -64,15 +79,22 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a) {
   const int units = (a.t128[a.nmat] + 1) / 2 * a.ksplit;   // pairs of tiles
   if (units < 1) return 0;
   const int grid = 2 * (units < g_llb.sms / 2 ? units : g_llb.sms / 2);
-  cudaError_t e;
+  cudaError_t e = cudaErrorInvalidValue;
+  const int ru = pf_unit_rows(a.R);
+#define PX_GO(F, RU) e = llb_launch(k_pfx1<F, RU>, dim3(grid), dim3(PX_THREADS), (size_t)px_smem(F, RU), s, a)
+#define PX_ONE(F) do { if (ru == 32) PX_GO(F, 32); else if (ru == 64) PX_GO(F, 64); else PX_GO(F, 128); } while (0)
+#define PX_TWO(F) e = llb_launch(k_pfx2<F>, dim3(grid), dim3(PX_THREADS), (size_t)px2_smem(F), s, a)
   switch (fmt) {
-    case LLB_FM_Q4_K: e = llb_launch(k_pfmm<LLB_FM_Q4_K>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); break;
-    case LLB_FM_Q5_K: e = llb_launch(k_pfmm<LLB_FM_Q5_K>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); break;
-    case LLB_FM_Q6_K: e = llb_launch(k_pfmm<LLB_FM_Q6_K>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); break;
-    case LLB_FM_Q8_0: e = llb_launch(k_pfmm<LLB_FM_Q8_0>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); break;
+    case LLB_FM_Q4_K: if (a.R > PF_R) PX_TWO(LLB_FM_Q4_K); else PX_ONE(LLB_FM_Q4_K); break;
+    case LLB_FM_Q5_K: if (a.R > PF_R) PX_TWO(LLB_FM_Q5_K); else PX_ONE(LLB_FM_Q5_K); break;
+    case LLB_FM_Q6_K: if (a.R > PF_R) e = llb_launch(k_pfmm<LLB_FM_Q6_K>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); else PX_ONE(LLB_FM_Q6_K); break;
+    case LLB_FM_Q8_0: if (a.R > PF_R) e = llb_launch(k_pfmm<LLB_FM_Q8_0>, dim3(grid), dim3(PF_THREADS), (size_t)PF_SMEM, s, a); else PX_ONE(LLB_FM_Q8_0); break;
     default: return llb_fail("pf gemm: format %d has no kernel", fmt);
   }
-  if (e != cudaSuccess) return llb_fail("k_pfmm launch: %s", cudaGetErrorString(e));
+#undef PX_TWO
+#undef PX_ONE
+#undef PX_GO
+  if (e != cudaSuccess) return llb_fail("dense GEMM launch: %s", cudaGetErrorString(e));
   return 0;
 }
 
@@ -117,7 +139,7 @@ int op_pf_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const int *ids
 #define PF_NORM_MAXT 1024
 template <int NI>
 __global__ void __launch_bounds__(PF_NORM_MAXT) k_pf_norm(const float *__restrict__ xin, PartIn add, const float *__restrict__ w, float eps, int d,
-                                                          float *__restrict__ xout, __half *__restrict__ kg, int kg_K, int kg_col0, float *__restrict__ hn_out) {
+                                                          float *__restrict__ xout, __half *__restrict__ kg, int kg_K, int kg_col0, int ru, float *__restrict__ hn_out) {
   float4 wv[NI];
 #pragma unroll
   for (int i = 0; i < NI; i++) {
@@ -150,17 +172,17 @@ __global__ void __launch_bounds__(PF_NORM_MAXT) k_pf_norm(const float *__restric
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
-    if (c >= d) continue;
+    if (c >= d) continue;   // whole warps: d is a multiple of 128
     const float h0 = v[i].x * sc * wv[i].x, h1 = v[i].y * sc * wv[i].y, h2 = v[i].z * sc * wv[i].z, h3 = v[i].w * sc * wv[i].w;
     if (hn_out) *(float4 *)(hn_out + row + c) = make_float4(h0, h1, h2, h3);
-    if (kg) pf_kg_store4(kg, kg_K, t, kg_col0 + c, h0, h1, h2, h3);
+    if (kg) pf_kg_store4(kg, kg_K, ru, t, kg_col0 + c, h0, h1, h2, h3);
   }
 }
 int op_pf_norm(cudaStream_t s, const float *xin, PartIn add, const float *w, float eps, int d, float *xout, __half *kg, int kg_K, int kg_col0, float *hn_out, int R) {
-  if (d % 8 || kg_col0 % 8 || d > 4 * 4 * PF_NORM_MAXT) return llb_fail("pf norm: d %d at column %d", d, kg_col0);
+  if (d % 128 || kg_col0 % 128 || d > 4 * 4 * PF_NORM_MAXT) return llb_fail("pf norm: d %d at column %d", d, kg_col0);
   const int d4 = d / 4, ni = (d4 + PF_NORM_MAXT - 1) / PF_NORM_MAXT;
   const int threads = (((d4 + ni - 1) / ni) + 31) & ~31;
-#define PF_NORM_GO(NI) CU_OK(llb_launch(k_pf_norm<NI>, dim3(R), dim3(threads), (size_t)0, s, xin, add, w, eps, d, xout, kg, kg_K, kg_col0, hn_out))
+#define PF_NORM_GO(NI) CU_OK(llb_launch(k_pf_norm<NI>, dim3(R), dim3(threads), (size_t)0, s, xin, add, w, eps, d, xout, kg, kg_K, kg_col0, pf_unit_rows(R), hn_out))
   switch (ni) {
     case 1: PF_NORM_GO(1); break;
     case 2: PF_NORM_GO(2); break;
@@ -172,17 +194,17 @@ int op_pf_norm(cudaStream_t s, const float *xin, PartIn add, const float *w, flo
 }
 
 // silu(gate) * up -> activations of ffn_down (llb_t_siluq)
-__global__ void __launch_bounds__(256) k_pf_silu(PartIn g, PartIn u, int f, __half *__restrict__ kg) {
+__global__ void __launch_bounds__(256) k_pf_silu(PartIn g, PartIn u, int f, int ru, __half *__restrict__ kg) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.y, c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (c >= f) return;
+  if (c >= f) return;   // whole warps
   const size_t i = (size_t)t * f + c;
   const float4 gv = part_get4(g, i), uv = part_get4(u, i);
-  pf_kg_store4(kg, f, t, c, pf_silu(gv.x) * uv.x, pf_silu(gv.y) * uv.y, pf_silu(gv.z) * uv.z, pf_silu(gv.w) * uv.w);
+  pf_kg_store4(kg, f, ru, t, c, pf_silu(gv.x) * uv.x, pf_silu(gv.y) * uv.y, pf_silu(gv.z) * uv.z, pf_silu(gv.w) * uv.w);
 }
 int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R) {
-  CU_OK(llb_launch(k_pf_silu, dim3((f / 4 + 255) / 256, R), dim3(256), (size_t)0, s, g, u, f, kg));
+  CU_OK(llb_launch(k_pf_silu, dim3((f / 4 + 255) / 256, R), dim3(256), (size_t)0, s, g, u, f, pf_unit_rows(R), kg));
   return 0;
 }
 
@@ -345,11 +367,6 @@ __global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const 
 // 3011-token prompt (48 layers, 48 heads), 47 -> 28 ms of 4096 tokens (24 layers, 32 heads), 23 -> 9.7 ms of 2000 tokens (18
 // layers, 8 heads).
 // Rows come through double-buffered shared memory, the next eight requested before the present ones are computed.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 x2_pack(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ void x2_unpack(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 x2_fma(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ f32x2 x2_mul(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
                                                      const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R) {
   constexpr int NT = 32 * PF_SCAN_NW, NJ = 8 * PF_SCAN_NW, VS = NJ + 4;   // a block's threads and state rows; v rows padded so that eight lanes' reads miss one another's banks
@@ -508,7 +525,7 @@ __global__ void __launch_bounds__(256) k_pf_gnorm(const float *__restrict__ o, P
   const size_t idx = (size_t)t * sh.vdc + hh * 128 + 4 * i;
   const float4 v = __ldcg((const float4 *)(o + idx)), zz = part_get4(z, idx);
   const float r = 1.0f / sqrtf(pf_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) / 128.0f + sh.eps);
-  pf_kg_store4(kg, sh.vdc, t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
+  pf_kg_store4(kg, sh.vdc, pf_unit_rows(R), t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
 }
 
 // One DeltaNet layer's ops between its input GEMM (qkv | z | beta | alpha) and its output GEMM, for R rows at p0 ...
@@ -531,16 +548,16 @@ int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, floa
 
 // ---- operator entry point: the dense GEMM alone ------------------------------------------------------
 // f32 rows [R][K] -> fp16, k-group major
-__global__ void __launch_bounds__(256) k_pf_pack(const float *__restrict__ x, int K, __half *__restrict__ kg) {
+__global__ void __launch_bounds__(256) k_pf_pack(const float *__restrict__ x, int K, int ru, __half *__restrict__ kg) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.y, c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (c >= K) return;
+  if (c >= K) return;   // whole warps: K is a multiple of 128
   const float4 v = __ldcg((const float4 *)(x + (size_t)t * K + c));
-  pf_kg_store4(kg, K, t, c, v.x, v.y, v.z, v.w);
+  pf_kg_store4(kg, K, ru, t, c, v.x, v.y, v.z, v.w);
 }
 int op_pf_pack(cudaStream_t s, const float *x, int K, int R, __half *kg) {
-  CU_OK(llb_launch(k_pf_pack, dim3((K / 4 + 255) / 256, R), dim3(256), (size_t)0, s, x, K, kg));
+  CU_OK(llb_launch(k_pf_pack, dim3((K / 4 + 255) / 256, R), dim3(256), (size_t)0, s, x, K, pf_unit_rows(R), kg));
   return 0;
 }
 
@@ -555,8 +572,8 @@ int llb_b200_pf_gemm(int fmt, unsigned long long w, int rows, int K, unsigned lo
   if (ksplit > nsb) return llb_fail("pf_gemm: %d K-slices of %d super-blocks", ksplit, nsb);
   __half *kg = nullptr;
   float *parts = nullptr;
-  CU_OK(cudaMalloc(&kg, 2 * pf_kg_halves(K) * 2));      // two units of 128 rows
-  CU_OK(cudaMemsetAsync(kg, 0, 2 * pf_kg_halves(K) * 2, g_llb.stream));
+  CU_OK(cudaMalloc(&kg, 2 * pf_kg_halves(K, PF_R) * 2));      // two units of 128 rows
+  CU_OK(cudaMemsetAsync(kg, 0, 2 * pf_kg_halves(K, PF_R) * 2, g_llb.stream));
   if (ksplit > 1) CU_OK(cudaMalloc(&parts, (size_t)ksplit * R * rows * 4));
   int rc = op_pf_pack(g_llb.stream, (const float *)(uintptr_t)x_f32, K, R, kg);
   PfArgs a;

@@ -1,5 +1,5 @@
 // pfmm.cuh -- the prompt path's dense GEMM on the fifth-generation tensor cores: Y[r][n] = sum_k W[n][k] X[r][k] for a
-// chunk of up to 256 prompt rows against Q4_K / Q5_K / Q6_K / Q8_0 weights.  It replaces, for this library, the
+// chunk of 129 to 256 prompt rows against Q6_K / Q8_0 weights (the others, and fewer rows: pfx.cuh).  It replaces, for this library, the
 // reference's chunked tensor-core prefill GEMM (tools/pf27/pfmm.cuh:311-384: int8 mma.sync + cp.async on sm_86; its
 // caller host/llb_pf.h:551 pf_take) with a design for sm_100a:
 //
@@ -55,7 +55,7 @@ __device__ __forceinline__ void pf_bulk_copy(uint32_t dst_s, const void *src, ui
 // ---- weights: packed super-blocks -> fp16 core-matrix rows ------------------------------------------
 // A thread takes the 32 weights of one row that start at column c0 (a multiple of 32): raw words with pf_load, fp32
 // values with pf_deq, then pf_split8 turns every eight of them into a 16-byte row of each plane (k-groups c0/8 .. + 3).
-struct PfRaw { uint32_t w[8], x[8], h[4]; };
+struct PfRaw { uint32_t w[8], x[8], h[2]; };
 
 // row: the row's block in the first super-block of its row tile;  doff: from there to the row's d (Q6_K)
 template <int FMT> __device__ __forceinline__ void pf_load(const uint8_t *row, int doff, int c0, PfRaw &r) {
@@ -65,7 +65,7 @@ template <int FMT> __device__ __forceinline__ void pf_load(const uint8_t *row, i
     const uint4 a = ldg128(blk + i), b = ldg128(blk + i + 16);
     r.w[0] = a.x; r.w[1] = a.y; r.w[2] = a.z; r.w[3] = a.w; r.w[4] = b.x; r.w[5] = b.y; r.w[6] = b.z; r.w[7] = b.w;
     r.h[0] = *(const unsigned short *)(blk + 256 + 2 * (i >> 5));
-  } else if constexpr (FMT == LLB_FM_Q6_K) {
+  } else {
     const int j8 = (c0 >> 5) & 7, hf = j8 >> 2, qd = j8 & 3;
     const uint4 a = ldg128(blk + 64 * hf + 32 * (qd & 1)), b = ldg128(blk + 64 * hf + 32 * (qd & 1) + 16);
     const uint4 c = ldg128(blk + 128 + 32 * hf), d = ldg128(blk + 128 + 32 * hf + 16);
@@ -73,23 +73,12 @@ template <int FMT> __device__ __forceinline__ void pf_load(const uint8_t *row, i
     r.x[0] = c.x; r.x[1] = c.y; r.x[2] = c.z; r.x[3] = c.w; r.x[4] = d.x; r.x[5] = d.y; r.x[6] = d.z; r.x[7] = d.w;
     r.h[0] = *(const unsigned short *)(blk + 192 + 8 * hf + 2 * qd);   // the two int8 scales of this quarter
     r.h[1] = *(const unsigned short *)(blk + doff);
-  } else {
-    constexpr int QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
-    const int g = (c0 >> 6) & 3;
-    const uint4 hd = ldg128(blk), a = ldg128(blk + QOFF + 32 * g), b = ldg128(blk + QOFF + 32 * g + 16);
-    r.h[0] = hd.x; r.h[1] = hd.y; r.h[2] = hd.z; r.h[3] = hd.w;
-    r.w[0] = a.x; r.w[1] = a.y; r.w[2] = a.z; r.w[3] = a.w; r.w[4] = b.x; r.w[5] = b.y; r.w[6] = b.z; r.w[7] = b.w;
-    if constexpr (FMT == LLB_FM_Q5_K) {
-      const uint4 c = ldg128(blk + 16), d = ldg128(blk + 32);
-      r.x[0] = c.x; r.x[1] = c.y; r.x[2] = c.z; r.x[3] = c.w; r.x[4] = d.x; r.x[5] = d.y; r.x[6] = d.z; r.x[7] = d.w;
-    }
   }
 }
 
 // An integer code c < 128 sitting in bits 16.. of a word becomes the float 128 + c by OR-ing 0x43000000 (no conversion
 // instruction); one FMA then gives scale * c - offset: fmaf(128 + c, scale, -(128 scale + offset)).  The constant is rounded
-// once per sub-block (about 1e-6 of a weight), instead of every weight being rounded twice as in the reference's
-// d * sc * q - dmin * m; both planes together still carry the result to about 22 bits.
+// once per sub-block (about 1e-6 of a weight); both planes together still carry the result to about 22 bits.
 __device__ __forceinline__ float pf_code_f(uint32_t x, int j, uint32_t mask) {
   // byte j of x, masked, moved to bits 16..: shifts by 16, 8, 0, -8
   const uint32_t v = j == 0 ? x << 16 : j == 1 ? x << 8 : j == 2 ? x : x >> 8;
@@ -109,7 +98,7 @@ template <int FMT> __device__ __forceinline__ void pf_deq(const PfRaw &r, int c0
         w[4 * i + j] = fmaf(__uint_as_float((v & (0xffu << 15)) | 0x43800000u), d, c);
       }
     }
-  } else if constexpr (FMT == LLB_FM_Q6_K) {
+  } else {
     const int qd = (c0 >> 5) & 3;
     const float d = h2f_bits(r.h[1]);
     const float s0 = __fmul_rn(d, (float)(int8_t)(r.h[0] & 0xff)), s1 = __fmul_rn(d, (float)(int8_t)(r.h[0] >> 8));
@@ -121,29 +110,16 @@ template <int FMT> __device__ __forceinline__ void pf_deq(const PfRaw &r, int c0
 #pragma unroll
       for (int j = 0; j < 4; j++) w[4 * i + j] = fmaf(pf_code_f(c6, j, 0x3fu), i < 4 ? s0 : s1, i < 4 ? k0 : k1);
     }
-  } else {
-    const int j8 = (c0 >> 5) & 7, hi = j8 & 1;
-    uint32_t scA, scB, mnA, mnB;
-    k4_scales(r.h[1], r.h[2], r.h[3], scA, scB, mnA, mnB);
-    const float sc = (float)(((j8 < 4 ? scA : scB) >> (8 * (j8 & 3))) & 0xffu), mn = (float)(((j8 < 4 ? mnA : mnB) >> (8 * (j8 & 3))) & 0xffu);
-    const float ds = __fmul_rn(h2f_bits(r.h[0] & 0xffffu), sc), dm = __fmul_rn(h2f_bits(r.h[0] >> 16), mn);
-    const float c = -fmaf(128.0f, ds, dm);
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      uint32_t x = (hi ? r.w[i] >> 4 : r.w[i]) & 0x0f0f0f0fu;
-      if constexpr (FMT == LLB_FM_Q5_K) x |= ((r.x[i] >> j8) & 0x01010101u) << 4;   // the fifth bit of column l is bit j8 of qh byte l
-#pragma unroll
-      for (int j = 0; j < 4; j++) w[4 * i + j] = fmaf(pf_code_f(x, j, 0x1fu), ds, c);
-    }
   }
 }
-// eight weights -> one 16-byte row of the hi plane and one of the lo plane.  hi is the weight with its low 13 mantissa
+// eight weights -> one 16-byte row of the hi plane and one of the lo plane, in the activations' order of columns (xp_perm).  hi is the weight with its low 13 mantissa
 // bits cleared (exactly an fp16 number for normal magnitudes), lo the exact remainder times 2048.
 __device__ __forceinline__ void pf_split8(const float *w, uint4 &hi, uint4 &lo) {
   uint32_t h[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const float a = w[2 * i], b = w[2 * i + 1];
+    const int c = (i >> 1) * 4 + (i & 1);
+    const float a = w[c], b = w[c + 2];
     const float ah = __uint_as_float(__float_as_uint(a) & 0xffffe000u), bh = __uint_as_float(__float_as_uint(b) & 0xffffe000u);
     const __half2 hh = __floats2half2_rn(ah, bh), ll = __floats2half2_rn((a - ah) * XP_LO_SCALE, (b - bh) * XP_LO_SCALE);
     h[i] = *(const uint32_t *)&hh; l[i] = *(const uint32_t *)&ll;
@@ -272,7 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1) k_pfm
     if (lane == 0) {
       int it = 0;
       pdl_wait();   // the activations come from the kernel in front; the weights do not, and nothing is written before MMAs have read activations
-      const __half *x = a.x + (size_t)rank * pf_kg_halves(a.K);   // a unit's planes follow the previous unit's (common.cuh)
+      const __half *x = a.x + (size_t)rank * pf_kg_halves(a.K, PF_R);   // a unit's planes follow the previous unit's (common.cuh)
       for (int u = unit0; u < nunits; u += ustep) {
         int kbase, nst;
         pf_slice(a, u, npairs, kbase, nst);

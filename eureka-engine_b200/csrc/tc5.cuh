@@ -50,6 +50,19 @@ __device__ __forceinline__ void t5_ld8(uint32_t taddr, float (&v)[8]) {
 #pragma unroll
   for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
+// ---- two fp32 numbers a register pair ----
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 x2_pack(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void x2_unpack(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 x2_fma(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 x2_mul(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// tensor-memory columns as pairs
+__device__ __forceinline__ void t5_ld16x2(uint32_t taddr, f32x2 (&v)[8]) {
+  float f[16];
+  t5_ld16(taddr, f);
+#pragma unroll
+  for (int i = 0; i < 8; i++) v[i] = x2_pack(f[2 * i], f[2 * i + 1]);
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar_s, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_s), "r"(count) : "memory");
 }
