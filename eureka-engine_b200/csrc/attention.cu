@@ -312,7 +312,7 @@ int att_prompt_split(int KV, int hd, int nz, int total, int sms, int cap) {
 }
 
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,
-                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg, int kg_ru, int nz) {
+                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg, int kg_row0, int kg_ru, int nz) {
   const int G = sh.H / sh.KV, NQ = G * Tmax, nqg = (NQ + 7) / 8;
   dim3 grid(sh.KV, nsplit, nz);
   int rc;
@@ -321,7 +321,7 @@ int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *V
   else return llb_fail("attention: head_dim %d", sh.hd);
   if (rc) return rc;
   CU_OK(cudaGetLastError());
-  CU_OK(llb_launch(k_attn_comb, dim3(sh.H, Tmax, nz), dim3(256), (size_t)(0), s, pm, pl, po, qg, sh, nsplit, Tmax, xp, rs, kg, 0, kg_ru));
+  CU_OK(llb_launch(k_attn_comb, dim3(sh.H, Tmax, nz), dim3(256), (size_t)(0), s, pm, pl, po, qg, sh, nsplit, Tmax, xp, rs, kg, kg_row0, kg_ru));
   CU_OK(cudaGetLastError());
   return 0;
 }

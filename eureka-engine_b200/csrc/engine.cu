@@ -8,10 +8,11 @@
 //     the next cycle's inputs) is taken on the device (k_accept / k_draft_pick), so a cycle is one
 //     graph launch and one small result record, instead of k blocking reads plus one host round
 //     trip per served row;
-//   * the prompt is fed through the same T-row pass in chunks of k+1 given tokens.
+//   * a prompt goes through dense GEMMs in pieces of 128 rows (pf_chunk), a short one through the same T-row pass as chunks of given tokens.
 #include <math.h>
 #include <stdlib.h>
 
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -39,10 +40,13 @@ struct LayerW { bool full = false; float *attn_norm = nullptr; AttnW at; DeltaW 
 // blocked: Q8_0 in GGUF's [f16 d][32 x int8] blocks (host memory only), re-sliced to the row-split layout at upload
 struct TensorRec { uint64_t off, bytes; int rows, cols, fmt; bool blocked = false; };
 
-// Buffers of the prompt path (pf.cu), allocated at the first fast prefill: residual rows, fp16 activations in the
-// dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows, and the row sets of the chunk.
+// Buffers of the prompt path (pf.cu), allocated at the first prompt that takes it: residual rows, fp16 activations in the
+// dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows, and the row sets of the chunk.  Nothing in them
+// outlives a prompt, so the engine that has the weights keeps them for its siblings too; a prompt holds them (`busy`) while it is enqueued,
+// and the library's one stream keeps the chunks of several prompts apart.
 struct PfState {
-  bool ready = false;
+  bool ready = false, none = false;   // none: there was no room for them
+  std::mutex busy;
   float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *gram = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
   __half *kg_d = nullptr, *kg_f = nullptr, *kg_qa = nullptr, *kg_v = nullptr, *kg_2d = nullptr;
   OutBuf q, k, v, qkv, z, bp, ap, a, g, u, dn, eh;
@@ -141,8 +145,11 @@ struct llb_spec {
   int Hf = 0, KVf = 0, ff = 0, GKf = 0, TRf = 0, kdcf = 0, vdcf = 0, convdf = 0;
   OutBuf r_a, r_dn;
   PfState pf;
-  int prefill_mode = 0;   // 0: every prompt row through the T-row pass; 1: chunks of PF_RMAX rows through the dense path (LLB_PREFILL=fast)
-  double pf_rows = 0;     // prompt rows the dense path has processed since the engine was opened
+  // 1: all but the last k + 1 prompt rows in chunks of PF_RMAX rows through the dense path (LLB_PREFILL=fast).  0: prompts in pieces of PF_R rows
+  // through the dense path's exact forms, short ones in T-row passes (px_takes)
+  int prefill_mode = 0;
+  bool rows_set = false;  // LLB_PREFILL_ROWS asks for T-row passes of that many rows
+  double pf_rows = 0;     // prompt rows that mode 1 has put through the dense path since the engine was opened
   // graphs
   cudaGraphExec_t g_spec = nullptr, g_prefill = nullptr, g_verify = nullptr;
   // where the logits of a captured pass lie: K-slices, their stride, a stream's rows (the head's split follows the pass's width)
@@ -571,7 +578,7 @@ static int enq_attn(llb_spec *m, const AttnW &w, float *Kc, float *Vc, const Row
                m->B > 1 ? (int)sizeof(SpecCtl) : 0, m->B > 1 ? m->kv_group : 0};
   PK("gemm qkv", site_gemm(m, {{&w.q, &m->b_q, nullptr, nullptr, 0}, {&w.k, &m->b_k, nullptr, nullptr, 0}, {&w.v, &m->b_v, nullptr, nullptr, 0}}, m->xp_d, 0));
   PK("qkrope", op_qkrope(s, as_in(m->b_q), as_in(m->b_k), as_in(m->b_v), w.qn, w.kn, m->invfreq, sh, m->qn, Kc, Vc, rs, m->Tmax));
-  PK("attention", op_attention(s, m->qn, Kc, Vc, as_in(m->b_q), sh, m->att_split, m->pm, m->pl, m->po, m->xp_qa, rs, m->per, nullptr, 0, m->B));
+  PK("attention", op_attention(s, m->qn, Kc, Vc, as_in(m->b_q), sh, m->att_split, m->pm, m->pl, m->po, m->xp_qa, rs, m->per, nullptr, 0, 0, m->B));
   PK("gemm attn_out", site_gemm(m, {{&w.o, &m->b_a, nullptr, nullptr, 0}}, m->xp_qa, 0));
   PK("all-reduce", tp_reduce(m, m->b_a, m->r_a));
   return 0;
@@ -834,7 +841,7 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
     // rows of a prompt chunk: 8, fewer where (H / KV) x rows would pass the attention kernel's 48 queries per kv head
     int pf = 8;
     const char *e = getenv("LLB_PREFILL_ROWS");
-    if (e && atoi(e) >= 1 && atoi(e) <= SPEC_MAXT) pf = atoi(e);
+    if (e && atoi(e) >= 1 && atoi(e) <= SPEC_MAXT) { pf = atoi(e); m->rows_set = true; }
     if (pf > 48 / (m->H / m->KV)) pf = 48 / (m->H / m->KV);
     m->Tpf = pf > m->Tspec ? pf : m->Tspec;
     // several streams: the sixteen rows of a pass shared out among them (eight streams of plain decoding feed two rows each)
@@ -1050,27 +1057,37 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
 }
 
 // ---- the prompt path: chunks of up to PF_RMAX rows through dense tcgen05 GEMMs (pf.cu) ----------------------------
-#define PF_GROUPS (PF_RMAX + 1)
+#define PF_PIECES 16                           // most sequences in a chunk
+#define PF_GROUPS (PF_RMAX + 2 * PF_PIECES)
+static llb_spec *pf_owner(llb_spec *m) { return m->share ? m->share : m; }
+// rows of an attention group (at most 48 queries a kv head) and most K-slices: of the model alone, so that a prompt's sums do not depend on
+// how many streams its engine has
+static int pf_group(const llb_spec *m) { const int q = 48 / (m->H / m->KV); return q < 1 ? 1 : q < SPEC_MAXT ? q : SPEC_MAXT; }
+static int pf_split_cap(const llb_spec *m) { const int n = g_llb.sms / m->KV; return n < 1 ? 1 : n > 128 ? 128 : n; }
 static int pf_alloc(llb_spec *m) {
-  PfState &f = m->pf;
+  llb_spec *o = pf_owner(m);
+  PfState &f = o->pf;
   if (f.ready) return 0;
+  if (f.none) return llb_fail("prompt path: no room for its buffers");
   CK(pf_setup());
+  f.none = true;          // until all of them are there
   const int d = m->d, qa = m->H * m->hd;
-  auto kg = [&](int K) { return (__half *)dalloc(m, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
-  f.x = falloc(m, (size_t)PF_RMAX * d); f.x1 = falloc(m, (size_t)PF_RMAX * d); f.hn = falloc(m, (size_t)(PF_RMAX + 1) * d); f.e = falloc(m, (size_t)PF_RMAX * d);
-  f.qn = falloc(m, (size_t)PF_RMAX * qa); f.y = falloc(m, (size_t)PF_RMAX * m->convd); f.beta = falloc(m, (size_t)PF_RMAX * m->TR); f.gram = falloc(m, (size_t)PF_RMAX / 8 * 64 * m->GK);
-  f.decay = falloc(m, (size_t)PF_RMAX * m->TR); f.o = falloc(m, (size_t)PF_RMAX * m->vdc);
+  auto kg = [&](int K) { return (__half *)dalloc(o, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
+  f.x = falloc(o, (size_t)PF_RMAX * d); f.x1 = falloc(o, (size_t)PF_RMAX * d); f.hn = falloc(o, (size_t)(PF_RMAX + PF_PIECES) * d); f.e = falloc(o, (size_t)PF_RMAX * d);
+  f.qn = falloc(o, (size_t)PF_RMAX * qa); f.y = falloc(o, (size_t)PF_RMAX * m->convd); f.beta = falloc(o, (size_t)PF_RMAX * m->TR); f.gram = falloc(o, (size_t)PF_RMAX / 8 * 64 * m->GK);
+  f.decay = falloc(o, (size_t)PF_RMAX * m->TR); f.o = falloc(o, (size_t)PF_RMAX * m->vdc);
   f.kg_d = kg(d); f.kg_f = kg(m->f); f.kg_qa = kg(qa); f.kg_v = kg(m->vdc); f.kg_2d = kg(2 * d);
   {
-    const size_t ng = (PF_RMAX + m->Tpf - 1) / m->Tpf, per = (size_t)m->H * m->Tpf * m->att_split;
-    f.pm = falloc(m, ng * per); f.pl = falloc(m, ng * per); f.po = falloc(m, ng * per * m->hd);
+    const int gsz = pf_group(m);
+    const size_t ng = (PF_RMAX + gsz - 1) / gsz, per = (size_t)m->H * gsz * pf_split_cap(m);
+    f.pm = falloc(o, ng * per); f.pl = falloc(o, ng * per); f.po = falloc(o, ng * per * m->hd);
     if (!f.pm || !f.pl || !f.po) return -1;
   }
-  f.rs = (RowSet *)dalloc(m, sizeof(RowSet) * (1 + PF_GROUPS));
-  f.ids = (int *)dalloc(m, (size_t)(PF_RMAX + 1) * 4);
+  f.rs = (RowSet *)dalloc(o, sizeof(RowSet) * PF_GROUPS);
+  f.ids = (int *)dalloc(o, (size_t)(PF_RMAX + 1) * 4);
   if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.gram || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
       !f.rs || !f.ids) return -1;
-  f.ready = true;
+  f.none = false; f.ready = true;
   return 0;
 }
 
@@ -1123,7 +1140,7 @@ static int pf_site(llb_spec *m, std::vector<PfSiteMat> mats, const __half *kg, i
       OutBuf &o = *sm.out;
       const size_t need = (size_t)a.ksplit * PF_RMAX * sm.w->rows;
       if (!o.p || o.cap < need) {
-        o.p = falloc(m, need);
+        o.p = falloc(pf_owner(m), need);
         if (!o.p) return -1;
         o.cap = need;
       }
@@ -1136,95 +1153,174 @@ static int pf_site(llb_spec *m, std::vector<PfSiteMat> mats, const __half *kg, i
   return 0;
 }
 
-// One chunk: rows of positions p0 .. p0 + R - 1 with the given tokens through every layer.  Leaves the trunk's K/V rows,
-// conv rings and DeltaNet states as the T-row pass would have (the state written back into the committed slot), the
-// drafter's K/V rows of the same positions, and in pf.hn row 0 the normed hidden of the chunk's last row.
-static int pf_chunk(llb_spec *m, int b, const int *ids, int p0, int R) {
-  PfState &f = m->pf;
+// One chunk: a piece of one or several streams' prompts (rows of positions p0 .. p0 + R - 1 of stream b, `off` of the chunk on) through every
+// layer.  Leaves the trunk's K/V rows, conv rings and DeltaNet states as the T-row pass would have (the state written back into
+// the committed slot), the drafter's K/V rows of the same positions, and in the stream's first row of hn_pf the normed hidden of its last
+// row.  The GEMMs and row-wise ops take all rows at once, what has a sequence's state its piece.
+// (whole: the last piece of a prompt that the dense path takes all of)
+struct PfPiece { int b; const int *ids; int p0, R; bool whole; int off; };
+// normed rows that a piece leaves behind (hn_pf)
+static int pf_keep(const llb_spec *m, const PfPiece &p) { return !p.whole ? 1 : p.p0 + p.R < m->Tspec ? p.p0 + p.R : m->Tspec; }
+static PartIn pf_rows_of(const OutBuf &o, int rows, int off) { return PartIn{o.p + (size_t)off * rows, o.ns, o.stride}; }
+static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
+  PfState &f = pf_owner(m)->pf;
   cudaStream_t s = g_llb.stream;
   StreamScope scope(m, true);   // the chunk's kernels see one stream: stream b's state is handed to them directly
-  const int d = m->d, qa = m->H * m->hd, gsz = m->Tpf, ngrp = (R + gsz - 1) / gsz, nsp = att_prompt_split(m->KV, m->hd, ngrp, p0 + R, g_llb.sms, m->att_split);
-  std::vector<RowSet> rs(1 + ngrp);
-  memset(rs.data(), 0, rs.size() * sizeof(RowSet));
-  rs[0].n = R; rs[0].pos0 = p0;
-  for (int g = 0; g < ngrp; g++) { rs[1 + g].n = R - g * gsz < gsz ? R - g * gsz : gsz; rs[1 + g].pos0 = p0 + g * gsz; }
+  const int d = m->d, qa = m->H * m->hd, kvd = m->KV * m->hd, gsz = pf_group(m);
+  int R = 0;
+  std::vector<RowSet> rs;
+  std::vector<int> rs0, ids;
+  for (PfPiece &p : pc) {       // row sets: the piece's, then those of its attention groups
+    p.off = R; R += p.R;
+    rs0.push_back((int)rs.size());
+    RowSet r;
+    memset(&r, 0, sizeof r);
+    r.n = p.R; r.pos0 = p.p0;
+    rs.push_back(r);
+    for (int g = 0; g < p.R; g += gsz) { r.n = p.R - g < gsz ? p.R - g : gsz; r.pos0 = p.p0 + g; rs.push_back(r); }
+    ids.insert(ids.end(), p.ids + p.p0, p.ids + p.p0 + p.R);
+  }
+  const int ru = pf_unit_rows(R), np = (int)pc.size();
   CU_OK(cudaMemcpyAsync(f.rs, rs.data(), rs.size() * sizeof(RowSet), cudaMemcpyHostToDevice, s));
-  CU_OK(cudaMemcpyAsync(f.ids, ids + p0, (size_t)R * 4, cudaMemcpyHostToDevice, s));
-  CU_OK(cudaStreamSynchronize(s));   // rs is a local: the copy must have read it before it goes
+  CU_OK(cudaMemcpyAsync(f.ids, ids.data(), (size_t)R * 4, cudaMemcpyHostToDevice, s));
+  CU_OK(cudaStreamSynchronize(s));   // the sources are locals: the copies must have read them before they go
   PartIn none{nullptr, 0, 0};
   AttnShape ash{m->H, m->KV, m->hd, m->rope_dim, m->eps, m->att_min, (long long)m->max_ctx * m->KV * m->hd, (int)sizeof(RowSet), 0};
   DeltaShape dsh{m->TR, m->GK, m->SZ, m->KC, m->convd, m->kdc, m->vdc, m->eps};
   PFK("embed", op_pf_embed(s, m->embd.fmt, m->embd.w, d, f.ids, R, f.x));
   for (int il = 0; il < m->L; il++) {
     const LayerW &l = m->layer[il];
-    PFK("norm", op_pf_norm(s, il ? f.x1 : f.x, il ? as_in(f.dn) : none, l.attn_norm, m->eps, d, f.x, f.kg_d, d, 0, nullptr, R));
+    PFK("norm", op_pf_norm(s, il ? f.x1 : f.x, il ? as_in(f.dn) : none, l.attn_norm, m->eps, d, f.x, f.kg_d, d, 0, nullptr, R, ru));
     if (l.full) {
       PFK("gemm qkv", pf_site(m, {{&l.at.q, &f.q}, {&l.at.k, &f.k}, {&l.at.v, &f.v}}, f.kg_d, d, R));
-      PFK("qkrope", op_qkrope(s, as_in(f.q), as_in(f.k), as_in(f.v), l.at.qn, l.at.kn, m->invfreq, ash, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), &f.rs[0], R));
-      // every group of gsz rows in one launch (grid z): each streams the K/V rows up to its own last position
-      PFK("attention", op_attention(s, f.qn, kc_of(m, m->Kc[il], b), kc_of(m, m->Vc[il], b), as_in(f.q), ash, nsp, f.pm, f.pl, f.po, m->xp_qa, &f.rs[1], gsz, f.kg_qa, pf_unit_rows(R), ngrp));
+      for (int i = 0; i < np; i++) {
+        const PfPiece &p = pc[i];
+        const PartIn q = pf_rows_of(f.q, 2 * qa, p.off);
+        float *qn = f.qn + (size_t)p.off * qa, *kc = kc_of(m, m->Kc[il], p.b), *vc = kc_of(m, m->Vc[il], p.b);
+        const int ngrp = (p.R + gsz - 1) / gsz, nsp = att_prompt_split(m->KV, m->hd, ngrp, p.p0 + p.R, g_llb.sms, pf_split_cap(m));
+        PFK("qkrope", op_qkrope(s, q, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), l.at.qn, l.at.kn, m->invfreq, ash, qn, kc, vc, &f.rs[rs0[i]], p.R));
+        // every group of gsz rows in one launch (grid z): each streams the K/V rows up to its own last position
+        PFK("attention", op_attention(s, qn, kc, vc, q, ash, nsp, f.pm, f.pl, f.po, m->xp_qa, &f.rs[rs0[i] + 1], gsz, f.kg_qa, p.off, ru, ngrp));
+      }
       PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
     } else {
       PFK("gemm qkv|z|b|a", pf_site(m, {{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));
-      PFK("delta", op_pf_delta(s, as_in(f.qkv), as_in(f.z), as_in(f.bp), as_in(f.ap), ring_of(m, il, b), m->ring_ks[il], l.dn.conv, l.dn.dt, l.dn.a, l.dn.norm, dsh,
-                     state_of(m, il, b), ctl_of(m, b), f.y, f.gram, f.beta, f.decay, f.o, f.kg_v, p0, R));
+      for (const PfPiece &p : pc)
+        PFK("delta", op_pf_delta(s, pf_rows_of(f.qkv, m->convd, p.off), pf_rows_of(f.z, m->vdc, p.off), pf_rows_of(f.bp, m->TR, p.off), pf_rows_of(f.ap, m->TR, p.off),
+                       ring_of(m, il, p.b), m->ring_ks[il], l.dn.conv, l.dn.dt, l.dn.a, l.dn.norm, dsh,
+                       state_of(m, il, p.b), ctl_of(m, p.b), f.y, f.gram, f.beta, f.decay, f.o, f.kg_v, p.p0, p.R, p.off, ru));
       PFK("gemm ssm_out", pf_site(m, {{&l.dn.out, &f.a}}, f.kg_v, m->vdc, R));
     }
-    PFK("norm", op_pf_norm(s, f.x, as_in(f.a), l.ffn.post, m->eps, d, f.x1, f.kg_d, d, 0, nullptr, R));
+    PFK("norm", op_pf_norm(s, f.x, as_in(f.a), l.ffn.post, m->eps, d, f.x1, f.kg_d, d, 0, nullptr, R, ru));
     PFK("gemm gate|up", pf_site(m, {{&l.ffn.gate, &f.g}, {&l.ffn.up, &f.u}}, f.kg_d, d, R));
-    PFK("silu", op_pf_silu(s, as_in(f.g), as_in(f.u), m->f, f.kg_f, R));
+    PFK("silu", op_pf_silu(s, as_in(f.g), as_in(f.u), m->f, f.kg_f, R, ru));
     PFK("gemm down", pf_site(m, {{&l.ffn.down, &f.dn}}, f.kg_f, m->f, R));
   }
-  // the trunk's output-normed rows: row r of the chunk into pf.hn row r + 1 (row 0 holds the row before the chunk)
-  CK(op_pf_norm(s, f.x1, as_in(f.dn), m->out_norm, m->eps, d, nullptr, nullptr, 0, 0, f.hn + d, R));
+  // the trunk's output-normed rows: piece i's from row off + i + 1 of pf.hn on, the row in front of them that of the position before (a fresh stream's is
+  // zero, host/llb_host.c:1816)
+  for (int i = 0; i < np; i++) {
+    const PfPiece &p = pc[i];
+    float *hn = f.hn + (size_t)(p.off + i) * d;
+    CU_OK(cudaMemcpyAsync(hn, m->hn_pf + (size_t)(m->B > 1 ? p.b * m->Tpf : 0) * d, (size_t)d * 4, cudaMemcpyDeviceToDevice, s));
+    CK(op_pf_norm(s, f.x1 + (size_t)p.off * d, pf_rows_of(f.dn, d, p.off), m->out_norm, m->eps, d, nullptr, nullptr, 0, 0, hn + d, p.R, ru));
+  }
   if (m->has_mtp) {
     // the drafter's row at position p pairs token p with the trunk's normed hidden of position p - 1
     // (host/llb_host.c:1775-1808); a prompt chunk only needs its K and V rows (:1831-1876)
     CK(op_pf_embed(s, m->embd.fmt, m->embd.w, d, f.ids, R, f.e));
-    CK(op_pf_norm(s, f.e, none, m->mt_enorm, m->eps, d, nullptr, f.kg_2d, 2 * d, 0, nullptr, R));
-    CK(op_pf_norm(s, f.hn, none, m->mt_hnorm, m->eps, d, nullptr, f.kg_2d, 2 * d, d, nullptr, R));
+    CK(op_pf_norm(s, f.e, none, m->mt_enorm, m->eps, d, nullptr, f.kg_2d, 2 * d, 0, nullptr, R, ru));
+    for (int i = 0; i < np; i++) CK(op_pf_norm(s, f.hn + (size_t)(pc[i].off + i) * d, none, m->mt_hnorm, m->eps, d, nullptr, f.kg_2d, 2 * d, d, nullptr, pc[i].R, ru, pc[i].off));
     CK(pf_site(m, {{&m->mt_eh, &f.eh}}, f.kg_2d, 2 * d, R));
-    CK(op_pf_norm(s, nullptr, as_in(f.eh), m->mt_attn_norm, m->eps, d, nullptr, f.kg_d, d, 0, nullptr, R));
+    CK(op_pf_norm(s, nullptr, as_in(f.eh), m->mt_attn_norm, m->eps, d, nullptr, f.kg_d, d, 0, nullptr, R, ru));
     CK(pf_site(m, {{&m->mt_at.k, &f.k}, {&m->mt_at.v, &f.v}}, f.kg_d, d, R));
-    CK(op_qkrope(s, none, as_in(f.k), as_in(f.v), m->mt_at.qn, m->mt_at.kn, m->invfreq, ash, f.qn, kc_of(m, m->mt_Kc, b), kc_of(m, m->mt_Vc, b), &f.rs[0], R, true));
+    for (int i = 0; i < np; i++) {
+      const PfPiece &p = pc[i];
+      const int rows = p.R - (pf_keep(m, p) - 1);   // the rest of a prompt is what the drafter catches up over
+      if (rows > 0) CK(op_qkrope(s, none, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), m->mt_at.qn, m->mt_at.kn, m->invfreq, ash, f.qn, kc_of(m, m->mt_Kc, p.b), kc_of(m, m->mt_Vc, p.b), &f.rs[rs0[i]], rows, true));
+    }
   }
-  CU_OK(cudaMemcpyAsync(f.hn, f.hn + (size_t)R * d, (size_t)d * 4, cudaMemcpyDeviceToDevice, s));
-  m->pf_rows += R;
+  for (int i = 0; i < np; i++) {
+    const PfPiece &p = pc[i];
+    const int keep = pf_keep(m, p);
+    float *dst = m->hn_pf + (size_t)(m->B > 1 ? p.b * m->Tpf : 0) * d;
+    CU_OK(cudaMemcpyAsync(dst, f.hn + (size_t)(p.off + i + p.R - keep + 1) * d, (size_t)keep * d * 4, cudaMemcpyDeviceToDevice, s));
+  }
   return 0;
 }
 
-// The fast part of a prompt: whole chunks from position 0 while more than `keep` rows remain for the T-row pass.
-// Returns the position the T-row pass continues from; the drafter's row there is left pending as a one-row catch-up
-// whose hidden (the normed row of the position before) is put where the catch-up reads it.
-static int pf_prefill(llb_spec *m, int b, const int *ids, int n_rows, int keep, int *p_out) {
+// Whether mode 0 puts a prompt of n_rows through the dense path: where T-row passes would read the weights more than once for it.  It then takes all
+// of them, and neither their number nor the rule knows k or the other streams: a prompt leaves the same bits behind in every engine.
+// (27B shape: a pass of eight rows 8.1 ms, a piece of up to 128 rows 14 to 17; 0.8B shape 0.8 and 1.7.)
+static int ctl_write(llb_spec *m, int b, const SpecCtl &c);
+static SpecCtl ctl_fresh(const llb_spec *m, int b);
+static bool px_takes(const llb_spec *m, int n_rows) {
+  return n_rows > SPEC_MAXT && !m->rows_set && m->ne == 0 && m->tp.size <= 1 && m->KC <= CONV_RING / 2 && m->d <= 16384;
+}
+// The dense part of the prompts of streams bs[i] (take[i] rows of ids[i] from position 0 on; 0: none), mode 1 a stream after the other in
+// chunks of PF_RMAX rows, mode 0 in pieces of PF_R rows, several streams' together as far as they fit.  Mode 1: a stream's drafter row at the
+// position it stops at is left pending as a one-row catch-up whose hidden (the normed row of the position before) is where the catch-up reads
+// it.  Mode 0 takes whole prompts, and leaves what the last T-row pass over them would have: its k + 1 normed rows, from which the
+// drafter catches up, and the next cycle's rows (px_logits: and its logits).
+static int pf_prefill(llb_spec *m, int nb, const int *bs, const int *const *ids, const int *take, bool fast) {
   CK(pf_alloc(m));
-  PfState &f = m->pf;
-  CU_OK(cudaMemsetAsync(f.hn, 0, (size_t)m->d * 4, g_llb.stream));   // the hidden before position 0 is zero (host/llb_host.c:1816)
-  int p = 0;
+  PfState &f = pf_owner(m)->pf;
+  std::lock_guard<std::mutex> hold(f.busy);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (pf_prof_on()) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, g_llb.stream); }
-  while (n_rows - p > keep) {
-    const int R = n_rows - p - keep < PF_RMAX ? n_rows - p - keep : PF_RMAX;
-    CK(pf_chunk(m, b, ids, p, R));
-    p += R;
+  std::vector<int> p(nb, 0);
+  int total = 0;
+  for (;;) {
+    std::vector<PfPiece> pc;
+    int room = fast ? PF_RMAX : PF_R;
+    for (int i = 0; i < nb && (int)pc.size() < (fast ? 1 : PF_PIECES); i++) {
+      // (a whole prompt's last piece has all the rows that are left behind for its drafter)
+      const int left = take[i] - p[i], most = fast ? PF_RMAX : left > PF_R && left < PF_R + SPEC_MAXT ? PF_R - SPEC_MAXT : PF_R, R = left < most ? left : most;
+      if (R < 1 || R > room) continue;
+      pc.push_back(PfPiece{bs[i], ids[i], p[i], R, !fast && R == left, 0});
+      p[i] += R; room -= R; total += R;
+    }
+    if (pc.empty()) break;
+    CK(pf_chunk(m, pc));
   }
+  if (fast) m->pf_rows += total;
   if (e0) {
     float ms = 0;
     cudaEventRecord(e1, g_llb.stream); cudaEventSynchronize(e1); cudaEventElapsedTime(&ms, e0, e1);
-    pf_prof_report(p, ms);
+    pf_prof_report(total, ms);
     cudaEventDestroy(e0); cudaEventDestroy(e1);
   }
-  if (p > 0) {
-    // the stream's first row of the trunk's normed hidden rows: what the pending catch-up row pairs with
-    CU_OK(cudaMemcpyAsync(m->hn_pf + (size_t)(m->B > 1 ? b * m->Tpf : 0) * m->d, f.hn, (size_t)m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
-    struct { int n, pos0, tok[SPEC_MAXT], slot[SPEC_MAXT]; } c;
-    memset(&c, 0, sizeof c);
-    c.n = m->has_mtp ? 1 : 0; c.pos0 = p; c.tok[0] = ids[p];
-    CU_OK(cudaMemcpyAsync(&ctl_of(m, b)->catchup, &c, sizeof c, cudaMemcpyHostToDevice, g_llb.stream));
-    CU_OK(cudaStreamSynchronize(g_llb.stream));
+  for (int i = 0; i < nb; i++) {
+    if (take[i] < 1) continue;
+    const int n = take[i];         // the position the stream is at
+    if (fast) {
+      struct { int n, pos0, tok[SPEC_MAXT], slot[SPEC_MAXT]; } c;
+      memset(&c, 0, sizeof c);
+      c.n = m->has_mtp ? 1 : 0; c.pos0 = n; c.tok[0] = ids[i][n];
+      CU_OK(cudaMemcpyAsync(&ctl_of(m, bs[i])->catchup, &c, sizeof c, cudaMemcpyHostToDevice, g_llb.stream));
+      CU_OK(cudaStreamSynchronize(g_llb.stream));
+      continue;
+    }
+    // as k_accept leaves the block behind a chunk's last rows
+    SpecCtl c = ctl_fresh(m, bs[i]);
+    c.catchup.n = n < m->Tspec ? n : m->Tspec; c.catchup.pos0 = n - c.catchup.n + 1;
+    for (int r = 0; r < c.catchup.n; r++) c.catchup.tok[r] = ids[i][c.catchup.pos0 + r];
+    c.verify.n = n + m->k + 1 > m->max_ctx ? (m->max_ctx - n > 0 ? m->max_ctx - n : 1) : m->k + 1;
+    c.verify.pos0 = n; c.verify.tok[0] = ids[i][n];
+    for (int r = 0; r < SPEC_MAXT; r++) c.verify.slot[r] = (n + r) & (CONV_RING - 1);
+    CK(ctl_write(m, bs[i], c));
+    if (m->lookup) CK(op_lookup_draft(g_llb.stream, ctl_of(m, bs[i])));
   }
-  *p_out = p;
   return 0;
+}
+// The logits of the prompt pass's rows, from the normed rows in hn_pf, where llb_spec_read_logits looks for those of the last pass
+static int px_logits(llb_spec *m) {
+  const int width = m->Tmax;
+  set_width(m, m->B * m->Tpf);
+  StreamScope scope(m);
+  const int rc = ops_xp_from_f32(g_llb.stream, m->hn_pf, m->Tmax, 2, m->xp_d) || site_gemm(m, {{&m->head, &m->b_lg, nullptr, nullptr, 0}}, m->xp_d, 0);
+  set_width(m, width);
+  m->last_pass = 1;
+  return rc ? -1 : 0;
 }
 
 static int ctl_write(llb_spec *m, int b, const SpecCtl &c) {
@@ -1463,11 +1559,22 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
     for (int r = 0; r < SPEC_MAXT; r++) c.verify.slot[r] = r & (CONV_RING - 1);
     CK(ctl_write(m, b, c));
   }
-  // LLB_PREFILL=fast: everything but the last k + 1 rows in chunks of PF_RMAX rows through the dense path (dense FFN only),
-  // one stream after the other (a chunk fills the tensor cores by itself)
-  for (int i = 0; i < nb; i++)
-    if (m->prefill_mode == 1 && m->ne == 0 && m->tp.size <= 1 && ns[i] - 1 >= m->Tspec + 32) CK(pf_prefill(m, bs[i], ids[i], ns[i] - 1, m->Tspec, &p[i]));
-  for (int i = 0; i < nb; i++) if (nb > 1 && p[i] >= ns[i] - 1) CK(park(bs[i]));   // a one-token prompt: nothing to run
+  // the dense path's rows: LLB_PREFILL=fast (dense FFN only) everything but the last k + 1, else as px_takes says; without room for its buffers
+  // mode 0 goes on in T-row passes
+  bool any_exact = false;
+  {
+    std::vector<int> fast(nb, 0), exact(nb, 0);
+    bool any_fast = false;
+    for (int i = 0; i < nb; i++) {
+      if (m->prefill_mode == 1 && m->ne == 0 && m->tp.size <= 1 && ns[i] - 1 >= m->Tspec + 32) { fast[i] = ns[i] - 1 - m->Tspec; any_fast = true; }
+      else if (px_takes(m, ns[i] - 1)) { exact[i] = ns[i] - 1; any_exact = true; }
+    }
+    if (any_fast) CK(pf_prefill(m, nb, bs, ids, fast.data(), true));
+    if (any_exact && pf_alloc(m)) { cudaGetLastError(); any_exact = false; }
+    if (any_exact) CK(pf_prefill(m, nb, bs, ids, exact.data(), false));
+    for (int i = 0; i < nb; i++) p[i] = fast[i] + (any_exact ? exact[i] : 0);
+  }
+  for (int i = 0; i < nb; i++) if (nb > 1 && p[i] >= ns[i] - 1) CK(park(bs[i]));   // nothing left to run
   for (;;) {
     std::vector<int> rows_of(nb, 0);
     int live = 0;
@@ -1502,6 +1609,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
       if (p[i] >= ns[i] - 1 && live > 1) CK(park(bs[i]));   // through, while others still have rows to feed
     }
   }
+  if (any_exact) CK(px_logits(m));
   if (m->B > 1)   // the rows that the first speculative cycle's drafter catches up over, where that cycle (and read_state) looks for them
     for (int i = 0; i < nb; i++)
       CU_OK(cudaMemcpyAsync(m->hn + (size_t)bs[i] * m->Tspec * m->d, m->hn_pf + (size_t)bs[i] * m->Tpf * m->d, (size_t)m->Tspec * m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
@@ -1516,8 +1624,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
   return 0;
 }
 static int prefill_stream(llb_spec *m, int b, const int *ids, int n) { return prefill_many(m, 1, &b, &ids, &n); }
-// Feed the prompt.  Positions 0 .. n-2 run through the verify pass in chunks of given rows (or, for long prompts with
-// LLB_PREFILL=fast, through the dense path); the last prompt token becomes the first speculative cycle's committed
+// Feed the prompt.  Positions 0 .. n-2 run through the dense path or, a few of them, through the verify pass in chunks of given rows; the last prompt token becomes the first speculative cycle's committed
 // input, exactly where the reference's first cycle after a prompt starts (host/llb_host.c:1911, pos = n-1).
 LLB_API int llb_spec_prefill(llb_spec *m, const int *ids, int n) { return prefill_stream(m, 0, ids, n); }
 // The same for stream b of an engine opened with llb_spec_open_streams; the other streams keep their state.
@@ -1870,7 +1977,7 @@ LLB_API int llb_spec_read_state_stream(llb_spec *m, int stream, int what, int il
     return (int)have;
   }
   else if (what == 4 && pos < (m->B > 1 ? m->Tspec : SPEC_MAXT)) { have = m->d; src = m->hn + (size_t)((m->B > 1 ? b * m->Tspec : 0) + pos) * m->d; }
-  else if (what == 6 && m->pf.ready && pos >= 0 && pos < PF_RMAX) { have = m->d; src = m->pf.hn + (size_t)(pos + 1) * m->d; }   // dense path: normed hidden of row `pos` of its last chunk
+  else if (what == 6 && pf_owner(m)->pf.ready && pos >= 0 && pos < PF_RMAX) { have = m->d; src = pf_owner(m)->pf.hn + (size_t)(pos + 1) * m->d; }   // dense path: normed hidden of row `pos` of its last chunk
   else return llb_fail("read_state: nothing of kind %d in layer %d", what, il);
   if (n < have) return llb_fail("read_state: buffer of %zu floats, %zu needed", n, have);
   CU_OK(cudaMemcpy(out, src, have * 4, cudaMemcpyDeviceToHost));

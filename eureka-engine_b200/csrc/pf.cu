@@ -4,7 +4,7 @@
 // spec_take): the trunk's K/V rows, conv history and DeltaNet state after the chunk, the drafter's K/V rows for the
 // chunk's positions (k and v only: no drafter attention, FFN or head), and the normed hidden row it continues from.
 // The arithmetic follows the CPU engine (tools/qwen35_engine.c:510-761) like the T-row kernels of ops_model.cu; what
-// differs is the GEMM operand precision (fp16, see pfmm.cuh) and that a DeltaNet layer scans the chunk's rows in one
+// differs is the order of the GEMMs' sums (pfx.cuh, pfmm.cuh) and that a DeltaNet layer scans the chunk's rows in one
 // kernel with the state in registers, writing the state once.
 #include "pfmm.cuh"
 #include "pfx.cuh"
@@ -17,19 +17,18 @@ template <int FMT> static int pf_attr() {
   CU_OK(cudaFuncSetAttribute(k_pfmm<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
   return 0;
 }
+// (their warpgroups trade registers: a launch with fewer than they were counted with would wait for ever)
+template <typename K> static int px_attr(K k, int smem, int regs) {
+  CU_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cudaFuncAttributes at;
+  CU_OK(cudaFuncGetAttributes(&at, k));
+  if (at.numRegs != regs) return llb_fail("pfx: built with %d registers a thread, its register split needs %d", at.numRegs, regs);
+  return 0;
+}
 template <int FMT> static int px_attr1() {
-  CU_OK(cudaFuncSetAttribute(k_pfx1<FMT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, px_smem(FMT, 32)));
-  CU_OK(cudaFuncSetAttribute(k_pfx1<FMT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, px_smem(FMT, 64)));
-  CU_OK(cudaFuncSetAttribute(k_pfx1<FMT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, px_smem(FMT, 128)));
-  return 0;
+  return px_attr(k_pfx1<FMT, 32>, px_smem(FMT, 32), PX1_REG_LAUNCH) || px_attr(k_pfx1<FMT, 64>, px_smem(FMT, 64), PX1_REG_LAUNCH) || px_attr(k_pfx1<FMT, 128>, px_smem(FMT, 128), PX1_REG_LAUNCH);
 }
-template <int FMT> static int px_attr2() {
-  CU_OK(cudaFuncSetAttribute(k_pfx2<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, px2_smem(FMT)));
-  cudaFuncAttributes at;   // its warpgroups trade registers: a launch with fewer than they were counted with would wait for ever
-  CU_OK(cudaFuncGetAttributes(&at, k_pfx2<FMT>));
-  if (at.numRegs != PX_REG_LAUNCH) return llb_fail("k_pfx2: built with %d registers a thread, its register split needs %d", at.numRegs, PX_REG_LAUNCH);
-  return 0;
-}
+template <int FMT> static int px_attr2() { return px_attr(k_pfx2<FMT>, px2_smem(FMT), PX_REG_LAUNCH); }
 #define PF_SCAN_NW 4                            // warps of a scan block, 8 state rows each
 #define PF_SCAN_BLOCKS (128 / (8 * PF_SCAN_NW)) // blocks of a head
 #define PF_SCAN_SMEM (220 * 1024)
@@ -81,7 +80,7 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a) {
   const int grid = 2 * (units < g_llb.sms / 2 ? units : g_llb.sms / 2);
   cudaError_t e = cudaErrorInvalidValue;
   const int ru = pf_unit_rows(a.R);
-#define PX_GO(F, RU) e = llb_launch(k_pfx1<F, RU>, dim3(grid), dim3(PX_THREADS), (size_t)px_smem(F, RU), s, a)
+#define PX_GO(F, RU) e = llb_launch(k_pfx1<F, RU>, dim3(grid), dim3(PX1_THREADS), (size_t)px_smem(F, RU), s, a)
 #define PX_ONE(F) do { if (ru == 32) PX_GO(F, 32); else if (ru == 64) PX_GO(F, 64); else PX_GO(F, 128); } while (0)
 #define PX_TWO(F) e = llb_launch(k_pfx2<F>, dim3(grid), dim3(PX_THREADS), (size_t)px2_smem(F), s, a)
   switch (fmt) {
@@ -139,7 +138,7 @@ int op_pf_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const int *ids
 #define PF_NORM_MAXT 1024
 template <int NI>
 __global__ void __launch_bounds__(PF_NORM_MAXT) k_pf_norm(const float *__restrict__ xin, PartIn add, const float *__restrict__ w, float eps, int d,
-                                                          float *__restrict__ xout, __half *__restrict__ kg, int kg_K, int kg_col0, int ru, float *__restrict__ hn_out) {
+                                                          float *__restrict__ xout, __half *__restrict__ kg, int kg_K, int kg_col0, int ru, int row0, float *__restrict__ hn_out) {
   float4 wv[NI];
 #pragma unroll
   for (int i = 0; i < NI; i++) {
@@ -175,14 +174,14 @@ __global__ void __launch_bounds__(PF_NORM_MAXT) k_pf_norm(const float *__restric
     if (c >= d) continue;   // whole warps: d is a multiple of 128
     const float h0 = v[i].x * sc * wv[i].x, h1 = v[i].y * sc * wv[i].y, h2 = v[i].z * sc * wv[i].z, h3 = v[i].w * sc * wv[i].w;
     if (hn_out) *(float4 *)(hn_out + row + c) = make_float4(h0, h1, h2, h3);
-    if (kg) pf_kg_store4(kg, kg_K, ru, t, kg_col0 + c, h0, h1, h2, h3);
+    if (kg) pf_kg_store4(kg, kg_K, ru, row0 + t, kg_col0 + c, h0, h1, h2, h3);
   }
 }
-int op_pf_norm(cudaStream_t s, const float *xin, PartIn add, const float *w, float eps, int d, float *xout, __half *kg, int kg_K, int kg_col0, float *hn_out, int R) {
+int op_pf_norm(cudaStream_t s, const float *xin, PartIn add, const float *w, float eps, int d, float *xout, __half *kg, int kg_K, int kg_col0, float *hn_out, int R, int ru, int row0) {
   if (d % 128 || kg_col0 % 128 || d > 4 * 4 * PF_NORM_MAXT) return llb_fail("pf norm: d %d at column %d", d, kg_col0);
   const int d4 = d / 4, ni = (d4 + PF_NORM_MAXT - 1) / PF_NORM_MAXT;
   const int threads = (((d4 + ni - 1) / ni) + 31) & ~31;
-#define PF_NORM_GO(NI) CU_OK(llb_launch(k_pf_norm<NI>, dim3(R), dim3(threads), (size_t)0, s, xin, add, w, eps, d, xout, kg, kg_K, kg_col0, pf_unit_rows(R), hn_out))
+#define PF_NORM_GO(NI) CU_OK(llb_launch(k_pf_norm<NI>, dim3(R), dim3(threads), (size_t)0, s, xin, add, w, eps, d, xout, kg, kg_K, kg_col0, ru, row0, hn_out))
   switch (ni) {
     case 1: PF_NORM_GO(1); break;
     case 2: PF_NORM_GO(2); break;
@@ -203,8 +202,8 @@ __global__ void __launch_bounds__(256) k_pf_silu(PartIn g, PartIn u, int f, int 
   const float4 gv = part_get4(g, i), uv = part_get4(u, i);
   pf_kg_store4(kg, f, ru, t, c, pf_silu(gv.x) * uv.x, pf_silu(gv.y) * uv.y, pf_silu(gv.z) * uv.z, pf_silu(gv.w) * uv.w);
 }
-int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R) {
-  CU_OK(llb_launch(k_pf_silu, dim3((f / 4 + 255) / 256, R), dim3(256), (size_t)0, s, g, u, f, pf_unit_rows(R), kg));
+int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R, int ru) {
+  CU_OK(llb_launch(k_pf_silu, dim3((f / 4 + 255) / 256, R), dim3(256), (size_t)0, s, g, u, f, ru, kg));
   return 0;
 }
 
@@ -506,7 +505,7 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__
 // block a head copies the chunk's last raw rows into the conv history: whole values into K-slice 0, zeros into the rest
 // (here, because the conv kernel's first rows still read the old history).
 __global__ void __launch_bounds__(256) k_pf_gnorm(const float *__restrict__ o, PartIn z, const float *__restrict__ nw, DeltaShape sh, __half *__restrict__ kg,
-                                                  PartIn qkv, float *__restrict__ ring, int ring_ks, int p0, int R) {
+                                                  PartIn qkv, float *__restrict__ ring, int ring_ks, int p0, int R, int row0, int ru) {
   const int hh = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5), i = threadIdx.x & 31;
   const float4 w = __ldg((const float4 *)(nw + 4 * i));
   pdl_trigger();
@@ -525,12 +524,12 @@ __global__ void __launch_bounds__(256) k_pf_gnorm(const float *__restrict__ o, P
   const size_t idx = (size_t)t * sh.vdc + hh * 128 + 4 * i;
   const float4 v = __ldcg((const float4 *)(o + idx)), zz = part_get4(z, idx);
   const float r = 1.0f / sqrtf(pf_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) / 128.0f + sh.eps);
-  pf_kg_store4(kg, sh.vdc, pf_unit_rows(R), t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
+  pf_kg_store4(kg, sh.vdc, ru, row0 + t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
 }
 
 // One DeltaNet layer's ops between its input GEMM (qkv | z | beta | alpha) and its output GEMM, for R rows at p0 ...
 int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, float *ring, int ring_ks, const float *cw, const float *dt, const float *sa,
-                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int p0, int R) {
+                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int p0, int R, int row0, int ru) {
   if (sh.SZ != 128 || sh.KC > CONV_RING / 2) return llb_fail("pf delta: state size %d, conv kernel %d", sh.SZ, sh.KC);
   const long long rstride = (long long)CONV_RING * sh.convd;
   const dim3 cgrid((sh.GK + 1) / 2 + (sh.TR + 3) / 4 + (PF_CH * sh.TR + 127) / 128, (R + PF_CH - 1) / PF_CH);
@@ -542,7 +541,7 @@ int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, floa
   const int blocks = sh.TR * PF_SCAN_BLOCKS, per = (blocks + g_llb.sms - 1) / g_llb.sms;
   const size_t pad = per < 6 ? (size_t)(PF_SCAN_SMEM / per - 24 * 1024) : 0;
   CU_OK(llb_launch(k_pf_scan, dim3(sh.TR, PF_SCAN_BLOCKS), dim3(32 * PF_SCAN_NW), pad, s, S, ctl, (const float *)y, (const float *)gram, (const float *)beta, (const float *)decay, sh, o, R));
-  CU_OK(llb_launch(k_pf_gnorm, dim3(sh.TR, (R + 7) / 8 + 1), dim3(256), (size_t)0, s, (const float *)o, z, nw, sh, kg, qkv, ring, ring_ks, p0, R));
+  CU_OK(llb_launch(k_pf_gnorm, dim3(sh.TR, (R + 7) / 8 + 1), dim3(256), (size_t)0, s, (const float *)o, z, nw, sh, kg, qkv, ring, ring_ks, p0, R, row0, ru));
   return 0;
 }
 

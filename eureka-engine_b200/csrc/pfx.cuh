@@ -30,7 +30,7 @@
 #include "pfmm.cuh"
 #include "gemm2.cuh"
 
-#define PX_THREADS 512      // warps 0-3 unpack, 4 loads weights, 5 activations, 6 issues MMAs, 7 forwards, 8-15 read accumulators
+#define PX_THREADS 512      // k_pfx2: warps 0-3 unpack, 4 loads weights, 5 activations, 6 issues MMAs, 7 forwards, 8-15 read accumulators
 #define PX_HDR 1024
 #define PX_SC (4 * 128 * 4)                    // scales of the last four super-blocks, a word a weight row
 #define PX_OA (2 * 128 * 16)                   // the offsets' step: weight rows' side
@@ -40,19 +40,24 @@ __host__ __device__ constexpr bool px_offs(int fmt) { return px_planes(fmt) == 1
 __host__ __device__ constexpr int px_a_bytes(int fmt) { return px_planes(fmt) * PF_A_BYTES; }
 __host__ __device__ constexpr int px_b_bytes(int RU) { return RU * PF_KS * 2; }          // one plane of a stage's activations
 __host__ __device__ constexpr int px_ob_bytes(int RU) { return RU * 32; }                // ... and of the offsets' step
-// k_pfx1's stages of 64 columns.  At most four: the offsets' step has one buffer, which a super-block's last stage fills and the same
-// stage of the next fills again, when the MMAs of the stage `px_stages` before that one are done.
-__host__ __device__ constexpr int px_stages(int fmt) { return px_planes(fmt) == 2 ? 3 : 4; }
-// super-blocks a weight copy brings (gemm2.cuh: a copy costs the SM's copy engine about 85 cycles), and the ring's depth
+// k_pfx1's rings: codes in stages of 64 columns (at most four: the offsets' step has one buffer on the weight rows' side, which a super-block's last
+// stage fills and the same stage of the next fills again, when the MMAs of the stage `px_na` before that one are done); activations in
+// slots of 16 KB and, where there is such a step, the means of a super-block behind them; weights in chunks of whole super-blocks (a copy costs
+// the SM's copy engine about 85 cycles, gemm2.cuh).
+#define PX_SLOT 16384
+__host__ __device__ constexpr int px_na(int fmt) { return px_planes(fmt) == 2 ? 3 : 4; }
+__host__ __device__ constexpr int px_slot_stages(int RU) { return PX_SLOT / px_b_bytes(RU); }
+__host__ __device__ constexpr int px_slot_bytes(int fmt, int RU) { return PX_SLOT + (px_offs(fmt) ? px_ob_bytes(RU) : 0); }
+__host__ __device__ constexpr int px_nb(int fmt) { return fmt == LLB_FM_Q8_0 ? 3 : 4; }
 __host__ __device__ constexpr int px_chunk(int fmt) { return fmt == LLB_FM_Q4_K ? 2 : 1; }
 __host__ __device__ constexpr int px_raw_bytes(int fmt) { return 8 * px_chunk(fmt) * tile_bytes(fmt); }
-__host__ __device__ constexpr int px_fixed(int fmt, int RU) { return PX_HDR + PX_SC + PX_OA + px_ob_bytes(RU) + px_stages(fmt) * (px_a_bytes(fmt) + px_b_bytes(RU)); }
+__host__ __device__ constexpr int px_fixed(int fmt, int RU) { return PX_HDR + PX_SC + (px_offs(fmt) ? PX_OA : 0) + px_na(fmt) * px_a_bytes(fmt) + px_nb(fmt) * px_slot_bytes(fmt, RU); }
 __host__ __device__ constexpr int px_raws(int fmt, int RU) {
   const int n = (PX_SMEM_MAX - px_fixed(fmt, RU)) / px_raw_bytes(fmt);
-  return n > 8 ? 8 : n;
+  return n > 4 ? 4 : n;
 }
 __host__ __device__ constexpr int px_smem(int fmt, int RU) { return px_fixed(fmt, RU) + px_raws(fmt, RU) * px_raw_bytes(fmt); }
-static_assert(px_stages(LLB_FM_Q4_K) <= 4, "one buffer of the offsets' step");
+static_assert(px_na(LLB_FM_Q4_K) <= 4, "one buffer of the offsets' step");
 // Stages after which k_pfx1's accumulators are read: the tensor core truncates where it adds to one, so that a sum loses about 2e-8 of itself an
 // MMA.  Its prompts take the place of verify rows, so it is read as often as that hides behind the MMAs.
 __host__ __device__ constexpr int px_drain(int fmt) { return px_planes(fmt) == 2 ? 1 : 2; }
@@ -71,13 +76,20 @@ static_assert(px2_smem(LLB_FM_Q5_K) <= PX_SMEM_MAX, "k_pfx2's rings");
 #define PX_REG_READ 192
 #define PX_REG_LAUNCH 128
 static_assert(PX_REG_UNPACK + PX_REG_ISSUE + 2 * PX_REG_READ == 4 * PX_REG_LAUNCH, "setmaxnreg.inc waits for ever where the shares are more than the launch's registers");
+// k_pfx1: warps 0-7 unpack, 8 loads weights, 9 activations, 10 issues MMAs, 11 forwards, 12-19 read accumulators
+#define PX1_THREADS 640
+#define PX1_REG_UNPACK 80
+#define PX1_REG_ISSUE 64
+#define PX1_REG_READ 128
+#define PX1_REG_LAUNCH 96
+static_assert(2 * PX1_REG_UNPACK + PX1_REG_ISSUE + 2 * PX1_REG_READ == 5 * PX1_REG_LAUNCH, "as above");
 __host__ __device__ constexpr uint32_t px_idesc(int N) { return 0x10000010u | ((uint32_t)(N >> 3) << 17); }   // kind::f16: D f32, A / B f16 K-major, M = 256 over the pair
 
 // ---- one 64-column stage s of a weight row's super-block into core-matrix rows of the code planes ----
 // What a super-block's row needs besides its codes.
 struct PxRow { uint32_t w[4]; uint32_t kap; };
 // Reads the row's header; scale = what the accumulators of the super-block are multiplied with; off: the offsets' step of the row
-template <int FMT> __device__ __forceinline__ void px_head(const uint8_t *row, const uint8_t *tile, int r16, PxRow &h, float &scale, uint4 (&off)[2]) {
+template <int FMT> __device__ __forceinline__ void px_head(const uint8_t *row, const uint8_t *tile, int r16, bool with_off, PxRow &h, float &scale, uint4 (&off)[2]) {
   if constexpr (px_offs(FMT)) {
     const uint4 hd = *(const uint4 *)row;
     k4_scales(hd.y, hd.z, hd.w, h.w[0], h.w[1], h.w[2], h.w[3]);
@@ -96,6 +108,7 @@ template <int FMT> __device__ __forceinline__ void px_head(const uint8_t *row, c
     const __half2 k2 = __floats2half2_rn(kap, kap);
     h.kap = *(const uint32_t *)&k2;
     scale = d * 16384.0f;
+    if (!with_off) return;
     constexpr float C = FMT == LLB_FM_Q4_K ? 8.0f : 16.0f;
     uint32_t hi[4], lo[4];
 #pragma unroll
@@ -133,7 +146,8 @@ template <int FMT> __device__ __forceinline__ void px_head(const uint8_t *row, c
 // k-group g of the stage, plane p: o[8 p + g].  (s is not unrolled over: with the super-block's four stages, and the eight of the MMAs, as
 // straight-line code the kernel's roles threw each other out of the instruction cache; gate|up of the 27B shape 182 us.)
 __device__ __forceinline__ uint32_t px_pick(const uint32_t (&w)[4], int s) { return s & 2 ? (s & 1 ? w[3] : w[2]) : (s & 1 ? w[1] : w[0]); }
-template <int FMT> __device__ __forceinline__ void px_stage(const uint8_t *row, int s, const PxRow &h, uint4 (&o)[8 * px_planes(FMT)]) {
+// P = 2: a thread has half of the stage's columns, part `part`: columns 16 part .. of both groups of 32 (Q8_0: 32 part ..)
+template <int FMT, int P = 1> __device__ __forceinline__ void px_stage(const uint8_t *row, int s, int part, const PxRow &h, uint4 (&o)[8 * px_planes(FMT) / P]) {
   if constexpr (px_offs(FMT)) {
     constexpr int QOFF = FMT == LLB_FM_Q4_K ? 16 : 48;
     const uint32_t sw = s < 2 ? h.w[0] : h.w[1];
@@ -145,7 +159,8 @@ template <int FMT> __device__ __forceinline__ void px_stage(const uint8_t *row, 
     constexpr uint32_t CL = FMT == LLB_FM_Q4_K ? 0x80088008u : 0x80108010u, CH = FMT == LLB_FM_Q4_K ? 0x80808080u : 0x81008100u;
     const uint32_t L8 = g2_hmul2(L, CL), H8 = g2_hmul2(H, CH);
 #pragma unroll
-    for (int g2 = 0; g2 < 2; g2++) {
+    for (int i2 = 0; i2 < 2 / P; i2++) {
+      const int g2 = P == 2 ? part : i2;
       const uint4 q = *(const uint4 *)(row + QOFF + 32 * s + 16 * g2);
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
       uint32_t z[4] = {0, 0, 0, 0};
@@ -163,14 +178,15 @@ template <int FMT> __device__ __forceinline__ void px_stage(const uint8_t *row, 
         lo[2 * i] = g2_hfma2(a0, L, L8); lo[2 * i + 1] = g2_hfma2(a1, L, L8);
         hi[2 * i] = g2_hfma2(b0, H, H8); hi[2 * i + 1] = g2_hfma2(b1, H, H8);
       }
-      o[2 * g2] = make_uint4(lo[0], lo[1], lo[2], lo[3]); o[2 * g2 + 1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
-      o[4 + 2 * g2] = make_uint4(hi[0], hi[1], hi[2], hi[3]); o[5 + 2 * g2] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+      o[2 * i2] = make_uint4(lo[0], lo[1], lo[2], lo[3]); o[2 * i2 + 1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+      o[4 / P + 2 * i2] = make_uint4(hi[0], hi[1], hi[2], hi[3]); o[4 / P + 2 * i2 + 1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
     }
   } else if constexpr (FMT == LLB_FM_Q6_K) {
     const int hf = s >> 1, odd = s & 1;
     const uint32_t scw = px_pick(h.w, s), nm = odd ? 0x00f000f0u : 0x000f000fu;
 #pragma unroll
-    for (int c = 0; c < 2; c++) {              // sixteen columns 16 c .. of both quarters
+    for (int i2 = 0; i2 < 2 / P; i2++) {       // sixteen columns 16 c .. of both quarters
+      const int c = P == 2 ? part : i2;
       const uint4 hq4 = *(const uint4 *)(row + 128 + 32 * hf + 16 * c);
       const uint32_t hw[4] = {hq4.x, hq4.y, hq4.z, hq4.w};
 #pragma unroll
@@ -189,16 +205,17 @@ template <int FMT> __device__ __forceinline__ void px_stage(const uint8_t *row, 
           P2[2 * i] = g2_hfma2(lw[i] & nm, S, S8); P2[2 * i + 1] = g2_hfma2((lw[i] >> 8) & nm, S, S8);
           P1[2 * i] = g2_hfma2(e & hm, M, M24); P1[2 * i + 1] = g2_hfma2(f & hm, M, M24);
         }
-        const int g = 4 * qq + 2 * c;
+        const int g = 4 / P * qq + 2 * i2;
         o[g] = make_uint4(P1[0], P1[1], P1[2], P1[3]); o[g + 1] = make_uint4(P1[4], P1[5], P1[6], P1[7]);
-        o[8 + g] = make_uint4(P2[0], P2[1], P2[2], P2[3]); o[8 + g + 1] = make_uint4(P2[4], P2[5], P2[6], P2[7]);
+        o[8 / P + g] = make_uint4(P2[0], P2[1], P2[2], P2[3]); o[8 / P + g + 1] = make_uint4(P2[4], P2[5], P2[6], P2[7]);
       }
     }
   } else {
     const uint32_t dw = px_pick(h.w, s);
 #pragma unroll
-    for (int c = 0; c < 4; c++) {              // sixteen columns of block 2 s + c / 2
-      const uint32_t dn = __byte_perm(dw, 0, c < 2 ? 0x1010 : 0x3232);
+    for (int i2 = 0; i2 < 4 / P; i2++) {       // sixteen columns of block 2 s + c / 2
+      const int c = P == 2 ? 2 * part + i2 : i2;
+      const uint32_t dn = __byte_perm(dw, 0, c < 2 ? 0x1010u : 0x3232u);
       const uint4 q = *(const uint4 *)(row + 64 * s + 16 * c);
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
       uint32_t P1[8], P2[8];
@@ -209,8 +226,8 @@ template <int FMT> __device__ __forceinline__ void px_stage(const uint8_t *row, 
           const uint32_t x = g2_hadd2(__byte_perm(w[i], 0x64646464u, e ? 0x4341 : 0x4240), 0xe480e480u), p = g2_hmul2(x, dn);
           P1[2 * i + e] = p; P2[2 * i + e] = g2_hfma2(x, dn, p ^ 0x80008000u);   // what the product's rounding left out
         }
-      o[2 * c] = make_uint4(P1[0], P1[1], P1[2], P1[3]); o[2 * c + 1] = make_uint4(P1[4], P1[5], P1[6], P1[7]);
-      o[8 + 2 * c] = make_uint4(P2[0], P2[1], P2[2], P2[3]); o[8 + 2 * c + 1] = make_uint4(P2[4], P2[5], P2[6], P2[7]);
+      o[2 * i2] = make_uint4(P1[0], P1[1], P1[2], P1[3]); o[2 * i2 + 1] = make_uint4(P1[4], P1[5], P1[6], P1[7]);
+      o[8 / P + 2 * i2] = make_uint4(P2[0], P2[1], P2[2], P2[3]); o[8 / P + 2 * i2 + 1] = make_uint4(P2[4], P2[5], P2[6], P2[7]);
     }
   }
 }
@@ -222,48 +239,55 @@ __device__ __forceinline__ void px_mma_scaled(uint32_t d_tmem, uint64_t adesc, u
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, 11;\n\t}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc)
       : "memory");
 }
+// the k-group of the stage that o[i] of a plane is (i < 8 / P)
+template <int FMT, int P> __device__ __forceinline__ int px_group(int i, int part) {
+  if (P == 1) return i;
+  if constexpr (FMT == LLB_FM_Q8_0) return 4 * part + i;
+  else return 4 * (i >> 1) + 2 * part + (i & 1);
+}
 template <int N> __device__ __forceinline__ void px_reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void px_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ---- the kernels: work units, tiles and slices as in pfmm.cuh.  Up to 128 prompt rows: ----
 template <int FMT, int RU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx1(const PfArgs a) {
-  constexpr int NST = px_stages(FMT), NPL = px_planes(FMT), N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), DG = px_drain(FMT);
-  constexpr int RAWB = px_raw_bytes(FMT), STB = px_a_bytes(FMT) + px_b_bytes(RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU);
-  static_assert(NRAW >= 1 && px_smem(FMT, RU) <= PX_SMEM_MAX, "a form that does not fit");
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pfx1(const PfArgs a) {
+  constexpr int NA = px_na(FMT), NB = px_nb(FMT), BS = px_slot_stages(RU), NPL = px_planes(FMT), N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), DG = px_drain(FMT);
+  constexpr int RAWB = px_raw_bytes(FMT), AB = px_a_bytes(FMT), SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU);
+  static_assert(NRAW >= 2 && px_smem(FMT, RU) <= PX_SMEM_MAX, "a form that does not fit");
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t bar_s = smem_u32(smem);
-  // The pair's first CTA (the leader) issues: its full counts both CTAs' unpacking warps, its own activations and the other CTA's (passed
-  // on from that one's full_b), its d_empty the reading warps of both; the MMAs' commits arrive in both CTAs.
-  const uint32_t lead = t5_map_rank(bar_s, 0);     // the leader's barriers, as both CTAs name them
-  auto full = [&](int s) { return bar_s + 8u * (uint32_t)s; };
-  auto empty = [&](int s) { return bar_s + 32u + 8u * (uint32_t)s; };
-  auto full_b = [&](int s) { return bar_s + 64u + 8u * (uint32_t)s; };
-  auto d_full = [&](int b) { return bar_s + 96u + 8u * (uint32_t)b; };
-  auto d_empty = [&](int b) { return bar_s + 128u + 8u * (uint32_t)b; };
-  auto sc_full = [&](int i) { return bar_s + 160u + 8u * (uint32_t)i; };
-  auto raw_full = [&](int i) { return bar_s + 192u + 8u * (uint32_t)i; };
+  const uint32_t lead = t5_map_rank(bar_s, 0);     // the leader's (the pair's first CTA's) barriers, as both CTAs name them
+  auto a_full = [&](int s) { return bar_s + 8u * (uint32_t)s; };               // leader: both CTAs' unpacking warps
+  auto a_empty = [&](int s) { return bar_s + 32u + 8u * (uint32_t)s; };
+  auto b_full = [&](int s) { return bar_s + 64u + 8u * (uint32_t)s; };         // leader: its own copy and the other CTA's, passed on from that one's b_here
+  auto b_empty = [&](int s) { return bar_s + 96u + 8u * (uint32_t)s; };
+  auto b_here = [&](int s) { return bar_s + 128u + 8u * (uint32_t)s; };
+  auto d_full = [&](int b) { return bar_s + 160u + 8u * (uint32_t)b; };
+  auto d_empty = [&](int b) { return bar_s + 176u + 8u * (uint32_t)b; };       // leader: the reading warps of both CTAs
+  auto sc_full = [&](int i) { return bar_s + 192u + 8u * (uint32_t)i; };
+  auto raw_full = [&](int i) { return bar_s + 224u + 8u * (uint32_t)i; };
   auto raw_empty = [&](int i) { return bar_s + 256u + 8u * (uint32_t)i; };
   uint32_t *tmem_slot = (uint32_t *)(smem + 320);
   volatile uint32_t *dead = (volatile uint32_t *)(smem + 324);
   float *scr = (float *)(smem + PX_HDR);
-  uint8_t *oa = smem + PX_HDR + PX_SC, *ob = oa + PX_OA, *ring = ob + px_ob_bytes(RU), *raw = ring + NST * STB;
-  const uint32_t oa_s = smem_u32(oa), ob_s = smem_u32(ob), ring_s = smem_u32(ring), raw_s = smem_u32(raw);
+  uint8_t *oa = smem + PX_HDR + PX_SC, *ra = oa + (px_offs(FMT) ? PX_OA : 0), *rb = ra + NA * AB, *raw = rb + NB * SLB;
+  const uint32_t oa_s = smem_u32(oa), ra_s = smem_u32(ra), rb_s = smem_u32(rb), raw_s = smem_u32(raw);
   const int ntiles = a.t128[a.nmat], npairs = (ntiles + 1) >> 1, nunits = npairs * a.ksplit;
   const int rank = blockIdx.x & 1, unit0 = blockIdx.x >> 1, ustep = gridDim.x >> 1;
   auto tile_of = [&](int u) { return 2 * (u % npairs) + rank; };
 
   pdl_trigger();
   if (tid == 0) {
-    for (int s = 0; s < NST; s++) { mbar_init(full(s), 10); mbar_init(empty(s), 1); mbar_init(full_b(s), 1); }
+    for (int s = 0; s < NA; s++) { mbar_init(a_full(s), 16); mbar_init(a_empty(s), 1); }
+    for (int s = 0; s < NB; s++) { mbar_init(b_full(s), 2); mbar_init(b_empty(s), 1); mbar_init(b_here(s), 1); }
     for (int b = 0; b < 2; b++) { mbar_init(d_full(b), 1); mbar_init(d_empty(b), 16); }
     for (int i = 0; i < 4; i++) mbar_init(sc_full(i), 4);
-    for (int i = 0; i < NRAW; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), 4); }
+    for (int i = 0; i < NRAW; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), 8); }
     *dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 6) {
+  if (warp == 10) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
@@ -278,9 +302,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
     }
   };
 
-  if (warp < 4) {
-    // ---- codes: a thread a weight row ----
-    const int r = tid, r16 = r & 15;
+  if (warp < 8) {
+    // ---- codes: two threads a weight row (with one the unpacking of a super-block took 3250 cycles and paced the kernel) ----
+    px_reg_dec<PX1_REG_UNPACK>();
+    const int r = tid & 127, part = tid >> 7, r16 = r & 15;
     const uint32_t roff = (uint32_t)(r >> 4) * (CH * TB);
     int slot = 0, rs = 0, jj = 0;
     uint32_t par = 1, rpar = 0;             // (the first round's waits on empty barriers pass)
@@ -295,25 +320,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
         PxRow h;
         float scale;
         uint4 off[2];
-        px_head<FMT>(row, tile, r16, h, scale, off);
+        px_head<FMT>(row, tile, r16, part == 0, h, scale, off);
 #pragma unroll 1
         for (int s = 0; s < 4; s++) {
-          uint4 o[8 * NPL];
-          px_stage<FMT>(row, s, h, o);
-          wait(empty(slot), par);
-          uint8_t *A = ring + slot * STB + r * 16;
+          uint4 o[4 * NPL];
+          px_stage<FMT, 2>(row, s, part, h, o);
+          wait(a_empty(slot), par);
+          uint8_t *A = ra + slot * AB + r * 16;
 #pragma unroll
-          for (int g = 0; g < 8 * NPL; g++) *(uint4 *)(A + (size_t)g * 2048) = o[g];
-          if (s == 0) {   // (the scales of the super-block four back have been read: its accumulators were, before the stages that were waited for here)
+          for (int i = 0; i < 4 * NPL; i++) *(uint4 *)(A + (i >> 2) * PF_A_BYTES + px_group<FMT, 2>(i & 3, part) * 2048) = o[i];
+          if (s == 0 && part == 0) {   // (the scales of the super-block four back have been read: its accumulators were, before the stages that were waited for here)
             scr[(jj & 3) * 128 + r] = scale;
             __syncwarp();
             if (lane == 0) mbar_arrive(sc_full(jj & 3));
           }
-          if (s == 3 && px_offs(FMT)) { *(uint4 *)(oa + r * 16) = off[0]; *(uint4 *)(oa + (128 + r) * 16) = off[1]; }
+          if (s == 3 && part == 0 && px_offs(FMT)) { *(uint4 *)(oa + r * 16) = off[0]; *(uint4 *)(oa + (128 + r) * 16) = off[1]; }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads these bytes through the async proxy
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(lead + (full(slot) - bar_s));
-          if (++slot == NST) { slot = 0; par ^= 1u; }
+          if (lane == 0) mbar_arrive_cluster(lead + (a_full(slot) - bar_s));
+          if (++slot == NA) { slot = 0; par ^= 1u; }
         }
         if (c % CH == CH - 1 || c == nsl - 1) {
           if (lane == 0) mbar_arrive(raw_empty(rs));
@@ -321,8 +346,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
         }
       }
     }
-  } else if (warp < 8) {
-    if (warp == 4) {
+  } else if (warp < 12) {
+    px_reg_dec<PX1_REG_ISSUE>();
+    if (warp == 8) {
       // ---- weights: lane t requests the t-th 16-row tile of every chunk of the CTA's 128 rows ----
       int rs = 0;
       uint32_t rpar = 1;
@@ -345,7 +371,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
           if (++rs == NRAW) { rs = 0; rpar ^= 1u; }
         }
       }
-    } else if (warp == 5) {
+    } else if (warp == 9) {
       // ---- activations: the CTA's plane ----
       if (lane == 0) {
         int slot = 0;
@@ -355,20 +381,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
         for (int u = unit0; u < nunits; u += ustep) {
           int kbase, nst;
           pf_slice(a, u, npairs, kbase, nst);
-          for (int s = 0; s < nst; s++) {
-            wait(empty(slot), par);
+#pragma unroll 1
+          for (int s = 0; s < nst; s += BS) {
+            wait(b_empty(slot), par);
             if (!*dead) {
-              const bool last = px_offs(FMT) && (s & 3) == 3;
-              const uint32_t bar = rank ? full_b(slot) : full(slot), dst = ring_s + slot * STB + px_a_bytes(FMT);
-              mbar_expect(bar, (uint32_t)(PLB + (last ? OPB : 0)));
-              pf_bulk_copy(dst, x + (size_t)(kbase + s * PF_KS) * RU, PLB, bar);
-              if (last) pf_bulk_copy(ob_s, xs + (size_t)((kbase >> 8) + (s >> 2)) * 16 * RU, OPB, bar);
+              const bool last = px_offs(FMT) && ((s + BS) & 3) == 0;
+              const uint32_t bar = rank ? b_here(slot) : b_full(slot), dst = rb_s + slot * SLB;
+              mbar_expect(bar, (uint32_t)(PX_SLOT + (last ? OPB : 0)));
+              pf_bulk_copy(dst, x + (size_t)(kbase + s * PF_KS) * RU, PX_SLOT, bar);
+              if (last) pf_bulk_copy(dst + PX_SLOT, xs + (size_t)((kbase >> 8) + (s >> 2)) * 16 * RU, OPB, bar);
             }
-            if (++slot == NST) { slot = 0; par ^= 1u; }
+            if (++slot == NB) { slot = 0; par ^= 1u; }
           }
         }
       }
-    } else if (warp == 7) {
+    } else if (warp == 11) {
       // ---- tells the leader that the other CTA's activations are there ----
       if (lane == 0 && rank == 1) {
         int slot = 0;
@@ -376,54 +403,56 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
         for (int u = unit0; u < nunits; u += ustep) {
           int kbase, nst;
           pf_slice(a, u, npairs, kbase, nst);
-          for (int s = 0; s < nst; s++) {
-            wait(full_b(slot), par);
-            mbar_arrive_cluster(lead + (full(slot) - bar_s));
-            if (++slot == NST) { slot = 0; par ^= 1u; }
+#pragma unroll 1
+          for (int s = 0; s < nst; s += BS) {
+            wait(b_here(slot), par);
+            mbar_arrive_cluster(lead + (b_full(slot) - bar_s));
+            if (++slot == NB) { slot = 0; par ^= 1u; }
           }
         }
       }
     } else if (rank == 0) {
       // ---- the tensor cores of the pair, from the leader: the warp walks, an elected lane issues (descriptors stay in uniform registers) ----
       const bool el = t5_elect();
-      const uint64_t oad = g3_desc(oa_s, 2048, 128), obd = g3_desc(ob_s, RU * 16, 128);
-      int slot = 0, dd = 0;   // (dd: accumulators handed over)
-      uint32_t par = 0;
+      const uint64_t oad = g3_desc(oa_s, 2048, 128);
+      int as = 0, bs = 0, dd = 0;   // (dd: accumulators handed over)
+      uint32_t apar = 0, bpar = 0;
       for (int u = unit0; u < nunits; u += ustep) {
         int kbase, nst;
         pf_slice(a, u, npairs, kbase, nst);
 #pragma unroll 1
-        for (int c = 0; c < nst >> 2; c++) {
-#pragma unroll 1
-          for (int s = 0; s < 4; s++) {
-            const uint32_t D = tmem + (uint32_t)((dd & 1) * 256), first = s % DG == 0;
-            if (first && dd > 1) wait(d_empty(dd & 1), (uint32_t)((dd >> 1) - 1) & 1u);
-            wait(full(slot), par);
-            t5_fence_after();
-            const uint32_t st = ring_s + slot * STB;
-            const uint64_t ad = g3_desc(st, 2048, 128), bd = g3_desc(st + px_a_bytes(FMT), RU * 16, 128);
-            if (el) {
-              // (two planes: the smaller one first, while there is little for the additions to truncate)
+        for (int s = 0; s < nst; s++) {
+          const uint32_t D = tmem + (uint32_t)((dd & 1) * 256), first = s % DG == 0;
+          const bool last = s % DG == DG - 1, out = s % BS == BS - 1;      // of an accumulator; of a slot of activations
+          if (first && dd > 1) wait(d_empty(dd & 1), (uint32_t)((dd >> 1) - 1) & 1u);
+          if (s % BS == 0) wait(b_full(bs), bpar);
+          wait(a_full(as), apar);
+          t5_fence_after();
+          const uint64_t ad = g3_desc(ra_s + as * AB, 2048, 128), bd = g3_desc(rb_s + bs * SLB + s % BS * PLB, RU * 16, 128);
+          if (el) {
+            // (two planes: the smaller one first, while there is little for the additions to truncate)
 #pragma unroll
-              for (int pl = NPL - 1; pl >= 0; pl--)
+            for (int pl = NPL - 1; pl >= 0; pl--)
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                  pf_mma_ss(D, ad + (uint64_t)(pl * (PF_A_BYTES / 16) + k * 256), bd + (uint64_t)(k * 2 * RU), px_idesc(N), k != 0 || pl != NPL - 1 ? 1u : !first);
-              if (s == 3 && px_offs(FMT)) pf_mma_ss(D, oad, obd, px_idesc(N), 1u);
-              t5_commit_pair(empty(slot));
-              if (s % DG == DG - 1) t5_commit_pair(d_full(dd & 1));
-            }
-            __syncwarp();
-            if (s % DG == DG - 1) dd++;
-            if (++slot == NST) { slot = 0; par ^= 1u; }
+              for (int k = 0; k < 4; k++)
+                pf_mma_ss(D, ad + (uint64_t)(pl * (PF_A_BYTES / 16) + k * 256), bd + (uint64_t)(k * 2 * RU), px_idesc(N), k != 0 || pl != NPL - 1 ? 1u : !first);
+            if (px_offs(FMT) && (s & 3) == 3) pf_mma_ss(D, oad, g3_desc(rb_s + bs * SLB + PX_SLOT, RU * 16, 128), px_idesc(N), 1u);
+            t5_commit_pair(a_empty(as));
+            if (out) t5_commit_pair(b_empty(bs));
+            if (last) t5_commit_pair(d_full(dd & 1));
           }
+          __syncwarp();
+          if (last) dd++;
+          if (++as == NA) { as = 0; apar ^= 1u; }
+          if (out && ++bs == NB) { bs = 0; bpar ^= 1u; }
         }
       }
     }
   } else {
     // ---- accumulators into sums: lane quarter q, a weight row a thread; the two warps of a quarter have half of the prompt rows each ----
+    px_reg_inc<PX1_REG_READ>();
     constexpr int RH = RU / 2;
-    const int q = warp & 3, half = (warp - 8) >> 2, R = a.R;
+    const int q = warp & 3, half = (warp - 12) >> 2, R = a.R;
     const uint32_t t0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * RH);
     f32x2 acc[RH / 2];
     const f32x2 inv = x2_pack(XP_LO_INV, XP_LO_INV);
@@ -482,7 +511,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
   __syncwarp();
   t5_fence_before();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // no CTA leaves while the other still arrives here or reads its memory
-  if (warp == 6) {
+  if (warp == 10) {
     t5_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
@@ -558,11 +587,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX_THREADS, 1) k_pfx
         PxRow h;
         float scale;
         uint4 off[2];
-        px_head<FMT>(row, tile, r16, h, scale, off);
+        px_head<FMT>(row, tile, r16, true, h, scale, off);
 #pragma unroll 1
         for (int s = 0; s < 4; s++) {
           uint4 o[8];
-          px_stage<FMT>(row, s, h, o);
+          px_stage<FMT>(row, s, 0, h, o);
           wait(a_empty(slot), par);
           uint8_t *A = ra + slot * PF_A_BYTES + r * 16;
 #pragma unroll

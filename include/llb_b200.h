@@ -280,13 +280,15 @@ LLB_API int llb_spec_generate(llb_spec *m, int steps, int *ids, uint32_t *top2);
 /* the reference's per-token operator (spec_pass, host/llb_host.c:1902-1950): y = [v1, id1, v2, id2] */
 LLB_API int llb_spec_pass(llb_spec *m, int pos, int tok, float *y);
 LLB_API int llb_spec_position(const llb_spec *m);
-/* How llb_spec_prefill feeds a prompt.  mode 0 (default): every row through the T-row verify pass, eight rows a pass, at
- * the verify path's precision.  mode 1 (also LLB_PREFILL=fast in the environment at open, the reference's switch,
- * host/llb_host.c:206): all but the last k + 1 rows in chunks of 256 rows through dense tcgen05 GEMMs (operands as two fp16 planes)
+/* How llb_spec_prefill feeds a prompt.  mode 0 (default): at the verify path's precision; more than eight rows in pieces of up to 128
+ * rows through dense tcgen05 GEMMs on the exact weight codes, fewer (and every row of a model with routed experts, of a tensor-parallel rank, and
+ * where LLB_PREFILL_ROWS was set at open) through T-row verify passes.  What a prompt leaves behind depends on neither k nor the other streams.
+ * mode 1 (also LLB_PREFILL=fast in the environment at open, the reference's switch,
+ * host/llb_host.c:206): all but the last k + 1 rows in chunks of 256 rows through dense tcgen05 GEMMs (Q6_K and Q8_0 weights as two fp16 planes)
  * (replaces pf_take / spec_pf / spec_take, host/llb_pf.h:551, host/llb_host.c:1831-1899): trunk K/V, conv history and
  * DeltaNet state, and the drafter's K/V rows, are left as the T-row pass would have left them, within the path's
  * tolerance.  Models with routed experts always take mode 0.  Returns the previous mode.
- * llb_spec_fast_rows: prompt rows that went through the dense path since the engine was opened. */
+ * llb_spec_fast_rows: prompt rows that mode 1 put through the dense path since the engine was opened. */
 LLB_API int llb_spec_set_prefill(llb_spec *m, int mode);
 LLB_API double llb_spec_fast_rows(const llb_spec *m);
 /* n cycles enqueued back to back, no host round trip between them; returns the tokens emitted */
