@@ -40,27 +40,29 @@ __host__ __device__ constexpr bool px_offs(int fmt) { return px_planes(fmt) == 1
 __host__ __device__ constexpr int px_a_bytes(int fmt) { return px_planes(fmt) * PF_A_BYTES; }
 __host__ __device__ constexpr int px_b_bytes(int RU) { return RU * PF_KS * 2; }          // one plane of a stage's activations
 __host__ __device__ constexpr int px_ob_bytes(int RU) { return RU * 32; }                // ... and of the offsets' step
-// k_pfx1's rings: codes in stages of 64 columns (at most four: the offsets' step has one buffer on the weight rows' side, which a super-block's last
-// stage fills and the same stage of the next fills again, when the MMAs of the stage `px_na` before that one are done); activations in
-// slots of 16 KB and, where there is such a step, the means of a super-block behind them; weights in chunks of whole super-blocks (a copy costs
-// the SM's copy engine about 85 cycles, gemm2.cuh).
+// 64-column parts after which k_pfx1's accumulators are read, a stage's: the tensor core truncates where it adds to one, so that a sum loses about 2e-8 of itself an
+// MMA.  Its prompts take the place of verify rows, so it is read as often as that hides behind the MMAs.
+__host__ __device__ constexpr int px_drain(int fmt) { return px_planes(fmt) == 2 ? 1 : 2; }
+// k_pfx1's rings: codes in stages of eight MMAs, 128 columns of one plane or 64 of two (a stage costs the issuing warp and the unpacking ones
+// some 400 cycles whatever is in it); not more than a super-block, because the offsets' step has one buffer on the weight rows' side, which a
+// super-block's last stage fills and the same stage of the next fills again, when the MMAs of the stage `px_na` before that one are done;
+// activations in slots of 16 KB and, where there is such a step, the means of a super-block behind them; weights in chunks of whole
+// super-blocks (a copy costs the SM's copy engine about 85 cycles, gemm2.cuh).
 #define PX_SLOT 16384
-__host__ __device__ constexpr int px_na(int fmt) { return px_planes(fmt) == 2 ? 3 : 4; }
+__host__ __device__ constexpr int px_sub(int fmt) { return 3 - px_planes(fmt); }     // 64-column parts of a stage
+__host__ __device__ constexpr int px_na(int fmt) { return px_planes(fmt) == 2 ? 3 : 2; }
 __host__ __device__ constexpr int px_slot_stages(int RU) { return PX_SLOT / px_b_bytes(RU); }
 __host__ __device__ constexpr int px_slot_bytes(int fmt, int RU) { return PX_SLOT + (px_offs(fmt) ? px_ob_bytes(RU) : 0); }
 __host__ __device__ constexpr int px_nb(int fmt) { return fmt == LLB_FM_Q8_0 ? 3 : 4; }
 __host__ __device__ constexpr int px_chunk(int fmt) { return fmt == LLB_FM_Q4_K ? 2 : 1; }
 __host__ __device__ constexpr int px_raw_bytes(int fmt) { return 8 * px_chunk(fmt) * tile_bytes(fmt); }
-__host__ __device__ constexpr int px_fixed(int fmt, int RU) { return PX_HDR + PX_SC + (px_offs(fmt) ? PX_OA : 0) + px_na(fmt) * px_a_bytes(fmt) + px_nb(fmt) * px_slot_bytes(fmt, RU); }
+__host__ __device__ constexpr int px_fixed(int fmt, int RU) { return PX_HDR + PX_SC + (px_offs(fmt) ? PX_OA : 0) + px_na(fmt) * px_sub(fmt) * px_a_bytes(fmt) + px_nb(fmt) * px_slot_bytes(fmt, RU); }
 __host__ __device__ constexpr int px_raws(int fmt, int RU) {
   const int n = (PX_SMEM_MAX - px_fixed(fmt, RU)) / px_raw_bytes(fmt);
   return n > 4 ? 4 : n;
 }
 __host__ __device__ constexpr int px_smem(int fmt, int RU) { return px_fixed(fmt, RU) + px_raws(fmt, RU) * px_raw_bytes(fmt); }
-static_assert(px_na(LLB_FM_Q4_K) <= 4, "one buffer of the offsets' step");
-// Stages after which k_pfx1's accumulators are read: the tensor core truncates where it adds to one, so that a sum loses about 2e-8 of itself an
-// MMA.  Its prompts take the place of verify rows, so it is read as often as that hides behind the MMAs.
-__host__ __device__ constexpr int px_drain(int fmt) { return px_planes(fmt) == 2 ? 1 : 2; }
+static_assert(px_na(LLB_FM_Q4_K) * px_sub(LLB_FM_Q4_K) <= 4 && px_drain(LLB_FM_Q4_K) == px_sub(LLB_FM_Q4_K) && px_drain(LLB_FM_Q6_K) == px_sub(LLB_FM_Q6_K), "one buffer of the offsets' step; an accumulator a stage");
 // k_pfx2's rings: 64 columns of codes (a super-block's four stay until its hi products are done), 64 columns of one plane of the activations
 #define PX2_NA 6
 #define PX2_NB 4
@@ -251,8 +253,8 @@ template <int N> __device__ __forceinline__ void px_reg_dec() { asm volatile("se
 // ---- the kernels: work units, tiles and slices as in pfmm.cuh.  Up to 128 prompt rows: ----
 template <int FMT, int RU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pfx1(const PfArgs a) {
-  constexpr int NA = px_na(FMT), NB = px_nb(FMT), BS = px_slot_stages(RU), NPL = px_planes(FMT), N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), DG = px_drain(FMT);
-  constexpr int RAWB = px_raw_bytes(FMT), AB = px_a_bytes(FMT), SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU);
+  constexpr int NA = px_na(FMT), NB = px_nb(FMT), BS = px_slot_stages(RU), NPL = px_planes(FMT), N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), SS = px_sub(FMT);
+  constexpr int RAWB = px_raw_bytes(FMT), AB = px_a_bytes(FMT), STB = SS * AB, SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU);
   static_assert(NRAW >= 2 && px_smem(FMT, RU) <= PX_SMEM_MAX, "a form that does not fit");
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -271,7 +273,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
   uint32_t *tmem_slot = (uint32_t *)(smem + 320);
   volatile uint32_t *dead = (volatile uint32_t *)(smem + 324);
   float *scr = (float *)(smem + PX_HDR);
-  uint8_t *oa = smem + PX_HDR + PX_SC, *ra = oa + (px_offs(FMT) ? PX_OA : 0), *rb = ra + NA * AB, *raw = rb + NB * SLB;
+  uint8_t *oa = smem + PX_HDR + PX_SC, *ra = oa + (px_offs(FMT) ? PX_OA : 0), *rb = ra + NA * STB, *raw = rb + NB * SLB;
   const uint32_t oa_s = smem_u32(oa), ra_s = smem_u32(ra), rb_s = smem_u32(rb), raw_s = smem_u32(raw);
   const int ntiles = a.t128[a.nmat], npairs = (ntiles + 1) >> 1, nunits = npairs * a.ksplit;
   const int rank = blockIdx.x & 1, unit0 = blockIdx.x >> 1, ustep = gridDim.x >> 1;
@@ -322,19 +324,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
         uint4 off[2];
         px_head<FMT>(row, tile, r16, part == 0, h, scale, off);
 #pragma unroll 1
-        for (int s = 0; s < 4; s++) {
+        for (int s = 0; s < 4; s += SS) {
           uint4 o[4 * NPL];
           px_stage<FMT, 2>(row, s, part, h, o);
           wait(a_empty(slot), par);
-          uint8_t *A = ra + slot * AB + r * 16;
+          uint8_t *A = ra + slot * STB + r * 16;
 #pragma unroll
           for (int i = 0; i < 4 * NPL; i++) *(uint4 *)(A + (i >> 2) * PF_A_BYTES + px_group<FMT, 2>(i & 3, part) * 2048) = o[i];
+          if constexpr (SS == 2) {
+            px_stage<FMT, 2>(row, s + 1, part, h, o);
+#pragma unroll
+            for (int i = 0; i < 4; i++) *(uint4 *)(A + AB + px_group<FMT, 2>(i, part) * 2048) = o[i];
+          }
           if (s == 0 && part == 0) {   // (the scales of the super-block four back have been read: its accumulators were, before the stages that were waited for here)
             scr[(jj & 3) * 128 + r] = scale;
             __syncwarp();
             if (lane == 0) mbar_arrive(sc_full(jj & 3));
           }
-          if (s == 3 && part == 0 && px_offs(FMT)) { *(uint4 *)(oa + r * 16) = off[0]; *(uint4 *)(oa + (128 + r) * 16) = off[1]; }
+          if (s + SS == 4 && part == 0 && px_offs(FMT)) { *(uint4 *)(oa + r * 16) = off[0]; *(uint4 *)(oa + (128 + r) * 16) = off[1]; }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads these bytes through the async proxy
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(lead + (a_full(slot) - bar_s));
@@ -421,30 +428,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
         int kbase, nst;
         pf_slice(a, u, npairs, kbase, nst);
 #pragma unroll 1
-        for (int s = 0; s < nst; s++) {
-          const uint32_t D = tmem + (uint32_t)((dd & 1) * 256), first = s % DG == 0;
-          const bool last = s % DG == DG - 1, out = s % BS == BS - 1;      // of an accumulator; of a slot of activations
-          if (first && dd > 1) wait(d_empty(dd & 1), (uint32_t)((dd >> 1) - 1) & 1u);
-          if (s % BS == 0) wait(b_full(bs), bpar);
+        for (int s = 0; s < nst; s += SS, dd++) {
+          const uint32_t D = tmem + (uint32_t)((dd & 1) * 256);
+          if (dd > 1) wait(d_empty(dd & 1), (uint32_t)((dd >> 1) - 1) & 1u);
           wait(a_full(as), apar);
-          t5_fence_after();
-          const uint64_t ad = g3_desc(ra_s + as * AB, 2048, 128), bd = g3_desc(rb_s + bs * SLB + s % BS * PLB, RU * 16, 128);
-          if (el) {
-            // (two planes: the smaller one first, while there is little for the additions to truncate)
+          const uint64_t ad = g3_desc(ra_s + as * STB, 2048, 128);
 #pragma unroll
-            for (int pl = NPL - 1; pl >= 0; pl--)
+          for (int q = 0; q < SS; q++) {
+            const int in = (s + q) % BS;          // part of the slot of activations
+            if (in == 0) wait(b_full(bs), bpar);
+            t5_fence_after();
+            const uint64_t bd = g3_desc(rb_s + bs * SLB + in * PLB, RU * 16, 128);
+            if (el) {
+              // (two planes: the smaller one first, while there is little for the additions to truncate)
 #pragma unroll
-              for (int k = 0; k < 4; k++)
-                pf_mma_ss(D, ad + (uint64_t)(pl * (PF_A_BYTES / 16) + k * 256), bd + (uint64_t)(k * 2 * RU), px_idesc(N), k != 0 || pl != NPL - 1 ? 1u : !first);
-            if (px_offs(FMT) && (s & 3) == 3) pf_mma_ss(D, oad, g3_desc(rb_s + bs * SLB + PX_SLOT, RU * 16, 128), px_idesc(N), 1u);
-            t5_commit_pair(a_empty(as));
-            if (out) t5_commit_pair(b_empty(bs));
-            if (last) t5_commit_pair(d_full(dd & 1));
+              for (int pl = NPL - 1; pl >= 0; pl--)
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                  pf_mma_ss(D, ad + (uint64_t)(q * (AB / 16) + pl * (PF_A_BYTES / 16) + k * 256), bd + (uint64_t)(k * 2 * RU), px_idesc(N), k != 0 || pl != NPL - 1 || q != 0);
+              if (q == SS - 1) {
+                if (px_offs(FMT) && (s & 3) + SS == 4) pf_mma_ss(D, oad, g3_desc(rb_s + bs * SLB + PX_SLOT, RU * 16, 128), px_idesc(N), 1u);
+                t5_commit_pair(a_empty(as));
+                t5_commit_pair(d_full(dd & 1));
+              }
+              if (in == BS - 1) t5_commit_pair(b_empty(bs));
+            }
+            __syncwarp();
+            if (in == BS - 1 && ++bs == NB) { bs = 0; bpar ^= 1u; }
           }
-          __syncwarp();
-          if (last) dd++;
           if (++as == NA) { as = 0; apar ^= 1u; }
-          if (out && ++bs == NB) { bs = 0; bpar ^= 1u; }
         }
       }
     }
@@ -468,7 +480,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
         const float scf = scr[(jj & 3) * 128 + 32 * q + lane];
         const f32x2 sc = x2_pack(scf, scf);
 #pragma unroll 1
-        for (int p = 0; p < 4 / DG; p++, dd++) {
+        for (int p = 0; p < 4 / SS; p++, dd++) {
           const uint32_t t1 = t0 + (uint32_t)((dd & 1) * 256);
           wait(d_full(dd & 1), (uint32_t)(dd >> 1) & 1u);
           t5_fence_after();
