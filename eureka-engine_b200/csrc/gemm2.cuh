@@ -24,7 +24,7 @@
 
 #define G2_SMEM_MAX 226304   // 227 KB less the 6 KB that a phase may use beside the ring and the activation slice
 #define G2_MAXWARPS 16
-#define G2_WAIT_LIMIT (1u << 19)   // tries of a bounded wait (up to a microsecond each)
+#define G2_WAIT_LIMIT (1u << 19)   // tries of a bounded wait (up to 4 us each)
 #define G2_DRAIN_LIMIT (1u << 13)
 #define G2_BAR_BYTES 512     // one mbarrier per warp and stage (at most four)
 

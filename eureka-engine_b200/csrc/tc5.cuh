@@ -3,7 +3,7 @@
 #pragma once
 #include "common.cuh"
 
-#define T5_WAIT_LIMIT (1u << 22)   // tries of a bounded mbarrier wait (each parks the thread for up to a microsecond)
+#define T5_WAIT_LIMIT (1u << 22)   // tries of a bounded mbarrier wait (each parks the thread for up to 4 us)
 
 __device__ __forceinline__ void t5_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void t5_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -96,10 +96,10 @@ __device__ __forceinline__ bool t5_elect(void) {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar_s, uint32_t parity, uint32_t limit = T5_WAIT_LIMIT) {
   for (uint32_t it = 0; it < limit; it++) {
     uint32_t ok;
-    // the hint lets the hardware park the thread until the phase completes (or about a microsecond passes)
-    // instead of polling: sixteen worker warps and four issuing warps otherwise spend most issue slots on polls
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
-                 : "=r"(ok) : "r"(bar_s), "r"(parity), "r"(1000u) : "memory");
+    // (a try parks the thread until the phase completes or about 4 us have passed.  A time hint, 1 us, does not shorten that, and with it threads
+    // saw a complete phase later: gate|up of the 27B shape 27.1 -> 26.0 us at four rows, the dense GEMMs of a prompt 1.5 % slower)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(ok) : "r"(bar_s), "r"(parity) : "memory");
     if (ok) return true;
   }
   return false;
