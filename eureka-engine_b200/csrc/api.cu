@@ -237,9 +237,12 @@ int llb_b200_gemm(int fmt, int nmat, const llb_b200_dptr *w, const int *rows, co
     else { a.m[i].out = g_parts + off; a.m[i].split_stride = (long long)per_split; off += (size_t)xp->T * rows[i]; }
   }
   if (gemm_launch(g_llb.stream, fmt, a)) return -1;
-  if (a.ksplit > 1)
-    for (int i = 0; i < nmat; i++)
-      if (ops_sum_parts(g_llb.stream, a.m[i].out, a.ksplit, a.m[i].split_stride, xp->T * rows[i], (float *)(uintptr_t)out[i])) return -1;
+  if (a.ksplit > 1) {   // one launch for all matrices' slices
+    int n[GEMM_MAXMAT];
+    float *o[GEMM_MAXMAT];
+    for (int i = 0; i < nmat; i++) { n[i] = xp->T * rows[i]; o[i] = (float *)(uintptr_t)out[i]; }
+    return ops_sum_parts_of(g_llb.stream, g_parts, a.ksplit, (long long)per_split, nmat, n, o);
+  }
   return 0;
 }
 

@@ -313,8 +313,18 @@ int gemm_pick_ksplit(int fmt, int NC, int ntiles, int nsb, int sms) {
 
 int gemm_which(int fmt, int NC, int ntiles, int nsb, int sms, bool alone, int *ksplit) {
   bool g3 = false;
-  if (alone && *ksplit <= 0) *ksplit = gemm_pick_alone(fmt, NC, ntiles, nsb, sms, &g3);
-  else {
+  if (alone && *ksplit <= 0) {
+    // (the choice costs 1.5 us of a call of 9, and depends on nothing but these: a thread keeps its last ones)
+    struct Kept { int fmt, NC, ntiles, nsb, sms, mode, ks; bool g3; };
+    static thread_local Kept kept[64];
+    const int mode = g_llb.gemm3;
+    Kept &e = kept[((unsigned)ntiles * 31u + (unsigned)nsb * 7u + (unsigned)fmt * 3u + (unsigned)NC) & 63u];
+    if (e.ks < 1 || e.fmt != fmt || e.NC != NC || e.ntiles != ntiles || e.nsb != nsb || e.sms != sms || e.mode != mode) {
+      e = Kept{fmt, NC, ntiles, nsb, sms, mode, 0, false};
+      e.ks = gemm_pick_alone(fmt, NC, ntiles, nsb, sms, &e.g3);
+    }
+    *ksplit = e.ks; g3 = e.g3;
+  } else {
     *ksplit = gemm_fix_ksplit(fmt, NC, nsb, *ksplit > 0 ? *ksplit : gemm_pick_ksplit(fmt, NC, ntiles, nsb, sms), alone);
     g3 = g3_use(fmt, NC, ntiles, nsb, *ksplit, sms, alone);
   }

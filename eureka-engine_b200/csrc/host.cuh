@@ -93,4 +93,5 @@ int ops_setup(void);   // at init
 int ops_fence_hold(bool on);
 int ops_to_tiles(cudaStream_t s, int fmt, const uint8_t *src, int rows, int cols, uint8_t *dst);
 int ops_tile_slice(cudaStream_t s, int fmt, const uint8_t *src, int scols, uint8_t *dst, int dcols, int srow, int drow, int n, int scol, int dcol, int nc);
+int ops_sum_parts_of(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int nmat, const int *n, float *const *out);
 int ops_sum_parts(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int n, float *out);

@@ -158,12 +158,7 @@ int ops_tile_slice(cudaStream_t s, int fmt, const uint8_t *src, int scols, uint8
 // ---- fixed-order sum of K-slice partials --------------------------------------------------------
 // All slices of a value in one trip to L2 (NS of them; 0: any number, four a trip).  Loads to L2: the GEMM in front wrote the
 // partial sums, and the buffer is used by one call after another.
-template <int NS> __device__ __forceinline__ void sum_parts(const float *parts, int nsplit, long long stride, int n, float *out) {
-  pdl_trigger();
-  pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float *p = parts + i;
+template <int NS> __device__ __forceinline__ float sum_parts(const float *p, int nsplit, long long stride) {
   float v;
   if constexpr (NS > 0) {
     float l[NS];
@@ -177,11 +172,31 @@ template <int NS> __device__ __forceinline__ void sum_parts(const float *parts, 
 #pragma unroll 4
     for (int k = 1; k < nsplit; k++) v += __ldcg(p + k * stride);
   }
-  out[i] = v;
+  return v;
 }
-__global__ void k_sum_parts(const float *__restrict__ parts, int nsplit, long long stride, int n, float *__restrict__ out) { sum_parts<0>(parts, nsplit, stride, n, out); }
+__global__ void k_sum_parts(const float *__restrict__ parts, int nsplit, long long stride, int n, float *__restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = sum_parts<0>(parts + i, nsplit, stride);
+}
 template <int NS> __global__ void __launch_bounds__(256) k_sum_slices(const float *__restrict__ parts, long long stride, int n, float *__restrict__ out) {
-  sum_parts<NS>(parts, NS, stride, n, out);
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = sum_parts<NS>(parts + i, NS, stride);
+}
+// outputs of two to four matrices, one after the other in a slice: output m's first value is value at[m]
+struct SumOut { float *p[GEMM_MAXMAT]; int at[GEMM_MAXMAT]; };
+template <int NS> __global__ void __launch_bounds__(256) k_sum_slices_of(const float *__restrict__ parts, long long stride, int n, const SumOut o) {
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int m = 0;
+#pragma unroll
+  for (int k = 1; k < GEMM_MAXMAT; k++) if (i >= o.at[k]) m = k;
+  o.p[m][i - o.at[m]] = sum_parts<NS>(parts + i, NS, stride);
 }
 int ops_sum_parts(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int n, float *out) {
   const dim3 grid((n + 255) / 256);
@@ -190,6 +205,25 @@ int ops_sum_parts(cudaStream_t s, const float *parts, int nsplit, long long spli
     SUM_GO(2) SUM_GO(3) SUM_GO(4) SUM_GO(5) SUM_GO(6) SUM_GO(7) SUM_GO(8) SUM_GO(9) SUM_GO(10) SUM_GO(11) SUM_GO(12) SUM_GO(13) SUM_GO(14) SUM_GO(15) SUM_GO(16)
 #undef SUM_GO
     default: CU_OK(llb_launch(k_sum_parts, grid, dim3(256), (size_t)(0), s, parts, nsplit, split_stride, n, out));
+  }
+  CU_OK(cudaGetLastError());
+  return 0;
+}
+// ... of nmat outputs of n[i] values each, one after the other in a slice (2 <= nsplit <= GEMM_MAXSPLIT): a launch costs the host 1.4 us of a call's 10
+int ops_sum_parts_of(cudaStream_t s, const float *parts, int nsplit, long long split_stride, int nmat, const int *n, float *const *out) {
+  if (nmat == 1) return ops_sum_parts(s, parts, nsplit, split_stride, n[0], out[0]);
+  SumOut o;
+  int total = 0;
+  for (int i = 0; i < GEMM_MAXMAT; i++) {
+    o.p[i] = i < nmat ? out[i] : nullptr; o.at[i] = i < nmat ? total : 0x7fffffff;
+    if (i < nmat) total += n[i];
+  }
+  const dim3 grid((total + 255) / 256);
+  switch (nsplit) {
+#define SUM_GO(NS) case NS: CU_OK(llb_launch(k_sum_slices_of<NS>, grid, dim3(256), (size_t)(0), s, parts, split_stride, total, o)); break;
+    SUM_GO(2) SUM_GO(3) SUM_GO(4) SUM_GO(5) SUM_GO(6) SUM_GO(7) SUM_GO(8) SUM_GO(9) SUM_GO(10) SUM_GO(11) SUM_GO(12) SUM_GO(13) SUM_GO(14) SUM_GO(15) SUM_GO(16)
+#undef SUM_GO
+    default: return llb_fail("sum of %d slices", nsplit);
   }
   CU_OK(cudaGetLastError());
   return 0;

@@ -177,10 +177,20 @@ def arr(ty, vals):
     return (ty * len(vals))(*vals)
 
 
+_U64 = [C.c_uint64 * n for n in range(5)]   # (looked up, not made anew: a call is short)
+_I32 = [C.c_int * n for n in range(5)]
+
+
 def gemm(fmt: int, ws, rows, outs, K: int, xp, ksplit: int = 0):
     n = len(ws)
-    check(lib().llb_b200_gemm(fmt, n, arr(C.c_uint64, ws), arr(C.c_int, rows), arr(C.c_uint64, outs), K, xp, ksplit),
-          "llb_b200_gemm")
+    if n == 1 and len(rows) == 1 and len(outs) == 1:
+        rc = lib().llb_b200_gemm(fmt, 1, C.byref(C.c_uint64(ws[0])), C.byref(C.c_int(rows[0])), C.byref(C.c_uint64(outs[0])), K, xp, ksplit)
+    elif n <= 4 and len(rows) == n and len(outs) == n:
+        rc = lib().llb_b200_gemm(fmt, n, _U64[n](*ws), _I32[n](*rows), _U64[n](*outs), K, xp, ksplit)
+    else:
+        rc = lib().llb_b200_gemm(fmt, n, arr(C.c_uint64, ws), arr(C.c_int, rows), arr(C.c_uint64, outs), K, xp, ksplit)
+    if rc < 0:
+        check(rc, "llb_b200_gemm")
 
 
 class SmpParams(C.Structure):
