@@ -26,7 +26,8 @@ template <typename K> static int px_attr(K k, int smem, int regs) {
   return 0;
 }
 template <int FMT> static int px_attr1() {
-  return px_attr(k_pfx1<FMT, 32>, px_smem(FMT, 32), PX1_REG_LAUNCH) || px_attr(k_pfx1<FMT, 64>, px_smem(FMT, 64), PX1_REG_LAUNCH) || px_attr(k_pfx1<FMT, 128>, px_smem(FMT, 128), PX1_REG_LAUNCH);
+  CU_OK(cudaFuncSetAttribute(k_pft<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, pt_smem(FMT)));
+  return px_attr(k_pfx1<FMT, 64>, px_smem(FMT, 64), PX1_REG_LAUNCH) || px_attr(k_pfx1<FMT, 128>, px_smem(FMT, 128), PX1_REG_LAUNCH);
 }
 template <int FMT> static int px_attr2() { return px_attr(k_pfx2<FMT>, px2_smem(FMT), PX_REG_LAUNCH); }
 #define PF_SCAN_NW 4                            // warps of a scan block, 8 state rows each
@@ -80,8 +81,9 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a) {
   const int grid = 2 * (units < g_llb.sms / 2 ? units : g_llb.sms / 2);
   cudaError_t e = cudaErrorInvalidValue;
   const int ru = pf_unit_rows(a.R);
+#define PT_GO(F) e = llb_launch(k_pft<F>, dim3(grid), dim3(PX1_THREADS), (size_t)pt_smem(F), s, a)
 #define PX_GO(F, RU) e = llb_launch(k_pfx1<F, RU>, dim3(grid), dim3(PX1_THREADS), (size_t)px_smem(F, RU), s, a)
-#define PX_ONE(F) do { if (ru == 32) PX_GO(F, 32); else if (ru == 64) PX_GO(F, 64); else PX_GO(F, 128); } while (0)
+#define PX_ONE(F) do { if (ru == 32) PT_GO(F); else if (ru == 64) PX_GO(F, 64); else PX_GO(F, 128); } while (0)
 #define PX_TWO(F) e = llb_launch(k_pfx2<F>, dim3(grid), dim3(PX_THREADS), (size_t)px2_smem(F), s, a)
   switch (fmt) {
     case LLB_FM_Q4_K: if (a.R > PF_R) PX_TWO(LLB_FM_Q4_K); else PX_ONE(LLB_FM_Q4_K); break;
@@ -92,6 +94,7 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a) {
   }
 #undef PX_TWO
 #undef PX_ONE
+#undef PT_GO
 #undef PX_GO
   if (e != cudaSuccess) return llb_fail("dense GEMM launch: %s", cudaGetErrorString(e));
   return 0;

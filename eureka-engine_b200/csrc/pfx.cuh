@@ -16,8 +16,9 @@
 //           then, on top of that sum divided by 2048 (the MMA's own scaling of D), its codes . hi: one accumulator of 256
 //           columns, so that two fit tensor memory and one is read while the other fills.  128 sums a thread in the 256 threads that read
 //           them (setmaxnreg).
-//   k_pfx1  RU = 32, 64 or 128 prompt rows: the first CTA stages the hi plane, the second the lo plane, N = 2 RU, one MMA a step and
-//           plane of codes; two accumulators take turns, every px_drain stages.
+//   k_pfx1  RU = 64 or 128 prompt rows: the first CTA stages the hi plane, the second the lo plane, N = 2 RU, one MMA a step and
+//           plane of codes; two accumulators take turns, a stage each.
+//   k_pft   the same for up to 32 rows with the codes in tensor memory.
 // Weights come as bulk copies of whole super-blocks of a 16-row tile into a ring of their own.
 //
 // What bounds k_pfx2 is the power the tensor cores may draw: gate|up of the 27B shape, 256 rows, 223 GFLOP of products in 136 us = 1.64 PFLOP/s
@@ -49,6 +50,8 @@ __host__ __device__ constexpr int px_drain(int fmt) { return px_planes(fmt) == 2
 // activations in slots of 16 KB and, where there is such a step, the means of a super-block behind them; weights in chunks of whole
 // super-blocks (a copy costs the SM's copy engine about 85 cycles, gemm2.cuh).
 #define PX_SLOT 16384
+#define PT_RU 32              // rows of k_pft, the kernel of the fewest
+#define PT_NB 4               // its slots: its two groups have two each
 __host__ __device__ constexpr int px_sub(int fmt) { return 3 - px_planes(fmt); }     // 64-column parts of a stage
 __host__ __device__ constexpr int px_na(int fmt) { return px_planes(fmt) == 2 ? 3 : 2; }
 __host__ __device__ constexpr int px_slot_stages(int RU) { return PX_SLOT / px_b_bytes(RU); }
@@ -500,6 +503,310 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
           }
         }
       }
+      const int tile = tile_of(u);
+      pf_locate(a, min(tile, ntiles - 1), m, row0);
+      const int row = row0 + 32 * q + lane, n = R - half * RH;   // this warp's prompt rows in use
+      if (tile < ntiles && row < a.m[m].rows) {
+        const size_t os = a.m[m].ostride;
+        float *out = a.m[m].out + (size_t)(u / npairs) * a.m[m].split_stride + (size_t)(half * RH) * os + row;
+#pragma unroll
+        for (int j = 0; j < RH; j += 2) {
+          float y0, y1;
+          x2_unpack(acc[j / 2], y0, y1);
+          if (j < n) *out = y0;
+          out += os;
+          if (j + 1 < n) *out = y1;
+          out += os;
+        }
+      }
+    }
+  }
+  // after a wait ran out nothing is requested any more, but copies may be on their way into this CTA's rings
+  if (*dead) for (int i = 0; i < 64; i++) __nanosleep(1000);
+  __syncwarp();
+  t5_fence_before();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // no CTA leaves while the other still arrives here or reads its memory
+  if (warp == 10) {
+    t5_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// ---- up to 32 prompt rows: the codes as the MMAs' operand in TENSOR MEMORY ----
+// Two groups of four unpacking warps, a thread a weight row, take the super-blocks in turn, each with an issuing warp and accumulators of its own:
+// what one group waits for the other fills.  An ITEM is what 64 columns of tensor memory hold, 128 columns of one plane of codes or 64 of two; a
+// group has two such buffers and two accumulators, so that it unpacks one item while the other is multiplied, and multiplies one while the other
+// is read.  Sums are added in the columns' order, as k_pfx1 adds them: the same bits.  What bounds it is a group's chain, 4000 cycles a super-block, of
+// which unpacking is half.  Twenty rows, k_pfx1 with 32 / this: Q4_K 34816 x 5120 59.5 / 44 us, 5120 x 6144 17.8 / 15, Q6_K 5120 x 17408 56 / 43,
+// Q8_0 24576 x 4096 61 / 47, Q5_K 8192 x 4096 19 / 17.  With 64 rows only one accumulator a group fits: Q4_K 70 / 63, Q6_K 65 / 73, Q8_0 70 / 80, not kept.
+// A barrier is only ever waited for by one group, which sees every phase of it (a phase's parity tells nothing to one that missed the phase before).
+__host__ __device__ constexpr int pt_items(int fmt) { return 2 * px_planes(fmt); }       // of a super-block
+__host__ __device__ constexpr int pt_fixed(int fmt) { return PX_HDR + 2 * PX_SC + (px_offs(fmt) ? 2 * PX_OA : 0) + PT_NB * px_slot_bytes(fmt, PT_RU); }
+__host__ __device__ constexpr int pt_raws(int fmt) {
+  const int n = (PX_SMEM_MAX - pt_fixed(fmt)) / px_raw_bytes(fmt);
+  return n > 4 ? 4 : n;
+}
+__host__ __device__ constexpr int pt_smem(int fmt) { return pt_fixed(fmt) + pt_raws(fmt) * px_raw_bytes(fmt); }
+__device__ __forceinline__ void pt_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+template <int FMT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pft(const PfArgs a) {
+  constexpr int RU = PT_RU, NB = PT_NB, SPB = 4 / px_slot_stages(RU), NPL = px_planes(FMT), NP = pt_items(FMT), SI = 4 / NP, N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = pt_raws(FMT);
+  constexpr int RAWB = px_raw_bytes(FMT), SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU), ND = 128 / N;   // SPB: slots of activations a super-block (SI: 64-column parts an item); ND: accumulators a group
+  static_assert(NRAW >= 2 && pt_smem(FMT) <= PX_SMEM_MAX && NB % (2 * SPB) == 0 && ND >= 1, "a form that does not fit");
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t bar_s = smem_u32(smem), lead = t5_map_rank(bar_s, 0);   // the leader's (the pair's first CTA's) barriers, as both CTAs name them
+  auto a_full = [&](int i) { return bar_s + 8u * (uint32_t)i; };               // [group][buffer]; leader: both CTAs' unpacking warps of the group
+  auto a_empty = [&](int i) { return bar_s + 32u + 8u * (uint32_t)i; };
+  auto b_full = [&](int s) { return bar_s + 64u + 8u * (uint32_t)s; };         // leader: its own copy and the other CTA's, passed on from that one's b_here
+  auto b_empty = [&](int s) { return bar_s + 96u + 8u * (uint32_t)s; };
+  auto b_here = [&](int s) { return bar_s + 128u + 8u * (uint32_t)s; };
+  auto d_full = [&](int i) { return bar_s + 160u + 8u * (uint32_t)i; };        // [group][accumulator]
+  auto d_empty = [&](int i) { return bar_s + 192u + 8u * (uint32_t)i; };       // leader: the reading warps of both CTAs
+  auto sc_full = [&](int i) { return bar_s + 224u + 8u * (uint32_t)i; };
+  auto raw_full = [&](int i) { return bar_s + 256u + 8u * (uint32_t)i; };
+  auto raw_empty = [&](int i) { return bar_s + 288u + 8u * (uint32_t)i; };
+  uint32_t *tmem_slot = (uint32_t *)(smem + 320);
+  volatile uint32_t *dead = (volatile uint32_t *)(smem + 324);
+  float *scr = (float *)(smem + PX_HDR);
+  uint8_t *oa = smem + PX_HDR + 2 * PX_SC, *rb = oa + (px_offs(FMT) ? 2 * PX_OA : 0), *raw = rb + NB * SLB;
+  const uint32_t oa_s = smem_u32(oa), rb_s = smem_u32(rb), raw_s = smem_u32(raw);
+  const int ntiles = a.t128[a.nmat], npairs = (ntiles + 1) >> 1, nunits = npairs * a.ksplit;
+  const int rank = blockIdx.x & 1, unit0 = blockIdx.x >> 1, ustep = gridDim.x >> 1;
+  auto tile_of = [&](int u) { return 2 * (u % npairs) + rank; };
+
+  pdl_trigger();
+  if (tid == 0) {
+    for (int i = 0; i < 4; i++) { mbar_init(a_full(i), 8); mbar_init(a_empty(i), 1); mbar_init(d_full(i), 1); mbar_init(d_empty(i), 16); mbar_init(sc_full(i), 4); }
+    for (int s = 0; s < NB; s++) { mbar_init(b_full(s), 2); mbar_init(b_empty(s), 1); mbar_init(b_here(s), 1); }
+    for (int i = 0; i < NRAW; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), 8); }
+    *dead = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 10) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  t5_fence_before();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // both CTAs' barriers exist
+  t5_fence_after();
+  const uint32_t tmem = *tmem_slot;                    // codes: 64 columns a buffer, [group][buffer]; behind them the accumulators, 128 columns a group
+  auto wait = [&](uint32_t bar, uint32_t parity) {   // gives up for the whole CTA
+    for (uint32_t n = 0; !mbar_wait(bar, parity, 4); n += 4) {
+      if (*dead) return;
+      if (n >= T5_WAIT_LIMIT) { *dead = 1; if (a.err) atomicExch(a.err, 1u); return; }
+    }
+  };
+
+  if (warp < 8) {
+    // ---- codes: group g, a thread a weight row ----
+    const int g = warp >> 2, r = tid & 127, r16 = r & 15;
+    const uint32_t abuf = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(128 * g);
+    const uint32_t roff = (uint32_t)(r >> 4) * (CH * TB);
+    int rs = 0, jj = 0, it = 0;             // super-blocks of the CTA, items of the group so far
+    uint32_t rpar = 0;
+    for (int u = unit0; u < nunits; u += ustep) {
+      int kbase, nst;
+      pf_slice(a, u, npairs, kbase, nst);
+      const int nsl = nst >> 2;
+#pragma unroll 1
+      for (int c = 0; c < nsl; c++, jj++) {
+        if (c % CH == 0) wait(raw_full(rs), rpar);     // (by both groups, whichever has the super-block)
+        if ((jj & 1) == g) {
+          const uint8_t *tile = raw + rs * RAWB + roff + c % CH * TB, *row = tile + r16 * tile_row(FMT);
+          PxRow h;
+          float scale;
+          uint4 off[2];
+          px_head<FMT>(row, tile, r16, true, h, scale, off);
+#pragma unroll 1
+          for (int p = 0; p < NP; p++, it++) {
+            uint4 o[8 * NPL];
+            px_stage<FMT>(row, p * SI, 0, h, o);
+            wait(a_empty(2 * g + (it & 1)), (uint32_t)((it >> 1) & 1) ^ 1u);     // (the first round passes)
+            t5_fence_after();
+            const uint32_t A = abuf + 64u * (uint32_t)(it & 1);
+            auto put = [&](uint32_t at, const uint4 *q) {
+              const uint32_t v[32] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w, q[2].x, q[2].y, q[2].z, q[2].w, q[3].x, q[3].y, q[3].z, q[3].w,
+                                      q[4].x, q[4].y, q[4].z, q[4].w, q[5].x, q[5].y, q[5].z, q[5].w, q[6].x, q[6].y, q[6].z, q[6].w, q[7].x, q[7].y, q[7].z, q[7].w};
+              t5_st32(at, v);
+            };
+            put(A, o);
+            if constexpr (NPL == 2) put(A + 32, o + 8);
+            else {
+              px_stage<FMT>(row, p * SI + 1, 0, h, o);
+              put(A + 32, o);
+            }
+            if (p == 0) {   // (the scales of the super-block eight back: with the group's buffer free again, the one four back is being read at the earliest)
+              scr[(jj & 7) * 128 + r] = scale;
+              __syncwarp();
+              if (lane == 0) mbar_arrive(sc_full(jj & 3));
+            }
+            if (p == NP - 1 && px_offs(FMT)) {
+              uint8_t *O = oa + g * PX_OA + r * 16;
+              *(uint4 *)O = off[0]; *(uint4 *)(O + 2048) = off[1];
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads these bytes through the async proxy
+            }
+            t5_wait_st();
+            t5_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(lead + (a_full(2 * g + (it & 1)) - bar_s));
+          }
+        }
+        if (c % CH == CH - 1 || c == nsl - 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(raw_empty(rs));
+          if (++rs == NRAW) { rs = 0; rpar ^= 1u; }
+        }
+      }
+    }
+  } else if (warp == 8) {
+    // ---- weights: lane t requests the t-th 16-row tile of every chunk of the CTA's 128 rows ----
+    int rs = 0;
+    uint32_t rpar = 1;
+    for (int u = unit0; u < nunits; u += ustep) {
+      int kbase, nst, m, row0;
+      pf_slice(a, u, npairs, kbase, nst);
+      pf_locate(a, min(tile_of(u), ntiles - 1), m, row0);
+      const int nsl = nst >> 2, nsb = a.K >> 8, have = min(8, ((a.m[m].rows + 15) >> 4) - (row0 >> 4));
+      const uint8_t *src = a.m[m].W + ((size_t)((row0 >> 4) + min(lane, have - 1)) * nsb + (kbase >> 8)) * TB;
+#pragma unroll 1
+      for (int c = 0; c < nsl; c += CH) {
+        const int n = min(CH, nsl - c);
+        wait(raw_empty(rs), rpar);
+        // (one answer for the warp: lanes that saw the word differently would leave bytes expected that nobody requests)
+        if (!__any_sync(0xffffffffu, *dead != 0)) {
+          if (lane == 0) mbar_expect(raw_full(rs), (uint32_t)(have * n * TB));
+          __syncwarp();
+          if (lane < have) bulk_load(raw_s + rs * RAWB + lane * (CH * TB), src + (size_t)c * TB, (uint32_t)(n * TB), raw_full(rs));
+        }
+        __syncwarp();
+        if (++rs == NRAW) { rs = 0; rpar ^= 1u; }
+      }
+    }
+  } else if (warp == 9) {
+    // ---- activations: the CTA's plane; the other CTA's warp then tells the leader that they are there ----
+    if (lane == 0) {
+      int slot = 0;
+      uint32_t par = 1;
+      pdl_wait();
+      const __half *x = a.x + (size_t)rank * a.K * RU, *xs = a.x + (size_t)2 * a.K * RU + (size_t)rank * pf_sum_halves(a.K, RU);
+      for (int u = unit0; u < nunits; u += ustep) {
+        int kbase, nst;
+        pf_slice(a, u, npairs, kbase, nst);
+#pragma unroll 1
+        for (int i = 0; i < (nst >> 2) * SPB; i++) {
+          wait(b_empty(slot), par);
+          if (!*dead) {
+            const bool last = px_offs(FMT) && i % SPB == SPB - 1;
+            const uint32_t bar = rank ? b_here(slot) : b_full(slot), dst = rb_s + slot * SLB;
+            mbar_expect(bar, (uint32_t)(PX_SLOT + (last ? OPB : 0)));
+            pf_bulk_copy(dst, x + (size_t)kbase * RU + (size_t)i * (PX_SLOT / 2), PX_SLOT, bar);
+            if (last) pf_bulk_copy(dst + PX_SLOT, xs + (size_t)((kbase >> 8) + i / SPB) * 16 * RU, OPB, bar);
+          }
+          if (++slot == NB) { slot = 0; par ^= 1u; }
+        }
+      }
+    }
+  } else if (warp < 12) {
+    if (rank == 1) {
+      if (warp == 11 && lane == 0) {
+        int slot = 0;
+        uint32_t par = 0;
+        for (int u = unit0; u < nunits; u += ustep) {
+          int kbase, nst;
+          pf_slice(a, u, npairs, kbase, nst);
+#pragma unroll 1
+          for (int i = 0; i < (nst >> 2) * SPB; i++) {
+            wait(b_here(slot), par);
+            mbar_arrive_cluster(lead + (b_full(slot) - bar_s));
+            if (++slot == NB) { slot = 0; par ^= 1u; }
+          }
+        }
+      }
+    } else {
+      // ---- the tensor cores of the pair, from the leader: a warp a group; the whole warp walks, an elected lane issues ----
+      const int g = __shfl_sync(0xffffffffu, warp - 10, 0);
+      const bool el = t5_elect();
+      const uint64_t oad = g3_desc(oa_s + g * PX_OA, 2048, 128);
+      const uint32_t ab = tmem + (uint32_t)(128 * g), db = tmem + 256u + (uint32_t)(128 * g);
+      int jj = 0, it = 0;
+      for (int u = unit0; u < nunits; u += ustep) {
+        int kbase, nst;
+        pf_slice(a, u, npairs, kbase, nst);
+#pragma unroll 1
+        for (int c = 0; c < nst >> 2; c++, jj++) {
+          if ((jj & 1) != g) continue;
+#pragma unroll 1
+          for (int p = 0; p < NP; p++, it++) {
+            const int buf = 2 * g + (it & 1), di = it % ND, dbar = 2 * g + di;
+            const uint32_t D = db + (uint32_t)(di * N), A = ab + 64u * (uint32_t)(it & 1);
+            const int sl = (jj * SPB + p * SPB / NP) % NB, in = p * SI - (p * SPB / NP) * (4 / SPB);   // the item's slot of activations, its first 64-column part there
+            if (it >= ND) wait(d_empty(dbar), (uint32_t)((it / ND) - 1) & 1u);
+            if (in == 0) wait(b_full(sl), (uint32_t)(jj * SPB / NB) & 1u);
+            wait(a_full(buf), (uint32_t)(it >> 1) & 1u);
+            t5_fence_after();
+            const uint64_t bd = g3_desc(rb_s + sl * SLB + in * PLB, RU * 16, 128);
+            if (el) {
+              // (two planes: the smaller one first, while there is little for the additions to truncate)
+#pragma unroll
+              for (int pl = NPL - 1; pl >= 0; pl--)
+#pragma unroll
+                for (int k = 0; k < 4 * SI; k++)
+                  pt_mma(D, A + (uint32_t)(32 * pl + 8 * k), bd + (uint64_t)(k / 4 * (PLB / 16) + k % 4 * 2 * RU), px_idesc(N), k != 0 || pl != NPL - 1);
+              if (px_offs(FMT) && p == NP - 1) pf_mma_ss(D, oad, g3_desc(rb_s + sl * SLB + PX_SLOT, RU * 16, 128), px_idesc(N), 1u);
+              t5_commit_pair(a_empty(buf));
+              if (in + SI == 4 / SPB) t5_commit_pair(b_empty(sl));
+              t5_commit_pair(d_full(dbar));
+            }
+            __syncwarp();
+          }
+        }
+      }
+    }
+  } else {
+    // ---- accumulators into sums: lane quarter q, a weight row a thread; the two warps of a quarter have half of the prompt rows each ----
+    constexpr int RH = RU / 2;
+    const int q = warp & 3, half = (warp - 12) >> 2, R = a.R;
+    const uint32_t t0 = tmem + 256u + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * RH);
+    f32x2 acc[RH / 2];
+    const f32x2 inv = x2_pack(XP_LO_INV, XP_LO_INV);
+    int j0 = 0;
+    for (int u = unit0; u < nunits; u += ustep) {
+      int kbase, nst, m, row0;
+      pf_slice(a, u, npairs, kbase, nst);
+      const int nsl = nst >> 2;
+#pragma unroll
+      for (int j = 0; j < RH / 2; j++) acc[j] = 0;
+#pragma unroll 1
+      for (int k = 0; k < nsl * NP; k++) {
+        const int jj = j0 + k / NP, p = k % NP, g = jj & 1, it = (jj >> 1) * NP + p, di = it % ND, dbar = 2 * g + di;   // in the columns' order, as k_pfx1 adds them
+        if (p == 0) wait(sc_full(jj & 3), (uint32_t)(jj >> 2) & 1u);
+        const float scf = scr[(jj & 7) * 128 + 32 * q + lane];
+        const f32x2 sc = x2_pack(scf, scf);
+        const uint32_t t1 = t0 + (uint32_t)(128 * g + di * N);
+        wait(d_full(dbar), (uint32_t)(it / ND) & 1u);
+        t5_fence_after();
+#pragma unroll
+        for (int i0 = 0; i0 < RH; i0 += 16) {
+          f32x2 v[8], w[8];
+          t5_ld16x2(t1 + i0, v);
+          t5_ld16x2(t1 + RU + i0, w);
+          t5_wait_ld();
+          if (i0 + 16 == RH) {   // given back before the last of it are added up
+            t5_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(lead + (d_empty(dbar) - bar_s));
+          }
+#pragma unroll
+          for (int j = 0; j < 8; j++) acc[i0 / 2 + j] = x2_fma(sc, x2_fma(w[j], inv, v[j]), acc[i0 / 2 + j]);
+        }
+      }
+      j0 += nsl;
       const int tile = tile_of(u);
       pf_locate(a, min(tile, ntiles - 1), m, row0);
       const int row = row0 + 32 * q + lane, n = R - half * RH;   // this warp's prompt rows in use

@@ -1,4 +1,4 @@
-"""Prompts in mode 0 (llb_spec_set_prefill(0)): more than eight rows go through the dense path's exact forms in pieces of 128 rows, whole, without a
+"""Prompts in mode 0 (llb_spec_set_prefill(0)): more than four rows go through the dense path's exact forms in pieces of 128 rows, whole, without a
 T-row pass behind them.  Against T-row passes (LLB_PREFILL_ROWS) on the same model: state, K/V rows, the rows left for the drafter, logits of
 the last prompt row, ids; the same bits whatever k is and whether several streams' prompts are fed together or in turn."""
 import numpy as np
@@ -37,7 +37,7 @@ def _run(pkg, pack, mtp, k, prompt, last):
         eng.close()
 
 
-@pytest.mark.parametrize("n", [9, 10, 18, 41, 129, 130, 136, 137, 138, 260])   # rows at the edges of the rule, of units and of pieces (a last one under eight rows is not cut)
+@pytest.mark.parametrize("n", [5, 6, 9, 18, 41, 129, 130, 136, 137, 138, 260])   # rows at the edges of the rule, of units and of pieces (a last one under eight rows is not cut)
 def test_pieces_against_t_row_passes(pkg, packs, llb, monkeypatch, n):
     pack = packs.build_pack(packs.cfg_tiny(n_layers=4, seed=31, quant="q4_k_m"))
     mtp = packs.aux1_bytes(packs.build_mtp(pack))
@@ -61,7 +61,7 @@ def test_streams_together_and_in_turn(pkg, packs, llb):
     """Five prompts: two of several pieces, three that share a chunk with others, one in T-row passes, one of a single token."""
     pack = packs.build_pack(packs.cfg_tiny(n_layers=4, seed=32))
     mtp = packs.aux1_bytes(packs.build_mtp(pack))
-    lens = [40, 150, 9, 1, 261]
+    lens = [40, 150, 5, 1, 261]
     prompts = [packs.synth_prompt(200 + b, n, pack.cfg.vocab_size) for b, n in enumerate(lens)]
     out = []
     for together in (False, True):
