@@ -12,9 +12,9 @@
 //   output  O[d][q] += V_hi^T (P_hi + P_lo) + V_lo^T P_hi / 2048        warps split the head dimension
 // Per (query, slice) it leaves a running max, a sum and an unnormalised accumulator for k_attn_comb.
 // The scalar-FMA kernel this replaces spent 2400 warp instructions per 32 positions and warp; this one about 350.
-// A warp has 16 dims of the output: sixteen warps at head dimension 256, where shared memory leaves room for one block an SM
-// (with eight, a 256-row chunk's launch took 307 us at 1500 positions on the 27B shape, with sixteen 258).  A tile's phases
-// (scores, softmax, output) follow one another and their latencies are what bounds it: tensor pipe 30 %, shared memory 45 %.
+// A warp has 16 dims of the output: sixteen warps at head dimension 256, where shared memory leaves room for one block an SM.  A tile's
+// phases (scores, softmax, output) follow one another and their latencies are what bounds it: tensor pipe 30 %, shared memory 45 %.  The
+// rows of a prompt piece, where that would cost most, have pfatt.cuh.
 #include "host.cuh"
 #include "model.cuh"
 #include "rowops.cuh"
@@ -40,8 +40,7 @@ template <int HD, int NQG>
 __global__ void __launch_bounds__(2 * HD, HD > 128 ? 1 : 2) k_attn_mma(const float *__restrict__ q, const __half *__restrict__ Kc, const __half *__restrict__ Vc,
                                                   AttnShape sh, int Tmax, float *__restrict__ pm, float *__restrict__ pl,
                                                   float *__restrict__ po, const RowSet *rs) {
-  // blockIdx.z: one of several row groups -- the groups of a prompt chunk, which share a cache, or the streams of a pass,
-  // each with its own -- each with its own row set, Tmax query rows and partial results
+  // blockIdx.z: one of the streams of a pass, each with its own cache, row set, Tmax query rows and partial results
   {
     const size_t z = blockIdx.z, per = (size_t)sh.H * Tmax * gridDim.y;
     rs = (const RowSet *)((uintptr_t)rs + z * sh.rs_stride);
@@ -207,13 +206,12 @@ __global__ void __launch_bounds__(2 * HD, HD > 128 ? 1 : 2) k_attn_mma(const flo
 // (llb_attn4_combine + llb_t_ogq, tools/payload-sk8add.patch, tools/payload-spec2.patch:149-156)
 // block = (head, row); thread (sg, i4): split group sg, dims 4*i4 .. 4*i4+3
 __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm, const float *__restrict__ pl, const float *__restrict__ po, PartIn qg,
-                                                   AttnShape sh, int nsplit, int Tmax, XPlanes xp, const RowSet *rs, __half *__restrict__ kg, int kg_row0, int kg_ru) {
+                                                   AttnShape sh, int nsplit, int Tmax, XPlanes xp, const RowSet *rs) {
   {
     const size_t z = blockIdx.z, per = (size_t)sh.H * Tmax * nsplit;
     rs = (const RowSet *)((uintptr_t)rs + z * sh.rs_stride);
     pm += z * per; pl += z * per; po += z * per * sh.hd;
     qg.p += z * Tmax * 2 * sh.H * sh.hd;
-    kg_row0 += (int)z * Tmax;
   }
   const int xrow0 = blockIdx.z * Tmax;   // the group's rows in the planes
   int rs_n, rs_p0;
@@ -273,9 +271,7 @@ __global__ void __launch_bounds__(256) k_attn_comb(const float *__restrict__ pm,
     p_parts4(qg, (size_t)t * 2 * sh.H * hd + (size_t)h * 2 * hd + hd + 4 * i, gate);
     const float hv[4] = {(a.x / L) / (1.0f + expf(-gate.x)), (a.y / L) / (1.0f + expf(-gate.y)), (a.z / L) / (1.0f + expf(-gate.z)),
                          (a.w / L) / (1.0f + expf(-gate.w))};
-    // the prompt path takes the rows as fp16 in the dense GEMM's k-group-major order instead of the T-row planes
-    if (kg) pf_kg_store4(kg, sh.H * hd, kg_ru, kg_row0 + t, h * hd + 4 * i, hv[0], hv[1], hv[2], hv[3]);
-    else xp_store4(xp, xrow0 + t, 2, h * hd + 4 * i, hv, lane, true);
+    xp_store4(xp, xrow0 + t, 2, h * hd + 4 * i, hv, lane, true);
   }
 }
 
@@ -297,22 +293,8 @@ template <int HD> static int att_hd(cudaStream_t s, int nqg, dim3 grid, const fl
   return llb_fail("attention: %d queries per kv head", nqg * 8);
 }
 
-// K-slices of a prompt chunk's nz row groups: the fewest rounds of blocks, each as long as its slice's tiles plus about two for
-// the queries going in and the partial results coming out.  (With a decode pass's split, one wave for ONE group, a block had
-// two tiles to do and left 48 KB to merge: 92 ms of a 3011-token prompt on the 27B shape, 58 with one to eight slices.)
-int att_prompt_split(int KV, int hd, int nz, int total, int sms, int cap) {
-  const int slots = sms * (hd > 128 ? 1 : 2), tiles = (total + ATT_PT - 1) / ATT_PT;   // blocks on the chip at a time
-  int best = 1;
-  double best_cost = 1e30;
-  for (int ns = 1; ns <= cap && ns <= tiles; ns++) {
-    const double cost = (double)((KV * nz * ns + slots - 1) / slots) * ((tiles + ns - 1) / ns + 2.0);
-    if (cost < best_cost) { best_cost = cost; best = ns; }
-  }
-  return best;
-}
-
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,
-                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg, int kg_row0, int kg_ru, int nz) {
+                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, int nz) {
   const int G = sh.H / sh.KV, NQ = G * Tmax, nqg = (NQ + 7) / 8;
   dim3 grid(sh.KV, nsplit, nz);
   int rc;
@@ -321,7 +303,7 @@ int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *V
   else return llb_fail("attention: head_dim %d", sh.hd);
   if (rc) return rc;
   CU_OK(cudaGetLastError());
-  CU_OK(llb_launch(k_attn_comb, dim3(sh.H, Tmax, nz), dim3(256), (size_t)(0), s, pm, pl, po, qg, sh, nsplit, Tmax, xp, rs, kg, kg_row0, kg_ru));
+  CU_OK(llb_launch(k_attn_comb, dim3(sh.H, Tmax, nz), dim3(256), (size_t)(0), s, pm, pl, po, qg, sh, nsplit, Tmax, xp, rs));
   CU_OK(cudaGetLastError());
   return 0;
 }

@@ -578,7 +578,7 @@ static int enq_attn(llb_spec *m, const AttnW &w, float *Kc, float *Vc, const Row
                m->B > 1 ? (int)sizeof(SpecCtl) : 0, m->B > 1 ? m->kv_group : 0};
   PK("gemm qkv", site_gemm(m, {{&w.q, &m->b_q, nullptr, nullptr, 0}, {&w.k, &m->b_k, nullptr, nullptr, 0}, {&w.v, &m->b_v, nullptr, nullptr, 0}}, m->xp_d, 0));
   PK("qkrope", op_qkrope(s, as_in(m->b_q), as_in(m->b_k), as_in(m->b_v), w.qn, w.kn, m->invfreq, sh, m->qn, Kc, Vc, rs, m->Tmax));
-  PK("attention", op_attention(s, m->qn, Kc, Vc, as_in(m->b_q), sh, m->att_split, m->pm, m->pl, m->po, m->xp_qa, rs, m->per, nullptr, 0, 0, m->B));
+  PK("attention", op_attention(s, m->qn, Kc, Vc, as_in(m->b_q), sh, m->att_split, m->pm, m->pl, m->po, m->xp_qa, rs, m->per, m->B));
   PK("gemm attn_out", site_gemm(m, {{&w.o, &m->b_a, nullptr, nullptr, 0}}, m->xp_qa, 0));
   PK("all-reduce", tp_reduce(m, m->b_a, m->r_a));
   return 0;
@@ -1058,12 +1058,7 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
 
 // ---- the prompt path: chunks of up to PF_RMAX rows through dense tcgen05 GEMMs (pf.cu) ----------------------------
 #define PF_PIECES 16                           // most sequences in a chunk
-#define PF_GROUPS (PF_RMAX + 2 * PF_PIECES)
 static llb_spec *pf_owner(llb_spec *m) { return m->share ? m->share : m; }
-// rows of an attention group (at most 48 queries a kv head) and most K-slices: of the model alone, so that a prompt's sums do not depend on
-// how many streams its engine has
-static int pf_group(const llb_spec *m) { const int q = 48 / (m->H / m->KV); return q < 1 ? 1 : q < SPEC_MAXT ? q : SPEC_MAXT; }
-static int pf_split_cap(const llb_spec *m) { const int n = g_llb.sms / m->KV; return n < 1 ? 1 : n > 128 ? 128 : n; }
 static int pf_alloc(llb_spec *m) {
   llb_spec *o = pf_owner(m);
   PfState &f = o->pf;
@@ -1078,12 +1073,11 @@ static int pf_alloc(llb_spec *m) {
   f.decay = falloc(o, (size_t)PF_RMAX * m->TR); f.o = falloc(o, (size_t)PF_RMAX * m->vdc);
   f.kg_d = kg(d); f.kg_f = kg(m->f); f.kg_qa = kg(qa); f.kg_v = kg(m->vdc); f.kg_2d = kg(2 * d);
   {
-    const int gsz = pf_group(m);
-    const size_t ng = (PF_RMAX + gsz - 1) / gsz, per = (size_t)m->H * gsz * pf_split_cap(m);
-    f.pm = falloc(o, ng * per); f.pl = falloc(o, ng * per); f.po = falloc(o, ng * per * m->hd);
+    const size_t n = op_pf_attn_parts(m->H, m->KV);
+    f.pm = falloc(o, n); f.pl = falloc(o, n); f.po = falloc(o, n * m->hd);
     if (!f.pm || !f.pl || !f.po) return -1;
   }
-  f.rs = (RowSet *)dalloc(o, sizeof(RowSet) * PF_GROUPS);
+  f.rs = (RowSet *)dalloc(o, sizeof(RowSet) * PF_PIECES);
   f.ids = (int *)dalloc(o, (size_t)(PF_RMAX + 1) * 4);
   if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.gram || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
       !f.rs || !f.ids) return -1;
@@ -1166,18 +1160,16 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
   PfState &f = pf_owner(m)->pf;
   cudaStream_t s = g_llb.stream;
   StreamScope scope(m, true);   // the chunk's kernels see one stream: stream b's state is handed to them directly
-  const int d = m->d, qa = m->H * m->hd, kvd = m->KV * m->hd, gsz = pf_group(m);
+  const int d = m->d, qa = m->H * m->hd, kvd = m->KV * m->hd;
   int R = 0;
   std::vector<RowSet> rs;
-  std::vector<int> rs0, ids;
-  for (PfPiece &p : pc) {       // row sets: the piece's, then those of its attention groups
+  std::vector<int> ids;
+  for (PfPiece &p : pc) {
     p.off = R; R += p.R;
-    rs0.push_back((int)rs.size());
     RowSet r;
     memset(&r, 0, sizeof r);
     r.n = p.R; r.pos0 = p.p0;
     rs.push_back(r);
-    for (int g = 0; g < p.R; g += gsz) { r.n = p.R - g < gsz ? p.R - g : gsz; r.pos0 = p.p0 + g; rs.push_back(r); }
     ids.insert(ids.end(), p.ids + p.p0, p.ids + p.p0 + p.R);
   }
   const int ru = pf_unit_rows(R), np = (int)pc.size();
@@ -1197,10 +1189,8 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
         const PfPiece &p = pc[i];
         const PartIn q = pf_rows_of(f.q, 2 * qa, p.off);
         float *qn = f.qn + (size_t)p.off * qa, *kc = kc_of(m, m->Kc[il], p.b), *vc = kc_of(m, m->Vc[il], p.b);
-        const int ngrp = (p.R + gsz - 1) / gsz, nsp = att_prompt_split(m->KV, m->hd, ngrp, p.p0 + p.R, g_llb.sms, pf_split_cap(m));
-        PFK("qkrope", op_qkrope(s, q, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), l.at.qn, l.at.kn, m->invfreq, ash, qn, kc, vc, &f.rs[rs0[i]], p.R));
-        // every group of gsz rows in one launch (grid z): each streams the K/V rows up to its own last position
-        PFK("attention", op_attention(s, qn, kc, vc, q, ash, nsp, f.pm, f.pl, f.po, m->xp_qa, &f.rs[rs0[i] + 1], gsz, f.kg_qa, p.off, ru, ngrp));
+        PFK("qkrope", op_qkrope(s, q, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), l.at.qn, l.at.kn, m->invfreq, ash, qn, kc, vc, &f.rs[i], p.R));
+        PFK("attention", op_pf_attn(s, qn, kc, vc, q, ash, p.p0, p.R, f.pm, f.pl, f.po, f.kg_qa, p.off, ru));
       }
       PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
     } else {
@@ -1236,7 +1226,7 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
     for (int i = 0; i < np; i++) {
       const PfPiece &p = pc[i];
       const int rows = p.R - (pf_keep(m, p) - 1);   // the rest of a prompt is what the drafter catches up over
-      if (rows > 0) CK(op_qkrope(s, none, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), m->mt_at.qn, m->mt_at.kn, m->invfreq, ash, f.qn, kc_of(m, m->mt_Kc, p.b), kc_of(m, m->mt_Vc, p.b), &f.rs[rs0[i]], rows, true));
+      if (rows > 0) CK(op_qkrope(s, none, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), m->mt_at.qn, m->mt_at.kn, m->invfreq, ash, f.qn, kc_of(m, m->mt_Kc, p.b), kc_of(m, m->mt_Vc, p.b), &f.rs[i], rows, true));
     }
   }
   for (int i = 0; i < np; i++) {

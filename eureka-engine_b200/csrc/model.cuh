@@ -121,9 +121,8 @@ int op_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, c
 // kg != null: the gated rows go out as rows kg_row0 .. of a k-group-major chunk buffer with units of kg_ru rows (common.cuh) instead of the planes
 // nz > 1: that many consecutive groups of Tmax rows in one launch (rs, q, qg, pm / pl / po and the output rows advance
 // by one group per grid z)
-int att_prompt_split(int KV, int hd, int nz, int total, int sms, int cap);
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,
-                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, __half *kg = nullptr, int kg_row0 = 0, int kg_ru = 0, int nz = 1);
+                 float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, int nz = 1);
 // conv1d + gates + recurrent scan + gated norm -> planes.  S: the streams' state rings one after the other (s_group floats
 // apart); nz streams
 int op_delta(cudaStream_t s, float *S, const SpecCtl *ctl, PartIn ring, const float *cw, PartIn bp, PartIn ap, const float *dt, const float *sa,

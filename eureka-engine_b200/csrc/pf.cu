@@ -8,10 +8,13 @@
 // kernel with the state in registers, writing the state once.
 #include "pfmm.cuh"
 #include "pfx.cuh"
+#include "pfatt.cuh"
 #include "model.cuh"
 #include "pf.cuh"
 
 static unsigned int *g_pf_err = nullptr;   // device word: a bounded wait of k_pfmm ran out
+
+static decltype(&cuTensorMapEncodeTiled) g_tensor_map = nullptr;
 
 template <int FMT> static int pf_attr() {
   CU_OK(cudaFuncSetAttribute(k_pfmm<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
@@ -38,7 +41,13 @@ __global__ void k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl
 int pf_setup(void) {
   if (pf_attr<LLB_FM_Q6_K>() || pf_attr<LLB_FM_Q8_0>()) return -1;
   if (px_attr1<LLB_FM_Q4_K>() || px_attr1<LLB_FM_Q5_K>() || px_attr1<LLB_FM_Q6_K>() || px_attr1<LLB_FM_Q8_0>() || px_attr2<LLB_FM_Q4_K>() || px_attr2<LLB_FM_Q5_K>()) return -1;
+  if (px_attr(k_pf_attn<128>, pa_smem(128), PA_REG_LAUNCH) || px_attr(k_pf_attn<256>, pa_smem(256), PA_REG_LAUNCH)) return -1;
   CU_OK(cudaFuncSetAttribute(k_pf_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SCAN_SMEM - 24 * 1024));
+  if (!g_tensor_map) {
+    cudaDriverEntryPointQueryResult found;
+    CU_OK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&g_tensor_map, 12000, cudaEnableDefault, &found));
+    if (!g_tensor_map) return llb_fail("the driver has no cuTensorMapEncodeTiled");
+  }
   if (!g_pf_err) {
     CU_OK(cudaMalloc(&g_pf_err, 4));
     CU_OK(cudaMemset(g_pf_err, 0, 4));
@@ -207,6 +216,45 @@ __global__ void __launch_bounds__(256) k_pf_silu(PartIn g, PartIn u, int f, int 
 }
 int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R, int ru) {
   CU_OK(llb_launch(k_pf_silu, dim3((f / 4 + 255) / 256, R), dim3(256), (size_t)0, s, g, u, f, ru, kg));
+  return 0;
+}
+
+// ---- attention of a piece (pfatt.cuh) ---------------------------------------------------------------
+// Slices of the positions: the fewest rounds of blocks, each as long as its slice's tiles plus about five for the queries going in and the sums coming out.
+static int pa_pick(int blocks, int total) {
+  const int tiles = (total + 31) >> 5, sms = g_llb.sms;
+  int best = 1;
+  double best_cost = 1e30;
+  for (int ns = 1; ns <= tiles && (ns == 1 || blocks * ns <= 2 * sms); ns++) {
+    const double cost = (double)((blocks * ns + sms - 1) / sms) * ((tiles + ns - 1) / ns + 5.0);
+    if (cost < best_cost) { best_cost = cost; best = ns; }
+  }
+  return best;
+}
+// (head, row, slice) triples of the largest piece
+size_t op_pf_attn_parts(int H, int KV) {
+  const int most = KV * ((PF_RMAX * (H / KV) + 127) / 128);
+  return (size_t)128 * (most > 2 * g_llb.sms ? most : 2 * g_llb.sms);
+}
+// a layer's K or V rows of positions 0 .. total - 1, both planes: a box is 64 dims of 32 positions; what lies past the last is read as zeros
+static int pa_map(CUtensorMap *map, const float *base, AttnShape sh, int total) {
+  const cuuint64_t kvd = (cuuint64_t)sh.KV * sh.hd, dim[3] = {kvd, (cuuint64_t)total, 2}, step[2] = {kvd * 2, (cuuint64_t)sh.kv_plane * 2};
+  const cuuint32_t box[3] = {64, 32, 2}, one[3] = {1, 1, 1};
+  const CUresult r = g_tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void *)base, dim, step, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : llb_fail("attention: tensor map of %d positions: error %d", total, (int)r);
+}
+int op_pf_attn(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int p0, int R, float *pm, float *pl, float *po, __half *kg, int row0, int ru) {
+  const int tiles = (R * (sh.H / sh.KV) + 127) / 128, total = p0 + R;
+  const int want = pa_pick(sh.KV * tiles, total), per = ((total + 31) / 32 + want - 1) / want * 32, ns = (total + per - 1) / per;
+  const PaArgs a{q, sh.H, sh.KV, p0, R, per, pm, pl, po, g_pf_err};
+  CUtensorMap km, vm;
+  if (pa_map(&km, Kc, sh, total) || pa_map(&vm, Vc, sh, total)) return -1;
+  const dim3 grid(tiles, ns, sh.KV);
+  if (sh.hd == 128) CU_OK(llb_launch(k_pf_attn<128>, grid, dim3(PA_THREADS), (size_t)pa_smem(128), s, a, km, vm));
+  else if (sh.hd == 256) CU_OK(llb_launch(k_pf_attn<256>, grid, dim3(PA_THREADS), (size_t)pa_smem(256), s, a, km, vm));
+  else return llb_fail("attention: head_dim %d", sh.hd);
+  CU_OK(llb_launch(k_pf_attn_comb, dim3((R * sh.H + 7) / 8), dim3(256), (size_t)0, s, pm, pl, po, qg, sh.H, sh.hd, R, ns, kg, row0, ru));
   return 0;
 }
 
