@@ -41,7 +41,7 @@ struct LayerW { bool full = false; float *attn_norm = nullptr; AttnW at; DeltaW 
 struct TensorRec { uint64_t off, bytes; int rows, cols, fmt; bool blocked = false; };
 
 // Buffers of the prompt path (pf.cu), allocated at the first prompt that takes it: residual rows, fp16 activations in the
-// dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows, and the row sets of the chunk.  Nothing in them
+// dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows.  Nothing in them
 // outlives a prompt, so the engine that has the weights keeps them for its siblings too; a prompt holds them (`busy`) while it is enqueued,
 // and the library's one stream keeps the chunks of several prompts apart.
 struct PfState {
@@ -50,8 +50,7 @@ struct PfState {
   float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *gram = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
   __half *kg_d = nullptr, *kg_f = nullptr, *kg_qa = nullptr, *kg_v = nullptr, *kg_2d = nullptr;
   OutBuf q, k, v, qkv, z, bp, ap, a, g, u, dn, eh;
-  float *pm = nullptr, *pl = nullptr, *po = nullptr;   // split-K attention partials of every row group of a chunk
-  RowSet *rs = nullptr;    // [0] the whole chunk, [1 + i] its i-th group of attention rows
+  float *pm = nullptr, *pl = nullptr, *po = nullptr;   // attention's partial results of a piece's slices
   int *ids = nullptr;      // the chunk's tokens
 };
 
@@ -1077,10 +1076,9 @@ static int pf_alloc(llb_spec *m) {
     f.pm = falloc(o, n); f.pl = falloc(o, n); f.po = falloc(o, n * m->hd);
     if (!f.pm || !f.pl || !f.po) return -1;
   }
-  f.rs = (RowSet *)dalloc(o, sizeof(RowSet) * PF_PIECES);
   f.ids = (int *)dalloc(o, (size_t)(PF_RMAX + 1) * 4);
   if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.gram || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
-      !f.rs || !f.ids) return -1;
+      !f.ids) return -1;
   f.none = false; f.ready = true;
   return 0;
 }
@@ -1162,22 +1160,16 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
   StreamScope scope(m, true);   // the chunk's kernels see one stream: stream b's state is handed to them directly
   const int d = m->d, qa = m->H * m->hd, kvd = m->KV * m->hd;
   int R = 0;
-  std::vector<RowSet> rs;
   std::vector<int> ids;
   for (PfPiece &p : pc) {
     p.off = R; R += p.R;
-    RowSet r;
-    memset(&r, 0, sizeof r);
-    r.n = p.R; r.pos0 = p.p0;
-    rs.push_back(r);
     ids.insert(ids.end(), p.ids + p.p0, p.ids + p.p0 + p.R);
   }
   const int ru = pf_unit_rows(R), np = (int)pc.size();
-  CU_OK(cudaMemcpyAsync(f.rs, rs.data(), rs.size() * sizeof(RowSet), cudaMemcpyHostToDevice, s));
   CU_OK(cudaMemcpyAsync(f.ids, ids.data(), (size_t)R * 4, cudaMemcpyHostToDevice, s));
-  CU_OK(cudaStreamSynchronize(s));   // the sources are locals: the copies must have read them before they go
+  CU_OK(cudaStreamSynchronize(s));   // the source is a local: the copy must have read it before it goes
   PartIn none{nullptr, 0, 0};
-  AttnShape ash{m->H, m->KV, m->hd, m->rope_dim, m->eps, m->att_min, (long long)m->max_ctx * m->KV * m->hd, (int)sizeof(RowSet), 0};
+  AttnShape ash{m->H, m->KV, m->hd, m->rope_dim, m->eps, m->att_min, (long long)m->max_ctx * m->KV * m->hd, 0, 0};
   DeltaShape dsh{m->TR, m->GK, m->SZ, m->KC, m->convd, m->kdc, m->vdc, m->eps};
   PFK("embed", op_pf_embed(s, m->embd.fmt, m->embd.w, d, f.ids, R, f.x));
   for (int il = 0; il < m->L; il++) {
@@ -1189,7 +1181,7 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
         const PfPiece &p = pc[i];
         const PartIn q = pf_rows_of(f.q, 2 * qa, p.off);
         float *qn = f.qn + (size_t)p.off * qa, *kc = kc_of(m, m->Kc[il], p.b), *vc = kc_of(m, m->Vc[il], p.b);
-        PFK("qkrope", op_qkrope(s, q, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), l.at.qn, l.at.kn, m->invfreq, ash, qn, kc, vc, &f.rs[i], p.R));
+        PFK("qkrope", op_pf_qkrope(s, q, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), l.at.qn, l.at.kn, m->invfreq, ash, p.p0, p.R, qn, kc, vc));
         PFK("attention", op_pf_attn(s, qn, kc, vc, q, ash, p.p0, p.R, f.pm, f.pl, f.po, f.kg_qa, p.off, ru));
       }
       PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
@@ -1226,7 +1218,7 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
     for (int i = 0; i < np; i++) {
       const PfPiece &p = pc[i];
       const int rows = p.R - (pf_keep(m, p) - 1);   // the rest of a prompt is what the drafter catches up over
-      if (rows > 0) CK(op_qkrope(s, none, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), m->mt_at.qn, m->mt_at.kn, m->invfreq, ash, f.qn, kc_of(m, m->mt_Kc, p.b), kc_of(m, m->mt_Vc, p.b), &f.rs[i], rows, true));
+      if (rows > 0) CK(op_pf_qkrope(s, none, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), m->mt_at.qn, m->mt_at.kn, m->invfreq, ash, p.p0, rows, f.qn, kc_of(m, m->mt_Kc, p.b), kc_of(m, m->mt_Vc, p.b), true));
     }
   }
   for (int i = 0; i < np; i++) {

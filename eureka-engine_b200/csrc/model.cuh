@@ -115,11 +115,10 @@ int op_norm_xp(cudaStream_t s, const float *xin, PartIn add, const float *w, flo
 int op_silu_xp(cudaStream_t s, PartIn g, PartIn u, int f, XPlanes xp, const RowSet *rs, int Tmax);
 // router logits (ne rows + the shared gate row of Wr, F32) on the normed rows h[T][d]
 int op_moe_logits(cudaStream_t s, const float *Wr, const float *h, int d, int ne, float *lg, const RowSet *rs, int Tmax);
-// kv_only: only the K and V rows (the drafter's cache fill of the prompt path: no query rows)
+// kv_only: only the K and V rows (the drafter's cache fill of a prompt: no query rows)
 int op_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, const float *kn_w, const double *invfreq,
               AttnShape sh, float *qout, float *Kc, float *Vc, const RowSet *rs, int Tmax, bool kv_only = false);
-// kg != null: the gated rows go out as rows kg_row0 .. of a k-group-major chunk buffer with units of kg_ru rows (common.cuh) instead of the planes
-// nz > 1: that many consecutive groups of Tmax rows in one launch (rs, q, qg, pm / pl / po and the output rows advance
+// nz > 1: that many streams' groups of Tmax rows in one launch (rs, q, qg, pm / pl / po and the output rows advance
 // by one group per grid z)
 int op_attention(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int nsplit,
                  float *pm, float *pl, float *po, XPlanes xp, const RowSet *rs, int Tmax, int nz = 1);

@@ -219,6 +219,77 @@ int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R, int
   return 0;
 }
 
+// ---- per-head QK RMSNorm, partial NEOX RoPE, K and V rows into the cache (tools/qwen35_engine.c:523-533, 667-690) ----
+// A warp a (row, head), eight heads of a row a block: the query heads, then the key heads, then the value heads, from u0 on.  A row's angles are
+// computed once a block (in 64 bits, as the CPU engine does): with a block a head, as the passes of a few rows have it, they were most of a
+// launch, 36 us for 256 rows of 32 heads of 256.
+__global__ void __launch_bounds__(256) k_pf_qkrope(PartIn q, PartIn k, PartIn v, const float *__restrict__ qn_w, const float *__restrict__ kn_w, const double *__restrict__ invfreq,
+                                                   AttnShape sh, int p0, int u0, float *__restrict__ qout, __half *__restrict__ Kc, __half *__restrict__ Vc) {
+  __shared__ float cs[128], sn[128];
+  __shared__ __align__(16) float hv[8][256];
+  const int t = blockIdx.y, pos = p0 + t, wp = threadIdx.x >> 5, lane = threadIdx.x & 31, u = u0 + blockIdx.x * 8 + wp, hd = sh.hd, half = sh.rope_dim >> 1, kvd = sh.KV * hd;
+  pdl_trigger();
+  if (u0 + (int)blockIdx.x * 8 < sh.H + sh.KV) {   // (some head of the block turns)
+    const int i = threadIdx.x >> 1;
+    if (i < half) {
+      const double th = (double)(float)((double)pos * invfreq[i]);
+      if (threadIdx.x & 1) sn[i] = (float)sin(th);
+      else cs[i] = (float)cos(th);
+    }
+  }
+  __syncthreads();
+  pdl_wait();
+  if (u >= sh.H + 2 * sh.KV) return;
+  const int kind = u < sh.H ? 0 : u < sh.H + sh.KV ? 1 : 2, g = u - (kind == 0 ? 0 : kind == 1 ? sh.H : sh.H + sh.KV);
+  const PartIn &in = kind == 0 ? q : kind == 1 ? k : v;
+  const size_t at = kind == 0 ? (size_t)t * 2 * sh.H * hd + (size_t)g * 2 * hd : (size_t)t * kvd + g * hd;
+  float4 x[2];
+  float ss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    x[j] = 128 * j < hd ? part_get4(in, at + 128 * j + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    ss += x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
+  }
+  if (kind < 2) {
+    const float *w = kind ? kn_w : qn_w;
+    const float sc = 1.0f / sqrtf(pf_warp_sum(ss) / (float)hd + sh.eps);
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (128 * j < hd) {
+        const float4 n = *(const float4 *)(w + 128 * j + 4 * lane);
+        x[j].x = x[j].x * sc * n.x; x[j].y = x[j].y * sc * n.y; x[j].z = x[j].z * sc * n.z; x[j].w = x[j].w * sc * n.w;
+        *(float4 *)&hv[wp][128 * j + 4 * lane] = x[j];
+      }
+    __syncwarp();
+    for (int i = lane; i < half; i += 32) {
+      const float a = hv[wp][i], b = hv[wp][i + half], c = cs[i], s = sn[i];
+      hv[wp][i] = __fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s));
+      hv[wp][i + half] = __fadd_rn(__fmul_rn(a, s), __fmul_rn(b, c));
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    if (128 * j < hd) {
+      const int c = 128 * j + 4 * lane;
+      if (kind < 2) x[j] = *(const float4 *)&hv[wp][c];
+      if (kind == 0) { *(float4 *)(qout + ((size_t)t * sh.H + g) * hd + c) = x[j]; continue; }
+      __half *dst = (kind == 1 ? Kc : Vc) + (size_t)pos * kvd + g * hd + c;
+      const __half2 a = __floats2half2_rn(x[j].x, x[j].y), b = __floats2half2_rn(x[j].z, x[j].w);
+      const float2 af = __half22float2(a), bf = __half22float2(b);
+      const __half2 al = __floats2half2_rn((x[j].x - af.x) * XP_LO_SCALE, (x[j].y - af.y) * XP_LO_SCALE), bl = __floats2half2_rn((x[j].z - bf.x) * XP_LO_SCALE, (x[j].w - bf.y) * XP_LO_SCALE);
+      *(uint2 *)dst = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
+      *(uint2 *)(dst + sh.kv_plane) = make_uint2(*(const uint32_t *)&al, *(const uint32_t *)&bl);
+    }
+}
+// kv_only: only the K and V rows (the drafter's cache fill: no query rows)
+int op_pf_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, const float *kn_w, const double *invfreq, AttnShape sh, int p0, int R, float *qout, float *Kc, float *Vc, bool kv_only) {
+  if (sh.hd != 128 && sh.hd != 256) return llb_fail("attention: head_dim %d", sh.hd);
+  const int u0 = kv_only ? sh.H : 0;
+  CU_OK(llb_launch(k_pf_qkrope, dim3((sh.H + 2 * sh.KV - u0 + 7) / 8, R), dim3(256), (size_t)0, s, q, k, v, qn_w, kn_w, invfreq, sh, p0, u0, qout, (__half *)Kc, (__half *)Vc));
+  return 0;
+}
+
 // ---- attention of a piece (pfatt.cuh) ---------------------------------------------------------------
 // Slices of the positions: the fewest rounds of blocks, each as long as its slice's tiles plus about five for the queries going in and the sums coming out.
 static int pa_pick(int blocks, int total) {

@@ -27,6 +27,7 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a);  // fills the tile table; a.ksp
 int op_pf_embed(cudaStream_t s, int fmt, const uint8_t *W, int d, const int *ids, int R, float *x);
 int op_pf_norm(cudaStream_t s, const float *xin, PartIn add, const float *w, float eps, int d, float *xout, __half *kg, int kg_K, int kg_col0, float *hn_out, int R, int ru, int row0 = 0);   // rows row0 .. of kg, whose units have ru rows
 int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R, int ru);
+int op_pf_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, const float *kn_w, const double *invfreq, AttnShape sh, int p0, int R, float *qout, float *Kc, float *Vc, bool kv_only = false);
 size_t op_pf_attn_parts(int H, int KV);           // values of pm and pl; po has head_dim as many
 int op_pf_attn(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int p0, int R, float *pm, float *pl, float *po, __half *kg, int row0, int ru);
 int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, float *ring, int ring_ks, const float *cw, const float *dt, const float *sa,
