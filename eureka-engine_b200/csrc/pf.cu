@@ -480,15 +480,17 @@ __global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const 
 //     S      <- d[0, 7] S + sum_s d(s, 7] delta_s k_s
 // so the sixteen dot products of a state row with S run side by side, their sums over the sixteen lanes are one exchange
 // tree (64 values, 60 shuffles) that leaves row t's sums of two state rows in a lane, and the chain is the substitution: eight
-// steps of a shuffle (which hands every lane delta_s for the update) and a multiply-add.  The decays' products never
+// steps of a shuffle and a multiply-add; the update's deltas come by shuffles that wait for nothing.  The decays' products never
 // divide, so a decay of nearly zero does no harm.  Multiply-adds: three a state element and row instead of four, two an
 // instruction.  Sixteen lanes a state row, not eight: the loads of q and k, which every state row repeats, were the longer
 // part of a step with eight (shared memory: 66 us a chunk of the 48-head shape against 48).  What bounds it now is one warp's
-// chain: 580 instructions a step in 2500 cycles.  The ops between a DeltaNet layer's GEMMs, before and now: 84.5 -> 55 ms of a
+// chain: 960 instructions a step in 2300 cycles.  A lane takes its state rows and the step's rows in the order of its own lane bits (row
+// t ^ tq for t), which spares the exchange its selections, 150 instructions a step, and lets the update's k stay in registers: 45 -> 40 us a
+// chunk of 256 rows.  The ops between a DeltaNet layer's GEMMs, before and now: 84.5 -> 55 ms of a
 // 3011-token prompt (48 layers, 48 heads), 47 -> 28 ms of 4096 tokens (24 layers, 32 heads), 23 -> 9.7 ms of 2000 tokens (18
 // layers, 8 heads).
 // Rows come through double-buffered shared memory, the next eight requested before the present ones are computed.
-__global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
+__global__ void __launch_bounds__(32 * PF_SCAN_NW, 2) k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
                                                      const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R) {
   constexpr int NT = 32 * PF_SCAN_NW, NJ = 8 * PF_SCAN_NW, VS = NJ + 4;   // a block's threads and state rows; v rows padded so that eight lanes' reads miss one another's banks
   __shared__ __align__(16) float qs[2][PF_CH][128], ks[2][PF_CH][128], vs[2][PF_CH][VS], gs[2][PF_GRAM], bs[2][PF_CH], ds[2][PF_CH];
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__
 #pragma unroll
   for (int r = 0; r < 4; r++)
 #pragma unroll
-    for (int i = 0; i < 2; i++) { const float4 v = __ldcg(Sp + 32 * r + 16 * i); st[r][2 * i] = x2_pack(v.x, v.y); st[r][2 * i + 1] = x2_pack(v.z, v.w); }
+    for (int i = 0; i < 2; i++) { const float4 v = __ldcg(Sp + 32 * (r ^ 2 * rh) + 16 * i); st[r][2 * i] = x2_pack(v.x, v.y); st[r][2 * i + 1] = x2_pack(v.z, v.w); }
   pdl_wait();
   const int nb = (R + PF_CH - 1) / PF_CH;
   auto stage = [&](int b) {   // rows past the chunk repeat its last one; their beta counts as zero and their decay as one
@@ -529,35 +531,34 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__
     __syncthreads();   // the present rows are there, and nobody reads the buffer of the next ones any more
     if (b + 1 < nb) stage(b + 1);
     cp_async_commit();
-    f32x2 k[PF_CH][4];
+    f32x2 kk[PF_CH][4];
     float kv[4][PF_CH], qv[4][PF_CH];
 #pragma unroll
-    for (int t = 0; t < PF_CH; t++) {
-      f32x2 q[4];
+    for (int t = 0; t < PF_CH; t++) {   // row t ^ tq
+      f32x2 (&k)[4] = kk[t], q[4];
 #pragma unroll
       for (int i = 0; i < 2; i++) {
-        const ulonglong2 a = *(const ulonglong2 *)&ks[buf][t][64 * i + 4 * cq], c = *(const ulonglong2 *)&qs[buf][t][64 * i + 4 * cq];
-        k[t][2 * i] = a.x; k[t][2 * i + 1] = a.y; q[2 * i] = c.x; q[2 * i + 1] = c.y;
+        const ulonglong2 a = *(const ulonglong2 *)&ks[buf][t ^ tq][64 * i + 4 * cq], c = *(const ulonglong2 *)&qs[buf][t ^ tq][64 * i + 4 * cq];
+        k[2 * i] = a.x; k[2 * i + 1] = a.y; q[2 * i] = c.x; q[2 * i + 1] = c.y;
       }
 #pragma unroll
       for (int r = 0; r < 4; r++) {
-        f32x2 a = x2_mul(st[r][0], k[t][0]), c = x2_mul(st[r][0], q[0]);
+        f32x2 a = x2_mul(st[r][0], k[0]), c = x2_mul(st[r][0], q[0]);
 #pragma unroll
-        for (int i = 1; i < 4; i++) { a = x2_fma(st[r][i], k[t][i], a); c = x2_fma(st[r][i], q[i], c); }
+        for (int i = 1; i < 4; i++) { a = x2_fma(st[r][i], k[i], a); c = x2_fma(st[r][i], q[i], c); }
         float lo, hi;
         x2_unpack(a, lo, hi); kv[r][t] = lo + hi;
         x2_unpack(c, lo, hi); qv[r][t] = lo + hi;
       }
     }
-    // the exchange over lane bit 3 keeps two of the four state rows, those over bits 2 .. 0 row t of the eight
+    // the exchange over lane bit 3 keeps two of the four state rows, those over bits 2 .. 0 row tq of the eight: with a lane's state rows and
+    // rows of the step in the order of its own bits it keeps the first half of its values each time, and its partner's second half is the same rows'
 #pragma unroll
     for (int r = 0; r < 2; r++)
 #pragma unroll
       for (int t = 0; t < PF_CH; t++) {
-        const float kk = rh ? kv[r + 2][t] : kv[r][t], sk = rh ? kv[r][t] : kv[r + 2][t];
-        const float kq = rh ? qv[r + 2][t] : qv[r][t], sq = rh ? qv[r][t] : qv[r + 2][t];
-        kv[r][t] = kk + __shfl_xor_sync(0xffffffffu, sk, 8);
-        qv[r][t] = kq + __shfl_xor_sync(0xffffffffu, sq, 8);
+        kv[r][t] += __shfl_xor_sync(0xffffffffu, kv[r + 2][t], 8);
+        qv[r][t] += __shfl_xor_sync(0xffffffffu, qv[r + 2][t], 8);
       }
 #pragma unroll
     for (int m = 4; m > 0; m >>= 1)
@@ -565,10 +566,8 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__
       for (int i = 0; i < m; i++)
 #pragma unroll
         for (int r = 0; r < 2; r++) {
-          const float kk = tq & m ? kv[r][i + m] : kv[r][i], sk = tq & m ? kv[r][i] : kv[r][i + m];
-          const float kq = tq & m ? qv[r][i + m] : qv[r][i], sq = tq & m ? qv[r][i] : qv[r][i + m];
-          kv[r][i] = kk + __shfl_xor_sync(0xffffffffu, sk, m);
-          qv[r][i] = kq + __shfl_xor_sync(0xffffffffu, sq, m);
+          kv[r][i] += __shfl_xor_sync(0xffffffffu, kv[r][i + m], m);
+          qv[r][i] += __shfl_xor_sync(0xffffffffu, qv[r][i + m], m);
         }
     // lane tq is row t = tq from here on
     float dec[PF_CH], M[PF_CH], N[PF_CH], e[PF_CH];
@@ -596,20 +595,26 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__
       for (int i = 0; i < 4; i++) st[r][i] = x2_mul(st[r][i], pp);
 #pragma unroll
     for (int s = 0; s < PF_CH; s++) {
-      float d[4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) d[r] = __shfl_sync(0xffffffffu, x[r & 1], s + 8 * (r >> 1), 16);
+      float d[2];
 #pragma unroll
       for (int r = 0; r < 2; r++) {
-        const float dr = rh ? d[r + 2] : d[r];
-        x[r] -= M[s] * dr;
-        ov[r] += N[s] * dr;
+        d[r] = __shfl_sync(0xffffffffu, x[r], s, 8);
+        x[r] -= M[s] * d[r];
+        ov[r] += N[s] * d[r];
       }
+    }
+    float et = 1.0f;
+#pragma unroll
+    for (int s = 0; s < PF_CH; s++) et = s == tq ? e[s] : et;
+    x[0] *= et; x[1] *= et;
+#pragma unroll
+    for (int s = 0; s < PF_CH; s++) {   // row s ^ tq
 #pragma unroll
       for (int r = 0; r < 4; r++) {
-        const f32x2 d2 = x2_pack(e[s] * d[r], e[s] * d[r]);
+        const float d = s == 0 && r < 2 ? x[r] : __shfl_xor_sync(0xffffffffu, x[r & 1], s + 8 * (r >> 1));
+        const f32x2 d2 = x2_pack(d, d);
 #pragma unroll
-        for (int i = 0; i < 4; i++) st[r][i] = x2_fma(k[s][i], d2, st[r][i]);
+        for (int i = 0; i < 4; i++) st[r][i] = x2_fma(kk[s][i], d2, st[r][i]);
       }
     }
     if (tq < n) *(float2 *)(op + (size_t)(b * PF_CH + tq) * sh.vdc) = make_float2(ov[0], ov[1]);
@@ -620,7 +625,7 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW) k_pf_scan(float *__restrict__
     for (int i = 0; i < 2; i++) {
       float4 v;
       x2_unpack(st[r][2 * i], v.x, v.y); x2_unpack(st[r][2 * i + 1], v.z, v.w);
-      Sp[32 * r + 16 * i] = v;
+      Sp[32 * (r ^ 2 * rh) + 16 * i] = v;
     }
 }
 // gated RMSNorm of each head's output -> activations of ssm_out (:648-654); a warp per (head, row), eight rows a block.  One more
