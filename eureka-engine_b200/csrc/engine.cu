@@ -1056,7 +1056,6 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
 }
 
 // ---- the prompt path: chunks of up to PF_RMAX rows through dense tcgen05 GEMMs (pf.cu) ----------------------------
-#define PF_PIECES 16                           // most sequences in a chunk
 static llb_spec *pf_owner(llb_spec *m) { return m->share ? m->share : m; }
 static int pf_alloc(llb_spec *m) {
   llb_spec *o = pf_owner(m);
@@ -1068,8 +1067,8 @@ static int pf_alloc(llb_spec *m) {
   const int d = m->d, qa = m->H * m->hd;
   auto kg = [&](int K) { return (__half *)dalloc(o, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
   f.x = falloc(o, (size_t)PF_RMAX * d); f.x1 = falloc(o, (size_t)PF_RMAX * d); f.hn = falloc(o, (size_t)(PF_RMAX + PF_PIECES) * d); f.e = falloc(o, (size_t)PF_RMAX * d);
-  f.qn = falloc(o, (size_t)PF_RMAX * qa); f.y = falloc(o, (size_t)PF_RMAX * m->convd); f.beta = falloc(o, (size_t)PF_RMAX * m->TR); f.gram = falloc(o, (size_t)PF_RMAX / 8 * 64 * m->GK);
-  f.decay = falloc(o, (size_t)PF_RMAX * m->TR); f.o = falloc(o, (size_t)PF_RMAX * m->vdc);
+  f.qn = falloc(o, (size_t)PF_RMAX * qa); f.y = falloc(o, (size_t)PF_RMAX * m->convd); f.beta = falloc(o, (size_t)PF_STEPS * 8 * m->TR); f.gram = falloc(o, (size_t)PF_STEPS * 64 * m->GK);
+  f.decay = falloc(o, (size_t)PF_STEPS * 8 * m->TR); f.o = falloc(o, (size_t)PF_RMAX * m->vdc);
   f.kg_d = kg(d); f.kg_f = kg(m->f); f.kg_qa = kg(qa); f.kg_v = kg(m->vdc); f.kg_2d = kg(2 * d);
   {
     const size_t n = op_pf_attn_parts(m->H, m->KV);
@@ -1187,10 +1186,10 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
       PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
     } else {
       PFK("gemm qkv|z|b|a", pf_site(m, {{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));
-      for (const PfPiece &p : pc)
-        PFK("delta", op_pf_delta(s, pf_rows_of(f.qkv, m->convd, p.off), pf_rows_of(f.z, m->vdc, p.off), pf_rows_of(f.bp, m->TR, p.off), pf_rows_of(f.ap, m->TR, p.off),
-                       ring_of(m, il, p.b), m->ring_ks[il], l.dn.conv, l.dn.dt, l.dn.a, l.dn.norm, dsh,
-                       state_of(m, il, p.b), ctl_of(m, p.b), f.y, f.gram, f.beta, f.decay, f.o, f.kg_v, p.p0, p.R, p.off, ru));
+      PfSegs sg{};
+      sg.n = np;
+      for (int i = 0; i < np; i++) sg.s[i] = PfSeg{pc[i].p0, pc[i].R, pc[i].off, ring_of(m, il, pc[i].b), state_of(m, il, pc[i].b), ctl_of(m, pc[i].b)};
+      PFK("delta", op_pf_delta(s, as_in(f.qkv), as_in(f.z), as_in(f.bp), as_in(f.ap), m->ring_ks[il], l.dn.conv, l.dn.dt, l.dn.a, l.dn.norm, dsh, sg, f.y, f.gram, f.beta, f.decay, f.o, f.kg_v, ru));
       PFK("gemm ssm_out", pf_site(m, {{&l.dn.out, &f.a}}, f.kg_v, m->vdc, R));
     }
     PFK("norm", op_pf_norm(s, f.x, as_in(f.a), l.ffn.post, m->eps, d, f.x1, f.kg_d, d, 0, nullptr, R, ru));

@@ -36,8 +36,8 @@ template <int FMT> static int px_attr2() { return px_attr(k_pfx2<FMT>, px2_smem(
 #define PF_SCAN_NW 4                            // warps of a scan block, 8 state rows each
 #define PF_SCAN_BLOCKS (128 / (8 * PF_SCAN_NW)) // blocks of a head
 #define PF_SCAN_SMEM (220 * 1024)
-__global__ void k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
-                          const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R);
+__global__ void k_pf_scan(const PfSegs sg, const float *__restrict__ y, const float *__restrict__ gram, const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh,
+                          float *__restrict__ o);
 int pf_setup(void) {
   if (pf_attr<LLB_FM_Q6_K>() || pf_attr<LLB_FM_Q8_0>()) return -1;
   if (px_attr1<LLB_FM_Q4_K>() || px_attr1<LLB_FM_Q5_K>() || px_attr1<LLB_FM_Q6_K>() || px_attr1<LLB_FM_Q8_0>() || px_attr2<LLB_FM_Q4_K>() || px_attr2<LLB_FM_Q5_K>()) return -1;
@@ -330,6 +330,8 @@ int op_pf_attn(cudaStream_t s, const float *q, const float *Kc, const float *Vc,
 }
 
 // ---- gated DeltaNet over a chunk (tools/qwen35_engine.c:581-662) -----------------------------------
+// A chunk's sequences go through together, a step of eight rows of one of them at a time (four prompts of 25 to 40 tokens, 48 layers of 48
+// heads: 5.7 ms in turn, 2.6 together).
 // What the scan needs, one launch: a warp takes one unit of eight rows.
 //   q or k group   conv1d + SiLU of its columns, then q / max(|q|, eps) / sqrt(128) or k / max(|k|, eps) (no eps inside the root,
 //                  :613-620).  A group's two warps share a block: k passes through shared memory, the k warp makes the rows'
@@ -394,11 +396,16 @@ __device__ __forceinline__ float pf_lane_sums(float (&v)[32], int lane) {
   return v[0];
 }
 template <int MT>
-__global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const float *__restrict__ cw, PartIn bp, PartIn ap, const float *__restrict__ dt,
-                                                 const float *__restrict__ sa, DeltaShape sh, int p0, int R, float *__restrict__ y, float *__restrict__ gram,
+__global__ void __launch_bounds__(128) k_pf_conv(const PfSegs sg, PartIn qkv, int ring_ks, const float *__restrict__ cw, PartIn bp, PartIn ap, const float *__restrict__ dt,
+                                                 const float *__restrict__ sa, DeltaShape sh, float *__restrict__ y, float *__restrict__ gram,
                                                  float *__restrict__ beta, float *__restrict__ decay) {
   __shared__ __align__(16) float kx[2][PF_CH][128];
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, t0 = blockIdx.y * PF_CH, nqk = (sh.GK + 1) / 2, nv = (sh.TR + 3) / 4;
+  int si = 0, t0 = blockIdx.y * PF_CH;   // the sequence whose step this is, and the step's first row of it
+  for (; t0 >= sg.s[si].R; si++) t0 -= (sg.s[si].R + PF_CH - 1) / PF_CH * PF_CH;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, p0 = sg.s[si].p0, R = sg.s[si].R, nqk = (sh.GK + 1) / 2, nv = (sh.TR + 3) / 4;
+  const PartIn ring{sg.s[si].ring, ring_ks, (long long)CONV_RING * sh.convd};
+  const size_t off = sg.s[si].off;
+  qkv.p += off * sh.convd; y += off * sh.convd; bp.p += off * sh.TR; ap.p += off * sh.TR;
   int bx = blockIdx.x;
   pdl_trigger();
   pdl_wait();
@@ -417,7 +424,7 @@ __global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const 
       if (isk) *(float4 *)&kx[wp & 1][t][4 * lane] = x[t];
     }
     __syncthreads();
-    float *G = gram + ((size_t)g * (PF_RMAX / PF_CH) + blockIdx.y) * PF_GRAM;
+    float *G = gram + ((size_t)g * PF_STEPS + blockIdx.y) * PF_GRAM;
     float v[32];
     if (isk) {
 #pragma unroll
@@ -461,13 +468,13 @@ __global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const 
       if (t0 + t < R) *(float4 *)(y + (size_t)(t0 + t) * sh.convd + c) = v[t];
     return;
   }
-  const int i = (bx - nv) * 128 + threadIdx.x, t = t0 + i / sh.TR, h = i % sh.TR;
+  const int i = (bx - nv) * 128 + threadIdx.x, t = t0 + i / sh.TR, h = i % sh.TR, at = h * (PF_STEPS * PF_CH) + blockIdx.y * PF_CH + i / sh.TR;
   if (i >= PF_CH * sh.TR || t >= R) return;
   const float b = part_get(bp, (size_t)t * sh.TR + h), a = part_get(ap, (size_t)t * sh.TR + h);
-  beta[h * PF_RMAX + t] = 1.0f / (1.0f + (float)exp((double)-b));
+  beta[at] = 1.0f / (1.0f + (float)exp((double)-b));
   const float x = a + dt[h];
   const float sp = x > 20.0f ? x : (float)log1p((double)(float)exp((double)(x < 88.0f ? x : 88.0f)));
-  decay[h * PF_RMAX + t] = (float)exp((double)(sp * sa[h]));
+  decay[at] = (float)exp((double)(sp * sa[h]));
 }
 // The recurrence over the chunk's R rows.  Block (hh, y) keeps 32 state rows of value head hh in registers from the first
 // row of the chunk to the last and writes them back once (a lane: four state rows, columns 4 cq .. and 64 + 4 cq ..).
@@ -490,14 +497,19 @@ __global__ void __launch_bounds__(128) k_pf_conv(PartIn qkv, PartIn ring, const 
 // 3011-token prompt (48 layers, 48 heads), 47 -> 28 ms of 4096 tokens (24 layers, 32 heads), 23 -> 9.7 ms of 2000 tokens (18
 // layers, 8 heads).
 // Rows come through double-buffered shared memory, the next eight requested before the present ones are computed.
-__global__ void __launch_bounds__(32 * PF_SCAN_NW, 2) k_pf_scan(float *__restrict__ S, const SpecCtl *__restrict__ ctl, const float *__restrict__ y, const float *__restrict__ gram,
-                                                     const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh, float *__restrict__ o, int R) {
+__global__ void __launch_bounds__(32 * PF_SCAN_NW, 2) k_pf_scan(const PfSegs sg, const float *__restrict__ y, const float *__restrict__ gram, const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh,
+                                                     float *__restrict__ o) {
   constexpr int NT = 32 * PF_SCAN_NW, NJ = 8 * PF_SCAN_NW, VS = NJ + 4;   // a block's threads and state rows; v rows padded so that eight lanes' reads miss one another's banks
   __shared__ __align__(16) float qs[2][PF_CH][128], ks[2][PF_CH][128], vs[2][PF_CH][VS], gs[2][PF_GRAM], bs[2][PF_CH], ds[2][PF_CH];
   const int hh = blockIdx.x, jq = blockIdx.y, tid = threadIdx.x, g = hh % sh.GK, jg = tid >> 4, cq = tid & 15, tq = tid & 7, rh = (tid >> 3) & 1;
+  const PfSeg &me = sg.s[blockIdx.z];
+  const int R = me.R;
+  int step0 = 0;                          // its first step of the chunk's
+  for (int i = 0; i < (int)blockIdx.z; i++) step0 += (sg.s[i].R + PF_CH - 1) / PF_CH;
+  y += (size_t)me.off * sh.convd; o += (size_t)me.off * sh.vdc;
   pdl_trigger();
   const size_t head_sz = 128 * 128, slot_sz = (size_t)sh.TR * head_sz;
-  float4 *Sp = (float4 *)(S + (size_t)(*(const volatile int *)&ctl->sc) * slot_sz + (size_t)hh * head_sz + (size_t)(NJ * jq + 4 * jg) * 128 + 4 * cq);   // the committed slot: stable during the pass
+  float4 *Sp = (float4 *)(me.S + (size_t)(*(const volatile int *)&me.ctl->sc) * slot_sz + (size_t)hh * head_sz + (size_t)(NJ * jq + 4 * jg) * 128 + 4 * cq);   // the committed slot: stable during the pass
   f32x2 st[4][4];
 #pragma unroll
   for (int r = 0; r < 4; r++)
@@ -518,9 +530,9 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW, 2) k_pf_scan(float *__restric
       const int r = i / (NJ / 4), c = 4 * (i % (NJ / 4));
       cp_async16(smem_u32(&vs[buf][r][c]), y + (size_t)min(b * PF_CH + r, R - 1) * sh.convd + 2 * sh.kdc + hh * 128 + NJ * jq + c);
     }
-    if (tid < PF_GRAM / 4) cp_async16(smem_u32(&gs[buf][4 * tid]), gram + ((size_t)g * (PF_RMAX / PF_CH) + b) * PF_GRAM + 4 * tid);
-    else if (tid < PF_GRAM / 4 + 2) cp_async16(smem_u32(&bs[buf][4 * (tid & 1)]), beta + hh * PF_RMAX + b * PF_CH + 4 * (tid & 1));
-    else if (tid < PF_GRAM / 4 + 4) cp_async16(smem_u32(&ds[buf][4 * (tid & 1)]), decay + hh * PF_RMAX + b * PF_CH + 4 * (tid & 1));
+    if (tid < PF_GRAM / 4) cp_async16(smem_u32(&gs[buf][4 * tid]), gram + ((size_t)g * PF_STEPS + step0 + b) * PF_GRAM + 4 * tid);
+    else if (tid < PF_GRAM / 4 + 2) cp_async16(smem_u32(&bs[buf][4 * (tid & 1)]), beta + (hh * PF_STEPS + step0 + b) * PF_CH + 4 * (tid & 1));
+    else if (tid < PF_GRAM / 4 + 4) cp_async16(smem_u32(&ds[buf][4 * (tid & 1)]), decay + (hh * PF_STEPS + step0 + b) * PF_CH + 4 * (tid & 1));
   };
   stage(0);
   cp_async_commit();
@@ -632,43 +644,46 @@ __global__ void __launch_bounds__(32 * PF_SCAN_NW, 2) k_pf_scan(float *__restric
 // block a head copies the chunk's last raw rows into the conv history: whole values into K-slice 0, zeros into the rest
 // (here, because the conv kernel's first rows still read the old history).
 __global__ void __launch_bounds__(256) k_pf_gnorm(const float *__restrict__ o, PartIn z, const float *__restrict__ nw, DeltaShape sh, __half *__restrict__ kg,
-                                                  PartIn qkv, float *__restrict__ ring, int ring_ks, int p0, int R, int row0, int ru) {
+                                                  PartIn qkv, int ring_ks, const PfSegs sg, int ru) {
+  const int p0 = sg.s[blockIdx.z].p0, R = sg.s[blockIdx.z].R, row0 = sg.s[blockIdx.z].off;
+  float *ring = sg.s[blockIdx.z].ring;
   const int hh = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5), i = threadIdx.x & 31;
   const float4 w = __ldg((const float4 *)(nw + 4 * i));
   pdl_trigger();
   pdl_wait();
-  if (blockIdx.y == gridDim.y - 1) {
+  if (8 * (int)blockIdx.y >= R) {
+    if (8 * (int)blockIdx.y >= R + 8) return;   // (another sequence has more rows)
     const int nr = min(R, CONV_RING), nc = sh.convd / 4;
     for (int j = hh * 256 + threadIdx.x; j < nr * nc; j += sh.TR * 256) {
       const int tr = R - nr + j / nc, c = 4 * (j % nc);
       const size_t dst = (size_t)((p0 + tr) & (CONV_RING - 1)) * sh.convd + c;
-      *(float4 *)(ring + dst) = part_get4(qkv, (size_t)tr * sh.convd + c);
+      *(float4 *)(ring + dst) = part_get4(qkv, (size_t)(row0 + tr) * sh.convd + c);
       for (int k = 1; k < ring_ks; k++) *(float4 *)(ring + (size_t)k * CONV_RING * sh.convd + dst) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     return;
   }
   if (t >= R) return;
-  const size_t idx = (size_t)t * sh.vdc + hh * 128 + 4 * i;
+  const size_t idx = (size_t)(row0 + t) * sh.vdc + hh * 128 + 4 * i;
   const float4 v = __ldcg((const float4 *)(o + idx)), zz = part_get4(z, idx);
   const float r = 1.0f / sqrtf(pf_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) / 128.0f + sh.eps);
   pf_kg_store4(kg, sh.vdc, ru, row0 + t, hh * 128 + 4 * i, v.x * r * w.x * pf_silu(zz.x), v.y * r * w.y * pf_silu(zz.y), v.z * r * w.z * pf_silu(zz.z), v.w * r * w.w * pf_silu(zz.w));
 }
 
 // One DeltaNet layer's ops between its input GEMM (qkv | z | beta | alpha) and its output GEMM, for R rows at p0 ...
-int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, float *ring, int ring_ks, const float *cw, const float *dt, const float *sa,
-                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int p0, int R, int row0, int ru) {
+int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, int ring_ks, const float *cw, const float *dt, const float *sa,
+                const float *nw, DeltaShape sh, const PfSegs &sg, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int ru) {
   if (sh.SZ != 128 || sh.KC > CONV_RING / 2) return llb_fail("pf delta: state size %d, conv kernel %d", sh.SZ, sh.KC);
-  const long long rstride = (long long)CONV_RING * sh.convd;
-  const dim3 cgrid((sh.GK + 1) / 2 + (sh.TR + 3) / 4 + (PF_CH * sh.TR + 127) / 128, (R + PF_CH - 1) / PF_CH);
-  const PartIn rin{ring, ring_ks, rstride};
-  if (sh.KC <= 4) CU_OK(llb_launch(k_pf_conv<4>, cgrid, dim3(128), (size_t)0, s, qkv, rin, cw, bp, ap, dt, sa, sh, p0, R, y, gram, beta, decay));
-  else CU_OK(llb_launch(k_pf_conv<CONV_RING / 2>, cgrid, dim3(128), (size_t)0, s, qkv, rin, cw, bp, ap, dt, sa, sh, p0, R, y, gram, beta, decay));
+  int steps = 0, most = 0;
+  for (int i = 0; i < sg.n; i++) { const int n = (sg.s[i].R + PF_CH - 1) / PF_CH; steps += n; most = n > most ? n : most; }
+  const dim3 cgrid((sh.GK + 1) / 2 + (sh.TR + 3) / 4 + (PF_CH * sh.TR + 127) / 128, steps);
+  if (sh.KC <= 4) CU_OK(llb_launch(k_pf_conv<4>, cgrid, dim3(128), (size_t)0, s, sg, qkv, ring_ks, cw, bp, ap, dt, sa, sh, y, gram, beta, decay));
+  else CU_OK(llb_launch(k_pf_conv<CONV_RING / 2>, cgrid, dim3(128), (size_t)0, s, sg, qkv, ring_ks, cw, bp, ap, dt, sa, sh, y, gram, beta, decay));
   // A block's chain takes as long alone as with others on its SM, but the scheduler stacks blocks on few SMs while others idle
   // (32-head shape: 38 ms of a 4096-token prompt so, 28 ms spread): a block asks for the shared memory of its even share of an SM.
-  const int blocks = sh.TR * PF_SCAN_BLOCKS, per = (blocks + g_llb.sms - 1) / g_llb.sms;
+  const int blocks = sh.TR * PF_SCAN_BLOCKS * sg.n, per = (blocks + g_llb.sms - 1) / g_llb.sms;
   const size_t pad = per < 6 ? (size_t)(PF_SCAN_SMEM / per - 24 * 1024) : 0;
-  CU_OK(llb_launch(k_pf_scan, dim3(sh.TR, PF_SCAN_BLOCKS), dim3(32 * PF_SCAN_NW), pad, s, S, ctl, (const float *)y, (const float *)gram, (const float *)beta, (const float *)decay, sh, o, R));
-  CU_OK(llb_launch(k_pf_gnorm, dim3(sh.TR, (R + 7) / 8 + 1), dim3(256), (size_t)0, s, (const float *)o, z, nw, sh, kg, qkv, ring, ring_ks, p0, R, row0, ru));
+  CU_OK(llb_launch(k_pf_scan, dim3(sh.TR, PF_SCAN_BLOCKS, sg.n), dim3(32 * PF_SCAN_NW), pad, s, sg, (const float *)y, (const float *)gram, (const float *)beta, (const float *)decay, sh, o));
+  CU_OK(llb_launch(k_pf_gnorm, dim3(sh.TR, most + 1, sg.n), dim3(256), (size_t)0, s, (const float *)o, z, nw, sh, kg, qkv, ring_ks, sg, ru));
   return 0;
 }
 

@@ -30,5 +30,10 @@ int op_pf_silu(cudaStream_t s, PartIn g, PartIn u, int f, __half *kg, int R, int
 int op_pf_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w, const float *kn_w, const double *invfreq, AttnShape sh, int p0, int R, float *qout, float *Kc, float *Vc, bool kv_only = false);
 size_t op_pf_attn_parts(int H, int KV);           // values of pm and pl; po has head_dim as many
 int op_pf_attn(cudaStream_t s, const float *q, const float *Kc, const float *Vc, PartIn qg, AttnShape sh, int p0, int R, float *pm, float *pl, float *po, __half *kg, int row0, int ru);
-int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, float *ring, int ring_ks, const float *cw, const float *dt, const float *sa,
-                const float *nw, DeltaShape sh, float *S, const SpecCtl *ctl, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int p0, int R, int row0, int ru);   // gram: GK x PF_RMAX / 8 x 64
+// the sequences of a chunk: rows off .. off + R - 1 of it are positions p0 .. of one; its conv history, state and control block
+#define PF_PIECES 16                                 // most of them
+#define PF_STEPS (PF_RMAX / 8 + PF_PIECES)           // most steps of eight rows, each of one sequence
+struct PfSeg { int p0, R, off; float *ring, *S; const SpecCtl *ctl; };
+struct PfSegs { int n; PfSeg s[PF_PIECES]; };
+int op_pf_delta(cudaStream_t s, PartIn qkv, PartIn z, PartIn bp, PartIn ap, int ring_ks, const float *cw, const float *dt, const float *sa,
+                const float *nw, DeltaShape sh, const PfSegs &sg, float *y, float *gram, float *beta, float *decay, float *o, __half *kg, int ru);   // gram: GK x PF_STEPS x 64; beta, decay: TR x 8 PF_STEPS
