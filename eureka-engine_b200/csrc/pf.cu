@@ -1,4 +1,4 @@
-// pf.cu -- the prompt path: a chunk of up to PF_RMAX = 256 prompt rows per pass, dense GEMMs on tcgen05 (pfmm.cuh) and
+// pf.cu -- the prompt path: a chunk of up to PF_RMAX = 256 prompt rows per pass, dense GEMMs (pfx.cuh, pfmm.cuh) and attention (pfatt.cuh) on tcgen05,
 // row-batched small ops.  It stands where the reference has its fast prefill tier (host/llb_pf.h:551 pf_take; kernels
 // tools/pf27/pfmm.cuh, host/llb_pf.cuh; hand-off into the speculative state host/llb_host.c:1831-1899 spec_pf /
 // spec_take): the trunk's K/V rows, conv history and DeltaNet state after the chunk, the drafter's K/V rows for the
@@ -12,7 +12,7 @@
 #include "model.cuh"
 #include "pf.cuh"
 
-static unsigned int *g_pf_err = nullptr;   // device word: a bounded wait of k_pfmm ran out
+static unsigned int *g_pf_err = nullptr;   // device word: a bounded wait of one of the tcgen05 kernels here ran out
 
 static decltype(&cuTensorMapEncodeTiled) g_tensor_map = nullptr;
 
@@ -291,13 +291,15 @@ int op_pf_qkrope(cudaStream_t s, PartIn q, PartIn k, PartIn v, const float *qn_w
 }
 
 // ---- attention of a piece (pfatt.cuh) ---------------------------------------------------------------
-// Slices of the positions: the fewest rounds of blocks, each as long as its slice's tiles plus about five for the queries going in and the sums coming out.
+// Slices of the positions: the fewest rounds of blocks, each as long as its slice's tiles plus about five for the queries going in and the sums coming out, and a
+// quarter of a tile a slice for the merge.  Measured, with the merge: 256 rows of 24 heads of 256 over 4 behind 1280 positions 90 us with one slice, 58 with two, 48 with three
+// (144 blocks), 70 with four; 9 rows behind 8000 positions 61 with 8, 38 with 24, 35 with 32, 40 with 63; 128 rows of 8 heads over 2 behind 384 27 with two, 21 with 8, 24 with 16.
 static int pa_pick(int blocks, int total) {
   const int tiles = (total + 31) >> 5, sms = g_llb.sms;
   int best = 1;
   double best_cost = 1e30;
   for (int ns = 1; ns <= tiles && (ns == 1 || blocks * ns <= 2 * sms); ns++) {
-    const double cost = (double)((blocks * ns + sms - 1) / sms) * ((tiles + ns - 1) / ns + 5.0);
+    const double cost = (double)((blocks * ns + sms - 1) / sms) * ((tiles + ns - 1) / ns + 5.0) + 0.25 * ns;
     if (cost < best_cost) { best_cost = cost; best = ns; }
   }
   return best;

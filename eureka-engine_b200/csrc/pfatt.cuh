@@ -382,18 +382,29 @@ __global__ void __launch_bounds__(256) k_pf_attn_comb(const float *__restrict__ 
   for (int i = 16; i > 0; i >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, i));
   float4 o[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
   float L = 0.0f;
-#pragma unroll 4
-  for (int s = 0; s < ns; s++) {
-    const float m = __ldcg(pm + qb + s), w = m == -INFINITY ? 0.0f : expf(m - M);
-    if (w == 0.0f) continue;                     // (a slice that the row sees nothing of has no sums)
-    L += __ldcg(pl + qb + s) * w;
+#pragma unroll 1
+  for (int s0 = 0; s0 < ns; s0 += 32) {          // a lane a slice's weight, then the slices' rows two at a time
+    const float m = s0 + lane < ns ? __ldcg(pm + qb + s0 + lane) : -INFINITY, w = m == -INFINITY ? 0.0f : expf(m - M);
+    if (w != 0.0f) L += __ldcg(pl + qb + s0 + lane) * w;
+#pragma unroll 1
+    for (int j = 0; j < 32 && s0 + j < ns; j += 2) {
+      float ws[2];
+      float4 v[2][2];
 #pragma unroll
-    for (int i = 0; i < 2; i++)
-      if (128 * i < hd) {
-        const float4 v = __ldcg((const float4 *)(po + (qb + s) * hd + 128 * i + 4 * lane));
-        o[i].x += v.x * w; o[i].y += v.y * w; o[i].z += v.z * w; o[i].w += v.w * w;
+      for (int q = 0; q < 2; q++) {
+        ws[q] = __shfl_sync(0xffffffffu, w, j + q);
+#pragma unroll
+        for (int i = 0; i < 2; i++)              // (a slice that the row sees nothing of has no sums)
+          v[q][i] = ws[q] != 0.0f && 128 * i < hd ? __ldcg((const float4 *)(po + (qb + s0 + j + q) * hd + 128 * i + 4 * lane)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) { o[i].x += v[q][i].x * ws[q]; o[i].y += v[q][i].y * ws[q]; o[i].z += v[q][i].z * ws[q]; o[i].w += v[q][i].w * ws[q]; }
+    }
   }
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) L += __shfl_xor_sync(0xffffffffu, L, i);
 #pragma unroll
   for (int i = 0; i < 2; i++)
     if (128 * i < hd) {
