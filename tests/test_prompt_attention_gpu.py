@@ -45,5 +45,6 @@ def test_rows_and_tiles(pkg, packs, llb, monkeypatch, form, n):
 
 
 def test_many_slices(pkg, packs, llb, monkeypatch):
+    """A last piece of ten rows behind 12800 positions: 37 slices, more than the lanes that hold their weights."""
     pack = packs.build_pack(packs.cfg_tiny(n_layers=4, seed=51, **FORMS[1]))
-    _check(pkg, pack, monkeypatch, packs.synth_prompt(3, 1800 + 9, pack.cfg.vocab_size))
+    _check(pkg, pack, monkeypatch, packs.synth_prompt(3, 12800 + 11, pack.cfg.vocab_size))
