@@ -732,3 +732,225 @@ int llb_b200_pf_gemm(int fmt, unsigned long long w, int rows, int K, unsigned lo
   if (!rc && cudaGetLastError() != cudaSuccess) rc = llb_fail("pf_gemm: a kernel failed");
   return rc;
 }
+
+// ---- what the agents of the kernels here do with their barriers --------------------------------------
+// For a check without a GPU: every warp's waits and arrivals in its order, with the kernels' own rings and numbering.  ops: {0 wait, barrier, phase},
+// {1 arrive, barrier, times}, {2 arrive, barrier, once a copy requested or an MMA issued here is done}; a pair's second CTA has the same
+// barriers from PT_BARS on.  Returns the operations' number, 0 for an agent that has none, -1 past the last agent.
+struct PfTrace {
+  int *ops, cap, n = 0;
+  void put(int kind, int b, int v) { if (3 * n + 2 < cap) { ops[3 * n] = kind; ops[3 * n + 1] = b; ops[3 * n + 2] = v; } n++; }
+  void wait(int b, int phase) { put(0, b, phase); }
+  void free_again(int b, int use) { if (use > 0) put(0, b, use - 1); }     // a ring's buffer at its use-th use
+  void arrive(int b) { put(1, b, 1); }
+  void later(int b) { put(2, b, 1); }
+};
+#define PT_BARS 64
+static int pa_trace(PfTrace &t, int NS, int n, int agent) {
+  const int full = 0, empty = 8, s_full = 16, p_full = 18, pv_done = 20, o_empty = 22, q_full = 23;
+  if (agent < 4) {            // softmax
+    t.arrive(q_full);
+    for (int it = 0; it < n; it++) {
+      t.wait(s_full + (it & 1), it >> 1);
+      if (it >= 2) t.wait(pv_done + (it & 1), (it >> 1) - 1);
+      t.arrive(p_full + (it & 1));
+    }
+  } else if (agent == 4) {    // loads
+    int k = 0;
+    auto load = [&] {
+      const int slot = k % NS;
+      if (k >= NS) t.wait(empty + slot, k / NS - 1);
+      else if (k == NS - 2) t.wait(q_full, 0);
+      t.later(full + slot);
+      k++;
+    };
+    for (int i = -2; i < n; i++) {
+      if (i >= 0) load();
+      if (i + 2 < n) load();
+    }
+  } else if (agent == 5) {    // issues the MMAs
+    int k = 0;
+    t.wait(q_full, 0);
+    for (int i = -2; i < n; i++) {
+      if (i >= 0) {
+        t.wait(p_full + (i & 1), i >> 1);
+        t.wait(o_empty, i);
+        t.wait(full + k % NS, k / NS);
+        t.later(pv_done + (i & 1)); t.later(empty + k % NS);
+        k++;
+      }
+      if (i + 2 < n) {
+        t.wait(full + k % NS, k / NS);
+        t.later(s_full + (i & 1)); t.later(empty + k % NS);
+        k++;
+      }
+    }
+  } else if (agent < 14) {    // O
+    for (int it = 0; it < n; it++) {
+      t.wait(p_full + (it & 1), it >> 1);
+      t.arrive(o_empty);
+      t.wait(pv_done + (it & 1), it >> 1);
+    }
+  } else return -1;
+  return t.n;
+}
+static int pa_count(int b) { return b == 22 ? 8 : b == 18 || b == 19 || b == 23 ? 4 : 1; }
+
+enum { PT_A_FULL = 0, PT_A_EMPTY = 8, PT_B_FULL = 16, PT_B_EMPTY = 20, PT_B_HERE = 24, PT_D_FULL = 28, PT_D_EMPTY = 32, PT_SC = 36, PT_RAW_FULL = 40, PT_RAW_EMPTY = 44 };
+// the roles that the GEMM kernels have alike; me: the CTA's barriers
+static void pt_weights(PfTrace &t, int me, int NRAW, int CH, int units, int nsl) {
+  int k = 0;
+  for (int u = 0; u < units; u++)
+    for (int c = 0; c < nsl; c += CH, k++) { t.free_again(me + PT_RAW_EMPTY + k % NRAW, k / NRAW); t.later(me + PT_RAW_FULL + k % NRAW); }
+}
+static void pt_activations(PfTrace &t, int rank, int NB, int slots) {
+  for (int i = 0; i < slots; i++) { t.free_again(rank * PT_BARS + PT_B_EMPTY + i % NB, i / NB); t.later((rank ? PT_BARS + PT_B_HERE : PT_B_FULL) + i % NB); }
+}
+static void pt_forward(PfTrace &t, int NB, int slots) {
+  for (int i = 0; i < slots; i++) { t.wait(PT_BARS + PT_B_HERE + i % NB, i / NB); t.arrive(PT_B_FULL + i % NB); }
+}
+static void pt_both(PfTrace &t, int b) { t.later(b); t.later(PT_BARS + b); }
+template <int FMT, int RU> static int px1_trace(PfTrace &t, int units, int nsl, int agent) {
+  constexpr int NA = px_na(FMT), NB = px_nb(FMT), BS = px_slot_stages(RU), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), SS = px_sub(FMT);
+  const int rank = agent / 20, w = agent % 20, me = rank * PT_BARS;
+  if (agent >= 40) return -1;
+  if (w < 8) {
+    int k = 0, rk = 0, jj = 0;
+    for (int u = 0; u < units; u++)
+      for (int c = 0; c < nsl; c++, jj++) {
+        if (c % CH == 0) t.wait(me + PT_RAW_FULL + rk % NRAW, rk / NRAW);
+        for (int s = 0; s < 4; s += SS, k++) {
+          t.free_again(me + PT_A_EMPTY + k % NA, k / NA);
+          if (s == 0 && w < 4) t.arrive(me + PT_SC + (jj & 3));
+          t.arrive(PT_A_FULL + k % NA);
+        }
+        if (c % CH == CH - 1 || c == nsl - 1) { t.arrive(me + PT_RAW_EMPTY + rk % NRAW); rk++; }
+      }
+  } else if (w == 8) pt_weights(t, me, NRAW, CH, units, nsl);
+  else if (w == 9) pt_activations(t, rank, NB, units * (4 * nsl / BS));
+  else if (w == 10 && rank == 0) {
+    int k = 0, bk = 0;
+    for (int i = 0; i < units * nsl * 4; i += SS, k++) {
+      if (k > 1) t.wait(PT_D_EMPTY + (k & 1), (k >> 1) - 1);
+      t.wait(PT_A_FULL + k % NA, k / NA);
+      for (int q = 0; q < SS; q++) {
+        const int in = (i + q) % BS;
+        if (in == 0) t.wait(PT_B_FULL + bk % NB, bk / NB);
+        if (q == SS - 1) { pt_both(t, PT_A_EMPTY + k % NA); pt_both(t, PT_D_FULL + (k & 1)); }
+        if (in == BS - 1) { pt_both(t, PT_B_EMPTY + bk % NB); bk++; }
+      }
+    }
+  } else if (w == 11 && rank == 1) pt_forward(t, NB, units * (4 * nsl / BS));
+  else if (w >= 12) {
+    for (int jj = 0, k = 0; jj < units * nsl; jj++) {
+      t.wait(me + PT_SC + (jj & 3), jj >> 2);
+      for (int p = 0; p < 4 / SS; p++, k++) { t.wait(me + PT_D_FULL + (k & 1), k >> 1); t.arrive(PT_D_EMPTY + (k & 1)); }
+    }
+  }
+  return t.n;
+}
+static int px1_count(int b) { return b < 8 || (b >= 32 && b < 36) ? 16 : b >= 16 && b < 20 ? 2 : b >= 36 && b < 40 ? 4 : b >= 44 ? 8 : 1; }
+template <int FMT> static int pt_trace(PfTrace &t, int units, int nsl, int agent) {
+  constexpr int NB = PT_NB, SPB = 4 / px_slot_stages(PT_RU), NP = pt_items(FMT), SI = 4 / NP, ND = 128 / (2 * PT_RU), CH = px_chunk(FMT), NRAW = pt_raws(FMT);
+  const int rank = agent / 20, w = agent % 20, me = rank * PT_BARS;
+  if (agent >= 40) return -1;
+  if (w < 8) {
+    const int g = w >> 2;
+    int it = 0, rk = 0, jj = 0;
+    for (int u = 0; u < units; u++)
+      for (int c = 0; c < nsl; c++, jj++) {
+        if (c % CH == 0) t.wait(me + PT_RAW_FULL + rk % NRAW, rk / NRAW);
+        if ((jj & 1) == g)
+          for (int p = 0; p < NP; p++, it++) {
+            t.free_again(me + PT_A_EMPTY + 2 * g + (it & 1), it >> 1);
+            if (p == 0) t.arrive(me + PT_SC + (jj & 3));
+            t.arrive(PT_A_FULL + 2 * g + (it & 1));
+          }
+        if (c % CH == CH - 1 || c == nsl - 1) { t.arrive(me + PT_RAW_EMPTY + rk % NRAW); rk++; }
+      }
+  } else if (w == 8) pt_weights(t, me, NRAW, CH, units, nsl);
+  else if (w == 9) pt_activations(t, rank, NB, units * nsl * SPB);
+  else if (w < 12) {
+    if (rank == 1) { if (w == 11) pt_forward(t, NB, units * nsl * SPB); }
+    else {
+      const int g = w - 10;
+      for (int jj = g, it = 0; jj < units * nsl; jj += 2)
+        for (int p = 0; p < NP; p++, it++) {
+          const int buf = 2 * g + (it & 1), dbar = 2 * g + it % ND, sl = (jj * SPB + p * SPB / NP) % NB, in = p * SI - (p * SPB / NP) * (4 / SPB);
+          if (it >= ND) t.wait(PT_D_EMPTY + dbar, it / ND - 1);
+          if (in == 0) t.wait(PT_B_FULL + sl, jj * SPB / NB);
+          t.wait(PT_A_FULL + buf, it >> 1);
+          pt_both(t, PT_A_EMPTY + buf);
+          if (in + SI == 4 / SPB) pt_both(t, PT_B_EMPTY + sl);
+          pt_both(t, PT_D_FULL + dbar);
+        }
+    }
+  } else {
+    for (int jj = 0; jj < units * nsl; jj++)
+      for (int p = 0; p < NP; p++) {
+        const int g = jj & 1, it = (jj >> 1) * NP + p, dbar = 2 * g + it % ND;
+        if (p == 0) t.wait(me + PT_SC + (jj & 3), jj >> 2);
+        t.wait(me + PT_D_FULL + dbar, it / ND);
+        t.arrive(PT_D_EMPTY + dbar);
+      }
+  }
+  return t.n;
+}
+static int pt_count(int b) { return b < 8 || b >= 44 ? 8 : b >= 32 && b < 36 ? 16 : b >= 16 && b < 20 ? 2 : b >= 36 && b < 40 ? 4 : 1; }
+static int px2_trace(PfTrace &t, int units, int nsl, int agent) {
+  const int rank = agent / 16, w = agent % 16, me = rank * PT_BARS, NA = PX2_NA, NB = PX2_NB;
+  if (agent >= 32) return -1;
+  if (w < 4) {
+    for (int jj = 0, k = 0; jj < units * nsl; jj++) {
+      t.wait(me + PT_RAW_FULL + jj % PX2_NRAW, jj / PX2_NRAW);
+      for (int s = 0; s < 4; s++, k++) {
+        t.free_again(me + PT_A_EMPTY + k % NA, k / NA);
+        if (s == 0) t.arrive(me + PT_SC + (jj & 3));
+        t.arrive(PT_A_FULL + k % NA);
+      }
+      t.arrive(me + PT_RAW_EMPTY + jj % PX2_NRAW);
+    }
+  } else if (w == 4) pt_weights(t, me, PX2_NRAW, 1, units, nsl);
+  else if (w == 5) pt_activations(t, rank, NB, units * nsl * 8);
+  else if (w == 6 && rank == 0) {
+    for (int jj = 0; jj < units * nsl; jj++) {
+      if (jj > 1) t.wait(PT_D_EMPTY + (jj & 1), (jj >> 1) - 1);
+      for (int i = 0; i < 8; i++) {
+        const int s = i & 3, k = 4 * jj + s, as = k % NA;
+        if (i < 4) t.wait(PT_A_FULL + as, k / NA);
+        t.wait(PT_B_FULL + s, 2 * jj + (i >> 2));
+        pt_both(t, PT_B_EMPTY + s);
+        if (i >= 4) pt_both(t, PT_A_EMPTY + as);
+        if (i == 7) pt_both(t, PT_D_FULL + (jj & 1));
+      }
+    }
+  } else if (w == 7 && rank == 1) pt_forward(t, NB, units * nsl * 8);
+  else if (w >= 8) {
+    for (int jj = 0; jj < units * nsl; jj++) { t.wait(me + PT_SC + (jj & 3), jj >> 2); t.wait(me + PT_D_FULL + (jj & 1), jj >> 1); t.arrive(PT_D_EMPTY + (jj & 1)); }
+  }
+  return t.n;
+}
+static int px2_count(int b) { return b < 8 ? 8 : b >= 32 && b < 36 ? 16 : b >= 16 && b < 20 ? 2 : b >= 36 && b < 40 || b >= 44 ? 4 : 1; }
+// kernel: 0 k_pf_attn (form: head dimension; units x nsl tiles of positions), 1 k_pfx1 / k_pft of `form` rows, 2 k_pfx2
+extern "C" __attribute__((visibility("default")))
+int llb_b200_pf_trace(int kernel, int form, int fmt, int units, int nsl, int agent, int *ops, int cap) {
+  PfTrace t{ops, cap};
+  if (kernel == 0) return form == 128 || form == 256 ? pa_trace(t, pa_slots(form), units * nsl, agent) : -1;
+#define PT_ALL(F) (form == 32 ? pt_trace<F>(t, units, nsl, agent) : form == 64 ? px1_trace<F, 64>(t, units, nsl, agent) : px1_trace<F, 128>(t, units, nsl, agent))
+  if (kernel == 1)
+    switch (fmt) {
+      case LLB_FM_Q4_K: return PT_ALL(LLB_FM_Q4_K);
+      case LLB_FM_Q5_K: return PT_ALL(LLB_FM_Q5_K);
+      case LLB_FM_Q6_K: return PT_ALL(LLB_FM_Q6_K);
+      case LLB_FM_Q8_0: return PT_ALL(LLB_FM_Q8_0);
+      default: return -1;
+    }
+#undef PT_ALL
+  return kernel == 2 ? px2_trace(t, units, nsl, agent) : -1;
+}
+// arrivals that complete a phase of barrier `bar`
+extern "C" __attribute__((visibility("default")))
+int llb_b200_pf_bar_count(int kernel, int form, int bar) {
+  bar %= PT_BARS;
+  return kernel == 0 ? pa_count(bar) : kernel == 2 ? px2_count(bar) : form == 32 ? pt_count(bar) : px1_count(bar);
+}

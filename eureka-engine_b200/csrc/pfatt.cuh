@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) k_pf_attn(const PaArgs a, const
         if (i >= 0) {
           const int b = i & 1, slot = t % NS;
           wait(p_full(b), (uint32_t)(i >> 1) & 1u);
-          if (i > 0) wait(o_empty, (uint32_t)(i - 1) & 1u);
+          wait(o_empty, (uint32_t)i & 1u);       // P(i) has been seen, O(i - 1) has been read
           wait(full(slot), (uint32_t)(t / NS) & 1u);
           t5_fence_after();
           const uint64_t vh = pa_desc(ring_s + slot * SLB, PA_BOX), vl = vh + PA_BOX / 32;
@@ -314,13 +314,13 @@ __global__ void __launch_bounds__(PA_THREADS, 1) k_pf_attn(const PaArgs a, const
 #pragma unroll 1
     for (int it = 0; it < n; it++) {
       const int b = it & 1;
-      // (the tile before is given back only once this tile's P has been seen: until then P and the factors two tiles on cannot come, so that a
-      // phase of p_full is never missed)
+      // (the products of a tile, the first one's too, wait until its P and factors have been seen here and the tile before has been read: until
+      // then P and the factors two tiles on cannot come, so that a phase of p_full is never missed)
       wait(p_full(b), (uint32_t)(it >> 1) & 1u);
       const float c = corr[b * 128 + 32 * q + lane];
       const f32x2 c2 = x2_pack(c, c);
       __syncwarp();
-      if (it > 0 && lane == 0) mbar_arrive(o_empty);
+      if (lane == 0) mbar_arrive(o_empty);
       wait(pv_done(b), (uint32_t)(it >> 1) & 1u);
       t5_fence_after();
 #pragma unroll
