@@ -42,11 +42,12 @@ struct TensorRec { uint64_t off, bytes; int rows, cols, fmt; bool blocked = fals
 
 // Buffers of the prompt path (pf.cu), allocated at the first prompt that takes it: residual rows, fp16 activations in the
 // dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows.  Nothing in them
-// outlives a prompt, so the engine that has the weights keeps them for its siblings too; a prompt holds them (`busy`) while it is enqueued,
-// and the library's one stream keeps the chunks of several prompts apart.
+// outlives a prompt, so the engine that has the weights keeps them for its siblings too; a prompt holds them (`busy`) from looking whether they
+// are there until it is enqueued, and the library's one stream keeps the chunks of several prompts apart.
 struct PfState {
   bool ready = false, none = false;   // none: there was no room for them
   std::mutex busy;
+  std::vector<void *> mem;            // (the owner's own list is its thread's)
   float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *gram = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
   __half *kg_d = nullptr, *kg_f = nullptr, *kg_qa = nullptr, *kg_v = nullptr, *kg_2d = nullptr;
   OutBuf q, k, v, qkv, z, bp, ap, a, g, u, dn, eh;
@@ -197,14 +198,15 @@ static void prof_mark(const char *name) {
 #define RING_MAXSPLIT 8   // most K-slices a conv ring keeps per row
 static float bits_float(unsigned int u) { float f; memcpy(&f, &u, 4); return f; }
 
-static void *dalloc(llb_spec *m, size_t bytes) {
+static void *dalloc(std::vector<void *> &list, size_t bytes) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes ? bytes : 256);
   if (e != cudaSuccess) { llb_fail("cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e)); cudaGetLastError(); return nullptr; }
   cudaMemsetAsync(p, 0, bytes, g_llb.stream);
-  m->allocs.push_back(p);
+  list.push_back(p);
   return p;
 }
+static void *dalloc(llb_spec *m, size_t bytes) { return dalloc(m->allocs, bytes); }
 static float *falloc(llb_spec *m, size_t n) { return (float *)dalloc(m, n * 4); }
 // storage of a weight: allocated (fresh: the caller uploads into it), or, in a sibling, the first engine's
 static void *walloc(llb_spec *m, size_t bytes, bool *fresh) {
@@ -1057,25 +1059,26 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
 
 // ---- the prompt path: chunks of up to PF_RMAX rows through dense tcgen05 GEMMs (pf.cu) ----------------------------
 static llb_spec *pf_owner(llb_spec *m) { return m->share ? m->share : m; }
+// (the caller holds `busy`)
 static int pf_alloc(llb_spec *m) {
-  llb_spec *o = pf_owner(m);
-  PfState &f = o->pf;
+  PfState &f = pf_owner(m)->pf;
   if (f.ready) return 0;
   if (f.none) return llb_fail("prompt path: no room for its buffers");
   CK(pf_setup());
   f.none = true;          // until all of them are there
   const int d = m->d, qa = m->H * m->hd;
-  auto kg = [&](int K) { return (__half *)dalloc(o, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
-  f.x = falloc(o, (size_t)PF_RMAX * d); f.x1 = falloc(o, (size_t)PF_RMAX * d); f.hn = falloc(o, (size_t)(PF_RMAX + PF_PIECES) * d); f.e = falloc(o, (size_t)PF_RMAX * d);
-  f.qn = falloc(o, (size_t)PF_RMAX * qa); f.y = falloc(o, (size_t)PF_RMAX * m->convd); f.beta = falloc(o, (size_t)PF_STEPS * 8 * m->TR); f.gram = falloc(o, (size_t)PF_STEPS * 64 * m->GK);
-  f.decay = falloc(o, (size_t)PF_STEPS * 8 * m->TR); f.o = falloc(o, (size_t)PF_RMAX * m->vdc);
+  auto falloc = [&](size_t n) { return (float *)dalloc(f.mem, n * 4); };
+  auto kg = [&](int K) { return (__half *)dalloc(f.mem, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
+  f.x = falloc((size_t)PF_RMAX * d); f.x1 = falloc((size_t)PF_RMAX * d); f.hn = falloc((size_t)(PF_RMAX + PF_PIECES) * d); f.e = falloc((size_t)PF_RMAX * d);
+  f.qn = falloc((size_t)PF_RMAX * qa); f.y = falloc((size_t)PF_RMAX * m->convd); f.beta = falloc((size_t)PF_STEPS * 8 * m->TR); f.gram = falloc((size_t)PF_STEPS * 64 * m->GK);
+  f.decay = falloc((size_t)PF_STEPS * 8 * m->TR); f.o = falloc((size_t)PF_RMAX * m->vdc);
   f.kg_d = kg(d); f.kg_f = kg(m->f); f.kg_qa = kg(qa); f.kg_v = kg(m->vdc); f.kg_2d = kg(2 * d);
   {
     const size_t n = op_pf_attn_parts(m->H, m->KV);
-    f.pm = falloc(o, n); f.pl = falloc(o, n); f.po = falloc(o, n * m->hd);
+    f.pm = falloc(n); f.pl = falloc(n); f.po = falloc(n * m->hd);
     if (!f.pm || !f.pl || !f.po) return -1;
   }
-  f.ids = (int *)dalloc(o, (size_t)(PF_RMAX + 1) * 4);
+  f.ids = (int *)dalloc(f.mem, (size_t)(PF_RMAX + 1) * 4);
   if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.gram || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
       !f.ids) return -1;
   f.none = false; f.ready = true;
@@ -1131,7 +1134,7 @@ static int pf_site(llb_spec *m, std::vector<PfSiteMat> mats, const __half *kg, i
       OutBuf &o = *sm.out;
       const size_t need = (size_t)a.ksplit * PF_RMAX * sm.w->rows;
       if (!o.p || o.cap < need) {
-        o.p = falloc(pf_owner(m), need);
+        o.p = (float *)dalloc(pf_owner(m)->pf.mem, need * 4);
         if (!o.p) return -1;
         o.cap = need;
       }
@@ -1242,11 +1245,9 @@ static bool px_takes(const llb_spec *m, int n_rows) {
 // chunks of PF_RMAX rows, mode 0 in pieces of PF_R rows, several streams' together as far as they fit.  Mode 1: a stream's drafter row at the
 // position it stops at is left pending as a one-row catch-up whose hidden (the normed row of the position before) is where the catch-up reads
 // it.  Mode 0 takes whole prompts, and leaves what the last T-row pass over them would have: its k + 1 normed rows, from which the
-// drafter catches up, and the next cycle's rows (px_logits: and its logits).
+// drafter catches up, and the next cycle's rows (px_logits: and its logits).  The caller holds the buffers.
 static int pf_prefill(llb_spec *m, int nb, const int *bs, const int *const *ids, const int *take, bool fast) {
   CK(pf_alloc(m));
-  PfState &f = pf_owner(m)->pf;
-  std::lock_guard<std::mutex> hold(f.busy);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (pf_prof_on()) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, g_llb.stream); }
   std::vector<int> p(nb, 0);
@@ -1473,6 +1474,7 @@ LLB_API void llb_spec_close(llb_spec *m) {
   if (m->g_prefill) cudaGraphExecDestroy(m->g_prefill);
   if (m->g_verify) cudaGraphExecDestroy(m->g_verify);
   for (void *p : m->allocs) cudaFree(p);
+  for (void *p : m->pf.mem) cudaFree(p);
   if (m->res_host) cudaFreeHost(m->res_host);
   delete m;
 }
@@ -1551,6 +1553,8 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
       if (m->prefill_mode == 1 && m->ne == 0 && m->tp.size <= 1 && ns[i] - 1 >= m->Tspec + 32) { fast[i] = ns[i] - 1 - m->Tspec; any_fast = true; }
       else if (px_takes(m, ns[i] - 1)) { exact[i] = ns[i] - 1; any_exact = true; }
     }
+    std::unique_lock<std::mutex> hold(pf_owner(m)->pf.busy, std::defer_lock);
+    if (any_fast || any_exact) hold.lock();
     if (any_fast) CK(pf_prefill(m, nb, bs, ids, fast.data(), true));
     if (any_exact && pf_alloc(m)) { cudaGetLastError(); any_exact = false; }
     if (any_exact) CK(pf_prefill(m, nb, bs, ids, exact.data(), false));

@@ -1,0 +1,86 @@
+"""The prompt path's buffers belong to the engine that has the weights and serve all of its siblings: prompts of several engines at once from
+threads, the first ones included, and prompts between another engine's prompt and cycles, leave what each leaves alone."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 6
+LENS = [300, 40, 150, 9]
+
+
+@pytest.fixture(scope="module")
+def model(pkg, packs, llb):
+    pack = packs.build_pack(packs.cfg_tiny(n_layers=4, seed=61))
+    return pack, packs.aux1_bytes(packs.build_mtp(pack))
+
+
+def _open(pkg, model, n):
+    first = pkg.llb.SpecEngine(model[0], model[1], k=3, max_ctx=360)
+    return [first] + [first.sibling(k=i % 4, max_ctx=360) for i in range(n - 1)]
+
+
+def _result(eng, cfg):
+    st = [eng.read_state(0, il) for il in range(cfg.n_layers) if not cfg.is_full(il)] + [eng.read_state(4, 0, 0)]
+    return st, eng.generate(STEPS)
+
+
+def _same(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a[0], b[0])) and all(np.array_equal(x, y) for x, y in zip(a[1], b[1]))
+
+
+@pytest.mark.parametrize("fast", [False, True])
+def test_first_prompts_at_once(pkg, packs, model, fast):
+    cfg = model[0].cfg
+    prompts = [packs.synth_prompt(70 + i, n, cfg.vocab_size) for i, n in enumerate(LENS)]
+    want = []
+    for i, p in enumerate(prompts):
+        engs = _open(pkg, model, len(prompts))
+        engs[i].set_prefill(fast)
+        engs[i].prefill(p)
+        want.append(_result(engs[i], cfg))
+        for e in engs:
+            e.close()
+    for _ in range(3):
+        engs = _open(pkg, model, len(prompts))
+        gate, errors = threading.Barrier(len(engs)), []
+
+        def feed(eng, p):
+            try:
+                gate.wait()
+                eng.prefill(p)
+            except Exception as e:   # noqa: BLE001 - any failure of a thread is the test's
+                errors.append(repr(e))
+
+        for e in engs:
+            e.set_prefill(fast)
+        ts = [threading.Thread(target=feed, args=a) for a in zip(engs, prompts)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        assert not errors
+        for e, w in zip(engs, want):
+            assert _same(_result(e, cfg), w)
+        for e in engs:
+            e.close()
+
+
+def test_prompt_between_another_ones_prompt_and_cycles(pkg, packs, model):
+    cfg = model[0].cfg
+    a, b = (packs.synth_prompt(90 + i, n, cfg.vocab_size) for i, n in enumerate((290, 133)))
+    engs = _open(pkg, model, 2)
+    engs[0].prefill(a)
+    want = _result(engs[0], cfg)
+    engs[0].prefill(a)
+    engs[1].prefill(b)
+    assert _same(_result(engs[0], cfg), want)
+    engs[1].prefill(b)
+    other = _result(engs[1], cfg)
+    engs[1].prefill(b)
+    engs[0].prefill(a)
+    assert _same(_result(engs[1], cfg), other)
+    for e in engs:
+        e.close()
