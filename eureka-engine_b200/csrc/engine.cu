@@ -40,14 +40,14 @@ struct LayerW { bool full = false; float *attn_norm = nullptr; AttnW at; DeltaW 
 // blocked: Q8_0 in GGUF's [f16 d][32 x int8] blocks (host memory only), re-sliced to the row-split layout at upload
 struct TensorRec { uint64_t off, bytes; int rows, cols, fmt; bool blocked = false; };
 
-// Buffers of the prompt path (pf.cu), allocated at the first prompt that takes it: residual rows, fp16 activations in the
+// Buffers of the prompt path (pf.cu), allocated in one piece at the first prompt that takes it: residual rows, fp16 activations in the
 // dense GEMM's k-group-major order, GEMM outputs as K-slice partial sums of PF_RMAX rows.  Nothing in them
 // outlives a prompt, so the engine that has the weights keeps them for its siblings too; a prompt holds them (`busy`) from looking whether they
 // are there until it is enqueued, and the library's one stream keeps the chunks of several prompts apart.
 struct PfState {
-  bool ready = false, none = false;   // none: there was no room for them
   std::mutex busy;
-  std::vector<void *> mem;            // (the owner's own list is its thread's)
+  void *mem = nullptr;
+  size_t extra = 0;                   // llb_spec_prefill_extra
   float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *gram = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
   __half *kg_d = nullptr, *kg_f = nullptr, *kg_qa = nullptr, *kg_v = nullptr, *kg_2d = nullptr;
   OutBuf q, k, v, qkv, z, bp, ap, a, g, u, dn, eh;
@@ -198,15 +198,14 @@ static void prof_mark(const char *name) {
 #define RING_MAXSPLIT 8   // most K-slices a conv ring keeps per row
 static float bits_float(unsigned int u) { float f; memcpy(&f, &u, 4); return f; }
 
-static void *dalloc(std::vector<void *> &list, size_t bytes) {
+static void *dalloc(llb_spec *m, size_t bytes) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes ? bytes : 256);
   if (e != cudaSuccess) { llb_fail("cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e)); cudaGetLastError(); return nullptr; }
   cudaMemsetAsync(p, 0, bytes, g_llb.stream);
-  list.push_back(p);
+  m->allocs.push_back(p);
   return p;
 }
-static void *dalloc(llb_spec *m, size_t bytes) { return dalloc(m->allocs, bytes); }
 static float *falloc(llb_spec *m, size_t n) { return (float *)dalloc(m, n * 4); }
 // storage of a weight: allocated (fresh: the caller uploads into it), or, in a sibling, the first engine's
 static void *walloc(llb_spec *m, size_t bytes, bool *fresh) {
@@ -1059,29 +1058,82 @@ static int open_impl(llb_spec *m, const char *index_text, const uint8_t *pack, i
 
 // ---- the prompt path: chunks of up to PF_RMAX rows through dense tcgen05 GEMMs (pf.cu) ----------------------------
 static llb_spec *pf_owner(llb_spec *m) { return m->share ? m->share : m; }
-// (the caller holds `busy`)
-static int pf_alloc(llb_spec *m) {
-  PfState &f = pf_owner(m)->pf;
-  if (f.ready) return 0;
-  if (f.none) return llb_fail("prompt path: no room for its buffers");
-  CK(pf_setup());
-  f.none = true;          // until all of them are there
-  const int d = m->d, qa = m->H * m->hd;
-  auto falloc = [&](size_t n) { return (float *)dalloc(f.mem, n * 4); };
-  auto kg = [&](int K) { return (__half *)dalloc(f.mem, (PF_RMAX / PF_R) * pf_kg_halves(K, PF_R) * 2); };   // the chunk's units one after the other
-  f.x = falloc((size_t)PF_RMAX * d); f.x1 = falloc((size_t)PF_RMAX * d); f.hn = falloc((size_t)(PF_RMAX + PF_PIECES) * d); f.e = falloc((size_t)PF_RMAX * d);
-  f.qn = falloc((size_t)PF_RMAX * qa); f.y = falloc((size_t)PF_RMAX * m->convd); f.beta = falloc((size_t)PF_STEPS * 8 * m->TR); f.gram = falloc((size_t)PF_STEPS * 64 * m->GK);
-  f.decay = falloc((size_t)PF_STEPS * 8 * m->TR); f.o = falloc((size_t)PF_RMAX * m->vdc);
-  f.kg_d = kg(d); f.kg_f = kg(m->f); f.kg_qa = kg(qa); f.kg_v = kg(m->vdc); f.kg_2d = kg(2 * d);
-  {
-    const size_t n = op_pf_attn_parts(m->H, m->KV);
-    f.pm = falloc(n); f.pl = falloc(n); f.po = falloc(n * m->hd);
-    if (!f.pm || !f.pl || !f.po) return -1;
+struct PfSiteMat { const DevMat *w; OutBuf *out; };
+// The matrices of a site that one launch takes, those of the first undone one's format, and the launch's K-slices
+static int pf_group(const std::vector<PfSiteMat> &mats, size_t i, int K, std::vector<bool> &done, std::vector<size_t> &grp) {
+  int ntiles = 0;
+  grp.clear();
+  for (size_t j = i; j < mats.size() && grp.size() < PF_MAXMAT; j++)
+    if (!done[j] && mats[j].w->fmt == mats[i].w->fmt) { grp.push_back(j); done[j] = true; ntiles += (mats[j].w->rows + 127) / 128; }
+  return pf_pick_ksplit(ntiles, K / 256, g_llb.sms);
+}
+// every site of the prompt path: its matrices, their outputs and the columns
+template <class F> static void pf_sites(const llb_spec *o, PfState &f, F &&site) {
+  const int d = o->d;
+  for (const LayerW &l : o->layer) {
+    if (l.full) {
+      site({{&l.at.q, &f.q}, {&l.at.k, &f.k}, {&l.at.v, &f.v}}, d);
+      site({{&l.at.o, &f.a}}, o->H * o->hd);
+    } else {
+      site({{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, d);
+      site({{&l.dn.out, &f.a}}, o->vdc);
+    }
+    site({{&l.ffn.gate, &f.g}, {&l.ffn.up, &f.u}}, d);
+    site({{&l.ffn.down, &f.dn}}, o->f);
   }
-  f.ids = (int *)dalloc(f.mem, (size_t)(PF_RMAX + 1) * 4);
-  if (!f.x || !f.x1 || !f.hn || !f.e || !f.qn || !f.y || !f.gram || !f.beta || !f.decay || !f.o || !f.kg_d || !f.kg_f || !f.kg_qa || !f.kg_v || !f.kg_2d ||
-      !f.ids) return -1;
-  f.none = false; f.ready = true;
+  if (o->has_mtp) { site({{&o->mt_eh, &f.eh}}, 2 * d); site({{&o->mt_at.k, &f.k}, {&o->mt_at.v, &f.v}}, d); }
+}
+// 1 where there is no room for the buffers, and nothing is kept: the next prompt looks again.  The caller holds `busy`.
+static int pf_alloc(llb_spec *m) {
+  llb_spec *o = pf_owner(m);
+  PfState &f = o->pf;
+  if (f.mem) return 0;
+  if (const int rc = pf_setup()) return rc;
+  OutBuf *const outs[] = {&f.q, &f.k, &f.v, &f.qkv, &f.z, &f.bp, &f.ap, &f.a, &f.g, &f.u, &f.dn, &f.eh};
+  for (OutBuf *b : outs) *b = OutBuf();
+  pf_sites(o, f, [&](const std::vector<PfSiteMat> &mats, int K) {
+    std::vector<bool> done(mats.size(), false);
+    std::vector<size_t> grp;
+    for (size_t i = 0; i < mats.size(); i++) {
+      if (done[i]) continue;
+      const int ks = pf_group(mats, i, K, done, grp);
+      for (size_t g : grp) { const size_t need = (size_t)ks * PF_RMAX * mats[g].w->rows; if (mats[g].out->cap < need) mats[g].out->cap = need; }
+    }
+  });
+  const int d = o->d, qa = o->H * o->hd;
+  const size_t parts = op_pf_attn_parts(o->H, o->KV);
+  size_t at = 0;
+  auto lay = [&](auto *&p, size_t n) {   // its place behind the others, once there is a block also as an address
+    p = f.mem ? (decltype(&*p))((uint8_t *)f.mem + at) : nullptr;
+    at += (n * sizeof *p + 1023) & ~(size_t)1023;
+  };
+  for (;;) {
+    at = 0;
+    lay(f.x, (size_t)PF_RMAX * d); lay(f.x1, (size_t)PF_RMAX * d); lay(f.hn, (size_t)(PF_RMAX + PF_PIECES) * d); lay(f.e, (size_t)PF_RMAX * d);
+    lay(f.qn, (size_t)PF_RMAX * qa); lay(f.y, (size_t)PF_RMAX * o->convd); lay(f.gram, (size_t)PF_STEPS * 64 * o->GK); lay(f.o, (size_t)PF_RMAX * o->vdc);
+    lay(f.beta, (size_t)PF_STEPS * 8 * o->TR); lay(f.decay, (size_t)PF_STEPS * 8 * o->TR);
+    const size_t units = PF_RMAX / PF_R;   // a chunk's, one after the other
+    lay(f.kg_d, units * pf_kg_halves(d, PF_R)); lay(f.kg_f, units * pf_kg_halves(o->f, PF_R)); lay(f.kg_qa, units * pf_kg_halves(qa, PF_R));
+    lay(f.kg_v, units * pf_kg_halves(o->vdc, PF_R)); lay(f.kg_2d, units * pf_kg_halves(2 * d, PF_R));
+    lay(f.pm, parts); lay(f.pl, parts); lay(f.po, parts * o->hd);
+    lay(f.ids, PF_RMAX + 1);
+    for (OutBuf *b : outs) lay(b->p, b->cap);
+    if (f.mem) break;
+    const cudaError_t e = cudaMalloc(&f.mem, at + f.extra);
+    if (e != cudaSuccess) {
+      f.mem = nullptr;
+      cudaGetLastError();
+      llb_fail("prompt path: its buffers take %zu bytes: %s", at + f.extra, cudaGetErrorString(e));
+      return e == cudaErrorMemoryAllocation ? 1 : -1;
+    }
+  }
+  CU_OK(cudaMemsetAsync(f.mem, 0, at, g_llb.stream));
+  return 0;
+}
+// Test entry: bytes that the prompt path's buffers take beyond their need when they are allocated (more than the GPU has: there is no room)
+LLB_API int llb_spec_prefill_extra(llb_spec *m, size_t bytes) {
+  std::lock_guard<std::mutex> hold(pf_owner(m)->pf.busy);
+  pf_owner(m)->pf.extra = bytes;
   return 0;
 }
 
@@ -1114,33 +1166,23 @@ static void pf_prof_report(int rows, double wall_ms) {
 }
 #define PFK(name, call) do { PfTimer t_(name); if ((call)) return -1; } while (0)
 
-struct PfSiteMat { const DevMat *w; OutBuf *out; };
 // the dense GEMMs of one site: matrices sharing the activations `kg` of K columns, one launch per format
-static int pf_site(llb_spec *m, std::vector<PfSiteMat> mats, const __half *kg, int K, int R) {
+static int pf_site(const std::vector<PfSiteMat> &mats, const __half *kg, int K, int R) {
   std::vector<bool> done(mats.size(), false);
+  std::vector<size_t> grp;
   for (size_t i = 0; i < mats.size(); i++) {
     if (done[i]) continue;
     PfArgs a;
     memset(&a, 0, sizeof a);
     a.K = K; a.R = R; a.x = kg;
-    int ntiles = 0;
-    std::vector<size_t> grp;
-    for (size_t j = i; j < mats.size() && grp.size() < PF_MAXMAT; j++)
-      if (!done[j] && mats[j].w->fmt == mats[i].w->fmt) { grp.push_back(j); ntiles += (mats[j].w->rows + 127) / 128; }
-    a.ksplit = pf_pick_ksplit(ntiles, K / 256, g_llb.sms);
+    a.ksplit = pf_group(mats, i, K, done, grp);
     a.nmat = (int)grp.size();
     for (size_t g = 0; g < grp.size(); g++) {
       const PfSiteMat &sm = mats[grp[g]];
       OutBuf &o = *sm.out;
-      const size_t need = (size_t)a.ksplit * PF_RMAX * sm.w->rows;
-      if (!o.p || o.cap < need) {
-        o.p = (float *)dalloc(pf_owner(m)->pf.mem, need * 4);
-        if (!o.p) return -1;
-        o.cap = need;
-      }
+      if (o.cap < (size_t)a.ksplit * PF_RMAX * sm.w->rows) return llb_fail("prompt path: %d K-slices of %d rows have no buffer", a.ksplit, sm.w->rows);
       o.ns = a.ksplit; o.stride = (long long)PF_RMAX * sm.w->rows;
       a.m[g].W = sm.w->w; a.m[g].rows = sm.w->rows; a.m[g].ostride = sm.w->rows; a.m[g].out = o.p; a.m[g].split_stride = o.stride;
-      done[grp[g]] = true;
     }
     CK(pf_gemm(g_llb.stream, mats[i].w->fmt, a));
   }
@@ -1178,7 +1220,7 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
     const LayerW &l = m->layer[il];
     PFK("norm", op_pf_norm(s, il ? f.x1 : f.x, il ? as_in(f.dn) : none, l.attn_norm, m->eps, d, f.x, f.kg_d, d, 0, nullptr, R, ru));
     if (l.full) {
-      PFK("gemm qkv", pf_site(m, {{&l.at.q, &f.q}, {&l.at.k, &f.k}, {&l.at.v, &f.v}}, f.kg_d, d, R));
+      PFK("gemm qkv", pf_site({{&l.at.q, &f.q}, {&l.at.k, &f.k}, {&l.at.v, &f.v}}, f.kg_d, d, R));
       for (int i = 0; i < np; i++) {
         const PfPiece &p = pc[i];
         const PartIn q = pf_rows_of(f.q, 2 * qa, p.off);
@@ -1186,19 +1228,19 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
         PFK("qkrope", op_pf_qkrope(s, q, pf_rows_of(f.k, kvd, p.off), pf_rows_of(f.v, kvd, p.off), l.at.qn, l.at.kn, m->invfreq, ash, p.p0, p.R, qn, kc, vc));
         PFK("attention", op_pf_attn(s, qn, kc, vc, q, ash, p.p0, p.R, f.pm, f.pl, f.po, f.kg_qa, p.off, ru));
       }
-      PFK("gemm attn_out", pf_site(m, {{&l.at.o, &f.a}}, f.kg_qa, qa, R));
+      PFK("gemm attn_out", pf_site({{&l.at.o, &f.a}}, f.kg_qa, qa, R));
     } else {
-      PFK("gemm qkv|z|b|a", pf_site(m, {{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));
+      PFK("gemm qkv|z|b|a", pf_site({{&l.dn.qkv, &f.qkv}, {&l.dn.z, &f.z}, {&l.dn.beta, &f.bp}, {&l.dn.alpha, &f.ap}}, f.kg_d, d, R));
       PfSegs sg{};
       sg.n = np;
       for (int i = 0; i < np; i++) sg.s[i] = PfSeg{pc[i].p0, pc[i].R, pc[i].off, ring_of(m, il, pc[i].b), state_of(m, il, pc[i].b), ctl_of(m, pc[i].b)};
       PFK("delta", op_pf_delta(s, as_in(f.qkv), as_in(f.z), as_in(f.bp), as_in(f.ap), m->ring_ks[il], l.dn.conv, l.dn.dt, l.dn.a, l.dn.norm, dsh, sg, f.y, f.gram, f.beta, f.decay, f.o, f.kg_v, ru));
-      PFK("gemm ssm_out", pf_site(m, {{&l.dn.out, &f.a}}, f.kg_v, m->vdc, R));
+      PFK("gemm ssm_out", pf_site({{&l.dn.out, &f.a}}, f.kg_v, m->vdc, R));
     }
     PFK("norm", op_pf_norm(s, f.x, as_in(f.a), l.ffn.post, m->eps, d, f.x1, f.kg_d, d, 0, nullptr, R, ru));
-    PFK("gemm gate|up", pf_site(m, {{&l.ffn.gate, &f.g}, {&l.ffn.up, &f.u}}, f.kg_d, d, R));
+    PFK("gemm gate|up", pf_site({{&l.ffn.gate, &f.g}, {&l.ffn.up, &f.u}}, f.kg_d, d, R));
     PFK("silu", op_pf_silu(s, as_in(f.g), as_in(f.u), m->f, f.kg_f, R, ru));
-    PFK("gemm down", pf_site(m, {{&l.ffn.down, &f.dn}}, f.kg_f, m->f, R));
+    PFK("gemm down", pf_site({{&l.ffn.down, &f.dn}}, f.kg_f, m->f, R));
   }
   // the trunk's output-normed rows: piece i's from row off + i + 1 of pf.hn on, the row in front of them that of the position before (a fresh stream's is
   // zero, host/llb_host.c:1816)
@@ -1214,9 +1256,9 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
     CK(op_pf_embed(s, m->embd.fmt, m->embd.w, d, f.ids, R, f.e));
     CK(op_pf_norm(s, f.e, none, m->mt_enorm, m->eps, d, nullptr, f.kg_2d, 2 * d, 0, nullptr, R, ru));
     for (int i = 0; i < np; i++) CK(op_pf_norm(s, f.hn + (size_t)(pc[i].off + i) * d, none, m->mt_hnorm, m->eps, d, nullptr, f.kg_2d, 2 * d, d, nullptr, pc[i].R, ru, pc[i].off));
-    CK(pf_site(m, {{&m->mt_eh, &f.eh}}, f.kg_2d, 2 * d, R));
+    CK(pf_site({{&m->mt_eh, &f.eh}}, f.kg_2d, 2 * d, R));
     CK(op_pf_norm(s, nullptr, as_in(f.eh), m->mt_attn_norm, m->eps, d, nullptr, f.kg_d, d, 0, nullptr, R, ru));
-    CK(pf_site(m, {{&m->mt_at.k, &f.k}, {&m->mt_at.v, &f.v}}, f.kg_d, d, R));
+    CK(pf_site({{&m->mt_at.k, &f.k}, {&m->mt_at.v, &f.v}}, f.kg_d, d, R));
     for (int i = 0; i < np; i++) {
       const PfPiece &p = pc[i];
       const int rows = p.R - (pf_keep(m, p) - 1);   // the rest of a prompt is what the drafter catches up over
@@ -1247,7 +1289,6 @@ static bool px_takes(const llb_spec *m, int n_rows) {
 // it.  Mode 0 takes whole prompts, and leaves what the last T-row pass over them would have: its k + 1 normed rows, from which the
 // drafter catches up, and the next cycle's rows (px_logits: and its logits).  The caller holds the buffers.
 static int pf_prefill(llb_spec *m, int nb, const int *bs, const int *const *ids, const int *take, bool fast) {
-  CK(pf_alloc(m));
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (pf_prof_on()) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, g_llb.stream); }
   std::vector<int> p(nb, 0);
@@ -1474,7 +1515,7 @@ LLB_API void llb_spec_close(llb_spec *m) {
   if (m->g_prefill) cudaGraphExecDestroy(m->g_prefill);
   if (m->g_verify) cudaGraphExecDestroy(m->g_verify);
   for (void *p : m->allocs) cudaFree(p);
-  for (void *p : m->pf.mem) cudaFree(p);
+  cudaFree(m->pf.mem);
   if (m->res_host) cudaFreeHost(m->res_host);
   delete m;
 }
@@ -1544,7 +1585,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
     CK(ctl_write(m, b, c));
   }
   // the dense path's rows: LLB_PREFILL=fast (dense FFN only) everything but the last k + 1, else as px_takes says; without room for its buffers
-  // mode 0 goes on in T-row passes
+  // mode 0 goes on in T-row passes, and mode 1, which asked for it, is an error
   bool any_exact = false;
   {
     std::vector<int> fast(nb, 0), exact(nb, 0);
@@ -1554,9 +1595,13 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
       else if (px_takes(m, ns[i] - 1)) { exact[i] = ns[i] - 1; any_exact = true; }
     }
     std::unique_lock<std::mutex> hold(pf_owner(m)->pf.busy, std::defer_lock);
-    if (any_fast || any_exact) hold.lock();
+    if (any_fast || any_exact) {
+      hold.lock();
+      const int rc = pf_alloc(m);
+      if (rc < 0 || (rc && any_fast)) return -1;
+      if (rc) any_exact = false;
+    }
     if (any_fast) CK(pf_prefill(m, nb, bs, ids, fast.data(), true));
-    if (any_exact && pf_alloc(m)) { cudaGetLastError(); any_exact = false; }
     if (any_exact) CK(pf_prefill(m, nb, bs, ids, exact.data(), false));
     for (int i = 0; i < nb; i++) p[i] = fast[i] + (any_exact ? exact[i] : 0);
   }
@@ -1963,7 +2008,7 @@ LLB_API int llb_spec_read_state_stream(llb_spec *m, int stream, int what, int il
     return (int)have;
   }
   else if (what == 4 && pos < (m->B > 1 ? m->Tspec : SPEC_MAXT)) { have = m->d; src = m->hn + (size_t)((m->B > 1 ? b * m->Tspec : 0) + pos) * m->d; }
-  else if (what == 6 && pf_owner(m)->pf.ready && pos >= 0 && pos < PF_RMAX) { have = m->d; src = pf_owner(m)->pf.hn + (size_t)(pos + 1) * m->d; }   // dense path: normed hidden of row `pos` of its last chunk
+  else if (what == 6 && pf_owner(m)->pf.mem && pos >= 0 && pos < PF_RMAX) { have = m->d; src = pf_owner(m)->pf.hn + (size_t)(pos + 1) * m->d; }   // dense path: normed hidden of row `pos` of its last chunk
   else return llb_fail("read_state: nothing of kind %d in layer %d", what, il);
   if (n < have) return llb_fail("read_state: buffer of %zu floats, %zu needed", n, have);
   CU_OK(cudaMemcpy(out, src, have * 4, cudaMemcpyDeviceToHost));

@@ -6,6 +6,8 @@
 // The arithmetic follows the CPU engine (tools/qwen35_engine.c:510-761) like the T-row kernels of ops_model.cu; what
 // differs is the order of the GEMMs' sums (pfx.cuh, pfmm.cuh) and that a DeltaNet layer scans the chunk's rows in one
 // kernel with the state in registers, writing the state once.
+#include <mutex>
+
 #include "pfmm.cuh"
 #include "pfx.cuh"
 #include "pfatt.cuh"
@@ -38,7 +40,7 @@ template <int FMT> static int px_attr2() { return px_attr(k_pfx2<FMT>, px2_smem(
 #define PF_SCAN_SMEM (220 * 1024)
 __global__ void k_pf_scan(const PfSegs sg, const float *__restrict__ y, const float *__restrict__ gram, const float *__restrict__ beta, const float *__restrict__ decay, DeltaShape sh,
                           float *__restrict__ o);
-int pf_setup(void) {
+static int setup(void) {
   if (pf_attr<LLB_FM_Q6_K>() || pf_attr<LLB_FM_Q8_0>()) return -1;
   if (px_attr1<LLB_FM_Q4_K>() || px_attr1<LLB_FM_Q5_K>() || px_attr1<LLB_FM_Q6_K>() || px_attr1<LLB_FM_Q8_0>() || px_attr2<LLB_FM_Q4_K>() || px_attr2<LLB_FM_Q5_K>()) return -1;
   if (px_attr(k_pf_attn<128>, pa_smem(128), PA_REG_LAUNCH) || px_attr(k_pf_attn<256>, pa_smem(256), PA_REG_LAUNCH)) return -1;
@@ -53,6 +55,14 @@ int pf_setup(void) {
     CU_OK(cudaMemset(g_pf_err, 0, 4));
   }
   return 0;
+}
+// 1 where the device has no room for the kernels
+int pf_setup(void) {
+  static std::mutex one;
+  std::lock_guard<std::mutex> hold(one);
+  cudaGetLastError();
+  const int rc = setup();
+  return rc && cudaGetLastError() == cudaErrorMemoryAllocation ? 1 : rc;
 }
 int pf_wait_errors(void) {
   unsigned int v = 0;

@@ -19,7 +19,7 @@ struct PfArgs {
 };
 
 
-int pf_setup(void);
+int pf_setup(void);                               // -1, or 1: no room on the device
 int pf_wait_errors_clear(void);
 int pf_wait_errors(void);                         // 1 when a bounded wait of the dense GEMM ran out
 int pf_pick_ksplit(int ntiles, int nsb, int sms);

@@ -82,7 +82,7 @@ def lib() -> C.CDLL:
             "llb_spec_cycle_streams": (i32, [vp, vp, vp, vp]), "llb_spec_run_cycles_streams": (i32, [vp, i32, vp]),
             "llb_spec_position_stream": (i32, [vp, i32]), "llb_spec_stats_stream": (i32, [vp, i32, vp]),
             "llb_spec_read_state_stream": (i32, [vp, i32, i32, i32, i32, vp, sz]),
-            "llb_spec_set_prefill": (i32, [vp, i32]), "llb_spec_fast_rows": (C.c_double, [vp]),
+            "llb_spec_set_prefill": (i32, [vp, i32]), "llb_spec_fast_rows": (C.c_double, [vp]), "llb_spec_prefill_extra": (i32, [vp, C.c_size_t]),
             "llb_b200_pf_gemm": (i32, [i32, u64, i32, i32, u64, i32, u64, i32]),
             "llb_b200_gemm_fits": (i32, [i32, i32, i32, i32]), "llb_b200_gemm_kernel": (i32, [i32, i32, i32, i32, i32, i32, C.POINTER(i32)]),
             "llb_b200_gemm3_trace": (i32, [i32, i32, i32, i32, C.POINTER(i32), i32]), "llb_b200_gemm3_bar_count": (i32, [i32, i32]),

@@ -295,6 +295,9 @@ LLB_API int llb_spec_position(const llb_spec *m);
  * llb_spec_fast_rows: prompt rows that mode 1 put through the dense path since the engine was opened. */
 LLB_API int llb_spec_set_prefill(llb_spec *m, int mode);
 LLB_API double llb_spec_fast_rows(const llb_spec *m);
+/* Test entry: bytes that the dense path's buffers take beyond their need when the next prompt allocates them; more than the GPU has stands for
+ * a GPU with no room. */
+LLB_API int llb_spec_prefill_extra(llb_spec *m, size_t bytes);
 /* n cycles enqueued back to back, no host round trip between them; returns the tokens emitted */
 LLB_API int llb_spec_run_cycles(llb_spec *m, int n, int *ids, int cap);
 /* measurement helpers: device time (CUDA events on the library's stream) of the verify pass alone and

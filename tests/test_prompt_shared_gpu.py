@@ -84,3 +84,43 @@ def test_prompt_between_another_ones_prompt_and_cycles(pkg, packs, model):
     assert _same(_result(engs[1], cfg), other)
     for e in engs:
         e.close()
+
+
+def test_no_room(pkg, packs, model, monkeypatch):
+    """No room for the prompt path's buffers: a default prompt goes through T-row passes, one of mode 1 is refused; once there is room both take them."""
+    cfg, L = model[0].cfg, pkg.llb.lib()
+    p = packs.synth_prompt(80, 140, cfg.vocab_size)
+
+    def alone(fast):
+        eng = pkg.llb.SpecEngine(model[0], model[1], k=3, max_ctx=200)
+        eng.set_prefill(fast)
+        eng.prefill(p)
+        r = _result(eng, cfg)
+        eng.close()
+        return r
+
+    want = [alone(False), alone(True)]
+    monkeypatch.setenv("LLB_PREFILL_ROWS", "8")
+    t_rows = alone(False)
+    monkeypatch.delenv("LLB_PREFILL_ROWS")
+    assert not _same(t_rows, want[0])      # (sums in another order: which path a prompt took shows)
+    engs = _open(pkg, model, 2)
+    engs[1].close()
+    first, sib = engs[0], engs[0].sibling(k=3, max_ctx=200)
+    for _ in range(2):
+        L.llb_spec_prefill_extra(first.h, 1 << 50)
+        for e in (first, sib):
+            e.set_prefill(False)
+            e.prefill(p)
+            assert _same(_result(e, cfg), t_rows)
+            e.set_prefill(True)
+            with pytest.raises(Exception, match="buffers take"):
+                e.prefill(p)
+    L.llb_spec_prefill_extra(sib.h, 0)
+    for fast in (False, True):
+        for e in (sib, first):
+            e.set_prefill(fast)
+            e.prefill(p)
+            assert _same(_result(e, cfg), want[fast])
+    sib.close()
+    first.close()
