@@ -48,6 +48,9 @@ struct PfState {
   std::mutex busy;
   void *mem = nullptr;
   size_t extra = 0;                   // llb_spec_prefill_extra
+  const llb_spec *last = nullptr;     // whose chunk was the last, and that chunk's pieces: stream, first row in hn, rows
+  struct Kept { int b, row, n; };
+  std::vector<Kept> kept;
   float *x = nullptr, *x1 = nullptr, *hn = nullptr, *e = nullptr, *qn = nullptr, *y = nullptr, *gram = nullptr, *beta = nullptr, *decay = nullptr, *o = nullptr;
   __half *kg_d = nullptr, *kg_f = nullptr, *kg_qa = nullptr, *kg_v = nullptr, *kg_2d = nullptr;
   OutBuf q, k, v, qkv, z, bp, ap, a, g, u, dn, eh;
@@ -1205,7 +1208,9 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
   const int d = m->d, qa = m->H * m->hd, kvd = m->KV * m->hd;
   int R = 0;
   std::vector<int> ids;
+  f.last = nullptr; f.kept.clear();
   for (PfPiece &p : pc) {
+    f.kept.push_back({p.b, R + (int)f.kept.size() + 1, p.R});
     p.off = R; R += p.R;
     ids.insert(ids.end(), p.ids + p.p0, p.ids + p.p0 + p.R);
   }
@@ -1271,6 +1276,7 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
     float *dst = m->hn_pf + (size_t)(m->B > 1 ? p.b * m->Tpf : 0) * d;
     CU_OK(cudaMemcpyAsync(dst, f.hn + (size_t)(p.off + i + p.R - keep + 1) * d, (size_t)keep * d * 4, cudaMemcpyDeviceToDevice, s));
   }
+  f.last = m;
   return 0;
 }
 
@@ -1507,6 +1513,7 @@ LLB_API void llb_spec_close(llb_spec *m) {
   cudaStreamSynchronize(g_llb.stream);
   if (m->sharers > 0) { m->closed = true; return; }   // its weights are in use: freed when the last sibling closes
   if (llb_spec *first = m->share) {
+    { std::lock_guard<std::mutex> hold(first->pf.busy); if (first->pf.last == m) first->pf.last = nullptr; }
     m->share = nullptr;
     first->sharers -= 1;
     if (first->sharers == 0 && first->closed) llb_spec_close(first);
@@ -2008,7 +2015,18 @@ LLB_API int llb_spec_read_state_stream(llb_spec *m, int stream, int what, int il
     return (int)have;
   }
   else if (what == 4 && pos < (m->B > 1 ? m->Tspec : SPEC_MAXT)) { have = m->d; src = m->hn + (size_t)((m->B > 1 ? b * m->Tspec : 0) + pos) * m->d; }
-  else if (what == 6 && pf_owner(m)->pf.mem && pos >= 0 && pos < PF_RMAX) { have = m->d; src = pf_owner(m)->pf.hn + (size_t)(pos + 1) * m->d; }   // dense path: normed hidden of row `pos` of its last chunk
+  else if (what == 6) {   // dense path: normed hidden of row `pos` of the stream's piece of its last chunk, while no sibling's came after it
+    PfState &f = pf_owner(m)->pf;
+    std::lock_guard<std::mutex> hold(f.busy);
+    const float *row = nullptr;
+    if (f.last == m)
+      for (const PfState::Kept &k : f.kept) if (k.b == b && pos >= 0 && pos < k.n) row = f.hn + (size_t)(k.row + pos) * m->d;
+    if (!row) return llb_fail("read_state: the prompt path's last chunk has no row %d of stream %d of this engine", pos, b);
+    if (n < (size_t)m->d) return llb_fail("read_state: buffer of %zu floats, %d needed", n, m->d);
+    CU_OK(cudaMemcpyAsync(out, row, (size_t)m->d * 4, cudaMemcpyDeviceToHost, g_llb.stream));
+    CU_OK(cudaStreamSynchronize(g_llb.stream));
+    return m->d;
+  }
   else return llb_fail("read_state: nothing of kind %d in layer %d", what, il);
   if (n < have) return llb_fail("read_state: buffer of %zu floats, %zu needed", n, have);
   CU_OK(cudaMemcpy(out, src, have * 4, cudaMemcpyDeviceToHost));

@@ -124,3 +124,22 @@ def test_no_room(pkg, packs, model, monkeypatch):
             assert _same(_result(e, cfg), want[fast])
     sib.close()
     first.close()
+
+
+def test_rows_of_the_last_chunk(pkg, packs, model):
+    """read_state of kind 6: a stream's own rows of a chunk that several streams share, and nothing once a sibling's chunk came after it."""
+    cfg = model[0].cfg
+    first = pkg.llb.SpecEngine(model[0], model[1], k=3, max_ctx=360)
+    eng, lens = first.sibling(k=3, max_ctx=360, streams=3), (41, 31, 21)
+    eng.prefill_streams([packs.synth_prompt(50 + b, n, cfg.vocab_size) for b, n in enumerate(lens)])
+    for b, n in enumerate(lens):
+        for r in range(4):          # the rows left for the drafter are the piece's last
+            assert np.array_equal(eng.read_state_stream(b, 6, 0, n - 1 - 4 + r), eng.read_state_stream(b, 4, 0, r)), (b, r)
+        with pytest.raises(Exception, match="no row"):
+            eng.read_state_stream(b, 6, 0, n - 1)
+    first.prefill(packs.synth_prompt(55, 150, cfg.vocab_size))
+    with pytest.raises(Exception, match="no row"):
+        eng.read_state_stream(0, 6, 0, 0)
+    assert np.array_equal(first.read_state(6, 0, 149 - 128 - 1), first.read_state(4, 0, 3))
+    eng.close()
+    first.close()
