@@ -1652,6 +1652,7 @@ static int prefill_many(llb_spec *m, int nb, const int *bs, const int *const *id
     for (int i = 0; i < nb; i++)
       CU_OK(cudaMemcpyAsync(m->hn + (size_t)bs[i] * m->Tspec * m->d, m->hn_pf + (size_t)bs[i] * m->Tpf * m->d, (size_t)m->Tspec * m->d * 4, cudaMemcpyDeviceToDevice, g_llb.stream));
   for (int o = 0; o < m->B; o++) if (kept[o]) CK(ctl_write(m, o, keep[o]));
+  if (any_exact) CU_OK(cudaStreamSynchronize(g_llb.stream));   // as behind the last T-row pass: nothing of the prompt is left to the next call
   for (int i = 0; i < nb; i++) {
     SeqHost &q = m->sq[bs[i]];
     q.pos = ns[i] - 1;        // n == 1: nothing ran, the first cycle starts at position 0 with the single prompt token

@@ -83,3 +83,19 @@ def test_streams_together_and_in_turn(pkg, packs, llb):
     assert out[0][0] == out[1][0]
     for a, b in zip(out[0][1], out[1][1]):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("streams", [1, 3])
+def test_nothing_is_left_to_the_next_call(pkg, packs, llb, streams):
+    """The library's stream is idle when a prompt's call returns, the pass over its last rows' logits included (a head that takes a while)."""
+    import torch
+    pack = packs.build_pack(packs.cfg_tiny(n_layers=4, seed=33, vocab_size=200000))
+    eng = pkg.llb.SpecEngine(pack, None, k=0, max_ctx=96, streams=streams)
+    try:
+        stream = torch.cuda.ExternalStream(pkg.llb.lib().llb_b200_stream())
+        prompts = [packs.synth_prompt(300 + b, 40, pack.cfg.vocab_size) for b in range(streams)]
+        for _ in range(5):
+            eng.prefill_streams(prompts) if streams > 1 else eng.prefill(prompts[0])
+            assert stream.query()
+    finally:
+        eng.close()
