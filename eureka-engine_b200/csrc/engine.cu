@@ -1280,14 +1280,15 @@ static int pf_chunk(llb_spec *m, std::vector<PfPiece> &pc) {
   return 0;
 }
 
-// Whether mode 0 puts a prompt of n_rows through the dense path: where T-row passes of k <= 3 would read the weights more than once for it.  It then takes all
-// of them, and neither their number nor the rule knows k or the other streams: a prompt leaves the same bits behind in every engine.
+// Whether mode 0 puts a prompt of n_rows through the dense path: where T-row passes would read the weights more than once for it, which with k <= 3 is from five rows
+// on, beyond that from k + 2.  It then takes all of them, and neither their number nor the other streams' matters: a prompt of more than eight rows leaves the same bits
+// behind in every engine, a shorter one in every engine of k <= 3.
 // (27B shape: a T-row pass of up to eight rows 6.8 ms, the last of them with the k + 1 rows in front of the first cycle; a piece of up to 32 rows 9.7, up to 128 13
 // to 16.  0.8B shape 0.85, 1.5, 1.8 to 2.1.)
 static int ctl_write(llb_spec *m, int b, const SpecCtl &c);
 static SpecCtl ctl_fresh(const llb_spec *m, int b);
 static bool px_takes(const llb_spec *m, int n_rows) {
-  return n_rows > SPEC_MAXT / 2 && !m->rows_set && m->ne == 0 && m->tp.size <= 1 && m->KC <= CONV_RING / 2 && m->d <= 16384;
+  return n_rows > (m->Tspec > SPEC_MAXT / 2 ? m->Tspec : SPEC_MAXT / 2) && !m->rows_set && m->ne == 0 && m->tp.size <= 1 && m->KC <= CONV_RING / 2 && m->d <= 16384;
 }
 // The dense part of the prompts of streams bs[i] (take[i] rows of ids[i] from position 0 on; 0: none), mode 1 a stream after the other in
 // chunks of PF_RMAX rows, mode 0 in pieces of PF_R rows, several streams' together as far as they fit.  Mode 1: a stream's drafter row at the

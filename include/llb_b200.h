@@ -284,9 +284,9 @@ LLB_API int llb_spec_generate(llb_spec *m, int steps, int *ids, uint32_t *top2);
 /* the reference's per-token operator (spec_pass, host/llb_host.c:1902-1950): y = [v1, id1, v2, id2] */
 LLB_API int llb_spec_pass(llb_spec *m, int pos, int tok, float *y);
 LLB_API int llb_spec_position(const llb_spec *m);
-/* How llb_spec_prefill feeds a prompt.  mode 0 (default): at the verify path's precision; more than four rows in pieces of up to 128
+/* How llb_spec_prefill feeds a prompt.  mode 0 (default): at the verify path's precision; more than four rows, and more than k + 1, in pieces of up to 128
  * rows through dense tcgen05 GEMMs on the exact weight codes, fewer (and every row of a model with routed experts, of a tensor-parallel rank, and
- * where LLB_PREFILL_ROWS was set at open) through T-row verify passes.  What a prompt leaves behind depends on neither k nor the other streams.
+ * where LLB_PREFILL_ROWS was set at open) through T-row verify passes.  What the dense path leaves behind depends on neither k nor the other streams.
  * mode 1 (also LLB_PREFILL=fast in the environment at open, the reference's switch,
  * host/llb_host.c:206): all but the last k + 1 rows in chunks of 256 rows through dense tcgen05 GEMMs (Q6_K and Q8_0 weights as two fp16 planes)
  * (replaces pf_take / spec_pf / spec_take, host/llb_pf.h:551, host/llb_host.c:1831-1899): trunk K/V, conv history and

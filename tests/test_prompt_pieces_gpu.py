@@ -1,4 +1,4 @@
-"""Prompts in mode 0 (llb_spec_set_prefill(0)): more than four rows go through the dense path's exact forms in pieces of 128 rows, whole, without a
+"""Prompts in mode 0 (llb_spec_set_prefill(0)): more than four rows (and k + 1) go through the dense path's exact forms in pieces of 128 rows, whole, without a
 T-row pass behind them.  Against T-row passes (LLB_PREFILL_ROWS) on the same model: state, K/V rows, the rows left for the drafter, logits of
 the last prompt row, ids; the same bits whatever k is and whether several streams' prompts are fed together or in turn."""
 import numpy as np
@@ -55,6 +55,28 @@ def test_pieces_against_t_row_passes(pkg, packs, llb, monkeypatch, n):
         if ids[i] != runs[3][1][i]:
             assert _f(t2[i])[1] - _f(t2[i])[3] < 1e-3, i
             break
+
+
+@pytest.mark.parametrize("k", [4, 7])
+def test_prompts_that_one_t_row_pass_takes(pkg, packs, llb, monkeypatch, k):
+    """With k >= 4 a prompt of five to k + 1 rows is one T-row pass and stays that; one row more takes the dense path, as with any k."""
+    pack = packs.build_pack(packs.cfg_tiny(n_layers=4, seed=34, quant="q4_k_m"))
+    mtp = packs.aux1_bytes(packs.build_mtp(pack))
+
+    def state(kk, rows):
+        eng = pkg.llb.SpecEngine(pack, mtp, k=kk, max_ctx=96)
+        try:
+            eng.prefill(packs.synth_prompt(rows, rows + 1, pack.cfg.vocab_size))
+            return np.concatenate([eng.read_state(0, il) for il in range(pack.cfg.n_layers) if not pack.cfg.is_full(il)]).view(np.uint32)
+        finally:
+            eng.close()
+
+    one, more, dense = state(k, k + 1), state(k, k + 2), state(3, k + 2)
+    assert np.array_equal(more, dense)
+    assert not np.array_equal(one, state(3, k + 1))
+    monkeypatch.setenv("LLB_PREFILL_ROWS", "8")
+    assert np.array_equal(one, state(k, k + 1))
+    assert not np.array_equal(more, state(k, k + 2))
 
 
 def test_streams_together_and_in_turn(pkg, packs, llb):
