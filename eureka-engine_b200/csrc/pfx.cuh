@@ -4,7 +4,9 @@
 //
 //   Q4_K, Q5_K  sc (q - 8) and sc (q - 16), at most 504 and 1008.  What the centring took and the mins are one more K = 16 step of a
 //               super-block, 32 (8 sc - (dmin / d) m) as two fp16 halves against the means of the activations' 32-column groups
-//   Q6_K        sc (l - 8) and 8 sc (2 h - 3), l the code's low four bits and h its high two: two planes, both exact
+//   Q6_K        sc (q - 32), at most 4096: fp16 product and its exact remainder, two planes.  (Planes of the code's low four and high two bits are exact too and cheaper to
+//               unpack, but they are large and cancel where codes are small: with weights of N^3 and activations of one sign, 17408 columns, what is truncated off
+//               their sums came to 2.9e-6 of the result)
 //   Q8_0        d q with the eight d's of the super-block scaled by a common power of two: fp16 product and its exact remainder, two planes
 //
 // and the activations are their two fp16 planes, so the products are exact but for the activations' 22 bits.  The accumulators of a
@@ -188,7 +190,8 @@ template <int FMT, int P = 1> __device__ __forceinline__ void px_stage(const uin
     }
   } else if constexpr (FMT == LLB_FM_Q6_K) {
     const int hf = s >> 1, odd = s & 1;
-    const uint32_t scw = px_pick(h.w, s), nm = odd ? 0x00f000f0u : 0x000f000fu;
+    // codes as fp16 subnormals q 2^-24, those of high nibbles four bits up, then (q - 32) 2^-9 times sc 2^-7
+    const uint32_t scw = px_pick(h.w, s), nm = odd ? 0x00f000f0u : 0x000f000fu, hm = odd ? 0x03000300u : 0x00300030u, up = odd ? 0x68006800u : 0x78007800u;
 #pragma unroll
     for (int i2 = 0; i2 < 2 / P; i2++) {       // sixteen columns 16 c .. of both quarters
       const int c = P == 2 ? part : i2;
@@ -197,18 +200,18 @@ template <int FMT, int P = 1> __device__ __forceinline__ void px_stage(const uin
 #pragma unroll
       for (int qq = 0; qq < 2; qq++) {
         const uint32_t sv = g2_hadd2(__byte_perm(scw, 0x64646464u, 0x4040u + 0x0101u * (2 * qq + c)), 0xe480e480u);   // (1024 + 128 + sc) - 1152
-        // low bits: l 2^-24 * sc 2^8 (four bits up: sc 2^4) - 8 sc 2^-16;  high bits, p = 4 or 6 bits up: h 2^(p - 24) * sc 2^(12 - p) - 24 sc 2^-16
-        const uint32_t S = g2_hmul2(sv, odd ? 0x4c004c00u : 0x5c005c00u), S8 = g2_hmul2(S, odd ? 0x80808080u : 0x80088008u);
-        const uint32_t M = g2_hmul2(sv, qq ? 0x54005400u : 0x5c005c00u), M24 = g2_hmul2(M, qq ? 0x80608060u : 0x80188018u);
-        const uint32_t hm = qq ? 0x00c000c0u : 0x00300030u;
+        const uint32_t S = g2_hmul2(sv, 0x20002000u);
         const uint4 l4 = *(const uint4 *)(row + 64 * hf + 32 * qq + 16 * c);
         const uint32_t lw[4] = {l4.x, l4.y, l4.z, l4.w};
         uint32_t P1[8], P2[8];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          const uint32_t e = hw[i] << (4 - 4 * odd), f = hw[i] >> (4 + 4 * odd);
-          P2[2 * i] = g2_hfma2(lw[i] & nm, S, S8); P2[2 * i + 1] = g2_hfma2((lw[i] >> 8) & nm, S, S8);
-          P1[2 * i] = g2_hfma2(e & hm, M, M24); P1[2 * i + 1] = g2_hfma2(f & hm, M, M24);
+          const uint32_t a0 = (lw[i] & nm) | (hw[i] << (4 - 2 * qq) & hm), a1 = ((lw[i] >> 8) & nm) | (hw[i] >> (4 + 2 * qq) & hm);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const uint32_t x = g2_hfma2(e ? a1 : a0, up, 0xac00ac00u), p = g2_hmul2(x, S);
+            P1[2 * i + e] = p; P2[2 * i + e] = g2_hfma2(x, S, p ^ 0x80008000u);
+          }
         }
         const int g = 4 / P * qq + 2 * i2;
         o[g] = make_uint4(P1[0], P1[1], P1[2], P1[3]); o[g + 1] = make_uint4(P1[4], P1[5], P1[6], P1[7]);

@@ -66,3 +66,20 @@ def test_scales_of_many_magnitudes(llb, packs, oracle, dev, ty, R):
     mass = np.abs(x).astype(np.float64) @ (np.abs(deq) + 2 * mins).T
     bar = 1e-5 if R > 128 and ty in ("Q6_K", "Q8_0") else 3e-6
     assert np.all(np.abs(got - ref) <= bar * mass + 1e-6), float((np.abs(got - ref) / (mass + 1e-9)).max())
+
+
+@pytest.mark.parametrize("power", [1, 3])
+def test_sums_do_not_climb(llb, packs, oracle, dev, power):
+    """Q6_K on activations of one sign, many columns: the planes of codes, of weights with heavy tails too, have no part that cancels between them and that truncated
+    sums would add up."""
+    rows, K = 512, 17408
+    rng = np.random.default_rng(9)
+    raw = packs.quant_q6_k(torch.from_numpy(rng.standard_normal((rows, K), dtype=np.float32) ** power * 0.02)).numpy()
+    deq = oracle.Oracle.deq_rows(packs.FMT["Q6_K"], raw, rows, K).astype(np.float64)
+    err = {}
+    for kind in ("N", "|N|"):
+        x = rng.standard_normal((40, K), dtype=np.float32)
+        x = x if kind == "N" else np.abs(x)
+        ref = x.astype(np.float64) @ deq.T
+        err[kind] = np.linalg.norm(_run(llb, packs, dev, "Q6_K", raw, rows, K, x, 4) - ref) / np.linalg.norm(ref)
+    assert err["|N|"] < 1.25 * err["N"], err
