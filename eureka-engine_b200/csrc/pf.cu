@@ -32,7 +32,7 @@ template <typename K> static int px_attr(K k, int smem, int regs) {
 }
 template <int FMT> static int px_attr1() {
   CU_OK(cudaFuncSetAttribute(k_pft<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, pt_smem(FMT)));
-  return px_attr(k_pfx1<FMT, 64>, px_smem(FMT, 64), PX1_REG_LAUNCH) || px_attr(k_pfx1<FMT, 128>, px_smem(FMT, 128), PX1_REG_LAUNCH);
+  return px_attr(k_pfx1<FMT, 64>, px_smem(FMT, 64), px1_reg_launch(FMT, 64)) || px_attr(k_pfx1<FMT, 128>, px_smem(FMT, 128), px1_reg_launch(FMT, 128));
 }
 template <int FMT> static int px_attr2() { return px_attr(k_pfx2<FMT>, px2_smem(FMT), PX_REG_LAUNCH); }
 #define PF_SCAN_NW 4                            // warps of a scan block, 8 state rows each
@@ -100,8 +100,8 @@ int pf_gemm(cudaStream_t s, int fmt, PfArgs &a) {
   const int grid = 2 * (units < g_llb.sms / 2 ? units : g_llb.sms / 2);
   cudaError_t e = cudaErrorInvalidValue;
   const int ru = pf_unit_rows(a.R);
-#define PT_GO(F) e = llb_launch(k_pft<F>, dim3(grid), dim3(PX1_THREADS), (size_t)pt_smem(F), s, a)
-#define PX_GO(F, RU) e = llb_launch(k_pfx1<F, RU>, dim3(grid), dim3(PX1_THREADS), (size_t)px_smem(F, RU), s, a)
+#define PT_GO(F) e = llb_launch(k_pft<F>, dim3(grid), dim3(PT_THREADS), (size_t)pt_smem(F), s, a)
+#define PX_GO(F, RU) e = llb_launch(k_pfx1<F, RU>, dim3(grid), dim3(px1_threads(F, RU)), (size_t)px_smem(F, RU), s, a)
 #define PX_ONE(F) do { if (ru == 32) PT_GO(F); else if (ru == 64) PX_GO(F, 64); else PX_GO(F, 128); } while (0)
 #define PX_TWO(F) e = llb_launch(k_pfx2<F>, dim3(grid), dim3(PX_THREADS), (size_t)px2_smem(F), s, a)
   switch (fmt) {
@@ -822,9 +822,10 @@ static void pt_forward(PfTrace &t, int NB, int slots) {
 static void pt_both(PfTrace &t, int b) { t.later(b); t.later(PT_BARS + b); }
 template <int FMT, int RU> static int px1_trace(PfTrace &t, int units, int nsl, int agent) {
   constexpr int NA = px_na(FMT), NB = px_nb(FMT), BS = px_slot_stages(RU), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), SS = px_sub(FMT);
-  const int rank = agent / 20, w = agent % 20, me = rank * PT_BARS;
-  if (agent >= 40) return -1;
-  if (w < 8) {
+  constexpr int UW = px1_unpack(FMT, RU), AG = UW + 12;
+  const int rank = agent / AG, w = agent % AG, me = rank * PT_BARS;
+  if (agent >= 2 * AG) return -1;
+  if (w < UW) {
     int k = 0, rk = 0, jj = 0;
     for (int u = 0; u < units; u++)
       for (int c = 0; c < nsl; c++, jj++) {
@@ -836,9 +837,9 @@ template <int FMT, int RU> static int px1_trace(PfTrace &t, int units, int nsl, 
         }
         if (c % CH == CH - 1 || c == nsl - 1) { t.arrive(me + PT_RAW_EMPTY + rk % NRAW); rk++; }
       }
-  } else if (w == 8) pt_weights(t, me, NRAW, CH, units, nsl);
-  else if (w == 9) pt_activations(t, rank, NB, units * (4 * nsl / BS));
-  else if (w == 10 && rank == 0) {
+  } else if (w == UW) pt_weights(t, me, NRAW, CH, units, nsl);
+  else if (w == UW + 1) pt_activations(t, rank, NB, units * (4 * nsl / BS));
+  else if (w == UW + 2 && rank == 0) {
     int k = 0, bk = 0;
     for (int i = 0; i < units * nsl * 4; i += SS, k++) {
       if (k > 1) t.wait(PT_D_EMPTY + (k & 1), (k >> 1) - 1);
@@ -850,8 +851,8 @@ template <int FMT, int RU> static int px1_trace(PfTrace &t, int units, int nsl, 
         if (in == BS - 1) { pt_both(t, PT_B_EMPTY + bk % NB); bk++; }
       }
     }
-  } else if (w == 11 && rank == 1) pt_forward(t, NB, units * (4 * nsl / BS));
-  else if (w >= 12) {
+  } else if (w == UW + 3 && rank == 1) pt_forward(t, NB, units * (4 * nsl / BS));
+  else if (w >= UW + 4) {
     for (int jj = 0, k = 0; jj < units * nsl; jj++) {
       t.wait(me + PT_SC + (jj & 3), jj >> 2);
       for (int p = 0; p < 4 / SS; p++, k++) { t.wait(me + PT_D_FULL + (k & 1), k >> 1); t.arrive(PT_D_EMPTY + (k & 1)); }
@@ -859,7 +860,7 @@ template <int FMT, int RU> static int px1_trace(PfTrace &t, int units, int nsl, 
   }
   return t.n;
 }
-static int px1_count(int b) { return b < 8 || (b >= 32 && b < 36) ? 16 : b >= 16 && b < 20 ? 2 : b >= 36 && b < 40 ? 4 : b >= 44 ? 8 : 1; }
+static int px1_count(int b, int UW) { return b < 8 ? 2 * UW : b >= 32 && b < 36 ? 16 : b >= 16 && b < 20 ? 2 : b >= 36 && b < 40 ? 4 : b >= 44 ? UW : 1; }
 template <int FMT> static int pt_trace(PfTrace &t, int units, int nsl, int agent) {
   constexpr int NB = PT_NB, SPB = 4 / px_slot_stages(PT_RU), NP = pt_items(FMT), SI = 4 / NP, ND = 128 / (2 * PT_RU), CH = px_chunk(FMT), NRAW = pt_raws(FMT);
   const int rank = agent / 20, w = agent % 20, me = rank * PT_BARS;
@@ -960,7 +961,7 @@ int llb_b200_pf_trace(int kernel, int form, int fmt, int units, int nsl, int age
 }
 // arrivals that complete a phase of barrier `bar`
 extern "C" __attribute__((visibility("default")))
-int llb_b200_pf_bar_count(int kernel, int form, int bar) {
+int llb_b200_pf_bar_count(int kernel, int form, int fmt, int bar) {
   bar %= PT_BARS;
-  return kernel == 0 ? pa_count(bar) : kernel == 2 ? px2_count(bar) : form == 32 ? pt_count(bar) : px1_count(bar);
+  return kernel == 0 ? pa_count(bar) : kernel == 2 ? px2_count(bar) : form == 32 ? pt_count(bar) : px1_count(bar, px1_unpack(fmt, form));
 }

@@ -54,6 +54,7 @@ __host__ __device__ constexpr int px_drain(int fmt) { return px_planes(fmt) == 2
 #define PX_SLOT 16384
 #define PT_RU 32              // rows of k_pft, the kernel of the fewest
 #define PT_NB 4               // its slots: its two groups have two each
+#define PT_THREADS 640        // warps 0-7 unpack, 8 loads weights, 9 activations, 10 and 11 issue MMAs (in the second CTA 11 forwards), 12-19 read accumulators
 __host__ __device__ constexpr int px_sub(int fmt) { return 3 - px_planes(fmt); }     // 64-column parts of a stage
 __host__ __device__ constexpr int px_na(int fmt) { return px_planes(fmt) == 2 ? 3 : 2; }
 __host__ __device__ constexpr int px_slot_stages(int RU) { return PX_SLOT / px_b_bytes(RU); }
@@ -83,13 +84,18 @@ static_assert(px2_smem(LLB_FM_Q5_K) <= PX_SMEM_MAX, "k_pfx2's rings");
 #define PX_REG_READ 192
 #define PX_REG_LAUNCH 128
 static_assert(PX_REG_UNPACK + PX_REG_ISSUE + 2 * PX_REG_READ == 4 * PX_REG_LAUNCH, "setmaxnreg.inc waits for ever where the shares are more than the launch's registers");
-// k_pfx1: warps 0-7 unpack, 8 loads weights, 9 activations, 10 issues MMAs, 11 forwards, 12-19 read accumulators
-#define PX1_THREADS 640
+// k_pfx1: eight warps unpack (four where a thread that reads has 128 sums, below: the registers are needed there, and the MMAs of 128 rows and two planes take longer
+// than four warps' unpacking), then one that loads weights, one activations, one issues MMAs, one forwards, eight read accumulators
+__host__ __device__ constexpr int px1_unpack(int fmt, int RU) { return px_planes(fmt) == 2 && RU == 128 ? 4 : 8; }
+__host__ __device__ constexpr int px1_threads(int fmt, int RU) { return 32 * (px1_unpack(fmt, RU) + 12); }
 #define PX1_REG_UNPACK 80
-#define PX1_REG_ISSUE 64
-#define PX1_REG_READ 128
-#define PX1_REG_LAUNCH 96
-static_assert(2 * PX1_REG_UNPACK + PX1_REG_ISSUE + 2 * PX1_REG_READ == 5 * PX1_REG_LAUNCH, "as above");
+__host__ __device__ constexpr int px1_reg_issue(int fmt, int RU) { return px1_unpack(fmt, RU) == 4 ? 48 : 64; }
+__host__ __device__ constexpr int px1_reg_read(int fmt, int RU) { return px1_unpack(fmt, RU) == 4 ? 192 : 128; }
+__host__ __device__ constexpr int px1_reg_launch(int fmt, int RU) { return px1_unpack(fmt, RU) == 4 ? 128 : 96; }
+constexpr bool px1_split(int fmt, int RU) {
+  return px1_unpack(fmt, RU) / 4 * PX1_REG_UNPACK + px1_reg_issue(fmt, RU) + 2 * px1_reg_read(fmt, RU) == px1_threads(fmt, RU) / 128 * px1_reg_launch(fmt, RU);
+}
+static_assert(px1_split(LLB_FM_Q4_K, 64) && px1_split(LLB_FM_Q4_K, 128) && px1_split(LLB_FM_Q6_K, 64) && px1_split(LLB_FM_Q6_K, 128), "as above");
 __host__ __device__ constexpr uint32_t px_idesc(int N) { return 0x10000010u | ((uint32_t)(N >> 3) << 17); }   // kind::f16: D f32, A / B f16 K-major, M = 256 over the pair
 
 // ---- one 64-column stage s of a weight row's super-block into core-matrix rows of the code planes ----
@@ -253,14 +259,16 @@ template <int FMT, int P> __device__ __forceinline__ int px_group(int i, int par
   if constexpr (FMT == LLB_FM_Q8_0) return 4 * part + i;
   else return 4 * (i >> 1) + 2 * part + (i & 1);
 }
+// Sums of two planes: a super-block's four stages first, then the super-blocks.  One sum over all stages lost 2.5e-8 sqrt(stages / 2) of the result by its own rounding: 17408
+// columns in three slices 2.1e-7, so 1.5e-7, 5120 columns 1.46e-7, so 1.33e-7.  (Two super-blocks together, where a slice has many: 1.4e-7, but 2 to 4 % of a prompt's time.)
 template <int N> __device__ __forceinline__ void px_reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void px_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ---- the kernels: work units, tiles and slices as in pfmm.cuh.  Up to 128 prompt rows: ----
 template <int FMT, int RU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pfx1(const PfArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(px1_threads(FMT, RU), 1) k_pfx1(const PfArgs a) {
   constexpr int NA = px_na(FMT), NB = px_nb(FMT), BS = px_slot_stages(RU), NPL = px_planes(FMT), N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = px_raws(FMT, RU), SS = px_sub(FMT);
-  constexpr int RAWB = px_raw_bytes(FMT), AB = px_a_bytes(FMT), STB = SS * AB, SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU);
+  constexpr int RAWB = px_raw_bytes(FMT), AB = px_a_bytes(FMT), STB = SS * AB, SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU), UW = px1_unpack(FMT, RU);
   static_assert(NRAW >= 2 && px_smem(FMT, RU) <= PX_SMEM_MAX, "a form that does not fit");
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -287,15 +295,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
 
   pdl_trigger();
   if (tid == 0) {
-    for (int s = 0; s < NA; s++) { mbar_init(a_full(s), 16); mbar_init(a_empty(s), 1); }
+    for (int s = 0; s < NA; s++) { mbar_init(a_full(s), 2 * UW); mbar_init(a_empty(s), 1); }
     for (int s = 0; s < NB; s++) { mbar_init(b_full(s), 2); mbar_init(b_empty(s), 1); mbar_init(b_here(s), 1); }
     for (int b = 0; b < 2; b++) { mbar_init(d_full(b), 1); mbar_init(d_empty(b), 16); }
     for (int i = 0; i < 4; i++) mbar_init(sc_full(i), 4);
-    for (int i = 0; i < NRAW; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), 8); }
+    for (int i = 0; i < NRAW; i++) { mbar_init(raw_full(i), 1); mbar_init(raw_empty(i), UW); }
     *dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 10) {
+  if (warp == UW + 2) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
@@ -310,10 +318,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
     }
   };
 
-  if (warp < 8) {
-    // ---- codes: two threads a weight row (with one the unpacking of a super-block took 3250 cycles and paced the kernel) ----
+  if (warp < UW) {
+    // ---- codes: two threads a weight row (with one the unpacking of a super-block took 3250 cycles and paced the kernel), or one ----
     px_reg_dec<PX1_REG_UNPACK>();
-    const int r = tid & 127, part = tid >> 7, r16 = r & 15;
+    const int r = tid & 127, part0 = tid >> 7, r16 = r & 15;
     const uint32_t roff = (uint32_t)(r >> 4) * (CH * TB);
     int slot = 0, rs = 0, jj = 0;
     uint32_t par = 1, rpar = 0;             // (the first round's waits on empty barriers pass)
@@ -328,26 +336,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
         PxRow h;
         float scale;
         uint4 off[2];
-        px_head<FMT>(row, tile, r16, part == 0, h, scale, off);
+        px_head<FMT>(row, tile, r16, part0 == 0, h, scale, off);
 #pragma unroll 1
         for (int s = 0; s < 4; s += SS) {
           uint4 o[4 * NPL];
-          px_stage<FMT, 2>(row, s, part, h, o);
+          px_stage<FMT, 2>(row, s, part0, h, o);
           wait(a_empty(slot), par);
           uint8_t *A = ra + slot * STB + r * 16;
 #pragma unroll
-          for (int i = 0; i < 4 * NPL; i++) *(uint4 *)(A + (i >> 2) * PF_A_BYTES + px_group<FMT, 2>(i & 3, part) * 2048) = o[i];
-          if constexpr (SS == 2) {
-            px_stage<FMT, 2>(row, s + 1, part, h, o);
+          for (int i = 0; i < 4 * NPL; i++) *(uint4 *)(A + (i >> 2) * PF_A_BYTES + px_group<FMT, 2>(i & 3, part0) * 2048) = o[i];
+          if constexpr (UW == 4) {
+            px_stage<FMT, 2>(row, s, 1, h, o);
 #pragma unroll
-            for (int i = 0; i < 4; i++) *(uint4 *)(A + AB + px_group<FMT, 2>(i, part) * 2048) = o[i];
+            for (int i = 0; i < 4 * NPL; i++) *(uint4 *)(A + (i >> 2) * PF_A_BYTES + px_group<FMT, 2>(i & 3, 1) * 2048) = o[i];
           }
-          if (s == 0 && part == 0) {   // (the scales of the super-block four back have been read: its accumulators were, before the stages that were waited for here)
+          if constexpr (SS == 2) {
+            px_stage<FMT, 2>(row, s + 1, part0, h, o);
+#pragma unroll
+            for (int i = 0; i < 4; i++) *(uint4 *)(A + AB + px_group<FMT, 2>(i, part0) * 2048) = o[i];
+          }
+          if (s == 0 && part0 == 0) {   // (the scales of the super-block four back have been read: its accumulators were, before the stages that were waited for here)
             scr[(jj & 3) * 128 + r] = scale;
             __syncwarp();
             if (lane == 0) mbar_arrive(sc_full(jj & 3));
           }
-          if (s + SS == 4 && part == 0 && px_offs(FMT)) { *(uint4 *)(oa + r * 16) = off[0]; *(uint4 *)(oa + (128 + r) * 16) = off[1]; }
+          if (s + SS == 4 && part0 == 0 && px_offs(FMT)) { *(uint4 *)(oa + r * 16) = off[0]; *(uint4 *)(oa + (128 + r) * 16) = off[1]; }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads these bytes through the async proxy
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(lead + (a_full(slot) - bar_s));
@@ -359,9 +372,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
         }
       }
     }
-  } else if (warp < 12) {
-    px_reg_dec<PX1_REG_ISSUE>();
-    if (warp == 8) {
+  } else if (warp < UW + 4) {
+    px_reg_dec<px1_reg_issue(FMT, RU)>();
+    if (warp == UW) {
       // ---- weights: lane t requests the t-th 16-row tile of every chunk of the CTA's 128 rows ----
       int rs = 0;
       uint32_t rpar = 1;
@@ -384,7 +397,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
           if (++rs == NRAW) { rs = 0; rpar ^= 1u; }
         }
       }
-    } else if (warp == 9) {
+    } else if (warp == UW + 1) {
       // ---- activations: the CTA's plane ----
       if (lane == 0) {
         int slot = 0;
@@ -408,7 +421,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
           }
         }
       }
-    } else if (warp == 11) {
+    } else if (warp == UW + 3) {
       // ---- tells the leader that the other CTA's activations are there ----
       if (lane == 0 && rank == 1) {
         int slot = 0;
@@ -468,11 +481,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
     }
   } else {
     // ---- accumulators into sums: lane quarter q, a weight row a thread; the two warps of a quarter have half of the prompt rows each ----
-    px_reg_inc<PX1_REG_READ>();
+    px_reg_inc<px1_reg_read(FMT, RU)>();
     constexpr int RH = RU / 2;
-    const int q = warp & 3, half = (warp - 12) >> 2, R = a.R;
+    const int q = warp & 3, half = (warp - UW - 4) >> 2, R = a.R;
     const uint32_t t0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * RH);
-    f32x2 acc[RH / 2];
+    f32x2 acc[RH / 2], sum[NPL == 2 ? RH / 2 : 1];
     const f32x2 inv = x2_pack(XP_LO_INV, XP_LO_INV);
     int jj = 0, dd = 0;
     for (int u = unit0; u < nunits; u += ustep) {
@@ -485,6 +498,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
         wait(sc_full(jj & 3), (uint32_t)(jj >> 2) & 1u);
         const float scf = scr[(jj & 3) * 128 + 32 * q + lane];
         const f32x2 sc = x2_pack(scf, scf);
+        if constexpr (NPL == 2) {
+#pragma unroll
+          for (int j = 0; j < RH / 2; j++) sum[j] = 0;
+        }
 #pragma unroll 1
         for (int p = 0; p < 4 / SS; p++, dd++) {
           const uint32_t t1 = t0 + (uint32_t)((dd & 1) * 256);
@@ -502,8 +519,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
               if (lane == 0) mbar_arrive_cluster(lead + (d_empty(dd & 1) - bar_s));
             }
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc[j0 / 2 + j] = x2_fma(sc, x2_fma(w[j], inv, v[j]), acc[j0 / 2 + j]);
+            for (int j = 0; j < 8; j++) {
+              const f32x2 x = x2_fma(w[j], inv, v[j]);
+              if constexpr (NPL == 2) sum[j0 / 2 + j] = x2_add(sum[j0 / 2 + j], x);
+              else acc[j0 / 2 + j] = x2_fma(sc, x, acc[j0 / 2 + j]);
+            }
           }
+        }
+        if constexpr (NPL == 2) {
+#pragma unroll
+          for (int j = 0; j < RH / 2; j++) acc[j] = x2_fma(sc, sum[j], acc[j]);
         }
       }
       const int tile = tile_of(u);
@@ -529,7 +554,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
   __syncwarp();
   t5_fence_before();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // no CTA leaves while the other still arrives here or reads its memory
-  if (warp == 10) {
+  if (warp == UW + 2) {
     t5_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
@@ -557,7 +582,7 @@ __device__ __forceinline__ void pt_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_
       : "memory");
 }
 template <int FMT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pft(const PfArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_THREADS, 1) k_pft(const PfArgs a) {
   constexpr int RU = PT_RU, NB = PT_NB, SPB = 4 / px_slot_stages(RU), NPL = px_planes(FMT), NP = pt_items(FMT), SI = 4 / NP, N = 2 * RU, TB = tile_bytes(FMT), CH = px_chunk(FMT), NRAW = pt_raws(FMT);
   constexpr int RAWB = px_raw_bytes(FMT), SLB = px_slot_bytes(FMT, RU), PLB = px_b_bytes(RU), OPB = px_ob_bytes(RU), ND = 128 / N;   // SPB: slots of activations a super-block (SI: 64-column parts an item); ND: accumulators a group
   static_assert(NRAW >= 2 && pt_smem(FMT) <= PX_SMEM_MAX && NB % (2 * SPB) == 0 && ND >= 1, "a form that does not fit");
@@ -776,7 +801,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
     constexpr int RH = RU / 2;
     const int q = warp & 3, half = (warp - 12) >> 2, R = a.R;
     const uint32_t t0 = tmem + 256u + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * RH);
-    f32x2 acc[RH / 2];
+    f32x2 acc[RH / 2], sum[NPL == 2 ? RH / 2 : 1];
     const f32x2 inv = x2_pack(XP_LO_INV, XP_LO_INV);
     int j0 = 0;
     for (int u = unit0; u < nunits; u += ustep) {
@@ -786,27 +811,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PX1_THREADS, 1) k_pf
 #pragma unroll
       for (int j = 0; j < RH / 2; j++) acc[j] = 0;
 #pragma unroll 1
-      for (int k = 0; k < nsl * NP; k++) {
-        const int jj = j0 + k / NP, p = k % NP, g = jj & 1, it = (jj >> 1) * NP + p, di = it % ND, dbar = 2 * g + di;   // in the columns' order, as k_pfx1 adds them
-        if (p == 0) wait(sc_full(jj & 3), (uint32_t)(jj >> 2) & 1u);
+      for (int c = 0; c < nsl; c++) {
+        const int jj = j0 + c, g = jj & 1;
+        wait(sc_full(jj & 3), (uint32_t)(jj >> 2) & 1u);
         const float scf = scr[(jj & 7) * 128 + 32 * q + lane];
         const f32x2 sc = x2_pack(scf, scf);
-        const uint32_t t1 = t0 + (uint32_t)(128 * g + di * N);
-        wait(d_full(dbar), (uint32_t)(it / ND) & 1u);
-        t5_fence_after();
+        if constexpr (NPL == 2) {
 #pragma unroll
-        for (int i0 = 0; i0 < RH; i0 += 16) {
-          f32x2 v[8], w[8];
-          t5_ld16x2(t1 + i0, v);
-          t5_ld16x2(t1 + RU + i0, w);
-          t5_wait_ld();
-          if (i0 + 16 == RH) {   // given back before the last of it are added up
-            t5_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(lead + (d_empty(dbar) - bar_s));
+          for (int j = 0; j < RH / 2; j++) sum[j] = 0;
+        }
+#pragma unroll (NPL == 2 ? NP : 1)   // (not unrolled, the sums of two planes cost 20 rows of the 9B shape 6 %)
+        for (int p = 0; p < NP; p++) {   // in the columns' order, as k_pfx1 adds them
+          const int it = (jj >> 1) * NP + p, di = it % ND, dbar = 2 * g + di;
+          const uint32_t t1 = t0 + (uint32_t)(128 * g + di * N);
+          wait(d_full(dbar), (uint32_t)(it / ND) & 1u);
+          t5_fence_after();
+#pragma unroll
+          for (int i0 = 0; i0 < RH; i0 += 16) {
+            f32x2 v[8], w[8];
+            t5_ld16x2(t1 + i0, v);
+            t5_ld16x2(t1 + RU + i0, w);
+            t5_wait_ld();
+            if (i0 + 16 == RH) {   // given back before the last of it are added up
+              t5_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(lead + (d_empty(dbar) - bar_s));
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+              const f32x2 x = x2_fma(w[j], inv, v[j]);
+              if constexpr (NPL == 2) sum[i0 / 2 + j] = x2_add(sum[i0 / 2 + j], x);
+              else acc[i0 / 2 + j] = x2_fma(sc, x, acc[i0 / 2 + j]);
+            }
           }
+        }
+        if constexpr (NPL == 2) {
 #pragma unroll
-          for (int j = 0; j < 8; j++) acc[i0 / 2 + j] = x2_fma(sc, x2_fma(w[j], inv, v[j]), acc[i0 / 2 + j]);
+          for (int j = 0; j < RH / 2; j++) acc[j] = x2_fma(sc, sum[j], acc[j]);
         }
       }
       j0 += nsl;

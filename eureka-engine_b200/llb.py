@@ -86,7 +86,7 @@ def lib() -> C.CDLL:
             "llb_b200_pf_gemm": (i32, [i32, u64, i32, i32, u64, i32, u64, i32]),
             "llb_b200_gemm_fits": (i32, [i32, i32, i32, i32]), "llb_b200_gemm_kernel": (i32, [i32, i32, i32, i32, i32, i32, C.POINTER(i32)]),
             "llb_b200_gemm3_trace": (i32, [i32, i32, i32, i32, C.POINTER(i32), i32]), "llb_b200_gemm3_bar_count": (i32, [i32, i32]),
-            "llb_b200_pf_trace": (i32, [i32, i32, i32, i32, i32, i32, C.POINTER(i32), i32]), "llb_b200_pf_bar_count": (i32, [i32, i32, i32]),
+            "llb_b200_pf_trace": (i32, [i32, i32, i32, i32, i32, i32, C.POINTER(i32), i32]), "llb_b200_pf_bar_count": (i32, [i32, i32, i32, i32]),
             "llb_b200_gemm_ksplit": (i32, [i32, i32, i32, i32, i32]), "llb_b200_ring_ksplit": (i32, [i32, i32, i32, i32, i32, i32]),
             "llb_b200_kernel_by_name": (vp, [C.c_char_p]),
             "llb_b200_launch": (i32, [vp, C.c_uint, C.c_uint, C.c_uint, C.c_uint, C.POINTER(vp), C.c_uint]),

@@ -273,7 +273,7 @@ LLB_API int llb_b200_gemm3_bar_count(int nc, int bar);
 /* The same for the prompt path's kernels: 0 k_pf_attn (form: head dimension; units x nsl tiles of 32 positions), 1 k_pfx1 or k_pft (form: 32, 64
  * or 128 rows), 2 k_pfx2; a CTA's `units` work units of nsl super-blocks each.  A pair's second CTA has its barriers 64 numbers on. */
 LLB_API int llb_b200_pf_trace(int kernel, int form, int fmt, int units, int nsl, int agent, int *ops, int cap);
-LLB_API int llb_b200_pf_bar_count(int kernel, int form, int bar);
+LLB_API int llb_b200_pf_bar_count(int kernel, int form, int fmt, int bar);
 LLB_API void llb_spec_close(llb_spec *m);
 LLB_API int llb_spec_reset(llb_spec *m);                       /* host/llb_host.c:1915-1928 */
 LLB_API int llb_spec_prefill(llb_spec *m, const int *ids, int n);

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+BARS = (1.5e-7, 1.55e-7, 1.7e-7)   # what is measured, 1.28 to 1.38, 1.33 to 1.45 and 1.5 to 1.62e-7, and a few percent
 
 
 def _run(llb, packs, dev, ty, raw, rows, K, x, ksplit):
@@ -83,3 +84,30 @@ def test_sums_do_not_climb(llb, packs, oracle, dev, power):
         ref = x.astype(np.float64) @ deq.T
         err[kind] = np.linalg.norm(_run(llb, packs, dev, "Q6_K", raw, rows, K, x, 4) - ref) / np.linalg.norm(ref)
     assert err["|N|"] < 1.25 * err["N"], err
+
+
+@pytest.mark.parametrize("ty", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
+def test_forms_give_the_same_bits(llb, packs, dev, ty):
+    """A row's sums do not depend on how many rows come with it (up to 128: three forms of the kernel)."""
+    rows, K = 400, 5120
+    rng = np.random.default_rng(13)
+    raw = packs.QUANT[ty](torch.from_numpy(rng.standard_normal((rows, K), dtype=np.float32) * 0.02)).numpy()
+    x = rng.standard_normal((128, K), dtype=np.float32)
+    got = [_run(llb, packs, dev, ty, raw, rows, K, x[:n], 3) for n in (20, 32, 33, 64, 65, 128)]
+    for g in got[:-1]:
+        assert np.array_equal(g, got[-1][:len(g)])
+
+
+@pytest.mark.parametrize("ty", ["Q6_K", "Q8_0"])
+@pytest.mark.parametrize("kind", ["N", "|N|", "silu", "1+.1N"])
+def test_error_against_64_bits(llb, packs, oracle, dev, ty, kind):
+    """The formats whose T-row passes are exact but for the activations' 22 bits and fp32 sums (1.0e-7 to 1.2e-7 of Q6_K, 0.9e-7 to 2.0e-7 of Q8_0), at the K-slices that
+    a prompt takes."""
+    rng = np.random.default_rng(17)
+    for rows, K, ksplit, bar in ((512, 1024, 4, BARS[0]), (512, 5120, 3, BARS[1]), (512, 17408, 3, BARS[2])):
+        raw = packs.QUANT[ty](torch.from_numpy(rng.standard_normal((rows, K), dtype=np.float32) * 0.02)).numpy()
+        r = rng.standard_normal((40, K), dtype=np.float32)
+        x = {"N": r, "|N|": np.abs(r), "1+.1N": 1 + np.float32(0.1) * r, "silu": r / (1 + np.exp(-r)) * rng.standard_normal((40, K), dtype=np.float32)}[kind]
+        ref = x.astype(np.float64) @ oracle.Oracle.deq_rows(packs.FMT[ty], raw, rows, K).astype(np.float64).T
+        err = np.linalg.norm(_run(llb, packs, dev, ty, raw, rows, K, x, ksplit) - ref) / np.linalg.norm(ref)
+        assert err < bar, (K, err)
