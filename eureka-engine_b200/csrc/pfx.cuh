@@ -26,8 +26,9 @@
 // What bounds k_pfx2 is the power the tensor cores may draw: gate|up of the 27B shape, 256 rows, 223 GFLOP of products in 136 us = 1.64 PFLOP/s
 // (a loop of nothing but these MMAs on random operands runs at 1.37 to 1.44 GHz and 1.65 to 1.74 PFLOP/s, on zeros at 1.82 GHz); the kernel
 // of three products took 185 us.  A 3011-token prompt on that shape 515 -> 432 ms.  Error against 64 bits, N(0, 1) activations,
-// 5120 / 17408 columns: Q4_K 3.1e-7 / 3.4e-7, Q5_K 3.5e-7 / 3.7e-7 (6.1e-6 / 2.0e-5 before); k_pfx1 2.1e-7 / 2.8e-7, Q6_K and Q8_0
-// 2.0e-7 / 3.2e-7.
+// 5120 / 17408 columns in a prompt's K-slices: k_pfx2 Q4_K 3.1e-7 / 3.4e-7, Q5_K 3.5e-7 / 3.7e-7 (k_pfmm 6.1e-6 / 2.0e-5); k_pfx1 and k_pft beside the passes of eight rows
+// whose place they take: Q4_K 1.9e-7 / 2.2e-7 (10e-7 / 3.2e-7 there), Q5_K 2.1e-7 / 2.3e-7 (4.1e-7 / 3.8e-7), Q6_K 1.07e-7 / 1.29e-7 (1.08e-7 / 1.20e-7), Q8_0 1.11e-7 /
+// 1.34e-7 (1.27e-7 / 2.0e-7); 1024 columns of Q8_0 1.00e-7 (0.90e-7); with silu(g) u Q6_K 1.10e-7 / 1.32e-7 (1.12e-7 / 1.22e-7), Q8_0 1.14e-7 / 1.36e-7 (1.33e-7 / 2.05e-7).
 // Every wait is bounded; one that runs out sets *err, all roles then run through, tensor memory is freed and the kernel returns.
 #pragma once
 #include "pfmm.cuh"
@@ -46,6 +47,10 @@ __host__ __device__ constexpr int px_ob_bytes(int RU) { return RU * 32; }       
 // 64-column parts after which k_pfx1's accumulators are read, a stage's: the tensor core truncates where it adds to one, so that a sum loses about 2e-8 of itself an
 // MMA.  Its prompts take the place of verify rows, so it is read as often as that hides behind the MMAs.
 __host__ __device__ constexpr int px_drain(int fmt) { return px_planes(fmt) == 2 ? 1 : 2; }
+// The part of a sum of two planes that the truncations of its four additions with the larger plane take off, always towards zero: measured 8.9e-8 for Q8_0 and 8.2e-8 for
+// Q6_K, whatever the columns, and for activations of either sign or one, with short or long tails (8.8e-8 for silu(g) u).  The sums are given it back at the end, which is
+// one unit of the last place.  Where the sums are exact without it they lose by that: 1 + 0.1 N 1.02e-7 both ways, activations of which 2 % are not zero 0.8 -> 1.1e-7.
+constexpr float PX_LOST = 8.5e-8f;
 // k_pfx1's rings: codes in stages of eight MMAs, 128 columns of one plane or 64 of two (a stage costs the issuing warp and the unpacking ones
 // some 400 cycles whatever is in it); not more than a super-block, because the offsets' step has one buffer on the weight rows' side, which a
 // super-block's last stage fills and the same stage of the next fills again, when the MMAs of the stage `px_na` before that one are done;
@@ -541,6 +546,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(px1_threads(FMT, RU)
         for (int j = 0; j < RH; j += 2) {
           float y0, y1;
           x2_unpack(acc[j / 2], y0, y1);
+          if (NPL == 2) { y0 = fmaf(y0, PX_LOST, y0); y1 = fmaf(y1, PX_LOST, y1); }
           if (j < n) *out = y0;
           out += os;
           if (j + 1 < n) *out = y1;
@@ -861,6 +867,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_THREADS, 1) k_pft
         for (int j = 0; j < RH; j += 2) {
           float y0, y1;
           x2_unpack(acc[j / 2], y0, y1);
+          if (NPL == 2) { y0 = fmaf(y0, PX_LOST, y0); y1 = fmaf(y1, PX_LOST, y1); }
           if (j < n) *out = y0;
           out += os;
           if (j + 1 < n) *out = y1;

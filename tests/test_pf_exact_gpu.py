@@ -6,7 +6,9 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
-BARS = (1.5e-7, 1.55e-7, 1.7e-7)   # what is measured, 1.28 to 1.38, 1.33 to 1.45 and 1.5 to 1.62e-7, and a few percent
+# what two seeds show, 0.97 to 1.07, 1.07 to 1.22 and 1.26 to 1.36e-7, and 7 %: with 1 + 0.1 N the forty results of a weight row are nearly the same, so that the norm
+# is that of 512 independent roundings, whose size goes with their mantissas (1.10 and 1.22e-7 for the two seeds)
+BARS = (1.15e-7, 1.31e-7, 1.46e-7)
 
 
 def _run(llb, packs, dev, ty, raw, rows, K, x, ksplit):
