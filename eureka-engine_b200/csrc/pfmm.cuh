@@ -13,7 +13,7 @@
 //   * a pair because each CTA then stages half of the chunk's rows only: a step of 16 columns moves 40 KB through its shared
 //     memory (60 KB alone), and a third stage fits.  N = 256 because a dequantised weight (14.5 thread instructions)
 //     then serves all rows of a chunk.  What bounds it is the tensor pipe, 384 cycles a step of 433.  gate|up of the 27B shape,
-//     256 rows: 270 us with two units of N = 128 a stage, 232 us with one CTA and N = 256, 194 us now (single CTAs took
+//     256 rows: 270 us with two units of N = 128 a stage, 232 us with one CTA and N = 256, 185 us so (single CTAs took
 //     528 cycles a step: the issuing threads' three barriers a stage and MMAs out of vector registers were their chain);
 //   * the activation planes arrive by TMA: the chunk's activations are kept in global memory in the order the operand
 //     wants (two units of 128 rows, k-group major, common.cuh), so a CTA's 64-column stage of one plane is ONE contiguous

@@ -23,9 +23,9 @@
 //   k_pft   the same for up to 32 rows with the codes in tensor memory.
 // Weights come as bulk copies of whole super-blocks of a 16-row tile into a ring of their own.
 //
-// What bounds k_pfx2 is the power the tensor cores may draw: gate|up of the 27B shape, 256 rows, 223 GFLOP of products in 136 us = 1.64 PFLOP/s
-// (a loop of nothing but these MMAs on random operands runs at 1.37 to 1.44 GHz and 1.65 to 1.74 PFLOP/s, on zeros at 1.82 GHz); the kernel
-// of three products took 185 us.  A 3011-token prompt on that shape 515 -> 432 ms.  Error against 64 bits, N(0, 1) activations,
+// gate|up of the 27B shape, 256 rows: 194 GFLOP of products in 136 us = 1.43 PFLOP/s, 87 % of cuBLAS's measured burst; the kernel of three products took 185 us.  What bounds
+// k_pfx2 is the tensor pipe, 83 % active at the 1.57 GHz that the power limit leaves it (a loop of nothing but these MMAs on random operands runs at 1.37 to 1.44 GHz and 1.65
+// to 1.74 PFLOP/s, on zeros at 1.82 GHz), and how the tiles fill the chip: 136 units on 74 pairs of SMs are 92 % of two rounds.  A 3011-token prompt on that shape 515 -> 432 ms.  Error against 64 bits, N(0, 1) activations,
 // 5120 / 17408 columns in a prompt's K-slices: k_pfx2 Q4_K 3.1e-7 / 3.4e-7, Q5_K 3.5e-7 / 3.7e-7 (k_pfmm 6.1e-6 / 2.0e-5); k_pfx1 and k_pft beside the passes of eight rows
 // whose place they take: Q4_K 1.9e-7 / 2.2e-7 (10e-7 / 3.2e-7 there), Q5_K 2.1e-7 / 2.3e-7 (4.1e-7 / 3.8e-7), Q6_K 1.07e-7 / 1.29e-7 (1.08e-7 / 1.20e-7), Q8_0 1.11e-7 /
 // 1.34e-7 (1.27e-7 / 2.0e-7); 1024 columns of Q8_0 1.00e-7 (0.90e-7); with silu(g) u Q6_K 1.10e-7 / 1.32e-7 (1.12e-7 / 1.22e-7), Q8_0 1.14e-7 / 1.36e-7 (1.33e-7 / 2.05e-7).
