@@ -124,8 +124,8 @@ LLB_API int llb_b200_gemm_host(int fmt, llb_b200_dptr w, int rows, int K, const 
                        llb_b200_dptr x_dev, llb_b200_dptr y_dev);
 
 /* The prompt path's dense GEMM alone (replaces the reference's chunked tensor-core prefill GEMM, tools/pf27/pfmm.cuh:311-384):
- * Y[r][n] = sum_c W[n][c] x[r][c] for R <= 256 rows (two units of 128 against every dequantised weight stage) of f32 activations x [R][K] against a weight matrix in the device
- * layout, out f32 [R][rows]; tcgen05.mma with both operands as two fp16 planes (about 22 bits) and fp32 sums in tensor memory.  ksplit = 0
+ * Y[r][n] = sum_c W[n][c] x[r][c] for R <= 256 rows of f32 activations x [R][K] against a weight matrix in the device layout, out f32 [R][rows]; tcgen05.mma on the
+ * activations' two fp16 planes (about 22 bits) and the weights' exact codes (Q6_K and Q8_0 beyond 128 rows: their two fp16 planes), sums in fp32.  ksplit = 0
  * picks the K-split (at most K / 256 slices of whole super-blocks).  Synchronises; scratch is allocated and freed inside the call. */
 LLB_API int llb_b200_pf_gemm(int fmt, llb_b200_dptr w, int rows, int K, llb_b200_dptr x_f32, int R, llb_b200_dptr out_f32, int ksplit);
 
@@ -287,6 +287,9 @@ LLB_API int llb_spec_position(const llb_spec *m);
 /* How llb_spec_prefill feeds a prompt.  mode 0 (default): at the verify path's precision; more than four rows, and more than k + 1, in pieces of up to 128
  * rows through dense tcgen05 GEMMs on the exact weight codes, fewer (and every row of a model with routed experts, of a tensor-parallel rank, and
  * where LLB_PREFILL_ROWS was set at open) through T-row verify passes.  What the dense path leaves behind depends on neither k nor the other streams.
+ * Its buffers (0.1 GB at the 0.8B shape, 0.3 at the 27B one) are allocated at the first prompt that takes it, in one block that the weights' engines share, and go
+ * with the weights; engines on one set of weights may be given prompts from several threads at once.  Without room mode 0 takes T-row passes, mode 1 is an error, and the next
+ * prompt looks for room again.
  * mode 1 (also LLB_PREFILL=fast in the environment at open, the reference's switch,
  * host/llb_host.c:206): all but the last k + 1 rows in chunks of 256 rows through dense tcgen05 GEMMs (Q6_K and Q8_0 weights as two fp16 planes)
  * (replaces pf_take / spec_pf / spec_take, host/llb_pf.h:551, host/llb_host.c:1831-1899): trunk K/V, conv history and
