@@ -174,7 +174,9 @@ static inline float *ring_of(const llb_spec *m, int il, int b) { return m->ring[
 static inline float *state_of(const llb_spec *m, int il, int b) { return m->S[il] + (size_t)b * m->s_group; }
 static inline int *hist_of(const llb_spec *m, int b) { return m->hist ? m->hist + (size_t)b * (m->max_ctx + 16) : nullptr; }
 // the launchers' stream geometry and GEMM kernels while this engine enqueues (engines of different shapes may coexist)
+static std::recursive_mutex g_enqueue;
 struct StreamScope {
+  std::lock_guard<std::recursive_mutex> hold{g_enqueue};   // (a prompt enqueues kernels outside any graph, and another thread's engine may at the same time)
   Streams was;
   const int was_gemm3;
   explicit StreamScope(const llb_spec *m, bool single = false) : was(ops_streams()), was_gemm3(g_llb.gemm3) {

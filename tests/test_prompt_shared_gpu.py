@@ -31,6 +31,24 @@ def _same(a, b):
     return all(np.array_equal(x, y) for x, y in zip(a[0], b[0])) and all(np.array_equal(x, y) for x, y in zip(a[1], b[1]))
 
 
+def _at_once(calls):
+    gate, errors = threading.Barrier(len(calls)), []
+
+    def run(call):
+        try:
+            gate.wait()
+            call()
+        except Exception as e:   # noqa: BLE001 - any failure of a thread is the test's
+            errors.append(repr(e))
+
+    ts = [threading.Thread(target=run, args=(c,)) for c in calls]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors
+
+
 @pytest.mark.parametrize("fast", [False, True])
 def test_first_prompts_at_once(pkg, packs, model, fast):
     cfg = model[0].cfg
@@ -45,23 +63,9 @@ def test_first_prompts_at_once(pkg, packs, model, fast):
             e.close()
     for _ in range(3):
         engs = _open(pkg, model, len(prompts))
-        gate, errors = threading.Barrier(len(engs)), []
-
-        def feed(eng, p):
-            try:
-                gate.wait()
-                eng.prefill(p)
-            except Exception as e:   # noqa: BLE001 - any failure of a thread is the test's
-                errors.append(repr(e))
-
         for e in engs:
             e.set_prefill(fast)
-        ts = [threading.Thread(target=feed, args=a) for a in zip(engs, prompts)]
-        for t in ts:
-            t.start()
-        for t in ts:
-            t.join()
-        assert not errors
+        _at_once([lambda e=e, p=p: e.prefill(p) for e, p in zip(engs, prompts)])
         for e, w in zip(engs, want):
             assert _same(_result(e, cfg), w)
         for e in engs:
@@ -143,3 +147,31 @@ def test_rows_of_the_last_chunk(pkg, packs, model):
     assert np.array_equal(first.read_state(6, 0, 149 - 128 - 1), first.read_state(4, 0, 3))
     eng.close()
     first.close()
+
+
+def test_engines_of_different_streams_at_once(pkg, packs, model):
+    """One engine feeds the prompts of three streams, others one each, from threads: nobody enqueues with another one's stream geometry."""
+    cfg = model[0].cfg
+    first = pkg.llb.SpecEngine(model[0], model[1], k=3, max_ctx=360)
+    many, other = first.sibling(k=3, max_ctx=360, streams=3), first.sibling(k=0, max_ctx=360)
+    three = [packs.synth_prompt(30 + b, n, cfg.vocab_size) for b, n in enumerate((150, 40, 30))]
+    ones = [packs.synth_prompt(35 + b, 60 + b, cfg.vocab_size) for b in range(2)]
+
+    def three_result():
+        return [many.read_state_stream(b, 0, 0) for b in range(3)], [many.cycle_streams() for _ in range(3)]
+
+    def same(a, b):
+        return all(np.array_equal(x, y) for x, y in zip(a[0], b[0])) and all(
+            np.array_equal(i, j) and np.array_equal(t, u) for x, y in zip(a[1], b[1]) for (i, t), (j, u) in zip(x, y))
+
+    many.prefill_streams(three)
+    want = [three_result()]
+    for e, p in zip((first, other), ones):
+        e.prefill(p)
+        want.append(_result(e, cfg))
+    for _ in range(5):
+        _at_once([lambda: many.prefill_streams(three), lambda: first.prefill(ones[0]), lambda: other.prefill(ones[1])])
+        assert same(three_result(), want[0])
+        assert _same(_result(first, cfg), want[1]) and _same(_result(other, cfg), want[2])
+    for e in (many, other, first):
+        e.close()
