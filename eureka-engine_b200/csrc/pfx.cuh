@@ -5,7 +5,7 @@
 //   Q4_K, Q5_K  sc (q - 8) and sc (q - 16), at most 504 and 1008.  What the centring took and the mins are one more K = 16 step of a
 //               super-block, 32 (8 sc - (dmin / d) m) as two fp16 halves against the means of the activations' 32-column groups
 //   Q6_K        sc (q - 32), at most 4096: fp16 product and its exact remainder, two planes.  (Planes of the code's low four and high two bits are exact too and cheaper to
-//               unpack, but they are large and cancel where codes are small: with weights of N^3 and activations of one sign, 17408 columns, what is truncated off
+//               unpack, 5120 x 17408 and 20 / 50 / 120 rows 40 / 60 / 70 us where this takes 46 / 66 / 70, but they are large and cancel where codes are small: with weights of N^3 and activations of one sign, 17408 columns, what is truncated off
 //               their sums came to 2.9e-6 of the result)
 //   Q8_0        d q with the eight d's of the super-block scaled by a common power of two: fp16 product and its exact remainder, two planes
 //
@@ -571,7 +571,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(px1_threads(FMT, RU)
 // what one group waits for the other fills.  An ITEM is what 64 columns of tensor memory hold, 128 columns of one plane of codes or 64 of two; a
 // group has two such buffers and two accumulators, so that it unpacks one item while the other is multiplied, and multiplies one while the other
 // is read.  Sums are added in the columns' order, as k_pfx1 adds them: the same bits.  What bounds it is a group's chain, 4000 cycles a super-block, of
-// which unpacking is half.  Twenty rows, k_pfx1 with 32 / this: Q4_K 34816 x 5120 59.5 / 44 us, 5120 x 6144 17.8 / 15, Q6_K 5120 x 17408 56 / 43,
+// which unpacking is half.  Twenty rows, k_pfx1 with 32 / this: Q4_K 34816 x 5120 59.5 / 44 us, 5120 x 6144 17.8 / 15, Q6_K 5120 x 17408 (planes of bits) 56 / 43,
 // Q8_0 24576 x 4096 61 / 47, Q5_K 8192 x 4096 19 / 17.  With 64 rows only one accumulator a group fits: Q4_K 70 / 63, Q6_K 65 / 73, Q8_0 70 / 80, not kept.
 // A barrier is only ever waited for by one group, which sees every phase of it (a phase's parity tells nothing to one that missed the phase before).
 __host__ __device__ constexpr int pt_items(int fmt) { return 2 * px_planes(fmt); }       // of a super-block
